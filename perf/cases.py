@@ -34,6 +34,9 @@ SIZES = {
 EXPERTS, CAPACITY_FACTOR, AUX_FACTOR, ROUTER_Z_FACTOR = 8, 1.25, 1e-2, 1e-3
 Z_LOSS = 1e-4
 LEARNING_RATE = 0.01  # constant * rsqrt_decay after 10000 warm-up steps
+# Training goes on from this step with these second moments: at step 0 the update of a vector is
+# the sign of its gradient, which says nothing about how well a small gradient was computed.
+STEP, SECOND_MOMENT = 1000, 1.0
 EOS = 1
 
 
@@ -235,18 +238,19 @@ def _weights(case, seed):
     # a trained router sends a token by what it is: its direction is part of the embedding
     emb = w["token_embedder/embedding"]
     u = torch.linalg.qr(torch.randn(d, EXPERTS, generator=g, device="cuda"))[0]
-    emb.add_(6.0 * u.t()[torch.arange(vocab, device="cuda") % EXPERTS])
+    emb.add_(12.0 * u.t()[torch.arange(vocab, device="cuda") % EXPERTS])
     for name in w:
       if name.endswith("router_weights/w/kernel"):
-        w[name] = u + 0.02 * d ** -0.5 * w[name]
+        w[name] = 0.4 * u + 0.02 * d ** -0.5 * w[name]
   if case["job"] == "decode":
-    # a trained model is sure of most tokens: each has a successor that stands out, and the
+    # as in a trained model some token stands out at every step: each has a successor, far above
+    # the rest of the vocabulary together with which it shares the probability; the
     # end-of-sequence token does not come up before the last step
     emb, nxt = w["token_embedder/embedding"], _successors(vocab, seed)
     logits = torch.zeros(vocab, d, device="cuda")
     src = torch.cat([torch.arange(1, device="cuda"), torch.arange(2, vocab, device="cuda")])
     logits.index_add_(0, nxt[src], emb[src])
-    w["decoder/logits_dense/kernel"] = (logits.t() * (16.5 / d)).contiguous()
+    w["decoder/logits_dense/kernel"] = (logits.t() * (10.0 / d)).contiguous()
   return {k: v.bfloat16().float() for k, v in w.items()}
 
 
@@ -257,9 +261,9 @@ def _lengths(b, full, g):
 
 
 def _tokens(b, l, lengths, vocab, g):
-  """Zipf-like ids, zero after each row's length."""
+  """Zipf-like ids (the most frequent one is about 2 % of them), zero after each row's length."""
   u = torch.rand(b, l, generator=g, device="cuda", dtype=torch.float64)
-  ids = (2 + (vocab - 2) ** u - 1).long().clamp(2, vocab - 1)
+  ids = (2 + (vocab - 2) ** (u ** 0.7) - 1).long().clamp(2, vocab - 1)
   return torch.where(torch.arange(l, device="cuda")[None] < lengths[:, None], ids, 0)
 
 
@@ -351,8 +355,11 @@ def prepare(case, seed):
   state = {"case": dict(case), "model": model, "batch": _batch(case, seed), "flat": flat,
            "params": variables["params"]}
   if case["job"] in ("train", "grads"):
-    state["train_state"] = train_state_lib.FlaxOptimTrainState.create(model.optimizer_def,
-                                                                      variables)
+    train_state = train_state_lib.FlaxOptimTrainState.create(model.optimizer_def, variables)
+    for name, slot in tree_utils.flatten_dict(train_state.param_states).items():
+      if name.rsplit("/", 1)[-1] in ("v", "v_row", "v_col"):
+        slot.fill_(SECOND_MOMENT)
+    state["train_state"] = train_state.replace_step(STEP)
     trainer.attach_compute_buffers(state["train_state"].params)
   else:
     trainer.attach_compute_buffers(variables["params"], main_grad=False)
@@ -505,14 +512,16 @@ class _Model64:
     return x @ self.w["decoder/logits_dense/kernel"]
 
 
-def _adafactor_first_step(name, p, g):
-  """Adafactor's update at step 0 (the second moments are the squared gradient's alone)."""
+def _adafactor(name, p, g):
+  """One Adafactor update from STEP with every second moment at SECOND_MOMENT."""
+  decay = 1.0 - (STEP + 1.0) ** -0.8
+  ema = lambda m: decay * SECOND_MOMENT + (1.0 - decay) * m
   gsq = g * g + 1e-30
   if p.dim() >= 2 and "rel_embedding" not in name and "router_weights" not in name:
-    row, col = gsq.mean(-1, keepdim=True), gsq.mean(-2, keepdim=True)
+    row, col = ema(gsq.mean(-1, keepdim=True)), ema(gsq.mean(-2, keepdim=True))
     v = row * col / row.mean(-2, keepdim=True)
   else:
-    v = gsq
+    v = ema(gsq)
   dims = (-2, -1) if p.dim() >= 2 else (-1,)  # experts are updated one by one
   y = g * v.rsqrt()
   y = y / y.square().mean(dims, keepdim=True).sqrt().clamp(min=1.0)
@@ -559,7 +568,7 @@ def exact(case, seed):
     out["grads"] = grads
     return out
   with torch.no_grad():
-    out["params"] = {k: _adafactor_first_step(k, w[k].detach(), g) for k, g in grads.items()}
+    out["params"] = {k: _adafactor(k, w[k].detach(), g) for k, g in grads.items()}
   if len(w) <= 31:
     out["grads"] = grads
   return out
@@ -568,9 +577,11 @@ def exact(case, seed):
 def tolerance(case):
   # bf16 activations and matrix operands with 32-bit sums. Measured against 64 bits: gradients
   # 0.002 to 0.012 (the key projections are the noisiest), token log-likelihoods 0.0005 to 0.001,
-  # sums of log-probabilities 0.01; tokens are the same unless two are nearly tied.
+  # sums of log-probabilities 0.01; tokens are the same unless two are nearly tied. A single
+  # gradient may be further off: a frequent token's row of the embedding gradient is an order of
+  # magnitude above the table's root mean square, and its small elements carry the row's error.
   if case["job"] == "decode":
-    return {"rel": 2e-2, "max": 0.2, "differ": 2e-3}
+    return {"rel": 3e-2, "max": 0.2, "differ": 2e-3}
   if case["job"] == "score":
     return {"rel": 4e-3, "max": 0.1}
-  return {"rel": 3e-2, "max": 0.5}
+  return {"rel": 3e-2, "max": 0.99}
