@@ -7,7 +7,12 @@ namespace t5x {
 
 constexpr int kBM = 128;
 constexpr int kBK = 64;
-constexpr int kGemmThreads = 192;
+// Epilogue warps of the plain kernels: two per TMEM lane quarter, each taking half of a tile's
+// columns. Four warps (one per quarter) need longer for a 128 x 256 tile than the tensor cores
+// need for K < ~1500, so that short-K products ran at the epilogue's pace (see the kernels).
+constexpr int kEpiWarps = 8;
+constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
+constexpr int kTpEpiWarps = 4;  // tensor-parallel kernels: one per quarter
 constexpr int kKernelIdGemm = 1;
 constexpr int kGemmTraceSlots = 8;
 long long* gemm_trace_buffer();  // host: the calling thread's trace buffer, or null
@@ -15,6 +20,8 @@ long long* gemm_trace_buffer();  // host: the calling thread's trace buffer, or 
   do {                                                                                    \
     if (p.trace != nullptr) p.trace[blockIdx.x * kGemmTraceSlots + (slot)] = global_timer_ns(); \
   } while (0)
+
+constexpr int kCeTileCols = 128;  // columns that one warp folds into one partial
 
 enum GemmEpilogue : int {
   kEpiPlain = 0,
@@ -48,8 +55,9 @@ struct GemmParams {
   // Cross-entropy epilogues. Column c of the product is vocabulary entry ce_vocab_start + c.
   const long long* ce_targets;  // [M] target ids
   int ce_vocab_start;
-  float* ce_part;          // kEpiCeStats: [M, tiles_n, 4] = max, sum exp(x - max), sum x, largest x
-  int* ce_arg;             // kEpiCeStats: [M, tiles_n] column of the largest x
+  int ce_tiles;            // kEpiCeStats: partials per row, one per kCeTileCols columns
+  float* ce_part;          // kEpiCeStats: [M, ce_tiles, 4] = max, sum exp(x - max), sum x, largest x
+  int* ce_arg;             // kEpiCeStats: [M, ce_tiles] column of the largest x
   float* ce_target_logit;  // kEpiCeStats: [M], written by the tile that holds the target
   const float* ce_lse;     // kEpiCeGrad: [M] log-sum-exp of the row over the whole vocabulary
   const float* ce_row_scale;  // kEpiCeGrad: [M] upstream gradient of the row's loss
@@ -125,7 +133,10 @@ __device__ __forceinline__ void store_row_bf16(__nv_bfloat16* dst, const float* 
       reinterpret_cast<uint4*>(dst)[i] = u;
     }
   } else {
-    for (int i = 0; i < 32 && i < n_valid; ++i) dst[i] = __float2bfloat16(v[i]);
+    // unrolled: an index known only at run time would put the caller's array in local memory
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (i < n_valid) dst[i] = __float2bfloat16(v[i]);
   }
 }
 
@@ -144,6 +155,7 @@ __device__ __forceinline__ void load_row_bf16(const __nv_bfloat16* src, float* v
       }
     }
   } else {
+#pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = (i < n_valid) ? __bfloat162float(src[i]) : 0.f;
   }
 }
@@ -222,6 +234,45 @@ __device__ __forceinline__ void staged_store_bf16(float* stage, const float (&v)
   __syncwarp();
 }
 
+// Reads a 32 x 32 bf16 block (rows `ldr` elements apart) into the staging block as 64-byte row
+// segments, and adds one row of it to a lane's 32 values. A residual read straight from its row
+// by each lane costs 32 separate lines per instruction, as described above.
+__device__ __forceinline__ void staged_load_bf16(float* stage, const __nv_bfloat16* src,
+                                                 long long ldr, int rows_valid, int lane) {
+  uint4* st4 = reinterpret_cast<uint4*>(stage);
+  const int c = lane & 3;
+  uint4 u[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int row = j * 8 + (lane >> 2);
+    u[j] = make_uint4(0u, 0u, 0u, 0u);
+    if (row < rows_valid)
+      u[j] = *reinterpret_cast<const uint4*>(src + static_cast<long long>(row) * ldr + c * 8);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int row = j * 8 + (lane >> 2);
+    st4[row * 8 + (c ^ (row & 7))] = u[j];
+  }
+  __syncwarp();
+}
+
+__device__ __forceinline__ void staged_add_row(const float* stage, float (&v)[32], int lane) {
+  const uint4* st4 = reinterpret_cast<const uint4*>(stage);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const uint4 u = st4[lane * 8 + (c ^ (lane & 7))];
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __bfloat1622float2(h[j]);
+      v[c * 8 + j * 2] += f.x;
+      v[c * 8 + j * 2 + 1] += f.y;
+    }
+  }
+  __syncwarp();  // the block may be overwritten
+}
+
 // Tile order: groups of kRasterGroup row tiles are walked column by column, so that the tiles
 // in flight at one time (one per SM or SM pair) share a few A row blocks and a few B column
 // blocks instead of one A block and every B block; the operands of a wave then fit in L2.
@@ -244,11 +295,11 @@ __device__ __forceinline__ void gemm_tile_coords(const GemmParams& p, int tile, 
 }
 
 // Epilogue of one 128-row accumulator tile held in TMEM columns [t_cols, t_cols + BN): the
-// calling warp owns lane quarter q (rows m0 + 32q .. +31), `c_vec_ok` says whether 16-byte
-// stores to C are legal.
-template <int BN, int EPI>
+// calling warp owns lane quarter q (rows m0 + 32q .. +31) and part `part` of PARTS of the tile's
+// columns, `c_vec_ok` says whether 16-byte stores to C are legal.
+template <int BN, int EPI, int PARTS>
 __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t t_row, int m0,
-                                                   int n0, int b, int q, int lane,
+                                                   int n0, int b, int q, int part, int lane,
                                                    bool c_vec_ok, float* stage = nullptr) {
   const int row = m0 + q * 32 + lane;
   const bool row_ok = row < p.M;
@@ -259,7 +310,8 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + b * p.c_batch_stride +
                          static_cast<long long>(row) * p.ldc;
 #pragma unroll 1
-    for (int c = 0; c < kHalf / 32; ++c) {
+    for (int c = part * (kHalf / 32 / PARTS); c < (part + 1) * (kHalf / 32 / PARTS); ++c) {
+      if (n0 + c * 32 >= p.N) break;  // warp-uniform: columns beyond the output
       uint32_t r0[32], r1[32];
       tmem_ld32(t_row + c * 32, r0);
       tmem_ld32(t_row + kHalf + c * 32, r1);
@@ -307,27 +359,38 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
     }
   } else {
 #pragma unroll 1
-    for (int c = 0; c < BN / 32; ++c) {
-      uint32_t r[32];
-      tmem_ld32(t_row + c * 32, r);
-      tmem_ld_wait();
+    for (int c = part * (BN / 32 / PARTS); c < (part + 1) * (BN / 32 / PARTS); ++c) {
       const int col = n0 + c * 32;
       const int n_valid = p.N - col;
+      if (n_valid <= 0) break;  // warp-uniform: columns beyond the output
+      uint32_t r[32];
+      tmem_ld32(t_row + c * 32, r);
       // whole 32-column blocks go out through the staging buffer (warp-uniform condition)
       const bool staged = stage != nullptr && n_valid >= 32 && rows_valid > 0 &&
                           (p.out_fp32 ? (p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0)
                                       : (c_vec_ok && p.accumulate == 0));
       if (staged) {
+        const bool r_vec_ok = EPI == kEpiResidual && p.ldr % 8 == 0 &&
+                              p.r_batch_stride % 8 == 0 &&
+                              (reinterpret_cast<uintptr_t>(p.R) & 15) == 0;
+        if (EPI == kEpiResidual && r_vec_ok)
+          staged_load_bf16(stage, p.R + b * p.r_batch_stride +
+                                      static_cast<long long>(m0 + q * 32) * p.ldr + col,
+                           p.ldr, rows_valid, lane);
+        tmem_ld_wait();
         float v[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
-        if (EPI == kEpiResidual && row_ok) {
-          float rr[32];
-          const bool rv = (p.ldr % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.R) & 15) == 0);
-          load_row_bf16(p.R + b * p.r_batch_stride + static_cast<long long>(row) * p.ldr + col,
-                        rr, n_valid, rv);
+        if (EPI == kEpiResidual) {
+          if (r_vec_ok) {
+            staged_add_row(stage, v, lane);
+          } else if (row_ok) {
+            float rr[32];
+            load_row_bf16(p.R + b * p.r_batch_stride + static_cast<long long>(row) * p.ldr + col,
+                          rr, n_valid, false);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] += rr[i];
+            for (int i = 0; i < 32; ++i) v[i] += rr[i];
+          }
         }
         const long long first = b * p.c_batch_stride +
                                 static_cast<long long>(m0 + q * 32) * p.ldc + col;
@@ -344,7 +407,8 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
                             rows_valid, lane);
         continue;
       }
-      if (row_ok && n_valid > 0) {
+      tmem_ld_wait();
+      if (row_ok) {
         float v[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
@@ -378,7 +442,9 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
               reinterpret_cast<float4*>(out)[i] = o;
             }
           } else {
-            for (int i = 0; i < 32 && i < n_valid; ++i) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              if (i >= n_valid) break;
               if (p.accumulate == 2)
                 atomicAdd(out + i, v[i]);
               else
@@ -401,85 +467,129 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
   }
 }
 
-// Cross-entropy forward epilogue of one accumulator tile: the calling thread owns one row of
-// logits x = alpha * acc and folds the tile's BN columns into (max, sum exp(x - max), sum x,
-// largest x and its column), which a small kernel merges over the column tiles afterwards.
-// The logits themselves are never stored.
+// Cross-entropy forward epilogue of kCeTileCols columns (part `part` of the tile) of an
+// accumulator tile: the calling thread owns one row of logits x = alpha * acc and folds them into
+// (max, sum exp(x - max), sum x, largest x and its column), which a small kernel merges over the
+// partials of a row afterwards. The logits themselves are never stored.
+//
+// Bound by the instructions per logit: whole 32-column chunks run without bounds checks, the
+// column of the maximum comes from one compare-and-select per logit, and the target is looked for
+// only in the chunk that holds it.
 template <int BN>
 __device__ __forceinline__ void gemm_epilogue_ce_stats(const GemmParams& p, uint32_t t_row, int m0,
-                                                       int n0, int nt, int q, int lane) {
+                                                       int n0, int q, int part, int lane) {
   const int row = m0 + q * 32 + lane;
   const bool row_ok = row < p.M;
   const long long tgt = row_ok ? p.ce_targets[row] - p.ce_vocab_start : -1;
-  float mx = -3.0e38f, se = 0.f, sx = 0.f, best = -3.0e38f;
+  float mx = -3.0e38f, se = 0.f, sx = 0.f;
   int best_col = 0;
+  const int first = n0 + part * kCeTileCols;
+  if (first >= p.N) return;  // warp-uniform: no such partial
 #pragma unroll 1
-  for (int c = 0; c < BN / 32; ++c) {
-    uint32_t r[32];
-    tmem_ld32(t_row + c * 32, r);
-    tmem_ld_wait();
-    const int col = n0 + c * 32;
+  for (int c = 0; c < kCeTileCols / 32; ++c) {
+    const int col = first + c * 32;
     const int n_valid = p.N - col;
-    if (!row_ok || n_valid <= 0) continue;
+    if (n_valid <= 0) break;  // warp-uniform
+    uint32_t r[32];
+    tmem_ld32(t_row + part * kCeTileCols + c * 32, r);
+    tmem_ld_wait();
     float v[32];
-    float cm = -3.0e38f;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      v[i] = __uint_as_float(r[i]) * p.alpha;
-      if (i < n_valid) {
-        cm = fmaxf(cm, v[i]);
-        sx += v[i];
-        if (v[i] > best) {
-          best = v[i];
-          best_col = col + i;
-        }
-        if (col + i == tgt) p.ce_target_logit[row] = v[i];
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
+    float s0 = 0.f, s1 = 0.f;
+    if (n_valid >= 32) {
+#pragma unroll
+      for (int i = 0; i < 32; i += 2) {
+        s0 += v[i];
+        s1 += v[i + 1];
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        if (i < n_valid) s0 += v[i];
+        else v[i] = -3.0e38f;  // never the maximum, exp gives zero
       }
     }
-    const float nm = fmaxf(mx, cm);
-    float add = 0.f;
+    sx += s0 + s1;
+    float cm = v[0], cm1 = v[1];
 #pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (i < n_valid) add += __expf(v[i] - nm);
-    se = se * __expf(mx - nm) + add;
+    for (int i = 2; i < 32; i += 2) {
+      cm = fmaxf(cm, v[i]);
+      cm1 = fmaxf(cm1, v[i + 1]);
+    }
+    cm = fmaxf(cm, cm1);
+    int ci = 0;
+#pragma unroll
+    for (int i = 31; i >= 0; --i) ci = v[i] == cm ? i : ci;
+    if (cm > mx) best_col = col + ci;
+    const long long off = tgt - col;
+    if (off >= 0 && off < 32 && off < n_valid) {
+      float t = v[0];
+#pragma unroll
+      for (int i = 1; i < 32; ++i) t = off == i ? v[i] : t;
+      p.ce_target_logit[row] = t;
+    }
+    const float nm = fmaxf(mx, cm);
+    float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+      a0 += __expf(v[i] - nm);
+      a1 += __expf(v[i + 1] - nm);
+    }
+    se = se * __expf(mx - nm) + (a0 + a1);
     mx = nm;
   }
   if (row_ok) {
-    float4* out = reinterpret_cast<float4*>(p.ce_part) + static_cast<long long>(row) * p.tiles_n + nt;
-    *out = make_float4(mx, se, sx, best);
-    p.ce_arg[static_cast<long long>(row) * p.tiles_n + nt] = best_col + p.ce_vocab_start;
+    const long long at = static_cast<long long>(row) * p.ce_tiles + first / kCeTileCols;
+    reinterpret_cast<float4*>(p.ce_part)[at] = make_float4(mx, se, sx, mx);
+    p.ce_arg[at] = best_col + p.ce_vocab_start;
   }
 }
 
 // Cross-entropy backward epilogue: the logits tile is recomputed by the GEMM and turned into
 //   dlogits = row_scale * ((1 + 2 z lse) * exp(x - lse) - soft_target)        (bf16)
-// which the two gradient GEMMs of the projection read next. C is the bf16 [M, N] output.
-template <int BN>
+// which the two gradient GEMMs of the projection read next. C is the bf16 [M, N] output; whole
+// chunks leave through the warp's staging block as 64-byte row segments.
+template <int BN, int PARTS>
 __device__ __forceinline__ void gemm_epilogue_ce_grad(const GemmParams& p, uint32_t t_row, int m0,
-                                                      int n0, int q, int lane, bool c_vec_ok) {
+                                                      int n0, int q, int part, int lane,
+                                                      bool c_vec_ok, float* stage) {
   const int row = m0 + q * 32 + lane;
   const bool row_ok = row < p.M;
+  const int rows_valid = p.M - (m0 + q * 32);
   const float lse = row_ok ? p.ce_lse[row] : 0.f;
   const float g = row_ok ? p.ce_row_scale[row] : 0.f;
   const float zf = 1.f + 2.f * p.ce_z * lse;
   const long long tgt = row_ok ? p.ce_targets[row] - p.ce_vocab_start : -1;
-  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(row) * p.ldc;
+  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C);
 #pragma unroll 1
-  for (int c = 0; c < BN / 32; ++c) {
+  for (int c = part * (BN / 32 / PARTS); c < (part + 1) * (BN / 32 / PARTS); ++c) {
+    const int col = n0 + c * 32;
+    const int n_valid = p.N - col;
+    if (n_valid <= 0) break;  // warp-uniform
     uint32_t r[32];
     tmem_ld32(t_row + c * 32, r);
     tmem_ld_wait();
-    const int col = n0 + c * 32;
-    const int n_valid = p.N - col;
-    if (!row_ok || n_valid <= 0) continue;
     float v[32];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float x = __uint_as_float(r[i]) * p.alpha;
-      const float soft = (col + i == tgt) ? p.ce_conf : p.ce_low;
-      v[i] = g == 0.f ? 0.f : g * (zf * __expf(x - lse) - soft);
+    for (int i = 0; i < 32; ++i)
+      v[i] = g * (zf * __expf(__uint_as_float(r[i]) * p.alpha - lse) - p.ce_low);
+    const long long off = tgt - col;
+    if (off >= 0 && off < 32) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (off == i)
+          v[i] = g * (zf * __expf(__uint_as_float(r[i]) * p.alpha - lse) - p.ce_conf);
     }
-    store_row_bf16(out + col, v, n_valid, c_vec_ok);
+    if (g == 0.f) {  // a token without weight: exactly zero, whatever its logits are
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = 0.f;
+    }
+    if (n_valid >= 32 && c_vec_ok && rows_valid > 0)
+      staged_store_bf16(stage, v, out + static_cast<long long>(m0 + q * 32) * p.ldc + col, p.ldc,
+                        rows_valid, lane);
+    else if (row_ok)
+      store_row_bf16(out + static_cast<long long>(row) * p.ldc + col, v, n_valid, c_vec_ok);
   }
 }
 

@@ -7,12 +7,13 @@
 // columns of B (the tensor cores of both SMs read both B halves), a third less shared-memory
 // traffic per FLOP.
 //
-// Roles per CTA (192 threads): warp 0 = TMA producer (both CTAs, own halves), warp 1 = MMA
-// issuer (even CTA only; owns the TMEM allocation in both), warps 2..5 = epilogue of the
-// CTA's own 128 accumulator rows. Barriers: `full` lives in the even CTA and counts the bytes
+// Roles per CTA (320 threads): warp 0 = TMA producer (both CTAs, own halves), warp 1 = MMA
+// issuer (even CTA only; owns the TMEM allocation in both), warps 2..9 = epilogue of the
+// CTA's own 128 accumulator rows, two warps per TMEM lane quarter (tensor-parallel kernels:
+// warps 2..5, one per quarter). Barriers: `full` lives in the even CTA and counts the bytes
 // of both CTAs' loads; `empty` and `tmem_full` exist in both CTAs and are signalled by one
 // tcgen05.commit addressed to both; `tmem_empty` lives in the even CTA and collects the
-// arrivals of all eight epilogue warps. Every wait is bounded and TMA loads never use
+// arrivals of the epilogue warps of both CTAs. Every wait is bounded and TMA loads never use
 // cluster multicast.
 #include <algorithm>
 
@@ -51,14 +52,19 @@ constexpr int kTpStageBytes = kTpPiece * kTpSlots;
 constexpr int kTpFlagLimit = 1 << 24;  // polls (>= 64 ns apart) before a flag wait gives up: 1-3 s
 
 template <int MODE>
-constexpr int pair_threads() { return MODE == kTpAllGather ? kGemmThreads + 32 : kGemmThreads; }
+constexpr int pair_epi_warps() { return MODE == kTpNone ? kEpiWarps : kTpEpiWarps; }
+template <int MODE>
+constexpr int pair_threads() {
+  return 64 + 32 * pair_epi_warps<MODE>() + (MODE == kTpAllGather ? 32 : 0);
+}
 template <int MODE>
 constexpr int pair_smem() {
   return MODE == kTpAllGather       ? kPairSmemTotal + kTpStageBytes
          : MODE == kTpReduceScatter ? kPairSmemTotal + 4 * kRsStageBytesPerWarp
-                                    : kPairSmemTotal + 4 * kEpiStageBytesPerWarp;
+                                    : kPairSmemTotal + kEpiWarps * kEpiStageBytesPerWarp;
 }
 static_assert(kPairSmemTotal + 4 * kRsStageBytesPerWarp <= 232448, "shared memory per CTA");
+static_assert(kPairSmemTotal + kEpiWarps * kEpiStageBytesPerWarp <= 232448, "shared memory per CTA");
 
 template <int EPI, int MODE = kTpNone>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>(), 1)
@@ -98,7 +104,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full[a], 1);
-      mbar_init(&tmem_empty[a], 8);
+      mbar_init(&tmem_empty[a], 2 * pair_epi_warps<MODE>());
     }
     if (MODE == kTpAllGather)
       for (int a = 0; a < kTpSlots; ++a) mbar_init(&copy_full[a], 1);
@@ -385,6 +391,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
   } else {
     // ------------------------------ epilogue (own 128 rows) ------------------------------
     const int q = warp & 3;
+    const int part = (warp - 2) >> 2;  // which half of the tile's columns (MODE none)
     int local = 0;
     bool ok = true;
     chain_wait();  // the epilogue reads residuals and writes C
@@ -409,12 +416,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
         gemm_epilogue_tile_rs<BN, EPI>(p, tp, t_row, m0, n0, q, lane,
                                        staging + (warp - 2) * kRsStageBytesPerWarp);
       else if (EPI == kEpiCeStats)
-        gemm_epilogue_ce_stats<BN>(p, t_row, m0, n0, nt, q, lane);
+        gemm_epilogue_ce_stats<BN>(p, t_row, m0, n0, q, part, lane);
       else if (EPI == kEpiCeGrad)
-        gemm_epilogue_ce_grad<BN>(p, t_row, m0, n0, q, lane, c_vec_ok);
+        gemm_epilogue_ce_grad<BN, 2>(
+            p, t_row, m0, n0, q, part, lane, c_vec_ok,
+            reinterpret_cast<float*>(staging + (warp - 2) * kEpiStageBytesPerWarp));
       else
-        gemm_epilogue_tile<BN, EPI>(
-            p, t_row, m0, n0, b, q, lane, c_vec_ok,
+        gemm_epilogue_tile<BN, EPI, pair_epi_warps<MODE>() / 4>(
+            p, t_row, m0, n0, b, q, part, lane, c_vec_ok,
             MODE == kTpNone
                 ? reinterpret_cast<float*>(staging + (warp - 2) * kEpiStageBytesPerWarp)
                 : nullptr);

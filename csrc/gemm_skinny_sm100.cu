@@ -31,6 +31,7 @@ namespace t5x {
 
 constexpr int kSkBN = 128;
 constexpr int kSkStages = 4;
+constexpr int kSkThreads = 192;
 constexpr int kSkABytes = kBM * kBK * 2;
 constexpr int kSkBBytes = kSkBN * kBK * 2;
 constexpr int kSkStageBytes = kSkABytes + kSkBBytes;
@@ -73,7 +74,7 @@ __device__ __forceinline__ void epilogue_bar_sync() {  // the four epilogue warp
   asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(kSkThreads, 1)
     gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA,
                        const __grid_constant__ CUtensorMap tmB, const SkinnyParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -348,9 +349,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     float* stage = staging + (warp - 2) * (kEpiStageBytesPerWarp / 4);
     const bool c_vec16 = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
     if (p.R != nullptr)
-      gemm_epilogue_tile<kSkBN, kEpiResidual>(gp, t_row, m0, n0, 0, q, lane, c_vec16, stage);
+      gemm_epilogue_tile<kSkBN, kEpiResidual, 1>(gp, t_row, m0, n0, 0, q, 0, lane, c_vec16, stage);
     else
-      gemm_epilogue_tile<kSkBN, kEpiPlain>(gp, t_row, m0, n0, 0, q, lane, c_vec16, stage);
+      gemm_epilogue_tile<kSkBN, kEpiPlain, 1>(gp, t_row, m0, n0, 0, q, 0, lane, c_vec16, stage);
   }
 
   // Teardown: loads still in flight after an abort get a bounded time to land.
@@ -451,7 +452,7 @@ T5X_API int t5x_gemm_skinny_bf16(const void* A, const void* B, void* C, const vo
   const int tiles = ((M + kBM - 1) / kBM) * p.tiles_n;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles * splits);
-  cfg.blockDim = dim3(kGemmThreads);
+  cfg.blockDim = dim3(kSkThreads);
   cfg.dynamicSmemBytes = kSkSmemTotal;
   cfg.stream = static_cast<cudaStream_t>(stream);
   cudaLaunchAttribute attr[2];

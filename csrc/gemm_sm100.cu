@@ -7,8 +7,8 @@
 // MN-major (row-major [K,N]). That covers forward (x * W[in,out]), dgrad (dy * W^T)
 // and wgrad (x^T * dy) of a dense layer without a transpose pass.
 //
-// Roles per CTA (192 threads): warp 0 = TMA producer, warp 1 = tcgen05 MMA issuer
-// (owns TMEM alloc/free), warps 2..5 = epilogue (one TMEM lane quarter each).
+// Roles per CTA (320 threads): warp 0 = TMA producer, warp 1 = tcgen05 MMA issuer
+// (owns TMEM alloc/free), warps 2..9 = epilogue (two per TMEM lane quarter, half the columns each).
 // smem ring of kStages {A 128x64, B BNx64} tiles in the 128-byte swizzle that both
 // TMA and the UMMA descriptors use; two accumulators in TMEM so the epilogue of tile
 // i overlaps the main loop of tile i+1. No cluster multicast is used anywhere.
@@ -32,7 +32,7 @@ struct GemmSmem {
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kStages = (BN == 256) ? 4 : 6;
   static constexpr int kBarrierBytes = 1024;
-  static constexpr int kEpiStageBytes = 4 * kEpiStageBytesPerWarp;  // coalesced epilogue stores
+  static constexpr int kEpiStageBytes = kEpiWarps * kEpiStageBytesPerWarp;  // coalesced epilogue stores
   static constexpr int kTotal =
       kStages * kStageBytes + kBarrierBytes + kEpiStageBytes + 1024;  // +1024 align slack
 };
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full[a], 1);
-      mbar_init(&tmem_empty[a], 4);
+      mbar_init(&tmem_empty[a], kEpiWarps);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -234,6 +234,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
   } else {
     // ------------------------------ epilogue ------------------------------
+    const int part = (warp - 2) >> 2;  // which half of the tile's columns
     const int q = warp & 3;  // TMEM lanes [32q, 32q+32) belong to warps with id % 4 == q
     int local = 0;
     bool ok = true;
@@ -255,13 +256,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       tc_fence_after();
       if (local == 0 && warp == 2 && lane == 0) T5X_GEMM_TRACE(5);
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
+      float* stage_buf = epi_stage + (warp - 2) * (kEpiStageBytesPerWarp / 4);
       if (EPI == kEpiCeStats)
-        gemm_epilogue_ce_stats<BN>(p, t_row, m0, n0, nt, q, lane);
+        gemm_epilogue_ce_stats<BN>(p, t_row, m0, n0, q, part, lane);
       else if (EPI == kEpiCeGrad)
-        gemm_epilogue_ce_grad<BN>(p, t_row, m0, n0, q, lane, c_vec_ok);
+        gemm_epilogue_ce_grad<BN, 2>(p, t_row, m0, n0, q, part, lane, c_vec_ok, stage_buf);
       else
-        gemm_epilogue_tile<BN, EPI>(p, t_row, m0, n0, b, q, lane, c_vec_ok,
-                                    epi_stage + (warp - 2) * (kEpiStageBytesPerWarp / 4));
+        gemm_epilogue_tile<BN, EPI, 2>(p, t_row, m0, n0, b, q, part, lane, c_vec_ok, stage_buf);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[acc]);
@@ -425,6 +426,7 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
   p.ce_target_logit = nullptr;
   p.ce_lse = p.ce_row_scale = nullptr;
   p.ce_vocab_start = 0;
+  p.ce_tiles = 0;
   p.ce_z = p.ce_conf = p.ce_low = 0.f;
 
   const CUtensorMap* tA = operand_map(A, a_mn_major, M, K, lda, a_batch_stride, batch, 128);
@@ -466,6 +468,7 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
     p.ce_targets = ce->targets;
     p.ce_vocab_start = ce->vocab_start;
     p.ce_part = ce->part;
+    p.ce_tiles = (N + kCeTileCols - 1) / kCeTileCols;
     p.ce_arg = ce->arg;
     p.ce_target_logit = ce->target_logit;
     p.ce_lse = ce->lse;
@@ -630,8 +633,8 @@ T5X_API int t5x_gemm_reducescatter_bf16(const void* A, const void* B, void* cons
 }
 
 // ---- logits projection fused with the cross-entropy: the [M, N] logits are never stored ----
-// Number of column tiles (partials per row) the forward produces for a vocabulary slice of N.
-T5X_API int t5x_gemm_ce_tiles(int N) { return (N + 255) / 256; }
+// Number of partials per row the forward produces for a vocabulary slice of N.
+T5X_API int t5x_gemm_ce_tiles(int N) { return (N + t5x::kCeTileCols - 1) / t5x::kCeTileCols; }
 
 // Forward: logits = alpha * A[M, K] @ B[K, N] are folded, tile by tile in the GEMM epilogue,
 // into part[M, tiles, 4] (max, sum exp(x - max), sum x, largest x), arg[M, tiles] (vocabulary

@@ -1,0 +1,74 @@
+"""Epilogues of the bf16 GEMMs at the edges of their tiles: column ranges that end inside a warp's
+half of a tile or before it, rows that end inside a warp, residuals on and off the 16-byte path,
+and the cross-entropy epilogues, which fold 128 columns into one partial. Bounds: the operands are
+exact in both forms, the fp32 sums of K products differ by their order (K * 2^-24 of the sum of
+magnitudes, far below the bf16 rounding of the output, 2^-9 relative)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1, 8, 64), (40, 96, 64), (129, 136, 72), (256, 264, 128), (300, 392, 64), (513, 640, 192)]
+
+
+def _operands(M, N, K, seed):
+  g = torch.Generator(device="cuda").manual_seed(seed)
+  a = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+  b = (torch.randn(K, N, device="cuda", generator=g) * K ** -0.5).bfloat16()
+  return a, b, g
+
+
+@pytest.mark.parametrize("pair", [0, 2])
+@pytest.mark.parametrize("M,N,K", SHAPES)
+def test_residual_and_accumulate(M, N, K, pair):
+  from t5x_b200.ops import native
+  a, b, g = _operands(M, N, K, M + N)
+  want = a.double() @ b.double()
+  wide = torch.randn(M, N + 4, device="cuda", generator=g).bfloat16()
+  native.gemm_set_pair_mode(pair)
+  try:
+    for res in (wide[:, :N].contiguous(), wide[:, :N], wide[:, 1:N + 1]):
+      y = native.gemm(a, b, residual=res)
+      torch.testing.assert_close(y.double(), want + res.double(), rtol=2 ** -8, atol=2 ** -8)
+    acc = torch.randn(M, N, device="cuda", generator=g)
+    out = acc.clone()
+    native.gemm(a, b, out=out, accumulate=True)
+    torch.testing.assert_close(out.double(), want + acc.double(), rtol=1e-5, atol=1e-5)
+  finally:
+    native.gemm_set_pair_mode(1)
+  native.check_status()
+
+
+@pytest.mark.parametrize("pair", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(1, 64, 64), (37, 129, 64), (256, 128, 64), (300, 1000, 128),
+                                   (515, 2184, 64)])
+def test_cross_entropy(M, N, K, pair):
+  from t5x_b200.ops import native
+  ldb = -(-N // 8) * 8
+  a, b, g = _operands(M, ldb, K, 3 * M + N)
+  b = b[:, :N]
+  t = torch.randint(0, N, (M,), device="cuda", generator=g)
+  t[0], t[-1] = 0, N - 1
+  x = (a.double() @ b.double()) * 0.5
+  native.gemm_set_pair_mode(pair)
+  try:
+    stats, _, arg = native.gemm_ce_stats(a, b, t, alpha=0.5)
+    lse = stats[:, 0] + torch.log(stats[:, 1])
+    want_lse = torch.logsumexp(x, -1)
+    torch.testing.assert_close(lse.double(), want_lse, rtol=1e-5, atol=1e-5)
+    torch.testing.assert_close(stats[:, 2].double(), x.gather(1, t[:, None])[:, 0], rtol=1e-5,
+                               atol=1e-5)
+    torch.testing.assert_close(stats[:, 3].double(), x.sum(-1), rtol=1e-4, atol=1e-3)
+    top = x.gather(1, arg.long()[:, None])[:, 0]
+    assert bool((top >= x.max(-1).values - 1e-5).all())
+    scale = torch.rand(M, device="cuda", generator=g)
+    scale[M // 2] = 0.0
+    d = native.gemm_ce_grad(a, b, t, want_lse.float(), scale, 1e-3, 0.9, 0.1 / (N - 1), alpha=0.5)
+    soft = torch.full_like(x, 0.1 / (N - 1)).scatter_(1, t[:, None], 0.9)
+    want = scale.double()[:, None] * ((1 + 2e-3 * want_lse)[:, None] *
+                                      torch.exp(x - want_lse[:, None]) - soft)
+    torch.testing.assert_close(d.double(), want, rtol=2 ** -8, atol=1e-5)
+    assert not bool(d[M // 2].any())
+  finally:
+    native.gemm_set_pair_mode(1)
+  native.check_status()
