@@ -433,24 +433,90 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// dtable[id] += dout rows of the tokens with that id, in fp32.
+//
+// A CTA takes CHUNK consecutive tokens and a range of columns (four per thread). It ranks the
+// chunk's tokens by id, walks them in that order, keeps the running sum of equal ids in
+// registers and adds one row per DISTINCT id to the table with 16-byte atomics. Natural text
+// is Zipf-distributed and every padding position is id 0: with one atomic add per token, the
+// adds to the few hot rows queued up in L2 and set the time (65536 x 768: 0.69 ms for the
+// 134 MB it moves); a chunk of 128 leaves at most 1/128 of them. Short inputs take chunks of 16 so
+// that more CTAs share the walk and every row of a chunk is in flight at once.
+template <int CHUNK>
 __global__ void __launch_bounds__(256)
     embedding_bwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dout,
                          float* __restrict__ dtable, long long tokens, int d, int vocab_start,
-                         int vocab_rows) {
-  const int nvec = d / 8;
-  const long long total = tokens * nvec;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long t = i / nvec;
-    const int v = static_cast<int>(i - t * nvec);
-    const long long id = ids[t] - vocab_start;
-    if (id < 0 || id >= vocab_rows) continue;
-    float f[8];
-    unpack8(reinterpret_cast<const Bf16x8*>(dout + t * d)[v], f);
-    float* dst = dtable + id * d + v * 8;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) atomicAdd(dst + j, f[j]);
+                         int vocab_rows, int vec_ok) {
+  __shared__ int s_id[CHUNK];      // row of the table, -1 when it is not in this slice
+  __shared__ int s_order[CHUNK];   // token of the chunk at each place of the sorted order
+  const long long t0 = static_cast<long long>(blockIdx.x) * CHUNK;
+  const int n = static_cast<int>(min(static_cast<long long>(CHUNK), tokens - t0));
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const long long id = ids[t0 + i] - vocab_start;
+    s_id[i] = (id >= 0 && id < vocab_rows) ? static_cast<int>(id) : -1;
   }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int mine = s_id[i];
+    int rank = 0;
+    for (int j = 0; j < n; ++j) {
+      const int other = s_id[j];
+      rank += (other < mine || (other == mine && j < i)) ? 1 : 0;
+    }
+    s_order[rank] = i;
+  }
+  __syncthreads();
+  const int col = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  if (col >= d) return;
+  const __nv_bfloat16* src = dout + t0 * d + col;
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+  int current = -1;
+  auto flush = [&]() {
+    if (current < 0) return;
+    float* dst = dtable + static_cast<long long>(current) * d + col;
+    if (vec_ok) {
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(sum.x),
+                   "f"(sum.y), "f"(sum.z), "f"(sum.w)
+                   : "memory");
+    } else {
+      atomicAdd(dst, sum.x);
+      atomicAdd(dst + 1, sum.y);
+      atomicAdd(dst + 2, sum.z);
+      atomicAdd(dst + 3, sum.w);
+    }
+  };
+  constexpr int kAhead = 16;  // rows in flight per thread
+  for (int s = 0; s < n; s += kAhead) {
+    uint2 u[kAhead];
+    int id[kAhead];
+#pragma unroll
+    for (int x = 0; x < kAhead; ++x) {
+      id[x] = -1;
+      u[x] = make_uint2(0u, 0u);
+      if (s + x < n) {
+        const int t = s_order[s + x];
+        id[x] = s_id[t];
+        if (id[x] >= 0)
+          u[x] = *reinterpret_cast<const uint2*>(src + static_cast<long long>(t) * d);
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < kAhead; ++x) {
+      if (id[x] < 0) continue;
+      if (id[x] != current) {
+        flush();
+        current = id[x];
+        sum = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[x].x));
+      const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[x].y));
+      sum.x += lo.x;
+      sum.y += lo.y;
+      sum.z += hi.x;
+      sum.w += hi.y;
+    }
+  }
+  flush();
 }
 
 // fp32 -> bf16 cast with independent leading dimensions (to fill slices of fused weights).
@@ -599,10 +665,16 @@ T5X_API int t5x_embedding_bwd(const void* ids, const void* dout, void* dtable, l
                               int d, int vocab_start, int vocab_rows, void* stream) {
   if (tokens <= 0) return 0;
   if (d % 8) return set_error("embedding: d must be a multiple of 8");
-  embedding_bwd_kernel<<<ew_grid(tokens * (d / 8), 256), 256, 0,
-                         static_cast<cudaStream_t>(stream)>>>(
+  // four columns per thread; whole warps, at most 256 threads
+  const int threads = d / 4 >= 256 ? 256 : (d / 4 + 31) / 32 * 32;
+  const int chunk = tokens >= 8192 ? 128 : 16;
+  const dim3 grid(static_cast<unsigned>((tokens + chunk - 1) / chunk),
+                  static_cast<unsigned>((d / 4 + threads - 1) / threads));
+  const int vec_ok = (reinterpret_cast<uintptr_t>(dtable) & 15) == 0;
+  auto kernel = chunk == 128 ? embedding_bwd_kernel<128> : embedding_bwd_kernel<16>;
+  kernel<<<grid, threads, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const long long*>(ids), static_cast<const __nv_bfloat16*>(dout),
-      static_cast<float*>(dtable), tokens, d, vocab_start, vocab_rows);
+      static_cast<float*>(dtable), tokens, d, vocab_start, vocab_rows, vec_ok);
   CHECK_LAUNCH("embedding_bwd");
   return 0;
 }
