@@ -17,8 +17,9 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 struct AttnParams {
   int B, H, Lq, Lk;
-  const float* rel_bias;  // [H, nrel] or null
-  int nrel, rel_off;
+  const float* rel_bias;     // [H, num_buckets] or null: the T5 bucket table
+  const int* rel_bucket;     // [nrel]: bucket of the relative position (k - q) = t - rel_off
+  int nrel, rel_off, num_buckets;
   const uint8_t* key_mask;  // [B, Lk] (1 = attend) or null
   const int* q_seg;         // [B, Lq] or null
   const int* kv_seg;        // [B, Lk] or null
@@ -32,9 +33,14 @@ struct AttnParams {
   __nv_bfloat16* dK;        // [B, Lk, H, D]
   __nv_bfloat16* dV;
   long long dk_sb, dk_sl, dk_sh;
-  float* d_rel_bias;        // [H, nrel] or null
+  float* d_rel_bias;        // [H, num_buckets] (added to) or null
   int* status;
 };
+
+// The bias of head h at relative index t = (k - q) + rel_off (0 outside the table).
+__device__ __forceinline__ float rel_bias_at(const AttnParams& p, const float* head_table, int t) {
+  return (t >= 0 && t < p.nrel) ? __ldg(head_table + __ldg(p.rel_bucket + t)) : 0.f;
+}
 
 __device__ __forceinline__ void softmax_bar_sync() {
   asm volatile("bar.sync 1, %0;" ::"n"(kSoftmaxThreads) : "memory");

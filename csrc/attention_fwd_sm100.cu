@@ -231,21 +231,21 @@ __global__ void __launch_bounds__(kFsThreads, 1)
     float* rel_stage = sRel + t * 2 * 4 * kFsRelCopy;
     int* key_stage = sKey + t * 2 * 132;
     uint8_t* p_tile = sP + t * 2 * kFsPanel;
-    const float* tab = has_bias ? p.rel_bias + static_cast<long long>(h) * p.nrel : nullptr;
+    const float* tab = has_bias ? p.rel_bias + static_cast<long long>(h) * p.num_buckets : nullptr;
     const int shift = (127 - r) & 3;
     bool ok = true;
 
     // Per-block metadata is fetched one block ahead into registers and published to the other
     // shared-memory stage after the arithmetic of the current block.
-    float pf_rel0 = 0.f, pf_rel1 = 0.f;
+    int pf_rel0 = -1, pf_rel1 = -1;
     int pf_seg = -1;
     auto fetch_meta = [&](int j) {
       if (has_bias) {
         const int base = j * 128 - q0 - 127 + p.rel_off;  // index of window entry 0
         const int i0 = base + g, i1 = base + g + 128;
-        // raw values only: anything computed from them here would wait for the loads at once
-        pf_rel0 = (i0 >= 0 && i0 < p.nrel) ? __ldg(tab + i0) : 0.f;
-        pf_rel1 = (g < 127 && i1 >= 0 && i1 < p.nrel) ? __ldg(tab + i1) : 0.f;
+        // only the buckets: anything computed from them here would wait for the loads at once
+        pf_rel0 = (i0 >= 0 && i0 < p.nrel) ? __ldg(p.rel_bucket + i0) : -1;
+        pf_rel1 = (g < 127 && i1 >= 0 && i1 < p.nrel) ? __ldg(p.rel_bucket + i1) : -1;
       }
       const int k = j * 128 + g;
       pf_seg = -1;
@@ -259,7 +259,8 @@ __global__ void __launch_bounds__(kFsThreads, 1)
       float* rs = rel_stage + (j & 1) * 4 * kFsRelCopy;
       int* ks = key_stage + (j & 1) * 132;
       if (has_bias) {
-        const float r0 = pf_rel0 * kLog2e, r1 = pf_rel1 * kLog2e;
+        const float r0 = pf_rel0 >= 0 ? __ldg(tab + pf_rel0) * kLog2e : 0.f;
+        const float r1 = pf_rel1 >= 0 ? __ldg(tab + pf_rel1) * kLog2e : 0.f;
 #pragma unroll
         for (int m = 0; m < 4; ++m) {  // copy m holds window[i + m] at i
           if (g - m >= 0) rs[m * kFsRelCopy + g - m] = r0;
@@ -487,7 +488,8 @@ T5X_API int t5x_attention_fwd_stream(const void* q, const void* k, const void* v
                                      long long k_sb, long long k_sl, long long k_sh,
                                      long long v_sb, long long v_sl, long long v_sh,
                                      long long o_sb, long long o_sl, long long o_sh,
-                                     const void* rel_bias, int nrel, int rel_off,
+                                     const void* rel_bias, const void* rel_bucket,
+                                     int num_buckets, int nrel, int rel_off,
                                      const void* key_mask, const void* q_seg, const void* kv_seg,
                                      int causal, int causal_off, void* stream) {
   if (B <= 0 || H <= 0 || Lq <= 0 || Lk <= 0) return 0;
@@ -502,6 +504,8 @@ T5X_API int t5x_attention_fwd_stream(const void* q, const void* k, const void* v
   AttnParams p = {};
   p.B = B; p.H = H; p.Lq = Lq; p.Lk = Lk;
   p.rel_bias = static_cast<const float*>(rel_bias);
+  p.rel_bucket = static_cast<const int*>(rel_bucket);
+  p.num_buckets = num_buckets;
   p.nrel = nrel; p.rel_off = rel_off;
   p.key_mask = static_cast<const uint8_t*>(key_mask);
   p.q_seg = static_cast<const int*>(q_seg);

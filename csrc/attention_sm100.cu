@@ -6,8 +6,8 @@
 // probability / dS tiles are written by the softmax warps straight into the swizzled shared
 // layout that the next MMA reads as its A operand. The [b,h,q,k] score matrix never exists in
 // global memory. Bias and masks are generated in-kernel from per-token metadata:
-//   bias      : rel_bias[h][(k - q) + rel_off]  (the T5 bucket table expanded by relative
-//               offset on the host, so the bucket arithmetic is bit-identical to the oracle)
+//   bias      : rel_bias[h][rel_bucket[(k - q) + rel_off]]  (the T5 bucket table; the bucket of
+//               each relative position comes from the host, bit-identical to the oracle)
 //   masks     : key padding [B,Lk], causal (k <= q + causal_off), packed-segment ids.
 // Masked logits take the value -1e10 (not -inf): a fully masked row gives a uniform
 // distribution, exactly like the additive-mask formulation of the reference.
@@ -35,7 +35,8 @@ struct FwdSmem {
   static constexpr int kRel = kP + 4 * kTile;   // bias by (k - q): up to 512 + 512 floats
   static constexpr int kStat = kRel + 1024 * 4; // 128 x 4 floats (row max parts), then sums
   static constexpr int kKeySeg = kStat + 128 * 4 * 4 * 2;  // 512 ints: segment id of key k, -1 = hidden
-  static constexpr int kBars = kKeySeg + 512 * 4;
+  static constexpr int kKeyWord = kKeySeg + 512 * 4;  // 16 words: bit x of word w, key 32 w + x is visible
+  static constexpr int kBars = kKeyWord + 16 * 4;
   static constexpr int kTotal = kBars + 256 + 1024;
 };
 constexpr int kFwdMaxLq = 512;  // sRel covers (k - q) for Lq, Lk <= 512
@@ -53,6 +54,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   float* sRel = reinterpret_cast<float*>(smem + FwdSmem::kRel);
   float* sStat = reinterpret_cast<float*>(smem + FwdSmem::kStat);
   int* sKeySeg = reinterpret_cast<int*>(smem + FwdSmem::kKeySeg);
+  uint32_t* sKeyWord = reinterpret_cast<uint32_t*>(smem + FwdSmem::kKeyWord);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FwdSmem::kBars);
   uint64_t* bar_q = bars;           // Q tile landed (once per query block)
   uint64_t* bar_kv = bars + 1;      // 4: K_j and V_j landed (once per CTA)
@@ -87,24 +89,6 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   if (warp == kCtrlWarp) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
-  }
-  // Bias by relative offset for this head: sRel[u], u = (k - q) + lq_pad - 1.
-  if (p.rel_bias != nullptr) {
-    const float* tab = p.rel_bias + static_cast<long long>(h) * p.nrel;
-    for (int u = threadIdx.x; u < lq_pad + nblk * 128; u += kAttnThreads) {
-      const int idx = u - (lq_pad - 1) + p.rel_off;
-      sRel[u] = (idx >= 0 && idx < p.nrel) ? tab[idx] : 0.f;
-    }
-  }
-  // Per-key metadata: segment id (0 when unpacked), -1 for padded / out-of-range keys.
-  for (int k = threadIdx.x; k < 512; k += kAttnThreads) {
-    int sgm = -1;
-    if (k < p.Lk) {
-      const long long off = static_cast<long long>(b) * p.Lk + k;
-      sgm = p.kv_seg ? p.kv_seg[off] : 0;
-      if (p.key_mask && p.key_mask[off] == 0) sgm = -1;
-    }
-    sKeySeg[k] = sgm;
   }
   tc_fence_before();
   __syncthreads();
@@ -180,6 +164,26 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     }
   } else {
     // ------------------------------ softmax warps ------------------------------
+    // (the operand loads and the first score MMAs are under way while these tables are filled)
+    // Bias by relative offset for this head: sRel[u], u = (k - q) + lq_pad - 1.
+    if (p.rel_bias != nullptr) {
+      const float* tab = p.rel_bias + static_cast<long long>(h) * p.num_buckets;
+      for (int u = threadIdx.x; u < lq_pad + nblk * 128; u += kSoftmaxThreads)
+        sRel[u] = rel_bias_at(p, tab, u - (lq_pad - 1) + p.rel_off);
+    }
+    // Per-key metadata: segment id (0 when unpacked), -1 for padded / out-of-range keys.
+    for (int k = threadIdx.x; k < 512; k += kSoftmaxThreads) {
+      int sgm = -1;
+      if (k < p.Lk) {
+        const long long off = static_cast<long long>(b) * p.Lk + k;
+        sgm = p.kv_seg ? p.kv_seg[off] : 0;
+        if (p.key_mask && p.key_mask[off] == 0) sgm = -1;
+      }
+      sKeySeg[k] = sgm;
+      const uint32_t word = __ballot_sync(0xffffffffu, sgm >= 0);
+      if (lane == 0) sKeyWord[k >> 5] = word;
+    }
+    softmax_bar_sync();
     const int quarter = warp & 3, part = warp >> 2;  // 4 threads per row, 32 columns each
     const int r = quarter * 32 + lane;               // row of the tile == TMEM lane
     const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -189,16 +193,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     uint32_t kvis[4], inr[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      uint32_t m_vis = 0, m_in = 0;
-      if (j < nblk) {
-        for (int x = 0; x < 32; ++x) {
-          const int kk = j * 128 + part * 32 + x;
-          m_vis |= (sKeySeg[kk] >= 0 ? 1u : 0u) << x;
-          m_in |= (kk < p.Lk ? 1u : 0u) << x;
-        }
-      }
-      kvis[j] = m_vis;
-      inr[j] = m_in;
+      const int left = p.Lk - (j * 128 + part * 32);  // keys from this chunk's first to the end
+      kvis[j] = sKeyWord[j * 4 + part];
+      inr[j] = left >= 32 ? 0xffffffffu : (left <= 0 ? 0u : ((1u << left) - 1u));
     }
     for (int i = 0; i < nq && ok; ++i) {
       const uint32_t ph = i & 1;
@@ -411,6 +408,7 @@ __global__ void __launch_bounds__(256)
 // softmax warps work, dQ partial tiles alternate between two TMEM buffers. head_dim 128: operand
 // tiles are twice as large and dK, dV take twice the TMEM columns, so Q / dO have one stage, dQ
 // reuses the columns of S^T and the query blocks run one after the other.
+constexpr int kSmemBuckets = 128;  // tables with more buckets add to memory directly
 template <int D>
 struct BwdSmem {
   static constexpr int kTile = 128 * 128;  // bytes of a [128 x 64] bf16 panel
@@ -425,7 +423,8 @@ struct BwdSmem {
   static constexpr int kVec = kDST + 2 * kTile;     // 2 stages x {lse[128], delta[128], qseg[128]}
   static constexpr int kRel = kVec + 2 * 3 * 128 * 4;   // bias by rel for the (i, j) pair: 2 x 256 floats
   static constexpr int kDRel = kRel + 2 * 256 * 4;      // d bias by rel accumulators: (Lq_pad + 128) floats
-  static constexpr int kBars = kDRel + (4096 + 128) * 4;
+  static constexpr int kBucket = kDRel + (4096 + 128) * 4;  // bias gradient by bucket
+  static constexpr int kBars = kBucket + kSmemBuckets * 4;
   static constexpr int kTotal = kBars + 256 + 1024;
 };
 
@@ -449,6 +448,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   float* sVec = reinterpret_cast<float*>(smem + Smem::kVec);
   float* sRelAll = reinterpret_cast<float*>(smem + Smem::kRel);
   float* sDRel = reinterpret_cast<float*>(smem + Smem::kDRel);
+  float* sBucket = reinterpret_cast<float*>(smem + Smem::kBucket);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Smem::kBars);
   uint64_t* bar_kv = bars;          // 1
   uint64_t* bar_qdo = bars + 1;     // 2 (full, per stage)
@@ -492,8 +492,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  if (p.d_rel_bias != nullptr)
+  if (p.d_rel_bias != nullptr) {
     for (int t = threadIdx.x; t < lq_pad + 128; t += kAttnThreads) sDRel[t] = 0.f;
+    if (threadIdx.x < kSmemBuckets) sBucket[threadIdx.x] = 0.f;
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -659,6 +661,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     // arithmetic of the current block, so their latency is off the critical path.
     float pf_a = 0.f, pf_b = 0.f;
     int pf_c = 0;
+    const float* head_table =
+        has_bias ? p.rel_bias + static_cast<long long>(h) * p.num_buckets : nullptr;
     auto fetch_vectors = [&](int i) {
       const int qb = i * 128;
       const int t = threadIdx.x;
@@ -670,10 +674,14 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         pf_c = (p.q_seg && q < p.Lq) ? p.q_seg[static_cast<long long>(b) * p.Lq + q] : 0;
       } else if (t < 128 + 255 && has_bias) {
         const int u = t - 128;
-        const float* tab = p.rel_bias + static_cast<long long>(h) * p.nrel;
         const int idx = (k0 - qb) + (u - 127) + p.rel_off;
-        pf_a = (idx >= 0 && idx < p.nrel) ? tab[idx] : 0.f;
+        pf_c = (idx >= 0 && idx < p.nrel) ? __ldg(p.rel_bucket + idx) : -1;
       }
+    };
+    // bucket -> bias, once the bucket has arrived and still ahead of its use
+    auto resolve_bias = [&]() {
+      if (has_bias && threadIdx.x >= 128 && threadIdx.x < 128 + 255)
+        pf_a = pf_c >= 0 ? __ldg(head_table + pf_c) : 0.f;
     };
     auto publish_vectors = [&](int i) {
       float* sLse = sVec + (i & 1) * 384;
@@ -717,6 +725,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     };
 
     fetch_vectors(0);
+    resolve_bias();
     publish_vectors(0);
     softmax_bar_sync();
     for (int i = 0; i < nq && ok; ++i) {
@@ -815,6 +824,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
             }
           }
         }
+        if (hc == 0 && i + 1 < nq) resolve_bias();
         if (D == 64 && hc == 0 && i > 0) {
           // the gradient MMAs of block i - 1 still read P^T / dS^T; they also produce dQ_{i-1}
           // (head_dim 128 has waited for them already, at the end of block i - 1)
@@ -852,6 +862,13 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       if (i + 1 < nq) publish_vectors(i + 1);  // other stage than the one block i used
       softmax_bar_sync();  // the vectors of block i+1 are complete; those of block i are dead
     }
+    // the bucket of this thread's first relative position, requested before the last MMAs are
+    // waited for
+    int first_bucket = -1;
+    if (p.d_rel_bias != nullptr) {
+      const int idx = k0 + (static_cast<int>(threadIdx.x) - lq_pad) + p.rel_off;
+      if (idx >= 0 && idx < p.nrel) first_bucket = __ldg(p.rel_bucket + idx);
+    }
     if (D == 64 && ok) {
       ok = mbar_wait_relaxed(bar_dq, (nq - 1) & 1, abort_flag);
       if (ok) {
@@ -876,14 +893,36 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       }
       softmax_bar_sync();
       if (p.d_rel_bias != nullptr) {
-        // sDRel[t] holds sum dS over (k - q) = k0 + t - lq_pad for this key block
-        float* out = p.d_rel_bias + static_cast<long long>(h) * p.nrel;
-        for (int t = threadIdx.x; t < lq_pad + 128; t += kSoftmaxThreads) {
-          const float g = sDRel[t];
-          if (g != 0.f) {
-            const int idx = k0 + (t - lq_pad) + p.rel_off;  // (k - q) + rel_off
-            if (idx >= 0 && idx < p.nrel) atomicAdd(out + idx, g);
+        // sDRel[t] holds sum dS over (k - q) = k0 + t - lq_pad for this key block. The relative
+        // positions are folded into their buckets here (a few dozen sums per head), so that one
+        // CTA adds num_buckets values to memory and no expanded gradient exists.
+        // Neighbouring positions share buckets (far ones a single bucket): each run of equal
+        // buckets in a warp is summed by shuffles and added once.
+        float* out = p.d_rel_bias + static_cast<long long>(h) * p.num_buckets;
+        const bool in_smem = p.num_buckets <= kSmemBuckets;
+        float* bucket_sum = in_smem ? sBucket : out;
+        for (int t = threadIdx.x; t < lq_pad + 128; t += kSoftmaxThreads) {  // whole warps
+          float g = sDRel[t];
+          const int idx = k0 + (t - lq_pad) + p.rel_off;  // (k - q) + rel_off
+          const int bucket =
+              t == threadIdx.x ? first_bucket
+                               : ((idx >= 0 && idx < p.nrel) ? __ldg(p.rel_bucket + idx) : -1);
+          const int before = __shfl_up_sync(0xffffffffu, bucket, 1);
+          const bool head = lane == 0 || before != bucket;
+          const uint32_t heads = __ballot_sync(0xffffffffu, head);
+          const uint32_t later = lane == 31 ? 0u : heads >> (lane + 1);
+          const int run_end = later ? lane + __ffs(later) : 32;  // first lane of the next run
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const float v = __shfl_down_sync(0xffffffffu, g, o);
+            if (lane + o < run_end) g += v;
           }
+          if (head && bucket >= 0 && g != 0.f) atomicAdd(bucket_sum + bucket, g);
+        }
+        if (in_smem) {
+          softmax_bar_sync();
+          for (int t = threadIdx.x; t < p.num_buckets; t += kSoftmaxThreads)
+            if (bucket_sum[t] != 0.f) atomicAdd(out + t, bucket_sum[t]);
         }
       }
     } else if (lane == 0) {
@@ -906,14 +945,16 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
 using namespace t5x;
 
 // q [B,Lq,H,64], k/v [B,Lk,H,64] bf16 with element strides (sb, sl, sh), innermost contiguous.
-// rel_bias [H, nrel] fp32 or null: bias = rel_bias[h][(k - q) + rel_off].
+// rel_bias [H, num_buckets] fp32 or null, rel_bucket [nrel] int32 in [0, num_buckets):
+// bias = rel_bias[h][rel_bucket[(k - q) + rel_off]].
 T5X_API int t5x_attention_fwd(const void* q, const void* k, const void* v, void* o, void* lse, int B,
                               int H, int Lq, int Lk, long long q_sb, long long q_sl, long long q_sh,
                               long long k_sb, long long k_sl, long long k_sh, long long v_sb,
                               long long v_sl, long long v_sh, long long o_sb, long long o_sl,
-                              long long o_sh, const void* rel_bias, int nrel, int rel_off,
-                              const void* key_mask, const void* q_seg, const void* kv_seg,
-                              int causal, int causal_off, void* stream) {
+                              long long o_sh, const void* rel_bias, const void* rel_bucket,
+                              int num_buckets, int nrel, int rel_off, const void* key_mask,
+                              const void* q_seg, const void* kv_seg, int causal, int causal_off,
+                              void* stream) {
   if (B <= 0 || H <= 0 || Lq <= 0 || Lk <= 0) return 0;
   if (Lk > 512) return set_error("attention_fwd: Lk=%d > 512 is not covered by this kernel", Lk);
   if (causal == 2) return set_error("attention_fwd: prefix-LM masks need the streaming kernel");
@@ -926,6 +967,8 @@ T5X_API int t5x_attention_fwd(const void* q, const void* k, const void* v, void*
   AttnParams p = {};
   p.B = B; p.H = H; p.Lq = Lq; p.Lk = Lk;
   p.rel_bias = static_cast<const float*>(rel_bias);
+  p.rel_bucket = static_cast<const int*>(rel_bucket);
+  p.num_buckets = num_buckets;
   p.nrel = nrel; p.rel_off = rel_off;
   p.key_mask = static_cast<const uint8_t*>(key_mask);
   p.q_seg = static_cast<const int*>(q_seg);
@@ -993,8 +1036,9 @@ T5X_API int t5x_attention_bwd(const void* q, const void* k, const void* v, const
                               long long k_sh, long long v_sb, long long v_sl, long long v_sh,
                               long long o_sb, long long o_sl, long long o_sh, long long do_sb,
                               long long do_sl, long long do_sh, long long dk_sb, long long dk_sl,
-                              long long dk_sh, const void* rel_bias, void* d_rel_bias, int nrel,
-                              int rel_off, const void* key_mask, const void* q_seg,
+                              long long dk_sh, const void* rel_bias, const void* rel_bucket,
+                              void* d_rel_bias, int num_buckets, int nrel, int rel_off,
+                              const void* key_mask, const void* q_seg,
                               const void* kv_seg, int causal, int causal_off, void* stream) {
   if (B <= 0 || H <= 0 || Lq <= 0 || Lk <= 0) return 0;
   if (D != 64 && D != 128) return set_error("attention_bwd: head_dim %d not in {64, 128}", D);
@@ -1010,6 +1054,8 @@ T5X_API int t5x_attention_bwd(const void* q, const void* k, const void* v, const
   AttnParams p = {};
   p.B = B; p.H = H; p.Lq = Lq; p.Lk = Lk;
   p.rel_bias = static_cast<const float*>(rel_bias);
+  p.rel_bucket = static_cast<const int*>(rel_bucket);
+  p.num_buckets = num_buckets;
   p.d_rel_bias = static_cast<float*>(d_rel_bias);
   p.nrel = nrel; p.rel_off = rel_off;
   p.key_mask = static_cast<const uint8_t*>(key_mask);

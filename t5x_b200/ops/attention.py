@@ -1,10 +1,12 @@
 """Flash attention with in-kernel T5 relative-position bias (CUDA path of `functional.attention`).
 
-The [heads, buckets] bias table is expanded on the host into a per-relative-offset table
-`rel_bias[h, (k - q) + Lq - 1]` with the oracle's own bucket function (so bucket boundaries are
-bit-identical); the kernels index it by `k - q`, build the masks from per-token metadata and
-never materialise [b, h, q, k] scores. The gradient of the expanded table comes back from the
-backward kernel and autograd folds it into the bucket table.
+The kernels read the [heads, buckets] bias table itself and the bucket of every relative offset,
+`bucket[(k - q) + Lq - 1]`, which comes from the oracle's own bucket function (so bucket
+boundaries are bit-identical); they build the masks from per-token metadata and never
+materialise [b, h, q, k] scores. The backward kernel folds the bias gradient into the buckets
+and adds it to the table's gradient, in `main_grad` when the table has one. (With the table
+expanded per offset by tensor ops, each layer paid an indexing kernel forward and five kernels
+backward, 27 to 57 us a layer for the sort-based index backward alone.)
 """
 from __future__ import annotations
 
@@ -17,15 +19,15 @@ from t5x_b200.ops import reference as ref
 
 c_void_p, c_int, c_ll = native.c_void_p, native.c_int, native.c_ll
 native.register_signature("t5x_attention_fwd", [c_void_p] * 5 + [c_int] * 4 + [c_ll] * 12 +
-                          [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
-                           c_void_p])
+                          [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                           c_int, c_int, c_void_p])
 native.register_signature("t5x_attention_bwd", [c_void_p] * 10 + [c_int] * 5 + [c_ll] * 18 +
-                          [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int,
-                           c_int, c_void_p])
+                          [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
+                           c_void_p, c_int, c_int, c_void_p])
 
 native.register_signature("t5x_attention_fwd_stream", [c_void_p] * 5 + [c_int] * 5 + [c_ll] * 12 +
-                          [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
-                           c_void_p])
+                          [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                           c_int, c_int, c_void_p])
 
 # The short-range forward kernel keeps the scores of a whole key range in TMEM.
 CLASSIC_MAX_LK = 512
@@ -77,10 +79,16 @@ def _packed_qkv(q, k, v) -> bool:
           k.data_ptr() == q.data_ptr() + step and v.data_ptr() == q.data_ptr() + 2 * step)
 
 
+def _bias_sizes(rel_bias, buckets):
+  """(number of buckets, number of relative offsets)."""
+  return (0, 0) if rel_bias is None else (rel_bias.shape[1], buckets.shape[0])
+
+
 class _FlashAttentionFn(torch.autograd.Function):
 
   @staticmethod
-  def forward(ctx, q, k, v, rel_bias, key_mask, q_seg, kv_seg, causal, causal_off, rel_off):
+  def forward(ctx, q, k, v, rel_bias, buckets, key_mask, q_seg, kv_seg, causal, causal_off,
+              rel_off):
     q = q if _strides_ok(q) else q.contiguous()
     k = k if _strides_ok(k) else k.contiguous()
     v = v if _strides_ok(v) else v.contiguous()
@@ -88,9 +96,9 @@ class _FlashAttentionFn(torch.autograd.Function):
     Lk = k.shape[1]
     o = torch.empty((B, Lq, H, D), dtype=torch.bfloat16, device=q.device)
     lse = torch.empty((B, H, Lq), dtype=torch.float32, device=q.device)
-    nrel = rel_bias.shape[1] if rel_bias is not None else 0
-    tail = (*_sbh(q), *_sbh(k), *_sbh(v), *_sbh(o), native.ptr(rel_bias), nrel, rel_off,
-            native.ptr(key_mask), native.ptr(q_seg), native.ptr(kv_seg), int(causal), causal_off,
+    nb, nrel = _bias_sizes(rel_bias, buckets)
+    tail = (*_sbh(q), *_sbh(k), *_sbh(v), *_sbh(o), native.ptr(rel_bias), native.ptr(buckets), nb,
+            nrel, rel_off, native.ptr(key_mask), native.ptr(q_seg), native.ptr(kv_seg), int(causal), causal_off,
             native.stream_ptr())
     if forward_kernel(Lq, Lk, D, int(causal) == 2) == "classic":
       rc = native.lib().t5x_attention_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
@@ -100,13 +108,13 @@ class _FlashAttentionFn(torch.autograd.Function):
                                                  o.data_ptr(), lse.data_ptr(), B, H, Lq, Lk, D,
                                                  *tail)
     native._check(rc, "attention_fwd")
-    ctx.save_for_backward(q, k, v, o, lse, rel_bias, key_mask, q_seg, kv_seg)
+    ctx.save_for_backward(q, k, v, o, lse, rel_bias, buckets, key_mask, q_seg, kv_seg)
     ctx.cfg = (causal, causal_off, rel_off)
     return o
 
   @staticmethod
   def backward(ctx, do):
-    q, k, v, o, lse, rel_bias, key_mask, q_seg, kv_seg = ctx.saved_tensors
+    q, k, v, o, lse, rel_bias, buckets, key_mask, q_seg, kv_seg = ctx.saved_tensors
     causal, causal_off, rel_off = ctx.cfg
     B, Lq, H, D = q.shape
     Lk = k.shape[1]
@@ -120,21 +128,30 @@ class _FlashAttentionFn(torch.autograd.Function):
       dk = torch.empty((B, Lk, H, D), dtype=torch.bfloat16, device=q.device)
       dv = torch.empty((B, Lk, H, D), dtype=torch.bfloat16, device=q.device)
     delta = torch.empty((B, H, Lq), dtype=torch.float32, device=q.device)
-    d_rel = torch.zeros_like(rel_bias) if rel_bias is not None else None
-    nrel = rel_bias.shape[1] if rel_bias is not None else 0
+    nb, nrel = _bias_sizes(rel_bias, buckets)
+    d_rel = ret_rel = None  # the buffer the kernel adds to, and what autograd gets
+    if rel_bias is not None and ctx.needs_input_grad[3]:
+      mg = getattr(rel_bias, "main_grad", None)
+      if mg is not None and mg.is_contiguous():
+        if not getattr(rel_bias, "grad_ready", False):
+          mg.zero_()
+          rel_bias.grad_ready = True
+        d_rel = mg
+      else:
+        d_rel = ret_rel = torch.zeros_like(rel_bias)
     rc = native.lib().t5x_attention_bwd(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
         delta.data_ptr(), dq32.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Lq, Lk, D,
         *_sbh(q),
         *_sbh(k), *_sbh(v), *_sbh(o), *_sbh(do), *_sbh(dk), native.ptr(rel_bias),
-        native.ptr(d_rel), nrel, rel_off, native.ptr(key_mask), native.ptr(q_seg),
+        native.ptr(buckets), native.ptr(d_rel), nb, nrel, rel_off, native.ptr(key_mask), native.ptr(q_seg),
         native.ptr(kv_seg), int(causal), causal_off, native.stream_ptr())
     native._check(rc, "attention_bwd")
     if packed:
       dq.copy_(dq32)
     else:
       dq = dq32.to(torch.bfloat16)
-    return dq, dk, dv, d_rel, None, None, None, None, None, None
+    return dq, dk, dv, ret_rel, None, None, None, None, None, None, None
 
 
 _BUCKET_CACHE: dict = {}
@@ -147,7 +164,7 @@ def _rel_buckets(Lq, Lk, q_offset, bidirectional, num_buckets, max_distance, dev
   b = _BUCKET_CACHE.get(key)
   if b is None:
     rel = torch.arange(Lq + Lk - 1, device=device) - (Lq - 1) - q_offset
-    b = ref.relative_position_bucket(rel, bidirectional, num_buckets, max_distance)
+    b = ref.relative_position_bucket(rel, bidirectional, num_buckets, max_distance).to(torch.int32)
     if len(_BUCKET_CACHE) > 256:
       _BUCKET_CACHE.clear()
     _BUCKET_CACHE[key] = b
@@ -163,10 +180,13 @@ def flash_attention(q, k, v, *, bias_table: Optional[torch.Tensor] = None,
   `key_mask` and the segment ids (which it contains)."""
   B, Lq, H, D = q.shape
   Lk = k.shape[1]
-  rel_bias = None
+  rel_bias = buckets = None
   if bias_table is not None:
-    rel_bias = bias_table.float()[:, _rel_buckets(Lq, Lk, q_offset, bidirectional, num_buckets,
-                                                  max_distance, q.device)].contiguous()
+    # an fp32 parameter goes in as it is, so that its gradient buffer is found in backward
+    rel_bias = bias_table.float().contiguous()
+    if rel_bias.shape[1] < num_buckets:
+      raise ValueError(f"bias table has {rel_bias.shape[1]} buckets, {num_buckets} are indexed")
+    buckets = _rel_buckets(Lq, Lk, q_offset, bidirectional, num_buckets, max_distance, q.device)
   km = key_mask.to(torch.uint8).contiguous() if key_mask is not None else None
   qs = q_segment_ids.to(torch.int32).contiguous() if q_segment_ids is not None else None
   ks = kv_segment_ids.to(torch.int32).contiguous() if kv_segment_ids is not None else None
@@ -178,5 +198,5 @@ def flash_attention(q, k, v, *, bias_table: Optional[torch.Tensor] = None,
     valid = prefix_lm.valid.to(torch.uint8)
     km = valid.contiguous() if km is None else (km & valid).contiguous()
     mode = 2
-  return _FlashAttentionFn.apply(q, k, v, rel_bias, km, qs, ks, mode,
+  return _FlashAttentionFn.apply(q, k, v, rel_bias, buckets, km, qs, ks, mode,
                                  (Lk - Lq) if mode else 0, Lq - 1)

@@ -184,3 +184,30 @@ def test_prefix_lm_visibility_from_per_token_codes(length):
   for n, g, w in zip(["out", "dq", "dk", "dv", "dbias"], got,
                      [exp.detach(), q.grad, k.grad, v.grad, table.grad]):
     assert rel(g, w) < TOL, (n, rel(g, w))
+
+
+@pytest.mark.parametrize("buckets,lq,lk,main_grad", [(32, 130, 70, True), (32, 600, 600, False),
+                                                     (300, 257, 257, True)])
+def test_bias_gradient_by_bucket(buckets, lq, lk, main_grad):
+  """The kernels read the bucket table and add its gradient per bucket: in shared memory up to 128
+  buckets, straight to memory beyond; into `main_grad` (cleared by the first use of a step,
+  added to by the next) or through autograd. fp32 sums over bf16-rounded dS: 1e-2 relative."""
+  from t5x_b200.ops import attention as attn, reference as ref
+  g = torch.Generator(device="cuda").manual_seed(lq)
+  q, k, v, do = (torch.randn(2, l, 2, 64, device="cuda", generator=g).bfloat16().requires_grad_()
+                 for l in (lq, lk, lk, lq))
+  table = torch.nn.Parameter(torch.randn(2, buckets, device="cuda", generator=g))
+  kw = dict(bidirectional=True, num_buckets=buckets, max_distance=400)
+  if main_grad:
+    table.main_grad = torch.full_like(table, 7.0)
+    table.grad_ready = False
+  for _ in range(2):
+    attn.flash_attention(q, k, v, bias_table=table, **kw).backward(do.detach())
+  got = table.main_grad if main_grad else table.grad
+  want_table = table.detach().clone().requires_grad_()
+  bias = ref.relative_position_bias(want_table, lq, lk, True, buckets, 400)
+  ref.attention(q.detach().float(), k.detach().float(), v.detach().float(),
+                bias=bias).backward(do.detach().float())
+  want = 2 * want_table.grad
+  assert float((got - want).norm() / want.norm()) < 1e-2
+  assert (table.grad is None) == main_grad
