@@ -173,6 +173,36 @@ __global__ void __launch_bounds__(kDecWarps * 32)
   }
 }
 
+// First kernel of a decode step: looks up the embedding row of every live row's token at the
+// current position and lays out the T5 bias of that position, bias_row[h][t] =
+// table[h][bucket_of_distance[cur - t]] for t <= cur (bucket 0 beyond it, as for any key not
+// before its query). One block per row, then one per head. As tensor operations this was some
+// sixteen launches of 2 us each per step.
+constexpr int kBeginThreads = 128;
+__global__ void __launch_bounds__(kBeginThreads)
+    decode_begin_kernel(const long long* __restrict__ live_seqs,  // [rows, L]
+                        const int* __restrict__ cur_index, const __nv_bfloat16* __restrict__ emb,
+                        __nv_bfloat16* __restrict__ x, const float* __restrict__ table,
+                        const int* __restrict__ bucket_of_distance, float* __restrict__ bias_row,
+                        int rows, int L, int d, int vocab, int num_buckets) {
+  chain_release();
+  chain_wait();
+  const int cur = min(max(*cur_index, 0), L - 1);
+  if (static_cast<int>(blockIdx.x) < rows) {
+    const int row = blockIdx.x;
+    const long long id = live_seqs[static_cast<long long>(row) * L + cur];
+    const long long tok = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
+    const uint4* src = reinterpret_cast<const uint4*>(emb + tok * d);
+    uint4* dst = reinterpret_cast<uint4*>(x + static_cast<long long>(row) * d);
+    for (int v = threadIdx.x; v < d / 8; v += kBeginThreads) dst[v] = src[v];
+    return;
+  }
+  const int h = blockIdx.x - rows;
+  for (int t = threadIdx.x; t < L; t += kBeginThreads)
+    bias_row[static_cast<long long>(h) * L + t] =
+        table[static_cast<long long>(h) * num_buckets + bucket_of_distance[max(cur - t, 0)]];
+}
+
 constexpr int kCrossWarps = 8;
 constexpr int kCrossThreads = kCrossWarps * 32;
 constexpr int kCrossMaxKeys = 1024;
@@ -332,6 +362,30 @@ using namespace t5x;
 // batch * beams; cache_k / cache_v: [batch, beams, heads, max_len, 64] bf16; ancestry:
 // [batch, beams, max_len] int32; bias_row: [heads, max_len] fp32 or null; cur_index: device
 // int32 (position being decoded).
+// live_seqs [rows, L] int64, cur_index device int32, emb [vocab, d] bf16 (d % 8 == 0, 16-byte
+// aligned), x [rows, d] bf16; table [H, num_buckets] fp32, bucket_of_distance [L] int32 in
+// [0, num_buckets), bias_row [H, L] fp32.
+T5X_API int t5x_decode_begin(const void* live_seqs, const void* cur_index, const void* emb, void* x,
+                             const void* table, const void* bucket_of_distance, void* bias_row,
+                             int rows, int H, int L, int d, int vocab, int num_buckets,
+                             void* stream) {
+  using namespace t5x;
+  if (rows <= 0 || L <= 0) return 0;
+  if (d % 8 || ((reinterpret_cast<uintptr_t>(emb) | reinterpret_cast<uintptr_t>(x)) & 15))
+    return set_error("decode_begin: embedding rows must be 16-byte aligned (d=%d)", d);
+  cudaError_t e = launch_chained(
+      decode_begin_kernel, dim3(rows + H), dim3(kBeginThreads), 0,
+      static_cast<cudaStream_t>(stream), static_cast<const long long*>(live_seqs),
+      static_cast<const int*>(cur_index), static_cast<const __nv_bfloat16*>(emb),
+      static_cast<__nv_bfloat16*>(x), static_cast<const float*>(table),
+      static_cast<const int*>(bucket_of_distance), static_cast<float*>(bias_row), rows, L, d, vocab,
+      num_buckets);
+  count_launches(1);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) return set_error("decode_begin: %s", cudaGetErrorString(e));
+  return 0;
+}
+
 T5X_API int t5x_decode_self_attention(const void* q, const void* k_new, const void* v_new,
                                       void* cache_k, void* cache_v, const void* ancestry,
                                       const void* bias_row, const void* cur_index, void* out,

@@ -29,6 +29,7 @@ from t5x_b200.ops import reference as ref
 c_void_p, c_int, c_ll = native.c_void_p, native.c_int, native.c_ll
 native.register_signature("t5x_decode_self_attention",
                           [c_void_p] * 9 + [c_ll, c_int, c_int, c_int, c_int, c_int, c_void_p])
+native.register_signature("t5x_decode_begin", [c_void_p] * 7 + [c_int] * 6 + [c_void_p])
 native.register_signature("t5x_decode_cross_attention",
                           [c_void_p] * 5 + [c_ll, c_int, c_int, c_int, c_int, c_int, c_void_p])
 native.register_signature("t5x_decode_self_attention_mma",
@@ -39,6 +40,16 @@ native.register_signature("t5x_decode_cross_attention_mma",
                            c_void_p])
 
 NEG_INF = decoding.NEG_INF
+# Up to this many rows (batch * beams) a decode step runs `native.gemm_rows` where it covers a
+# product. Without a norm in front it was faster at every shape it covers (us, cold weights; against
+# the cluster split-K GEMM: 4 rows 768 x 768 3.5 / 7.5, 2048 x 768 4.9 / 8.7, 2048 x 2048 6.1 / 17.3;
+# 64 rows 768 x 768 8.1 / 9.8).
+FEW_ROWS = 64
+# With a norm in front every CTA normalises all rows for itself, which pays up to this many
+# elements (against a norm launch and the tcgen05 GEMM: 4 x 768 to 2304 columns 4.3 / 10.3, 32 x 768
+# 7.8 / 10.6, 8 x 2048 to 6144 11.9 / 16.9; beyond the line 32 x 1024 to 3072 15.4 / 12.6,
+# 16 x 2048 to 6144 17.7 / 17.0).
+FUSED_NORM_ELEMENTS = 24576
 
 
 def decode_self_attention(q, k_new, v_new, cache_k, cache_v, ancestry, bias_row, cur_index, out,
@@ -313,6 +324,7 @@ class GraphBeamDecoder:
     wl = w.bf16
     self.w_logits = wl if wl.shape[0] == c.emb_dim else wl.t()
     self.rel_table = dec.relpos_bias.rel_embedding
+    self.few_rows = self.tp == 1 and self.rows <= FEW_ROWS
     bf = dict(dtype=torch.bfloat16, device=dev)
     # [batch, beam slot, head, position, dim]: one (slot, head) history is contiguous. For the
     # tensor-core kernel the cache is padded to a multiple of 32 positions and the values are
@@ -345,7 +357,10 @@ class GraphBeamDecoder:
     self.fin_flags = torch.zeros(batch, beams, dtype=torch.bool, device=dev)
     self.anc = torch.zeros(batch, beams, self.L, dtype=torch.int32, device=dev)
     self.terminated = torch.zeros(1, dtype=torch.bool, device=dev)
-    self.positions = torch.arange(self.L, device=dev)
+    # bucket of key position minus query position = -distance
+    self.bucket_of_distance = ref.relative_position_bucket(
+        -torch.arange(self.L, device=dev), False, c.relpos_num_buckets,
+        c.relpos_max_distance).to(torch.int32)
     self.min_brevity = float(decoding.brevity_penalty(alpha, self.L))
     self.graph: Optional[torch.cuda.CUDAGraph] = None
     self._graph_enc_len = -1
@@ -386,16 +401,69 @@ class GraphBeamDecoder:
       from t5x_b200.parallel import tp_fused
       tp_fused.end_step()  # the encoder pass is over: its arena blocks are free again
 
+  def _rows_ok(self, w: torch.Tensor, gated: bool = False) -> bool:
+    """Whether `native.gemm_rows` covers the product of this decoder's rows with weight `w`."""
+    return (w.stride(1) == 1 and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0 and
+            native.gemm_rows_ok(self.rows, w.shape[1], w.shape[0], gated))
+
+  def _norm_matmul(self, x, scale, w, w2=None, out_dtype=torch.bfloat16, alpha: float = 1.0):
+    """alpha * norm(x) @ w, or with `w2` the gated GELU of both, for few rows."""
+    if x.numel() <= FUSED_NORM_ELEMENTS and self._rows_ok(w, w2 is not None) and \
+        (w2 is None or w2.data_ptr() % 16 == 0) and scale.dtype == torch.float32 and \
+        scale.is_contiguous() and scale.data_ptr() % 16 == 0:
+      return native.gemm_rows(x, w, b2=w2, norm_scale=scale, out_dtype=out_dtype, alpha=alpha)
+    h = native.rmsnorm_fwd(x, scale, 1e-6)[0]
+    if w2 is None and out_dtype == torch.bfloat16 and w.shape[1] == self.H * self.D:
+      return self._skinny(h, w)
+    return native.gemm(h, w, b2=w2, out_dtype=out_dtype, alpha=alpha)
+
+  def _layers_few_rows(self, x: torch.Tensor, bias_row: torch.Tensor) -> torch.Tensor:
+    """The decoder layers of one step for few rows: eight launches a layer where `gemm_rows`
+    covers every product."""
+    rows, H, D = self.rows, self.H, self.D
+    ctx = torch.empty(rows, H, D, dtype=torch.bfloat16, device=self.dev)
+    for i, ly in enumerate(self.layers):
+      qkv = self._norm_matmul(x, ly.ln1, ly.qkv).view(rows, 3, H, D)
+      self._self_attention(i, qkv, bias_row, ctx)
+      x = self._skinny(ctx.view(rows, H * D), ly.o, residual=x)
+      qc = self._norm_matmul(x, ly.ln2, ly.cq).view(rows, H, D)
+      cc = self._cross_attention(i, qc, ctx)
+      x = self._skinny(cc.reshape(rows, H * D), ly.co, residual=x)
+      x = self._skinny(self._norm_matmul(x, ly.ln3, ly.wi0, ly.wi1), ly.wo, residual=x)
+    return x
+
+  def _self_attention(self, i: int, qkv, bias_row, ctx) -> None:
+    if self.self_mma:
+      decode_self_attention_mma(qkv[:, 0], qkv[:, 1], qkv[:, 2], self.cache_k[i], self.cache_v[i],
+                                self.anc, bias_row, self.cur, ctx, self.k, self.L)
+    else:
+      decode_self_attention(qkv[:, 0], qkv[:, 1], qkv[:, 2], self.cache_k[i], self.cache_v[i],
+                            self.anc, bias_row, self.cur, ctx, self.k)
+
+  def _cross_attention(self, i: int, qc, ctx) -> torch.Tensor:
+    """Writes into `ctx` where the tensor-core kernel covers the call; returns the result."""
+    if self.cross_mma:
+      decode_cross_attention_mma(qc, self.cross_k[i], self.cross_v[i], self.enc_mask_u8, ctx,
+                                 self.k, self.enc_len)
+      return ctx
+    return attn_ops.flash_attention(qc.view(self.b, self.k, self.H, self.D),
+                                    self.cross_k[i].transpose(1, 2),
+                                    self.cross_v[i].transpose(1, 2), key_mask=self.enc_mask)
+
   def _model_step(self) -> torch.Tensor:
     """Logits [rows, vocab] (fp32) of the token at position `cur` of every live beam."""
     c, rows, H, D = self.c, self.rows, self.H, self.D
-    ci = self.cur.long()
-    tok = self.live_seqs.gather(2, ci.view(1, 1, 1).expand(self.b, self.k, 1)).reshape(rows)
-    x = self.emb.index_select(0, tok)
-    rel = self.positions - ci  # key position minus query position
-    buckets = ref.relative_position_bucket(rel, False, c.relpos_num_buckets,
-                                           c.relpos_max_distance)
-    bias_row = self.rel_table.float()[:, buckets].contiguous()  # [H, L]
+    x = torch.empty(rows, c.emb_dim, dtype=torch.bfloat16, device=self.dev)
+    bias_row = torch.empty(H, self.L, dtype=torch.float32, device=self.dev)
+    # the embedding rows of the current tokens, and the bias of every position for the current one
+    table = self.rel_table.float().contiguous()
+    native._check(native.lib().t5x_decode_begin(
+        self.live_seqs.data_ptr(), self.cur.data_ptr(), self.emb.data_ptr(), x.data_ptr(),
+        table.data_ptr(), self.bucket_of_distance.data_ptr(), bias_row.data_ptr(), rows, H, self.L,
+        c.emb_dim, self.emb.shape[0], table.shape[1], native.stream_ptr()), "decode_begin")
+    if self.few_rows:
+      return self._norm_matmul(self._layers_few_rows(x, bias_row), self.final_ln, self.w_logits,
+                               out_dtype=torch.float32, alpha=self.logit_scale)
     ctx = torch.empty(rows, H, D, dtype=torch.bfloat16, device=self.dev)
     if self.link is not None:
       self.link.begin_step()
@@ -406,23 +474,10 @@ class GraphBeamDecoder:
       # residual stream and its normed form (one finishing kernel on the single-GPU path)
       next_ln1 = norms[i + 1][0] if i + 1 < len(self.layers) else self.final_ln
       qkv = native.gemm(h, ly.qkv).view(rows, 3, H, D)
-      if self.self_mma:
-        decode_self_attention_mma(qkv[:, 0], qkv[:, 1], qkv[:, 2], self.cache_k[i],
-                                  self.cache_v[i], self.anc, bias_row, self.cur, ctx, self.k,
-                                  self.L)
-      else:
-        decode_self_attention(qkv[:, 0], qkv[:, 1], qkv[:, 2], self.cache_k[i], self.cache_v[i],
-                              self.anc, bias_row, self.cur, ctx, self.k)
+      self._self_attention(i, qkv, bias_row, ctx)
       x, h = self._row_parallel(ctx.view(rows, H * D), ly.o, x, ly.ln2)
       qc = self._skinny(h, ly.cq).view(rows, H, D)
-      if self.cross_mma:
-        decode_cross_attention_mma(qc, self.cross_k[i], self.cross_v[i], self.enc_mask_u8, ctx,
-                                   self.k, self.enc_len)
-        cc = ctx
-      else:
-        cc = attn_ops.flash_attention(qc.view(self.b, self.k, H, D),
-                                      self.cross_k[i].transpose(1, 2),
-                                      self.cross_v[i].transpose(1, 2), key_mask=self.enc_mask)
+      cc = self._cross_attention(i, qc, ctx)
       x, h = self._row_parallel(cc.reshape(rows, H * D), ly.co, x, ly.ln3)
       g = native.gemm(h, ly.wi0, b2=ly.wi1)
       x, h = self._row_parallel(g, ly.wo, x, next_ln1)
@@ -448,7 +503,10 @@ class GraphBeamDecoder:
                                    workspace=self._workspace())
 
   def _skinny(self, a, w, residual=None):
-    """a[rows, K] @ w[K, N] (+ residual) with K split over CTAs when rows are few."""
+    """a[rows, K] @ w[K, N] (+ residual) for few rows: the whole K per CTA up to FEW_ROWS rows,
+    K split over CTAs up to 512."""
+    if self.few_rows and self._rows_ok(w):
+      return native.gemm_rows(a, w, residual=residual)
     if self.rows > 512:
       return native.gemm(a, w, residual=residual)
     if self.cluster_gemm:

@@ -1,0 +1,68 @@
+"""The few-row GEMM with its norm, residual and gated-GELU forms at 1 to 64 rows, K and N down to
+one step, and the decode step built from it. The bf16 output rounds to 2^-9 relative; the
+normalised operand is rounded to bf16 in both forms."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 16, 16), (4, 768, 768), (8, 32, 144), (16, 48, 2048),
+                                   (17, 64, 1024), (33, 16, 1040), (64, 80, 512)])
+@pytest.mark.parametrize("norm", [False, True])
+def test_gemm_rows(M, N, K, norm):
+  from t5x_b200.ops import native
+  assert native.gemm_rows_ok(M, N, K) and native.gemm_rows_ok(M, N, K, gated=True)
+  g = torch.Generator(device="cuda").manual_seed(M * N + K)
+  rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+  a = (rnd(M, K + 8) * 3).bfloat16()[:, :K]
+  b, b2 = ((rnd(K, N + 8) * K ** -0.5).bfloat16()[:, :N] for _ in range(2))
+  scale = 1 + 0.1 * rnd(K) if norm else None
+  h = a.double()
+  if norm:
+    h = native.rmsnorm_fwd(a.contiguous(), scale, 1e-6)[0].double()
+  res = rnd(M, N).bfloat16()
+  tol = dict(rtol=2 ** -7, atol=2 ** -7)
+  y = native.gemm_rows(a, b, norm_scale=scale, residual=res)
+  torch.testing.assert_close(y.double(), h @ b.double() + res.double(), **tol)
+  z = native.gemm_rows(a, b, norm_scale=scale, out_dtype=torch.float32, alpha=0.5)
+  # one operand in a few thousand may round the other way where the norm's sum order differs
+  torch.testing.assert_close(z.double(), 0.5 * (h @ b.double()), rtol=1e-3, atol=4e-3)
+  y = native.gemm_rows(a, b, b2=b2, norm_scale=scale)
+  gelu = torch.nn.functional.gelu(h @ b.double(), approximate="tanh")
+  torch.testing.assert_close(y.double(), gelu * (h @ b2.double()), rtol=2 ** -6, atol=2 ** -5)
+
+
+def test_refuses_what_it_does_not_cover():
+  from t5x_b200.ops import native
+  for m, n, k in [(0, 16, 16), (65, 16, 16), (4, 24, 16), (4, 16, 24), (64, 16, 2048)]:
+    assert not native.gemm_rows_ok(m, n, k)
+  a = torch.zeros(4, 32, device="cuda", dtype=torch.bfloat16)
+  with pytest.raises(native.NativeError):
+    native.gemm_rows(a, torch.zeros(32, 24, device="cuda", dtype=torch.bfloat16))
+
+
+@pytest.mark.parametrize("batch,beams", [(1, 1), (3, 4), (16, 4)])
+def test_decode_step_agrees_with_the_other_kernels(batch, beams):
+  """The same search with and without the few-row products: the same logits up to bf16."""
+  from t5x_b200 import decoding_fast, trainer
+  from t5x_b200.models.t5 import network
+  torch.manual_seed(0)
+  cfg = network.T5Config(vocab_size=256, dtype="bfloat16", emb_dim=256, num_heads=4, head_dim=64,
+                         num_encoder_layers=1, num_decoder_layers=2, mlp_dim=512,
+                         mlp_activations=("gelu", "linear"), dropout_rate=0.0)
+  module = network.Transformer(cfg, device="cuda")
+  for p in module.parameters():
+    p.bf16 = p.detach().bfloat16()
+  enc = torch.randint(2, 256, (batch, 19), device="cuda")
+  logits = []
+  for few in (True, False):
+    d = decoding_fast.GraphBeamDecoder(module, batch, beams, 12, 1, use_graph=False)
+    assert d.few_rows == (batch * beams <= decoding_fast.FEW_ROWS)
+    d.few_rows = few
+    with torch.no_grad():
+      d._encode(enc)
+      d._reset()
+      logits.append(d._model_step())
+  scale = logits[1].abs().max()
+  assert float((logits[0] - logits[1]).abs().max() / scale) < 0.03
