@@ -24,21 +24,23 @@ constexpr int kAfThreads = 256;
 constexpr int kAfTileR = 64;
 constexpr int kAfTileC = 512;
 
+// One 64 x 512 tile (tile_x, tile_y) of batch element b: row and column sums of g^2 + eps1, sum p^2.
 template <bool VEC>
-__global__ void __launch_bounds__(kAfThreads)
-    af_stats_kernel(const float* __restrict__ g, const float* __restrict__ p,
-                    float* __restrict__ rowsum, float* __restrict__ colsum,
-                    AdafactorScalars* __restrict__ scal, int R, int C, float eps1) {
+__device__ __forceinline__ void af_stats_tile(const float* __restrict__ g,
+                                              const float* __restrict__ p,
+                                              float* __restrict__ rowsum,
+                                              float* __restrict__ colsum,
+                                              AdafactorScalars* __restrict__ scal, int R, int C,
+                                              float eps1, int tile_x, int tile_y, int b) {
   __shared__ float scol[kAfTileC];
   __shared__ float red[32];
-  const int b = blockIdx.z;
   const long long base = static_cast<long long>(b) * R * C;
   g += base;
   p += base;
   rowsum += static_cast<long long>(b) * R;
   colsum += static_cast<long long>(b) * C;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int tile_r = blockIdx.y * kAfTileR, tile_c = blockIdx.x * kAfTileC;
+  const int tile_r = tile_y * kAfTileR, tile_c = tile_x * kAfTileC;
   for (int i = threadIdx.x; i < kAfTileC; i += kAfThreads) scol[i] = 0.f;
   __syncthreads();
   float cacc[4][4];
@@ -134,17 +136,25 @@ __global__ void __launch_bounds__(kAfThreads)
   }
 }
 
+template <bool VEC>
+__global__ void __launch_bounds__(kAfThreads)
+    af_stats_kernel(const float* __restrict__ g, const float* __restrict__ p,
+                    float* __restrict__ rowsum, float* __restrict__ colsum,
+                    AdafactorScalars* __restrict__ scal, int R, int C, float eps1) {
+  af_stats_tile<VEC>(g, p, rowsum, colsum, scal, R, C, eps1, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
 // EMA of the two second-moment vectors; one CTA per batch element. `row_is_normalized`: the
 // vector indexed by matrix rows is the one divided by its mean (T5X "v_row"); otherwise the
 // column-indexed vector is. row_div / col_div are the GLOBAL column / row counts (the means are
 // over the unsharded dims); the local sums were combined across ranks beforehand if needed.
-__global__ void __launch_bounds__(1024)
-    af_ema_kernel(float* __restrict__ v_rvec, float* __restrict__ v_cvec,
-                  const float* __restrict__ rowsum, const float* __restrict__ colsum,
-                  AdafactorScalars* __restrict__ scal, int R, int C, float row_div, float col_div,
-                  float decay, int row_is_normalized, int skip_nan) {
+__device__ __forceinline__ void af_ema(float* __restrict__ v_rvec, float* __restrict__ v_cvec,
+                                       const float* __restrict__ rowsum,
+                                       const float* __restrict__ colsum,
+                                       AdafactorScalars* __restrict__ scal, int R, int C,
+                                       float row_div, float col_div, float decay,
+                                       int row_is_normalized, int skip_nan, int b) {
   __shared__ float red[32];
-  const int b = blockIdx.x;
   v_rvec += static_cast<long long>(b) * R;
   v_cvec += static_cast<long long>(b) * C;
   rowsum += static_cast<long long>(b) * R;
@@ -175,14 +185,21 @@ __global__ void __launch_bounds__(1024)
   }
 }
 
+__global__ void __launch_bounds__(1024)
+    af_ema_kernel(float* __restrict__ v_rvec, float* __restrict__ v_cvec,
+                  const float* __restrict__ rowsum, const float* __restrict__ colsum,
+                  AdafactorScalars* __restrict__ scal, int R, int C, float row_div, float col_div,
+                  float decay, int row_is_normalized, int skip_nan) {
+  af_ema(v_rvec, v_cvec, rowsum, colsum, scal, R, C, row_div, col_div, decay, row_is_normalized,
+         skip_nan, blockIdx.x);
+}
+
 // Factor vectors from the updated moments: (v_row / mean(v_row))^-1/2 and v_col^-1/2.
 // norm_count = GLOBAL length of the normalised vector.
-__global__ void __launch_bounds__(1024)
-    af_finalize_kernel(const float* __restrict__ v_rvec, const float* __restrict__ v_cvec,
-                       float* __restrict__ rf, float* __restrict__ cf,
-                       const AdafactorScalars* __restrict__ scal, int R, int C, float norm_count,
-                       int row_is_normalized) {
-  const int b = blockIdx.x;
+__device__ __forceinline__ void af_finalize(const float* v_rvec, const float* v_cvec,
+                                            float* __restrict__ rf, float* __restrict__ cf,
+                                            const AdafactorScalars* scal, int R, int C,
+                                            float norm_count, int row_is_normalized, int b) {
   v_rvec += static_cast<long long>(b) * R;
   v_cvec += static_cast<long long>(b) * C;
   rf += static_cast<long long>(b) * R;
@@ -192,6 +209,14 @@ __global__ void __launch_bounds__(1024)
     rf[i] = row_is_normalized ? rsqrtf(v_rvec[i] / mean) : rsqrtf(v_rvec[i]);
   for (int i = threadIdx.x; i < C; i += blockDim.x)
     cf[i] = row_is_normalized ? rsqrtf(v_cvec[i]) : rsqrtf(v_cvec[i] / mean);
+}
+
+__global__ void __launch_bounds__(1024)
+    af_finalize_kernel(const float* __restrict__ v_rvec, const float* __restrict__ v_cvec,
+                       float* __restrict__ rf, float* __restrict__ cf,
+                       const AdafactorScalars* __restrict__ scal, int R, int C, float norm_count,
+                       int row_is_normalized) {
+  af_finalize(v_rvec, v_cvec, rf, cf, scal, R, C, norm_count, row_is_normalized, blockIdx.x);
 }
 
 __global__ void __launch_bounds__(kAfThreads)
@@ -222,13 +247,12 @@ __global__ void __launch_bounds__(kAfThreads)
 
 // FACTORED: u = g * rf[r] * cf[c].  !FACTORED: u = g * rsqrt(v) with v already updated.
 template <bool FACTORED>
-__global__ void __launch_bounds__(kAfThreads)
-    af_apply_kernel(float* __restrict__ p, const float* __restrict__ g, const float* __restrict__ rf,
-                    const float* __restrict__ cf, const float* __restrict__ v, float* __restrict__ m,
-                    __nv_bfloat16* __restrict__ p_bf16, long long ld_bf16, long long bf16_batch_stride,
-                    const AdafactorScalars* __restrict__ scal, int R, int C, float n_global,
-                    AfHyper h) {
-  const int b = blockIdx.y;
+__device__ __forceinline__ void af_apply_elements(
+    float* __restrict__ p, const float* __restrict__ g, const float* __restrict__ rf,
+    const float* __restrict__ cf, const float* __restrict__ v, float* __restrict__ m,
+    __nv_bfloat16* __restrict__ p_bf16, long long ld_bf16, long long bf16_batch_stride,
+    const AdafactorScalars* __restrict__ scal, int R, int C, float n_global, const AfHyper& h,
+    int block, int blocks, int b) {
   const long long n = static_cast<long long>(R) * C;
   const long long base = static_cast<long long>(b) * n;
   const float scale = af_update_scale(scal[b], n_global, h);
@@ -236,8 +260,8 @@ __global__ void __launch_bounds__(kAfThreads)
     rf += static_cast<long long>(b) * R;
     cf += static_cast<long long>(b) * C;
   }
-  for (long long i = blockIdx.x * static_cast<long long>(kAfThreads) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * kAfThreads) {
+  for (long long i = block * static_cast<long long>(kAfThreads) + threadIdx.x; i < n;
+       i += static_cast<long long>(blocks) * kAfThreads) {
     const int r = static_cast<int>(i / C), c = static_cast<int>(i - static_cast<long long>(r) * C);
     const float gv = g[base + i];
     const float u = FACTORED ? gv * rf[r] * cf[c] : gv * rsqrtf(v[base + i]);
@@ -257,18 +281,30 @@ __global__ void __launch_bounds__(kAfThreads)
   }
 }
 
-// Unfactored pass 1: v <- decay v + (1-decay)(g^2+eps1); accumulates sum u^2 and sum p^2.
+template <bool FACTORED>
 __global__ void __launch_bounds__(kAfThreads)
-    af_unfactored_stats_kernel(const float* __restrict__ g, const float* __restrict__ p,
-                               float* __restrict__ v, AdafactorScalars* __restrict__ scal,
-                               long long n, float decay, float eps1, int skip_nan) {
+    af_apply_kernel(float* __restrict__ p, const float* __restrict__ g, const float* __restrict__ rf,
+                    const float* __restrict__ cf, const float* __restrict__ v, float* __restrict__ m,
+                    __nv_bfloat16* __restrict__ p_bf16, long long ld_bf16, long long bf16_batch_stride,
+                    const AdafactorScalars* __restrict__ scal, int R, int C, float n_global,
+                    AfHyper h) {
+  af_apply_elements<FACTORED>(p, g, rf, cf, v, m, p_bf16, ld_bf16, bf16_batch_stride, scal, R, C,
+                              n_global, h, blockIdx.x, gridDim.x, blockIdx.y);
+}
+
+// Unfactored pass 1: v <- decay v + (1-decay)(g^2+eps1); accumulates sum u^2 and sum p^2.
+__device__ __forceinline__ void af_unfactored_stats(const float* __restrict__ g,
+                                                    const float* __restrict__ p,
+                                                    float* __restrict__ v,
+                                                    AdafactorScalars* __restrict__ scal,
+                                                    long long n, float decay, float eps1,
+                                                    int skip_nan, int block, int blocks, int b) {
   __shared__ float red[2][32];
-  const int b = blockIdx.y;
   const long long base = static_cast<long long>(b) * n;
   float usq = 0.f, psq = 0.f;
   const float mix = 1.f - decay;
-  for (long long i = blockIdx.x * static_cast<long long>(kAfThreads) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * kAfThreads) {
+  for (long long i = block * static_cast<long long>(kAfThreads) + threadIdx.x; i < n;
+       i += static_cast<long long>(blocks) * kAfThreads) {
     const float gv = g[base + i], pv = p[base + i], old = v[base + i];
     float nv = decay * old + mix * (gv * gv + eps1);
     if (skip_nan && isnan(nv)) nv = old;
@@ -295,6 +331,13 @@ __global__ void __launch_bounds__(kAfThreads)
   }
 }
 
+__global__ void __launch_bounds__(kAfThreads)
+    af_unfactored_stats_kernel(const float* __restrict__ g, const float* __restrict__ p,
+                               float* __restrict__ v, AdafactorScalars* __restrict__ scal,
+                               long long n, float decay, float eps1, int skip_nan) {
+  af_unfactored_stats(g, p, v, scal, n, decay, eps1, skip_nan, blockIdx.x, gridDim.x, blockIdx.y);
+}
+
 // Tiled forms of the two element-wise factored passes: a CTA covers kAfRowsPerCta rows x 1024
 // columns, a thread 4 adjacent columns of each row, so the row / column factors are indexed
 // without a division per element and loads are 16 bytes wide when C % 4 == 0.
@@ -302,17 +345,17 @@ constexpr int kAfRowsPerCta = 32;
 constexpr int kAfColsPerCta = kAfThreads * 4;
 
 template <bool VEC>
-__global__ void __launch_bounds__(kAfThreads)
-    af_usq_tiled_kernel(const float* __restrict__ g, const float* __restrict__ rf,
-                        const float* __restrict__ cf, AdafactorScalars* __restrict__ scal, int R,
-                        int C) {
+__device__ __forceinline__ void af_usq_tile(const float* __restrict__ g,
+                                            const float* __restrict__ rf,
+                                            const float* __restrict__ cf,
+                                            AdafactorScalars* __restrict__ scal, int R, int C,
+                                            int tile_x, int tile_y, int b) {
   __shared__ float red[kAfThreads / 32];
-  const int b = blockIdx.z;
   g += static_cast<long long>(b) * R * C;
   rf += static_cast<long long>(b) * R;
   cf += static_cast<long long>(b) * C;
-  const int r0 = blockIdx.y * kAfRowsPerCta;
-  const int col = blockIdx.x * kAfColsPerCta + threadIdx.x * 4;
+  const int r0 = tile_y * kAfRowsPerCta;
+  const int col = tile_x * kAfColsPerCta + threadIdx.x * 4;
   const int rows = min(kAfRowsPerCta, R - r0);
   float acc = 0.f;
   if (col < C) {
@@ -350,16 +393,21 @@ __global__ void __launch_bounds__(kAfThreads)
 
 template <bool VEC>
 __global__ void __launch_bounds__(kAfThreads)
-    af_apply_tiled_kernel(float* __restrict__ p, const float* __restrict__ g,
-                          const float* __restrict__ rf, const float* __restrict__ cf,
-                          float* __restrict__ m, __nv_bfloat16* __restrict__ p_bf16,
-                          long long ld_bf16, long long bf16_batch_stride,
-                          const AdafactorScalars* __restrict__ scal, int R, int C, float n_global,
-                          AfHyper h) {
-  const int b = blockIdx.z;
+    af_usq_tiled_kernel(const float* __restrict__ g, const float* __restrict__ rf,
+                        const float* __restrict__ cf, AdafactorScalars* __restrict__ scal, int R,
+                        int C) {
+  af_usq_tile<VEC>(g, rf, cf, scal, R, C, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+template <bool VEC>
+__device__ __forceinline__ void af_apply_tile(
+    float* __restrict__ p, const float* __restrict__ g, const float* __restrict__ rf,
+    const float* __restrict__ cf, float* __restrict__ m, __nv_bfloat16* __restrict__ p_bf16,
+    long long ld_bf16, long long bf16_batch_stride, const AdafactorScalars* __restrict__ scal, int R,
+    int C, float n_global, const AfHyper& h, int tile_x, int tile_y, int b) {
   const long long base = static_cast<long long>(b) * R * C;
-  const int r0 = blockIdx.y * kAfRowsPerCta;
-  const int col = blockIdx.x * kAfColsPerCta + threadIdx.x * 4;
+  const int r0 = tile_y * kAfRowsPerCta;
+  const int col = tile_x * kAfColsPerCta + threadIdx.x * 4;
   if (col >= C) return;
   const float scale = af_update_scale(scal[b], n_global, h);
   rf += static_cast<long long>(b) * R;
@@ -440,6 +488,122 @@ __global__ void __launch_bounds__(kAfThreads)
       }
     }
     }
+  }
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(kAfThreads)
+    af_apply_tiled_kernel(float* __restrict__ p, const float* __restrict__ g,
+                          const float* __restrict__ rf, const float* __restrict__ cf,
+                          float* __restrict__ m, __nv_bfloat16* __restrict__ p_bf16,
+                          long long ld_bf16, long long bf16_batch_stride,
+                          const AdafactorScalars* __restrict__ scal, int R, int C, float n_global,
+                          AfHyper h) {
+  af_apply_tile<VEC>(p, g, rf, cf, m, p_bf16, ld_bf16, bf16_batch_stride, scal, R, C, n_global, h,
+                     blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// ---------------------------------------------------------------------------------------
+// Many parameters per launch. The update of one parameter is a chain of five short kernels
+// and a fill; a model has dozens of parameters of a few megabytes and dozens of vectors, so
+// the chain's launches, not its bytes, set the time (T5.1.1 small, one layer pair: 140 launches
+// and 0.9 ms for 2 x 35 M parameters, 0.13 ms worth of traffic). Here a phase of the chain is one
+// launch over up to kAfGroupMax parameters, described in the kernel's parameters; a CTA finds
+// its parameter by its block number and runs the same tile as the kernels above.
+// ---------------------------------------------------------------------------------------
+constexpr int kAfGroupMax = 64;
+struct AfItem {
+  float* p;
+  const float* g;
+  float* v0;  // factored: second moments by matrix row; unfactored: the full second moment
+  float* v1;  // factored: second moments by matrix column
+  float* m;
+  __nv_bfloat16* out;
+  long long ld, bbs;
+  float *rowsum, *colsum, *rf, *cf;  // factored scratch
+  AdafactorScalars* scal;
+  float n;             // elements per batch element
+  int batch, R, C;
+  int factored, row_is_normalized, param_scale;
+  int vec;             // 16-byte accesses to p and g
+  int first[3];        // first block of phases stats, vectors, elements (usq and apply)
+  int blocks;          // unfactored: blocks per batch element
+};
+struct AfGroup {
+  AfItem item[kAfGroupMax];
+  int count;
+  AfHyper h;
+  float decay, eps1;
+};
+static_assert(sizeof(AfGroup) <= 32000, "kernel parameters");
+
+__device__ __forceinline__ int af_item_of(const AfGroup& grp, int phase, int block) {
+  int lo = 0, hi = grp.count - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (grp.item[mid].first[phase] <= block) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+__global__ void __launch_bounds__(kAfThreads) af_group_stats_kernel(const __grid_constant__ AfGroup grp) {
+  const AfItem& it = grp.item[af_item_of(grp, 0, blockIdx.x)];
+  const int k = blockIdx.x - it.first[0];
+  if (!it.factored) {
+    af_unfactored_stats(it.g, it.p, it.v0, it.scal, static_cast<long long>(it.R) * it.C, grp.decay,
+                        grp.eps1, grp.h.skip_nan, k % it.blocks, it.blocks, k / it.blocks);
+    return;
+  }
+  const int tx = (it.C + kAfTileC - 1) / kAfTileC, ty = (it.R + kAfTileR - 1) / kAfTileR;
+  const int b = k / (tx * ty), t = k - b * tx * ty;
+  if (it.vec)
+    af_stats_tile<true>(it.g, it.p, it.rowsum, it.colsum, it.scal, it.R, it.C, grp.eps1, t % tx,
+                        t / tx, b);
+  else
+    af_stats_tile<false>(it.g, it.p, it.rowsum, it.colsum, it.scal, it.R, it.C, grp.eps1, t % tx,
+                         t / tx, b);
+}
+
+// One CTA per factored parameter and batch element: moments, then the factor vectors.
+__global__ void __launch_bounds__(1024) af_group_vectors_kernel(const __grid_constant__ AfGroup grp) {
+  const AfItem& it = grp.item[af_item_of(grp, 1, blockIdx.x)];
+  const int b = blockIdx.x - it.first[1];
+  af_ema(it.v0, it.v1, it.rowsum, it.colsum, it.scal, it.R, it.C, static_cast<float>(it.C),
+         static_cast<float>(it.R), grp.decay, it.row_is_normalized, grp.h.skip_nan, b);
+  __syncthreads();  // the sum and the moments of this CTA, read back below
+  af_finalize(it.v0, it.v1, it.rf, it.cf, it.scal, it.R, it.C,
+              static_cast<float>(it.row_is_normalized ? it.R : it.C), it.row_is_normalized, b);
+}
+
+template <bool APPLY>
+__global__ void __launch_bounds__(kAfThreads) af_group_elements_kernel(const __grid_constant__ AfGroup grp) {
+  const AfItem& it = grp.item[af_item_of(grp, 2, blockIdx.x)];
+  const int k = blockIdx.x - it.first[2];
+  AfHyper h = grp.h;
+  h.multiply_by_parameter_scale = it.param_scale;
+  if (!it.factored) {
+    if (APPLY)
+      af_apply_elements<false>(it.p, it.g, nullptr, nullptr, it.v0, it.m, it.out, it.ld, it.bbs,
+                               it.scal, it.R, it.C, it.n, h, k % it.blocks, it.blocks,
+                               k / it.blocks);
+    return;
+  }
+  const int tx = (it.C + kAfColsPerCta - 1) / kAfColsPerCta;
+  const int ty = (it.R + kAfRowsPerCta - 1) / kAfRowsPerCta;
+  const int b = k / (tx * ty), t = k - b * tx * ty;
+  if (APPLY) {
+    if (it.vec)
+      af_apply_tile<true>(it.p, it.g, it.rf, it.cf, it.m, it.out, it.ld, it.bbs, it.scal, it.R,
+                          it.C, it.n, h, t % tx, t / tx, b);
+    else
+      af_apply_tile<false>(it.p, it.g, it.rf, it.cf, it.m, it.out, it.ld, it.bbs, it.scal, it.R,
+                           it.C, it.n, h, t % tx, t / tx, b);
+  } else {
+    if (it.vec)
+      af_usq_tile<true>(it.g, it.rf, it.cf, it.scal, it.R, it.C, t % tx, t / tx, b);
+    else
+      af_usq_tile<false>(it.g, it.rf, it.cf, it.scal, it.R, it.C, t % tx, t / tx, b);
   }
 }
 
@@ -664,6 +828,121 @@ T5X_API int t5x_adafactor_unfactored(void* p, const void* g, void* v, void* m, v
   return t5x_adafactor_unfactored_apply(p, g, v, m, p_bf16, ld_bf16, bf16_batch_stride, scratch,
                                         batch, R, C, n, lr, eps2, clip_threshold, weight_decay,
                                         beta1, max_param_scale, flags, stream);
+}
+
+// One parameter of t5x_adafactor_group (plain C layout; the Python binding packs it).
+struct T5xAdafactorItem {
+  void *p, *v0, *v1, *m, *out;  // v1 null: unfactored (v0 is the full second moment)
+  const void* g;
+  long long ld, bbs;            // row and batch stride of the bf16 copy `out` (may be null)
+  int batch, R, C, row_is_normalized, param_scale, pad;
+};
+
+// Scratch floats of one item, a multiple of four.
+static long long af_item_scratch(const T5xAdafactorItem& x) {
+  const long long n = x.v1 ? t5x_adafactor_scratch_floats(x.batch, x.R, x.C) : 4ll * x.batch;
+  return (n + 3) / 4 * 4;
+}
+
+T5X_API long long t5x_adafactor_group_scratch_floats(const void* items, int count) {
+  const T5xAdafactorItem* x = static_cast<const T5xAdafactorItem*>(items);
+  long long n = 0;
+  for (int i = 0; i < count; ++i) n += af_item_scratch(x[i]);
+  return n;
+}
+
+// Adafactor update of `count` fp32 parameters of one GPU, four launches for every kAfGroupMax of
+// them: the same arithmetic as t5x_adafactor_factored / _unfactored, whose flags these are (bit 0
+// is taken from each item instead). `scratch`: t5x_adafactor_group_scratch_floats values,
+// 16-byte aligned.
+T5X_API int t5x_adafactor_group(const void* items, int count, void* scratch, float lr, float decay,
+                                float eps1, float eps2, float clip_threshold, float weight_decay,
+                                float beta1, float max_param_scale, int flags, void* stream) {
+  if (count <= 0) return 0;
+  if (items == nullptr || scratch == nullptr)
+    return set_error("adafactor_group: items and scratch must not be null");
+  const T5xAdafactorItem* src = static_cast<const T5xAdafactorItem*>(items);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const long long total = t5x_adafactor_group_scratch_floats(items, count);
+  cudaError_t e = cudaMemsetAsync(scratch, 0, total * sizeof(float), st);
+  if (e != cudaSuccess) return set_error("adafactor_group: memset: %s", cudaGetErrorString(e));
+  float* next = static_cast<float*>(scratch);
+  AfGroup grp;
+  grp.h = af_hyper(lr, eps2, clip_threshold, weight_decay, beta1, max_param_scale, flags);
+  grp.decay = decay;
+  grp.eps1 = eps1;
+  for (int at = 0; at < count;) {
+    long long blocks[3] = {0, 0, 0};
+    bool factored = false;
+    grp.count = 0;
+    for (; at < count && grp.count < kAfGroupMax; ++at) {
+      const T5xAdafactorItem& x = src[at];
+      if (x.batch <= 0 || x.R <= 0 || x.C <= 0) continue;
+      if (int rc = af_validate("adafactor_group", x.p, x.g, x.v0, x.v1 ? x.v1 : x.v0, x.m, flags))
+        return rc;
+      AfItem& it = grp.item[grp.count];
+      it.p = static_cast<float*>(x.p);
+      it.g = static_cast<const float*>(x.g);
+      it.v0 = static_cast<float*>(x.v0);
+      it.v1 = static_cast<float*>(x.v1);
+      it.m = static_cast<float*>(x.m);
+      it.out = static_cast<__nv_bfloat16*>(x.out);
+      it.ld = x.ld;
+      it.bbs = x.bbs;
+      it.batch = x.batch;
+      it.R = x.R;
+      it.C = x.C;
+      it.factored = x.v1 != nullptr;
+      it.row_is_normalized = x.row_is_normalized;
+      it.param_scale = x.param_scale;
+      it.vec = af_stats_vec_ok(x.p, x.g, x.C);
+      it.n = static_cast<float>(static_cast<long long>(x.R) * x.C);
+      it.blocks = af_grid(static_cast<long long>(x.R) * x.C);
+      long long mine[3] = {0, 0, 0};
+      if (it.factored) {
+        const AfScratch a = af_split(next, x.batch, x.R, x.C);
+        it.rowsum = a.rowsum;
+        it.colsum = a.colsum;
+        it.rf = a.rf;
+        it.cf = a.cf;
+        it.scal = a.scal;
+        const dim3 tg = af_tiled_grid(x.batch, x.R, x.C);
+        mine[0] = 1ll * ((x.C + kAfTileC - 1) / kAfTileC) * ((x.R + kAfTileR - 1) / kAfTileR) * x.batch;
+        mine[1] = x.batch;
+        mine[2] = 1ll * tg.x * tg.y * tg.z;
+        factored = true;
+      } else {
+        it.rowsum = it.colsum = it.rf = it.cf = nullptr;
+        it.scal = reinterpret_cast<AdafactorScalars*>(next);
+        mine[0] = mine[2] = 1ll * it.blocks * x.batch;
+      }
+      next += af_item_scratch(x);
+      bool fits = true;
+      for (int k = 0; k < 3; ++k) fits = fits && blocks[k] + mine[k] <= 0x7fffffffll;
+      if (!fits) return set_error("adafactor_group: too many blocks");
+      for (int k = 0; k < 3; ++k) {
+        it.first[k] = static_cast<int>(blocks[k]);
+        blocks[k] += mine[k];
+      }
+      ++grp.count;
+    }
+    if (grp.count == 0) continue;
+    const unsigned nb[3] = {static_cast<unsigned>(blocks[0]), static_cast<unsigned>(blocks[1]),
+                            static_cast<unsigned>(blocks[2])};
+    af_group_stats_kernel<<<nb[0], kAfThreads, 0, st>>>(grp);
+    int launched = 1;
+    if (factored) {
+      af_group_vectors_kernel<<<nb[1], 1024, 0, st>>>(grp);
+      ++launched;
+      if (grp.h.use_clip) {
+        af_group_elements_kernel<false><<<nb[2], kAfThreads, 0, st>>>(grp);
+        ++launched;
+      }
+    }
+    af_group_elements_kernel<true><<<nb[2], kAfThreads, 0, st>>>(grp);
+    count_launches(launched + 1);
+  }
+  return af_check("adafactor_group");
 }
 
 // ---------------------------------------------------------------------------------------

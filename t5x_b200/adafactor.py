@@ -268,6 +268,49 @@ class Adafactor(OptimizerDef):
                            skip_rank=zinfo.push_skip_rank())
     return param, state
 
+  def apply_param_gradients(self, step, hyper_params, items, pre_reduced: bool = False) -> None:
+    """`apply_param_gradient` for a list of (param, state, grad, path). Parameters that live
+    whole on this GPU go through the grouped kernels, a few launches for all of them (four per
+    64 parameters; one by one each parameter is five launches and a fill); the others one by
+    one."""
+    hp = hyper_params
+    st = pstate.get()
+    # a subclass with an update of its own keeps it
+    own = type(self).apply_param_gradient is Adafactor.apply_param_gradient
+    groups = {}  # device -> [(layout, param, state, grad, scaled by the parameter's size)]
+    for param, state, grad, path in items:
+      layout = None
+      if own and getattr(param, "zero", None) is None and param.is_cuda and not (
+          getattr(param, "shard_dim", None) is not None and st.model_size > 1):
+        averaging_dims, factored_dims = self._resolve(self._global_shape(param), path)
+        layout = self._native_layout(param, state, grad, averaging_dims, factored_dims)
+      if layout is None or hp.learning_rate is None:
+        self.apply_param_gradient(step, hp, param, state, grad, path, pre_reduced=pre_reduced)
+        continue
+      mbps = hp.multiply_by_parameter_scale
+      if isinstance(mbps, HParamMap):
+        mbps = mbps[path]
+      groups.setdefault(param.device, []).append((layout, param, state, grad, bool(mbps)))
+    if not groups:
+      return
+    from t5x_b200.ops import native
+    lr = float(hp.learning_rate)
+    weight_decay_rate = hp.weight_decay_rate
+    if hp.weight_decay_rate_lr_exponent:
+      weight_decay_rate = (weight_decay_rate or 1.0) * lr ** hp.weight_decay_rate_lr_exponent
+    decay = self._decay_rate_pow(int(step) - hp.step_offset, exponent=hp.decay_rate)
+    for device, members in groups.items():
+      packed = native.AdafactorItems()
+      for (_, batch, R, C, row_norm, v0, v1, ld, bbs, _, _), param, state, grad, mbps in members:
+        packed.add(param, grad, v0, v1, state["m"] if hp.beta1 is not None else None,
+                   getattr(param, "bf16", None), ld, bbs, batch, R, C, row_norm, mbps)
+      native.adafactor_group_(
+          packed, _scratch(device, packed.scratch_floats()), lr=lr, decay=decay, eps1=hp.epsilon1,
+          eps2=hp.epsilon2, clip_threshold=hp.clipping_threshold or 1.0,
+          weight_decay=weight_decay_rate or 0.0, beta1=hp.beta1 or 0.0,
+          max_param_scale=hp.max_parameter_scale or 0.0,
+          flags=self._native_flags(False, weight_decay_rate))
+
   def _fused_sharded_ok(self, param, state, grad, averaging_dims, factored_dims) -> bool:
     """True when the NVLink-fused kernels cover this parameter: a factored [batch, R, C]
     fp32 matrix with C % 4 == 0 that is not also tensor-parallel sharded."""
@@ -376,95 +419,110 @@ class Adafactor(OptimizerDef):
         bf.copy_(p)
     return param, state
 
-  # Fused CUDA path for fp32 parameters laid out [batch..., rows, cols].
-  def _try_native(self, param, state, grad, path, lr, decay, mbps, weight_decay_rate,
-                  averaging_dims, factored_dims, zinfo=None) -> bool:
+  # How the kernels see a parameter: [batch, R, C], or None when they do not cover it.
+  def _native_layout(self, param, state, grad, averaging_dims, factored_dims):
+    """(batch dims, batch, R, C, row_is_normalized, v_rvec, v_cvec, ld_bf16, bf16 batch stride,
+    row dims, col dims); v_cvec is None and v_rvec the full second moment for an unfactored
+    parameter."""
     if not (param.is_cuda and param.dtype == torch.float32 and grad.dtype == torch.float32 and
             param.is_contiguous() and grad.is_contiguous()):
-      return False
-    hp = self.hyper_params
+      return None
+    if self.hyper_params.beta1 is not None and self.dtype_momentum != torch.float32:
+      return None
     nd = param.dim()
     batch_dims = tuple(i for i in range(nd) if i not in averaging_dims)
-    if batch_dims != tuple(range(len(batch_dims))):
-      return False  # batch dims must lead
     nb = len(batch_dims)
-    from t5x_b200.ops import native
-    st = pstate.get()
-    shard_dim = getattr(param, "shard_dim", None)
-    sharded = shard_dim is not None and st.model_size > 1
-    gshape = self._global_shape(param)
+    if batch_dims != tuple(range(nb)):
+      return None  # batch dims must lead
     batch = int(np.prod(param.shape[:nb])) if nb else 1
-    flags = 0
-    if mbps:
-      flags |= native.AF_PARAM_SCALE
-    if hp.clipping_threshold is not None:
-      flags |= native.AF_CLIP
-    if weight_decay_rate is not None:
-      flags |= native.AF_WD
-    if hp.beta1 is not None:
-      if self.dtype_momentum != torch.float32:
-        return False
-      flags |= native.AF_MOMENTUM
-    if hp.max_parameter_scale is not None:
-      flags |= native.AF_MAX_SCALE
-    if hp.skip_nan_updates:
-      flags |= native.AF_SKIP_NAN
-    common = dict(lr=lr, eps2=hp.epsilon2, clip_threshold=hp.clipping_threshold or 1.0,
-                  weight_decay=weight_decay_rate or 0.0, beta1=hp.beta1 or 0.0,
-                  max_param_scale=hp.max_parameter_scale or 0.0, flags=flags)
     bf = getattr(param, "bf16", None)
-    m = state["m"] if hp.beta1 is not None else None
-    n_global = int(np.prod(gshape[nb:])) if nd > nb else 1
-
+    ld_bf16, bbs = (0, 0)
     if factored_dims is None:
       rows = 1 if nd - nb <= 1 else int(np.prod(param.shape[nb:-1]))
       cols = int(param.shape[-1]) if nd > nb else 1
-      n_local = rows * cols
-      ld_bf16, bbs = (0, 0)
       if bf is not None:
         if not bf.is_contiguous():
-          return False
-        ld_bf16, bbs = cols, n_local
-      scratch = _scratch(param.device, 4 * batch)
-      native.adafactor_unfactored_stats_(param, grad, state["v"], scratch, batch, n_local, decay,
-                                         hp.epsilon1, bool(hp.skip_nan_updates))
-      if sharded:
-        dist.all_reduce(scratch[:4 * batch], group=st.model_group)
-      native.adafactor_unfactored_apply_(param, grad, state["v"], m, bf, scratch, batch, rows,
-                                         cols, n_global, ld_bf16=ld_bf16, bf16_batch_stride=bbs,
-                                         **common)
-      return True
-
+          return None
+        ld_bf16, bbs = cols, rows * cols
+      return nb, batch, rows, cols, False, state["v"], None, ld_bf16, bbs, (), ()
     d1, d0 = factored_dims  # v_row reduces d0; v_col reduces d1
     rest = tuple(range(nb, nd))
     # The non-batch dims must split into a leading group and a trailing group that are exactly
     # (d0, d1) in one of the two orders, so the tensor is a [batch, R, C] matrix.
-    if tuple(sorted(d0 + d1)) != rest:
-      return False
     if tuple(d1) + tuple(d0) == rest:
       row_dims, col_dims, row_is_normalized = d1, d0, True    # v_row indexed by rows (= d1)
     elif tuple(d0) + tuple(d1) == rest:
       row_dims, col_dims, row_is_normalized = d0, d1, False   # v_row indexed by cols (= d1)
     else:
-      return False
+      return None
     R = int(np.prod([param.shape[d] for d in row_dims]))
     C = int(np.prod([param.shape[d] for d in col_dims]))
-    gR = int(np.prod([gshape[d] for d in row_dims]))
-    gC = int(np.prod([gshape[d] for d in col_dims]))
     # state vectors: the one indexed by matrix rows has the column dims removed.
     v_rvec = state["v_row"] if row_is_normalized else state["v_col"]
     v_cvec = state["v_col"] if row_is_normalized else state["v_row"]
-    ld_bf16, bbs = (0, 0)
     if bf is not None:
       if bf.dim() != param.dim() or bf.stride(-1) != 1:
-        return False
+        return None
       if len(col_dims) != 1 or (len(row_dims) != 1) or nb > 1:
         if not bf.is_contiguous():
-          return False
+          return None
         ld_bf16, bbs = C, R * C
       else:
         ld_bf16 = bf.stride(-2)
         bbs = bf.stride(0) if nb == 1 else 0
+    return nb, batch, R, C, row_is_normalized, v_rvec, v_cvec, ld_bf16, bbs, row_dims, col_dims
+
+  def _native_flags(self, mbps, weight_decay_rate) -> int:
+    from t5x_b200.ops import native
+    hp = self.hyper_params
+    flags = native.AF_PARAM_SCALE if mbps else 0
+    if hp.clipping_threshold is not None:
+      flags |= native.AF_CLIP
+    if weight_decay_rate is not None:
+      flags |= native.AF_WD
+    if hp.beta1 is not None:
+      flags |= native.AF_MOMENTUM
+    if hp.max_parameter_scale is not None:
+      flags |= native.AF_MAX_SCALE
+    if hp.skip_nan_updates:
+      flags |= native.AF_SKIP_NAN
+    return flags
+
+  # Fused CUDA path for fp32 parameters laid out [batch..., rows, cols].
+  def _try_native(self, param, state, grad, path, lr, decay, mbps, weight_decay_rate,
+                  averaging_dims, factored_dims, zinfo=None) -> bool:
+    layout = self._native_layout(param, state, grad, averaging_dims, factored_dims)
+    if layout is None:
+      return False
+    nb, batch, R, C, row_is_normalized, v_rvec, v_cvec, ld_bf16, bbs, row_dims, col_dims = layout
+    hp = self.hyper_params
+    nd = param.dim()
+    from t5x_b200.ops import native
+    st = pstate.get()
+    shard_dim = getattr(param, "shard_dim", None)
+    sharded = shard_dim is not None and st.model_size > 1
+    gshape = self._global_shape(param)
+    common = dict(lr=lr, eps2=hp.epsilon2, clip_threshold=hp.clipping_threshold or 1.0,
+                  weight_decay=weight_decay_rate or 0.0, beta1=hp.beta1 or 0.0,
+                  max_param_scale=hp.max_parameter_scale or 0.0,
+                  flags=self._native_flags(mbps, weight_decay_rate))
+    bf = getattr(param, "bf16", None)
+    m = state["m"] if hp.beta1 is not None else None
+    n_global = int(np.prod(gshape[nb:])) if nd > nb else 1
+
+    if v_cvec is None:
+      scratch = _scratch(param.device, 4 * batch)
+      native.adafactor_unfactored_stats_(param, grad, v_rvec, scratch, batch, R * C, decay,
+                                         hp.epsilon1, bool(hp.skip_nan_updates))
+      if sharded:
+        dist.all_reduce(scratch[:4 * batch], group=st.model_group)
+      native.adafactor_unfactored_apply_(param, grad, v_rvec, m, bf, scratch, batch, R, C,
+                                         n_global, ld_bf16=ld_bf16, bf16_batch_stride=bbs,
+                                         **common)
+      return True
+
+    gR = int(np.prod([gshape[d] for d in row_dims]))
+    gC = int(np.prod([gshape[d] for d in col_dims]))
     scratch = _scratch(param.device, native.adafactor_scratch_floats(batch, R, C))
     if zinfo is not None:
       from t5x_b200.ops import comm
@@ -550,14 +608,15 @@ class Adafactor(OptimizerDef):
           flat_g[k].mul_(scale.to(flat_g[k].dtype))
       from t5x_b200.parallel import zero
       done = zero.done_this_step()
+      todo = []
       for k, p in flat_p.items():
         zinfo = getattr(p, "zero", None)
         if zinfo is not None and not zinfo.mine:
           continue  # its owner updates it and pushes the new bf16 weights here
         if k in done:
           continue  # already updated while the backward pass was running
-        self.apply_param_gradient(step, hyper_params, p, flat_s[k], flat_g[k], k,
-                                  pre_reduced=pre_reduced)
+        todo.append((p, flat_s[k], flat_g[k], k))
+      self.apply_param_gradients(step, hyper_params, todo, pre_reduced=pre_reduced)
     finally:
       self.hyper_params = saved_hp
     return params, OptimizerState(step + 1, state.param_states)

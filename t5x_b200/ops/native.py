@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 import threading
 from typing import Optional
 
@@ -111,6 +112,8 @@ def _declare_optional(l):
   for name, argtypes in _OPTIONAL_SIGNATURES.items():
     if hasattr(l, name):
       getattr(l, name).argtypes = argtypes
+  if hasattr(l, "t5x_adafactor_group_scratch_floats"):
+    l.t5x_adafactor_group_scratch_floats.restype = c_ll
 
 
 _OPTIONAL_SIGNATURES: dict = {}
@@ -740,6 +743,48 @@ def adafactor_unfactored_apply_(p, g, v, m, p_bf16, scratch, batch, rows, cols, 
       p.data_ptr(), g.data_ptr(), v.data_ptr(), ptr(m), ptr(p_bf16), ld_bf16, bf16_batch_stride,
       scratch.data_ptr(), batch, rows, cols, n_global, lr, eps2, clip_threshold, weight_decay,
       beta1, max_param_scale, flags, stream_ptr()), "adafactor_unfactored_apply")
+
+
+register_signature("t5x_adafactor_group_scratch_floats", [c_void_p, c_int])
+register_signature("t5x_adafactor_group", [c_void_p, c_int, c_void_p] + [c_float] * 8 +
+                   [c_int, c_void_p])
+
+
+class AdafactorItems:
+  """The parameters of one `adafactor_group_` call in the library's item layout. Keeps no
+  reference to the tensors: the caller holds them until the call has been issued."""
+  _ITEM = struct.Struct("=6Q2q6i")
+
+  def __init__(self):
+    self._packed, self._scratch, self.count = [], 0, 0
+
+  def add(self, p, g, v0, v1, m, out, ld: int, bbs: int, batch: int, rows: int, cols: int,
+          row_is_normalized: bool, param_scale: bool) -> None:
+    """`v1` None: unfactored, `v0` is the full second moment."""
+    for t in (p, g, v0, v1, m):
+      assert t is None or (t.dtype == torch.float32 and t.is_contiguous())
+    assert out is None or out.dtype == torch.bfloat16
+    self._packed.append(self._ITEM.pack(p.data_ptr(), v0.data_ptr(), ptr(v1), ptr(m), ptr(out),
+                                        g.data_ptr(), ld, bbs, batch, rows, cols,
+                                        int(row_is_normalized), int(param_scale), 0))
+    self._scratch += -(-(4 * batch + (2 * batch * (rows + cols) if v1 is not None else 0)) // 4) * 4
+    self.count += 1
+
+  def scratch_floats(self) -> int:
+    return self._scratch
+
+  def buffer(self):
+    return ctypes.create_string_buffer(b"".join(self._packed), self._ITEM.size * self.count)
+
+
+def adafactor_group_(items: AdafactorItems, scratch: torch.Tensor, *, lr, decay, eps1, eps2,
+                     clip_threshold, weight_decay, beta1, max_param_scale, flags) -> None:
+  """One Adafactor step of every item (csrc/adafactor.cu, `t5x_adafactor_group`)."""
+  buf = items.buffer()
+  assert scratch.dtype == torch.float32 and scratch.numel() >= items.scratch_floats()
+  _check(lib().t5x_adafactor_group(ctypes.addressof(buf), items.count, scratch.data_ptr(), lr, decay,
+                                   eps1, eps2, clip_threshold, weight_decay, beta1,
+                                   max_param_scale, flags, stream_ptr()), "adafactor_group")
 
 
 # ----------------------------------------------------------------------------

@@ -539,9 +539,9 @@ class LocalUpdateOverlap:
       self._opt_def.hyper_params = hp
       try:
         with torch.no_grad():
-          for k in names:
-            p = self.params[k]
-            self._opt_def.apply_param_gradient(step, hp, p, self._state_of(k), p.main_grad, k)
+          self._opt_def.apply_param_gradients(
+              step, hp, [(self.params[k], self._state_of(k), self.params[k].main_grad, k)
+                         for k in names])
       finally:
         self._opt_def.hyper_params = saved
     self.done_this_step.update(names)
