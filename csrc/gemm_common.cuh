@@ -46,6 +46,7 @@ struct GemmParams {
   float alpha;
   int tiles_m, tiles_n;
   int mt_rot;  // the row-tile walk starts at this tile (tensor-parallel kernels); 0 otherwise
+  int split_k;     // CTA pairs: pieces that the tiles of the last wave are cut into (see GemmWork)
   int b_constant;  // B is not written by any kernel in flight: it may be loaded before chain_wait()
   // Optional phase trace (t5x_gemm_set_trace): 8 timestamps per CTA for its first tile: entry,
   // set-up done, first loads issued, first operands landed, last MMA issued, accumulator
@@ -294,13 +295,51 @@ __device__ __forceinline__ void gemm_tile_coords(const GemmParams& p, int tile, 
   }
 }
 
+// The work of a CTA pair, in order: every num_units-th tile, whole, except that with split_k > 1
+// the tiles of the last wave, which would leave most of the chip idle (160 tiles on 74 pairs: 2.16
+// waves of work in the time of 3), are cut into split_k pieces along K and dealt out piece by
+// piece; the pieces of a tile are added to fp32 memory with atomics. Pieces of the same k range
+// run at the same time, so they share operands in L2. (Equal shares of all k blocks laid end to
+// end balance better, but every pair is then at another k: 2048 x 2048 x 32768 went from 193 to
+// 265 us on operand traffic.)
+struct GemmWork {
+  int at, step, whole, total, tail, splits, num_kb;
+  __device__ GemmWork(const GemmParams& p, int unit, int num_units, int total_tiles, int num_kb_)
+      : at(unit), step(num_units), whole(total_tiles), total(total_tiles), tail(0), splits(1),
+        num_kb(num_kb_) {
+    if (p.split_k > 1) {
+      tail = total_tiles % num_units;
+      whole = total_tiles - tail;
+      splits = p.split_k;
+      total = whole + tail * splits;
+    }
+  }
+  // Next piece of work: k blocks [kb0, kb1) of `tile`; false when there is none.
+  __device__ __forceinline__ bool next(int& tile, int& kb0, int& kb1) {
+    if (at >= total) return false;
+    if (at < whole) {
+      tile = at;
+      kb0 = 0;
+      kb1 = num_kb;
+    } else {
+      const int piece = at - whole, s = piece / tail;
+      tile = whole + piece - s * tail;
+      kb0 = static_cast<int>(static_cast<long long>(num_kb) * s / splits);
+      kb1 = static_cast<int>(static_cast<long long>(num_kb) * (s + 1) / splits);
+    }
+    at += step;
+    return true;
+  }
+};
+
 // Epilogue of one 128-row accumulator tile held in TMEM columns [t_cols, t_cols + BN): the
 // calling warp owns lane quarter q (rows m0 + 32q .. +31) and part `part` of PARTS of the tile's
 // columns, `c_vec_ok` says whether 16-byte stores to C are legal.
 template <int BN, int EPI, int PARTS>
 __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t t_row, int m0,
                                                    int n0, int b, int q, int part, int lane,
-                                                   bool c_vec_ok, float* stage = nullptr) {
+                                                   bool c_vec_ok, int accumulate,
+                                                   float* stage = nullptr) {
   const int row = m0 + q * 32 + lane;
   const bool row_ok = row < p.M;
   const int rows_valid = p.M - (m0 + q * 32);  // of this warp's 32 rows (may exceed 32 or be <= 0)
@@ -358,6 +397,7 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
       }
     }
   } else {
+    const bool b_step_ok = p.c_batch_stride % 8 == 0;
 #pragma unroll 1
     for (int c = part * (BN / 32 / PARTS); c < (part + 1) * (BN / 32 / PARTS); ++c) {
       const int col = n0 + c * 32;
@@ -368,7 +408,8 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
       // whole 32-column blocks go out through the staging buffer (warp-uniform condition)
       const bool staged = stage != nullptr && n_valid >= 32 && rows_valid > 0 &&
                           (p.out_fp32 ? (p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0)
-                                      : (c_vec_ok && p.accumulate == 0));
+                                      : (c_vec_ok && (accumulate == 0 ||
+                                                       (EPI != kEpiResidual && b_step_ok))));
       if (staged) {
         const bool r_vec_ok = EPI == kEpiResidual && p.ldr % 8 == 0 &&
                               p.r_batch_stride % 8 == 0 &&
@@ -377,10 +418,19 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
           staged_load_bf16(stage, p.R + b * p.r_batch_stride +
                                       static_cast<long long>(m0 + q * 32) * p.ldr + col,
                            p.ldr, rows_valid, lane);
+        const long long first = b * p.c_batch_stride +
+                                static_cast<long long>(m0 + q * 32) * p.ldc + col;
+        // bf16 C += : what is there comes in the same way as a residual (65536 x 768 x 768
+        // 118 us with 16-byte reads of 32 rows, 94 so)
+        const bool add_c = EPI != kEpiResidual && accumulate != 0 && !p.out_fp32;
+        if (add_c)
+          staged_load_bf16(stage, reinterpret_cast<const __nv_bfloat16*>(p.C) + first, p.ldc,
+                           rows_valid, lane);
         tmem_ld_wait();
         float v[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
+        if (add_c) staged_add_row(stage, v, lane);
         if (EPI == kEpiResidual) {
           if (r_vec_ok) {
             staged_add_row(stage, v, lane);
@@ -392,13 +442,11 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
             for (int i = 0; i < 32; ++i) v[i] += rr[i];
           }
         }
-        const long long first = b * p.c_batch_stride +
-                                static_cast<long long>(m0 + q * 32) * p.ldc + col;
         if (p.out_fp32) {
           float* dst = reinterpret_cast<float*>(p.C) + first;
-          if (p.accumulate == 2)
+          if (accumulate == 2)
             staged_store_f32<2>(stage, v, dst, p.ldc, rows_valid, lane);
-          else if (p.accumulate == 1)
+          else if (accumulate == 1)
             staged_store_f32<1>(stage, v, dst, p.ldc, rows_valid, lane);
           else
             staged_store_f32<0>(stage, v, dst, p.ldc, rows_valid, lane);
@@ -428,11 +476,11 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               float4 o = make_float4(v[i * 4], v[i * 4 + 1], v[i * 4 + 2], v[i * 4 + 3]);
-              if (p.accumulate == 2) {  // several CTAs (split K) add into the same tile
+              if (accumulate == 2) {  // several CTAs (split K) add into the same tile
                 atomicAdd(reinterpret_cast<float4*>(out) + i, o);
                 continue;
               }
-              if (p.accumulate) {
+              if (accumulate) {
                 float4 old = reinterpret_cast<float4*>(out)[i];
                 o.x += old.x;
                 o.y += old.y;
@@ -445,16 +493,16 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
               if (i >= n_valid) break;
-              if (p.accumulate == 2)
+              if (accumulate == 2)
                 atomicAdd(out + i, v[i]);
               else
-                out[i] = p.accumulate ? out[i] + v[i] : v[i];
+                out[i] = accumulate ? out[i] + v[i] : v[i];
             }
           }
         } else {
           __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + b * p.c_batch_stride +
                                static_cast<long long>(row) * p.ldc + col;
-          if (p.accumulate) {
+          if (accumulate) {
             float old[32];
             load_row_bf16(out, old, n_valid, c_vec_ok);
 #pragma unroll

@@ -166,8 +166,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
       bool ok = true;
       // B is constant (weights that no kernel in flight writes): the B halves of the first
       // stages are requested before the wait for the preceding kernel, the A halves after it.
+      GemmWork work(p, pair, num_pairs, total_tiles, num_kb);
       int preloaded = 0;
-      if (MODE == kTpNone && p.b_constant && pair < total_tiles) {
+      if (MODE == kTpNone && p.b_constant && p.split_k <= 1 && pair < total_tiles) {
         int b, mt, nt;
         gemm_tile_coords(p, pair, tiles_per_batch, b, mt, nt);
         preloaded = min(kStages, num_kb);
@@ -183,7 +184,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
       } else {
         chain_wait();
       }
-      for (int tile = pair; tile < total_tiles && ok; tile += num_pairs) {
+      for (int tile, kb0, kb1; ok && work.next(tile, kb0, kb1);) {
         int b, mt, nt;
         gemm_tile_coords(p, tile, tiles_per_batch, b, mt, nt);
         const int m0 = mt * (2 * kBM) + static_cast<int>(cta) * kBM;
@@ -224,7 +225,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
           if (!ok) break;
           fence_proxy_async_all();  // the bulk stores that wrote A, before this TMA reads it
         }
-        for (int kb = preloaded; kb < num_kb; ++kb) {
+        for (int kb = kb0 + preloaded; kb < kb1; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) {
             report_status(p.status, kStatusTimeoutProducer, kKernelIdGemmPair, tile, kb);
             *abort_flag = 1;
@@ -255,7 +256,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
       uint32_t phase = 0;
       int local = 0;
       bool ok = true;
-      for (int tile = pair; tile < total_tiles && ok; tile += num_pairs, ++local) {
+      GemmWork work(p, pair, num_pairs, total_tiles, num_kb);
+      for (int tile, kb0, kb1; ok && work.next(tile, kb0, kb1); ++local) {
         const int acc = local & 1;
         const uint32_t acc_phase = (local >> 1) & 1;
         if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag)) {
@@ -266,7 +268,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&full[stage], phase, abort_flag)) {
             report_status(p.status, kStatusTimeoutMma, kKernelIdGemmPair, tile, kb);
             *abort_flag = 1;
@@ -280,7 +282,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
           for (int s = 0; s < kBK / 16; ++s) {
             const uint64_t ad = make_smem_desc_sw128(a_addr + s * a_kstep, a_lbo, 1024);
             const uint64_t bd = make_smem_desc_sw128(b_addr + s * b_kstep, b_lbo, 1024);
-            umma_bf16_pair(d_tmem, ad, bd, idesc, (kb | s) != 0 ? 1u : 0u);
+            umma_bf16_pair(d_tmem, ad, bd, idesc, (kb > kb0 || s != 0) ? 1u : 0u);
           }
           umma_commit_pair(&empty[stage], 0x3);
           if (++stage == kStages) {
@@ -397,7 +399,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
     chain_wait();  // the epilogue reads residuals and writes C
     const bool c_vec_ok = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
     const uint32_t drained = mapa_shared(smem_u32(&tmem_empty[0]), 0);
-    for (int tile = pair; tile < total_tiles && ok; tile += num_pairs, ++local) {
+    GemmWork work(p, pair, num_pairs, total_tiles, num_kb);
+    for (int tile, kb0, kb1; ok && work.next(tile, kb0, kb1); ++local) {
       const int acc = local & 1;
       const uint32_t acc_phase = (local >> 1) & 1;
       int b, mt, nt;
@@ -424,6 +427,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
       else
         gemm_epilogue_tile<BN, EPI, pair_epi_warps<MODE>() / 4>(
             p, t_row, m0, n0, b, q, part, lane, c_vec_ok,
+            kb1 - kb0 == num_kb ? p.accumulate : 2,  // a piece of a tile: atomic adds
             MODE == kTpNone
                 ? reinterpret_cast<float*>(staging + (warp - 2) * kEpiStageBytesPerWarp)
                 : nullptr);
@@ -484,7 +488,7 @@ static int launch_pair(const CUtensorMap* tA, const CUtensorMap* tB, const CUten
   const int total = p.tiles_m * p.tiles_n * p.batch;
   int pairs = num_sms() / 2;
   if (max_ctas > 0) pairs = std::min(pairs, std::max(1, max_ctas / 2));
-  pairs = std::max(1, std::min(pairs, total));
+  pairs = std::max(1, p.split_k > 1 ? pairs : std::min(pairs, total));
   cudaError_t e;
   if (MODE == kTpNone) {
     p.b_constant = chained_launches_constant_b() ? 1 : 0;

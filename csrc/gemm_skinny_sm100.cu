@@ -349,9 +349,9 @@ __global__ void __launch_bounds__(kSkThreads, 1)
     float* stage = staging + (warp - 2) * (kEpiStageBytesPerWarp / 4);
     const bool c_vec16 = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
     if (p.R != nullptr)
-      gemm_epilogue_tile<kSkBN, kEpiResidual, 1>(gp, t_row, m0, n0, 0, q, 0, lane, c_vec16, stage);
+      gemm_epilogue_tile<kSkBN, kEpiResidual, 1>(gp, t_row, m0, n0, 0, q, 0, lane, c_vec16, 0, stage);
     else
-      gemm_epilogue_tile<kSkBN, kEpiPlain, 1>(gp, t_row, m0, n0, 0, q, 0, lane, c_vec16, stage);
+      gemm_epilogue_tile<kSkBN, kEpiPlain, 1>(gp, t_row, m0, n0, 0, q, 0, lane, c_vec16, 0, stage);
   }
 
   // Teardown: loads still in flight after an abort get a bounded time to land.

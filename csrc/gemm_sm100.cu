@@ -262,7 +262,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       else if (EPI == kEpiCeGrad)
         gemm_epilogue_ce_grad<BN, 2>(p, t_row, m0, n0, q, part, lane, c_vec_ok, stage_buf);
       else
-        gemm_epilogue_tile<BN, EPI, 2>(p, t_row, m0, n0, b, q, part, lane, c_vec_ok, stage_buf);
+        gemm_epilogue_tile<BN, EPI, 2>(p, t_row, m0, n0, b, q, part, lane, c_vec_ok, p.accumulate,
+                                       stage_buf);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[acc]);
@@ -418,6 +419,7 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
   p.status = device_status_buffer();
   p.tiles_m = (M + kBM - 1) / kBM;
   p.mt_rot = 0;
+  p.split_k = 1;
   p.b_constant = 0;
   p.trace = nullptr;
   p.ce_targets = nullptr;
@@ -496,6 +498,40 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
       return launch_gemm_pair(kEpiGatedGelu, tA, tB, tB2, p, max_ctas, st);
     }
     return launch_gemm<256, kEpiGatedGelu>(tA, tB, tB2, p, max_ctas, st);
+  }
+  // A weight gradient (fp32 output, long K) whose tiles leave the last wave of pairs mostly empty:
+  // the tiles of that wave are cut along K. That costs a fill of C (430 / K of the product's time
+  // at the measured copy and GEMM rates) and atomic adds, so it has to save more than both.
+  // (us, whole tiles / cut: 768 x 768 x 12216 75 / 31, 768 x 3072 x 12216 80 / 56,
+  // 1472 x 3584 x 16384 189 / 132, 1024 x 16384 x 8192 240 / 217, 2048 x 5120 x 32768 705 / 519.)
+  if (pair_mode != 0 && epilogue == kEpiPlain && out_fp32 && accumulate != 2 && M >= 2 * kBM &&
+      N >= 256 && max_ctas <= 0 && ldc == N &&
+      (batch == 1 || c_batch_stride == static_cast<long long>(M) * N)) {
+    const int tn = (N + 255) / 256, pairs = sms / 2;
+    const long long tiles = 1ll * pair_tiles_m * tn * batch;
+    const int kb = (K + kBK - 1) / kBK;
+    const int tail = static_cast<int>(tiles % pairs);
+    double best = 1.0;  // time of the last wave, in waves
+    int splits = 1;
+    for (int s = 2; tail > 0 && s <= 16 && kb / s >= 8; ++s) {
+      const double t = static_cast<double>((1ll * tail * s + pairs - 1) / pairs) / s;
+      if (t < best - 0.02) {
+        best = t;
+        splits = s;
+      }
+    }
+    const double waves = static_cast<double>(tiles / pairs);
+    const double saved = (1.0 - best) / (waves + 1.0);
+    if (splits > 1 && saved > 0.08 + 430.0 / K) {
+      if (!accumulate) {
+        cudaError_t e = cudaMemsetAsync(C, 0, sizeof(float) * static_cast<size_t>(M) * N * batch, st);
+        if (e != cudaSuccess) return set_error("gemm: memset: %s", cudaGetErrorString(e));
+      }
+      p.split_k = splits;
+      p.tiles_m = pair_tiles_m;
+      p.tiles_n = tn;
+      return launch_gemm_pair(epilogue, tA, tB, tB, p, max_ctas, st);
+    }
   }
   // Tile width: 256 unless N is small or 128-wide tiles fill the SMs markedly better.
   const double e128 = waves_eff(1ll * p.tiles_m * ((N + 127) / 128) * batch, sms);

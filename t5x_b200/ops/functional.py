@@ -40,7 +40,9 @@ def _accumulate_wgrad(weight: torch.Tensor, a_t: torch.Tensor, b: torch.Tensor):
   if mg is not None:
     first = not getattr(weight, "grad_ready", False)
     out = mg.view(a_t.shape[0], b.shape[1])
-    splits = native.wgrad_splits(a_t.shape[0], b.shape[1], a_t.shape[1])
+    # (from 256 x 256 outputs on `gemm` itself cuts the tiles of the last wave along K)
+    narrow = a_t.shape[0] < 256 or b.shape[1] < 256
+    splits = native.wgrad_splits(a_t.shape[0], b.shape[1], a_t.shape[1]) if narrow else 1
     if splits > 1 and out.is_contiguous():
       native.gemm_splitk_accumulate(a_t, b, out, splits, accumulate=not first)
     else:

@@ -72,3 +72,32 @@ def test_cross_entropy(M, N, K, pair):
   finally:
     native.gemm_set_pair_mode(1)
   native.check_status()
+
+
+@pytest.mark.parametrize("batch,M,N,K", [(1, 768, 768, 4264), (1, 1472, 384, 8200),
+                                         (1, 256, 256, 40000), (3, 256, 520, 13000),
+                                         (1, 704, 304, 6000), (1, 2048, 2600, 8000)])
+@pytest.mark.parametrize("ta", [0, 1])
+def test_weight_gradient_with_a_split_last_wave(batch, M, N, K, ta):
+  """fp32 outputs whose last wave of tiles is cut along K, the pieces added atomically (also with
+  whole tiles before them, batches, and K off the block size). The tensor core
+  adds 16 products at a time and truncates: at most one unit in the last place of an accumulator
+  of up to 5 sqrt(K) per step, K / 16 steps."""
+  from t5x_b200.ops import native
+  g = torch.Generator(device="cuda").manual_seed(K)
+  rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+  a = rnd(batch, K, M).transpose(1, 2) if ta else rnd(batch, M, K)
+  b = rnd(batch, K, N)
+  if batch == 1:
+    a, b = a[0], b[0]
+  want = a.double() @ b.double()
+  out = torch.full(want.shape, 3.0, device="cuda")
+  native.gemm(a, b, out=out)
+  tol = K / 16 * 2 ** -23 * 5 * K ** 0.5
+  assert float((out - want).abs().max()) < tol
+  native.gemm(a, b, out=out, accumulate=True)
+  assert float((out - 2 * want).abs().max()) < 2 * tol
+  wide = torch.zeros(*want.shape[:-1], N + 8, device="cuda")  # rows apart: whole tiles
+  native.gemm(a, b, out=wide[..., :N])
+  assert float((wide[..., :N] - want).abs().max()) < tol and not bool(wide[..., N:].any())
+  native.check_status()
