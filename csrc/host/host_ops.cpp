@@ -1,0 +1,368 @@
+// Host side of the T5 block's ops, from tensors to kernel launches.
+//
+// What bounds it: a training step of a small model, and a forward pass of one sentence, are
+// limited by the host: through ctypes a GEMM took some 20 us from the Python call to the launch
+// (28 converted arguments, a dozen tensor attributes, the current stream, an output allocation)
+// while the kernel runs for 4 to 8 us. (T5.1.1 small with 8 + 8 layers, one sentence scored:
+// 9.7 ms through ctypes, 3.8 ms so, of which the device works 1.3.) These functions do the same
+// from C++ for the plain case, contiguous activations and row-major bf16 weights, one call per op
+// and direction. They return None for anything else, before doing anything; the Python wrappers
+// then take their general path, which handles or rejects the call.
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/extension.h>
+
+#include <optional>
+#include <string>
+#include <tuple>
+#include <vector>
+
+extern "C" {
+const char* t5x_last_error();
+int t5x_gemm_bf16(const void* A, const void* B, const void* B2, void* C, int M, int N, int K,
+                  int batch, long long lda, long long ldb, long long ldc, long long a_batch_stride,
+                  long long b_batch_stride, long long c_batch_stride, int a_mn_major, int b_mn_major,
+                  int out_fp32, int accumulate, int epilogue, const void* R, long long ldr,
+                  long long r_batch_stride, void* H0, void* H1, long long ldh, float alpha,
+                  int max_ctas, void* stream);
+int t5x_rmsnorm_fwd(const void* x, const void* scale, void* y, void* rstd, int rows, int d, float eps,
+                    void* stream);
+int t5x_rmsnorm_bwd(const void* dy, const void* x, const void* scale, const void* rstd,
+                    const void* dres, void* dx, void* dscale, int rows, int d, void* stream);
+int t5x_attention_fwd(const void* q, const void* k, const void* v, void* o, void* lse, int B, int H,
+                      int Lq, int Lk, long long q_sb, long long q_sl, long long q_sh, long long k_sb,
+                      long long k_sl, long long k_sh, long long v_sb, long long v_sl, long long v_sh,
+                      long long o_sb, long long o_sl, long long o_sh, const void* rel_bias,
+                      const void* rel_bucket, int num_buckets, int nrel, int rel_off,
+                      const void* key_mask, const void* q_seg, const void* kv_seg, int causal,
+                      int causal_off, void* stream);
+int t5x_attention_fwd_stream(const void* q, const void* k, const void* v, void* o, void* lse, int B,
+                             int H, int Lq, int Lk, int D, long long q_sb, long long q_sl,
+                             long long q_sh, long long k_sb, long long k_sl, long long k_sh,
+                             long long v_sb, long long v_sl, long long v_sh, long long o_sb,
+                             long long o_sl, long long o_sh, const void* rel_bias,
+                             const void* rel_bucket, int num_buckets, int nrel, int rel_off,
+                             const void* key_mask, const void* q_seg, const void* kv_seg, int causal,
+                             int causal_off, void* stream);
+int t5x_attention_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
+                      const void* lse, void* delta, void* dq_f32, void* dk, void* dv, int B, int H,
+                      int Lq, int Lk, int D, long long q_sb, long long q_sl, long long q_sh,
+                      long long k_sb, long long k_sl, long long k_sh, long long v_sb, long long v_sl,
+                      long long v_sh, long long o_sb, long long o_sl, long long o_sh, long long do_sb,
+                      long long do_sl, long long do_sh, long long dk_sb, long long dk_sl,
+                      long long dk_sh, const void* rel_bias, const void* rel_bucket, void* d_rel_bias,
+                      int num_buckets, int nrel, int rel_off, const void* key_mask, const void* q_seg,
+                      const void* kv_seg, int causal, int causal_off, void* stream);
+int t5x_gated_gelu_bwd(void* dg, void* h, long long rows, int dff, long long ldh, long long ldg,
+                       int write_g, void* stream);
+}
+
+namespace {
+
+using at::Tensor;
+using std::optional;
+
+void check(int rc, const char* what) {
+  if (rc != 0) throw std::runtime_error(std::string(what) + ": " + t5x_last_error());
+}
+
+void* stream_of() { return at::cuda::getCurrentCUDAStream().stream(); }
+
+bool aligned(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
+
+// Contiguous bf16 activations [..., k] on the current device.
+bool plain(const Tensor& x) {
+  return x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() >= 1 && x.is_contiguous() &&
+         x.numel() > 0 && x.get_device() == c10::cuda::current_device() && aligned(x);
+}
+
+struct Weight {
+  const Tensor& t;
+  int64_t k, n, ld;  // row-major [k, n], rows ld apart
+  bool ok;
+  // [k, out...] as a [k, n] matrix
+  explicit Weight(const Tensor& w, int64_t k_) : t(w), k(k_), n(0), ld(0), ok(false) {
+    if (!w.is_cuda() || w.scalar_type() != at::kBFloat16 || w.dim() < 2 || w.size(0) != k || !aligned(w))
+      return;
+    if (w.dim() == 2 && w.stride(1) == 1) {
+      n = w.size(1);
+      ld = w.stride(0);
+    } else if (w.is_contiguous()) {
+      n = w.numel() / k;
+      ld = n;
+    } else {
+      return;
+    }
+    // (a dimension below 8 can have the strides of either order)
+    ok = k >= 8 && n >= 8 && k % 8 == 0 && n % 8 == 0 && ld % 8 == 0 && ld >= n;
+  }
+};
+
+std::vector<int64_t> with_last(const Tensor& x, int64_t n) {
+  std::vector<int64_t> s(x.sizes().begin(), x.sizes().end());
+  s.back() = n;
+  return s;
+}
+
+bool fits(int64_t v) { return v <= 0x7fffffff; }
+
+// y[M, n] = x[M, k] @ w (+ residual)
+void forward(const Tensor& x, int64_t m, const Weight& w, const Tensor* residual, Tensor& y, void* st) {
+  check(t5x_gemm_bf16(x.data_ptr(), w.t.data_ptr(), nullptr, y.data_ptr(), m, w.n, w.k, 1, w.k, w.ld,
+                      w.n, 0, 0, 0, 0, 1, 0, 0, residual ? 2 : 0,
+                      residual ? residual->data_ptr() : nullptr, residual ? w.n : 0, 0, nullptr,
+                      nullptr, 0, 1.f, 0, st),
+        "gemm");
+}
+// dx[M, k] (+)= dy[M, n] @ w^T; dy rows ld_dy apart
+void input_grad(const void* dy, int64_t ld_dy, int64_t m, const Weight& w, Tensor& dx, bool accumulate,
+                void* st) {
+  check(t5x_gemm_bf16(dy, w.t.data_ptr(), nullptr, dx.data_ptr(), m, w.k, w.n, 1, ld_dy, w.ld, w.k, 0,
+                      0, 0, 0, 0, 0, accumulate, 0, nullptr, 0, 0, nullptr, nullptr, 0, 1.f, 0, st),
+        "gemm");
+}
+// grad[k, n] (fp32) (+)= x^T @ dy
+void weight_grad(const Tensor& x, const void* dy, int64_t ld_dy, int64_t m, const Weight& w,
+                 Tensor& grad, bool accumulate, void* st) {
+  check(t5x_gemm_bf16(x.data_ptr(), dy, nullptr, grad.data_ptr(), w.k, w.n, m, 1, w.k, ld_dy, w.n, 0,
+                      0, 0, 1, 1, 1, accumulate, 0, nullptr, 0, 0, nullptr, nullptr, 0, 1.f, 0, st),
+        "gemm");
+}
+
+// A gradient buffer the weight-gradient GEMM can write whole; narrow outputs over many rows are
+// cut into K slices by the caller's general path.
+bool grad_ok(const optional<Tensor>& g, const Weight& w, int64_t m) {
+  return g.has_value() && g->is_cuda() && g->scalar_type() == at::kFloat && g->is_contiguous() &&
+         g->numel() == w.k * w.n && ((w.k >= 256 && w.n >= 256) || m < 8192);
+}
+
+optional<Tensor> linear(const Tensor& x, const Tensor& weight, const optional<Tensor>& residual) {
+  if (!plain(x)) return std::nullopt;
+  const int64_t k = x.size(-1), m = x.numel() / k;
+  const Weight w(weight, k);
+  if (!w.ok || !fits(m)) return std::nullopt;
+  if (residual && !(plain(*residual) && residual->numel() == m * w.n)) return std::nullopt;
+  Tensor y = at::empty(with_last(x, w.n), x.options());
+  forward(x, m, w, residual ? &*residual : nullptr, y, stream_of());
+  return y;
+}
+
+optional<std::vector<Tensor>> multi_linear(const Tensor& x, const std::vector<Tensor>& weights) {
+  if (!plain(x)) return std::nullopt;
+  const int64_t k = x.size(-1), m = x.numel() / k;
+  if (!fits(m)) return std::nullopt;
+  for (const Tensor& t : weights)
+    if (!Weight(t, k).ok) return std::nullopt;
+  std::vector<Tensor> out;
+  for (const Tensor& t : weights) {
+    const Weight w(t, k);
+    out.push_back(at::empty(with_last(x, w.n), x.options()));
+    forward(x, m, w, nullptr, out.back(), stream_of());
+  }
+  return out;
+}
+
+// Input gradient (None unless wanted) of x @ W_0, x @ W_1, ...; the weight gradients go into
+// `grads` (cleared of what was there unless `accumulate`). The outer value tells whether the call
+// was covered.
+optional<std::tuple<optional<Tensor>>> multi_linear_bwd(
+    const std::vector<Tensor>& dys, const Tensor& x, const std::vector<Tensor>& weights,
+    const std::vector<optional<Tensor>>& grads, const std::vector<bool>& accumulate, bool need_dx,
+    bool need_dw) {
+  if (!plain(x)) return std::nullopt;
+  const int64_t k = x.size(-1), m = x.numel() / k;
+  if (!fits(m)) return std::nullopt;
+  for (size_t i = 0; i < dys.size(); ++i) {
+    const Weight w(weights[i], k);
+    if (!w.ok || !plain(dys[i]) || dys[i].numel() != m * w.n) return std::nullopt;
+    if (need_dw && !grad_ok(grads[i], w, m)) return std::nullopt;
+  }
+  void* st = stream_of();
+  optional<Tensor> dx;
+  if (need_dx) dx = at::empty_like(x);
+  for (size_t i = 0; i < dys.size(); ++i) {
+    const Weight w(weights[i], k);
+    if (need_dx) input_grad(dys[i].data_ptr(), w.n, m, w, *dx, i > 0, st);
+    if (need_dw) {
+      Tensor g = *grads[i];
+      weight_grad(x, dys[i].data_ptr(), w.n, m, w, g, accumulate[i], st);
+    }
+  }
+  return std::make_tuple(dx);
+}
+
+// (gelu(x @ w0) * (x @ w1), the two pre-activations side by side)
+optional<std::tuple<Tensor, Tensor>> gated_in(const Tensor& x, const Tensor& w0, const Tensor& w1) {
+  if (!plain(x)) return std::nullopt;
+  const int64_t k = x.size(-1), m = x.numel() / k;
+  const Weight a(w0, k), b(w1, k);
+  if (!a.ok || !b.ok || !fits(m) || w0.dim() != 2 || w1.dim() != 2 || a.n != b.n || a.ld != b.ld)
+    return std::nullopt;
+  Tensor g = at::empty(with_last(x, a.n), x.options());
+  Tensor h = at::empty({m, 2 * a.n}, x.options());
+  char* h0 = static_cast<char*>(h.data_ptr());
+  check(t5x_gemm_bf16(x.data_ptr(), w0.data_ptr(), w1.data_ptr(), g.data_ptr(), m, a.n, k, 1, k, a.ld,
+                      a.n, 0, 0, 0, 0, 1, 0, 0, 1, nullptr, 0, 0, h0, h0 + a.n * 2, 2 * a.n, 1.f, 0,
+                      stream_of()),
+        "gemm");
+  return std::make_tuple(g, h);
+}
+
+// Backward of gated_in; `h` is overwritten with the gradients of the pre-activations.
+optional<std::tuple<optional<Tensor>>> gated_in_bwd(const Tensor& dg, const Tensor& x,
+                                                    const Tensor& w0, const Tensor& w1, Tensor h,
+                                                    const optional<Tensor>& grad0,
+                                                    const optional<Tensor>& grad1, bool acc0,
+                                                    bool acc1, bool need_dx, bool need_dw) {
+  if (!plain(x) || !plain(dg) || !plain(h)) return std::nullopt;
+  const int64_t k = x.size(-1), m = x.numel() / k;
+  const Weight a(w0, k), b(w1, k);
+  if (!a.ok || !b.ok || !fits(m) || a.n != b.n || dg.numel() != m * a.n || h.numel() != 2 * m * a.n)
+    return std::nullopt;
+  if (need_dw && !(grad_ok(grad0, a, m) && grad_ok(grad1, b, m))) return std::nullopt;
+  void* st = stream_of();
+  check(t5x_gated_gelu_bwd(dg.data_ptr(), h.data_ptr(), m, a.n, 2 * a.n, a.n, 0, st),
+        "gated_gelu_bwd");
+  const char* d0 = static_cast<const char*>(h.data_ptr());
+  const char* d1 = d0 + a.n * 2;
+  optional<Tensor> dx;
+  if (need_dx) {
+    dx = at::empty_like(x);
+    input_grad(d0, 2 * a.n, m, a, *dx, false, st);
+    input_grad(d1, 2 * a.n, m, b, *dx, true, st);
+  }
+  if (need_dw) {
+    Tensor g0 = *grad0, g1 = *grad1;
+    weight_grad(x, d0, 2 * a.n, m, a, g0, acc0, st);
+    weight_grad(x, d1, 2 * a.n, m, b, g1, acc1, st);
+  }
+  return std::make_tuple(dx);
+}
+
+optional<std::tuple<Tensor, Tensor>> rmsnorm(const Tensor& x, const Tensor& scale, double eps) {
+  if (!plain(x) || scale.scalar_type() != at::kFloat || !scale.is_contiguous() ||
+      scale.numel() != x.size(-1) || !scale.is_cuda())
+    return std::nullopt;
+  const int64_t d = x.size(-1), rows = x.numel() / d;
+  if (!fits(rows)) return std::nullopt;
+  Tensor y = at::empty_like(x);
+  Tensor rstd = at::empty({rows}, x.options().dtype(at::kFloat));
+  check(t5x_rmsnorm_fwd(x.data_ptr(), scale.data_ptr(), y.data_ptr(), rstd.data_ptr(), rows, d, eps,
+                        stream_of()),
+        "rmsnorm_fwd");
+  return std::make_tuple(y, rstd);
+}
+
+// dx (+ dres); adds to `dscale`
+optional<Tensor> rmsnorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& scale,
+                             const Tensor& rstd, const optional<Tensor>& dres, Tensor dscale) {
+  if (!plain(x) || !plain(dy) || dy.numel() != x.numel() || scale.scalar_type() != at::kFloat ||
+      !scale.is_contiguous() || scale.numel() != x.size(-1) || dscale.scalar_type() != at::kFloat ||
+      !dscale.is_contiguous() || dscale.numel() != scale.numel())
+    return std::nullopt;
+  if (dres && !(plain(*dres) && dres->numel() == x.numel())) return std::nullopt;
+  const int64_t d = x.size(-1), rows = x.numel() / d;
+  Tensor dx = at::empty_like(x);
+  check(t5x_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), scale.data_ptr(), rstd.data_ptr(),
+                        dres ? dres->data_ptr() : nullptr, dx.data_ptr(), dscale.data_ptr(), rows, d,
+                        stream_of()),
+        "rmsnorm_bwd");
+  return dx;
+}
+
+// [B, L, H, D] bf16 on the current device, channels contiguous, rows on 16-byte boundaries.
+bool heads_ok(const Tensor& t) {
+  return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.dim() == 4 && t.numel() > 0 &&
+         t.stride(3) == 1 && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0 && t.stride(2) % 8 == 0 &&
+         aligned(t) && t.get_device() == c10::cuda::current_device();
+}
+
+const void* data_or_null(const optional<Tensor>& t) { return t ? t->data_ptr() : nullptr; }
+
+// Flash attention; what the caller has prepared: an fp32 bias table with int32 buckets, a uint8 key
+// mask, int32 segment codes, all contiguous (checked where they are made).
+optional<std::tuple<Tensor, Tensor>> attention(
+    const Tensor& q, const Tensor& k, const Tensor& v, const optional<Tensor>& rel_bias,
+    const optional<Tensor>& buckets, const optional<Tensor>& key_mask, const optional<Tensor>& q_seg,
+    const optional<Tensor>& kv_seg, int64_t causal, int64_t causal_off, int64_t rel_off,
+    bool short_range) {
+  if (!heads_ok(q) || !heads_ok(k) || !heads_ok(v)) return std::nullopt;
+  const int B = q.size(0), Lq = q.size(1), H = q.size(2), D = q.size(3), Lk = k.size(1);
+  Tensor o = at::empty({B, Lq, H, D}, q.options());
+  Tensor lse = at::empty({B, H, Lq}, q.options().dtype(at::kFloat));
+  const int nb = rel_bias ? rel_bias->size(1) : 0, nrel = rel_bias ? buckets->size(0) : 0;
+  const void *table = data_or_null(rel_bias), *bucket = rel_bias ? buckets->data_ptr() : nullptr;
+  if (short_range)
+    check(t5x_attention_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), B,
+                            H, Lq, Lk, q.stride(0), q.stride(1), q.stride(2), k.stride(0),
+                            k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2),
+                            o.stride(0), o.stride(1), o.stride(2), table, bucket, nb, nrel, rel_off,
+                            data_or_null(key_mask), data_or_null(q_seg), data_or_null(kv_seg), causal,
+                            causal_off, stream_of()),
+          "attention_fwd");
+  else
+    check(t5x_attention_fwd_stream(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
+                                   lse.data_ptr(), B, H, Lq, Lk, D, q.stride(0), q.stride(1),
+                                   q.stride(2), k.stride(0), k.stride(1), k.stride(2), v.stride(0),
+                                   v.stride(1), v.stride(2), o.stride(0), o.stride(1), o.stride(2),
+                                   table, bucket, nb, nrel, rel_off, data_or_null(key_mask),
+                                   data_or_null(q_seg), data_or_null(kv_seg), causal, causal_off,
+                                   stream_of()),
+          "attention_fwd");
+  return std::make_tuple(o, lse);
+}
+
+// (dq, dk, dv); dq, dk and dv are the column blocks of one buffer when q, k and v are (`packed`).
+optional<std::tuple<Tensor, Tensor, Tensor>> attention_bwd(
+    const Tensor& d_o, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o,
+    const Tensor& lse, const optional<Tensor>& rel_bias, const optional<Tensor>& buckets,
+    const optional<Tensor>& key_mask, const optional<Tensor>& q_seg, const optional<Tensor>& kv_seg,
+    const optional<Tensor>& d_rel, int64_t causal, int64_t causal_off, int64_t rel_off, bool packed) {
+  if (!heads_ok(d_o) || !heads_ok(q) || !heads_ok(k) || !heads_ok(v) || !heads_ok(o))
+    return std::nullopt;
+  const int B = q.size(0), Lq = q.size(1), H = q.size(2), D = q.size(3), Lk = k.size(1);
+  const auto f32 = q.options().dtype(at::kFloat);
+  Tensor dq32 = at::zeros({B, Lq, H, D}, f32), delta = at::empty({B, H, Lq}, f32);
+  Tensor dq, dk, dv;
+  if (packed) {
+    Tensor all = at::empty({B, Lq, 3, H, D}, q.options());
+    dq = all.select(2, 0);
+    dk = all.select(2, 1);
+    dv = all.select(2, 2);
+  } else {
+    dk = at::empty({B, Lk, H, D}, q.options());
+    dv = at::empty({B, Lk, H, D}, q.options());
+  }
+  const int nb = rel_bias ? rel_bias->size(1) : 0, nrel = rel_bias ? buckets->size(0) : 0;
+  check(t5x_attention_bwd(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), lse.data_ptr(),
+            delta.data_ptr(), dq32.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Lq, Lk, D,
+            q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2), v.stride(0),
+            v.stride(1), v.stride(2), o.stride(0), o.stride(1), o.stride(2), d_o.stride(0),
+            d_o.stride(1), d_o.stride(2), dk.stride(0), dk.stride(1), dk.stride(2),
+            data_or_null(rel_bias), rel_bias ? buckets->data_ptr() : nullptr,
+            d_rel ? d_rel->data_ptr() : nullptr, nb, nrel, rel_off, data_or_null(key_mask),
+            data_or_null(q_seg), data_or_null(kv_seg), causal, causal_off, stream_of()),
+        "attention_bwd");
+  if (packed)
+    dq.copy_(dq32);
+  else
+    dq = dq32.to(at::kBFloat16);
+  return std::make_tuple(dq, dk, dv);
+}
+
+}  // namespace
+
+// The GIL is released for the duration of a call: a launch waits when the device's queue is full,
+// and the threads that prepare batches have to go on meanwhile.
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("linear", torch::wrap_pybind_function_no_gil(linear));
+  m.def("multi_linear", torch::wrap_pybind_function_no_gil(multi_linear));
+  m.def("multi_linear_bwd", torch::wrap_pybind_function_no_gil(multi_linear_bwd));
+  m.def("gated_in", torch::wrap_pybind_function_no_gil(gated_in));
+  m.def("gated_in_bwd", torch::wrap_pybind_function_no_gil(gated_in_bwd));
+  m.def("rmsnorm", torch::wrap_pybind_function_no_gil(rmsnorm));
+  m.def("attention", torch::wrap_pybind_function_no_gil(attention));
+  m.def("attention_bwd", torch::wrap_pybind_function_no_gil(attention_bwd));
+  m.def("rmsnorm_bwd", torch::wrap_pybind_function_no_gil(rmsnorm_bwd));
+}

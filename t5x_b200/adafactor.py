@@ -16,7 +16,8 @@ from __future__ import annotations
 import dataclasses
 import enum
 import re
-from typing import Any, Mapping, Optional, Sequence, Tuple, Union
+from collections.abc import Mapping
+from typing import Any, Optional, Sequence, Tuple, Union
 
 import numpy as np
 import torch

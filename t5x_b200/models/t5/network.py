@@ -51,6 +51,13 @@ def _dropout(x, rate, enable, broadcast=True, **kw):
   return F.dropout(x, rate, enable, broadcast_dims=(-2,) if broadcast else (), **kw)
 
 
+def _segment_codes(segment_ids):
+  """The segment ids in the type that the attention kernels read, once for all layers."""
+  if segment_ids is not None and segment_ids.is_cuda:
+    return segment_ids.to(torch.int32)
+  return segment_ids
+
+
 class EncoderLayer(nn.Module):
   """pre-LN self-attention and pre-LN MLP, each with a residual (network.py:47-96)."""
 
@@ -229,6 +236,7 @@ class Encoder(nn.Module):
   def forward(self, encoder_input_tokens, encoder_segment_ids=None, enable_dropout=False):
     c = self.config
     key_mask = encoder_input_tokens > 0
+    encoder_segment_ids = _segment_codes(encoder_segment_ids)
     x = self._shared[0](encoder_input_tokens.long())
     b, l, d = x.shape
     if tp_fused.usable(x, b * l) and _sp_dropout_ok(x, c, enable_dropout):
@@ -289,6 +297,8 @@ class Decoder(nn.Module):
              decode=False, cache=None, beams_per_kv: int = 1):
     """Final-norm hidden states [batch, len, emb] (what the logits projection consumes)."""
     c = self.config
+    encoder_segment_ids = _segment_codes(encoder_segment_ids)
+    decoder_segment_ids = _segment_codes(decoder_segment_ids)
     y = self._shared[0](decoder_input_tokens.long())
     b, l, d = y.shape
     if (tp_fused.usable(y, b * l) and not decode and cache is None and

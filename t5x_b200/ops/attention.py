@@ -89,6 +89,15 @@ class _FlashAttentionFn(torch.autograd.Function):
   @staticmethod
   def forward(ctx, q, k, v, rel_bias, buckets, key_mask, q_seg, kv_seg, causal, causal_off,
               rel_off):
+    ctx.cfg = (causal, causal_off, rel_off)
+    host = native.host()
+    if host is not None:
+      short = forward_kernel(q.shape[1], k.shape[1], q.shape[3], int(causal) == 2) == "classic"
+      done = host.attention(q, k, v, rel_bias, buckets, key_mask, q_seg, kv_seg, int(causal),
+                            causal_off, rel_off, short)
+      if done is not None:
+        ctx.save_for_backward(q, k, v, *done, rel_bias, buckets, key_mask, q_seg, kv_seg)
+        return done[0]
     q = q if _strides_ok(q) else q.contiguous()
     k = k if _strides_ok(k) else k.contiguous()
     v = v if _strides_ok(v) else v.contiguous()
@@ -98,8 +107,8 @@ class _FlashAttentionFn(torch.autograd.Function):
     lse = torch.empty((B, H, Lq), dtype=torch.float32, device=q.device)
     nb, nrel = _bias_sizes(rel_bias, buckets)
     tail = (*_sbh(q), *_sbh(k), *_sbh(v), *_sbh(o), native.ptr(rel_bias), native.ptr(buckets), nb,
-            nrel, rel_off, native.ptr(key_mask), native.ptr(q_seg), native.ptr(kv_seg), int(causal), causal_off,
-            native.stream_ptr())
+            nrel, rel_off, native.ptr(key_mask), native.ptr(q_seg), native.ptr(kv_seg),
+            int(causal), causal_off, native.stream_ptr())
     if forward_kernel(Lq, Lk, D, int(causal) == 2) == "classic":
       rc = native.lib().t5x_attention_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
                                           lse.data_ptr(), B, H, Lq, Lk, *tail)
@@ -109,26 +118,12 @@ class _FlashAttentionFn(torch.autograd.Function):
                                                  *tail)
     native._check(rc, "attention_fwd")
     ctx.save_for_backward(q, k, v, o, lse, rel_bias, buckets, key_mask, q_seg, kv_seg)
-    ctx.cfg = (causal, causal_off, rel_off)
     return o
 
   @staticmethod
   def backward(ctx, do):
     q, k, v, o, lse, rel_bias, buckets, key_mask, q_seg, kv_seg = ctx.saved_tensors
     causal, causal_off, rel_off = ctx.cfg
-    B, Lq, H, D = q.shape
-    Lk = k.shape[1]
-    do = do if _strides_ok(do) else do.contiguous()
-    dq32 = torch.zeros((B, Lq, H, D), dtype=torch.float32, device=q.device)
-    packed = _packed_qkv(q, k, v)
-    if packed:
-      dqkv = torch.empty((B, Lq, 3, H, D), dtype=torch.bfloat16, device=q.device)
-      dq, dk, dv = dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]
-    else:
-      dk = torch.empty((B, Lk, H, D), dtype=torch.bfloat16, device=q.device)
-      dv = torch.empty((B, Lk, H, D), dtype=torch.bfloat16, device=q.device)
-    delta = torch.empty((B, H, Lq), dtype=torch.float32, device=q.device)
-    nb, nrel = _bias_sizes(rel_bias, buckets)
     d_rel = ret_rel = None  # the buffer the kernel adds to, and what autograd gets
     if rel_bias is not None and ctx.needs_input_grad[3]:
       mg = getattr(rel_bias, "main_grad", None)
@@ -139,13 +134,31 @@ class _FlashAttentionFn(torch.autograd.Function):
         d_rel = mg
       else:
         d_rel = ret_rel = torch.zeros_like(rel_bias)
+    packed = _packed_qkv(q, k, v)
+    host = native.host()
+    if host is not None:
+      done = host.attention_bwd(do, q, k, v, o, lse, rel_bias, buckets, key_mask, q_seg, kv_seg,
+                                d_rel, int(causal), causal_off, rel_off, packed)
+      if done is not None:
+        return (*done, ret_rel, None, None, None, None, None, None, None)
+    B, Lq, H, D = q.shape
+    Lk = k.shape[1]
+    do = do if _strides_ok(do) else do.contiguous()
+    dq32 = torch.zeros((B, Lq, H, D), dtype=torch.float32, device=q.device)
+    if packed:
+      dqkv = torch.empty((B, Lq, 3, H, D), dtype=torch.bfloat16, device=q.device)
+      dq, dk, dv = dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]
+    else:
+      dk = torch.empty((B, Lk, H, D), dtype=torch.bfloat16, device=q.device)
+      dv = torch.empty((B, Lk, H, D), dtype=torch.bfloat16, device=q.device)
+    delta = torch.empty((B, H, Lq), dtype=torch.float32, device=q.device)
+    nb, nrel = _bias_sizes(rel_bias, buckets)
     rc = native.lib().t5x_attention_bwd(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
         delta.data_ptr(), dq32.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Lq, Lk, D,
-        *_sbh(q),
-        *_sbh(k), *_sbh(v), *_sbh(o), *_sbh(do), *_sbh(dk), native.ptr(rel_bias),
-        native.ptr(buckets), native.ptr(d_rel), nb, nrel, rel_off, native.ptr(key_mask), native.ptr(q_seg),
-        native.ptr(kv_seg), int(causal), causal_off, native.stream_ptr())
+        *_sbh(q), *_sbh(k), *_sbh(v), *_sbh(o), *_sbh(do), *_sbh(dk), native.ptr(rel_bias),
+        native.ptr(buckets), native.ptr(d_rel), nb, nrel, rel_off, native.ptr(key_mask),
+        native.ptr(q_seg), native.ptr(kv_seg), int(causal), causal_off, native.stream_ptr())
     native._check(rc, "attention_bwd")
     if packed:
       dq.copy_(dq32)
@@ -171,6 +184,14 @@ def _rel_buckets(Lq, Lk, q_offset, bidirectional, num_buckets, max_distance, dev
   return b
 
 
+def _byte_mask(mask: torch.Tensor) -> torch.Tensor:
+  """`mask` as contiguous uint8. Where nothing is kept for a backward pass a boolean one is read as
+  it is (its bytes are 0 and 1), not copied."""
+  if mask.dtype == torch.bool and not torch.is_grad_enabled():
+    return mask.contiguous().view(torch.uint8)
+  return mask.to(torch.uint8).contiguous()
+
+
 def flash_attention(q, k, v, *, bias_table: Optional[torch.Tensor] = None,
                     bidirectional: bool = True, num_buckets: int = 32, max_distance: int = 128,
                     key_mask: Optional[torch.Tensor] = None, causal: bool = False,
@@ -187,7 +208,7 @@ def flash_attention(q, k, v, *, bias_table: Optional[torch.Tensor] = None,
     if rel_bias.shape[1] < num_buckets:
       raise ValueError(f"bias table has {rel_bias.shape[1]} buckets, {num_buckets} are indexed")
     buckets = _rel_buckets(Lq, Lk, q_offset, bidirectional, num_buckets, max_distance, q.device)
-  km = key_mask.to(torch.uint8).contiguous() if key_mask is not None else None
+  km = _byte_mask(key_mask) if key_mask is not None else None
   qs = q_segment_ids.to(torch.int32).contiguous() if q_segment_ids is not None else None
   ks = kv_segment_ids.to(torch.int32).contiguous() if kv_segment_ids is not None else None
   if qs is None or ks is None:
@@ -195,8 +216,9 @@ def flash_attention(q, k, v, *, bias_table: Optional[torch.Tensor] = None,
   mode = int(bool(causal))
   if prefix_lm is not None:
     qs, ks = prefix_lm.token_codes()
-    valid = prefix_lm.valid.to(torch.uint8)
-    km = valid.contiguous() if km is None else (km & valid).contiguous()
+    valid = _byte_mask(prefix_lm.valid)
+    km = valid if km is None else km & valid
     mode = 2
-  return _FlashAttentionFn.apply(q, k, v, rel_bias, buckets, km, qs, ks, mode,
-                                 (Lk - Lq) if mode else 0, Lq - 1)
+  from t5x_b200.ops import functional
+  return functional._apply(_FlashAttentionFn, q, k, v, rel_bias, buckets, km, qs, ks, mode,
+                           (Lk - Lq) if mode else 0, Lq - 1)

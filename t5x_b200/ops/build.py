@@ -16,6 +16,9 @@ CSRC = os.path.join(ROOT, "csrc")
 LIB_DIR = os.path.join(ROOT, "t5x_b200", "lib")
 OBJ_DIR = os.path.join(LIB_DIR, "obj")
 LIB_PATH = os.path.join(LIB_DIR, "libt5x_b200.so")
+HOST_SRC = os.path.join(CSRC, "host", "host_ops.cpp")
+HOST_NAME = "_t5x_host"
+HOST_PATH = os.path.join(LIB_DIR, HOST_NAME + ".so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -72,7 +75,49 @@ def build(verbose: bool = False, force: bool = False, ptxas_v: bool = False) -> 
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
       raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+  build_host(verbose, force)
   return LIB_PATH
+
+
+def build_host(verbose: bool = False, force: bool = False) -> str:
+  """Compiles the Python extension that takes tensors to kernel launches; it is linked with the
+  kernel library beside it."""
+  if not force and os.path.exists(HOST_PATH) and \
+      os.path.getmtime(HOST_PATH) >= os.path.getmtime(HOST_SRC):
+    return HOST_PATH
+  import sysconfig
+  import torch
+  root = os.path.dirname(torch.__file__)
+  cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+  includes = [os.path.join(root, "include"),
+              os.path.join(root, "include", "torch", "csrc", "api", "include"),
+              os.path.join(cuda, "include"), sysconfig.get_path("include")]
+  cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+         f"-DTORCH_EXTENSION_NAME={HOST_NAME}", "-DTORCH_API_INCLUDE_EXTENSION_H",
+         *(f"-I{d}" for d in includes), HOST_SRC, "-o", HOST_PATH + ".tmp",
+         f"-L{LIB_DIR}", "-lt5x_b200", f"-L{os.path.join(root, 'lib')}", "-lc10", "-ltorch",
+         "-ltorch_cpu", "-ltorch_python", "-lc10_cuda", "-ltorch_cuda", "-Wl,-rpath,$ORIGIN"]
+  if verbose:
+    print(" ".join(cmd), flush=True)
+  r = subprocess.run(cmd, capture_output=True, text=True)
+  if r.returncode != 0:
+    raise RuntimeError(f"g++ failed for {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
+  os.replace(HOST_PATH + ".tmp", HOST_PATH)
+  return HOST_PATH
+
+
+def load_host():
+  """The extension module, built first if it is missing."""
+  import importlib.machinery
+  import importlib.util
+  if not os.path.exists(HOST_PATH):
+    build_host()
+  loader = importlib.machinery.ExtensionFileLoader(HOST_NAME, HOST_PATH)
+  spec = importlib.util.spec_from_file_location(HOST_NAME, HOST_PATH, loader=loader)
+  module = importlib.util.module_from_spec(spec)
+  loader.exec_module(module)
+  return module
 
 
 if __name__ == "__main__":

@@ -52,22 +52,87 @@ def _accumulate_wgrad(weight: torch.Tensor, a_t: torch.Tensor, b: torch.Tensor):
   return native.gemm(a_t, b, out_dtype=torch.float32).view(weight.shape).to(weight.dtype)
 
 
+class _NoGraph:
+  """Stands in for the context of an autograd function whose forward runs outside autograd."""
+
+  def save_for_backward(self, *tensors):
+    pass
+
+  def mark_non_differentiable(self, *tensors):
+    pass
+
+
+def _apply(fn, *args):
+  """fn.apply(*args). Where nothing can record or transform the call (no gradients, no function
+  transform, no forward-mode level, no tracing) the forward runs directly, without building
+  an autograd node for it."""
+  if (not torch.is_grad_enabled() and torch._C._functorch.peek_interpreter_stack() is None and
+      torch.autograd.forward_ad._current_level < 0 and torch._C._get_tracing_state() is None):
+    return fn.forward(_NoGraph(), *args)
+  return fn.apply(*args)
+
+
+def _take_grad_flags(weights):
+  """(accumulate into main_grad?) per weight, which from here on counts as written."""
+  flags = []
+  for w in weights:
+    flags.append(bool(getattr(w, "grad_ready", False)))
+    w.grad_ready = True
+  return flags
+
+
+def _restore_grad_flags(weights, flags):
+  for w, f in zip(reversed(weights), reversed(flags)):
+    w.grad_ready = f
+
+
+def _host_linear_bwd(dys, x, weights, needs):
+  """Backward of x @ W_0, x @ W_1, ... through the compiled host path: (covered, dx)."""
+  host = native.host()
+  if host is None or any(dy is None for dy in dys):
+    return False, None
+  need_dw = needs[1]
+  if any(n != need_dw for n in needs[2:1 + len(weights)]):
+    return False, None
+  grads, flags = [None] * len(weights), [False] * len(weights)
+  if need_dw:
+    grads = [getattr(w, "main_grad", None) for w in weights]
+    if any(g is None for g in grads):
+      return False, None
+    flags = _take_grad_flags(weights)
+  done = host.multi_linear_bwd(list(dys), x, [compute_weight(w, torch.bfloat16) for w in weights],
+                               grads, flags, bool(needs[0]), bool(need_dw))
+  if done is None:
+    if need_dw:
+      _restore_grad_flags(weights, flags)
+    return False, None
+  return True, done[0]
+
+
 class _LinearFn(torch.autograd.Function):
 
   @staticmethod
   def forward(ctx, x, weight, residual):
+    ctx.save_for_backward(x, weight)
+    ctx.has_res = residual is not None
+    host = native.host()
+    if host is not None:
+      y = host.linear(x, compute_weight(weight, torch.bfloat16), residual)
+      if y is not None:
+        return y
     k = x.shape[-1]
     w2 = compute_weight(weight, torch.bfloat16).reshape(k, -1)
     x2 = x.reshape(-1, k)
     r2 = residual.reshape(-1, w2.shape[1]) if residual is not None else None
     y = native.gemm(x2, w2, residual=r2)
-    ctx.save_for_backward(x, weight)
-    ctx.has_res = residual is not None
     return y.view(*x.shape[:-1], w2.shape[1])
 
   @staticmethod
   def backward(ctx, dy):
     x, weight = ctx.saved_tensors
+    covered, dx = _host_linear_bwd([dy], x, [weight], ctx.needs_input_grad)
+    if covered:
+      return dx, None, (dy if ctx.has_res else None)
     k = x.shape[-1]
     w2 = compute_weight(weight, torch.bfloat16).reshape(k, -1)
     dy2 = dy.reshape(-1, w2.shape[1])
@@ -91,18 +156,26 @@ class _MultiLinearFn(torch.autograd.Function):
 
   @staticmethod
   def forward(ctx, x, *weights):
+    ctx.save_for_backward(x, *weights)
+    host = native.host()
+    if host is not None:
+      outs = host.multi_linear(x, [compute_weight(w, torch.bfloat16) for w in weights])
+      if outs is not None:
+        return tuple(outs)
     k = x.shape[-1]
     x2 = x.reshape(-1, k)
     outs = []
     for w in weights:
       w2 = compute_weight(w, torch.bfloat16).reshape(k, -1)
       outs.append(native.gemm(x2, w2).view(*x.shape[:-1], w2.shape[1]))
-    ctx.save_for_backward(x, *weights)
     return tuple(outs)
 
   @staticmethod
   def backward(ctx, *dys):
     x, *weights = ctx.saved_tensors
+    covered, dx = _host_linear_bwd(dys, x, weights, ctx.needs_input_grad)
+    if covered:
+      return (dx,) + (None,) * len(weights)
     k = x.shape[-1]
     x2 = x.reshape(-1, k)
     dx = None
@@ -128,7 +201,7 @@ def multi_linear(x: torch.Tensor, weights: Sequence[torch.Tensor],
                  dtype: Optional[torch.dtype] = None):
   """[x @ W for W in weights] with one fused backward for the shared input."""
   if _native_ok(x):
-    return list(_MultiLinearFn.apply(x, *weights))
+    return list(_apply(_MultiLinearFn, x, *weights))
   return [linear(x, w, dtype=dtype) for w in weights]
 
 
@@ -137,7 +210,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, residual: Optional[torch.Tenso
   """y = x @ W (+ residual). W is [in, out...] (T5X kernel layout); trailing kernel dims are
   flattened for the contraction and kept flat in the output."""
   if _native_ok(x):
-    return _LinearFn.apply(x, weight, residual)
+    return _apply(_LinearFn, x, weight, residual)
   dt = dtype or x.dtype
   w = compute_weight(weight, dt).reshape(x.shape[-1], -1)
   y = x.to(dt) @ w
@@ -177,17 +250,37 @@ def batched_linear(x: torch.Tensor, weight: torch.Tensor,
                    dtype: Optional[torch.dtype] = None) -> torch.Tensor:
   """x [E, N, in] @ weight [E, in, out] -> [E, N, out]."""
   if _native_ok(x):
-    return _BatchedLinearFn.apply(x, weight)
+    return _apply(_BatchedLinearFn, x, weight)
   dt = dtype or x.dtype
   return torch.bmm(x.to(dt), compute_weight(weight, dt))
+
+
+def _rmsnorm_fwd(x, scale, eps, out):
+  """(norm, contiguous x, 1 / rms)"""
+  host = native.host()
+  if host is not None and out is None:
+    done = host.rmsnorm(x, scale, eps)
+    if done is not None:
+      return done[0], x, done[1]
+  xc = x.contiguous()
+  y, rstd = native.rmsnorm_fwd(xc, scale.float(), eps, out=out)
+  return y, xc, rstd
+
+
+def _rmsnorm_bwd(dy, x, scale, rstd, dres, dscale):
+  host = native.host()
+  if host is not None:
+    dx = host.rmsnorm_bwd(dy, x, scale, rstd, dres, dscale)
+    if dx is not None:
+      return dx
+  return native.rmsnorm_bwd(dy.contiguous(), x, scale.float(), rstd, dres, dscale)
 
 
 class _RmsNormFn(torch.autograd.Function):
 
   @staticmethod
   def forward(ctx, x, scale, eps, out=None):
-    xc = x.contiguous()
-    y, rstd = native.rmsnorm_fwd(xc, scale.float(), eps, out=out)
+    y, xc, rstd = _rmsnorm_fwd(x, scale, eps, out)
     ctx.save_for_backward(xc, scale, rstd)
     return y
 
@@ -203,7 +296,7 @@ class _RmsNormFn(torch.autograd.Function):
     else:
       dscale_buf = torch.zeros_like(scale, dtype=torch.float32)
       ret = dscale_buf
-    dx = native.rmsnorm_bwd(dy.contiguous(), x, scale.float(), rstd, None, dscale_buf)
+    dx = _rmsnorm_bwd(dy, x, scale, rstd, None, dscale_buf)
     return dx, ret, None, None
 
 
@@ -214,8 +307,7 @@ class _ResidualRmsNormFn(torch.autograd.Function):
 
   @staticmethod
   def forward(ctx, x, scale, eps, out=None):
-    xc = x.contiguous()
-    y, rstd = native.rmsnorm_fwd(xc, scale.float(), eps, out=out)
+    y, xc, rstd = _rmsnorm_fwd(x, scale, eps, out)
     ctx.save_for_backward(xc, scale, rstd)
     return x.view_as(x), y
 
@@ -235,7 +327,7 @@ class _ResidualRmsNormFn(torch.autograd.Function):
       ret = dscale_buf
     if dres is not None:
       dres = dres.to(torch.bfloat16).contiguous()
-    dx = native.rmsnorm_bwd(dy.contiguous(), x, scale.float(), rstd, dres, dscale_buf)
+    dx = _rmsnorm_bwd(dy, x, scale, rstd, dres, dscale_buf)
     return dx, ret, None, None
 
 
@@ -244,7 +336,7 @@ def residual_rmsnorm(x: torch.Tensor, scale: torch.Tensor, eps: float = 1e-6,
   """(x, rmsnorm(x)); use the first element as the residual input of the block the norm
   feeds, so that the two gradient paths into x meet inside the norm's backward kernel."""
   if _native_ok(x):
-    return _ResidualRmsNormFn.apply(x, scale, eps, out)
+    return _apply(_ResidualRmsNormFn, x, scale, eps, out)
   return x, ref.rmsnorm(x, scale, eps)
 
 
@@ -252,7 +344,7 @@ def rmsnorm(x: torch.Tensor, scale: torch.Tensor, eps: float = 1e-6,
             out: Optional[torch.Tensor] = None) -> torch.Tensor:
   """`out` (CUDA path only): a bf16 buffer of x's shape that receives the result."""
   if _native_ok(x):
-    return _RmsNormFn.apply(x, scale, eps, out)
+    return _apply(_RmsNormFn, x, scale, eps, out)
   return ref.rmsnorm(x, scale, eps)
 
 
@@ -261,6 +353,13 @@ class _GatedGeluMlpInFn(torch.autograd.Function):
 
   @staticmethod
   def forward(ctx, x, wi_0, wi_1):
+    host = native.host()
+    if host is not None:
+      done = host.gated_in(x, compute_weight(wi_0, torch.bfloat16),
+                           compute_weight(wi_1, torch.bfloat16))
+      if done is not None:
+        ctx.save_for_backward(x, wi_0, wi_1, done[1])
+        return done[0]
     k = x.shape[-1]
     x2 = x.reshape(-1, k)
     w0 = compute_weight(wi_0, torch.bfloat16)
@@ -274,6 +373,17 @@ class _GatedGeluMlpInFn(torch.autograd.Function):
   @staticmethod
   def backward(ctx, dg):
     x, wi_0, wi_1, h = ctx.saved_tensors
+    host, (need_dx, need_0, need_1) = native.host(), ctx.needs_input_grad[:3]
+    g0, g1 = getattr(wi_0, "main_grad", None), getattr(wi_1, "main_grad", None)
+    if host is not None and need_0 == need_1 and not (need_0 and (g0 is None or g1 is None)):
+      flags = _take_grad_flags([wi_0, wi_1]) if need_0 else [False, False]
+      done = host.gated_in_bwd(dg, x, compute_weight(wi_0, torch.bfloat16),
+                               compute_weight(wi_1, torch.bfloat16), h, g0, g1, *flags,
+                               bool(need_dx), bool(need_0))
+      if done is not None:
+        return done[0], None, None
+      if need_0:
+        _restore_grad_flags([wi_0, wi_1], flags)
     k = x.shape[-1]
     dff = h.shape[1] // 2
     x2 = x.reshape(-1, k)
@@ -295,7 +405,7 @@ class _GatedGeluMlpInFn(torch.autograd.Function):
 
 def gated_gelu_mlp_in(x, wi_0, wi_1, dtype: Optional[torch.dtype] = None):
   if _native_ok(x):
-    return _GatedGeluMlpInFn.apply(x, wi_0, wi_1)
+    return _apply(_GatedGeluMlpInFn, x, wi_0, wi_1)
   dt = dtype or x.dtype
   return ref.gelu_tanh(x.to(dt) @ compute_weight(wi_0, dt)) * (x.to(dt) @ compute_weight(wi_1, dt))
 
@@ -324,7 +434,7 @@ class _EmbeddingFn(torch.autograd.Function):
 
 def embedding(ids: torch.Tensor, table: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
   if table.is_cuda and dtype == torch.bfloat16:
-    return _EmbeddingFn.apply(ids, table)
+    return _apply(_EmbeddingFn, ids, table)
   return compute_weight(table, dtype)[ids]
 
 
@@ -561,8 +671,8 @@ def logits_cross_entropy(hidden, weight, targets, *, z_loss: float = 0.0,
   constant, as `compute_weighted_cross_entropy` does before weighting (t5x/losses.py:132-193).
   """
   if _native_ok(hidden):
-    return _LogitsCrossEntropyFn.apply(hidden, weight, targets, z_loss, label_smoothing,
-                                       logits_scale)
+    return _apply(_LogitsCrossEntropyFn, hidden, weight, targets, z_loss, label_smoothing,
+                  logits_scale)
   k = hidden.shape[-1]
   w = weight.float()
   if w.shape[0] != k:

@@ -125,6 +125,47 @@ def register_signature(name: str, argtypes) -> None:
     getattr(_lib, name).argtypes = argtypes
 
 
+class _HostOps:
+  """The functions of the compiled host path (csrc/host/host_ops.cpp) with this module's error
+  type. They return None, before doing anything, for calls that they do not cover."""
+  NAMES = ("linear", "multi_linear", "multi_linear_bwd", "gated_in", "gated_in_bwd", "rmsnorm",
+           "rmsnorm_bwd", "attention", "attention_bwd")
+
+  def __init__(self, module):
+    for name in self.NAMES:
+      setattr(self, name, self._wrap(getattr(module, name)))
+
+  @staticmethod
+  def _wrap(fn):
+    def call(*args):
+      try:
+        return fn(*args)
+      except RuntimeError as e:
+        if type(e) is RuntimeError:
+          raise NativeError(str(e)) from None
+        raise
+    return call
+
+
+_host = None
+
+
+def host():
+  """The compiled host path; None with `T5X_B200_HOST_OPS=0`. Like the kernel library it has to be
+  there on a machine with a GPU."""
+  global _host
+  if _host is None:
+    lib()  # the kernel library it is linked with
+    with _lock:
+      if _host is None:
+        if os.environ.get("T5X_B200_HOST_OPS", "1") == "0":
+          _host = False
+        else:
+          from t5x_b200.ops import build as _build
+          _host = _HostOps(_build.load_host())
+  return _host or None
+
+
 def launch_count() -> int:
   """Kernels launched by the native library so far in this process."""
   return int(lib().t5x_launch_count())
@@ -163,7 +204,7 @@ def _check(rc: int, what: str) -> None:
 
 
 def stream_ptr() -> int:
-  return torch.cuda.current_stream().cuda_stream
+  return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def ptr(t: Optional[torch.Tensor]) -> int:

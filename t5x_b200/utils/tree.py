@@ -1,7 +1,8 @@
 """Nested-dict ("pytree") helpers: the containers for params, optimizer state and caches."""
 from __future__ import annotations
 
-from typing import Any, Callable, Dict, Mapping, Tuple
+from collections.abc import Mapping
+from typing import Any, Callable, Dict, Tuple
 
 
 def is_leaf_default(x) -> bool:
@@ -13,8 +14,10 @@ def flatten_dict(tree: Mapping[str, Any], sep: str = "/", keep_empty_nodes: bool
   """{'a': {'b': x}} -> {'a/b': x} (flax.traverse_util.flatten_dict with a separator)."""
   out: Dict[str, Any] = {}
 
+  plain = is_leaf is is_leaf_default  # a plain dict is then a container without further tests
+
   def rec(prefix, node):
-    if isinstance(node, Mapping) and not is_leaf(node):
+    if (plain and type(node) is dict) or (isinstance(node, Mapping) and not is_leaf(node)):
       if not node and keep_empty_nodes and prefix:
         out[prefix] = {}
       for k, v in node.items():
