@@ -45,6 +45,8 @@ __device__ __forceinline__ float sum_over_row_groups(float x) {  // the 4 row gr
   return x;
 }
 
+// kFirst: positions per lane group whose key and value are held in registers (see below).
+template <int kFirst>
 __global__ void __launch_bounds__(kDecWarps * 32)
     decode_self_attention_kernel(const __nv_bfloat16* __restrict__ q,      // [rows, H, 64]
                                  const __nv_bfloat16* __restrict__ k_new,  // [rows, H, 64]
@@ -65,7 +67,6 @@ __global__ void __launch_bounds__(kDecWarps * 32)
   if (item >= rows * H) return;
   const int row = item / H, h = item - row * H;
   const int b = row / beams;
-  const int cur = min(max(*cur_index, 0), L - 1);
   const int g = lane >> 3, part = lane & 7;
   const long long rh = static_cast<long long>(row) * in_ld + h * kDecHeadDim;  // inputs
   const long long oh = (static_cast<long long>(row) * H + h) * kDecHeadDim;   // output
@@ -76,11 +77,39 @@ __global__ void __launch_bounds__(kDecWarps * 32)
                                static_cast<long long>(h) * L * kDecHeadDim;
   const int* anc = ancestry + static_cast<long long>(row) * L;
 
+  // With few (row, head) items the kernel is a chain of dependent loads, so with kFirst = 8 the
+  // chain is kept to two links: the position, the slots of the first 32 positions and this step's
+  // vectors together, then the keys AND values of those positions. Later positions are streamed
+  // below, and with kFirst = 0 all are.
+  constexpr int kU = 4;  // positions in flight per lane group in the streams
+  constexpr int kHeld = kFirst > 0 ? kFirst : 1;
+  int slot[kHeld];
+#pragma unroll
+  for (int u = 0; u < kFirst; ++u) {
+    const int t = u * 4 + g;
+    slot[u] = t < L ? anc[t] : 0;
+  }
+  const int cur = min(max(*cur_index, 0), L - 1);
   // 1. this step's query / key / value (8 dims per lane); append key / value at position
   //    `cur` of the row's own slot
   const uint4 qu = reinterpret_cast<const uint4*>(q + rh)[part];
   const uint4 kn = reinterpret_cast<const uint4*>(k_new + rh)[part];
   const uint4 vn = reinterpret_cast<const uint4*>(v_new + rh)[part];
+  uint4 kf4[kHeld], vf4[kHeld];
+  float bf[kHeld];
+#pragma unroll
+  for (int u = 0; u < kFirst; ++u) {
+    const int t = u * 4 + g;
+    kf4[u] = kn;
+    vf4[u] = vn;
+    bf[u] = 0.f;
+    if (t < cur) {
+      const long long at = batch_base + slot[u] * slot_stride + t * tstride;
+      kf4[u] = reinterpret_cast<const uint4*>(cache_k + at)[part];
+      vf4[u] = reinterpret_cast<const uint4*>(cache_v + at)[part];
+    }
+    if (bias_row != nullptr && t <= cur) bf[u] = bias_row[static_cast<long long>(h) * L + t];
+  }
   if (g == 0) {
     const long long dst = batch_base + (row - b * beams) * slot_stride + cur * tstride;
     reinterpret_cast<uint4*>(cache_k + dst)[part] = kn;
@@ -88,11 +117,27 @@ __global__ void __launch_bounds__(kDecWarps * 32)
   }
   float qf[8];
   unpack8(qu, qf);
+  auto dot = [&](const uint4& u) {
+    float kf[8];
+    unpack8(u, kf);
+    float s = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s = fmaf(qf[e], kf[e], s);
+    return sum_over_row_lanes(s);
+  };
 
   // 2. scores over positions 0..cur (no 1/sqrt(d): T5 folds it into the query init)
   float mx = -INFINITY;
-  constexpr int kU = 4;  // positions in flight per lane group
-  for (int t0 = 0; t0 <= cur; t0 += 4 * kU) {
+#pragma unroll
+  for (int u = 0; u < kFirst; ++u) {
+    const int t = u * 4 + g;
+    const float s = dot(kf4[u]) + bf[u];
+    if (t <= cur) {
+      if (part == 0) sprob[warp][t] = s;
+      mx = fmaxf(mx, s);
+    }
+  }
+  for (int t0 = 4 * kFirst; t0 <= cur; t0 += 4 * kU) {
     uint4 ku[kU];
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
@@ -105,12 +150,7 @@ __global__ void __launch_bounds__(kDecWarps * 32)
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       const int t = t0 + u * 4 + g;
-      float kf[8];
-      unpack8(ku[u], kf);
-      float s = 0.f;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) s = fmaf(qf[e], kf[e], s);
-      s = sum_over_row_lanes(s);
+      float s = dot(ku[u]);
       if (t <= cur) {
         if (bias_row != nullptr) s += bias_row[static_cast<long long>(h) * L + t];
         if (part == 0) sprob[warp][t] = s;
@@ -133,7 +173,18 @@ __global__ void __launch_bounds__(kDecWarps * 32)
   float acc[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-  for (int t0 = 0; t0 <= cur; t0 += 4 * kU) {
+#pragma unroll
+  for (int u = 0; u < kFirst; ++u) {
+    const int t = u * 4 + g;
+    if (t <= cur) {
+      const float pt = sprob[warp][t];
+      float vf[8];
+      unpack8(vf4[u], vf);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] = fmaf(pt, vf[e], acc[e]);
+    }
+  }
+  for (int t0 = 4 * kFirst; t0 <= cur; t0 += 4 * kU) {
     uint4 vu[kU];
     float pt[kU];
 #pragma unroll
@@ -201,6 +252,45 @@ __global__ void __launch_bounds__(kBeginThreads)
   for (int t = threadIdx.x; t < L; t += kBeginThreads)
     bias_row[static_cast<long long>(h) * L + t] =
         table[static_cast<long long>(h) * num_buckets + bucket_of_distance[max(cur - t, 0)]];
+}
+
+// Encoder keys and values [B, Lk, H, 64] in the layout of the tensor-core cross attention: keys
+// [B, H, Lp, 64], values transposed [B, H, 64, Lp], zero beyond Lk. One CTA per 64 keys of a
+// head; both sides move whole 128-byte rows, the values through shared memory. As tensor
+// operations this was two fills and two strided copies of 0.22 ms each per layer at 64 x 512
+// positions x 32 heads, against 0.08 ms for the bytes.
+constexpr int kLayoutThreads = 256;
+__global__ void __launch_bounds__(kLayoutThreads)
+    decode_cross_layout_kernel(const __nv_bfloat16* __restrict__ k,
+                               const __nv_bfloat16* __restrict__ v, __nv_bfloat16* __restrict__ kp,
+                               __nv_bfloat16* __restrict__ vt, int Lk, int Lp, int H) {
+  // [key][channel], the 16-byte pieces of a row permuted by key / 8: neither side has conflicts
+  __shared__ __align__(16) __nv_bfloat16 tile[64][64];
+  const int parts = (Lp + 63) / 64;
+  const int bh = blockIdx.x / parts, t0 = (blockIdx.x - bh * parts) * 64;
+  const int b = bh / H, h = bh - b * H;
+  const int piece = threadIdx.x & 7;
+  for (int r = threadIdx.x >> 3; r < 64; r += kLayoutThreads / 8) {
+    const int key = t0 + r;
+    uint4 ku = make_uint4(0u, 0u, 0u, 0u), vu = ku;
+    if (key < Lk) {
+      const long long at = ((static_cast<long long>(b) * Lk + key) * H + h) * 8 + piece;
+      ku = reinterpret_cast<const uint4*>(k)[at];
+      vu = reinterpret_cast<const uint4*>(v)[at];
+    }
+    if (key < Lp) reinterpret_cast<uint4*>(kp)[(static_cast<long long>(bh) * Lp + key) * 8 + piece] = ku;
+    *reinterpret_cast<uint4*>(&tile[r][(piece ^ (r >> 3)) * 8]) = vu;
+  }
+  __syncthreads();
+  // Lp is a multiple of 32: a row of the transposed tile is four or eight pieces of eight keys
+  if (t0 + piece * 8 >= Lp) return;
+  for (int c = threadIdx.x >> 3; c < 64; c += kLayoutThreads / 8) {
+    __align__(16) __nv_bfloat16 o[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[j] = tile[piece * 8 + j][((c >> 3) ^ piece) * 8 + (c & 7)];
+    *reinterpret_cast<uint4*>(vt + (static_cast<long long>(bh) * 64 + c) * Lp + t0 + piece * 8) =
+        *reinterpret_cast<const uint4*>(o);
+  }
 }
 
 constexpr int kCrossWarps = 8;
@@ -357,11 +447,27 @@ __global__ void __launch_bounds__(kCrossThreads, BEAMS <= 4 ? 4 : 2)
 
 using namespace t5x;
 
-// q, k_new, v_new: [rows, heads, 64] bf16 with row stride `in_ld` elements (views into one
-// fused projection are fine; 16-byte aligned), out: [rows, heads, 64] contiguous; rows =
-// batch * beams; cache_k / cache_v: [batch, beams, heads, max_len, 64] bf16; ancestry:
-// [batch, beams, max_len] int32; bias_row: [heads, max_len] fp32 or null; cur_index: device
-// int32 (position being decoded).
+// k, v [B, Lk, H, 64] bf16 contiguous; kp [B, H, Lp, 64], vt [B, H, 64, Lp], Lp a multiple of 32.
+T5X_API int t5x_decode_cross_layout(const void* k, const void* v, void* kp, void* vt, int B, int Lk,
+                                    int H, int Lp, void* stream) {
+  using namespace t5x;
+  if (B <= 0 || Lp <= 0 || H <= 0) return 0;
+  const long long blocks = static_cast<long long>((Lp + 63) / 64) * H * B;
+  if (Lp % 32 || Lp < Lk || blocks > 0x7fffffff)
+    return set_error("decode_cross_layout: B=%d H=%d Lk=%d Lp=%d is not covered", B, H, Lk, Lp);
+  if ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
+       reinterpret_cast<uintptr_t>(kp) | reinterpret_cast<uintptr_t>(vt)) & 15)
+    return set_error("decode_cross_layout: tensors must start on 16-byte boundaries");
+  decode_cross_layout_kernel<<<static_cast<unsigned>(blocks), kLayoutThreads, 0,
+                               static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v),
+      static_cast<__nv_bfloat16*>(kp), static_cast<__nv_bfloat16*>(vt), Lk, Lp, H);
+  count_launches(1);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return set_error("decode_cross_layout: %s", cudaGetErrorString(e));
+  return 0;
+}
+
 // live_seqs [rows, L] int64, cur_index device int32, emb [vocab, d] bf16 (d % 8 == 0, 16-byte
 // aligned), x [rows, d] bf16; table [H, num_buckets] fp32, bucket_of_distance [L] int32 in
 // [0, num_buckets), bias_row [H, L] fp32.
@@ -386,6 +492,11 @@ T5X_API int t5x_decode_begin(const void* live_seqs, const void* cur_index, const
   return 0;
 }
 
+// q, k_new, v_new: [rows, heads, 64] bf16 with row stride `in_ld` elements (views into one
+// fused projection are fine; 16-byte aligned), out: [rows, heads, 64] contiguous; rows =
+// batch * beams; cache_k / cache_v: [batch, beams, heads, max_len, 64] bf16; ancestry:
+// [batch, beams, max_len] int32; bias_row: [heads, max_len] fp32 or null; cur_index: device
+// int32 (position being decoded).
 T5X_API int t5x_decode_self_attention(const void* q, const void* k_new, const void* v_new,
                                       void* cache_k, void* cache_v, const void* ancestry,
                                       const void* bias_row, const void* cur_index, void* out,
@@ -397,8 +508,13 @@ T5X_API int t5x_decode_self_attention(const void* q, const void* k_new, const vo
   if (beams <= 0 || rows % beams) return set_error("decode_self_attention: rows %% beams != 0");
   if (in_ld % 8) return set_error("decode_self_attention: input row stride must be a multiple of 8");
   const int items = rows * heads;
+  // Up to 16 warps an SM the loads' latency counts, beyond that the warps hide it and the 118
+  // registers of the wide form cost occupancy. us, wide / narrow: 4 rows x 12 heads at position 40
+  // 5.5 / 7.2, 64 x 32 10.4 / 12.2, 256 rows x 32 heads over 64 steps 28.2 / 22.5.
+  auto kernel = items <= 16 * num_sms() ? decode_self_attention_kernel<8>
+                                        : decode_self_attention_kernel<0>;
   cudaError_t e = launch_chained(
-      decode_self_attention_kernel, dim3((items + kDecWarps - 1) / kDecWarps), dim3(kDecWarps * 32),
+      kernel, dim3((items + kDecWarps - 1) / kDecWarps), dim3(kDecWarps * 32),
       0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(q),
       static_cast<const __nv_bfloat16*>(k_new), static_cast<const __nv_bfloat16*>(v_new),
       static_cast<__nv_bfloat16*>(cache_k), static_cast<__nv_bfloat16*>(cache_v),

@@ -66,3 +66,15 @@ def test_decode_step_agrees_with_the_other_kernels(batch, beams):
       logits.append(d._model_step())
   scale = logits[1].abs().max()
   assert float((logits[0] - logits[1]).abs().max() / scale) < 0.03
+
+
+@pytest.mark.parametrize("b,lk,h", [(1, 1, 1), (2, 31, 3), (3, 33, 2), (2, 64, 4), (1, 129, 2)])
+def test_cross_layout(b, lk, h):
+  """A rearrangement: equal to the tensor-op statement bit by bit, the padding zero."""
+  from t5x_b200 import decoding_fast
+  k, v = (torch.randn(b, lk, h, 64, device="cuda").bfloat16() for _ in range(2))
+  kp, vt = decoding_fast.cross_kv_layout(k, v)
+  kc, vc = decoding_fast.cross_kv_layout(k.cpu(), v.cpu())
+  assert torch.equal(kp.cpu(), kc) and torch.equal(vt.cpu(), vc)
+  again = decoding_fast.cross_kv_layout(v, k, out=(kp, vt))
+  assert again[0] is kp and torch.equal(kp[:, :, :lk], v.transpose(1, 2))
