@@ -393,7 +393,7 @@ def gemm_skinny_splits(M: int, N: int, K: int) -> int:
 
 def gemm_skinny(a: torch.Tensor, b: torch.Tensor, *, residual: Optional[torch.Tensor] = None,
                 out: Optional[torch.Tensor] = None, splits: Optional[int] = None,
-                alpha: float = 1.0) -> Optional[torch.Tensor]:
+                alpha: float = 1.0, tile_n: int = 0) -> Optional[torch.Tensor]:
   """out[M, N] (bf16) = alpha * a[M, K] @ b[K, N] (+ residual) for few rows: K is cut over the
   CTAs of a thread-block cluster, which add their partial products through distributed shared
   memory and store finished bf16 rows (no workspace, no second kernel). `b` may be row-major
@@ -420,11 +420,12 @@ def gemm_skinny(a: torch.Tensor, b: torch.Tensor, *, residual: Optional[torch.Te
   assert out.stride(1) == 1 and out.stride(0) % 4 == 0 and out.dtype == torch.bfloat16
   l = lib()
   l.t5x_gemm_skinny_bf16.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-                                     c_ll, c_ll, c_ll, c_ll, c_int, c_int, c_float, c_void_p]
+                                     c_ll, c_ll, c_ll, c_ll, c_int, c_int, c_int, c_float,
+                                     c_void_p]
   _check(l.t5x_gemm_skinny_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), ptr(residual), M, N, K,
                                 a.stride(0), ldb, out.stride(0),
                                 residual.stride(0) if residual is not None else 0, b_mn, s,
-                                float(alpha), stream_ptr()), "gemm_skinny")
+                                tile_n, float(alpha), stream_ptr()), "gemm_skinny")
   return out
 
 

@@ -78,3 +78,24 @@ def test_cross_layout(b, lk, h):
   assert torch.equal(kp.cpu(), kc) and torch.equal(vt.cpu(), vc)
   again = decoding_fast.cross_kv_layout(v, k, out=(kp, vt))
   assert again[0] is kp and torch.equal(kp[:, :, :lk], v.transpose(1, 2))
+
+
+@pytest.mark.parametrize("m,k,n,splits,transposed,with_res", [
+    (256, 2048, 2048, 4, False, True), (37, 128, 384, 2, True, False),
+    (200, 1024, 256, 8, False, True), (128, 192, 128, 1, False, False), (1, 64, 128, 1, True, True),
+    (300, 512, 640, 2, True, True)])
+def test_skinny_with_half_width_tiles(m, k, n, splits, transposed, with_res):
+  """The cluster split-K GEMM with 128 x 64 tiles: every cluster size, rings that are not filled
+  and rings that wrap, both weight layouts, row tails. fp32 accumulation, one rounding to bf16
+  (2^-9 of a value), with a factor of two for the fp32 sums."""
+  from t5x_b200.ops import native
+  torch.manual_seed(m + k + n)
+  a = torch.randn(m, k, device="cuda").bfloat16()
+  w = (torch.randn(n, k, device="cuda") * 0.05).bfloat16().t() if transposed else \
+      (torch.randn(k, n, device="cuda") * 0.05).bfloat16()
+  res = torch.randn(m, n, device="cuda").bfloat16() if with_res else None
+  out = native.gemm_skinny(a, w, residual=res, splits=splits, tile_n=64)
+  native.check_status()
+  ref = a.double() @ w.double() + (0 if res is None else res.double())
+  assert float((out.double() - ref).abs().max() / ref.abs().max()) < 2 * 2.0 ** -9
+  assert torch.equal(out, native.gemm_skinny(a, w, residual=res, splits=splits, tile_n=64))
