@@ -480,8 +480,8 @@ int launch_stream(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMa
 using namespace t5x;
 
 // q [B,Lq,H,D], k/v [B,Lk,H,D] bf16 with element strides (sb, sl, sh), innermost contiguous,
-// D = 64 or 128, any Lq and Lk. rel_bias [H, nrel] fp32 or null: bias = rel_bias[h][(k - q) +
-// rel_off]. lse [B,H,Lq] fp32 or null.
+// D = 64 or 128, any Lq and Lk. rel_bias [H, num_buckets] fp32 or null, rel_bucket [nrel] int32:
+// bias = rel_bias[h][rel_bucket[(k - q) + rel_off]]. lse [B,H,Lq] fp32 or null.
 T5X_API int t5x_attention_fwd_stream(const void* q, const void* k, const void* v, void* o,
                                      void* lse, int B, int H, int Lq, int Lk, int D,
                                      long long q_sb, long long q_sl, long long q_sh,

@@ -2,6 +2,8 @@
 // residual gradient folded in), gated-GELU backward, embedding gather and its
 // scatter-add backward, and fp32->bf16 casts. All are written as grid-stride /
 // persistent loops sized from the SM count, with 16-byte vector accesses.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace t5x {
@@ -42,7 +44,8 @@ __device__ __forceinline__ Bf16x8 pack8(const float* f) {
 
 // ---------------------------------------------------------------------------
 // RMSNorm forward: y = x * rsqrt(mean(x^2) + eps) * scale      (fp32 statistics)
-// One CTA per row at a time (grid-stride over rows). d % 8 == 0.
+// One CTA per row at a time (grid-stride over rows): wide rows, and few of them; the others go
+// to rmsnorm_fwd_warp_kernel. d % 8 == 0.
 // ---------------------------------------------------------------------------
 constexpr int kNormThreads = 256;
 constexpr int kNormMaxVec = 4;  // up to 256*8*4 = 8192 features kept in registers
@@ -96,8 +99,33 @@ __global__ void __launch_bounds__(kNormThreads)
 // SM for d <= 4096: the kernel is bound by how many rows are in flight. The per-feature sums
 // for dscale are kept in registers over the CTA's rows and written to `partial`
 // ([gridDim.x, d], plain stores); rmsnorm_dscale_reduce_kernel adds them up.
+// The operands of one row of the backward pass, packed: thread `t` of THREADS holds 16-byte pieces
+// t, t + THREADS, ... of it. Loaded one row ahead of their use; the residual's gradient only
+// where the registers last for it (RES).
+template <int NV, int THREADS, bool RES>
+struct NormRow {
+  Bf16x8 x[NV], dy[NV], res[RES ? NV : 1];
+  float rstd;
+  __device__ __forceinline__ void load(const __nv_bfloat16* xs, const __nv_bfloat16* dys,
+                                       const __nv_bfloat16* ress, const float* rstds, int row, int d,
+                                       int t) {
+    const long long off = static_cast<long long>(row) * d;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int v = t + i * THREADS;
+      if (v < d / 8) {
+        x[i] = reinterpret_cast<const Bf16x8*>(xs + off)[v];
+        dy[i] = reinterpret_cast<const Bf16x8*>(dys + off)[v];
+        if (RES && ress) res[RES ? i : 0] = reinterpret_cast<const Bf16x8*>(ress + off)[v];
+      }
+    }
+    rstd = rstds[row];
+  }
+};
+constexpr int norm_bwd_ctas(int nv) { return nv <= 2 ? 4 : 2; }  // per SM
+
 template <int NV>
-__global__ void __launch_bounds__(kNormThreads, NV <= 2 ? 4 : 2)
+__global__ void __launch_bounds__(kNormThreads, norm_bwd_ctas(NV))
     rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                        const float* __restrict__ scale, const float* __restrict__ rstd_in,
                        const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
@@ -109,28 +137,27 @@ __global__ void __launch_bounds__(kNormThreads, NV <= 2 ? 4 : 2)
   for (int i = 0; i < NV; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) ds_acc[i][j] = 0.f;
+  // The next row is requested while this one is worked on, where the registers last for it (us,
+  // with / without, with a residual: 163840 x 2048 520 / 572, 16384 x 1472 49 / 56; but
+  // 8192 x 4096, two pieces a thread, 71 / 63).
+  constexpr bool kAhead = NV == 1;
+  NormRow<NV, kNormThreads, kAhead> next;
+  if (kAhead && blockIdx.x < rows) next.load(x, dy, dres, rstd_in, blockIdx.x, d, threadIdx.x);
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
+    if (!kAhead) next.load(x, dy, dres, rstd_in, row, d, threadIdx.x);
+    const NormRow<NV, kNormThreads, kAhead> cur = next;
+    if (kAhead && row + static_cast<int>(gridDim.x) < rows)
+      next.load(x, dy, dres, rstd_in, row + gridDim.x, d, threadIdx.x);
     const long long off = static_cast<long long>(row) * d;
-    const Bf16x8* xr = reinterpret_cast<const Bf16x8*>(x + off);
-    const Bf16x8* dyr = reinterpret_cast<const Bf16x8*>(dy + off);
-    Bf16x8 xp[NV], dyp[NV];
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {  // all loads of the row before the first use
-      const int v = threadIdx.x + i * kNormThreads;
-      if (v < nvec) {
-        xp[i] = xr[v];
-        dyp[i] = dyr[v];
-      }
-    }
-    const float rstd = rstd_in[row];
+    const float rstd = cur.rstd;
     float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int v = threadIdx.x + i * kNormThreads;
       if (v < nvec) {
         float xv[8], dyv[8];
-        unpack8(xp[i], xv);
-        unpack8(dyp[i], dyv);
+        unpack8(cur.x[i], xv);
+        unpack8(cur.dy[i], dyv);
         const float4 s0 = reinterpret_cast<const float4*>(scale)[2 * v];
         const float4 s1 = reinterpret_cast<const float4*>(scale)[2 * v + 1];
         const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
@@ -145,22 +172,22 @@ __global__ void __launch_bounds__(kNormThreads, NV <= 2 ? 4 : 2)
     const float tot = block_sum(dot, red);
     const float c = tot / static_cast<float>(d) * rstd * rstd;
     Bf16x8* dxr = reinterpret_cast<Bf16x8*>(dx + off);
-    const Bf16x8* rr = dres ? reinterpret_cast<const Bf16x8*>(dres + off) : nullptr;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int v = threadIdx.x + i * kNormThreads;
       if (v < nvec) {
         float xv[8], dyv[8], o[8];
-        unpack8(xp[i], xv);
-        unpack8(dyp[i], dyv);
+        unpack8(cur.x[i], xv);
+        unpack8(cur.dy[i], dyv);
         const float4 s0 = reinterpret_cast<const float4*>(scale)[2 * v];
         const float4 s1 = reinterpret_cast<const float4*>(scale)[2 * v + 1];
         const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = rstd * (dyv[j] * sc[j] - xv[j] * c);
-        if (rr) {
+        if (dres) {
           float r8[8];
-          unpack8(rr[v], r8);
+          unpack8(kAhead ? cur.res[kAhead ? i : 0]
+                         : reinterpret_cast<const Bf16x8*>(dres + off)[v], r8);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += r8[j];
         }
@@ -217,82 +244,124 @@ __global__ void __launch_bounds__(256)
 // ---------------------------------------------------------------------------
 constexpr int kNormWarpMaxVec = 4;  // 32 lanes x 4 vectors x 8 = 1024 features
 
-__global__ void __launch_bounds__(kNormThreads)
+// Forward, d <= 2048: a warp takes ROWS rows at a time and a lane holds NV 16-byte pieces of each,
+// packed, all requested before the first use; no barrier, and the scale is read once for the
+// ROWS rows. Bound by the bytes in flight: one CTA per row with its barriers takes 450 us for
+// 163840 x 2048 and 42.5 for 16384 x 1472, this 228 and 20.8.
+// The squares are added in the order of rmsnorm_fwd_kernel above 1024 features (piece i of the
+// lanes is what warp i of that kernel holds), so that a row's result does not depend on how many
+// rows there are.
+constexpr int kNormFwdThreads = 128;
+template <int NV, int ROWS>
+__global__ void __launch_bounds__(kNormFwdThreads)
     rmsnorm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ scale,
                             __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, int rows,
                             int d, float eps) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nvec = d / 8;
-  const int wpb = kNormThreads / 32;
-  for (int row = blockIdx.x * wpb + warp; row < rows; row += gridDim.x * wpb) {
-    const Bf16x8* xr = reinterpret_cast<const Bf16x8*>(x + static_cast<long long>(row) * d);
-    float vals[kNormWarpMaxVec][8];
-    float ss = 0.f;
+  const long long first = (static_cast<long long>(blockIdx.x) * (kNormFwdThreads / 32) + warp) * ROWS;
+  if (first >= rows) return;
+  const int n = static_cast<int>(min(static_cast<long long>(ROWS), rows - first));
+  Bf16x8 u[ROWS][NV];
 #pragma unroll
-    for (int i = 0; i < kNormWarpMaxVec; ++i) {
+  for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
       const int v = lane + i * 32;
-      if (v < nvec) {
-        unpack8(xr[v], vals[i]);
+      if (r < n && v < nvec)
+        u[r][i] = reinterpret_cast<const Bf16x8*>(x + (first + r) * d)[v];
+    }
+  float rstd[ROWS];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ss += vals[i][j] * vals[i][j];
+  for (int r = 0; r < ROWS; ++r) {
+    float part[8] = {};
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      float& ss = part[NV <= kNormWarpMaxVec ? 0 : i];
+      if (r < n && lane + i * 32 < nvec) {
+        float f[8];
+        unpack8(u[r][i], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
       }
     }
-    ss = warp_sum(ss);
-    const float rstd = rsqrtf(ss / static_cast<float>(d) + eps);
-    if (lane == 0 && rstd_out) rstd_out[row] = rstd;
-    Bf16x8* yr = reinterpret_cast<Bf16x8*>(y + static_cast<long long>(row) * d);
+    float ss;
+    if constexpr (NV <= kNormWarpMaxVec) {
+      ss = warp_sum(part[0]);
+    } else {
 #pragma unroll
-    for (int i = 0; i < kNormWarpMaxVec; ++i) {
-      const int v = lane + i * 32;
-      if (v < nvec) {
-        const float4 s0 = reinterpret_cast<const float4*>(scale)[2 * v];
-        const float4 s1 = reinterpret_cast<const float4*>(scale)[2 * v + 1];
-        const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-        float o[8];
+      for (int i = 0; i < NV; ++i) part[i] = warp_sum(part[i]);
+      ss = ((part[0] + part[4]) + (part[2] + part[6])) +
+           ((part[1] + part[5]) + (part[3] + part[7]));
+    }
+    rstd[r] = rsqrtf(ss / static_cast<float>(d) + eps);
+    if (lane == 0 && r < n && rstd_out) rstd_out[first + r] = rstd[r];
+  }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = vals[i][j] * rstd * sc[j];
-        yr[v] = pack8(o);
+  for (int i = 0; i < NV; ++i) {
+    const int v = lane + i * 32;
+    if (v >= nvec) break;
+    const float4 s0 = __ldg(reinterpret_cast<const float4*>(scale) + 2 * v);
+    const float4 s1 = __ldg(reinterpret_cast<const float4*>(scale) + 2 * v + 1);
+    const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      if (r < n) {
+        float f[8];
+        unpack8(u[r][i], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd[r] * sc[j];
+        reinterpret_cast<Bf16x8*>(y + (first + r) * d)[v] = pack8(f);
       }
     }
   }
 }
 
-__global__ void __launch_bounds__(kNormThreads)
+template <int NV, int ROWS>
+static void launch_rmsnorm_fwd(const void* x, const void* scale, void* y, void* rstd, int rows, int d,
+                               float eps, cudaStream_t st) {
+  const int per_cta = kNormFwdThreads / 32 * ROWS;
+  rmsnorm_fwd_warp_kernel<NV, ROWS><<<(rows + per_cta - 1) / per_cta, kNormFwdThreads, 0, st>>>(
+      static_cast<const __nv_bfloat16*>(x), static_cast<const float*>(scale),
+      static_cast<__nv_bfloat16*>(y), static_cast<float*>(rstd), rows, d, eps);
+}
+
+// AHEAD: the next row is requested while this one is worked on (us, with / without, with a
+// residual: 65536 x 768 87 / 91, 14592 x 768 25 / 28; a few hundred rows of 768 0.5 us slower,
+// and with the fourth piece of 1024 features it spills, 8192 x 1024 30 / 23).
+template <int NV, bool kAhead>
+__global__ void __launch_bounds__(kNormThreads, 2)
     rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                             const float* __restrict__ scale, const float* __restrict__ rstd_in,
                             const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                             float* __restrict__ partial, int rows, int d) {
-  __shared__ float sacc[kNormThreads / 32][kNormWarpMaxVec * 32 * 8 / 4];  // one quarter at a time
+  __shared__ float sacc[kNormThreads / 32][256];  // one quarter at a time
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nvec = d / 8;
   const int wpb = kNormThreads / 32;
-  float ds_acc[kNormWarpMaxVec][8];
+  float ds_acc[NV][8];
 #pragma unroll
-  for (int i = 0; i < kNormWarpMaxVec; ++i)
+  for (int i = 0; i < NV; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) ds_acc[i][j] = 0.f;
-  for (int row = blockIdx.x * wpb + warp; row < rows; row += gridDim.x * wpb) {
+  const int step = gridDim.x * wpb;
+  NormRow<NV, 32, kAhead> next;
+  if (kAhead && blockIdx.x * wpb + warp < rows)
+    next.load(x, dy, dres, rstd_in, blockIdx.x * wpb + warp, d, lane);
+  for (int row = blockIdx.x * wpb + warp; row < rows; row += step) {
+    if (!kAhead) next.load(x, dy, dres, rstd_in, row, d, lane);
+    const NormRow<NV, 32, kAhead> cur = next;
+    if (kAhead && row + step < rows) next.load(x, dy, dres, rstd_in, row + step, d, lane);
     const long long off = static_cast<long long>(row) * d;
-    const Bf16x8* xr = reinterpret_cast<const Bf16x8*>(x + off);
-    const Bf16x8* dyr = reinterpret_cast<const Bf16x8*>(dy + off);
-    Bf16x8 xp[kNormWarpMaxVec], dyp[kNormWarpMaxVec];
-#pragma unroll
-    for (int i = 0; i < kNormWarpMaxVec; ++i) {
-      const int v = lane + i * 32;
-      if (v < nvec) {
-        xp[i] = xr[v];
-        dyp[i] = dyr[v];
-      }
-    }
-    const float rstd = rstd_in[row];
+    const float rstd = cur.rstd;
     float dot = 0.f;
 #pragma unroll
-    for (int i = 0; i < kNormWarpMaxVec; ++i) {
+    for (int i = 0; i < NV; ++i) {
       const int v = lane + i * 32;
       if (v < nvec) {
         float xv[8], dyv[8];
-        unpack8(xp[i], xv);
-        unpack8(dyp[i], dyv);
+        unpack8(cur.x[i], xv);
+        unpack8(cur.dy[i], dyv);
         const float4 s0 = reinterpret_cast<const float4*>(scale)[2 * v];
         const float4 s1 = reinterpret_cast<const float4*>(scale)[2 * v + 1];
         const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
@@ -307,22 +376,22 @@ __global__ void __launch_bounds__(kNormThreads)
     dot = warp_sum(dot);
     const float c = dot / static_cast<float>(d) * rstd * rstd;
     Bf16x8* dxr = reinterpret_cast<Bf16x8*>(dx + off);
-    const Bf16x8* rr = dres ? reinterpret_cast<const Bf16x8*>(dres + off) : nullptr;
 #pragma unroll
-    for (int i = 0; i < kNormWarpMaxVec; ++i) {
+    for (int i = 0; i < NV; ++i) {
       const int v = lane + i * 32;
       if (v < nvec) {
         float xv[8], dyv[8], o[8];
-        unpack8(xp[i], xv);
-        unpack8(dyp[i], dyv);
+        unpack8(cur.x[i], xv);
+        unpack8(cur.dy[i], dyv);
         const float4 s0 = reinterpret_cast<const float4*>(scale)[2 * v];
         const float4 s1 = reinterpret_cast<const float4*>(scale)[2 * v + 1];
         const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = rstd * (dyv[j] * sc[j] - xv[j] * c);
-        if (rr) {
+        if (dres) {
           float r8[8];
-          unpack8(rr[v], r8);
+          unpack8(kAhead ? cur.res[kAhead ? i : 0]
+                         : reinterpret_cast<const Bf16x8*>(dres + off)[v], r8);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += r8[j];
         }
@@ -335,7 +404,7 @@ __global__ void __launch_bounds__(kNormThreads)
     // vector slot (32 lanes x 8 features) at a time
     float* out = partial + static_cast<long long>(blockIdx.x) * d;
 #pragma unroll
-    for (int i = 0; i < kNormWarpMaxVec; ++i) {
+    for (int i = 0; i < NV; ++i) {
       __syncthreads();
 #pragma unroll
       for (int j = 0; j < 8; ++j) sacc[warp][lane * 8 + j] = ds_acc[i][j];
@@ -561,18 +630,29 @@ T5X_API int t5x_rmsnorm_fwd(const void* x, const void* scale, void* y, void* rst
   if (d % 8 || d > kNormThreads * 8 * kNormMaxVec)
     return set_error("rmsnorm: d=%d must be a multiple of 8 and <= %d", d,
                      kNormThreads * 8 * kNormMaxVec);
-  if (d <= kNormWarpMaxVec * 32 * 8) {  // narrow rows: one warp per row
-    const int wpb = kNormThreads / 32;
-    int blocks = (rows + wpb - 1) / wpb;
-    if (blocks > num_sms() * 8) blocks = num_sms() * 8;
-    rmsnorm_fwd_warp_kernel<<<blocks, kNormThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<const float*>(scale),
-        static_cast<__nv_bfloat16*>(y), static_cast<float*>(rstd), rows, d, eps);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // Wide rows need enough of them for the warp kernel (us, warp / CTA per row: 4096 x 2048
+  // 9.0 / 13.6, 256 x 2048 5.5 / 2.3).
+  if (d <= 1024 || (d <= 2048 && rows >= 16 * num_sms())) {
+    // two rows per warp share the scale where there are enough rows for every SM
+    const bool two = rows >= 64 * num_sms();
+    if (d <= 768)
+      two ? launch_rmsnorm_fwd<3, 2>(x, scale, y, rstd, rows, d, eps, st)
+          : launch_rmsnorm_fwd<3, 1>(x, scale, y, rstd, rows, d, eps, st);
+    else if (d <= 1024)
+      two ? launch_rmsnorm_fwd<4, 2>(x, scale, y, rstd, rows, d, eps, st)
+          : launch_rmsnorm_fwd<4, 1>(x, scale, y, rstd, rows, d, eps, st);
+    else if (d <= 1536)
+      two ? launch_rmsnorm_fwd<6, 2>(x, scale, y, rstd, rows, d, eps, st)
+          : launch_rmsnorm_fwd<6, 1>(x, scale, y, rstd, rows, d, eps, st);
+    else
+      two ? launch_rmsnorm_fwd<8, 2>(x, scale, y, rstd, rows, d, eps, st)
+          : launch_rmsnorm_fwd<8, 1>(x, scale, y, rstd, rows, d, eps, st);
     CHECK_LAUNCH("rmsnorm_fwd");
     return 0;
   }
   int grid = rows < num_sms() * 8 ? rows : num_sms() * 8;
-  rmsnorm_fwd_kernel<<<grid, kNormThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  rmsnorm_fwd_kernel<<<grid, kNormThreads, 0, st>>>(
       static_cast<const __nv_bfloat16*>(x), static_cast<const float*>(scale),
       static_cast<__nv_bfloat16*>(y), static_cast<float*>(rstd), rows, d, eps);
   CHECK_LAUNCH("rmsnorm_fwd");
@@ -598,7 +678,7 @@ T5X_API int t5x_rmsnorm_bwd(const void* dy, const void* x, const void* scale, co
       return set_error("rmsnorm_bwd: workspace allocation failed");
   }
   const int nv = d <= 2048 ? 1 : (d <= 4096 ? 2 : 4);
-  int grid = num_sms() * (nv <= 2 ? 4 : 2);
+  int grid = num_sms() * norm_bwd_ctas(nv);
   if (grid > rows) grid = rows;
   if (grid > kMaxParts) grid = kMaxParts;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -612,9 +692,12 @@ T5X_API int t5x_rmsnorm_bwd(const void* dy, const void* x, const void* scale, co
   if (d <= kNormWarpMaxVec * 32 * 8) {  // narrow rows: one warp per row, eight rows per CTA
     const int wpb = kNormThreads / 32;
     grid = (rows + wpb - 1) / wpb;
-    if (grid > num_sms() * 4) grid = num_sms() * 4;
-    if (grid > kMaxParts) grid = kMaxParts;
-    launch(rmsnorm_bwd_warp_kernel);
+    const bool ahead = d <= 768 && rows >= 8192;
+    const int most = std::min(num_sms() * (ahead ? 2 : 4), kMaxParts);
+    if (grid > most) grid = most;
+    if (!ahead) launch(rmsnorm_bwd_warp_kernel<4, false>);
+    else if (d <= 512) launch(rmsnorm_bwd_warp_kernel<2, true>);
+    else launch(rmsnorm_bwd_warp_kernel<3, true>);
   } else if (nv == 1) launch(rmsnorm_bwd_kernel<1>);
   else if (nv == 2) launch(rmsnorm_bwd_kernel<2>);
   else launch(rmsnorm_bwd_kernel<4>);
