@@ -409,6 +409,45 @@ __global__ void __launch_bounds__(256)
 // tiles are twice as large and dK, dV take twice the TMEM columns, so Q / dO have one stage, dQ
 // reuses the columns of S^T and the query blocks run one after the other.
 constexpr int kSmemBuckets = 128;  // tables with more buckets add to memory directly
+// P and dS of 16 scores of one key that all count: rel points at the bias of the first, the next
+// ones lie below it.
+template <bool kBias>
+__device__ __forceinline__ void visible_scores(const uint32_t (&sv)[16], const uint32_t (&dpv)[16],
+                                               const float* rel, const float (&lse)[16],
+                                               const float (&delta)[16], float (&pr)[16],
+                                               float (&ds)[16]) {
+#pragma unroll
+  for (int x = 0; x < 16; ++x) {
+    float s = __uint_as_float(sv[x]);
+    if (kBias) s += rel[-x];
+    s = fmaxf(s, kMaskValue);
+    pr[x] = exp2f(fmaf(s, kLog2e, -lse[x]));
+    ds[x] = pr[x] * (__uint_as_float(dpv[x]) - delta[x]);
+  }
+}
+
+// The 4 x 4 transpose of 16-byte pieces among four adjacent lanes: lane j brings pieces 0..3 of its
+// row and leaves with piece j of the four rows, in order of the lanes.
+__device__ __forceinline__ void transpose_pieces(uint32_t* v, int lane) {
+  const bool odd = lane & 1, high = lane & 2;
+#pragma unroll
+  for (int c = 0; c < 16; c += 8)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {  // pieces c / 4 and c / 4 + 1 with the neighbour
+      const uint32_t a = v[c + e], b = v[c + 4 + e];
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+      v[c + e] = odd ? got : a;
+      v[c + 4 + e] = odd ? b : got;
+    }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {  // the pairs with the lane two away
+    const uint32_t a = v[c], b = v[c + 8];
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, high ? a : b, 2);
+    v[c] = high ? got : a;
+    v[c + 8] = high ? b : got;
+  }
+}
+
 template <int D>
 struct BwdSmem {
   static constexpr int kTile = 128 * 128;  // bytes of a [128 x 64] bf16 panel
@@ -711,16 +750,24 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_dq_read);
       }
-      const int q = blk * 128 + r;
-      if (q < p.Lq) {
-        float* dst = p.dQ + ((static_cast<long long>(b) * p.Lq + q) * p.H + h) * D +
-                     part * kColsPerPart;
+      // Four lanes exchange their 16-byte pieces, so that an instruction adds 64 contiguous bytes
+      // of 8 rows instead of 16 of 32 (128 x 12 heads x 512 x 512 1009 / 976 us).
+      const int q0 = blk * 128 + quarter * 32 + (lane & ~3);
+      float* dst = p.dQ + ((static_cast<long long>(b) * p.Lq + q0) * p.H + h) * D +
+                   part * kColsPerPart + (lane & 3) * 4;
+      const long long row_step = static_cast<long long>(p.H) * D;
 #pragma unroll
-        for (int x = 0; x < kColsPerPart; x += 4)
-          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + x),
-                       "f"(__uint_as_float(v[x])), "f"(__uint_as_float(v[x + 1])),
-                       "f"(__uint_as_float(v[x + 2])), "f"(__uint_as_float(v[x + 3]))
-                       : "memory");
+      for (int x = 0; x < kColsPerPart; x += 16) {
+        transpose_pieces(v + x, lane);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (q0 + i < p.Lq)
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(
+                             dst + i * row_step + x),
+                         "f"(__uint_as_float(v[x + 4 * i])), "f"(__uint_as_float(v[x + 4 * i + 1])),
+                         "f"(__uint_as_float(v[x + 4 * i + 2])),
+                         "f"(__uint_as_float(v[x + 4 * i + 3]))
+                         : "memory");
       }
     };
 
@@ -757,10 +804,13 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       // 16 columns (queries) at a time keeps the working set in registers: scores and dP of
       // the chunk, its per-query statistics, and the packed bf16 results.
       const float* rel = sRel + (r - col0 + 127);
-      const bool interior = simple_mask && k0 + 128 <= p.Lk && qb + 128 <= p.Lq;
-      // interior tile with a key-only mask: the mask is one additive constant per thread
-      // (-1e10 absorbs any score: |s| is far below the fp32 spacing at 1e10)
-      const float madd = kvis ? 0.f : kMaskValue;
+      // The kernel is bound by the instructions per score (42 with every case in one body, at half
+      // of the issue slots). Where all of a warp's 32 x 32 block counts, and no query in it has all
+      // its keys hidden, it takes a body without any of those cases (us: 128 x 12 heads x 512 x 512
+      // 976 / 925, 8 x 32 x 1024 x 1024 of 128 features 880 / 805).
+      const bool fast = qb + col0 + 32 <= p.Lq &&
+                        __all_sync(0xffffffffu,
+                                   mv == 0xffffffffu && sLse[col0 + lane] >= -5e9f);
       uint8_t* pt_tile = sPT + (part >> 1) * Smem::kTile;
       uint8_t* dst_tile = sDST + (part >> 1) * Smem::kTile;
       // Bias gradient: dS[key r][query c] belongs to bin (r - c). Within the warp's 32 x 32
@@ -794,23 +844,26 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           del_c[4 * g] = d.x, del_c[4 * g + 1] = d.y, del_c[4 * g + 2] = d.z, del_c[4 * g + 3] = d.w;
         }
         float pr[16], ds[16];
+        if (fast) {
+          if (has_bias)
+            visible_scores<true>(sv, dpv, rel - hc * 16, lse_c, del_c, pr, ds);
+          else
+            visible_scores<false>(sv, dpv, rel, lse_c, del_c, pr, ds);
+        } else {
 #pragma unroll
-        for (int x = 0; x < 16; ++x) {
-          const int xx = hc * 16 + x;
-          float s = __uint_as_float(sv[x]);
-          if (has_bias) s += rel[-xx];
-          if (interior) {
-            s = fmaxf(s + madd, kMaskValue);
-          } else {
+          for (int x = 0; x < 16; ++x) {
+            const int xx = hc * 16 + x;
+            float s = __uint_as_float(sv[x]);
+            if (has_bias) s += rel[-xx];
             s = ((mv >> xx) & 1u) ? s : kMaskValue;
+            float e = exp2f(fmaf(s, kLog2e, -lse_c[x]));
+            // A row with every key masked has lse = -1e10 + log(Lk), which fp32 rounds to -1e10:
+            // its probabilities are uniform over the Lk keys.
+            if (lse_c[x] < -5e9f) e = inv_lk;
+            if (!k_ok || qb + col0 + xx >= p.Lq) e = 0.f;
+            pr[x] = e;
+            ds[x] = e * (__uint_as_float(dpv[x]) - del_c[x]);
           }
-          float e = exp2f(fmaf(s, kLog2e, -lse_c[x]));
-          // A row with every key masked has lse = -1e10 + log(Lk), which fp32 rounds to -1e10:
-          // its probabilities are uniform over the Lk keys.
-          if (lse_c[x] < -5e9f) e = inv_lk;
-          if (!interior && (!k_ok || qb + col0 + xx >= p.Lq)) e = 0.f;
-          pr[x] = e;
-          ds[x] = e * (__uint_as_float(dpv[x]) - del_c[x]);
         }
         if (want_drel) {
 #pragma unroll

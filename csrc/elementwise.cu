@@ -247,7 +247,7 @@ constexpr int kNormWarpMaxVec = 4;  // 32 lanes x 4 vectors x 8 = 1024 features
 // Forward, d <= 2048: a warp takes ROWS rows at a time and a lane holds NV 16-byte pieces of each,
 // packed, all requested before the first use; no barrier, and the scale is read once for the
 // ROWS rows. Bound by the bytes in flight: one CTA per row with its barriers takes 450 us for
-// 163840 x 2048 and 42.5 for 16384 x 1472, this 228 and 20.8.
+// 163840 x 2048 and 42.5 for 16384 x 1472, this 247 and 21.9.
 // The squares are added in the order of rmsnorm_fwd_kernel above 1024 features (piece i of the
 // lanes is what warp i of that kernel holds), so that a row's result does not depend on how many
 // rows there are.
@@ -632,7 +632,7 @@ T5X_API int t5x_rmsnorm_fwd(const void* x, const void* scale, void* y, void* rst
                      kNormThreads * 8 * kNormMaxVec);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // Wide rows need enough of them for the warp kernel (us, warp / CTA per row: 4096 x 2048
-  // 9.0 / 13.6, 256 x 2048 5.5 / 2.3).
+  // 9.5 / 13.6, 256 x 2048 5.5 / 2.3).
   if (d <= 1024 || (d <= 2048 && rows >= 16 * num_sms())) {
     // two rows per warp share the scale where there are enough rows for every SM
     const bool two = rows >= 64 * num_sms();

@@ -211,3 +211,34 @@ def test_bias_gradient_by_bucket(buckets, lq, lk, main_grad):
   want = 2 * want_table.grad
   assert float((got - want).norm() / want.norm()) < 1e-2
   assert (table.grad is None) == main_grad
+
+
+@pytest.mark.parametrize("lq,lk,d,masked", [(32, 32, 64, False), (31, 129, 64, False),
+                                            (95, 128, 64, True), (160, 160, 64, True),
+                                            (129, 300, 128, True), (64, 96, 128, False)])
+def test_backward_of_whole_and_partial_blocks(lq, lk, d, masked):
+  """Warps whose 32 x 32 block counts in full beside warps that hold a hidden key, the end of the
+  queries or the end of the keys, and an example without a visible key. TOL as above: P and dS are
+  rounded to bf16 (2^-9 of each value), the rest is fp32."""
+  from t5x_b200.ops import attention as A
+  from t5x_b200.ops import native
+  from t5x_b200.ops import reference as ref
+  g = torch.Generator(device="cuda").manual_seed(lq * 7 + lk)
+  leaf = lambda l: (torch.randn(3, l, 2, d, device="cuda", generator=g) * 0.5).bfloat16()
+  q, k, v = (leaf(l).requires_grad_() for l in (lq, lk, lk))
+  table = torch.randn(2, 32, device="cuda", generator=g).requires_grad_()
+  mask = None
+  if masked:
+    mask = torch.ones(3, lk, dtype=torch.bool, device="cuda")
+    mask[0, 37] = False
+    mask[1] = False
+  do = leaf(lq)
+  got = torch.autograd.grad(A.flash_attention(q, k, v, bias_table=table, key_mask=mask),
+                            (q, k, v, table), do)
+  native.check_status()
+  want = torch.autograd.grad(
+      ref.attention(q.float(), k.float(), v.float(), key_mask=mask,
+                    bias=ref.relative_position_bias(table, lq, lk, True)),
+      (q, k, v, table), do.float())
+  for n, a, b in zip(("dq", "dk", "dv", "dbias"), got, want):
+    assert rel(a, b) < TOL, (n, rel(a, b))
