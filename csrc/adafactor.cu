@@ -25,14 +25,35 @@ constexpr int kAfTileR = 64;
 constexpr int kAfTileC = 512;
 
 // One 64 x 512 tile (tile_x, tile_y) of batch element b: row and column sums of g^2 + eps1, sum p^2.
-template <bool VEC>
+// Sums that meet in memory by atomic adds (F: their type, S: the struct of the scalar ones). In
+// fp32 their order shows in the last bit of every parameter; grouped launches hold them in fp64,
+// where it does not survive the rounding to fp32.
+struct AfScalars64 {  // per batch element, in scratch
+  double psq, usq;
+  float vsum, pad[3];
+};
+__device__ __forceinline__ AdafactorScalars af_rounded(const AdafactorScalars& s) { return s; }
+__device__ __forceinline__ AdafactorScalars af_rounded(const AfScalars64& s) {
+  AdafactorScalars r = {};
+  r.psq = static_cast<float>(s.psq);
+  r.usq = static_cast<float>(s.usq);
+  r.vsum = s.vsum;
+  return r;
+}
+
+// One slot per warp and column of a tile, for the column sums.
+__device__ __forceinline__ float (*af_column_slots())[kAfTileC] {
+  __shared__ float slots[kAfThreads / 32][kAfTileC];
+  return slots;
+}
+
+template <bool VEC, class F, class S>
 __device__ __forceinline__ void af_stats_tile(const float* __restrict__ g,
                                               const float* __restrict__ p,
-                                              float* __restrict__ rowsum,
-                                              float* __restrict__ colsum,
-                                              AdafactorScalars* __restrict__ scal, int R, int C,
-                                              float eps1, int tile_x, int tile_y, int b) {
-  __shared__ float scol[kAfTileC];
+                                              F* __restrict__ rowsum, F* __restrict__ colsum,
+                                              S* __restrict__ scal, int R, int C, float eps1,
+                                              int tile_x, int tile_y, int b) {
+  float (*scol)[kAfTileC] = af_column_slots();
   __shared__ float red[32];
   const long long base = static_cast<long long>(b) * R * C;
   g += base;
@@ -41,8 +62,6 @@ __device__ __forceinline__ void af_stats_tile(const float* __restrict__ g,
   colsum += static_cast<long long>(b) * C;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tile_r = tile_y * kAfTileR, tile_c = tile_x * kAfTileC;
-  for (int i = threadIdx.x; i < kAfTileC; i += kAfThreads) scol[i] = 0.f;
-  __syncthreads();
   float cacc[4][4];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
@@ -78,7 +97,7 @@ __device__ __forceinline__ void af_stats_tile(const float* __restrict__ g,
           psq += pv.x * pv.x + pv.y * pv.y + pv.z * pv.z + pv.w * pv.w;
         }
         rs = warp_sum(rs);
-        if (lane == 0) atomicAdd(&rowsum[row + u], rs);
+        if (lane == 0) atomicAdd(&rowsum[row + u], static_cast<F>(rs));
       }
     }
   } else
@@ -117,22 +136,27 @@ __device__ __forceinline__ void af_stats_tile(const float* __restrict__ g,
       }
     }
     rs = warp_sum(rs);
-    if (lane == 0) atomicAdd(&rowsum[row], rs);
+    if (lane == 0) atomicAdd(&rowsum[row], static_cast<F>(rs));
   }
 #pragma unroll
   for (int ch = 0; ch < 4; ++ch)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) atomicAdd(&scol[ch * 128 + lane * 4 + k], cacc[ch][k]);
+    for (int k = 0; k < 4; ++k) scol[warp][ch * 128 + lane * 4 + k] = cacc[ch][k];
   __syncthreads();
   for (int i = threadIdx.x; i < kAfTileC; i += kAfThreads)
-    if (tile_c + i < C) atomicAdd(&colsum[tile_c + i], scol[i]);
+    if (tile_c + i < C) {
+      float t = 0.f;
+#pragma unroll
+      for (int w = 0; w < kAfThreads / 32; ++w) t += scol[w][i];
+      atomicAdd(&colsum[tile_c + i], static_cast<F>(t));
+    }
   psq = warp_sum(psq);
   if (lane == 0) red[warp] = psq;
   __syncthreads();
   if (threadIdx.x == 0) {
     float t = 0.f;
     for (int w = 0; w < kAfThreads / 32; ++w) t += red[w];
-    atomicAdd(&scal[b].psq, t);
+    atomicAdd(&scal[b].psq, static_cast<F>(t));
   }
 }
 
@@ -148,10 +172,10 @@ __global__ void __launch_bounds__(kAfThreads)
 // vector indexed by matrix rows is the one divided by its mean (T5X "v_row"); otherwise the
 // column-indexed vector is. row_div / col_div are the GLOBAL column / row counts (the means are
 // over the unsharded dims); the local sums were combined across ranks beforehand if needed.
+template <class F, class S>
 __device__ __forceinline__ void af_ema(float* __restrict__ v_rvec, float* __restrict__ v_cvec,
-                                       const float* __restrict__ rowsum,
-                                       const float* __restrict__ colsum,
-                                       AdafactorScalars* __restrict__ scal, int R, int C,
+                                       const F* __restrict__ rowsum, const F* __restrict__ colsum,
+                                       S* __restrict__ scal, int R, int C,
                                        float row_div, float col_div, float decay,
                                        int row_is_normalized, int skip_nan, int b) {
   __shared__ float red[32];
@@ -163,14 +187,14 @@ __device__ __forceinline__ void af_ema(float* __restrict__ v_rvec, float* __rest
   float acc = 0.f;
   for (int i = threadIdx.x; i < R; i += blockDim.x) {
     const float old = v_rvec[i];
-    float nv = decay * old + mix * (rowsum[i] / row_div);
+    float nv = decay * old + mix * (static_cast<float>(rowsum[i]) / row_div);
     if (skip_nan && isnan(nv)) nv = old;
     v_rvec[i] = nv;
     if (row_is_normalized) acc += nv;
   }
   for (int i = threadIdx.x; i < C; i += blockDim.x) {
     const float old = v_cvec[i];
-    float nv = decay * old + mix * (colsum[i] / col_div);
+    float nv = decay * old + mix * (static_cast<float>(colsum[i]) / col_div);
     if (skip_nan && isnan(nv)) nv = old;
     v_cvec[i] = nv;
     if (!row_is_normalized) acc += nv;
@@ -196,9 +220,10 @@ __global__ void __launch_bounds__(1024)
 
 // Factor vectors from the updated moments: (v_row / mean(v_row))^-1/2 and v_col^-1/2.
 // norm_count = GLOBAL length of the normalised vector.
+template <class S>
 __device__ __forceinline__ void af_finalize(const float* v_rvec, const float* v_cvec,
                                             float* __restrict__ rf, float* __restrict__ cf,
-                                            const AdafactorScalars* scal, int R, int C,
+                                            const S* scal, int R, int C,
                                             float norm_count, int row_is_normalized, int b) {
   v_rvec += static_cast<long long>(b) * R;
   v_cvec += static_cast<long long>(b) * C;
@@ -246,16 +271,16 @@ __global__ void __launch_bounds__(kAfThreads)
 }
 
 // FACTORED: u = g * rf[r] * cf[c].  !FACTORED: u = g * rsqrt(v) with v already updated.
-template <bool FACTORED>
+template <bool FACTORED, class S>
 __device__ __forceinline__ void af_apply_elements(
     float* __restrict__ p, const float* __restrict__ g, const float* __restrict__ rf,
     const float* __restrict__ cf, const float* __restrict__ v, float* __restrict__ m,
     __nv_bfloat16* __restrict__ p_bf16, long long ld_bf16, long long bf16_batch_stride,
-    const AdafactorScalars* __restrict__ scal, int R, int C, float n_global, const AfHyper& h,
-    int block, int blocks, int b) {
+    const S* __restrict__ scal, int R, int C, float n_global, const AfHyper& h, int block, int blocks,
+    int b) {
   const long long n = static_cast<long long>(R) * C;
   const long long base = static_cast<long long>(b) * n;
-  const float scale = af_update_scale(scal[b], n_global, h);
+  const float scale = af_update_scale(af_rounded(scal[b]), n_global, h);
   if (FACTORED) {
     rf += static_cast<long long>(b) * R;
     cf += static_cast<long long>(b) * C;
@@ -293,10 +318,10 @@ __global__ void __launch_bounds__(kAfThreads)
 }
 
 // Unfactored pass 1: v <- decay v + (1-decay)(g^2+eps1); accumulates sum u^2 and sum p^2.
+template <class S>
 __device__ __forceinline__ void af_unfactored_stats(const float* __restrict__ g,
                                                     const float* __restrict__ p,
-                                                    float* __restrict__ v,
-                                                    AdafactorScalars* __restrict__ scal,
+                                                    float* __restrict__ v, S* __restrict__ scal,
                                                     long long n, float decay, float eps1,
                                                     int skip_nan, int block, int blocks, int b) {
   __shared__ float red[2][32];
@@ -326,8 +351,8 @@ __device__ __forceinline__ void af_unfactored_stats(const float* __restrict__ g,
       a += red[0][w];
       c += red[1][w];
     }
-    atomicAdd(&scal[b].usq, a);
-    atomicAdd(&scal[b].psq, c);
+    atomicAdd(&scal[b].usq, static_cast<decltype(scal->usq)>(a));
+    atomicAdd(&scal[b].psq, static_cast<decltype(scal->psq)>(c));
   }
 }
 
@@ -344,12 +369,11 @@ __global__ void __launch_bounds__(kAfThreads)
 constexpr int kAfRowsPerCta = 32;
 constexpr int kAfColsPerCta = kAfThreads * 4;
 
-template <bool VEC>
+template <bool VEC, class S>
 __device__ __forceinline__ void af_usq_tile(const float* __restrict__ g,
                                             const float* __restrict__ rf,
-                                            const float* __restrict__ cf,
-                                            AdafactorScalars* __restrict__ scal, int R, int C,
-                                            int tile_x, int tile_y, int b) {
+                                            const float* __restrict__ cf, S* __restrict__ scal,
+                                            int R, int C, int tile_x, int tile_y, int b) {
   __shared__ float red[kAfThreads / 32];
   g += static_cast<long long>(b) * R * C;
   rf += static_cast<long long>(b) * R;
@@ -387,7 +411,7 @@ __device__ __forceinline__ void af_usq_tile(const float* __restrict__ g,
     float t = 0.f;
 #pragma unroll
     for (int w = 0; w < kAfThreads / 32; ++w) t += red[w];
-    atomicAdd(&scal[b].usq, t);
+    atomicAdd(&scal[b].usq, static_cast<decltype(scal->usq)>(t));
   }
 }
 
@@ -399,17 +423,17 @@ __global__ void __launch_bounds__(kAfThreads)
   af_usq_tile<VEC>(g, rf, cf, scal, R, C, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-template <bool VEC>
+template <bool VEC, class S>
 __device__ __forceinline__ void af_apply_tile(
     float* __restrict__ p, const float* __restrict__ g, const float* __restrict__ rf,
     const float* __restrict__ cf, float* __restrict__ m, __nv_bfloat16* __restrict__ p_bf16,
-    long long ld_bf16, long long bf16_batch_stride, const AdafactorScalars* __restrict__ scal, int R,
-    int C, float n_global, const AfHyper& h, int tile_x, int tile_y, int b) {
+    long long ld_bf16, long long bf16_batch_stride, const S* __restrict__ scal, int R, int C,
+    float n_global, const AfHyper& h, int tile_x, int tile_y, int b) {
   const long long base = static_cast<long long>(b) * R * C;
   const int r0 = tile_y * kAfRowsPerCta;
   const int col = tile_x * kAfColsPerCta + threadIdx.x * 4;
   if (col >= C) return;
-  const float scale = af_update_scale(scal[b], n_global, h);
+  const float scale = af_update_scale(af_rounded(scal[b]), n_global, h);
   rf += static_cast<long long>(b) * R;
   cf += static_cast<long long>(b) * C;
   float c[4];
@@ -520,8 +544,9 @@ struct AfItem {
   float* m;
   __nv_bfloat16* out;
   long long ld, bbs;
-  float *rowsum, *colsum, *rf, *cf;  // factored scratch
-  AdafactorScalars* scal;
+  double *rowsum, *colsum;  // factored scratch
+  float *rf, *cf;
+  AfScalars64* scal;
   float n;             // elements per batch element
   int batch, R, C;
   int factored, row_is_normalized, param_scale;
@@ -840,7 +865,9 @@ struct T5xAdafactorItem {
 
 // Scratch floats of one item, a multiple of four.
 static long long af_item_scratch(const T5xAdafactorItem& x) {
-  const long long n = x.v1 ? t5x_adafactor_scratch_floats(x.batch, x.R, x.C) : 4ll * x.batch;
+  // the scalars, fp64 row and column sums, fp32 factors
+  const long long scalars = static_cast<long long>(sizeof(AfScalars64) / sizeof(float)) * x.batch;
+  const long long n = scalars + (x.v1 ? 3ll * x.batch * (static_cast<long long>(x.R) + x.C) : 0);
   return (n + 3) / 4 * 4;
 }
 
@@ -900,20 +927,21 @@ T5X_API int t5x_adafactor_group(const void* items, int count, void* scratch, flo
       it.blocks = af_grid(static_cast<long long>(x.R) * x.C);
       long long mine[3] = {0, 0, 0};
       if (it.factored) {
-        const AfScratch a = af_split(next, x.batch, x.R, x.C);
-        it.rowsum = a.rowsum;
-        it.colsum = a.colsum;
-        it.rf = a.rf;
-        it.cf = a.cf;
-        it.scal = a.scal;
+        const long long rows = 1ll * x.batch * x.R, cols = 1ll * x.batch * x.C;
+        it.scal = reinterpret_cast<AfScalars64*>(next);
+        it.rowsum = reinterpret_cast<double*>(it.scal + x.batch);
+        it.colsum = it.rowsum + rows;
+        it.rf = reinterpret_cast<float*>(it.colsum + cols);
+        it.cf = it.rf + rows;
         const dim3 tg = af_tiled_grid(x.batch, x.R, x.C);
         mine[0] = 1ll * ((x.C + kAfTileC - 1) / kAfTileC) * ((x.R + kAfTileR - 1) / kAfTileR) * x.batch;
         mine[1] = x.batch;
         mine[2] = 1ll * tg.x * tg.y * tg.z;
         factored = true;
       } else {
-        it.rowsum = it.colsum = it.rf = it.cf = nullptr;
-        it.scal = reinterpret_cast<AdafactorScalars*>(next);
+        it.rowsum = it.colsum = nullptr;
+        it.rf = it.cf = nullptr;
+        it.scal = reinterpret_cast<AfScalars64*>(next);
         mine[0] = mine[2] = 1ll * it.blocks * x.batch;
       }
       next += af_item_scratch(x);

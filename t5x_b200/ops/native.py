@@ -798,7 +798,7 @@ class AdafactorItems:
   _ITEM = struct.Struct("=6Q2q6i")
 
   def __init__(self):
-    self._packed, self._scratch, self.count = [], 0, 0
+    self._packed, self.count = [], 0
 
   def add(self, p, g, v0, v1, m, out, ld: int, bbs: int, batch: int, rows: int, cols: int,
           row_is_normalized: bool, param_scale: bool) -> None:
@@ -809,11 +809,11 @@ class AdafactorItems:
     self._packed.append(self._ITEM.pack(p.data_ptr(), v0.data_ptr(), ptr(v1), ptr(m), ptr(out),
                                         g.data_ptr(), ld, bbs, batch, rows, cols,
                                         int(row_is_normalized), int(param_scale), 0))
-    self._scratch += -(-(4 * batch + (2 * batch * (rows + cols) if v1 is not None else 0)) // 4) * 4
     self.count += 1
 
   def scratch_floats(self) -> int:
-    return self._scratch
+    buf = self.buffer()
+    return int(lib().t5x_adafactor_group_scratch_floats(ctypes.addressof(buf), self.count))
 
   def buffer(self):
     return ctypes.create_string_buffer(b"".join(self._packed), self._ITEM.size * self.count)

@@ -61,3 +61,30 @@ def test_group_matches_single(count, kwargs):
     torch.testing.assert_close(p1[k].bf16, p1[k].bfloat16(), rtol=0, atol=0, equal_nan=True)
     for name in s0[k]:
       torch.testing.assert_close(s1[k][name], s0[k][name], rtol=1e-5, atol=1e-30, equal_nan=True)
+
+
+@pytest.mark.parametrize("rows,cols,batch", [(256, 512, 1), (1, 7, 1), (33, 1030, 3)])
+def test_scratch_is_as_large_as_stated(rows, cols, batch):
+  """Nothing is written beyond `scratch_floats()`, and two runs agree bit by bit: the sums that meet
+  by atomic adds do so in fp64."""
+  from t5x_b200.ops import native
+  g = torch.Generator(device="cuda").manual_seed(rows)
+  rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+  p0, grad = rnd(batch, rows, cols), rnd(batch, rows, cols)
+  vec = rnd(77)
+  results = []
+  for _ in range(2):
+    p, v0, v1 = p0.clone(), torch.ones(batch, rows, device="cuda"), torch.ones(batch, cols, device="cuda")
+    q, full = vec.clone(), torch.ones(77, device="cuda")
+    items = native.AdafactorItems()
+    items.add(p, grad, v0, v1, None, None, 0, 0, batch, rows, cols, True, True)
+    items.add(q, vec, full, None, None, None, 0, 0, 1, 1, 77, False, True)
+    n = items.scratch_floats()
+    scratch = torch.full((n + 64,), 7.0, device="cuda")
+    native.adafactor_group_(items, scratch, lr=0.01, decay=0.8, eps1=1e-30, eps2=1e-3,
+                            clip_threshold=1.0, weight_decay=0.0, beta1=0.0, max_param_scale=0.0,
+                            flags=native.AF_CLIP)
+    assert bool((scratch[n:] == 7.0).all())
+    results.append((p, v0, v1, q, full))
+  for a, b in zip(*results):
+    assert torch.equal(a, b) and bool(torch.isfinite(a).all())
