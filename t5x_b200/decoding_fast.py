@@ -41,16 +41,6 @@ native.register_signature("t5x_decode_cross_attention_mma",
                            c_void_p])
 
 NEG_INF = decoding.NEG_INF
-# Up to this many rows (batch * beams) a decode step runs `native.gemm_rows` where it covers a
-# product. Without a norm in front it was faster at every shape it covers (us, cold weights; against
-# the cluster split-K GEMM: 4 rows 768 x 768 3.5 / 7.5, 2048 x 768 4.9 / 8.7, 2048 x 2048 6.1 / 17.3;
-# 64 rows 768 x 768 8.1 / 9.8).
-FEW_ROWS = 64
-# With a norm in front every CTA normalises all rows for itself, which pays up to this many
-# elements (against a norm launch and the tcgen05 GEMM: 4 x 768 to 2304 columns 4.3 / 10.3, 32 x 768
-# 7.8 / 10.6, 8 x 2048 to 6144 11.9 / 16.9; beyond the line 32 x 1024 to 3072 15.4 / 12.6,
-# 16 x 2048 to 6144 17.7 / 17.0).
-FUSED_NORM_ELEMENTS = 24576
 
 
 def decode_self_attention(q, k_new, v_new, cache_k, cache_v, ancestry, bias_row, cur_index, out,
@@ -310,14 +300,15 @@ class GraphBeamDecoder:
     self.check_period = max(1, int(os.environ.get("T5X_B200_DECODE_CHECK_PERIOD",
                                                   termination_check_period)))
     self.replays = 0           # graph replays so far
-    # Programmatic dependent launches inside the step (`native.chained_launches`). On for few rows:
-    # the products request their weights while the kernel in front of them finishes (4 sentences
-    # of T5.1.1 base, 32 steps: 18.0 -> 17.3 ms). Off otherwise (a 210 KB GEMM CTA cannot become
-    # resident beside its predecessor), and for the tensor-parallel step, whose kernels wait for
-    # other ranks.
-    few = self.tp == 1 and self.rows <= FEW_ROWS
-    self.chain_level = int(os.environ.get("T5X_B200_DECODE_CHAIN", "2" if few else "0")) \
-        if self.tp == 1 else 0
+    # Programmatic dependent launches inside the step (`native.chained_launches`): the products
+    # request their weights while the kernel in front of them finishes. On for up to 64 rows of a
+    # model up to T5.1.1 large (32 steps over 128 positions, ms, without / with: small, 8 layers,
+    # 1 row 15.8 / 14.8, 64 rows 18.7 / 17.2; base, 12 layers, 4 rows 28.6 / 26.5; large, 8 layers,
+    # 4 rows 22.3 / 20.7; but XL, 6 layers, 4 rows 22.2 / 23.0, where a wider product leaves no
+    # room beside its predecessor). Off for the tensor-parallel step: its kernels wait for other
+    # ranks.
+    chain = "2" if self.rows <= 64 and c.emb_dim <= 1024 else "0"
+    self.chain_level = int(os.environ.get("T5X_B200_DECODE_CHAIN", chain)) if self.tp == 1 else 0
     # residual projections through the cluster split-K GEMM (sum over K slices in distributed
     # shared memory) instead of fp32 atomics into a workspace plus a finishing kernel
     self.cluster_gemm = os.environ.get("T5X_B200_DECODE_CLUSTER_GEMM", "1") != "0"
@@ -342,7 +333,6 @@ class GraphBeamDecoder:
     wl = w.bf16
     self.w_logits = wl if wl.shape[0] == c.emb_dim else wl.t()
     self.rel_table = dec.relpos_bias.rel_embedding
-    self.few_rows = few
     bf = dict(dtype=torch.bfloat16, device=dev)
     # [batch, beam slot, head, position, dim]: one (slot, head) history is contiguous. For the
     # tensor-core kernel the cache is padded to a multiple of 32 positions and the values are
@@ -421,37 +411,6 @@ class GraphBeamDecoder:
       from t5x_b200.parallel import tp_fused
       tp_fused.end_step()  # the encoder pass is over: its arena blocks are free again
 
-  def _rows_ok(self, w: torch.Tensor, gated: bool = False) -> bool:
-    """Whether `native.gemm_rows` covers the product of this decoder's rows with weight `w`."""
-    return (w.stride(1) == 1 and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0 and
-            native.gemm_rows_ok(self.rows, w.shape[1], w.shape[0], gated))
-
-  def _norm_matmul(self, x, scale, w, w2=None, out_dtype=torch.bfloat16, alpha: float = 1.0):
-    """alpha * norm(x) @ w, or with `w2` the gated GELU of both, for few rows."""
-    if x.numel() <= FUSED_NORM_ELEMENTS and self._rows_ok(w, w2 is not None) and \
-        (w2 is None or w2.data_ptr() % 16 == 0) and scale.dtype == torch.float32 and \
-        scale.is_contiguous() and scale.data_ptr() % 16 == 0:
-      return native.gemm_rows(x, w, b2=w2, norm_scale=scale, out_dtype=out_dtype, alpha=alpha)
-    h = native.rmsnorm_fwd(x, scale, 1e-6)[0]
-    if w2 is None and out_dtype == torch.bfloat16 and w.shape[1] == self.H * self.D:
-      return self._skinny(h, w)
-    return native.gemm(h, w, b2=w2, out_dtype=out_dtype, alpha=alpha)
-
-  def _layers_few_rows(self, x: torch.Tensor, bias_row: torch.Tensor) -> torch.Tensor:
-    """The decoder layers of one step for few rows: eight launches a layer where `gemm_rows`
-    covers every product."""
-    rows, H, D = self.rows, self.H, self.D
-    ctx = torch.empty(rows, H, D, dtype=torch.bfloat16, device=self.dev)
-    for i, ly in enumerate(self.layers):
-      qkv = self._norm_matmul(x, ly.ln1, ly.qkv).view(rows, 3, H, D)
-      self._self_attention(i, qkv, bias_row, ctx)
-      x = self._skinny(ctx.view(rows, H * D), ly.o, residual=x)
-      qc = self._norm_matmul(x, ly.ln2, ly.cq).view(rows, H, D)
-      cc = self._cross_attention(i, qc, ctx)
-      x = self._skinny(cc.reshape(rows, H * D), ly.co, residual=x)
-      x = self._skinny(self._norm_matmul(x, ly.ln3, ly.wi0, ly.wi1), ly.wo, residual=x)
-    return x
-
   def _self_attention(self, i: int, qkv, bias_row, ctx) -> None:
     if self.self_mma:
       decode_self_attention_mma(qkv[:, 0], qkv[:, 1], qkv[:, 2], self.cache_k[i], self.cache_v[i],
@@ -481,9 +440,6 @@ class GraphBeamDecoder:
         self.live_seqs.data_ptr(), self.cur.data_ptr(), self.emb.data_ptr(), x.data_ptr(),
         table.data_ptr(), self.bucket_of_distance.data_ptr(), bias_row.data_ptr(), rows, H, self.L,
         c.emb_dim, self.emb.shape[0], table.shape[1], native.stream_ptr()), "decode_begin")
-    if self.few_rows:
-      return self._norm_matmul(self._layers_few_rows(x, bias_row), self.final_ln, self.w_logits,
-                               out_dtype=torch.float32, alpha=self.logit_scale)
     ctx = torch.empty(rows, H, D, dtype=torch.bfloat16, device=self.dev)
     if self.link is not None:
       self.link.begin_step()
@@ -523,10 +479,7 @@ class GraphBeamDecoder:
                                    workspace=self._workspace())
 
   def _skinny(self, a, w, residual=None):
-    """a[rows, K] @ w[K, N] (+ residual) for few rows: the whole K per CTA up to FEW_ROWS rows,
-    K split over CTAs up to 512."""
-    if self.few_rows and self._rows_ok(w):
-      return native.gemm_rows(a, w, residual=residual)
+    """a[rows, K] @ w[K, N] (+ residual) with K split over CTAs when rows are few."""
     if self.rows > 512:
       return native.gemm(a, w, residual=residual)
     if self.cluster_gemm:

@@ -429,44 +429,6 @@ def gemm_skinny(a: torch.Tensor, b: torch.Tensor, *, residual: Optional[torch.Te
   return out
 
 
-register_signature("t5x_gemm_rows_ok", [c_int, c_int, c_int, c_int])
-register_signature("t5x_gemm_rows_bf16", [c_void_p] * 4 + [c_int] * 3 + [c_ll] * 3 +
-                   [c_int, c_void_p, c_float, c_void_p, c_ll, c_float, c_void_p])
-
-
-def gemm_rows_ok(M: int, N: int, K: int, gated: bool = False) -> bool:
-  """Whether `gemm_rows` covers a product of this shape."""
-  return bool(lib().t5x_gemm_rows_ok(M, N, K, int(gated)))
-
-
-def gemm_rows(a: torch.Tensor, b: torch.Tensor, *, b2: Optional[torch.Tensor] = None,
-              norm_scale: Optional[torch.Tensor] = None, eps: float = 1e-6,
-              residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-              out_dtype: torch.dtype = torch.bfloat16, alpha: float = 1.0) -> torch.Tensor:
-  """out[M, N] = alpha * n(a)[M, K] @ b[K, N] (+ residual) for at most 64 rows in one launch
-  (csrc/gemm_rows_sm100.cu); n is the RMS norm with `norm_scale` (fp32 [K]) or nothing. With `b2`:
-  gelu(n(a) @ b) * (n(a) @ b2). `b` and `b2` are row-major."""
-  M, K = a.shape
-  N = b.shape[1]
-  assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.stride(1) == 1
-  assert b.shape[0] == K and b.stride(1) == 1
-  assert b2 is None or (b2.shape == b.shape and b2.stride() == b.stride() and
-                        b2.dtype == b.dtype and alpha == 1.0)
-  assert norm_scale is None or (norm_scale.dtype == torch.float32 and norm_scale.is_contiguous()
-                                and norm_scale.numel() == K)
-  assert residual is None or (residual.dtype == torch.bfloat16 and residual.shape == (M, N) and
-                              residual.stride(1) == 1)
-  if out is None:
-    out = torch.empty(M, N, dtype=out_dtype, device=a.device)
-  assert out.shape == (M, N) and out.stride(1) == 1
-  assert out.dtype in (torch.bfloat16, torch.float32)
-  _check(lib().t5x_gemm_rows_bf16(
-      a.data_ptr(), b.data_ptr(), ptr(b2), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
-      out.stride(0), int(out.dtype == torch.float32), ptr(norm_scale), float(eps), ptr(residual),
-      residual.stride(0) if residual is not None else 0, float(alpha), stream_ptr()), "gemm_rows")
-  return out
-
-
 def gemm_splitk_norm(a: torch.Tensor, b: torch.Tensor, splits: int, *, residual: torch.Tensor,
                      scale: torch.Tensor, eps: float, workspace: torch.Tensor):
   """(x, h): x = a @ b + residual (bf16), h = rmsnorm(x) * scale, with K cut into `splits`

@@ -1,0 +1,73 @@
+"""Kernels of the decode step for few rows, and a greedy decode of few sentences against the same
+sentences in a larger batch."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("emb,heads,mlp", [(256, 4, 512), (256, 32, 1024), (768, 12, 2048)])
+@pytest.mark.parametrize("few", [1, 4, 9])
+def test_a_sentence_does_not_depend_on_its_batch(emb, heads, mlp, few):
+  """The products of a step add up in one order whatever the number of rows (up to one tile of 128),
+  and so does the attention in both of its forms (32 heads: wide for few rows, narrow for 80). So
+  the logits of a sentence are the same bit by bit alone and in a batch of 80, and no near-tie
+  between two tokens is decided by who else is decoded."""
+  from t5x_b200 import decoding_fast
+  from t5x_b200.models.t5 import network
+  torch.manual_seed(emb + heads)
+  cfg = network.T5Config(vocab_size=512, dtype="bfloat16", emb_dim=emb, num_heads=heads, head_dim=64,
+                         num_encoder_layers=1, num_decoder_layers=3, mlp_dim=mlp,
+                         mlp_activations=("gelu", "linear"), dropout_rate=0.0)
+  module = network.Transformer(cfg, device="cuda")
+  for p in module.parameters():
+    p.bf16 = p.detach().bfloat16()
+  enc = torch.randint(2, 512, (80, 19), device="cuda")
+  steps = []
+  tokens = torch.zeros(80, 1, 41, dtype=torch.long, device="cuda")
+  tokens[:, :, 1:] = torch.randint(2, 512, (80, 1, 40), device="cuda")
+  for n in (few, 80):
+    d = decoding_fast.GraphBeamDecoder(module, n, 1, 40, 1, use_graph=False)
+    with torch.no_grad():
+      d._encode(enc[:n])
+      d._reset()
+      d.live_seqs.copy_(tokens[:n])
+      logits = []
+      for t in range(40):
+        d.cur.fill_(t)
+        logits.append(d._model_step()[:few].clone())
+    steps.append(torch.stack(logits))
+  assert torch.equal(steps[0], steps[1])
+
+
+@pytest.mark.parametrize("b,lk,h", [(1, 1, 1), (2, 31, 3), (3, 33, 2), (2, 64, 4), (1, 129, 2)])
+def test_cross_layout(b, lk, h):
+  """A rearrangement: equal to the tensor-op statement bit by bit, the padding zero."""
+  from t5x_b200 import decoding_fast
+  k, v = (torch.randn(b, lk, h, 64, device="cuda").bfloat16() for _ in range(2))
+  kp, vt = decoding_fast.cross_kv_layout(k, v)
+  kc, vc = decoding_fast.cross_kv_layout(k.cpu(), v.cpu())
+  assert torch.equal(kp.cpu(), kc) and torch.equal(vt.cpu(), vc)
+  again = decoding_fast.cross_kv_layout(v, k, out=(kp, vt))
+  assert again[0] is kp and torch.equal(kp[:, :, :lk], v.transpose(1, 2))
+
+
+@pytest.mark.parametrize("m,k,n,splits,transposed,with_res", [
+    (256, 2048, 2048, 4, False, True), (37, 128, 384, 2, True, False),
+    (200, 1024, 256, 8, False, True), (128, 192, 128, 1, False, False), (1, 64, 128, 1, True, True),
+    (300, 512, 640, 2, True, True)])
+def test_skinny_with_half_width_tiles(m, k, n, splits, transposed, with_res):
+  """The cluster split-K GEMM with 128 x 64 tiles: every cluster size, rings that are not filled
+  and rings that wrap, both weight layouts, row tails. fp32 accumulation, one rounding to bf16
+  (2^-9 of a value), with a factor of two for the fp32 sums."""
+  from t5x_b200.ops import native
+  torch.manual_seed(m + k + n)
+  a = torch.randn(m, k, device="cuda").bfloat16()
+  w = (torch.randn(n, k, device="cuda") * 0.05).bfloat16().t() if transposed else \
+      (torch.randn(k, n, device="cuda") * 0.05).bfloat16()
+  res = torch.randn(m, n, device="cuda").bfloat16() if with_res else None
+  out = native.gemm_skinny(a, w, residual=res, splits=splits, tile_n=64)
+  native.check_status()
+  ref = a.double() @ w.double() + (0 if res is None else res.double())
+  assert float((out.double() - ref).abs().max() / ref.abs().max()) < 2 * 2.0 ** -9
+  assert torch.equal(out, native.gemm_skinny(a, w, residual=res, splits=splits, tile_n=64))
