@@ -391,7 +391,8 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
                      long long c_batch_stride, int a_mn_major, int b_mn_major, int out_fp32,
                      int accumulate, int epilogue, const void* R, long long ldr,
                      long long r_batch_stride, void* H0, void* H1, long long ldh, float alpha,
-                     int max_ctas, void* stream, const GemmTp* tp, int tp_mode) {
+                     int max_ctas, void* stream, const GemmTp* tp, int tp_mode,
+                     int last_wave = 1) {
   if (M <= 0 || N <= 0 || batch <= 0) return 0;
   if (K <= 0) return set_error("gemm: K must be positive");
   if (lda % 8 || ldb % 8) return set_error("gemm: lda/ldb must be multiples of 8 elements");
@@ -504,8 +505,10 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
   // at the measured copy and GEMM rates) and atomic adds, so it has to save more than both.
   // (us, whole tiles / cut: 768 x 768 x 12216 75 / 31, 768 x 3072 x 12216 80 / 56,
   // 1472 x 3584 x 16384 189 / 132, 1024 x 16384 x 8192 240 / 217, 2048 x 5120 x 32768 705 / 519.)
-  if (pair_mode != 0 && epilogue == kEpiPlain && out_fp32 && accumulate != 2 && M >= 2 * kBM &&
-      N >= 256 && max_ctas <= 0 && ldc == N &&
+  // Only for callers that ask for it: more than two pieces meet in no fixed order, and the logits
+  // of a forward product have to be the same on every call.
+  if (last_wave != 1 && pair_mode != 0 && epilogue == kEpiPlain && out_fp32 && accumulate != 2 &&
+      M >= 2 * kBM && N >= 256 && max_ctas <= 0 && ldc == N &&
       (batch == 1 || c_batch_stride == static_cast<long long>(M) * N)) {
     const int tn = (N + 255) / 256, pairs = sms / 2;
     const long long tiles = 1ll * pair_tiles_m * tn * batch;
@@ -522,7 +525,9 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
     }
     const double waves = static_cast<double>(tiles / pairs);
     const double saved = (1.0 - best) / (waves + 1.0);
-    if (splits > 1 && saved > 0.08 + 430.0 / K) {
+    if (saved <= 0.08 + 430.0 / K) splits = 1;
+    if (last_wave > 1) splits = tail > 0 ? std::min(last_wave, kb) : 1;
+    if (splits > 1) {
       if (!accumulate) {
         cudaError_t e = cudaMemsetAsync(C, 0, sizeof(float) * static_cast<size_t>(M) * N * batch, st);
         if (e != cudaSuccess) return set_error("gemm: memset: %s", cudaGetErrorString(e));
@@ -578,6 +583,23 @@ T5X_API int t5x_gemm_bf16(const void* A, const void* B, const void* B2, void* C,
                         b_batch_stride, c_batch_stride, a_mn_major, b_mn_major, out_fp32,
                         accumulate, epilogue, R, ldr, r_batch_stride, H0, H1, ldh, alpha, max_ctas,
                         stream, nullptr, 0);
+}
+
+// C[batch, M, N] (fp32) (+)= A @ B for weight gradients: as t5x_gemm_bf16 with its plain epilogue,
+// except that the tiles of the last wave may be cut along K and added up by atomic adds, so that
+// the last bits of C depend on their order. last_wave_pieces: 0 the library's choice, 1 whole tiles,
+// n > 1 that many pieces (at most one per 64 of K) where the shape can be cut.
+T5X_API int t5x_gemm_wgrad_bf16(const void* A, const void* B, void* C, int M, int N, int K, int batch,
+                                long long lda, long long ldb, long long ldc,
+                                long long a_batch_stride, long long b_batch_stride,
+                                long long c_batch_stride, int a_mn_major, int b_mn_major,
+                                int accumulate, int last_wave_pieces, void* stream) {
+  if (accumulate != 0 && accumulate != 1) return t5x::set_error("gemm_wgrad: accumulate is 0 or 1");
+  if (last_wave_pieces < 0) return t5x::set_error("gemm_wgrad: pieces must not be negative");
+  return t5x::gemm_impl(A, B, nullptr, C, M, N, K, batch, lda, ldb, ldc, a_batch_stride,
+                        b_batch_stride, c_batch_stride, a_mn_major, b_mn_major, 1, accumulate,
+                        t5x::kEpiPlain, nullptr, 0, 0, nullptr, nullptr, 0, 1.f, 0, stream, nullptr,
+                        0, last_wave_pieces);
 }
 
 namespace t5x {

@@ -25,6 +25,10 @@ int t5x_gemm_bf16(const void* A, const void* B, const void* B2, void* C, int M, 
                   int out_fp32, int accumulate, int epilogue, const void* R, long long ldr,
                   long long r_batch_stride, void* H0, void* H1, long long ldh, float alpha,
                   int max_ctas, void* stream);
+int t5x_gemm_wgrad_bf16(const void* A, const void* B, void* C, int M, int N, int K, int batch,
+                        long long lda, long long ldb, long long ldc, long long a_batch_stride,
+                        long long b_batch_stride, long long c_batch_stride, int a_mn_major,
+                        int b_mn_major, int accumulate, int last_wave_pieces, void* stream);
 int t5x_rmsnorm_fwd(const void* x, const void* scale, void* y, void* rstd, int rows, int d, float eps,
                     void* stream);
 int t5x_rmsnorm_bwd(const void* dy, const void* x, const void* scale, const void* rstd,
@@ -124,9 +128,9 @@ void input_grad(const void* dy, int64_t ld_dy, int64_t m, const Weight& w, Tenso
 // grad[k, n] (fp32) (+)= x^T @ dy
 void weight_grad(const Tensor& x, const void* dy, int64_t ld_dy, int64_t m, const Weight& w,
                  Tensor& grad, bool accumulate, void* st) {
-  check(t5x_gemm_bf16(x.data_ptr(), dy, nullptr, grad.data_ptr(), w.k, w.n, m, 1, w.k, ld_dy, w.n, 0,
-                      0, 0, 1, 1, 1, accumulate, 0, nullptr, 0, 0, nullptr, nullptr, 0, 1.f, 0, st),
-        "gemm");
+  check(t5x_gemm_wgrad_bf16(x.data_ptr(), dy, grad.data_ptr(), w.k, w.n, m, 1, w.k, ld_dy, w.n, 0, 0, 0,
+                            1, 1, accumulate, 0, st),
+        "gemm_wgrad");
 }
 
 // A gradient buffer the weight-gradient GEMM can write whole; narrow outputs over many rows are

@@ -75,6 +75,13 @@ int t5x_gemm_bf16(const void* A, const void* B, const void* B2, void* C, int M, 
                   const void* R, long long ldr, long long r_batch_stride, void* H0, void* H1,
                   long long ldh, float alpha, int max_ctas, void* stream);
 
+/* Weight gradients: C[batch, M, N] (fp32) (+)= A @ B. The tiles of the last wave may be cut along K
+ * and added atomically: last_wave_pieces 0 = the library's choice, 1 = whole tiles, n = n pieces. */
+int t5x_gemm_wgrad_bf16(const void* A, const void* B, void* C, int M, int N, int K, int batch,
+                        long long lda, long long ldb, long long ldc, long long a_batch_stride,
+                        long long b_batch_stride, long long c_batch_stride, int a_mn_major,
+                        int b_mn_major, int accumulate, int last_wave_pieces, void* stream);
+
 /* ---- tensor parallelism with the collective inside the GEMM kernel ----
  * The M rows are split evenly over `world` ranks (rows_per_rank each). Peer pointers are the
  * other ranks' buffers as mapped into this process (symmetric memory).

@@ -40,16 +40,16 @@ def _accumulate_wgrad(weight: torch.Tensor, a_t: torch.Tensor, b: torch.Tensor):
   if mg is not None:
     first = not getattr(weight, "grad_ready", False)
     out = mg.view(a_t.shape[0], b.shape[1])
-    # (from 256 x 256 outputs on `gemm` itself cuts the tiles of the last wave along K)
+    # (from 256 x 256 outputs on `gemm_wgrad` cuts the tiles of the last wave along K)
     narrow = a_t.shape[0] < 256 or b.shape[1] < 256
     splits = native.wgrad_splits(a_t.shape[0], b.shape[1], a_t.shape[1]) if narrow else 1
     if splits > 1 and out.is_contiguous():
       native.gemm_splitk_accumulate(a_t, b, out, splits, accumulate=not first)
     else:
-      native.gemm(a_t, b, out=out, accumulate=not first)
+      native.gemm_wgrad(a_t, b, out=out, accumulate=not first)
     weight.grad_ready = True
     return None
-  return native.gemm(a_t, b, out_dtype=torch.float32).view(weight.shape).to(weight.dtype)
+  return native.gemm_wgrad(a_t, b).view(weight.shape).to(weight.dtype)
 
 
 class _NoGraph:
@@ -239,10 +239,10 @@ class _BatchedLinearFn(torch.autograd.Function):
       xt = x.contiguous().transpose(1, 2)
       if mg is not None:
         first = not getattr(weight, "grad_ready", False)
-        native.gemm(xt, dy, out=mg, accumulate=not first)
+        native.gemm_wgrad(xt, dy, out=mg, accumulate=not first)
         weight.grad_ready = True
       else:
-        dw = native.gemm(xt, dy, out_dtype=torch.float32).to(weight.dtype)
+        dw = native.gemm_wgrad(xt, dy).to(weight.dtype)
     return dx, dw
 
 
@@ -648,10 +648,10 @@ class _LogitsCrossEntropyFn(torch.autograd.Function):
         mg = getattr(weight, "main_grad", None)
         if mg is not None:
           first = not getattr(weight, "grad_ready", False)
-          native.gemm(dlogits.t(), h2, out=mg, accumulate=not first)
+          native.gemm_wgrad(dlogits.t(), h2, out=mg, accumulate=not first)
           weight.grad_ready = True
         else:
-          dw = native.gemm(dlogits.t(), h2, out_dtype=torch.float32).to(weight.dtype)
+          dw = native.gemm_wgrad(dlogits.t(), h2).to(weight.dtype)
       else:
         dw = _accumulate_wgrad(weight, h2.t(), dlogits)
     return dh, dw, None, None, None, None

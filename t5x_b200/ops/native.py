@@ -339,6 +339,39 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, out: Optional[torch.Tensor] = None
   return out
 
 
+register_signature("t5x_gemm_wgrad_bf16", [c_void_p] * 3 + [c_int] * 4 + [c_ll] * 6 + [c_int] * 4 +
+                   [c_void_p])
+
+
+def gemm_wgrad(a: torch.Tensor, b: torch.Tensor, *, out: Optional[torch.Tensor] = None,
+               accumulate: bool = False, pieces: int = 0) -> torch.Tensor:
+  """out[..., M, N] (fp32) (+)= a[..., M, K] @ b[..., K, N] for weight gradients: `gemm`, except that
+  the tiles of the last wave may be cut along K and added atomically, so that the last bits depend
+  on the order of the adds. `pieces`: 0 the library's choice, 1 whole tiles, n that many."""
+  assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
+  batch = a.shape[0] if a.dim() == 3 else 1
+  M, K = a.shape[-2], a.shape[-1]
+  N = b.shape[-1]
+  assert K == b.shape[-2], (a.shape, b.shape)
+  a_mn, lda, a_step = _mat_layout(a, M, K)
+  if b.stride(-2) == 1:
+    b_mn, ldb = 0, b.stride(-1)
+  elif b.stride(-1) == 1:
+    b_mn, ldb = 1, b.stride(-2)
+  else:
+    raise NativeError(f"b with strides {b.stride()} is neither row- nor column-major")
+  if out is None:
+    out = torch.empty((batch, M, N) if a.dim() == 3 else (M, N), dtype=torch.float32, device=a.device)
+  if out.dtype != torch.float32:
+    return gemm(a, b, out=out, accumulate=accumulate)
+  assert out.stride(-1) == 1 and out.shape[-2:] == (M, N), (out.shape, out.stride(), M, N)
+  _check(lib().t5x_gemm_wgrad_bf16(
+      a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, batch, lda, ldb, out.stride(-2), a_step,
+      b.stride(0) if b.dim() == 3 else 0, out.stride(0) if out.dim() == 3 else 0, a_mn, b_mn,
+      int(accumulate), pieces, stream_ptr()), "gemm_wgrad")
+  return out
+
+
 # ----------------------------------------------------------------------------
 # Normalisation / activations / embedding
 # ----------------------------------------------------------------------------

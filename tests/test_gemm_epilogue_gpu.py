@@ -91,13 +91,27 @@ def test_weight_gradient_with_a_split_last_wave(batch, M, N, K, ta):
   if batch == 1:
     a, b = a[0], b[0]
   want = a.double() @ b.double()
-  out = torch.full(want.shape, 3.0, device="cuda")
-  native.gemm(a, b, out=out)
   tol = K / 16 * 2 ** -23 * 5 * K ** 0.5
-  assert float((out - want).abs().max()) < tol
-  native.gemm(a, b, out=out, accumulate=True)
-  assert float((out - 2 * want).abs().max()) < 2 * tol
   wide = torch.zeros(*want.shape[:-1], N + 8, device="cuda")  # rows apart: whole tiles
-  native.gemm(a, b, out=wide[..., :N])
-  assert float((wide[..., :N] - want).abs().max()) < tol and not bool(wide[..., N:].any())
+  for pieces in (0, 2, 7):
+    out = torch.full(want.shape, 3.0, device="cuda")
+    native.gemm_wgrad(a, b, out=out, pieces=pieces)
+    assert float((out - want).abs().max()) < tol
+    native.gemm_wgrad(a, b, out=out, accumulate=True, pieces=pieces)
+    assert float((out - 2 * want).abs().max()) < 2 * tol
+    native.gemm_wgrad(a, b, out=wide[..., :N], pieces=pieces)
+    assert float((wide[..., :N] - want).abs().max()) < tol and not bool(wide[..., N:].any())
+  native.check_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 384, 2560), (256, 384, 2048), (256, 384, 4672), (512, 768, 8200)])
+def test_forward_products_keep_whole_tiles(M, N, K):
+  """fp32 logits are the same bit by bit on every call, and equal those of an output whose rows lie
+  apart, which is never cut: no product is cut along K unless its caller asks for it."""
+  from t5x_b200.ops import native
+  a, b, _ = _operands(M, N, K, K)
+  wide = torch.empty(M, N + 8, device="cuda")
+  native.gemm(a, b, out=wide[:, :N])
+  for _ in range(10):
+    assert torch.equal(native.gemm(a, b, out_dtype=torch.float32), wide[:, :N])
   native.check_status()
