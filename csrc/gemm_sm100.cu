@@ -501,10 +501,13 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
     return launch_gemm<256, kEpiGatedGelu>(tA, tB, tB2, p, max_ctas, st);
   }
   // A weight gradient (fp32 output, long K) whose tiles leave the last wave of pairs mostly empty:
-  // the tiles of that wave are cut along K. That costs a fill of C (430 / K of the product's time
-  // at the measured copy and GEMM rates) and atomic adds, so it has to save more than both.
-  // (us, whole tiles / cut: 768 x 768 x 12216 75 / 31, 768 x 3072 x 12216 80 / 56,
-  // 1472 x 3584 x 16384 189 / 132, 1024 x 16384 x 8192 240 / 217, 2048 x 5120 x 32768 705 / 519.)
+  // the tiles of that wave are cut along K. What a cut gives and costs, fitted to 4400 times (21
+  // outputs from 256 x 256 to 768 x 32128, K from 512 to 65536, 2 to 64 pieces), in us: a wave
+  // takes 0.0054 K; the adds 0.19 a MB; the fill of C and its launch 7.4 + 0.11 a MB. A product
+  // that adds to C needs no fill, and saves some 4 because whole tiles read C back first. (us, whole
+  // tiles / cut: 768 x 768 x 12216 75 / 31, 768 x 3072 x 12216 80 / 56, 1472 x 3584 x 16384
+  // 189 / 130, 2048 x 5120 x 32768 705 / 519; left whole: 1024 x 2816 x 2048 25.6 / 31.7 in three,
+  // 2048 x 2048 x 12216 83 / 91 in eight. The rule lost nowhere among them.)
   // Only for callers that ask for it: more than two pieces meet in no fixed order, and the logits
   // of a forward product have to be the same on every call.
   if (last_wave != 1 && pair_mode != 0 && epilogue == kEpiPlain && out_fp32 && accumulate != 2 &&
@@ -514,18 +517,19 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
     const long long tiles = 1ll * pair_tiles_m * tn * batch;
     const int kb = (K + kBK - 1) / kBK;
     const int tail = static_cast<int>(tiles % pairs);
-    double best = 1.0;  // time of the last wave, in waves
+    const double wave = 0.0054 * K;
+    const double fill = accumulate ? -4.0 : 7.4 + 0.11e-6 * sizeof(float) * M * N * batch;
+    const double tile_add = 0.19e-6 * sizeof(float) * (2 * kBM) * 256;
+    double best = 0.04 * (5.0 + wave * static_cast<double>((tiles + pairs - 1) / pairs));
     int splits = 1;
-    for (int s = 2; tail > 0 && s <= 16 && kb / s >= 8; ++s) {
-      const double t = static_cast<double>((1ll * tail * s + pairs - 1) / pairs) / s;
-      if (t < best - 0.02) {
-        best = t;
+    for (int s = 2; tail > 0 && s <= 64 && kb / s >= 8; ++s) {
+      const double last = static_cast<double>((1ll * tail * s + pairs - 1) / pairs) / s;  // waves
+      const double saved = (1.0 - last) * wave - fill - tile_add * tail * s;
+      if (saved > best) {
+        best = saved;
         splits = s;
       }
     }
-    const double waves = static_cast<double>(tiles / pairs);
-    const double saved = (1.0 - best) / (waves + 1.0);
-    if (saved <= 0.08 + 430.0 / K) splits = 1;
     if (last_wave > 1) splits = tail > 0 ? std::min(last_wave, kb) : 1;
     if (splits > 1) {
       if (!accumulate) {

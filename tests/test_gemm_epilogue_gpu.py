@@ -115,3 +115,17 @@ def test_forward_products_keep_whole_tiles(M, N, K):
   for _ in range(10):
     assert torch.equal(native.gemm(a, b, out_dtype=torch.float32), wide[:, :N])
   native.check_status()
+
+
+@pytest.mark.parametrize("M,N,K,cut", [(1024, 2816, 2048, False), (768, 2304, 2048, False),
+                                       (3072, 768, 2048, False), (2048, 2048, 12216, False),
+                                       (768, 768, 12216, True), (256, 256, 65536, True)])
+def test_weight_gradients_are_cut_where_it_pays(M, N, K, cut):
+  """Where the fill and the adds cost more than the last wave gives, the tiles stay whole (the sums
+  are then those of whole tiles, bit by bit); long products with few tiles are cut."""
+  from t5x_b200.ops import native
+  g = torch.Generator(device="cuda").manual_seed(M + K)
+  a, b = (torch.randn(K, n, device="cuda", generator=g).bfloat16() for n in (M, N))
+  whole = native.gemm_wgrad(a.t(), b, pieces=1)
+  assert torch.equal(native.gemm_wgrad(a.t(), b), whole) != cut
+  native.check_status()
