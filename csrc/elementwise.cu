@@ -504,22 +504,21 @@ __global__ void __launch_bounds__(256)
 
 // dtable[id] += dout rows of the tokens with that id, in fp32.
 //
-// A CTA takes CHUNK consecutive tokens and a range of columns (four per thread). It ranks the
+// A CTA takes `chunk` consecutive tokens and a range of columns (four per thread). It ranks the
 // chunk's tokens by id, walks them in that order, keeps the running sum of equal ids in
-// registers and adds one row per DISTINCT id to the table with 16-byte atomics. Natural text
-// is Zipf-distributed and every padding position is id 0: with one atomic add per token, the
+// registers and adds one row per DISTINCT id of the chunk to the table with 16-byte atomics. Natural
+// text is Zipf-distributed and every padding position is id 0: with one atomic add per token, the
 // adds to the few hot rows queued up in L2 and set the time (65536 x 768: 0.69 ms for the
-// 134 MB it moves); a chunk of 128 leaves at most 1/128 of them. Short inputs take chunks of 16 so
-// that more CTAs share the walk and every row of a chunk is in flight at once.
-template <int CHUNK>
+// 134 MB it moves).
+constexpr int kEmbMaxChunk = 128;
 __global__ void __launch_bounds__(256)
     embedding_bwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dout,
                          float* __restrict__ dtable, long long tokens, int d, int vocab_start,
-                         int vocab_rows, int vec_ok) {
-  __shared__ int s_id[CHUNK];      // row of the table, -1 when it is not in this slice
-  __shared__ int s_order[CHUNK];   // token of the chunk at each place of the sorted order
-  const long long t0 = static_cast<long long>(blockIdx.x) * CHUNK;
-  const int n = static_cast<int>(min(static_cast<long long>(CHUNK), tokens - t0));
+                         int vocab_rows, int chunk, int vec_ok) {
+  __shared__ int s_id[kEmbMaxChunk];     // row of the table, -1 when it is not in this slice
+  __shared__ int s_order[kEmbMaxChunk];  // token of the chunk at each place of the sorted order
+  const long long t0 = static_cast<long long>(blockIdx.x) * chunk;
+  const int n = static_cast<int>(min(static_cast<long long>(chunk), tokens - t0));
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const long long id = ids[t0 + i] - vocab_start;
     s_id[i] = (id >= 0 && id < vocab_rows) ? static_cast<int>(id) : -1;
@@ -750,14 +749,20 @@ T5X_API int t5x_embedding_bwd(const void* ids, const void* dout, void* dtable, l
   if (d % 8) return set_error("embedding: d must be a multiple of 8");
   // four columns per thread; whole warps, at most 256 threads
   const int threads = d / 4 >= 256 ? 256 : (d / 4 + 31) / 32 * 32;
-  const int chunk = tokens >= 8192 ? 128 : 16;
+  const int columns = (d / 4 + threads - 1) / threads;
+  // The longest chunk that still gives four CTAs an SM: long chunks save adds, but a CTA walks its
+  // tokens one after the other (us, chunks of 16 or 128 by the number of tokens / so / one add per
+  // token; uniform ids: 256 x 512 16.4 / 8.2 / 8.2, 3000 x 768 16.5 / 13.4 / 22.5, 8192 x 768
+  // 80 / 20.5 / 45, 16384 x 768 80 / 31 / 82, 65536 x 768 96 / 100 / 299, 20000 x 4096
+  // 197 / 198 / 486; all ids equal: 8192 x 768 76 / 20.5 / 637).
+  int chunk = kEmbMaxChunk;
+  while (chunk > 1 && (tokens + chunk - 1) / chunk * columns < 4 * num_sms()) chunk /= 2;
   const dim3 grid(static_cast<unsigned>((tokens + chunk - 1) / chunk),
-                  static_cast<unsigned>((d / 4 + threads - 1) / threads));
+                  static_cast<unsigned>(columns));
   const int vec_ok = (reinterpret_cast<uintptr_t>(dtable) & 15) == 0;
-  auto kernel = chunk == 128 ? embedding_bwd_kernel<128> : embedding_bwd_kernel<16>;
-  kernel<<<grid, threads, 0, static_cast<cudaStream_t>(stream)>>>(
+  embedding_bwd_kernel<<<grid, threads, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const long long*>(ids), static_cast<const __nv_bfloat16*>(dout),
-      static_cast<float*>(dtable), tokens, d, vocab_start, vocab_rows, vec_ok);
+      static_cast<float*>(dtable), tokens, d, vocab_start, vocab_rows, chunk, vec_ok);
   CHECK_LAUNCH("embedding_bwd");
   return 0;
 }
