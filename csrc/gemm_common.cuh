@@ -18,7 +18,8 @@ constexpr int kGemmTraceSlots = 8;
 long long* gemm_trace_buffer();  // host: the calling thread's trace buffer, or null
 #define T5X_GEMM_TRACE(slot)                                                              \
   do {                                                                                    \
-    if (p.trace != nullptr) p.trace[blockIdx.x * kGemmTraceSlots + (slot)] = global_timer_ns(); \
+    if (p.trace != nullptr && static_cast<int>(blockIdx.x) < p.trace_ctas)                  \
+      p.trace[blockIdx.x * kGemmTraceSlots + (slot)] = global_timer_ns();                   \
   } while (0)
 
 constexpr int kCeTileCols = 128;  // columns that one warp folds into one partial
@@ -52,6 +53,7 @@ struct GemmParams {
   // set-up done, first loads issued, first operands landed, last MMA issued, accumulator
   // complete, epilogue done, exit. Null in normal use.
   long long* trace;
+  int trace_ctas;  // CTAs that the buffer has room for: one per SM
   int* status;
   // Cross-entropy epilogues. Column c of the product is vocabulary entry ce_vocab_start + c.
   const long long* ce_targets;  // [M] target ids

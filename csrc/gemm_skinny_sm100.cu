@@ -69,6 +69,7 @@ struct SkinnyParams {
   // loads issued, first operands landed, accumulator complete, tile parked in shared memory,
   // peers' rows received, rows stored.
   long long* trace;
+  int trace_ctas;
 };
 
 // This CTA's shared memory -> another CTA's of the cluster; the bytes are counted on an
@@ -517,6 +518,7 @@ T5X_API int t5x_gemm_skinny_bf16(const void* A, const void* B, void* C, const vo
   p.b_constant = chained_launches_constant_b() ? 1 : 0;
   p.status = device_status_buffer();
   p.trace = gemm_trace_buffer();
+  p.trace_ctas = num_sms();
   // Half-width tiles wherever the tiles are split (us, cold weights, 128 / 64 columns: 256 rows x
   // 2048 x 2048 in 4 11.7 / 11.4, 768 x 768 in 4 9.0 / 7.1, 1024 x 1024 in 8 16.5 / 9.6, 128 rows
   // x 2048 x 2048 in 8 18.2 / 11.1; 5120 x 2048 in 4 16.1 / 16.7). Alone, a tile of 64 columns

@@ -305,6 +305,7 @@ static int launch_gemm(const CUtensorMap* tA, const CUtensorMap* tB, const CUten
   if (grid <= 0) return 0;
   p.b_constant = chained_launches_constant_b() ? 1 : 0;
   p.trace = g_gemm_trace;
+  p.trace_ctas = num_sms();
   cudaError_t e = launch_chained(gemm_bf16_kernel<BN, EPI>, dim3(grid), dim3(kGemmThreads),
                                  S::kTotal, stream, *tA, *tB, *tB2, p);
   count_launches(1);
@@ -423,6 +424,7 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
   p.split_k = 1;
   p.b_constant = 0;
   p.trace = nullptr;
+  p.trace_ctas = 0;
   p.ce_targets = nullptr;
   p.ce_part = nullptr;
   p.ce_arg = nullptr;
@@ -567,10 +569,10 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
 }
 }  // namespace t5x
 
-// Phase trace of the one-CTA-per-tile GEMM for profiling: while `buffer` (device memory, 8
-// int64 per CTA of the largest grid, i.e. 8 x the number of SMs) is set, every such GEMM
-// launched from the calling thread records nanosecond timestamps of its first tile's phases
-// (see GemmParams::trace). Null switches it off.
+// Phase trace of the one-CTA-per-tile and of the cluster GEMM for profiling: while `buffer` (device
+// memory, 8 int64 x the number of SMs) is set, every such GEMM launched from the calling thread
+// records nanosecond timestamps of its first tile's phases (see GemmParams::trace); of a grid of
+// more CTAs than SMs the first ones do. Null switches it off.
 T5X_API int t5x_gemm_set_trace(void* buffer) {
   t5x::g_gemm_trace = static_cast<long long*>(buffer);
   return 0;

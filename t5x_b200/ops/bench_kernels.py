@@ -332,8 +332,7 @@ def gemm_trace(m: int, n: int, k: int, splits: int):
   a = torch.randn(m, k, device="cuda").bfloat16()
   ws = torch.zeros(m, n, dtype=torch.float32, device="cuda")
   sms = torch.cuda.get_device_properties(0).multi_processor_count
-  ctas = 2 * sms  # the cluster kernel runs two per SM
-  trace = torch.zeros(ctas * 8, dtype=torch.int64, device="cuda")
+  trace = torch.zeros(sms * 8, dtype=torch.int64, device="cuda")
   l = native.lib()
   l.t5x_gemm_set_trace.argtypes = [ctypes.c_void_p]
   names = ["entry", "setup_done", "first_loads_issued", "first_operands_landed", "last_mma_issued",
@@ -360,7 +359,7 @@ def gemm_trace(m: int, n: int, k: int, splits: int):
     finally:
       l.t5x_gemm_set_trace(None)
     torch.cuda.synchronize()
-    t = trace.view(ctas, 8).cpu()
+    t = trace.view(sms, 8).cpu()
     t = t[t[:, 0] > 0]
     if it == 0 or not len(t):
       continue  # first launch: descriptor encoding and attribute set-up

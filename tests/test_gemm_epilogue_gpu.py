@@ -129,3 +129,26 @@ def test_weight_gradients_are_cut_where_it_pays(M, N, K, cut):
   whole = native.gemm_wgrad(a.t(), b, pieces=1)
   assert torch.equal(native.gemm_wgrad(a.t(), b), whole) != cut
   native.check_status()
+
+
+def test_phase_trace_stays_inside_its_buffer():
+  """8 int64 per SM are enough for every traced GEMM, also for the 256 CTAs of a cluster product."""
+  import ctypes
+  from t5x_b200.ops import native
+  sms = torch.cuda.get_device_properties(0).multi_processor_count
+  buf = torch.zeros(4 * sms * 8, dtype=torch.int64, device="cuda")
+  a = torch.randn(256, 2048, device="cuda").bfloat16()
+  b = torch.randn(2048, 2048, device="cuda").bfloat16()
+  set_trace = native.lib().t5x_gemm_set_trace
+  set_trace.argtypes = [ctypes.c_void_p]
+  for product in (lambda: native.gemm_skinny(a, b, splits=4), lambda: native.gemm_skinny(a, b, splits=8),
+                  lambda: native.gemm(a[:128], b)):
+    buf.zero_()
+    set_trace(buf.data_ptr())
+    try:
+      product()
+    finally:
+      set_trace(None)
+    t = buf.view(4 * sms, 8).cpu()
+    assert bool((t[0] > 0).any()) and not bool(t[sms:].any())
+  native.check_status()
