@@ -557,7 +557,7 @@ __device__ __forceinline__ void gemm_epilogue_ce_stats(const GemmParams& p, uint
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
         if (i < n_valid) s0 += v[i];
-        else v[i] = -3.0e38f;  // never the maximum, exp gives zero
+        else v[i] = -INFINITY;  // never the maximum, exp gives zero even where every logit is -inf
       }
     }
     sx += s0 + s1;

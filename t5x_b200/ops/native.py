@@ -663,7 +663,7 @@ def _b_layout(b: torch.Tensor):
 def gemm_ce_stats(h: torch.Tensor, w: torch.Tensor, targets: torch.Tensor, alpha: float = 1.0,
                   vocab_start: int = 0):
   """Cross-entropy statistics of logits = alpha * h[M, K] @ w[K, N] without storing the
-  logits: the GEMM epilogue folds every 256-column tile into softmax partials, which a second
+  logits: the GEMM epilogue folds every 128 columns into softmax partials, which a second
   small kernel merges. Returns what `ce_stats` returns: stats [M, 4] = (max, sum exp(x - max),
   target logit, sum x), arg_val [M], arg_idx [M] (vocabulary id of the largest logit)."""
   assert h.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and targets.dtype == torch.int64

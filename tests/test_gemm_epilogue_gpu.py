@@ -152,3 +152,28 @@ def test_phase_trace_stays_inside_its_buffer():
     t = buf.view(4 * sms, 8).cpu()
     assert bool((t[0] > 0).any()) and not bool(t[sms:].any())
   native.check_status()
+
+
+@pytest.mark.parametrize("N", [128, 136, 200])
+def test_cross_entropy_of_infinite_logits(N):
+  """Rows whose logits overflow: all -inf (nothing to sum: the columns that pad a tile to 32 do not
+  count either), one of them finite, one +inf."""
+  from t5x_b200.ops import native
+  big = 2.0 ** 100
+  a = torch.zeros(4, 64, device="cuda", dtype=torch.bfloat16)
+  b = torch.zeros(64, N, device="cuda", dtype=torch.bfloat16)
+  a[0, 0] = a[1, 0] = a[2, 1] = big
+  b[0], b[1, N - 1] = -big, big  # row 0: all -inf; row 2: the last +inf, zeros otherwise
+  a[1, 2], b[0, 5], b[2, 5] = 1.0, 0.0, 3.0  # row 1: 3 in column 5
+  b[0, 5] = 0.0
+  a[0, 3], b[3, 5] = big, -big  # row 0, column 5: -inf as well
+  t = torch.zeros(4, dtype=torch.long, device="cuda")
+  x = a.double() @ b.double()
+  x[x < -1e39], x[x > 1e39] = -float("inf"), float("inf")
+  assert bool((x[0] == -float("inf")).all()) and x[1, 5] == 3.0
+  stats, _, arg = native.gemm_ce_stats(a, b, t)
+  lse = stats[:, 0] + torch.log(stats[:, 1])
+  assert stats[0, 1] == 0 and lse[0] == -float("inf")
+  torch.testing.assert_close(lse[[1, 3]].double(), torch.logsumexp(x[[1, 3]], -1))
+  assert arg[1] == 5 and not bool(torch.isfinite(lse[2]))
+  native.check_status()
