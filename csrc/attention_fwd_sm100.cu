@@ -29,6 +29,7 @@
 // by log2(e) and stored four times with shifts 0..3, so that every thread reads its 128
 // consecutive entries with aligned 16-byte loads whatever its row.
 #include "attention_common.cuh"
+#include "t5x_ops.h"
 
 namespace t5x {
 namespace {

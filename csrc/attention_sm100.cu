@@ -20,6 +20,7 @@
 //           accumulate in TMEM, dQ partial tiles are added to an fp32 buffer with vector
 //           red.global.add.
 #include "attention_common.cuh"
+#include "t5x_ops.h"
 
 namespace t5x {
 

@@ -5,6 +5,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "t5x_ops.h"
 
 namespace t5x {
 

@@ -19,6 +19,7 @@
 #include <algorithm>
 
 #include "gemm_common.cuh"
+#include "t5x_b200.h"
 
 namespace t5x {
 

@@ -17,49 +17,8 @@
 #include <tuple>
 #include <vector>
 
-extern "C" {
-const char* t5x_last_error();
-int t5x_gemm_bf16(const void* A, const void* B, const void* B2, void* C, int M, int N, int K,
-                  int batch, long long lda, long long ldb, long long ldc, long long a_batch_stride,
-                  long long b_batch_stride, long long c_batch_stride, int a_mn_major, int b_mn_major,
-                  int out_fp32, int accumulate, int epilogue, const void* R, long long ldr,
-                  long long r_batch_stride, void* H0, void* H1, long long ldh, float alpha,
-                  int max_ctas, void* stream);
-int t5x_gemm_wgrad_bf16(const void* A, const void* B, void* C, int M, int N, int K, int batch,
-                        long long lda, long long ldb, long long ldc, long long a_batch_stride,
-                        long long b_batch_stride, long long c_batch_stride, int a_mn_major,
-                        int b_mn_major, int accumulate, int last_wave_pieces, void* stream);
-int t5x_rmsnorm_fwd(const void* x, const void* scale, void* y, void* rstd, int rows, int d, float eps,
-                    void* stream);
-int t5x_rmsnorm_bwd(const void* dy, const void* x, const void* scale, const void* rstd,
-                    const void* dres, void* dx, void* dscale, int rows, int d, void* stream);
-int t5x_attention_fwd(const void* q, const void* k, const void* v, void* o, void* lse, int B, int H,
-                      int Lq, int Lk, long long q_sb, long long q_sl, long long q_sh, long long k_sb,
-                      long long k_sl, long long k_sh, long long v_sb, long long v_sl, long long v_sh,
-                      long long o_sb, long long o_sl, long long o_sh, const void* rel_bias,
-                      const void* rel_bucket, int num_buckets, int nrel, int rel_off,
-                      const void* key_mask, const void* q_seg, const void* kv_seg, int causal,
-                      int causal_off, void* stream);
-int t5x_attention_fwd_stream(const void* q, const void* k, const void* v, void* o, void* lse, int B,
-                             int H, int Lq, int Lk, int D, long long q_sb, long long q_sl,
-                             long long q_sh, long long k_sb, long long k_sl, long long k_sh,
-                             long long v_sb, long long v_sl, long long v_sh, long long o_sb,
-                             long long o_sl, long long o_sh, const void* rel_bias,
-                             const void* rel_bucket, int num_buckets, int nrel, int rel_off,
-                             const void* key_mask, const void* q_seg, const void* kv_seg, int causal,
-                             int causal_off, void* stream);
-int t5x_attention_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
-                      const void* lse, void* delta, void* dq_f32, void* dk, void* dv, int B, int H,
-                      int Lq, int Lk, int D, long long q_sb, long long q_sl, long long q_sh,
-                      long long k_sb, long long k_sl, long long k_sh, long long v_sb, long long v_sl,
-                      long long v_sh, long long o_sb, long long o_sl, long long o_sh, long long do_sb,
-                      long long do_sl, long long do_sh, long long dk_sb, long long dk_sl,
-                      long long dk_sh, const void* rel_bias, const void* rel_bucket, void* d_rel_bias,
-                      int num_buckets, int nrel, int rel_off, const void* key_mask, const void* q_seg,
-                      const void* kv_seg, int causal, int causal_off, void* stream);
-int t5x_gated_gelu_bwd(void* dg, void* h, long long rows, int dff, long long ldh, long long ldg,
-                       int write_g, void* stream);
-}
+#include "t5x_b200.h"
+#include "t5x_ops.h"
 
 namespace {
 

@@ -13,6 +13,7 @@ import ctypes
 import os
 import struct
 import threading
+import warnings
 from typing import Optional
 
 import torch
@@ -151,8 +152,9 @@ _host = None
 
 
 def host():
-  """The compiled host path; None with `T5X_B200_HOST_OPS=0`. Like the kernel library it has to be
-  there on a machine with a GPU."""
+  """The compiled host path; None with `T5X_B200_HOST_OPS=0`. Where it can neither be found nor built
+  (no compiler or headers) a warning says so once and the ops launch the same kernels through
+  ctypes."""
   global _host
   if _host is None:
     lib()  # the kernel library it is linked with
@@ -162,7 +164,12 @@ def host():
           _host = False
         else:
           from t5x_b200.ops import build as _build
-          _host = _HostOps(_build.load_host())
+          try:
+            _host = _HostOps(_build.load_host())
+          except (OSError, RuntimeError, ImportError) as e:
+            warnings.warn(f"compiled host path not available, launching through ctypes: {e}",
+                          RuntimeWarning)
+            _host = False
   return _host or None
 
 
