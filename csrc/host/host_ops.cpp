@@ -184,13 +184,13 @@ optional<std::tuple<optional<Tensor>>> gated_in_bwd(const Tensor& dg, const Tens
     return std::nullopt;
   if (need_dw && !(grad_ok(grad0, a, m) && grad_ok(grad1, b, m))) return std::nullopt;
   void* st = stream_of();
+  optional<Tensor> dx;
+  if (need_dx) dx = at::empty_like(x);  // what can run out of memory comes before `h` is overwritten
   check(t5x_gated_gelu_bwd(dg.data_ptr(), h.data_ptr(), m, a.n, 2 * a.n, a.n, 0, st),
         "gated_gelu_bwd");
   const char* d0 = static_cast<const char*>(h.data_ptr());
   const char* d1 = d0 + a.n * 2;
-  optional<Tensor> dx;
   if (need_dx) {
-    dx = at::empty_like(x);
     input_grad(d0, 2 * a.n, m, a, *dx, false, st);
     input_grad(d1, 2 * a.n, m, b, *dx, true, st);
   }

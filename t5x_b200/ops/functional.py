@@ -100,13 +100,14 @@ def _host_linear_bwd(dys, x, weights, needs):
     if any(g is None for g in grads):
       return False, None
     flags = _take_grad_flags(weights)
-  done = host.multi_linear_bwd(list(dys), x, [compute_weight(w, torch.bfloat16) for w in weights],
-                               grads, flags, bool(needs[0]), bool(need_dw))
-  if done is None:
-    if need_dw:
+  done = None
+  try:
+    done = host.multi_linear_bwd(list(dys), x, [compute_weight(w, torch.bfloat16) for w in weights],
+                                 grads, flags, bool(needs[0]), bool(need_dw))
+  finally:
+    if done is None and need_dw:  # declined or raised
       _restore_grad_flags(weights, flags)
-    return False, None
-  return True, done[0]
+  return (False, None) if done is None else (True, done[0])
 
 
 class _LinearFn(torch.autograd.Function):
@@ -377,13 +378,16 @@ class _GatedGeluMlpInFn(torch.autograd.Function):
     g0, g1 = getattr(wi_0, "main_grad", None), getattr(wi_1, "main_grad", None)
     if host is not None and need_0 == need_1 and not (need_0 and (g0 is None or g1 is None)):
       flags = _take_grad_flags([wi_0, wi_1]) if need_0 else [False, False]
-      done = host.gated_in_bwd(dg, x, compute_weight(wi_0, torch.bfloat16),
-                               compute_weight(wi_1, torch.bfloat16), h, g0, g1, *flags,
-                               bool(need_dx), bool(need_0))
+      done = None
+      try:
+        done = host.gated_in_bwd(dg, x, compute_weight(wi_0, torch.bfloat16),
+                                 compute_weight(wi_1, torch.bfloat16), h, g0, g1, *flags,
+                                 bool(need_dx), bool(need_0))
+      finally:
+        if done is None and need_0:
+          _restore_grad_flags([wi_0, wi_1], flags)
       if done is not None:
         return done[0], None, None
-      if need_0:
-        _restore_grad_flags([wi_0, wi_1], flags)
     k = x.shape[-1]
     dff = h.shape[1] // 2
     x2 = x.reshape(-1, k)
