@@ -667,9 +667,12 @@ _SCRATCH = {}
 
 
 def _scratch(device, n_floats: int) -> torch.Tensor:
-  """Grow-only fp32 scratch per device for the kernel phases."""
-  buf = _SCRATCH.get(device)
+  """Grow-only fp32 scratch for the kernel phases, one per device and stream: an update on a side
+  stream may run beside one on another, and a buffer that is outgrown goes back to the stream
+  whose kernels may still use it."""
+  key = (device, torch._C._cuda_getCurrentRawStream(device.index))
+  buf = _SCRATCH.get(key)
   if buf is None or buf.numel() < n_floats:
     buf = torch.empty(max(n_floats, 1 << 16), dtype=torch.float32, device=device)
-    _SCRATCH[device] = buf
+    _SCRATCH[key] = buf
   return buf[:n_floats]

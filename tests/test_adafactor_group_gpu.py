@@ -88,3 +88,18 @@ def test_scratch_is_as_large_as_stated(rows, cols, batch):
     results.append((p, v0, v1, q, full))
   for a, b in zip(*results):
     assert torch.equal(a, b) and bool(torch.isfinite(a).all())
+
+
+def test_scratch_belongs_to_one_stream(monkeypatch):
+  """Updates on two streams share no scratch, and a buffer that grows is replaced on its own
+  stream only."""
+  from t5x_b200 import adafactor
+  dev = torch.device("cuda", torch.cuda.current_device())
+  monkeypatch.setattr(adafactor, "_SCRATCH", {})
+  here = adafactor._scratch(dev, 1000).data_ptr()
+  side = torch.cuda.Stream()
+  with torch.cuda.stream(side):
+    there = adafactor._scratch(dev, 1000).data_ptr()
+    grown = adafactor._scratch(dev, 1 << 20)
+  assert len({here, there, grown.data_ptr()}) == 3
+  assert adafactor._scratch(dev, 1000).data_ptr() == here
