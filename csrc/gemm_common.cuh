@@ -336,7 +336,7 @@ struct GemmWork {
 
 // Epilogue of one 128-row accumulator tile held in TMEM columns [t_cols, t_cols + BN): the
 // calling warp owns lane quarter q (rows m0 + 32q .. +31) and part `part` of PARTS of the tile's
-// columns, `c_vec_ok` says whether 16-byte stores to C are legal.
+// columns, `c_vec_ok` says whether 16-byte accesses to a bf16 C are legal in every batch.
 template <int BN, int EPI, int PARTS>
 __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t t_row, int m0,
                                                    int n0, int b, int q, int part, int lane,
@@ -392,14 +392,16 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
         }
         store_row_bf16(out + col, g, n_valid, c_vec_ok);
         if (p.H0 != nullptr) {
-          const bool hv = (p.ldh % 8 == 0);
-          store_row_bf16(p.H0 + static_cast<long long>(row) * p.ldh + col, h0, n_valid, hv);
-          store_row_bf16(p.H1 + static_cast<long long>(row) * p.ldh + col, h1, n_valid, hv);
+          store_row_bf16(p.H0 + static_cast<long long>(row) * p.ldh + col, h0, n_valid, hv16);
+          store_row_bf16(p.H1 + static_cast<long long>(row) * p.ldh + col, h1, n_valid, hv16);
         }
       }
     }
   } else {
-    const bool b_step_ok = p.c_batch_stride % 8 == 0;
+    const bool f32_vec_ok = p.ldc % 4 == 0 && p.c_batch_stride % 4 == 0 &&
+                            (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
+    const bool r_vec_ok = EPI == kEpiResidual && p.ldr % 8 == 0 && p.r_batch_stride % 8 == 0 &&
+                          (reinterpret_cast<uintptr_t>(p.R) & 15) == 0;
 #pragma unroll 1
     for (int c = part * (BN / 32 / PARTS); c < (part + 1) * (BN / 32 / PARTS); ++c) {
       const int col = n0 + c * 32;
@@ -409,13 +411,9 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
       tmem_ld32(t_row + c * 32, r);
       // whole 32-column blocks go out through the staging buffer (warp-uniform condition)
       const bool staged = stage != nullptr && n_valid >= 32 && rows_valid > 0 &&
-                          (p.out_fp32 ? (p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0)
-                                      : (c_vec_ok && (accumulate == 0 ||
-                                                       (EPI != kEpiResidual && b_step_ok))));
+                          (p.out_fp32 ? f32_vec_ok
+                                      : (c_vec_ok && (accumulate == 0 || EPI != kEpiResidual)));
       if (staged) {
-        const bool r_vec_ok = EPI == kEpiResidual && p.ldr % 8 == 0 &&
-                              p.r_batch_stride % 8 == 0 &&
-                              (reinterpret_cast<uintptr_t>(p.R) & 15) == 0;
         if (EPI == kEpiResidual && r_vec_ok)
           staged_load_bf16(stage, p.R + b * p.r_batch_stride +
                                       static_cast<long long>(m0 + q * 32) * p.ldr + col,
@@ -464,17 +462,15 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
         if (EPI == kEpiResidual) {
           float rr[32];
-          const bool rv = (p.ldr % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.R) & 15) == 0);
           load_row_bf16(p.R + b * p.r_batch_stride + static_cast<long long>(row) * p.ldr + col,
-                        rr, n_valid, rv);
+                        rr, n_valid, r_vec_ok);
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] += rr[i];
         }
         if (p.out_fp32) {
           float* out = reinterpret_cast<float*>(p.C) + b * p.c_batch_stride +
                        static_cast<long long>(row) * p.ldc + col;
-          const bool fv = (p.ldc % 4 == 0) && n_valid >= 32;
-          if (fv) {
+          if (f32_vec_ok && n_valid >= 32) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               float4 o = make_float4(v[i * 4], v[i * 4 + 1], v[i * 4 + 2], v[i * 4 + 3]);

@@ -397,7 +397,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
     int local = 0;
     bool ok = true;
     chain_wait();  // the epilogue reads residuals and writes C
-    const bool c_vec_ok = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
+    const bool c_vec_ok = p.ldc % 8 == 0 && p.c_batch_stride % 8 == 0 &&
+                          (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
     const uint32_t drained = mapa_shared(smem_u32(&tmem_empty[0]), 0);
     GemmWork work(p, pair, num_pairs, total_tiles, num_kb);
     for (int tile, kb0, kb1; ok && work.next(tile, kb0, kb1); ++local) {

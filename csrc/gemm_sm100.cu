@@ -240,7 +240,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     int local = 0;
     bool ok = true;
     chain_wait();  // the epilogue reads residuals and writes C
-    const bool c_vec_ok = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
+    const bool c_vec_ok = p.ldc % 8 == 0 && p.c_batch_stride % 8 == 0 &&
+                          (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++local) {
       const int acc = local & 1;
       const uint32_t acc_phase = (local >> 1) & 1;

@@ -39,6 +39,51 @@ def test_residual_and_accumulate(M, N, K, pair):
   native.check_status()
 
 
+def _views(M, N, dtype):
+  """(name, make): [M, N] and [3, M, N] outputs whose rows, start or batches lie on and off 16 bytes."""
+  unit = 8 if dtype == torch.bfloat16 else 4
+  ld = -(-N // unit) * unit
+
+  def of(batch, ld, step, start):
+    flat = torch.randn(max(batch, 1) * max(step, M * ld) + start + 64, device="cuda").to(dtype)
+    return flat.as_strided((M, N) if batch == 0 else (batch, M, N),
+                           (ld, 1) if batch == 0 else (step, ld, 1), start)
+  return [("whole", of(0, ld, 0, 0)), ("rows apart", of(0, ld + unit, 0, 0)),
+          ("odd rows", of(0, ld + 1, 0, 0)), ("odd start", of(0, ld, 0, 1)),
+          ("batches", of(3, ld, M * ld + unit, 0)), ("odd batches", of(3, ld, M * ld + 1, 0))]
+
+
+@pytest.mark.parametrize("pair", [0, 2])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,K", SHAPES + [(70, 100, 64)])
+def test_store_and_add_at_any_alignment(M, N, K, dtype, pair):
+  """C = and C += in both output types. A bf16 result is rounded once: 2^-9 relative, with a factor
+  of two; the fp32 sums of K products as above."""
+  from t5x_b200.ops import native
+  native.gemm_set_pair_mode(pair)
+  rtol = 2 ** -8 if dtype == torch.bfloat16 else 1e-5
+  try:
+    for name, out in _views(M, N, dtype):
+      batch = out.shape[0] if out.dim() == 3 else 1
+      ops = [_operands(M, -(-N // 8) * 8, K, M + N + i) for i in range(batch)]
+      a, b = (torch.stack([o[i] for o in ops]) for i in (0, 1))
+      if out.dim() == 2:
+        a, b = a[0], b[0]
+      b = b[..., :N]
+      want = a.double() @ b.double()
+      old = out.clone()
+      native.gemm(a, b, out=out, accumulate=True)
+      torch.testing.assert_close(out.double(), want + old.double(), rtol=rtol, atol=2e-5, msg=lambda m: name + m)
+      native.gemm(a, b, out=out)
+      torch.testing.assert_close(out.double(), want, rtol=rtol, atol=2e-5, msg=lambda m: name + m)
+      if dtype == torch.bfloat16:
+        y = native.gemm(a, b, residual=out)  # the same views as a residual
+        torch.testing.assert_close(y.double(), want + out.double(), rtol=rtol, atol=2e-5)
+  finally:
+    native.gemm_set_pair_mode(1)
+  native.check_status()
+
+
 @pytest.mark.parametrize("pair", [0, 1])
 @pytest.mark.parametrize("M,N,K", [(1, 64, 64), (37, 129, 64), (256, 128, 64), (300, 1000, 128),
                                    (515, 2184, 64)])
