@@ -1,7 +1,8 @@
 """The compiled host path and the general Python path run the same kernels on the same operands, so
-their results are equal bit by bit (weight gradients: up to the order of atomic adds). Forms that
-the compiled path declines (strided activations, 3-D weights, frozen weights, no gradient buffer,
-fp32 inputs to fused ops) give the same answers through the general path."""
+their results are equal bit by bit (weight gradients: up to the order of atomic adds). Which calls ran
+compiled is counted. Forms that the compiled path declines (strided activations and residuals) or is
+not asked for (weights partly frozen or without a gradient buffer) give the same answers through
+the general path."""
 import pytest
 import torch
 
@@ -18,10 +19,38 @@ def _param(*shape, main_grad=True, seed=0):
   return p
 
 
+class _Spy:
+  """The compiled path, with how often each function covered a call and how often it declined."""
+
+  def __init__(self, host):
+    self.covered, self.declined = {}, {}
+    for name in host.NAMES:
+      setattr(self, name, self._watch(name, getattr(host, name)))
+
+  def _watch(self, name, fn):
+    def call(*args):
+      out = fn(*args)
+      side = self.declined if out is None else self.covered
+      side[name] = side.get(name, 0) + 1
+      return out
+    return call
+
+
+def _spy(monkeypatch, host):
+  from t5x_b200.ops import native
+  spy = _Spy(native.host()) if host else None
+  monkeypatch.setattr(native, "host", lambda: spy)
+  return spy
+
+
 def _run(host, case, monkeypatch):
-  from t5x_b200.ops import functional as F, native
-  if not host:
-    monkeypatch.setattr(native, "host", lambda: None)
+  from t5x_b200.ops import functional as F
+  with monkeypatch.context() as m:
+    spy = _spy(m, host)
+    return _passes(F, case) + (spy,)
+
+
+def _passes(F, case):
   g = torch.Generator(device="cuda").manual_seed(3)
   rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
   x = rnd(3, 50, 256).requires_grad_()
@@ -52,8 +81,17 @@ def _run(host, case, monkeypatch):
 
 @pytest.mark.parametrize("case", ["plain", "strided", "three_dim", "frozen", "no_buffer"])
 def test_same_as_the_general_path(case, monkeypatch):
-  a, ga = _run(True, case, monkeypatch)
-  b, gb = _run(False, case, monkeypatch)
+  a, ga, spy = _run(True, case, monkeypatch)
+  b, gb, _ = _run(False, case, monkeypatch)
+  every = {"linear", "multi_linear", "multi_linear_bwd", "gated_in", "gated_in_bwd", "rmsnorm",
+           "rmsnorm_bwd"}
+  # the calls it declines; everything else ran compiled
+  declined = {"rmsnorm", "linear"} if case == "strided" else set()
+  assert set(spy.declined) == declined, (spy.covered, spy.declined)
+  if case in ("plain", "three_dim"):
+    assert set(spy.covered) == every
+  elif case == "no_buffer":
+    assert set(spy.covered) == every - {"multi_linear_bwd", "gated_in_bwd"}
   assert len(ga) == len(gb)
   for x, y in zip(a, b):
     assert torch.equal(x, y)
@@ -64,7 +102,7 @@ def test_same_as_the_general_path(case, monkeypatch):
 @pytest.mark.parametrize("lq,lk,d,packed,segments", [(130, 70, 64, False, False), (96, 96, 64, True, True),
                                                      (600, 600, 128, False, True)])
 def test_attention_same_as_the_general_path(lq, lk, d, packed, segments, monkeypatch):
-  from t5x_b200.ops import attention as attn, native
+  from t5x_b200.ops import attention as attn
   g = torch.Generator(device="cuda").manual_seed(lq)
   if packed:
     qkv = torch.randn(2, lq, 3, 2, d, device="cuda", generator=g).bfloat16().requires_grad_()
@@ -78,12 +116,14 @@ def test_attention_same_as_the_general_path(lq, lk, d, packed, segments, monkeyp
   mask = torch.rand(2, lk, device="cuda", generator=g) > 0.2
   res = []
   for host in (True, False):
-    if not host:
-      monkeypatch.setattr(native, "host", lambda: None)
-    table = torch.nn.Parameter(torch.linspace(-1, 1, 64, device="cuda").view(2, 32))
-    o = attn.flash_attention(q, k, v, bias_table=table, key_mask=mask, q_segment_ids=seg(lq),
-                             kv_segment_ids=seg(lk))
-    res.append([o.detach(), *torch.autograd.grad(o, leaves + [table], do)])
+    with monkeypatch.context() as m:
+      spy = _spy(m, host)
+      table = torch.nn.Parameter(torch.linspace(-1, 1, 64, device="cuda").view(2, 32))
+      o = attn.flash_attention(q, k, v, bias_table=table, key_mask=mask, q_segment_ids=seg(lq),
+                               kv_segment_ids=seg(lk))
+      res.append([o.detach(), *torch.autograd.grad(o, leaves + [table], do)])
+    if host:
+      assert spy.covered == {"attention": 1, "attention_bwd": 1} and not spy.declined
   for x, y in zip(*res):
     # dq and the bias gradient are sums of atomic adds, rounded to bf16
     assert float((x - y).float().norm() / y.float().norm()) < 2 ** -8
