@@ -24,7 +24,6 @@ constexpr int kAfThreads = 256;
 constexpr int kAfTileR = 64;
 constexpr int kAfTileC = 512;
 
-// One 64 x 512 tile (tile_x, tile_y) of batch element b: row and column sums of g^2 + eps1, sum p^2.
 // Sums that meet in memory by atomic adds (F: their type, S: the struct of the scalar ones). In
 // fp32 their order shows in the last bit of every parameter; grouped launches hold them in fp64,
 // where it does not survive the rounding to fp32.
@@ -47,6 +46,7 @@ __device__ __forceinline__ float (*af_column_slots())[kAfTileC] {
   return slots;
 }
 
+// One 64 x 512 tile (tile_x, tile_y) of batch element b: row and column sums of g^2 + eps1, sum p^2.
 template <bool VEC, class F, class S>
 __device__ __forceinline__ void af_stats_tile(const float* __restrict__ g,
                                               const float* __restrict__ p,

@@ -405,10 +405,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// head_dim 64: Q / dO double-buffered, the scores of the next query block are issued while the
-// softmax warps work, dQ partial tiles alternate between two TMEM buffers. head_dim 128: operand
-// tiles are twice as large and dK, dV take twice the TMEM columns, so Q / dO have one stage, dQ
-// reuses the columns of S^T and the query blocks run one after the other.
 constexpr int kSmemBuckets = 128;  // tables with more buckets add to memory directly
 // P and dS of 16 scores of one key that all count: rel points at the bias of the first, the next
 // ones lie below it.
@@ -449,6 +445,10 @@ __device__ __forceinline__ void transpose_pieces(uint32_t* v, int lane) {
   }
 }
 
+// head_dim 64: Q / dO double-buffered, the scores of the next query block are issued while the
+// softmax warps work, dQ partial tiles alternate between two TMEM buffers. head_dim 128: operand
+// tiles are twice as large and dK, dV take twice the TMEM columns, so Q / dO have one stage, dQ
+// reuses the columns of S^T and the query blocks run one after the other.
 template <int D>
 struct BwdSmem {
   static constexpr int kTile = 128 * 128;  // bytes of a [128 x 64] bf16 panel

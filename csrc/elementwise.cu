@@ -95,11 +95,6 @@ __global__ void __launch_bounds__(kNormThreads)
 //   g = dy * scale ;  dx = rstd * (g - x * rstd^2 * mean(g * x)) (+ dres)
 //   dscale[j] += sum_rows dy * x * rstd            (per-CTA partial sums, then one reduction)
 // ---------------------------------------------------------------------------
-// NV = 16-byte vectors per thread (d <= 2048 * NV). Operands stay packed (bf16) in registers
-// between the two passes over a row and the scale is re-read from L1, so that four CTAs fit an
-// SM for d <= 4096: the kernel is bound by how many rows are in flight. The per-feature sums
-// for dscale are kept in registers over the CTA's rows and written to `partial`
-// ([gridDim.x, d], plain stores); rmsnorm_dscale_reduce_kernel adds them up.
 // The operands of one row of the backward pass, packed: thread `t` of THREADS holds 16-byte pieces
 // t, t + THREADS, ... of it. Loaded one row ahead of their use; the residual's gradient only
 // where the registers last for it (RES).
@@ -125,6 +120,11 @@ struct NormRow {
 };
 constexpr int norm_bwd_ctas(int nv) { return nv <= 2 ? 4 : 2; }  // per SM
 
+// NV = 16-byte vectors per thread (d <= 2048 * NV). Operands stay packed (bf16) in registers
+// between the two passes over a row and the scale is re-read from L1, so that four CTAs fit an
+// SM for d <= 4096: the kernel is bound by how many rows are in flight. The per-feature sums
+// for dscale are kept in registers over the CTA's rows and written to `partial`
+// ([gridDim.x, d], plain stores); rmsnorm_dscale_reduce_kernel adds them up.
 template <int NV>
 __global__ void __launch_bounds__(kNormThreads, norm_bwd_ctas(NV))
     rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,

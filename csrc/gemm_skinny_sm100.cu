@@ -24,7 +24,8 @@
 // 256 rows x 2048 x 2048; with eight, and the parts requested together, 1.3 and 1.5). Every
 // thread reaches both cluster barriers (one right after set-up, one before exit) whatever
 // happened before (a wait that gave up raises the CTA's abort flag and a status word, and the
-// CTA skips its work but still arrives), so a failure cannot leave the cluster waiting. No TMA load uses cluster multicast.
+// CTA skips its work but still arrives), so a failure cannot leave the cluster waiting. No TMA
+// load uses cluster multicast.
 #include <algorithm>
 
 #include "gemm_common.cuh"

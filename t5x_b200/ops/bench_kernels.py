@@ -156,6 +156,20 @@ def bench_streaming():
   dres = torch.randn(T, d, **bf)
   report("rmsnorm_bwd_with_residual_grad",
          lambda: native.rmsnorm_bwd(dy, x, scale, rstd, dres, dscale), 4 * T * d * 2)
+  # the warp kernels of narrower rows (T5.1.1 base), at 65536 tokens
+  Tn, dn = 65536, 768
+  xn, sn = torch.randn(Tn, dn, **bf), torch.ones(dn, device=dev)
+  report("rmsnorm_fwd_narrow", lambda: native.rmsnorm_fwd(xn, sn, 1e-6), 2 * Tn * dn * 2, rows=Tn,
+         d=dn)
+  yn, rn = native.rmsnorm_fwd(xn, sn, 1e-6)
+  dsn = torch.zeros(dn, device=dev)
+  report("rmsnorm_bwd_narrow_with_residual_grad",
+         lambda: native.rmsnorm_bwd(xn, xn, sn, rn, yn, dsn), 4 * Tn * dn * 2)
+  # embedding gradient: gradients read once, every row of the table that occurs read and written
+  idn = torch.randint(0, 32128, (Tn,), device=dev)
+  dtab = torch.zeros(32128, dn, device=dev)
+  report("embedding_bwd", lambda: native.embedding_bwd_(idn, xn, dtab),
+         Tn * dn * 2 + 2 * int(idn.unique().numel()) * dn * 4)
   # gated GELU backward on the saved [T, 2 * d_ff] pre-activations
   ff = 10240
   h = torch.randn(T, 2 * ff, **bf)
@@ -185,6 +199,10 @@ def bench_streaming():
     # p read and written in fp32, g read twice (statistics, then the update), bf16 copy written
     report("adafactor_factored_update",
            lambda: opt.apply_param_gradient(3, hp, p, state, g, "mlp/wi_0/kernel"),
+           n * (4 + 4 + 2 * 4 + 2))
+    # the same parameter through the grouped kernels, four launches for a whole list
+    report("adafactor_grouped_update",
+           lambda: opt.apply_param_gradients(3, hp, [(p, state, g, "mlp/wi_0/kernel")]),
            n * (4 + 4 + 2 * 4 + 2))
   from t5x_b200.ops import comm
   mu, nu = torch.zeros_like(p), torch.zeros_like(p)
