@@ -127,7 +127,8 @@ class _FlashAttentionFn(torch.autograd.Function):
     d_rel = ret_rel = None  # the buffer the kernel adds to, and what autograd gets
     if rel_bias is not None and ctx.needs_input_grad[3]:
       mg = getattr(rel_bias, "main_grad", None)
-      if mg is not None and mg.is_contiguous():
+      if (mg is not None and mg.dtype == torch.float32 and mg.is_contiguous() and
+          mg.shape == rel_bias.shape and mg.device == rel_bias.device):
         if not getattr(rel_bias, "grad_ready", False):
           mg.zero_()
           rel_bias.grad_ready = True
@@ -205,8 +206,11 @@ def flash_attention(q, k, v, *, bias_table: Optional[torch.Tensor] = None,
   if bias_table is not None:
     # an fp32 parameter goes in as it is, so that its gradient buffer is found in backward
     rel_bias = bias_table.float().contiguous()
-    if rel_bias.shape[1] < num_buckets:
-      raise ValueError(f"bias table has {rel_bias.shape[1]} buckets, {num_buckets} are indexed")
+    if rel_bias.device != q.device:  # the kernels read it by its address
+      raise ValueError(f"bias table on {rel_bias.device}, queries on {q.device}")
+    if rel_bias.shape[0] < H or rel_bias.shape[1] < num_buckets:
+      raise ValueError(f"bias table {tuple(rel_bias.shape)}: {H} heads and {num_buckets} buckets are "
+                       "indexed")
     buckets = _rel_buckets(Lq, Lk, q_offset, bidirectional, num_buckets, max_distance, q.device)
   km = _byte_mask(key_mask) if key_mask is not None else None
   qs = q_segment_ids.to(torch.int32).contiguous() if q_segment_ids is not None else None

@@ -242,3 +242,21 @@ def test_backward_of_whole_and_partial_blocks(lq, lk, d, masked):
       (q, k, v, table), do.float())
   for n, a, b in zip(("dq", "dk", "dv", "dbias"), got, want):
     assert rel(a, b) < TOL, (n, rel(a, b))
+
+
+def test_bias_gradient_with_a_buffer_the_kernel_cannot_add_to():
+  """The kernel adds fp32 sums; a gradient buffer of another type or layout is left alone and the
+  gradient arrives through autograd."""
+  from t5x_b200.ops import attention as A
+  x = torch.randn(2, 40, 2, 64, device="cuda").bfloat16()
+  grads = []
+  for buf in (None, torch.full((2, 32), 7.0, device="cuda", dtype=torch.bfloat16),
+              torch.full((32, 2), 7.0, device="cuda").t()):
+    table = torch.nn.Parameter(torch.linspace(-1, 1, 64, device="cuda").view(2, 32))
+    if buf is not None:
+      table.main_grad = buf
+    A.flash_attention(x, x, x, bias_table=table).float().square().sum().backward()
+    assert buf is None or bool((buf == 7.0).all())
+    grads.append(table.grad)
+  for g in grads[1:]:
+    torch.testing.assert_close(g, grads[0], rtol=1e-3, atol=1e-3 * float(grads[0].abs().max()))

@@ -166,3 +166,14 @@ def test_relative_position_bucket_against_an_independent_implementation(bidirect
   got = ref.relative_position_bucket(rel, bidirectional, num_buckets, max_distance)
   assert got.tolist() == want.tolist()
   assert int(got.min()) >= 0 and int(got.max()) < num_buckets
+
+
+@pytest.mark.parametrize("table", [torch.zeros(4, 32), torch.zeros(3, 32, device="meta"),
+                                   torch.zeros(4, 31, device="meta")])
+def test_flash_attention_refuses_a_bias_table_it_would_read_out_of_range(table):
+  """On another device than the queries, with fewer heads, or with fewer buckets than are indexed:
+  refused before any kernel gets its address."""
+  from t5x_b200.ops import attention
+  q = torch.zeros(1, 8, 4, 64, dtype=torch.bfloat16, device="meta")
+  with pytest.raises(ValueError, match="bias table"):
+    attention.flash_attention(q, q, q, bias_table=table)
