@@ -33,6 +33,24 @@ enum GemmEpilogue : int {
   kEpiCeGrad = 4,   // gradient of the cross-entropy w.r.t. the logits, written as bf16
 };
 
+// Several products in one launch, three at most (the projections that share an input).
+//   kGroupColumns  C_i = A B_i: the tile columns of the outputs stand side by side, so that a wave
+//                  holds tiles of all of them and the rows of A are read once for all.
+//   kGroupSum      C = A_0 B_0 + A_1 B_1 + ...: the k blocks follow one another in one accumulator, so
+//                  that C is written once, from fp32 sums, instead of read and rounded in between.
+enum GemmGroupKind : int { kGroupNone = 0, kGroupColumns = 1, kGroupSum = 2 };
+constexpr int kMaxGroup = 3;
+template <bool GROUPED>
+struct GemmMaps {  // the operands' tensor maps; gated GELU: wi_0 and wi_1 are b[0] and b[1]
+  CUtensorMap a[GROUPED ? kMaxGroup : 1];
+  CUtensorMap b[GROUPED ? kMaxGroup : 2];
+};
+struct GemmOut {  // where a tile goes
+  void* C;
+  long long ldc;
+  int N;
+};
+
 struct GemmParams {
   int M, N, K, batch;
   int a_mn, b_mn;
@@ -48,6 +66,12 @@ struct GemmParams {
   int tiles_m, tiles_n;
   int mt_rot;  // the row-tile walk starts at this tile (tensor-parallel kernels); 0 otherwise
   int split_k;     // CTA pairs: pieces that the tiles of the last wave are cut into (see GemmWork)
+  // Groups: the first tile column of each output (kGroupColumns) or the first k block of each product
+  // (kGroupSum), INT_MAX where there is none; k blocks in all; the outputs.
+  int group_at[kMaxGroup];
+  int group_num_kb;
+  int vec_ok;              // groups: 16-byte accesses are legal in every bf16 output
+  GemmOut out[kMaxGroup];  // out[0] is C, ldc, N
   int b_constant;  // B is not written by any kernel in flight: it may be loaded before chain_wait()
   // Optional phase trace (t5x_gemm_set_trace): 8 timestamps per CTA for its first tile: entry,
   // set-up done, first loads issued, first operands landed, last MMA issued, accumulator
@@ -297,6 +321,11 @@ __device__ __forceinline__ void gemm_tile_coords(const GemmParams& p, int tile, 
   }
 }
 
+// Which output (product) tile column (k block) `at` belongs to.
+__device__ __forceinline__ int gemm_group_of(const GemmParams& p, int at) {
+  return (at >= p.group_at[1] ? 1 : 0) + (at >= p.group_at[2] ? 1 : 0);
+}
+
 // The work of a CTA pair, in order: every num_units-th tile, whole, except that with split_k > 1
 // the tiles of the last wave, which would leave most of the chip idle (160 tiles on 74 pairs: 2.16
 // waves of work in the time of 3), are cut into split_k pieces along K and dealt out piece by
@@ -336,9 +365,9 @@ struct GemmWork {
 
 // Epilogue of one 128-row accumulator tile held in TMEM columns [t_cols, t_cols + BN): the
 // calling warp owns lane quarter q (rows m0 + 32q .. +31) and part `part` of PARTS of the tile's
-// columns, `c_vec_ok` says whether 16-byte accesses to a bf16 C are legal in every batch.
+// columns of output `o`, `c_vec_ok` says whether 16-byte accesses to a bf16 C are legal in every batch.
 template <int BN, int EPI, int PARTS>
-__device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t t_row, int m0,
+__device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, const GemmOut& o, uint32_t t_row, int m0,
                                                    int n0, int b, int q, int part, int lane,
                                                    bool c_vec_ok, int accumulate,
                                                    float* stage = nullptr) {
@@ -348,17 +377,17 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
 
   if (EPI == kEpiGatedGelu) {
     constexpr int kHalf = BN / 2;
-    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + b * p.c_batch_stride +
-                         static_cast<long long>(row) * p.ldc;
+    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(o.C) + b * p.c_batch_stride +
+                         static_cast<long long>(row) * o.ldc;
 #pragma unroll 1
     for (int c = part * (kHalf / 32 / PARTS); c < (part + 1) * (kHalf / 32 / PARTS); ++c) {
-      if (n0 + c * 32 >= p.N) break;  // warp-uniform: columns beyond the output
+      if (n0 + c * 32 >= o.N) break;  // warp-uniform: columns beyond the output
       uint32_t r0[32], r1[32];
       tmem_ld32(t_row + c * 32, r0);
       tmem_ld32(t_row + kHalf + c * 32, r1);
       tmem_ld_wait();
       const int col = n0 + c * 32;
-      const int n_valid = p.N - col;
+      const int n_valid = o.N - col;
       const bool hv16 = p.H0 == nullptr ||
                         ((p.ldh % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.H0) |
                                                reinterpret_cast<uintptr_t>(p.H1)) & 15) == 0);
@@ -373,9 +402,9 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
         }
         const long long first_row = m0 + q * 32;
         staged_store_bf16(stage, g,
-                          reinterpret_cast<__nv_bfloat16*>(p.C) + b * p.c_batch_stride +
-                              first_row * p.ldc + col,
-                          p.ldc, rows_valid, lane);
+                          reinterpret_cast<__nv_bfloat16*>(o.C) + b * p.c_batch_stride +
+                              first_row * o.ldc + col,
+                          o.ldc, rows_valid, lane);
         if (p.H0 != nullptr) {
           staged_store_bf16(stage, h0, p.H0 + first_row * p.ldh + col, p.ldh, rows_valid, lane);
           staged_store_bf16(stage, h1, p.H1 + first_row * p.ldh + col, p.ldh, rows_valid, lane);
@@ -398,14 +427,14 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
       }
     }
   } else {
-    const bool f32_vec_ok = p.ldc % 4 == 0 && p.c_batch_stride % 4 == 0 &&
-                            (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
+    const bool f32_vec_ok = o.ldc % 4 == 0 && p.c_batch_stride % 4 == 0 &&
+                            (reinterpret_cast<uintptr_t>(o.C) & 15) == 0;
     const bool r_vec_ok = EPI == kEpiResidual && p.ldr % 8 == 0 && p.r_batch_stride % 8 == 0 &&
                           (reinterpret_cast<uintptr_t>(p.R) & 15) == 0;
 #pragma unroll 1
     for (int c = part * (BN / 32 / PARTS); c < (part + 1) * (BN / 32 / PARTS); ++c) {
       const int col = n0 + c * 32;
-      const int n_valid = p.N - col;
+      const int n_valid = o.N - col;
       if (n_valid <= 0) break;  // warp-uniform: columns beyond the output
       uint32_t r[32];
       tmem_ld32(t_row + c * 32, r);
@@ -419,12 +448,12 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
                                       static_cast<long long>(m0 + q * 32) * p.ldr + col,
                            p.ldr, rows_valid, lane);
         const long long first = b * p.c_batch_stride +
-                                static_cast<long long>(m0 + q * 32) * p.ldc + col;
+                                static_cast<long long>(m0 + q * 32) * o.ldc + col;
         // bf16 C += : what is there comes in the same way as a residual (65536 x 768 x 768
         // 118 us with 16-byte reads of 32 rows, 94 so)
         const bool add_c = EPI != kEpiResidual && accumulate != 0 && !p.out_fp32;
         if (add_c)
-          staged_load_bf16(stage, reinterpret_cast<const __nv_bfloat16*>(p.C) + first, p.ldc,
+          staged_load_bf16(stage, reinterpret_cast<const __nv_bfloat16*>(o.C) + first, o.ldc,
                            rows_valid, lane);
         tmem_ld_wait();
         float v[32];
@@ -443,15 +472,15 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
           }
         }
         if (p.out_fp32) {
-          float* dst = reinterpret_cast<float*>(p.C) + first;
+          float* dst = reinterpret_cast<float*>(o.C) + first;
           if (accumulate == 2)
-            staged_store_f32<2>(stage, v, dst, p.ldc, rows_valid, lane);
+            staged_store_f32<2>(stage, v, dst, o.ldc, rows_valid, lane);
           else if (accumulate == 1)
-            staged_store_f32<1>(stage, v, dst, p.ldc, rows_valid, lane);
+            staged_store_f32<1>(stage, v, dst, o.ldc, rows_valid, lane);
           else
-            staged_store_f32<0>(stage, v, dst, p.ldc, rows_valid, lane);
+            staged_store_f32<0>(stage, v, dst, o.ldc, rows_valid, lane);
         } else
-          staged_store_bf16(stage, v, reinterpret_cast<__nv_bfloat16*>(p.C) + first, p.ldc,
+          staged_store_bf16(stage, v, reinterpret_cast<__nv_bfloat16*>(o.C) + first, o.ldc,
                             rows_valid, lane);
         continue;
       }
@@ -468,24 +497,24 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
           for (int i = 0; i < 32; ++i) v[i] += rr[i];
         }
         if (p.out_fp32) {
-          float* out = reinterpret_cast<float*>(p.C) + b * p.c_batch_stride +
-                       static_cast<long long>(row) * p.ldc + col;
+          float* out = reinterpret_cast<float*>(o.C) + b * p.c_batch_stride +
+                       static_cast<long long>(row) * o.ldc + col;
           if (f32_vec_ok && n_valid >= 32) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              float4 o = make_float4(v[i * 4], v[i * 4 + 1], v[i * 4 + 2], v[i * 4 + 3]);
+              float4 w = make_float4(v[i * 4], v[i * 4 + 1], v[i * 4 + 2], v[i * 4 + 3]);
               if (accumulate == 2) {  // several CTAs (split K) add into the same tile
-                atomicAdd(reinterpret_cast<float4*>(out) + i, o);
+                atomicAdd(reinterpret_cast<float4*>(out) + i, w);
                 continue;
               }
               if (accumulate) {
                 float4 old = reinterpret_cast<float4*>(out)[i];
-                o.x += old.x;
-                o.y += old.y;
-                o.z += old.z;
-                o.w += old.w;
+                w.x += old.x;
+                w.y += old.y;
+                w.z += old.z;
+                w.w += old.w;
               }
-              reinterpret_cast<float4*>(out)[i] = o;
+              reinterpret_cast<float4*>(out)[i] = w;
             }
           } else {
 #pragma unroll
@@ -498,8 +527,8 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, uint32_t
             }
           }
         } else {
-          __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + b * p.c_batch_stride +
-                               static_cast<long long>(row) * p.ldc + col;
+          __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(o.C) + b * p.c_batch_stride +
+                               static_cast<long long>(row) * o.ldc + col;
           if (accumulate) {
             float old[32];
             load_row_bf16(out, old, n_valid, c_vec_ok);

@@ -66,11 +66,11 @@ constexpr int pair_smem() {
 static_assert(kPairSmemTotal + 4 * kRsStageBytesPerWarp <= 232448, "shared memory per CTA");
 static_assert(kPairSmemTotal + kEpiWarps * kEpiStageBytesPerWarp <= 232448, "shared memory per CTA");
 
-template <int EPI, int MODE = kTpNone>
+template <int EPI, int MODE = kTpNone, int GROUP = kGroupNone>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>(), 1)
-    gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                     const __grid_constant__ CUtensorMap tmB2, const GemmParams p,
+    gemm_pair_kernel(const __grid_constant__ GemmMaps<GROUP != kGroupNone> maps, const __grid_constant__ GemmParams p,
                      const __grid_constant__ GemmTp tp) {
+  static_assert(GROUP == kGroupNone || (EPI == kEpiPlain && MODE == kTpNone), "groups are plain");
   constexpr int BN = kPairBN;
   constexpr int kStages = kPairStages;
   constexpr int kTileN = (EPI == kEpiGatedGelu) ? BN / 2 : BN;
@@ -110,9 +110,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
       for (int a = 0; a < kTpSlots; ++a) mbar_init(&copy_full[a], 1);
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&tmA);
-    tma_prefetch_desc(&tmB);
-    if (EPI == kEpiGatedGelu) tma_prefetch_desc(&tmB2);
+    tma_prefetch_desc(&maps.a[0]);
+    tma_prefetch_desc(&maps.b[0]);
+    if (EPI == kEpiGatedGelu) tma_prefetch_desc(&maps.b[1]);
   }
   __syncthreads();
   if (warp == 1) {
@@ -125,22 +125,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const int num_kb = (p.K + kBK - 1) / kBK;
+  const int num_kb = GROUP == kGroupNone ? (p.K + kBK - 1) / kBK : p.group_num_kb;
   const int tiles_per_batch = p.tiles_m * p.tiles_n;  // tiles_m counts 256-row tiles here
   const int total_tiles = tiles_per_batch * p.batch;
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
     if (lane == 0) {
-      auto load_a = [&](int stage, int k0, int m0, int b) {
+      auto load_a = [&](int stage, const CUtensorMap* ta, int k0, int m0, int b) {
         const uint32_t bar = mapa_shared(smem_u32(&full[stage]), 0);
         uint8_t* a_dst = sA + stage * kPairABytes;
         if (!p.a_mn) {
-          tma_load_3d_pair(a_dst, &tmA, bar, k0, m0, b);  // box {64 k, 128 m, 1}
+          tma_load_3d_pair(a_dst, ta, bar, k0, m0, b);  // box {64 k, 128 m, 1}
         } else {
 #pragma unroll
           for (int j = 0; j < kBM / 64; ++j)  // box {64 m, 64 k, 1}
-            tma_load_3d_pair(a_dst + j * 8192, &tmA, bar, m0 + 64 * j, k0, b);
+            tma_load_3d_pair(a_dst + j * 8192, ta, bar, m0 + 64 * j, k0, b);
         }
       };
       auto load_b = [&](int stage, const CUtensorMap* tb, int k0, int n0, int b) {
@@ -160,7 +160,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
         const int n_tile = nt * kTileN;
         return (EPI == kEpiGatedGelu) ? n_tile : n_tile + static_cast<int>(cta) * (BN / 2);
       };
-      const CUtensorMap* tb = (EPI == kEpiGatedGelu && cta == 1) ? &tmB2 : &tmB;
+      const CUtensorMap* ta = &maps.a[0];
+      const CUtensorMap* tb = (EPI == kEpiGatedGelu && cta == 1) ? &maps.b[1] : &maps.b[0];
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -168,7 +169,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
       // stages are requested before the wait for the preceding kernel, the A halves after it.
       GemmWork work(p, pair, num_pairs, total_tiles, num_kb);
       int preloaded = 0;
-      if (MODE == kTpNone && p.b_constant && p.split_k <= 1 && pair < total_tiles) {
+      if (MODE == kTpNone && GROUP == kGroupNone && p.b_constant && p.split_k <= 1 && pair < total_tiles) {
         int b, mt, nt;
         gemm_tile_coords(p, pair, tiles_per_batch, b, mt, nt);
         preloaded = min(kStages, num_kb);
@@ -178,7 +179,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
         }
         chain_wait();
         for (int kb = 0; kb < preloaded; ++kb)
-          load_a(kb, kb * kBK, mt * (2 * kBM) + static_cast<int>(cta) * kBM, b);
+          load_a(kb, ta, kb * kBK, mt * (2 * kBM) + static_cast<int>(cta) * kBM, b);
         if (preloaded == kStages) phase = 1;
         else stage = preloaded;
       } else {
@@ -188,6 +189,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
         int b, mt, nt;
         gemm_tile_coords(p, tile, tiles_per_batch, b, mt, nt);
         const int m0 = mt * (2 * kBM) + static_cast<int>(cta) * kBM;
+        if (GROUP == kGroupColumns) {
+          const int g = gemm_group_of(p, nt);
+          tb = &maps.b[g];
+          nt -= p.group_at[g];
+        }
         const int n0 = b_col(nt);
         if (MODE == kTpAllGather && m0 < p.M) {
           // the rows of this CTA's A tile: wait for the row groups of other ranks among them
@@ -233,8 +239,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
             break;
           }
           if (cta == 0) mbar_expect_tx(&full[stage], 2 * kPairStageBytes);
-          const int k0 = kb * kBK;
-          load_a(stage, k0, m0, b);
+          int k0 = kb * kBK;
+          if (GROUP == kGroupSum) {
+            const int g = gemm_group_of(p, kb);
+            ta = &maps.a[g];
+            tb = &maps.b[g];
+            k0 -= p.group_at[g] * kBK;
+          }
+          load_a(stage, ta, k0, m0, b);
           load_b(stage, tb, k0, n0, b);
           if (++stage == kStages) {
             stage = 0;
@@ -397,8 +409,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
     int local = 0;
     bool ok = true;
     chain_wait();  // the epilogue reads residuals and writes C
-    const bool c_vec_ok = p.ldc % 8 == 0 && p.c_batch_stride % 8 == 0 &&
-                          (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
+    const bool c_vec_ok = GROUP == kGroupColumns
+                              ? p.vec_ok
+                              : p.ldc % 8 == 0 && p.c_batch_stride % 8 == 0 &&
+                                    (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
     const uint32_t drained = mapa_shared(smem_u32(&tmem_empty[0]), 0);
     GemmWork work(p, pair, num_pairs, total_tiles, num_kb);
     for (int tile, kb0, kb1; ok && work.next(tile, kb0, kb1); ++local) {
@@ -407,6 +421,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
       int b, mt, nt;
       gemm_tile_coords(p, tile, tiles_per_batch, b, mt, nt);
       const int m0 = mt * (2 * kBM) + static_cast<int>(cta) * kBM;
+      const int g = GROUP == kGroupColumns ? gemm_group_of(p, nt) : 0;
+      if (GROUP == kGroupColumns) nt -= p.group_at[g];
+      const GemmOut& out = p.out[g];
       const int n0 = nt * kTileN;
       if (!mbar_wait(&tmem_full[acc], acc_phase, abort_flag)) {
         if (lane == 0) report_status(p.status, kStatusTimeoutEpilogue, kKernelIdGemmPair, tile, 0);
@@ -427,7 +444,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
             reinterpret_cast<float*>(staging + (warp - 2) * kEpiStageBytesPerWarp));
       else
         gemm_epilogue_tile<BN, EPI, pair_epi_warps<MODE>() / 4>(
-            p, t_row, m0, n0, b, q, part, lane, c_vec_ok,
+            p, out, t_row, m0, n0, b, q, part, lane, c_vec_ok,
             kb1 - kb0 == num_kb ? p.accumulate : 2,  // a piece of a tile: atomic adds
             MODE == kTpNone
                 ? reinterpret_cast<float*>(staging + (warp - 2) * kEpiStageBytesPerWarp)
@@ -473,14 +490,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
   }
 }
 
-template <int EPI, int MODE>
-static int launch_pair(const CUtensorMap* tA, const CUtensorMap* tB, const CUtensorMap* tB2,
-                       GemmParams& p, const GemmTp& tp, int max_ctas, cudaStream_t stream) {
+template <int EPI, int MODE, int GROUP = kGroupNone>
+static int launch_pair(const GemmMaps<GROUP != kGroupNone>& maps, GemmParams& p, const GemmTp& tp, int max_ctas,
+                       cudaStream_t stream) {
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<EPI, MODE>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<EPI, MODE, GROUP>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          pair_smem<MODE>());
     if (e != cudaSuccess) return set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -493,12 +510,12 @@ static int launch_pair(const CUtensorMap* tA, const CUtensorMap* tB, const CUten
   cudaError_t e;
   if (MODE == kTpNone) {
     p.b_constant = chained_launches_constant_b() ? 1 : 0;
-    e = launch_chained(gemm_pair_kernel<EPI, MODE>, dim3(2 * pairs), dim3(pair_threads<MODE>()),
-                       pair_smem<MODE>(), stream, *tA, *tB, *tB2, p, tp);
+    e = launch_chained(gemm_pair_kernel<EPI, MODE, GROUP>, dim3(2 * pairs), dim3(pair_threads<MODE>()),
+                       pair_smem<MODE>(), stream, maps, p, tp);
   } else {
     // kernels that wait for other ranks are launched the ordinary way
-    gemm_pair_kernel<EPI, MODE><<<2 * pairs, pair_threads<MODE>(), pair_smem<MODE>(), stream>>>(
-        *tA, *tB, *tB2, p, tp);
+    gemm_pair_kernel<EPI, MODE, GROUP><<<2 * pairs, pair_threads<MODE>(), pair_smem<MODE>(), stream>>>(
+        maps, p, tp);
     e = cudaSuccess;
   }
   count_launches(1);
@@ -508,26 +525,25 @@ static int launch_pair(const CUtensorMap* tA, const CUtensorMap* tB, const CUten
 }
 
 template <int MODE>
-static int launch_pair_mode(int epilogue, const CUtensorMap* tA, const CUtensorMap* tB,
-                            const CUtensorMap* tB2, GemmParams& p, const GemmTp& tp, int max_ctas,
-                            cudaStream_t stream) {
+static int launch_pair_mode(int epilogue, const GemmMaps<false>& maps, GemmParams& p,
+                            const GemmTp& tp, int max_ctas, cudaStream_t stream) {
   switch (epilogue) {
     case kEpiPlain:
-      return launch_pair<kEpiPlain, MODE>(tA, tB, tB2, p, tp, max_ctas, stream);
+      return launch_pair<kEpiPlain, MODE>(maps, p, tp, max_ctas, stream);
     case kEpiGatedGelu:
       if (MODE == kTpReduceScatter) break;
       return launch_pair<kEpiGatedGelu, MODE == kTpReduceScatter ? kTpNone : MODE>(
-          tA, tB, tB2, p, tp, max_ctas, stream);
+          maps, p, tp, max_ctas, stream);
     case kEpiResidual:
       if (MODE == kTpAllGather) break;
       return launch_pair<kEpiResidual, MODE == kTpAllGather ? kTpNone : MODE>(
-          tA, tB, tB2, p, tp, max_ctas, stream);
+          maps, p, tp, max_ctas, stream);
     case kEpiCeStats:
       if (MODE != kTpNone) break;
-      return launch_pair<kEpiCeStats, kTpNone>(tA, tB, tB2, p, tp, max_ctas, stream);
+      return launch_pair<kEpiCeStats, kTpNone>(maps, p, tp, max_ctas, stream);
     case kEpiCeGrad:
       if (MODE != kTpNone) break;
-      return launch_pair<kEpiCeGrad, kTpNone>(tA, tB, tB2, p, tp, max_ctas, stream);
+      return launch_pair<kEpiCeGrad, kTpNone>(maps, p, tp, max_ctas, stream);
     default:
       break;
   }
@@ -538,20 +554,26 @@ static int launch_pair_mode(int epilogue, const CUtensorMap* tA, const CUtensorM
 // Called by t5x_gemm_bf16 for problems large enough to fill CTA pairs. `p.tiles_m` must count
 // 256-row tiles; the tensor maps are the same as for the one-CTA kernel with BN = 128-column
 // (K-major) or 64-column (MN-major) B boxes. `tp` is null for a plain GEMM.
-int launch_gemm_pair(int epilogue, const CUtensorMap* tA, const CUtensorMap* tB,
-                     const CUtensorMap* tB2, GemmParams& p, int max_ctas, cudaStream_t stream,
-                     const GemmTp* tp, int tp_mode) {
+int launch_gemm_pair(int epilogue, const GemmMaps<false>& maps, GemmParams& p, int max_ctas,
+                     cudaStream_t stream, const GemmTp* tp, int tp_mode) {
   static const GemmTp none = {};
   switch (tp == nullptr ? kTpNone : tp_mode) {
     case kTpNone:
-      return launch_pair_mode<kTpNone>(epilogue, tA, tB, tB2, p, none, max_ctas, stream);
+      return launch_pair_mode<kTpNone>(epilogue, maps, p, none, max_ctas, stream);
     case kTpAllGather:
-      return launch_pair_mode<kTpAllGather>(epilogue, tA, tB, tB2, p, *tp, max_ctas, stream);
+      return launch_pair_mode<kTpAllGather>(epilogue, maps, p, *tp, max_ctas, stream);
     case kTpReduceScatter:
-      return launch_pair_mode<kTpReduceScatter>(epilogue, tA, tB, tB2, p, *tp, max_ctas, stream);
+      return launch_pair_mode<kTpReduceScatter>(epilogue, maps, p, *tp, max_ctas, stream);
     default:
       return set_error("gemm_pair: unknown tensor-parallel mode %d", tp_mode);
   }
+}
+
+int launch_gemm_pair_group(int kind, const GemmMaps<true>& maps, GemmParams& p, cudaStream_t stream) {
+  static const GemmTp none = {};
+  return kind == kGroupColumns
+             ? launch_pair<kEpiPlain, kTpNone, kGroupColumns>(maps, p, none, 0, stream)
+             : launch_pair<kEpiPlain, kTpNone, kGroupSum>(maps, p, none, 0, stream);
 }
 
 }  // namespace t5x

@@ -373,15 +373,16 @@ __global__ void __launch_bounds__(kSkThreads, SkinnyCfg<BN>::kCtasPerSm)
     gp.C = p.C, gp.ldc = p.ldc, gp.c_batch_stride = 0;
     gp.R = p.R, gp.ldr = p.ldr, gp.r_batch_stride = 0;
     gp.alpha = p.alpha;
+    const GemmOut out = {p.C, p.ldc, p.N};
     const int q = warp & 3;
     const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     float* stage = staging + (warp - 2) * (kEpiStageBytesPerWarp / 4);
     const bool c_vec16 = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
     if (p.R != nullptr)
-      gemm_epilogue_tile<BN, kEpiResidual, 2>(gp, t_row, m0, n0, 0, q, (warp - 2) >> 2, lane, c_vec16,
+      gemm_epilogue_tile<BN, kEpiResidual, 2>(gp, out, t_row, m0, n0, 0, q, (warp - 2) >> 2, lane, c_vec16,
                                               0, stage);
     else
-      gemm_epilogue_tile<BN, kEpiPlain, 2>(gp, t_row, m0, n0, 0, q, (warp - 2) >> 2, lane, c_vec16, 0,
+      gemm_epilogue_tile<BN, kEpiPlain, 2>(gp, out, t_row, m0, n0, 0, q, (warp - 2) >> 2, lane, c_vec16, 0,
                                            stage);
   }
 

@@ -17,6 +17,7 @@
 // T5.1.1 gated-GELU (B = [wi_0 | wi_1], out = gelu(h0) * h1, optionally saving
 // h0/h1 for the backward pass).
 #include <algorithm>
+#include <climits>
 
 #include "gemm_common.cuh"
 #include "t5x_b200.h"
@@ -38,10 +39,11 @@ struct GemmSmem {
       kStages * kStageBytes + kBarrierBytes + kEpiStageBytes + 1024;  // +1024 align slack
 };
 
-template <int BN, int EPI>
+template <int BN, int EPI, int GROUP = kGroupNone>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-    gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                     const __grid_constant__ CUtensorMap tmB2, const GemmParams p) {
+    gemm_bf16_kernel(const __grid_constant__ GemmMaps<GROUP != kGroupNone> maps,
+                     const __grid_constant__ GemmParams p) {
+  static_assert(GROUP == kGroupNone || EPI == kEpiPlain, "groups have the plain epilogue");
   using S = GemmSmem<BN>;
   constexpr int kStages = S::kStages;
   // columns of C produced by one tile
@@ -77,9 +79,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&tmA);
-    tma_prefetch_desc(&tmB);
-    if (EPI == kEpiGatedGelu) tma_prefetch_desc(&tmB2);
+    tma_prefetch_desc(&maps.a[0]);
+    tma_prefetch_desc(&maps.b[0]);
+    if (EPI == kEpiGatedGelu) tma_prefetch_desc(&maps.b[1]);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -91,46 +93,46 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const uint32_t tmem_base = *tmem_slot;
   if (threadIdx.x == 0) T5X_GEMM_TRACE(1);
 
-  const int num_kb = (p.K + kBK - 1) / kBK;
+  const int num_kb = GROUP == kGroupNone ? (p.K + kBK - 1) / kBK : p.group_num_kb;
   const int tiles_per_batch = p.tiles_m * p.tiles_n;
   const int total_tiles = tiles_per_batch * p.batch;
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
-      auto load_a = [&](int stage, int k0, int m0, int b) {
+      auto load_a = [&](int stage, const CUtensorMap* ta, int k0, int m0, int b) {
         uint8_t* a_dst = sA + stage * S::kABytes;
         if (!p.a_mn) {
-          tma_load_3d(a_dst, &tmA, &full[stage], k0, m0, b);  // box {64, 128, 1}
+          tma_load_3d(a_dst, ta, &full[stage], k0, m0, b);  // box {64, 128, 1}
         } else {
 #pragma unroll
           for (int j = 0; j < kBM / 64; ++j)  // box {64 (m), 64 (k), 1}
-            tma_load_3d(a_dst + j * 8192, &tmA, &full[stage], m0 + 64 * j, k0, b);
+            tma_load_3d(a_dst + j * 8192, ta, &full[stage], m0 + 64 * j, k0, b);
         }
       };
-      auto load_b = [&](int stage, int k0, int n0, int b) {
+      auto load_b = [&](int stage, const CUtensorMap* tb, int k0, int n0, int b) {
         uint8_t* b_dst = sB + stage * S::kBBytes;
         if (EPI == kEpiGatedGelu) {
           constexpr int kHalf = BN / 2;  // 128 columns of each of wi_0 and wi_1
           if (!p.b_mn) {
-            tma_load_3d(b_dst, &tmB, &full[stage], k0, n0, b);
-            tma_load_3d(b_dst + kHalf * 128, &tmB2, &full[stage], k0, n0, b);
+            tma_load_3d(b_dst, tb, &full[stage], k0, n0, b);
+            tma_load_3d(b_dst + kHalf * 128, &maps.b[1], &full[stage], k0, n0, b);
           } else {
 #pragma unroll
             for (int j = 0; j < kHalf / 64; ++j) {
-              tma_load_3d(b_dst + j * 8192, &tmB, &full[stage], n0 + 64 * j, k0, b);
-              tma_load_3d(b_dst + (kHalf / 64 + j) * 8192, &tmB2, &full[stage], n0 + 64 * j, k0, b);
+              tma_load_3d(b_dst + j * 8192, tb, &full[stage], n0 + 64 * j, k0, b);
+              tma_load_3d(b_dst + (kHalf / 64 + j) * 8192, &maps.b[1], &full[stage], n0 + 64 * j, k0, b);
             }
           }
         } else {
           if (!p.b_mn) {
 #pragma unroll
             for (int j = 0; j < BN / 128; ++j)  // box {64, 128, 1}
-              tma_load_3d(b_dst + j * 16384, &tmB, &full[stage], k0, n0 + 128 * j, b);
+              tma_load_3d(b_dst + j * 16384, tb, &full[stage], k0, n0 + 128 * j, b);
           } else {
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)  // box {64 (n), 64 (k), 1}
-              tma_load_3d(b_dst + j * 8192, &tmB, &full[stage], n0 + 64 * j, k0, b);
+              tma_load_3d(b_dst + j * 8192, tb, &full[stage], n0 + 64 * j, k0, b);
           }
         }
       };
@@ -139,17 +141,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       bool ok = true;
       // B is constant (weights that no kernel in flight writes): the B halves of the first
       // stages are requested before the wait for the preceding kernel, the A halves after it.
+      const CUtensorMap *ta = &maps.a[0], *tb = &maps.b[0];
       int preloaded = 0;
-      if (p.b_constant && blockIdx.x < total_tiles) {
+      if (GROUP == kGroupNone && p.b_constant && blockIdx.x < total_tiles) {
         int b, mt, nt;
         gemm_tile_coords(p, blockIdx.x, tiles_per_batch, b, mt, nt);
         preloaded = min(kStages, num_kb);
         for (int kb = 0; kb < preloaded; ++kb) {
           mbar_expect_tx(&full[kb], S::kStageBytes);
-          load_b(kb, kb * kBK, nt * kTileN, b);
+          load_b(kb, tb, kb * kBK, nt * kTileN, b);
         }
         chain_wait();
-        for (int kb = 0; kb < preloaded; ++kb) load_a(kb, kb * kBK, mt * kBM, b);
+        for (int kb = 0; kb < preloaded; ++kb) load_a(kb, ta, kb * kBK, mt * kBM, b);
         T5X_GEMM_TRACE(2);
         if (preloaded == kStages) phase = 1;
         else stage = preloaded;
@@ -159,6 +162,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         int b, mt, nt;
         gemm_tile_coords(p, tile, tiles_per_batch, b, mt, nt);
+        if (GROUP == kGroupColumns) {
+          const int g = gemm_group_of(p, nt);
+          tb = &maps.b[g];
+          nt -= p.group_at[g];
+        }
         const int m0 = mt * kBM;
         const int n0 = nt * kTileN;
         for (int kb = preloaded; kb < num_kb; ++kb) {
@@ -169,9 +177,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             break;
           }
           mbar_expect_tx(&full[stage], S::kStageBytes);
-          const int k0 = kb * kBK;
-          load_a(stage, k0, m0, b);
-          load_b(stage, k0, n0, b);
+          int k0 = kb * kBK;
+          if (GROUP == kGroupSum) {
+            const int g = gemm_group_of(p, kb);
+            ta = &maps.a[g];
+            tb = &maps.b[g];
+            k0 -= p.group_at[g] * kBK;
+          }
+          load_a(stage, ta, k0, m0, b);
+          load_b(stage, tb, k0, n0, b);
           if (tile == blockIdx.x && kb == 0) T5X_GEMM_TRACE(2);
           if (++stage == kStages) {
             stage = 0;
@@ -240,13 +254,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     int local = 0;
     bool ok = true;
     chain_wait();  // the epilogue reads residuals and writes C
-    const bool c_vec_ok = p.ldc % 8 == 0 && p.c_batch_stride % 8 == 0 &&
-                          (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
+    const bool c_vec_ok = GROUP == kGroupColumns
+                              ? p.vec_ok
+                              : p.ldc % 8 == 0 && p.c_batch_stride % 8 == 0 &&
+                                    (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++local) {
       const int acc = local & 1;
       const uint32_t acc_phase = (local >> 1) & 1;
       int b, mt, nt;
       gemm_tile_coords(p, tile, tiles_per_batch, b, mt, nt);
+      const int g = GROUP == kGroupColumns ? gemm_group_of(p, nt) : 0;
+      if (GROUP == kGroupColumns) nt -= p.group_at[g];
+      const GemmOut& out = p.out[g];
       const int m0 = mt * kBM;
       const int n0 = nt * kTileN;
       if (!mbar_wait(&tmem_full[acc], acc_phase, abort_flag)) {
@@ -264,8 +283,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       else if (EPI == kEpiCeGrad)
         gemm_epilogue_ce_grad<BN, 2>(p, t_row, m0, n0, q, part, lane, c_vec_ok, stage_buf);
       else
-        gemm_epilogue_tile<BN, EPI, 2>(p, t_row, m0, n0, b, q, part, lane, c_vec_ok, p.accumulate,
-                                       stage_buf);
+        gemm_epilogue_tile<BN, EPI, 2>(p, out, t_row, m0, n0, b, q, part, lane, c_vec_ok,
+                                       p.accumulate, stage_buf);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[acc]);
@@ -288,15 +307,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   }
 }
 
-template <int BN, int EPI>
-static int launch_gemm(const CUtensorMap* tA, const CUtensorMap* tB, const CUtensorMap* tB2,
-                       GemmParams& p, int max_ctas, cudaStream_t stream) {
+template <int BN, int EPI, int GROUP = kGroupNone>
+static int launch_gemm(const GemmMaps<GROUP != kGroupNone>& maps, GemmParams& p, int max_ctas,
+                       cudaStream_t stream) {
   using S = GemmSmem<BN>;
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, EPI>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, EPI, GROUP>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal);
     if (e != cudaSuccess) return set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     attr_set[dev] = true;
@@ -308,17 +327,17 @@ static int launch_gemm(const CUtensorMap* tA, const CUtensorMap* tB, const CUten
   p.b_constant = chained_launches_constant_b() ? 1 : 0;
   p.trace = g_gemm_trace;
   p.trace_ctas = num_sms();
-  cudaError_t e = launch_chained(gemm_bf16_kernel<BN, EPI>, dim3(grid), dim3(kGemmThreads),
-                                 S::kTotal, stream, *tA, *tB, *tB2, p);
+  cudaError_t e = launch_chained(gemm_bf16_kernel<BN, EPI, GROUP>, dim3(grid), dim3(kGemmThreads),
+                                 S::kTotal, stream, maps, p);
   count_launches(1);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("gemm launch failed: %s", cudaGetErrorString(e));
   return 0;
 }
 
-static const CUtensorMap* operand_map(const void* ptr, int mn_major, long long rows_mn,
-                                      long long k, long long ld, long long batch_stride, int batch,
-                                      int box_rows_kmajor) {
+static bool operand_map(CUtensorMap* map, const void* ptr, int mn_major, long long rows_mn,
+                        long long k, long long ld, long long batch_stride, int batch,
+                        int box_rows_kmajor) {
   // K-major: memory is [rows_mn, k] (k contiguous, row stride ld). box {64 k, box_rows, 1}
   // MN-major: memory is [k, rows_mn] (mn contiguous, row stride ld). box {64 mn, 64 k, 1}
   uint64_t dims[3];
@@ -340,7 +359,9 @@ static const CUtensorMap* operand_map(const void* ptr, int mn_major, long long r
   strides[0] = static_cast<uint64_t>(ld) * 2;
   strides[1] = static_cast<uint64_t>(batch > 1 ? batch_stride : ld * dims[1]) * 2;
   if (strides[1] == 0) strides[1] = strides[0];
-  return get_tensor_map(ptr, 2, 3, dims, strides, box, 1);
+  const CUtensorMap* m = get_tensor_map(ptr, 2, 3, dims, strides, box, 1);
+  if (m != nullptr) *map = *m;
+  return m != nullptr;
 }
 
 }  // namespace t5x
@@ -351,9 +372,9 @@ static const CUtensorMap* operand_map(const void* ptr, int mn_major, long long r
 //           2 residual add (R bf16).
 // Returns 0 on success; a negative value with t5x_last_error() set otherwise.
 namespace t5x {
-int launch_gemm_pair(int epilogue, const CUtensorMap* tA, const CUtensorMap* tB,
-                     const CUtensorMap* tB2, GemmParams& p, int max_ctas, cudaStream_t stream,
-                     const GemmTp* tp = nullptr, int tp_mode = 0);
+int launch_gemm_pair(int epilogue, const GemmMaps<false>& maps, GemmParams& p, int max_ctas,
+                     cudaStream_t stream, const GemmTp* tp = nullptr, int tp_mode = 0);
+int launch_gemm_pair_group(int kind, const GemmMaps<true>& maps, GemmParams& p, cudaStream_t stream);
 
 // 0 = never use CTA pairs, 1 = when the shape suits them (default), 2 = always.
 // Read once from T5X_GEMM_PAIR; t5x_gemm_set_pair_mode overrides it.
@@ -386,6 +407,58 @@ struct GemmCe {
   const float* row_scale;
   float z, conf, low;
 };
+// How many pieces along K the tiles of the last wave of CTA pairs are cut into (1: not cut).
+// A weight gradient (fp32 output, long K) often leaves that wave mostly empty. What a cut gives and
+// costs, fitted to 4400 times (21 outputs from 256 x 256 to 768 x 32128, K from 512 to 65536, 2 to 64
+// pieces), in us: a wave takes 0.0054 K; the adds 0.19 a MB; the fill of C and its launch 7.4 + 0.11 a
+// MB. A product that adds to C needs no fill, and saves some 4 because whole tiles read C back first.
+// (us, whole tiles / cut: 768 x 768 x 12216 75 / 31, 768 x 3072 x 12216 80 / 56, 1472 x 3584 x 16384
+// 189 / 130, 2048 x 5120 x 32768 705 / 519; left whole: 1024 x 2816 x 2048 25.6 / 31.7 in three,
+// 2048 x 2048 x 12216 83 / 91 in eight. The rule lost nowhere among them.)
+// Only for callers that ask for it: more than two pieces meet in no fixed order, and the logits
+// of a forward product have to be the same on every call. `wanted`: 0 this choice, n that many.
+static int wgrad_pieces(long long tiles, long long K, int kb, int accumulate, size_t c_bytes,
+                        int wanted) {
+  const int pairs = num_sms() / 2;
+  const int tail = static_cast<int>(tiles % pairs);
+  if (wanted > 1) return tail > 0 ? std::min(wanted, kb) : 1;
+  const double wave = 0.0054 * K;
+  const double fill = accumulate ? -4.0 : 7.4 + 0.11e-6 * static_cast<double>(c_bytes);
+  const double tile_add = 0.19e-6 * sizeof(float) * (2 * kBM) * 256;
+  double best = 0.04 * (5.0 + wave * static_cast<double>((tiles + pairs - 1) / pairs));
+  int splits = 1;
+  for (int s = 2; tail > 0 && s <= 64 && kb / s >= 8; ++s) {
+    const double last = static_cast<double>((1ll * tail * s + pairs - 1) / pairs) / s;  // waves
+    const double saved = (1.0 - last) * wave - fill - tile_add * tail * s;
+    if (saved > best) {
+      best = saved;
+      splits = s;
+    }
+  }
+  return splits;
+}
+
+static double waves_eff(long long tiles, int units) {
+  const long long waves = (tiles + units - 1) / units;
+  return static_cast<double>(tiles) / static_cast<double>(waves * units);
+}
+
+static GemmParams gemm_params(int M, int N, int K, int batch, int a_mn, int b_mn) {
+  GemmParams p = {};
+  p.M = M;
+  p.N = N;
+  p.K = K;
+  p.batch = batch;
+  p.a_mn = a_mn;
+  p.b_mn = b_mn;
+  p.alpha = 1.f;
+  p.status = device_status_buffer();
+  p.tiles_m = (M + kBM - 1) / kBM;
+  p.split_k = 1;
+  for (int i = 1; i < kMaxGroup; ++i) p.group_at[i] = INT_MAX;
+  return p;
+}
+
 static thread_local const GemmCe* g_ce_extras = nullptr;  // set by the two entry points around gemm_impl
 
 static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int M, int N,
@@ -401,17 +474,12 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
   if (lda % 8 || ldb % 8) return set_error("gemm: lda/ldb must be multiples of 8 elements");
   if ((a_batch_stride % 8) || (b_batch_stride % 8))
     return set_error("gemm: batch strides must be multiples of 8 elements");
-  GemmParams p;
-  p.M = M;
-  p.N = N;
-  p.K = K;
-  p.batch = batch;
-  p.a_mn = a_mn_major;
-  p.b_mn = b_mn_major;
+  GemmParams p = gemm_params(M, N, K, batch, a_mn_major, b_mn_major);
   p.out_fp32 = out_fp32;
   p.accumulate = accumulate;
   p.C = C;
   p.ldc = ldc;
+  p.out[0] = {C, ldc, N};
   p.c_batch_stride = c_batch_stride;
   p.R = static_cast<const __nv_bfloat16*>(R);
   p.ldr = ldr;
@@ -420,31 +488,14 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
   p.H1 = static_cast<__nv_bfloat16*>(H1);
   p.ldh = ldh;
   p.alpha = alpha;
-  p.status = device_status_buffer();
-  p.tiles_m = (M + kBM - 1) / kBM;
-  p.mt_rot = 0;
-  p.split_k = 1;
-  p.b_constant = 0;
-  p.trace = nullptr;
-  p.trace_ctas = 0;
-  p.ce_targets = nullptr;
-  p.ce_part = nullptr;
-  p.ce_arg = nullptr;
-  p.ce_target_logit = nullptr;
-  p.ce_lse = p.ce_row_scale = nullptr;
-  p.ce_vocab_start = 0;
-  p.ce_tiles = 0;
-  p.ce_z = p.ce_conf = p.ce_low = 0.f;
 
-  const CUtensorMap* tA = operand_map(A, a_mn_major, M, K, lda, a_batch_stride, batch, 128);
-  const CUtensorMap* tB = operand_map(B, b_mn_major, N, K, ldb, b_batch_stride, batch, 128);
-  if (!tA || !tB) return -1;
+  GemmMaps<false> maps;
+  if (!operand_map(&maps.a[0], A, a_mn_major, M, K, lda, a_batch_stride, batch, 128) ||
+      !operand_map(&maps.b[0], B, b_mn_major, N, K, ldb, b_batch_stride, batch, 128))
+    return -1;
+  maps.b[1] = maps.b[0];
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int sms = num_sms();
-  auto waves_eff = [&](long long tiles, int units) {
-    long long waves = (tiles + units - 1) / units;
-    return static_cast<double>(tiles) / static_cast<double>(waves * units);
-  };
   // CTA pairs (256 x 256 tiles, a third less shared-memory traffic per FLOP) when the problem
   // has at least one full pair tile and pairs fill the machine about as well as single CTAs.
   const int pair_tiles_m = (M + 2 * kBM - 1) / (2 * kBM);
@@ -456,17 +507,15 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
     if (batch != 1 || out_fp32 || accumulate)
       return set_error("tensor-parallel gemm: batch 1, bf16 output, no accumulate");
     if (epilogue == kEpiResidual && R == nullptr) return set_error("residual epilogue needs R");
-    const CUtensorMap* tB2 = tB;
-    if (epilogue == kEpiGatedGelu) {
-      tB2 = operand_map(B2, b_mn_major, N, K, ldb, b_batch_stride, batch, 128);
-      if (!tB2) return -1;
-    }
+    if (epilogue == kEpiGatedGelu &&
+        !operand_map(&maps.b[1], B2, b_mn_major, N, K, ldb, b_batch_stride, batch, 128))
+      return -1;
     p.tiles_m = pair_tiles_m;
     p.tiles_n = epilogue == kEpiGatedGelu ? (N + 127) / 128 : (N + 255) / 256;
     const int first = tp_mode == kTpAllGather ? tp->rank : (tp->rank + 1) % tp->world;
     p.mt_rot = static_cast<int>((static_cast<long long>(first) * tp->rows_per_rank) / (2 * kBM));
     if (p.mt_rot >= p.tiles_m) p.mt_rot = 0;
-    return launch_gemm_pair(epilogue, tA, tB, tB2, p, max_ctas, st, tp, tp_mode);
+    return launch_gemm_pair(epilogue, maps, p, max_ctas, st, tp, tp_mode);
   }
 
   if (epilogue == kEpiCeStats || epilogue == kEpiCeGrad) {
@@ -486,64 +535,39 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
     p.tiles_n = (N + 255) / 256;
     if (pair_mode != 0 && M >= 2 * kBM) {
       p.tiles_m = pair_tiles_m;
-      return launch_gemm_pair(epilogue, tA, tB, tB, p, max_ctas, st);
+      return launch_gemm_pair(epilogue, maps, p, max_ctas, st);
     }
-    return epilogue == kEpiCeStats ? launch_gemm<256, kEpiCeStats>(tA, tB, tB, p, max_ctas, st)
-                                   : launch_gemm<256, kEpiCeGrad>(tA, tB, tB, p, max_ctas, st);
+    return epilogue == kEpiCeStats ? launch_gemm<256, kEpiCeStats>(maps, p, max_ctas, st)
+                                   : launch_gemm<256, kEpiCeGrad>(maps, p, max_ctas, st);
   }
   if (epilogue == kEpiGatedGelu) {
     if (out_fp32 || accumulate) return set_error("gated-GELU epilogue writes bf16 without accumulate");
-    const CUtensorMap* tB2 = operand_map(B2, b_mn_major, N, K, ldb, b_batch_stride, batch, 128);
-    if (!tB2) return -1;
+    if (!operand_map(&maps.b[1], B2, b_mn_major, N, K, ldb, b_batch_stride, batch, 128)) return -1;
     p.tiles_n = (N + 127) / 128;
     const double e1 = waves_eff(1ll * p.tiles_m * p.tiles_n * batch, sms);
     const double e2 = waves_eff(1ll * pair_tiles_m * p.tiles_n * batch, sms / 2);
     if (pair_mode == 2 || (pair_mode == 1 && M >= 2 * kBM && e2 * 1.2 >= e1)) {
       p.tiles_m = pair_tiles_m;
-      return launch_gemm_pair(kEpiGatedGelu, tA, tB, tB2, p, max_ctas, st);
+      return launch_gemm_pair(kEpiGatedGelu, maps, p, max_ctas, st);
     }
-    return launch_gemm<256, kEpiGatedGelu>(tA, tB, tB2, p, max_ctas, st);
+    return launch_gemm<256, kEpiGatedGelu>(maps, p, max_ctas, st);
   }
-  // A weight gradient (fp32 output, long K) whose tiles leave the last wave of pairs mostly empty:
-  // the tiles of that wave are cut along K. What a cut gives and costs, fitted to 4400 times (21
-  // outputs from 256 x 256 to 768 x 32128, K from 512 to 65536, 2 to 64 pieces), in us: a wave
-  // takes 0.0054 K; the adds 0.19 a MB; the fill of C and its launch 7.4 + 0.11 a MB. A product
-  // that adds to C needs no fill, and saves some 4 because whole tiles read C back first. (us, whole
-  // tiles / cut: 768 x 768 x 12216 75 / 31, 768 x 3072 x 12216 80 / 56, 1472 x 3584 x 16384
-  // 189 / 130, 2048 x 5120 x 32768 705 / 519; left whole: 1024 x 2816 x 2048 25.6 / 31.7 in three,
-  // 2048 x 2048 x 12216 83 / 91 in eight. The rule lost nowhere among them.)
-  // Only for callers that ask for it: more than two pieces meet in no fixed order, and the logits
-  // of a forward product have to be the same on every call.
   if (last_wave != 1 && pair_mode != 0 && epilogue == kEpiPlain && out_fp32 && accumulate != 2 &&
       M >= 2 * kBM && N >= 256 && max_ctas <= 0 && ldc == N &&
       (batch == 1 || c_batch_stride == static_cast<long long>(M) * N)) {
-    const int tn = (N + 255) / 256, pairs = sms / 2;
-    const long long tiles = 1ll * pair_tiles_m * tn * batch;
-    const int kb = (K + kBK - 1) / kBK;
-    const int tail = static_cast<int>(tiles % pairs);
-    const double wave = 0.0054 * K;
-    const double fill = accumulate ? -4.0 : 7.4 + 0.11e-6 * sizeof(float) * M * N * batch;
-    const double tile_add = 0.19e-6 * sizeof(float) * (2 * kBM) * 256;
-    double best = 0.04 * (5.0 + wave * static_cast<double>((tiles + pairs - 1) / pairs));
-    int splits = 1;
-    for (int s = 2; tail > 0 && s <= 64 && kb / s >= 8; ++s) {
-      const double last = static_cast<double>((1ll * tail * s + pairs - 1) / pairs) / s;  // waves
-      const double saved = (1.0 - last) * wave - fill - tile_add * tail * s;
-      if (saved > best) {
-        best = saved;
-        splits = s;
-      }
-    }
-    if (last_wave > 1) splits = tail > 0 ? std::min(last_wave, kb) : 1;
+    const int tn = (N + 255) / 256;
+    const size_t c_bytes = sizeof(float) * static_cast<size_t>(M) * N * batch;
+    const int splits = wgrad_pieces(1ll * pair_tiles_m * tn * batch, K, (K + kBK - 1) / kBK, accumulate,
+                                    c_bytes, last_wave);
     if (splits > 1) {
       if (!accumulate) {
-        cudaError_t e = cudaMemsetAsync(C, 0, sizeof(float) * static_cast<size_t>(M) * N * batch, st);
+        cudaError_t e = cudaMemsetAsync(C, 0, c_bytes, st);
         if (e != cudaSuccess) return set_error("gemm: memset: %s", cudaGetErrorString(e));
       }
       p.split_k = splits;
       p.tiles_m = pair_tiles_m;
       p.tiles_n = tn;
-      return launch_gemm_pair(epilogue, tA, tB, tB, p, max_ctas, st);
+      return launch_gemm_pair(epilogue, maps, p, max_ctas, st);
     }
   }
   // Tile width: 256 unless N is small or 128-wide tiles fill the SMs markedly better.
@@ -558,18 +582,196 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
     if (pair_mode == 2 || (pair_mode == 1 && M >= 2 * kBM && N >= 256 && e2 * 1.2 >= e1)) {
       p.tiles_m = pair_tiles_m;
       p.tiles_n = (N + 255) / 256;
-      return launch_gemm_pair(epilogue, tA, tB, tB, p, max_ctas, st);
+      return launch_gemm_pair(epilogue, maps, p, max_ctas, st);
     }
   }
   p.tiles_n = (N + bn - 1) / bn;
   if (epilogue == kEpiResidual) {
-    return bn == 256 ? launch_gemm<256, kEpiResidual>(tA, tB, tB, p, max_ctas, st)
-                     : launch_gemm<128, kEpiResidual>(tA, tB, tB, p, max_ctas, st);
+    return bn == 256 ? launch_gemm<256, kEpiResidual>(maps, p, max_ctas, st)
+                     : launch_gemm<128, kEpiResidual>(maps, p, max_ctas, st);
   }
-  return bn == 256 ? launch_gemm<256, kEpiPlain>(tA, tB, tB, p, max_ctas, st)
-                   : launch_gemm<128, kEpiPlain>(tA, tB, tB, p, max_ctas, st);
+  return bn == 256 ? launch_gemm<256, kEpiPlain>(maps, p, max_ctas, st)
+                   : launch_gemm<128, kEpiPlain>(maps, p, max_ctas, st);
+}
+// Several products in one launch (see GemmGroupKind). `width`: the columns of the outputs
+// (kGroupColumns) or the contracted widths of the products (kGroupSum, N columns). The choice of the
+// tile is that of one product with as many tiles; sums run in the same order as in separate launches
+// (kGroupColumns) or product after product (kGroupSum).
+struct GemmGroup {
+  int kind, n;
+  const void* A[kMaxGroup];
+  const void* B[kMaxGroup];
+  void* C[kMaxGroup];
+  int width[kMaxGroup];
+  long long lda[kMaxGroup], ldb[kMaxGroup], ldc[kMaxGroup];
+};
+
+// Clears up to three buffers in one launch (a fill of a few MB is bound by its launch).
+__global__ void __launch_bounds__(256) gemm_fill_kernel(float4* a, float4* b, float4* c, long long na,
+                                                        long long nb, long long nc) {
+  const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
+  const long long first = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (long long i = first; i < na; i += step) a[i] = zero;
+  for (long long i = first; i < nb; i += step) b[i] = zero;
+  for (long long i = first; i < nc; i += step) c[i] = zero;
+}
+
+static int fill_outputs(const GemmGroup& g, int M, cudaStream_t st) {
+  float4* at[kMaxGroup] = {nullptr, nullptr, nullptr};
+  long long n[kMaxGroup] = {0, 0, 0}, total = 0;
+  bool vec = true;
+  for (int i = 0; i < g.n; ++i) {
+    at[i] = static_cast<float4*>(g.C[i]);
+    const long long floats = static_cast<long long>(M) * g.width[i];
+    n[i] = floats / 4;
+    total += n[i];
+    vec = vec && floats % 4 == 0 && (reinterpret_cast<uintptr_t>(g.C[i]) & 15) == 0;
+  }
+  if (vec) {
+    const int grid = static_cast<int>(std::min<long long>((total + 1023) / 1024, 8ll * num_sms()));
+    gemm_fill_kernel<<<grid, 256, 0, st>>>(at[0], at[1], at[2], n[0], n[1], n[2]);
+    count_launches(1);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : set_error("gemm: fill: %s", cudaGetErrorString(e));
+  }
+  for (int i = 0; i < g.n; ++i) {
+    const cudaError_t e =
+        cudaMemsetAsync(g.C[i], 0, sizeof(float) * static_cast<size_t>(M) * g.width[i], st);
+    if (e != cudaSuccess) return set_error("gemm: memset: %s", cudaGetErrorString(e));
+  }
+  return 0;
+}
+
+template <int GROUP>
+static int gemm_group_tiles(const GemmGroup& g, GemmParams& p, const GemmMaps<true>& maps, int K,
+                            int last_wave, cudaStream_t st) {
+  const int sms = num_sms(), pair_tiles_m = (p.M + 2 * kBM - 1) / (2 * kBM), mode = gemm_pair_mode();
+  // tile columns of width bn; the outputs' first ones go into group_at when the launch is certain
+  auto columns = [&](int bn, bool set) {
+    if (GROUP == kGroupSum) return (p.N + bn - 1) / bn;
+    int at = 0;
+    for (int i = 0; i < g.n; ++i) {
+      if (set) p.group_at[i] = at;
+      at += (g.width[i] + bn - 1) / bn;
+    }
+    return at;
+  };
+  int narrowest = p.N;
+  bool dense = true;
+  size_t c_bytes = 0;
+  if (GROUP == kGroupColumns)
+    for (int i = 0; i < g.n; ++i) {
+      narrowest = std::min(narrowest, g.width[i]);
+      dense = dense && g.ldc[i] == g.width[i];
+      c_bytes += sizeof(float) * static_cast<size_t>(p.M) * g.width[i];
+    }
+  const int c128 = columns(128, false), c256 = columns(256, false);
+  const double e128 = waves_eff(1ll * p.tiles_m * c128, sms), e256 = waves_eff(1ll * p.tiles_m * c256, sms);
+  const int bn = (narrowest <= 128 || e128 > e256 * 1.15) ? 128 : 256;
+  const double e1 = bn == 256 ? e256 : e128 / 1.15;
+  const double e2 = waves_eff(1ll * pair_tiles_m * c256, sms / 2);
+  const bool pair_shape = p.M >= 2 * kBM && narrowest >= 256;
+  int pieces = 1;
+  if (GROUP == kGroupColumns && last_wave != 1 && mode != 0 && p.out_fp32 && pair_shape && dense)
+    pieces = wgrad_pieces(1ll * pair_tiles_m * c256, K, p.group_num_kb, p.accumulate, c_bytes, last_wave);
+  if (pieces > 1 || mode == 2 || (mode == 1 && pair_shape && e2 * 1.2 >= e1)) {
+    if (pieces > 1 && !p.accumulate)
+      if (int rc = fill_outputs(g, p.M, st)) return rc;
+    p.split_k = pieces;
+    p.tiles_m = pair_tiles_m;
+    p.tiles_n = columns(256, true);
+    return launch_gemm_pair_group(GROUP, maps, p, st);
+  }
+  p.tiles_n = columns(bn, true);
+  return bn == 256 ? launch_gemm<256, kEpiPlain, GROUP>(maps, p, 0, st)
+                   : launch_gemm<128, kEpiPlain, GROUP>(maps, p, 0, st);
+}
+
+static int gemm_group_impl(const GemmGroup& g, int M, int NK, int a_mn, int b_mn, int out_fp32,
+                           int accumulate, int last_wave, void* stream) {
+  if (g.n < 1 || g.n > kMaxGroup) return set_error("gemm group: 1 to %d products (got %d)", kMaxGroup, g.n);
+  if (M <= 0 || NK <= 0) return set_error("gemm group: sizes must be positive");
+  const bool sum = g.kind == kGroupSum;
+  GemmParams p = gemm_params(M, sum ? NK : g.width[0], sum ? 0 : NK, 1, a_mn, b_mn);
+  p.out_fp32 = out_fp32;
+  p.accumulate = accumulate;
+  p.C = g.C[0];
+  p.ldc = g.ldc[0];
+  p.vec_ok = 1;
+  GemmMaps<true> maps;
+  int kb = 0;
+  for (int i = 0; i < kMaxGroup; ++i) {
+    if (i >= g.n) {  // never read
+      maps.a[i] = maps.a[0];
+      maps.b[i] = maps.b[0];
+      continue;
+    }
+    const int n = sum ? NK : g.width[i], k = sum ? g.width[i] : NK;
+    if (g.width[i] <= 0) return set_error("gemm group: widths must be positive");
+    if (g.lda[i] % 8 || g.ldb[i] % 8) return set_error("gemm group: lda/ldb must be multiples of 8 elements");
+    if (!operand_map(&maps.a[i], g.A[i], a_mn, M, k, g.lda[i], 0, 1, 128) ||
+        !operand_map(&maps.b[i], g.B[i], b_mn, n, k, g.ldb[i], 0, 1, 128))
+      return -1;
+    if (sum) p.group_at[i] = kb;
+    p.out[i] = {g.C[i], g.ldc[i], n};
+    if (g.ldc[i] % 8 || (reinterpret_cast<uintptr_t>(g.C[i]) & 15)) p.vec_ok = 0;
+    kb = (sum ? kb : 0) + (k + kBK - 1) / kBK;
+  }
+  p.group_num_kb = kb;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return sum ? gemm_group_tiles<kGroupSum>(g, p, maps, 0, 1, st)
+             : gemm_group_tiles<kGroupColumns>(g, p, maps, NK, last_wave, st);
 }
 }  // namespace t5x
+
+// C_i[M, width_i] = A[M, K] @ B_i[K, width_i], i < n <= 3, in one launch. out_fp32 = 0: bf16 C_i.
+// out_fp32 = 1: weight gradients, fp32 C_i (+)=, as t5x_gemm_wgrad_bf16.
+T5X_API int t5x_gemm_shared_bf16(const void* A, const void* const* B, void* const* C, const int* widths,
+                                 int n, int M, int K, long long lda, const long long* ldb,
+                                 const long long* ldc, int a_mn_major, int b_mn_major, int out_fp32,
+                                 int accumulate, int last_wave_pieces, void* stream) {
+  using namespace t5x;
+  if (n < 1 || n > kMaxGroup) return set_error("gemm_shared: 1 to %d products (got %d)", kMaxGroup, n);
+  if (accumulate != 0 && !(accumulate == 1 && out_fp32)) return set_error("gemm_shared: accumulate");
+  if (last_wave_pieces < 0) return set_error("gemm_shared: pieces must not be negative");
+  GemmGroup g = {};
+  g.kind = kGroupColumns;
+  g.n = n;
+  for (int i = 0; i < n; ++i) {
+    g.A[i] = A;
+    g.lda[i] = lda;
+    g.B[i] = B[i];
+    g.ldb[i] = ldb[i];
+    g.C[i] = C[i];
+    g.ldc[i] = ldc[i];
+    g.width[i] = widths[i];
+  }
+  return gemm_group_impl(g, M, K, a_mn_major, b_mn_major, out_fp32, accumulate,
+                         out_fp32 ? last_wave_pieces : 1, stream);
+}
+
+// C[M, N] (bf16) = A_0[M, width_0] @ B_0[width_0, N] + A_1 @ B_1 + ..., n <= 3 products, in one
+// launch and one fp32 accumulator.
+T5X_API int t5x_gemm_sum_bf16(const void* const* A, const void* const* B, void* C, const int* widths,
+                              int n, int M, int N, const long long* lda, const long long* ldb,
+                              long long ldc, int a_mn_major, int b_mn_major, void* stream) {
+  using namespace t5x;
+  if (n < 1 || n > kMaxGroup) return set_error("gemm_sum: 1 to %d products (got %d)", kMaxGroup, n);
+  GemmGroup g = {};
+  g.kind = kGroupSum;
+  g.n = n;
+  g.C[0] = C;
+  g.ldc[0] = ldc;
+  for (int i = 0; i < n; ++i) {
+    g.A[i] = A[i];
+    g.lda[i] = lda[i];
+    g.B[i] = B[i];
+    g.ldb[i] = ldb[i];
+    g.width[i] = widths[i];
+  }
+  return gemm_group_impl(g, M, N, a_mn_major, b_mn_major, 0, 0, 1, stream);
+}
 
 // Phase trace of the one-CTA-per-tile and of the cluster GEMM for profiling: while `buffer` (device
 // memory, 8 int64 x the number of SMs) is set, every such GEMM launched from the calling thread

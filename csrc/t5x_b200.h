@@ -82,6 +82,17 @@ int t5x_gemm_wgrad_bf16(const void* A, const void* B, void* C, int M, int N, int
                         long long b_batch_stride, long long c_batch_stride, int a_mn_major,
                         int b_mn_major, int accumulate, int last_wave_pieces, void* stream);
 
+/* Up to three products in one launch. shared: C_i[M, widths[i]] = A[M, K] @ B_i (bf16 C_i, or fp32
+ * weight gradients (+)= with out_fp32). sum: C[M, N] (bf16) = sum of A_i[M, widths[i]] @ B_i, in one
+ * fp32 accumulator. */
+int t5x_gemm_shared_bf16(const void* A, const void* const* B, void* const* C, const int* widths, int n,
+                         int M, int K, long long lda, const long long* ldb, const long long* ldc,
+                         int a_mn_major, int b_mn_major, int out_fp32, int accumulate,
+                         int last_wave_pieces, void* stream);
+int t5x_gemm_sum_bf16(const void* const* A, const void* const* B, void* C, const int* widths, int n,
+                      int M, int N, const long long* lda, const long long* ldb, long long ldc,
+                      int a_mn_major, int b_mn_major, void* stream);
+
 /* ---- tensor parallelism with the collective inside the GEMM kernel ----
  * The M rows are split evenly over `world` ranks (rows_per_rank each). Peer pointers are the
  * other ranks' buffers as mapped into this process (symmetric memory).

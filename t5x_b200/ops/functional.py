@@ -110,6 +110,17 @@ def _host_linear_bwd(dys, x, weights, needs):
   return (False, None) if done is None else (True, done[0])
 
 
+def _input_grad(dys, mats):
+  """dys[0] @ mats[0] + dys[1] @ mats[1] + ...: two or three products in one launch where the matrices
+  lie the same way, else products that add to what the ones before stored."""
+  if 2 <= len(dys) <= 3 and all((m.stride(0) == 1) == (mats[0].stride(0) == 1) for m in mats):
+    return native.gemm_sum(dys, mats)
+  dx = native.gemm(dys[0], mats[0])
+  for dy, m in zip(dys[1:], mats[1:]):
+    native.gemm(dy, m, out=dx, accumulate=True)
+  return dx
+
+
 class _LinearFn(torch.autograd.Function):
 
   @staticmethod
@@ -151,9 +162,9 @@ class _LinearFn(torch.autograd.Function):
 
 class _MultiLinearFn(torch.autograd.Function):
   """(x @ W_0, x @ W_1, ...) for projections that share their input (q/k/v, cross k/v). In
-  backward the input gradient is built by accumulating GEMMs (dx = dy_0 W_0^T, then
-  dx += dy_i W_i^T in the epilogue), not by separate GEMMs whose results autograd would add
-  with elementwise kernels over the activations."""
+  backward the input gradient dy_0 W_0^T + dy_1 W_1^T + ... is one GEMM over all products
+  (`_input_grad`), not separate ones whose results autograd would add with elementwise kernels
+  over the activations."""
 
   @staticmethod
   def forward(ctx, x, *weights):
@@ -179,8 +190,7 @@ class _MultiLinearFn(torch.autograd.Function):
       return (dx,) + (None,) * len(weights)
     k = x.shape[-1]
     x2 = x.reshape(-1, k)
-    dx = None
-    dws = []
+    dws, grads, mats = [], [], []
     for i, (w, dy) in enumerate(zip(weights, dys)):
       if dy is None:
         dws.append(None)
@@ -189,13 +199,11 @@ class _MultiLinearFn(torch.autograd.Function):
       dy2 = dy.reshape(-1, w2.shape[1])
       if not dy2.is_contiguous():
         dy2 = dy2.contiguous()
-      if ctx.needs_input_grad[0]:
-        if dx is None:
-          dx = native.gemm(dy2, w2.t())
-        else:
-          native.gemm(dy2, w2.t(), out=dx, accumulate=True)
+      grads.append(dy2)
+      mats.append(w2.t())
       dws.append(_accumulate_wgrad(w, x2.t(), dy2) if ctx.needs_input_grad[1 + i] else None)
-    return (None if dx is None else dx.view(x.shape),) + tuple(dws)
+    dx = _input_grad(grads, mats).view(x.shape) if ctx.needs_input_grad[0] and grads else None
+    return (dx,) + tuple(dws)
 
 
 def multi_linear(x: torch.Tensor, weights: Sequence[torch.Tensor],
@@ -399,9 +407,7 @@ class _GatedGeluMlpInFn(torch.autograd.Function):
     dh0, dh1 = dh[:, :dff], dh[:, dff:]
     dx = None
     if ctx.needs_input_grad[0]:
-      dx = native.gemm(dh0, w0.t())
-      native.gemm(dh1, w1.t(), out=dx, accumulate=True)
-      dx = dx.view(x.shape)
+      dx = _input_grad([dh0, dh1], [w0.t(), w1.t()]).view(x.shape)
     d0 = _accumulate_wgrad(wi_0, x2.t(), dh0) if ctx.needs_input_grad[1] else None
     d1 = _accumulate_wgrad(wi_1, x2.t(), dh1) if ctx.needs_input_grad[2] else None
     return dx, d0, d1

@@ -379,6 +379,56 @@ def gemm_wgrad(a: torch.Tensor, b: torch.Tensor, *, out: Optional[torch.Tensor] 
   return out
 
 
+register_signature("t5x_gemm_sum_bf16", [c_void_p] * 4 + [c_int] * 3 + [c_void_p] * 2 + [c_ll] +
+                   [c_int] * 2 + [c_void_p])
+register_signature("t5x_gemm_shared_bf16", [c_void_p] * 4 + [c_int] * 3 + [c_ll] + [c_void_p] * 2 +
+                   [c_int] * 5 + [c_void_p])
+
+
+def _operands(mats, name: str):
+  """(mn_major, pointers, leading dimensions) of matrices [rows, contracted] of one orientation."""
+  layouts = [_mat_layout(t, *t.shape) for t in mats]
+  if any(l[0] != layouts[0][0] for l in layouts):
+    raise NativeError(f"{name}: operands of different orientation")
+  return (layouts[0][0], (c_void_p * len(mats))(*[t.data_ptr() for t in mats]),
+          (c_ll * len(mats))(*[l[1] for l in layouts]))
+
+
+def gemm_sum(a, b) -> torch.Tensor:
+  """bf16 a[0] @ b[0] + a[1] @ b[1] + ... (two or three products) from one fp32 accumulator."""
+  assert all(t.dtype == torch.bfloat16 and t.dim() == 2 for t in (*a, *b)) and len(a) == len(b)
+  M, N = a[0].shape[0], b[0].shape[1]
+  assert all(x.shape[0] == M and y.shape == (x.shape[1], N) for x, y in zip(a, b))
+  out = torch.empty((M, N), dtype=torch.bfloat16, device=a[0].device)
+  a_mn, a_ptr, lda = _operands(a, "gemm_sum")
+  b_mn, b_ptr, ldb = _operands([t.t() for t in b], "gemm_sum")
+  widths = (c_int * len(a))(*[t.shape[1] for t in a])
+  _check(lib().t5x_gemm_sum_bf16(a_ptr, b_ptr, out.data_ptr(), widths, len(a), M, N, lda, ldb, N, a_mn,
+                                 b_mn, stream_ptr()), "gemm_sum")
+  return out
+
+
+def gemm_shared(a: torch.Tensor, b, *, out=None, accumulate: bool = False, pieces: int = 0):
+  """[a @ w for w in b] (up to three) in one launch: bf16, or, with fp32 buffers `out` [M, N_i],
+  weight gradients as by `gemm_wgrad`."""
+  assert a.dtype == torch.bfloat16 and all(w.dtype == torch.bfloat16 for w in b)
+  M, K = a.shape
+  assert all(w.shape[0] == K for w in b)
+  fp32 = out is not None
+  if out is None:
+    out = [torch.empty((M, w.shape[1]), dtype=torch.bfloat16, device=a.device) for w in b]
+  assert all(o.shape == (M, w.shape[1]) and o.stride(1) == 1 for o, w in zip(out, b))
+  assert all(o.dtype == (torch.float32 if fp32 else torch.bfloat16) for o in out)
+  a_mn, lda, _ = _mat_layout(a, M, K)
+  b_mn, b_ptr, ldb = _operands([w.t() for w in b], "gemm_shared")
+  n = len(b)
+  _check(lib().t5x_gemm_shared_bf16(
+      a.data_ptr(), b_ptr, (c_void_p * n)(*[o.data_ptr() for o in out]),
+      (c_int * n)(*[w.shape[1] for w in b]), n, M, K, lda, ldb, (c_ll * n)(*[o.stride(0) for o in out]),
+      a_mn, b_mn, int(fp32), int(accumulate), pieces, stream_ptr()), "gemm_shared")
+  return out
+
+
 # ----------------------------------------------------------------------------
 # Normalisation / activations / embedding
 # ----------------------------------------------------------------------------
