@@ -324,47 +324,59 @@ bool heads_ok(const Tensor& t) {
 
 const void* data_or_null(const optional<Tensor>& t) { return t ? t->data_ptr() : nullptr; }
 
-// Flash attention; what the caller has prepared: an fp32 bias table with int32 buckets, a uint8 key
-// mask, int32 segment codes, all contiguous (checked where they are made).
-optional<std::tuple<Tensor, Tensor>> attention(
-    const Tensor& q, const Tensor& k, const Tensor& v, const optional<Tensor>& rel_bias,
-    const optional<Tensor>& buckets, const optional<Tensor>& key_mask, const optional<Tensor>& q_seg,
-    const optional<Tensor>& kv_seg, int64_t causal, int64_t causal_off, int64_t rel_off,
-    bool short_range) {
-  if (!heads_ok(q) || !heads_ok(k) || !heads_ok(v)) return std::nullopt;
+// What the caller has prepared for flash attention: an fp32 bias table with int32 buckets, a uint8
+// key mask, int32 segment codes, all contiguous (checked where they are made).
+struct Masks {
+  optional<Tensor> rel_bias, buckets, key_mask, q_seg, kv_seg;
+  int64_t causal, causal_off, rel_off;
+  int num_buckets() const { return rel_bias ? rel_bias->size(1) : 0; }
+  int nrel() const { return rel_bias ? buckets->size(0) : 0; }
+  const void* bucket_data() const { return rel_bias ? buckets->data_ptr() : nullptr; }
+};
+
+void attention_into(const Tensor& q, const Tensor& k, const Tensor& v, const Masks& m, bool short_range,
+                    Tensor& o, Tensor& lse, void* st) {
   const int B = q.size(0), Lq = q.size(1), H = q.size(2), D = q.size(3), Lk = k.size(1);
-  Tensor o = at::empty({B, Lq, H, D}, q.options());
-  Tensor lse = at::empty({B, H, Lq}, q.options().dtype(at::kFloat));
-  const int nb = rel_bias ? rel_bias->size(1) : 0, nrel = rel_bias ? buckets->size(0) : 0;
-  const void *table = data_or_null(rel_bias), *bucket = rel_bias ? buckets->data_ptr() : nullptr;
   if (short_range)
     check(t5x_attention_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), B,
                             H, Lq, Lk, q.stride(0), q.stride(1), q.stride(2), k.stride(0),
                             k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2),
-                            o.stride(0), o.stride(1), o.stride(2), table, bucket, nb, nrel, rel_off,
-                            data_or_null(key_mask), data_or_null(q_seg), data_or_null(kv_seg), causal,
-                            causal_off, stream_of()),
+                            o.stride(0), o.stride(1), o.stride(2), data_or_null(m.rel_bias),
+                            m.bucket_data(), m.num_buckets(), m.nrel(), m.rel_off,
+                            data_or_null(m.key_mask), data_or_null(m.q_seg), data_or_null(m.kv_seg),
+                            m.causal, m.causal_off, st),
           "attention_fwd");
   else
     check(t5x_attention_fwd_stream(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
                                    lse.data_ptr(), B, H, Lq, Lk, D, q.stride(0), q.stride(1),
                                    q.stride(2), k.stride(0), k.stride(1), k.stride(2), v.stride(0),
                                    v.stride(1), v.stride(2), o.stride(0), o.stride(1), o.stride(2),
-                                   table, bucket, nb, nrel, rel_off, data_or_null(key_mask),
-                                   data_or_null(q_seg), data_or_null(kv_seg), causal, causal_off,
-                                   stream_of()),
+                                   data_or_null(m.rel_bias), m.bucket_data(), m.num_buckets(),
+                                   m.nrel(), m.rel_off, data_or_null(m.key_mask),
+                                   data_or_null(m.q_seg), data_or_null(m.kv_seg), m.causal,
+                                   m.causal_off, st),
           "attention_fwd");
+}
+
+optional<std::tuple<Tensor, Tensor>> attention(
+    const Tensor& q, const Tensor& k, const Tensor& v, const optional<Tensor>& rel_bias,
+    const optional<Tensor>& buckets, const optional<Tensor>& key_mask, const optional<Tensor>& q_seg,
+    const optional<Tensor>& kv_seg, int64_t causal, int64_t causal_off, int64_t rel_off,
+    bool short_range) {
+  if (!heads_ok(q) || !heads_ok(k) || !heads_ok(v)) return std::nullopt;
+  Tensor o = at::empty(q.sizes(), q.options());
+  Tensor lse = at::empty({q.size(0), q.size(2), q.size(1)}, q.options().dtype(at::kFloat));
+  attention_into(q, k, v, {rel_bias, buckets, key_mask, q_seg, kv_seg, causal, causal_off, rel_off},
+                 short_range, o, lse, stream_of());
   return std::make_tuple(o, lse);
 }
 
 // (dq, dk, dv); dq, dk and dv are the column blocks of one buffer when q, k and v are (`packed`).
-optional<std::tuple<Tensor, Tensor, Tensor>> attention_bwd(
-    const Tensor& d_o, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o,
-    const Tensor& lse, const optional<Tensor>& rel_bias, const optional<Tensor>& buckets,
-    const optional<Tensor>& key_mask, const optional<Tensor>& q_seg, const optional<Tensor>& kv_seg,
-    const optional<Tensor>& d_rel, int64_t causal, int64_t causal_off, int64_t rel_off, bool packed) {
-  if (!heads_ok(d_o) || !heads_ok(q) || !heads_ok(k) || !heads_ok(v) || !heads_ok(o))
-    return std::nullopt;
+std::tuple<Tensor, Tensor, Tensor> attention_gradients(const Tensor& d_o, const Tensor& q,
+                                                       const Tensor& k, const Tensor& v,
+                                                       const Tensor& o, const Tensor& lse,
+                                                       const Masks& m, const optional<Tensor>& d_rel,
+                                                       bool packed, void* st) {
   const int B = q.size(0), Lq = q.size(1), H = q.size(2), D = q.size(3), Lk = k.size(1);
   const auto f32 = q.options().dtype(at::kFloat);
   Tensor dq32 = at::zeros({B, Lq, H, D}, f32), delta = at::empty({B, H, Lq}, f32);
@@ -378,22 +390,226 @@ optional<std::tuple<Tensor, Tensor, Tensor>> attention_bwd(
     dk = at::empty({B, Lk, H, D}, q.options());
     dv = at::empty({B, Lk, H, D}, q.options());
   }
-  const int nb = rel_bias ? rel_bias->size(1) : 0, nrel = rel_bias ? buckets->size(0) : 0;
   check(t5x_attention_bwd(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), lse.data_ptr(),
             delta.data_ptr(), dq32.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Lq, Lk, D,
             q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2), v.stride(0),
             v.stride(1), v.stride(2), o.stride(0), o.stride(1), o.stride(2), d_o.stride(0),
             d_o.stride(1), d_o.stride(2), dk.stride(0), dk.stride(1), dk.stride(2),
-            data_or_null(rel_bias), rel_bias ? buckets->data_ptr() : nullptr,
-            d_rel ? d_rel->data_ptr() : nullptr, nb, nrel, rel_off, data_or_null(key_mask),
-            data_or_null(q_seg), data_or_null(kv_seg), causal, causal_off, stream_of()),
+            data_or_null(m.rel_bias), m.bucket_data(), d_rel ? d_rel->data_ptr() : nullptr,
+            m.num_buckets(), m.nrel(), m.rel_off, data_or_null(m.key_mask), data_or_null(m.q_seg),
+            data_or_null(m.kv_seg), m.causal, m.causal_off, st),
         "attention_bwd");
   if (packed)
     dq.copy_(dq32);
   else
     dq = dq32.to(at::kBFloat16);
   return std::make_tuple(dq, dk, dv);
+}
+
+optional<std::tuple<Tensor, Tensor, Tensor>> attention_bwd(
+    const Tensor& d_o, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o,
+    const Tensor& lse, const optional<Tensor>& rel_bias, const optional<Tensor>& buckets,
+    const optional<Tensor>& key_mask, const optional<Tensor>& q_seg, const optional<Tensor>& kv_seg,
+    const optional<Tensor>& d_rel, int64_t causal, int64_t causal_off, int64_t rel_off, bool packed) {
+  if (!heads_ok(d_o) || !heads_ok(q) || !heads_ok(k) || !heads_ok(v) || !heads_ok(o))
+    return std::nullopt;
+  return attention_gradients(d_o, q, k, v, o, lse,
+                             {rel_bias, buckets, key_mask, q_seg, kv_seg, causal, causal_off, rel_off},
+                             d_rel, packed, stream_of());
+}
+
+// ------------------------------------------------------------------------------------------------
+// Whole blocks: a norm, the products around it and the residual, one call per direction. A layer
+// is then two or three calls instead of a module call, an autograd node and an op each for seven
+// or eleven kernels; what a step of a small model waits for is this (see ops/blocks.py for what is
+// covered, and the times).
+// ------------------------------------------------------------------------------------------------
+bool norm_ok(const Tensor& scale, const Tensor& x) {
+  return scale.is_cuda() && scale.scalar_type() == at::kFloat && scale.is_contiguous() &&
+         scale.numel() == x.size(-1);
+}
+bool rows_fit(const Tensor& x) { return fits(x.numel() / x.size(-1)); }
+int64_t rows_of(const Tensor& x) { return x.numel() / x.size(-1); }
+
+std::tuple<Tensor, Tensor> norm_forward(const Tensor& x, const Tensor& scale, double eps, void* st) {
+  const int64_t d = x.size(-1), rows = rows_of(x);
+  Tensor y = at::empty_like(x), rstd = at::empty({rows}, x.options().dtype(at::kFloat));
+  check(t5x_rmsnorm_fwd(x.data_ptr(), scale.data_ptr(), y.data_ptr(), rstd.data_ptr(), rows, d, eps, st),
+        "rmsnorm_fwd");
+  return std::make_tuple(y, rstd);
+}
+// The norm's input gradient plus that of the residual branch.
+Tensor norm_backward(const Tensor& dh, const Tensor& x, const Tensor& scale, const Tensor& rstd,
+                     const Tensor& dres, Tensor& dscale, void* st) {
+  Tensor dx = at::empty_like(x);
+  check(t5x_rmsnorm_bwd(dh.data_ptr(), x.data_ptr(), scale.data_ptr(), rstd.data_ptr(), dres.data_ptr(),
+                        dx.data_ptr(), dscale.data_ptr(), rows_of(x), x.size(-1), st),
+        "rmsnorm_bwd");
+  return dx;
+}
+
+// Weights wq, wk, wv, wo of an attention block over x [B, Lq, d] and (cross attention) kv.
+bool attention_weights_ok(const Tensor& x, const Tensor& kv, const std::vector<Tensor>& w, int64_t head_dim) {
+  if (w.size() != 4) return false;
+  const Weight q(w[0], x.size(-1)), k(w[1], kv.size(-1)), v(w[2], kv.size(-1));
+  if (!q.ok || !k.ok || !v.ok || q.n != k.n || q.n != v.n || q.n % head_dim) return false;
+  const Weight o(w[3], q.n);
+  return o.ok && o.n == x.size(-1);
+}
+bool mlp_weights_ok(const Tensor& x, const std::vector<Tensor>& w) {
+  if (w.size() != 3 || w[0].dim() != 2 || w[1].dim() != 2) return false;
+  const Weight a(w[0], x.size(-1)), b(w[1], x.size(-1));
+  if (!a.ok || !b.ok || a.n != b.n || a.ld != b.ld) return false;
+  const Weight o(w[2], a.n);
+  return o.ok && o.n == x.size(-1);
+}
+
+bool attention_block_ok(const Tensor& x, const optional<Tensor>& kv, const Tensor& scale,
+                        const std::vector<Tensor>& w, int64_t head_dim) {
+  const Tensor& in = kv ? *kv : x;
+  return x.dim() == 3 && plain(x) && rows_fit(x) && norm_ok(scale, x) &&
+         (!kv || (kv->dim() == 3 && plain(*kv) && rows_fit(*kv) && kv->size(0) == x.size(0))) &&
+         attention_weights_ok(x, in, w, head_dim);
+}
+bool mlp_block_ok(const Tensor& x, const Tensor& scale, const std::vector<Tensor>& w) {
+  return x.dim() >= 2 && plain(x) && rows_fit(x) && norm_ok(scale, x) && mlp_weights_ok(x, w);
+}
+// Gradient buffers that the weight-gradient kernels can write whole, for the weights above.
+bool attention_grads_ok(const Tensor& x, const optional<Tensor>& kv, const std::vector<Tensor>& w,
+                        const std::vector<optional<Tensor>>& g) {
+  const Tensor& in = kv ? *kv : x;
+  const Weight q(w[0], x.size(-1)), k(w[1], in.size(-1)), v(w[2], in.size(-1)), o(w[3], q.n);
+  return grad_ok(g[0], q, rows_of(x)) && grad_ok(g[1], k, rows_of(in)) && grad_ok(g[2], v, rows_of(in)) &&
+         grad_ok(g[3], o, rows_of(x));
+}
+bool mlp_grads_ok(const Tensor& x, const std::vector<Tensor>& w, const std::vector<optional<Tensor>>& g) {
+  const Weight a(w[0], x.size(-1)), b(w[1], x.size(-1)), o(w[2], a.n);
+  return grad_ok(g[0], a, rows_of(x)) && grad_ok(g[1], b, rows_of(x)) && grad_ok(g[2], o, rows_of(x));
+}
+
+// y = x + attention(rmsnorm(x)) wo, and what the backward pass needs: (y, h, rstd, q, k, v, o, lse).
+// The keys and values come from `kv` where there is one, else from h.
+std::vector<Tensor> attention_block(const Tensor& x, const optional<Tensor>& kv, const Tensor& scale,
+                                    double eps, const std::vector<Tensor>& weights, int64_t head_dim,
+                                    const optional<Tensor>& rel_bias, const optional<Tensor>& buckets,
+                                    const optional<Tensor>& key_mask, const optional<Tensor>& q_seg,
+                                    const optional<Tensor>& kv_seg, int64_t causal, int64_t causal_off,
+                                    int64_t rel_off, bool short_range) {
+  if (!attention_block_ok(x, kv, scale, weights, head_dim))
+    throw std::invalid_argument("attention_block: operands are not covered");
+  void* st = stream_of();
+  auto [h, rstd] = norm_forward(x, scale, eps, st);
+  const Tensor& in = kv ? *kv : h;
+  const int64_t B = x.size(0), Lq = x.size(1), Lk = in.size(1), d = x.size(-1);
+  const Weight wq(weights[0], d), wk(weights[1], in.size(-1)), wv(weights[2], in.size(-1)), wo(weights[3], wq.n);
+  const int64_t H = wq.n / head_dim;
+  std::vector<Tensor> out;
+  for (int64_t l : {Lq, Lk, Lk}) out.push_back(at::empty({B, l, H, head_dim}, x.options()));
+  if (kv) {
+    forward(h, B * Lq, wq, nullptr, out[0], st);
+    std::vector<Tensor> pair = {out[1], out[2]};
+    forward_group(in, B * Lk, {wk, wv}, pair, st);
+  } else {
+    forward_group(h, B * Lq, {wq, wk, wv}, out, st);
+  }
+  Tensor o = at::empty({B, Lq, H, head_dim}, x.options());
+  Tensor lse = at::empty({B, H, Lq}, x.options().dtype(at::kFloat));
+  attention_into(out[0], out[1], out[2],
+                 {rel_bias, buckets, key_mask, q_seg, kv_seg, causal, causal_off, rel_off}, short_range, o,
+                 lse, st);
+  Tensor y = at::empty_like(x);
+  forward(o, B * Lq, wo, &x, y, st);
+  return {y, h, rstd, out[0], out[1], out[2], o, lse};
+}
+
+// Gradients of attention_block: (dx, dkv or None). Weight gradients go into `grads` (cleared first
+// unless `accumulate`), the norm's are added to `dscale`, the bias table's to `d_rel`.
+std::tuple<Tensor, optional<Tensor>> attention_block_bwd(
+    const Tensor& dy, const Tensor& x, const optional<Tensor>& kv, const Tensor& scale,
+    const std::vector<Tensor>& weights, const std::vector<Tensor>& saved, const std::vector<Tensor>& grads,
+    const std::vector<bool>& accumulate, Tensor dscale, const optional<Tensor>& d_rel, bool need_dkv,
+    const optional<Tensor>& rel_bias, const optional<Tensor>& buckets, const optional<Tensor>& key_mask,
+    const optional<Tensor>& q_seg, const optional<Tensor>& kv_seg, int64_t causal, int64_t causal_off,
+    int64_t rel_off) {
+  const Tensor &h = saved[0], &rstd = saved[1], &q = saved[2], &k = saved[3], &v = saved[4], &o = saved[5],
+               &lse = saved[6];
+  const std::vector<optional<Tensor>> g(grads.begin(), grads.end());
+  if (!plain(dy) || dy.numel() != x.numel() ||
+      !attention_block_ok(x, kv, scale, weights, q.size(3)) || !attention_grads_ok(x, kv, weights, g))
+    throw std::invalid_argument("attention_block_bwd: operands are not covered");
+  void* st = stream_of();
+  const Tensor& in = kv ? *kv : h;
+  const int64_t m = rows_of(x), mk = rows_of(in);
+  const Weight wq(weights[0], x.size(-1)), wk(weights[1], in.size(-1)), wv(weights[2], in.size(-1)),
+      wo(weights[3], wq.n);
+  Tensor d_o = at::empty_like(o);
+  input_grad(dy.data_ptr(), wo.n, m, wo, d_o, false, st);
+  Tensor gwo = grads[3];
+  weight_grad(o, dy.data_ptr(), wo.n, m, wo, gwo, accumulate[3], st);
+  auto [dq, dk, dv] = attention_gradients(
+      d_o, q, k, v, o, lse, {rel_bias, buckets, key_mask, q_seg, kv_seg, causal, causal_off, rel_off}, d_rel,
+      false, st);
+  optional<Tensor> dh = at::empty_like(x), dkv;
+  if (kv) {
+    if (need_dkv) dkv = at::empty_like(in);
+    backward_products(in, mk, {dk.data_ptr(), dv.data_ptr()}, {wk.n, wv.n}, {wk, wv}, dkv,
+                      {grads[1], grads[2]}, {accumulate[1], accumulate[2]}, st);
+    backward_products(h, m, {dq.data_ptr()}, {wq.n}, {wq}, dh, {grads[0]}, {accumulate[0]}, st);
+  } else {
+    backward_products(h, m, {dq.data_ptr(), dk.data_ptr(), dv.data_ptr()}, {wq.n, wk.n, wv.n},
+                      {wq, wk, wv}, dh, {grads[0], grads[1], grads[2]},
+                      {accumulate[0], accumulate[1], accumulate[2]}, st);
+  }
+  return std::make_tuple(norm_backward(*dh, x, scale, rstd, dy, dscale, st), dkv);
+}
+
+// y = x + (gelu(h w0) * (h w1)) wo with h = rmsnorm(x): (y, h, rstd, g, pre-activations side by side).
+std::vector<Tensor> mlp_block(const Tensor& x, const Tensor& scale, double eps,
+                              const std::vector<Tensor>& weights, bool keep) {
+  if (!mlp_block_ok(x, scale, weights)) throw std::invalid_argument("mlp_block: operands are not covered");
+  void* st = stream_of();
+  auto [h, rstd] = norm_forward(x, scale, eps, st);
+  const int64_t m = rows_of(x), d = x.size(-1);
+  const Weight a(weights[0], d), b(weights[1], d), wo(weights[2], a.n);
+  Tensor g = at::empty({m, a.n}, x.options()), pre;
+  char* h0 = nullptr;
+  if (keep) {
+    pre = at::empty({m, 2 * a.n}, x.options());
+    h0 = static_cast<char*>(pre.data_ptr());
+  }
+  check(t5x_gemm_bf16(h.data_ptr(), a.t.data_ptr(), b.t.data_ptr(), g.data_ptr(), m, a.n, d, 1, d, a.ld, a.n, 0,
+                      0, 0, 0, 1, 0, 0, 1, nullptr, 0, 0, h0, keep ? h0 + a.n * 2 : nullptr, 2 * a.n, 1.f, 0,
+                      st),
+        "gemm");
+  Tensor y = at::empty_like(x);
+  forward(g, m, wo, &x, y, st);
+  if (!keep) return {y};
+  return {y, h, rstd, g, pre};
+}
+
+// Input gradient of mlp_block; the saved pre-activations are overwritten with their gradients.
+Tensor mlp_block_bwd(const Tensor& dy, const Tensor& x, const Tensor& scale,
+                     const std::vector<Tensor>& weights, const std::vector<Tensor>& saved,
+                     const std::vector<Tensor>& grads, const std::vector<bool>& accumulate, Tensor dscale) {
+  const Tensor &h = saved[0], &rstd = saved[1], &g = saved[2], &pre = saved[3];
+  const std::vector<optional<Tensor>> have(grads.begin(), grads.end());
+  if (!plain(dy) || dy.numel() != x.numel() || !mlp_block_ok(x, scale, weights) ||
+      !mlp_grads_ok(x, weights, have))
+    throw std::invalid_argument("mlp_block_bwd: operands are not covered");
+  void* st = stream_of();
+  const int64_t m = rows_of(x), d = x.size(-1);
+  const Weight a(weights[0], d), b(weights[1], d), wo(weights[2], a.n);
+  Tensor dg = at::empty_like(g);
+  optional<Tensor> dh = at::empty_like(x);  // what can run out of memory comes before `pre` is overwritten
+  input_grad(dy.data_ptr(), wo.n, m, wo, dg, false, st);
+  Tensor gwo = grads[2];
+  weight_grad(g, dy.data_ptr(), wo.n, m, wo, gwo, accumulate[2], st);
+  check(t5x_gated_gelu_bwd(dg.data_ptr(), pre.data_ptr(), m, a.n, 2 * a.n, a.n, 0, st), "gated_gelu_bwd");
+  const char* d0 = static_cast<const char*>(pre.data_ptr());
+  backward_products(h, m, {d0, d0 + a.n * 2}, {2 * a.n, 2 * a.n}, {a, b}, dh, {grads[0], grads[1]},
+                    {accumulate[0], accumulate[1]}, st);
+  return norm_backward(*dh, x, scale, rstd, dy, dscale, st);
 }
 
 }  // namespace
@@ -410,4 +626,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attention", torch::wrap_pybind_function_no_gil(attention));
   m.def("attention_bwd", torch::wrap_pybind_function_no_gil(attention_bwd));
   m.def("rmsnorm_bwd", torch::wrap_pybind_function_no_gil(rmsnorm_bwd));
+  m.def("attention_block_ok", attention_block_ok);
+  m.def("attention_grads_ok", attention_grads_ok);
+  m.def("attention_block", torch::wrap_pybind_function_no_gil(attention_block));
+  m.def("attention_block_bwd", torch::wrap_pybind_function_no_gil(attention_block_bwd));
+  m.def("mlp_block_ok", mlp_block_ok);
+  m.def("mlp_grads_ok", mlp_grads_ok);
+  m.def("mlp_block", torch::wrap_pybind_function_no_gil(mlp_block));
+  m.def("mlp_block_bwd", torch::wrap_pybind_function_no_gil(mlp_block_bwd));
 }

@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import dataclasses
 import enum
+import math
 import re
 from collections.abc import Mapping
 from typing import Any, Optional, Sequence, Tuple, Union
@@ -186,10 +187,10 @@ class Adafactor(OptimizerDef):
     """Heuristic: factor over the two largest dims if both >= min_dim_size_to_factor."""
     if not self.hyper_params.factored or len(shape) < 2:
       return None
-    sorted_dims = np.argsort(np.asarray(shape), kind="stable")
+    sorted_dims = sorted(range(len(shape)), key=shape.__getitem__)  # (stable)
     if shape[sorted_dims[-2]] < self.hyper_params.min_dim_size_to_factor:
       return None
-    return (int(sorted_dims[-2]),), (int(sorted_dims[-1]),)
+    return (sorted_dims[-2],), (sorted_dims[-1],)
 
   def _rule_for(self, path):
     if not self.hyper_params.factored:
@@ -335,7 +336,7 @@ class Adafactor(OptimizerDef):
       col_dims = d1
     else:
       return False
-    return int(np.prod([param.shape[d] for d in col_dims])) % 4 == 0
+    return math.prod(param.shape[d] for d in col_dims) % 4 == 0
 
   # PyTorch statement (any rank, any rule). Sharded dims are reduced over the model axis.
   def _apply_torch(self, param, state, grad, lr, decay, mbps, weight_decay_rate,
@@ -435,11 +436,11 @@ class Adafactor(OptimizerDef):
     nb = len(batch_dims)
     if batch_dims != tuple(range(nb)):
       return None  # batch dims must lead
-    batch = int(np.prod(param.shape[:nb])) if nb else 1
+    batch = math.prod(param.shape[:nb])
     bf = getattr(param, "bf16", None)
     ld_bf16, bbs = (0, 0)
     if factored_dims is None:
-      rows = 1 if nd - nb <= 1 else int(np.prod(param.shape[nb:-1]))
+      rows = 1 if nd - nb <= 1 else math.prod(param.shape[nb:-1])
       cols = int(param.shape[-1]) if nd > nb else 1
       if bf is not None:
         if not bf.is_contiguous():
@@ -456,8 +457,8 @@ class Adafactor(OptimizerDef):
       row_dims, col_dims, row_is_normalized = d0, d1, False   # v_row indexed by cols (= d1)
     else:
       return None
-    R = int(np.prod([param.shape[d] for d in row_dims]))
-    C = int(np.prod([param.shape[d] for d in col_dims]))
+    R = math.prod(param.shape[d] for d in row_dims)
+    C = math.prod(param.shape[d] for d in col_dims)
     # state vectors: the one indexed by matrix rows has the column dims removed.
     v_rvec = state["v_row"] if row_is_normalized else state["v_col"]
     v_cvec = state["v_col"] if row_is_normalized else state["v_row"]
@@ -509,7 +510,7 @@ class Adafactor(OptimizerDef):
                   flags=self._native_flags(mbps, weight_decay_rate))
     bf = getattr(param, "bf16", None)
     m = state["m"] if hp.beta1 is not None else None
-    n_global = int(np.prod(gshape[nb:])) if nd > nb else 1
+    n_global = math.prod(gshape[nb:])
 
     if v_cvec is None:
       scratch = _scratch(param.device, 4 * batch)
@@ -522,8 +523,8 @@ class Adafactor(OptimizerDef):
                                          **common)
       return True
 
-    gR = int(np.prod([gshape[d] for d in row_dims]))
-    gC = int(np.prod([gshape[d] for d in col_dims]))
+    gR = math.prod(gshape[d] for d in row_dims)
+    gC = math.prod(gshape[d] for d in col_dims)
     scratch = _scratch(param.device, native.adafactor_scratch_floats(batch, R, C))
     if zinfo is not None:
       from t5x_b200.ops import comm

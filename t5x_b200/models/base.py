@@ -50,6 +50,25 @@ def module_param_axes(module: torch.nn.Module) -> dict:
 
 
 def _owns(module: torch.nn.Module, params) -> bool:
+  """Whether every leaf of `params` is the module's own parameter of that name. Follows the tree
+  down the modules (a pass over one sentence called this for 0.6 ms of its 3.8 through the flattened
+  names of all parameters); names that are not a child or a parameter of the module at their place
+  are looked up the general way."""
+  if type(params) is dict:
+    for k, v in params.items():
+      child = module._modules.get(k)
+      if type(v) is dict and child is not None:
+        if not _owns(child, v):
+          return False
+      elif type(v) is dict or k not in module._parameters:
+        return _owns_by_name(module, params)
+      elif module._parameters[k] is not v:
+        return False
+    return True
+  return _owns_by_name(module, params)
+
+
+def _owns_by_name(module: torch.nn.Module, params) -> bool:
   flat = tree_utils.flatten_dict(params)
   own = dict(module.named_parameters())
   for k, v in flat.items():
@@ -240,11 +259,13 @@ class EncoderDecoderModel(BaseTransformerModel):
                                                           "logits_weight_and_scale"):
       return None
     self._seed_dropout(dropout_rng)
+    if params is not None and _owns(self.module, params):
+      params = None  # the module's own: it runs as it is
     hidden = call_module(self.module, params, None, batch["encoder_input_tokens"],
                          batch["decoder_input_tokens"], batch["decoder_target_tokens"],
                          enable_dropout=dropout_rng is not None, decode=False, return_hidden=True,
                          **self._module_kwargs(batch))
-    if params is not None and not _owns(self.module, params):
+    if params is not None:
       c = self.module.config
       if c.logits_via_embedding:
         weight, scale = params["token_embedder"]["embedding"], 1.0 / np.sqrt(c.emb_dim)

@@ -19,6 +19,7 @@ import torch
 from torch import nn
 
 from t5x_b200.models.t5 import layers
+from t5x_b200.ops import blocks
 from t5x_b200.ops import functional as F
 from t5x_b200.ops import reference as ref
 from t5x_b200.parallel import state as pstate
@@ -58,6 +59,24 @@ def _segment_codes(segment_ids):
   return segment_ids
 
 
+def _attention_block(x, kv, norm, attn, **kw):
+  """The attention half of a layer in one call, or None where that is not covered."""
+  return blocks.attention(x, kv, norm, attn, layers.LayerNorm, layers.MultiHeadDotProductAttention,
+                          layers.DenseGeneral, **kw)
+
+
+def _mlp_half(x, norm, mlp, dropout_rate: float):
+  """x + mlp(norm(x)), in one call where that is covered."""
+  if dropout_rate > 0:
+    x, h = norm(x, with_residual=True)
+    return x + _dropout(mlp(h, enable_dropout=True), dropout_rate, True)
+  y = blocks.gated_mlp(x, norm, mlp, layers.LayerNorm, layers.MlpBlock, layers.DenseGeneral)
+  if y is not None:
+    return y
+  x, h = norm(x, with_residual=True)
+  return mlp(h, residual=x)
+
+
 class EncoderLayer(nn.Module):
   """pre-LN self-attention and pre-LN MLP, each with a residual (network.py:47-96)."""
 
@@ -76,24 +95,18 @@ class EncoderLayer(nn.Module):
   def forward(self, x, *, bias_table, key_mask, segment_ids=None, enable_dropout=False):
     c = self.config
     drop = enable_dropout and c.dropout_rate > 0
-    x, h = self.pre_attention_layer_norm(x, with_residual=True)
-    if drop:
-      a = self.attention(h, h, bias_table=bias_table, bidirectional=True,
-                         num_buckets=c.relpos_num_buckets, max_distance=c.relpos_max_distance,
-                         key_mask=key_mask, q_segment_ids=segment_ids, kv_segment_ids=segment_ids,
-                         enable_dropout=True)
-      x = x + _dropout(a, c.dropout_rate, True)
-    else:
-      x = self.attention(h, h, bias_table=bias_table, bidirectional=True,
-                         num_buckets=c.relpos_num_buckets, max_distance=c.relpos_max_distance,
-                         key_mask=key_mask, q_segment_ids=segment_ids, kv_segment_ids=segment_ids,
-                         residual=x)
-    x, h = self.pre_mlp_layer_norm(x, with_residual=True)
-    if drop:
-      x = x + _dropout(self.mlp(h, enable_dropout=True), c.dropout_rate, True)
-    else:
-      x = self.mlp(h, residual=x)
-    return x
+    attn_kwargs = dict(bias_table=bias_table, bidirectional=True, num_buckets=c.relpos_num_buckets,
+                       max_distance=c.relpos_max_distance, key_mask=key_mask, q_segment_ids=segment_ids,
+                       kv_segment_ids=segment_ids)
+    y = None if drop else _attention_block(x, None, self.pre_attention_layer_norm, self.attention,
+                                           **attn_kwargs)
+    if y is None:
+      x, h = self.pre_attention_layer_norm(x, with_residual=True)
+      if drop:
+        y = x + _dropout(self.attention(h, h, enable_dropout=True, **attn_kwargs), c.dropout_rate, True)
+      else:
+        y = self.attention(h, h, residual=x, **attn_kwargs)
+    return _mlp_half(y, self.pre_mlp_layer_norm, self.mlp, c.dropout_rate if drop else 0.0)
 
   def forward_sp(self, x_sp, batch, length, *, bias_table, key_mask, segment_ids=None,
                  enable_dropout=False):
@@ -150,22 +163,28 @@ class DecoderLayer(nn.Module):
     c = self.config
     drop = enable_dropout and c.dropout_rate > 0
     rate = c.dropout_rate
-    x, h = self.pre_self_attention_layer_norm(x, with_residual=True)
     self_kwargs = dict(bias_table=bias_table, bidirectional=False,
                        num_buckets=c.relpos_num_buckets, max_distance=c.relpos_max_distance)
-    if decode:
-      a = self.self_attention(h, h, cache=cache["self_attention"], decode=True, **self_kwargs)
-      x = x + a
-    elif drop:
-      a = self.self_attention(h, h, key_mask=decoder_key_mask, causal=True,
-                              q_segment_ids=decoder_segment_ids,
-                              kv_segment_ids=decoder_segment_ids, enable_dropout=True,
-                              **self_kwargs)
-      x = x + _dropout(a, rate, True)
-    else:
-      x = self.self_attention(h, h, key_mask=decoder_key_mask, causal=True,
-                              q_segment_ids=decoder_segment_ids,
-                              kv_segment_ids=decoder_segment_ids, residual=x, **self_kwargs)
+    if not decode:
+      self_kwargs.update(key_mask=decoder_key_mask, causal=True, q_segment_ids=decoder_segment_ids,
+                         kv_segment_ids=decoder_segment_ids)
+    y = None if decode or drop else _attention_block(
+        x, None, self.pre_self_attention_layer_norm, self.self_attention, **self_kwargs)
+    if y is None:
+      x, h = self.pre_self_attention_layer_norm(x, with_residual=True)
+      if decode:
+        y = x + self.self_attention(h, h, cache=cache["self_attention"], decode=True, **self_kwargs)
+      elif drop:
+        y = x + _dropout(self.self_attention(h, h, enable_dropout=True, **self_kwargs), rate, True)
+      else:
+        y = self.self_attention(h, h, residual=x, **self_kwargs)
+    x = y
+    cross_kwargs = dict(key_mask=encoder_key_mask, q_segment_ids=decoder_segment_ids,
+                        kv_segment_ids=encoder_segment_ids)
+    y = None if decode or drop else _attention_block(
+        x, encoded, self.pre_cross_attention_layer_norm, self.encoder_decoder_attention, **cross_kwargs)
+    if y is not None:
+      return _mlp_half(y, self.pre_mlp_layer_norm, self.mlp, 0.0)
     x, h = self.pre_cross_attention_layer_norm(x, with_residual=True)
     if decode:
       cross = cache["encoder_decoder_attention"]
@@ -177,20 +196,11 @@ class DecoderLayer(nn.Module):
           precomputed_kv=(cross["cross_key"], cross["cross_value"]), residual=x,
           beams_per_kv=beams_per_kv)
     elif drop:
-      a = self.encoder_decoder_attention(h, encoded, key_mask=encoder_key_mask,
-                                         q_segment_ids=decoder_segment_ids,
-                                         kv_segment_ids=encoder_segment_ids, enable_dropout=True)
-      x = x + _dropout(a, rate, True)
+      x = x + _dropout(self.encoder_decoder_attention(h, encoded, enable_dropout=True, **cross_kwargs),
+                       rate, True)
     else:
-      x = self.encoder_decoder_attention(h, encoded, key_mask=encoder_key_mask,
-                                         q_segment_ids=decoder_segment_ids,
-                                         kv_segment_ids=encoder_segment_ids, residual=x)
-    x, h = self.pre_mlp_layer_norm(x, with_residual=True)
-    if drop:
-      x = x + _dropout(self.mlp(h, enable_dropout=True), rate, True)
-    else:
-      x = self.mlp(h, residual=x)
-    return x
+      x = self.encoder_decoder_attention(h, encoded, residual=x, **cross_kwargs)
+    return _mlp_half(x, self.pre_mlp_layer_norm, self.mlp, rate if drop else 0.0)
 
   def forward_sp(self, x_sp, encoded, batch, length, *, bias_table, decoder_key_mask,
                  encoder_key_mask, decoder_segment_ids=None, encoder_segment_ids=None,

@@ -202,16 +202,27 @@ def flash_attention(q, k, v, *, bias_table: Optional[torch.Tensor] = None,
   `key_mask` and the segment ids (which it contains)."""
   B, Lq, H, D = q.shape
   Lk = k.shape[1]
+  from t5x_b200.ops import functional
+  return functional._apply(_FlashAttentionFn, q, k, v,
+                           *prepare(Lq, Lk, H, q.device, bias_table, bidirectional, num_buckets,
+                                    max_distance, key_mask, causal, q_segment_ids, kv_segment_ids,
+                                    q_offset, prefix_lm))
+
+
+def prepare(Lq, Lk, H, device, bias_table, bidirectional, num_buckets, max_distance, key_mask, causal,
+            q_segment_ids, kv_segment_ids, q_offset=0, prefix_lm=None):
+  """What the kernels take beside q, k and v: (bias table, buckets, key mask, query codes, key codes,
+  mask mode, its offset, offset of the relative positions)."""
   rel_bias = buckets = None
   if bias_table is not None:
     # an fp32 parameter goes in as it is, so that its gradient buffer is found in backward
     rel_bias = bias_table.float().contiguous()
-    if rel_bias.device != q.device:  # the kernels read it by its address
-      raise ValueError(f"bias table on {rel_bias.device}, queries on {q.device}")
+    if rel_bias.device != device:  # the kernels read it by its address
+      raise ValueError(f"bias table on {rel_bias.device}, queries on {device}")
     if rel_bias.shape[0] < H or rel_bias.shape[1] < num_buckets:
       raise ValueError(f"bias table {tuple(rel_bias.shape)}: {H} heads and {num_buckets} buckets are "
                        "indexed")
-    buckets = _rel_buckets(Lq, Lk, q_offset, bidirectional, num_buckets, max_distance, q.device)
+    buckets = _rel_buckets(Lq, Lk, q_offset, bidirectional, num_buckets, max_distance, device)
   km = _byte_mask(key_mask) if key_mask is not None else None
   qs = q_segment_ids.to(torch.int32).contiguous() if q_segment_ids is not None else None
   ks = kv_segment_ids.to(torch.int32).contiguous() if kv_segment_ids is not None else None
@@ -223,6 +234,4 @@ def flash_attention(q, k, v, *, bias_table: Optional[torch.Tensor] = None,
     valid = _byte_mask(prefix_lm.valid)
     km = valid if km is None else km & valid
     mode = 2
-  from t5x_b200.ops import functional
-  return functional._apply(_FlashAttentionFn, q, k, v, rel_bias, buckets, km, qs, ks, mode,
-                           (Lk - Lq) if mode else 0, Lq - 1)
+  return rel_bias, buckets, km, qs, ks, mode, (Lk - Lq) if mode else 0, Lq - 1

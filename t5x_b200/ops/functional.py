@@ -66,10 +66,19 @@ def _apply(fn, *args):
   """fn.apply(*args). Where nothing can record or transform the call (no gradients, no function
   transform, no forward-mode level, no tracing) the forward runs directly, without building
   an autograd node for it."""
-  if (not torch.is_grad_enabled() and torch._C._functorch.peek_interpreter_stack() is None and
-      torch.autograd.forward_ad._current_level < 0 and torch._C._get_tracing_state() is None):
+  if _records_nothing():
     return fn.forward(_NoGraph(), *args)
   return fn.apply(*args)
+
+
+def _transformed() -> bool:
+  """Whether a function transform, a forward-mode level or a trace is active."""
+  return not (torch._C._functorch.peek_interpreter_stack() is None and
+              torch.autograd.forward_ad._current_level < 0 and torch._C._get_tracing_state() is None)
+
+
+def _records_nothing() -> bool:
+  return not torch.is_grad_enabled() and not _transformed()
 
 
 def _take_grad_flags(weights):

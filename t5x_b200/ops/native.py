@@ -130,7 +130,9 @@ class _HostOps:
   """The functions of the compiled host path (csrc/host/host_ops.cpp) with this module's error
   type. They return None, before doing anything, for calls that they do not cover."""
   NAMES = ("linear", "multi_linear", "multi_linear_bwd", "gated_in", "gated_in_bwd", "rmsnorm",
-           "rmsnorm_bwd", "attention", "attention_bwd")
+           "rmsnorm_bwd", "attention", "attention_bwd", "attention_block_ok", "attention_grads_ok",
+           "attention_block", "attention_block_bwd", "mlp_block_ok", "mlp_grads_ok", "mlp_block",
+           "mlp_block_bwd")
 
   def __init__(self, module):
     for name in self.NAMES:
