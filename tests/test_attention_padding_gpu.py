@@ -1,0 +1,67 @@
+"""Attention over batches with padding: whole blocks of hidden keys (which the kernels pass over), blocks with
+one visible key, hidden blocks in the middle, and an example without any visible key (whose rows are
+uniform over all keys), against float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _mask(kind, b, lk):
+  m = torch.ones(b, lk, dtype=torch.bool, device="cuda")
+  if kind == "tail":
+    for i, n in enumerate((lk, max(1, lk // 2), 1, min(lk, 129))):
+      m[i, n:] = False
+  elif kind == "middle":
+    m[1, lk // 4:3 * lk // 4] = False
+    m[2, :lk - 1] = False
+  elif kind == "none":
+    m[1] = False
+    m[2, 1:] = False
+  return m
+
+
+@pytest.mark.parametrize("kind", ["tail", "middle", "none"])
+@pytest.mark.parametrize("lq,lk,d,bias", [(130, 512, 64, True), (64, 385, 64, False), (200, 700, 64, True),
+                                          (600, 600, 64, True), (140, 520, 128, True), (128, 256, 128, False)])
+def test_hidden_blocks(kind, lq, lk, d, bias):
+  from t5x_b200.ops import attention, native, reference
+  g = torch.Generator(device="cuda").manual_seed(lq + lk)
+  b, h = 4, 2
+  rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+  q = (rnd(b, lq, h, d) * d ** -0.5).bfloat16().requires_grad_()
+  k, v = (rnd(b, lk, h, d).bfloat16().requires_grad_() for _ in range(2))
+  do = rnd(b, lq, h, d).bfloat16()
+  table = torch.nn.Parameter(rnd(h, 32) * 0.5) if bias else None
+  mask = _mask(kind, b, lk)
+  leaves = [q, k, v] + ([table] if bias else [])
+  o = attention.flash_attention(q, k, v, bias_table=table, key_mask=mask)
+  grads = torch.autograd.grad(o, leaves, do)
+  native.check_status()
+  q2, k2, v2 = (t.detach().double().requires_grad_() for t in (q, k, v))
+  s = torch.einsum("bqhd,bkhd->bhqk", q2, k2)
+  ref_leaves = [q2, k2, v2]
+  if bias:
+    t2 = table.detach().double().requires_grad_()
+    ref_leaves.append(t2)
+    rel = torch.arange(lk, device="cuda")[None] - torch.arange(lq, device="cuda")[:, None]
+    s = s + t2[:, reference.relative_position_bucket(rel, True, 32, 128)][None]
+  # hidden keys take the value -1e10 whatever their score: a row without visible keys is uniform
+  s = torch.where(mask[:, None, None, :], s, s * 0 - 1e10)
+  want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), v2)
+  ref = torch.autograd.grad(want, ref_leaves, do.double())
+  # probabilities and their gradients are rounded to bf16 once, as is the result
+  assert float((o.double() - want).norm() / want.norm()) < 2 * 2.0 ** -8
+  seen = mask.any(1)
+  for i, (x, y) in enumerate(zip(grads, ref)):
+    if i == 3 and kind == "none":
+      continue  # (the kernel hands the bias dS of every position, also where no key is visible)
+    x, y = (x, y) if i == 3 else (x[seen], y[seen])
+    assert float((x.double() - y).norm() / y.norm()) < 3 * 2.0 ** -8
+  hidden = ~mask & seen[:, None]
+  assert not grads[1][hidden].any() and not grads[2][hidden].any()
+  # what padding holds does not reach anything
+  with torch.no_grad():
+    k3, v3 = k.clone(), v.clone()
+    k3[hidden], v3[hidden] = 3.0, -2.0
+    assert torch.equal(attention.flash_attention(q, k3, v3, bias_table=table, key_mask=mask), o)
