@@ -61,7 +61,7 @@ struct GemmParams {
   long long ldr, r_batch_stride;
   __nv_bfloat16* H0;  // gated-GELU: optional copies of the two pre-activations
   __nv_bfloat16* H1;
-  long long ldh;
+  long long ldh, h_batch_stride;
   float alpha;
   int tiles_m, tiles_n;
   int mt_rot;  // the row-tile walk starts at this tile (tensor-parallel kernels); 0 otherwise
@@ -389,7 +389,8 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, const Ge
       const int col = n0 + c * 32;
       const int n_valid = o.N - col;
       const bool hv16 = p.H0 == nullptr ||
-                        ((p.ldh % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.H0) |
+                        ((p.ldh % 8 == 0) && (p.h_batch_stride % 8 == 0) &&
+                        ((reinterpret_cast<uintptr_t>(p.H0) |
                                                reinterpret_cast<uintptr_t>(p.H1)) & 15) == 0);
       if (stage != nullptr && n_valid >= 32 && rows_valid > 0 && c_vec_ok && hv16) {
         // whole 32-column blocks: row-contiguous stores through the staging block
@@ -406,8 +407,9 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, const Ge
                               first_row * o.ldc + col,
                           o.ldc, rows_valid, lane);
         if (p.H0 != nullptr) {
-          staged_store_bf16(stage, h0, p.H0 + first_row * p.ldh + col, p.ldh, rows_valid, lane);
-          staged_store_bf16(stage, h1, p.H1 + first_row * p.ldh + col, p.ldh, rows_valid, lane);
+          const long long at = b * p.h_batch_stride + first_row * p.ldh + col;
+          staged_store_bf16(stage, h0, p.H0 + at, p.ldh, rows_valid, lane);
+          staged_store_bf16(stage, h1, p.H1 + at, p.ldh, rows_valid, lane);
         }
         continue;
       }
@@ -421,8 +423,9 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, const Ge
         }
         store_row_bf16(out + col, g, n_valid, c_vec_ok);
         if (p.H0 != nullptr) {
-          store_row_bf16(p.H0 + static_cast<long long>(row) * p.ldh + col, h0, n_valid, hv16);
-          store_row_bf16(p.H1 + static_cast<long long>(row) * p.ldh + col, h1, n_valid, hv16);
+          const long long at = b * p.h_batch_stride + static_cast<long long>(row) * p.ldh + col;
+          store_row_bf16(p.H0 + at, h0, n_valid, hv16);
+          store_row_bf16(p.H1 + at, h1, n_valid, hv16);
         }
       }
     }

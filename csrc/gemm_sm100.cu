@@ -487,6 +487,7 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
   p.H0 = static_cast<__nv_bfloat16*>(H0);
   p.H1 = static_cast<__nv_bfloat16*>(H1);
   p.ldh = ldh;
+  p.h_batch_stride = static_cast<long long>(M) * ldh;  // (one after the other)
   p.alpha = alpha;
 
   GemmMaps<false> maps;

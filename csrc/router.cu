@@ -295,21 +295,34 @@ __global__ void __launch_bounds__(kRtThreads)
   }
 }
 
-// dw[c, e] = sum_t x[t, c] * dlogits[t, e] in two deterministic stages: every CTA reduces a
-// tile of kDwTile tokens into part[tile, c, e] (a thread owns feature columns, the tile's dlogits
-// sit in shared memory), then a second kernel adds the tiles in order.
-constexpr int kDwTile = 512;
-constexpr int kDwThreads = 256;
-constexpr int kDwMaxColsPerThread = 4;  // d <= 1024 per pass over the tile
+// dw[c, e] = sum_t x[t, c] * dlogits[t, e] in two deterministic stages: a CTA reduces a tile of
+// kDwTile tokens for 256 columns into part[tile, c, e] (a thread owns two adjacent columns, the
+// tile's dlogits sit in shared memory), then a second kernel adds the tiles in a fixed order.
+// Bound by the bytes of x in flight: with tiles of 512 tokens and one 2-byte load a column,
+// 32768 tokens were 64 CTAs that waited for each row in turn (32768 and 7296 tokens x 768, 8 experts, the
+// two calls together: 532 us, 49 so).
+constexpr int kDwTile = 128;
+constexpr int kDwThreads = 128;
+constexpr int kDwCols = 2 * kDwThreads;
+constexpr int kDwAhead = 8;  // rows requested before the first is used
 
 __global__ void __launch_bounds__(kDwThreads)
     router_dw_partial_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
-                             const float* __restrict__ dlogits, const RouterDims dm,
+                             const float* __restrict__ dlogits, const RouterDims dm, int vec_ok,
                              float* __restrict__ part /* [tiles, d, E] */) {
   __shared__ __align__(16) float dl[kDwTile * 8];
-  const int tile = blockIdx.x;
+  const int tile = blockIdx.x, c = blockIdx.y * kDwCols + 2 * threadIdx.x;
   const int t0 = tile * kDwTile, nt = min(kDwTile, dm.T - t0);
-  float* out = part + static_cast<long long>(tile) * dm.d * dm.E;
+  const bool both = c + 1 < dm.d;
+  const __nv_bfloat16* col = x + static_cast<long long>(t0) * ldx + c;
+  float* out = part + (static_cast<long long>(tile) * dm.d + c) * dm.E;
+  auto load = [&](int t) {
+    const __nv_bfloat16* at = col + t * ldx;
+    if (vec_ok && both) return *reinterpret_cast<const uint32_t*>(at);
+    const __nv_bfloat16 zero = __float2bfloat16(0.f);
+    const __nv_bfloat162 v = __halves2bfloat162(c < dm.d ? at[0] : zero, both ? at[1] : zero);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  };
   for (int e0 = 0; e0 < dm.E; e0 += 8) {
     const int ne = min(8, dm.E - e0);
     __syncthreads();
@@ -318,48 +331,55 @@ __global__ void __launch_bounds__(kDwThreads)
       dl[i] = j < ne ? dlogits[static_cast<long long>(t0 + t) * dm.E + e0 + j] : 0.f;
     }
     __syncthreads();
-    for (int c0 = 0; c0 < dm.d; c0 += kDwThreads * kDwMaxColsPerThread) {
-      float acc[kDwMaxColsPerThread][8];
+    if (c >= dm.d) continue;
+    float acc[2][8] = {};
+    auto add = [&](int t, uint32_t u) {
+      const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u));
+      const float4 a = *reinterpret_cast<const float4*>(dl + t * 8);
+      const float4 b = *reinterpret_cast<const float4*>(dl + t * 8 + 4);
+      const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-      for (int q = 0; q < kDwMaxColsPerThread; ++q)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[q][j] = 0.f;
-      for (int t = 0; t < nt; ++t) {
-        const __nv_bfloat16* row = x + static_cast<long long>(t0 + t) * ldx + c0;
-        const float4 a = *reinterpret_cast<const float4*>(dl + t * 8);
-        const float4 b = *reinterpret_cast<const float4*>(dl + t * 8 + 4);
-#pragma unroll
-        for (int q = 0; q < kDwMaxColsPerThread; ++q) {
-          const int c = c0 + q * kDwThreads + threadIdx.x;
-          const float xv = c < dm.d ? __bfloat162float(row[q * kDwThreads + threadIdx.x]) : 0.f;
-          acc[q][0] = fmaf(xv, a.x, acc[q][0]);
-          acc[q][1] = fmaf(xv, a.y, acc[q][1]);
-          acc[q][2] = fmaf(xv, a.z, acc[q][2]);
-          acc[q][3] = fmaf(xv, a.w, acc[q][3]);
-          acc[q][4] = fmaf(xv, b.x, acc[q][4]);
-          acc[q][5] = fmaf(xv, b.y, acc[q][5]);
-          acc[q][6] = fmaf(xv, b.z, acc[q][6]);
-          acc[q][7] = fmaf(xv, b.w, acc[q][7]);
-        }
+      for (int j = 0; j < 8; ++j) {
+        acc[0][j] = fmaf(xv.x, w[j], acc[0][j]);
+        acc[1][j] = fmaf(xv.y, w[j], acc[1][j]);
       }
+    };
+    int t = 0;
+    for (; t + kDwAhead <= nt; t += kDwAhead) {
+      uint32_t u[kDwAhead];
 #pragma unroll
-      for (int q = 0; q < kDwMaxColsPerThread; ++q) {
-        const int c = c0 + q * kDwThreads + threadIdx.x;
-        if (c < dm.d)
-          for (int j = 0; j < ne; ++j) out[static_cast<long long>(c) * dm.E + e0 + j] = acc[q][j];
-      }
+      for (int i = 0; i < kDwAhead; ++i) u[i] = load(t + i);
+#pragma unroll
+      for (int i = 0; i < kDwAhead; ++i) add(t + i, u[i]);
+    }
+    for (; t < nt; ++t) add(t, load(t));
+    for (int j = 0; j < ne; ++j) {
+      out[e0 + j] = acc[0][j];
+      if (both) out[dm.E + e0 + j] = acc[1][j];
     }
   }
 }
 
+// A block adds 32 values over the tiles: eight warps take every eighth tile, then meet in order.
 __global__ void __launch_bounds__(256)
     router_dw_reduce_kernel(const float* __restrict__ part, int tiles, int n,
                             float* __restrict__ dw) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  __shared__ float red[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int t = 0; t < tiles; ++t) s += part[static_cast<long long>(t) * n + i];
-  dw[i] = s;
+  if (i < n) {
+#pragma unroll 4
+    for (int t = warp; t < tiles; t += 8) s += part[static_cast<long long>(t) * n + i];
+  }
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && i < n) {
+    float tot = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) tot += red[w][lane];
+    dw[i] = tot;
+  }
 }
 
 static int router_check(const RouterDims& dm, size_t smem) {
@@ -447,11 +467,12 @@ T5X_API int t5x_moe_router_bwd(const void* x, long long ldx, const void* w, int 
       static_cast<const float*>(coef), static_cast<const float*>(w), dm,
       static_cast<float*>(dlogits), static_cast<__nv_bfloat16*>(dx), lddx);
   const int tiles = (T + kDwTile - 1) / kDwTile;
-  router_dw_partial_kernel<<<tiles, kDwThreads, 0, st>>>(static_cast<const __nv_bfloat16*>(x), ldx,
-                                                        static_cast<const float*>(dlogits), dm,
-                                                        static_cast<float*>(dw_part));
-  router_dw_reduce_kernel<<<(d * E + 255) / 256, 256, 0, st>>>(
-      static_cast<const float*>(dw_part), tiles, d * E, static_cast<float*>(dw));
+  const int vec_ok = ldx % 2 == 0 && (reinterpret_cast<uintptr_t>(x) & 3) == 0;
+  router_dw_partial_kernel<<<dim3(tiles, (d + kDwCols - 1) / kDwCols), kDwThreads, 0, st>>>(
+      static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const float*>(dlogits), dm, vec_ok,
+      static_cast<float*>(dw_part));
+  router_dw_reduce_kernel<<<(d * E + 31) / 32, 256, 0, st>>>(static_cast<const float*>(dw_part), tiles,
+                                                             d * E, static_cast<float*>(dw));
   count_launches(3);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("router_bwd launch: %s", cudaGetErrorString(e));

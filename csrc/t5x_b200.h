@@ -67,7 +67,8 @@ int t5x_adafactor_factored_static(void* p, const void* g, void* v_rvec, void* v_
  * a_mn_major / b_mn_major: 0 = the contraction dim is contiguous, 1 = the M (N) dim is.
  * out_fp32: C is fp32 (else bf16); accumulate: 0 store, 1 add to C, 2 add atomically (several
  * K slices as batches into one C). epilogue: 0 plain, 1 gated GELU (C = gelu(A B) * (A B2),
- * optional copies of both products in H0 / H1), 2 add the bf16 matrix R. */
+ * optional copies of both products in H0 / H1, the batches M rows after one another), 2 add the bf16
+ * matrix R. */
 int t5x_gemm_bf16(const void* A, const void* B, const void* B2, void* C, int M, int N, int K,
                   int batch, long long lda, long long ldb, long long ldc,
                   long long a_batch_stride, long long b_batch_stride, long long c_batch_stride,

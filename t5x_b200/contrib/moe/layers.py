@@ -368,6 +368,9 @@ class Experts(nn.Module):
 
   def forward(self, x: torch.Tensor) -> torch.Tensor:
     """x [E_local, N, d] -> [E_local, N, d]."""
+    if self.activations == ("gelu", "linear"):
+      h = F.batched_gated_mlp_in(x, self.wi_0.kernel, self.wi_1.kernel, self.dtype)
+      return F.batched_linear(h, self.wo.kernel, self.dtype)
     hs = []
     for n, act in zip(self._wi_names, self.activations):
       w = getattr(self, n).kernel

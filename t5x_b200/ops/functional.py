@@ -264,6 +264,52 @@ class _BatchedLinearFn(torch.autograd.Function):
     return dx, dw
 
 
+class _BatchedGatedMlpInFn(torch.autograd.Function):
+  """gelu(x[e] @ wi_0[e]) * (x[e] @ wi_1[e]) for stacked expert kernels, activation and product in the
+  GEMM's epilogue as in `_GatedGeluMlpInFn`."""
+
+  @staticmethod
+  def forward(ctx, x, wi_0, wi_1):
+    x = x.contiguous()
+    w0, w1 = compute_weight(wi_0, torch.bfloat16), compute_weight(wi_1, torch.bfloat16)
+    h = torch.empty(*x.shape[:2], 2 * w0.shape[2], dtype=torch.bfloat16, device=x.device)
+    g = native.gemm(x, w0, b2=w1, save_h=h)
+    ctx.save_for_backward(x, wi_0, wi_1, h)
+    return g
+
+  @staticmethod
+  def backward(ctx, dg):
+    x, wi_0, wi_1, h = ctx.saved_tensors
+    w0, w1 = compute_weight(wi_0, torch.bfloat16), compute_weight(wi_1, torch.bfloat16)
+    dff = w0.shape[2]
+    # the saved pre-activations are overwritten with their gradients (one backward per forward)
+    native.gated_gelu_bwd_(dg.reshape(-1, dff).contiguous(), h.view(-1, 2 * dff))
+    dhs = (h[..., :dff], h[..., dff:])
+    dx = None
+    if ctx.needs_input_grad[0]:
+      dx = native.gemm(dhs[0], w0.transpose(1, 2))
+      native.gemm(dhs[1], w1.transpose(1, 2), out=dx, accumulate=True)
+    dws = []
+    for need, weight, dh in zip(ctx.needs_input_grad[1:], (wi_0, wi_1), dhs):
+      mg = getattr(weight, "main_grad", None) if need else None
+      if mg is not None:
+        native.gemm_wgrad(x.transpose(1, 2), dh, out=mg,
+                          accumulate=bool(getattr(weight, "grad_ready", False)))
+        weight.grad_ready = True
+      dws.append(native.gemm_wgrad(x.transpose(1, 2), dh).to(weight.dtype) if need and mg is None
+                 else None)
+    return (dx, *dws)
+
+
+def batched_gated_mlp_in(x: torch.Tensor, wi_0: torch.Tensor, wi_1: torch.Tensor,
+                         dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+  """x [E, N, in], stacked kernels [E, in, out] -> gelu(x @ wi_0) * (x @ wi_1) [E, N, out]."""
+  if (_native_ok(x) and wi_0.shape == wi_1.shape and wi_0.stride() == wi_1.stride() and
+      wi_0.shape[2] % 8 == 0):
+    return _apply(_BatchedGatedMlpInFn, x, wi_0, wi_1)
+  return ref.gelu_tanh(batched_linear(x, wi_0, dtype)) * batched_linear(x, wi_1, dtype)
+
+
 def batched_linear(x: torch.Tensor, weight: torch.Tensor,
                    dtype: Optional[torch.dtype] = None) -> torch.Tensor:
   """x [E, N, in] @ weight [E, in, out] -> [E, N, out]."""

@@ -299,7 +299,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, out: Optional[torch.Tensor] = None
   `a` and `b` may be arbitrary 2-D/3-D views whose last two dims are row-major or
   transposed-row-major (no copy is made: the tensor-core descriptors read either).
   With `b2` the gated-GELU epilogue runs: out = gelu(a @ b) * (a @ b2); `save_h`
-  ([M, 2N], bf16) then receives the two pre-activations side by side.
+  ([M, 2N], or contiguous [batch, M, 2N], bf16) then receives the two pre-activations side by side.
   `residual` adds a bf16 tensor of the output's shape in the epilogue.
   """
   assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
@@ -336,6 +336,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, out: Optional[torch.Tensor] = None
     b2_ptr = b2.data_ptr()
     if save_h is not None:
       assert save_h.dtype == torch.bfloat16 and save_h.shape[-1] == 2 * N and save_h.stride(-1) == 1
+      assert save_h.dim() == a.dim() and save_h.shape[-2] == M and (batch == 1 or save_h.is_contiguous())
       h0 = save_h.data_ptr()
       h1 = h0 + N * 2
       ldh = save_h.stride(-2)

@@ -1,0 +1,56 @@
+"""The experts' gated MLP in batched launches, and the router's weight gradient, at tile edges."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("e,n,d,ff", [(1, 1, 64, 64), (3, 130, 72, 136), (8, 320, 256, 512), (2, 700, 768, 2048)])
+@pytest.mark.parametrize("buffers", [True, False])
+def test_gated_experts(e, n, d, ff, buffers):
+  """Against float64: forward one rounding to bf16 after fp32 sums (2^-9, a factor of two for the
+  sums and the activation); gradients pass two more bf16 tensors (3 x 2^-8 of the norm)."""
+  from t5x_b200.ops import functional as F
+  g = torch.Generator(device="cuda").manual_seed(n)
+  rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+  x = rnd(e, n, d).bfloat16().requires_grad_()
+  w = [torch.nn.Parameter((rnd(e, d, ff) * d ** -0.5).bfloat16().float()) for _ in range(2)]
+  for p in w:
+    p.bf16 = p.detach().bfloat16()
+    if buffers:
+      p.main_grad = torch.full_like(p, 9.0)
+      p.grad_ready = False
+  dy = rnd(e, n, ff).bfloat16()
+  y = F.batched_gated_mlp_in(x, *w)
+  y.backward(dy)
+  xd, wd = x.detach().double().requires_grad_(), [p.detach().double().requires_grad_() for p in w]
+  want = torch.nn.functional.gelu(xd @ wd[0], approximate="tanh") * (xd @ wd[1])
+  want.backward(dy.double())
+  assert float((y.double() - want).abs().max() / want.abs().max()) < 2 * 2.0 ** -9
+  for got, ref in [(x.grad, xd.grad)] + [(p.main_grad if buffers else p.grad, q.grad) for p, q in zip(w, wd)]:
+    assert float((got.double() - ref).norm() / ref.norm()) < 3 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("t,d,e", [(1, 64, 2), (127, 250, 8), (128, 258, 9), (129, 1024, 16), (5000, 768, 8),
+                                   (300, 33, 64)])
+def test_router_weight_gradient(t, d, e):
+  """fp32 sums over the tokens: below t 2^-24 of the sum of magnitudes, whatever the order."""
+  from t5x_b200.ops import native
+  g = torch.Generator(device="cuda").manual_seed(t)
+  x = torch.randn(t, d, device="cuda", generator=g).bfloat16()
+  w = torch.randn(d, e, device="cuda", generator=g) * d ** -0.5
+  k, capacity = 1, max(4, t)
+  fwd = native.moe_router_fwd(x, w, k, capacity)
+  dgate = torch.randn(t, k, device="cuda", generator=g)
+  coef = torch.zeros(2, device="cuda")
+  dx, dw = native.moe_router_bwd(x, w, k, capacity, fwd, dgate, coef)
+  native.check_status()
+  p = torch.softmax(x.double() @ w.double(), -1)
+  onehot = torch.nn.functional.one_hot(fwd["index"].long()[:, 0], e).double()
+  chosen = (p * onehot).sum(-1, keepdim=True)
+  dl = dgate.double() * chosen * (onehot - p)
+  ref, size = x.double().t() @ dl, x.double().abs().t() @ dl.abs()
+  # the logits' gradients themselves are fp32 values of a few operations (2^-18 of a magnitude)
+  assert bool(((dw.double() - ref).abs() <= (t * 2.0 ** -24 + 2.0 ** -15) * size + 1e-12).all())
+  again = native.moe_router_bwd(x, w, k, capacity, fwd, dgate, coef)[1]
+  assert torch.equal(dw, again)
