@@ -412,6 +412,12 @@ __device__ __forceinline__ float warp_max(float v) {
 // its first global write. `chain_release()` lets the kernel after this one start becoming
 // resident once every CTA of this grid has called it (or exited). Both are no-ops in a kernel
 // launched the ordinary way.
+//
+// A kernel that becomes resident early may find lines of its inputs in the SM's L1 that an older
+// kernel read before the memory was written anew (buffers are reused along a chain), and nothing
+// drops them when the wait returns. What earlier kernels of a chain write is therefore read through
+// L2 (`ld_chained`, TMA), never through L1 or the read-only path. A kernel launched the ordinary
+// way ends a chain: what it and the kernels before it wrote may be read either way.
 // Nanosecond timer shared by all SMs (for the optional per-CTA phase trace of the GEMM).
 __device__ __forceinline__ long long global_timer_ns() {
   long long t;
@@ -420,6 +426,10 @@ __device__ __forceinline__ long long global_timer_ns() {
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+template <typename T>
+__device__ __forceinline__ T ld_chained(const T* p) {
+  return __ldcg(p);
 }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() {

@@ -63,8 +63,10 @@ __global__ void __launch_bounds__(kDecWarps * 32)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int item = blockIdx.x * kDecWarps + warp;  // (row, head)
   chain_release();
-  chain_wait();  // q / k / v, the ancestry table and the position come from earlier kernels
-  if (item >= rows * H) return;
+  if (item >= rows * H) {
+    chain_wait();
+    return;
+  }
   const int row = item / H, h = item - row * H;
   const int b = row / beams;
   const int g = lane >> 3, part = lane & 7;
@@ -78,9 +80,10 @@ __global__ void __launch_bounds__(kDecWarps * 32)
   const int* anc = ancestry + static_cast<long long>(row) * L;
 
   // With few (row, head) items the kernel is a chain of dependent loads, so with kFirst = 8 the
-  // chain is kept to two links: the position, the slots of the first 32 positions and this step's
-  // vectors together, then the keys AND values of those positions. Later positions are streamed
-  // below, and with kFirst = 0 all are.
+  // history is requested ahead of the wait for the preceding kernel: the position, the slots of the
+  // first 32 positions, then the keys AND values of those positions. They come from before this
+  // chain of launches (earlier steps; the beam kernels, which are launched the ordinary way); q / k
+  // / v and the bias come from it. Later positions are streamed below, and with kFirst = 0 all are.
   constexpr int kU = 4;  // positions in flight per lane group in the streams
   constexpr int kHeld = kFirst > 0 ? kFirst : 1;
   int slot[kHeld];
@@ -90,25 +93,32 @@ __global__ void __launch_bounds__(kDecWarps * 32)
     slot[u] = t < L ? anc[t] : 0;
   }
   const int cur = min(max(*cur_index, 0), L - 1);
-  // 1. this step's query / key / value (8 dims per lane); append key / value at position
-  //    `cur` of the row's own slot
-  const uint4 qu = reinterpret_cast<const uint4*>(q + rh)[part];
-  const uint4 kn = reinterpret_cast<const uint4*>(k_new + rh)[part];
-  const uint4 vn = reinterpret_cast<const uint4*>(v_new + rh)[part];
   uint4 kf4[kHeld], vf4[kHeld];
   float bf[kHeld];
 #pragma unroll
   for (int u = 0; u < kFirst; ++u) {
     const int t = u * 4 + g;
-    kf4[u] = kn;
-    vf4[u] = vn;
-    bf[u] = 0.f;
     if (t < cur) {
       const long long at = batch_base + slot[u] * slot_stride + t * tstride;
       kf4[u] = reinterpret_cast<const uint4*>(cache_k + at)[part];
       vf4[u] = reinterpret_cast<const uint4*>(cache_v + at)[part];
     }
-    if (bias_row != nullptr && t <= cur) bf[u] = bias_row[static_cast<long long>(h) * L + t];
+  }
+  chain_wait();
+  // 1. this step's query / key / value (8 dims per lane); append key / value at position
+  //    `cur` of the row's own slot
+  const uint4 qu = ld_chained(reinterpret_cast<const uint4*>(q + rh) + part);
+  const uint4 kn = ld_chained(reinterpret_cast<const uint4*>(k_new + rh) + part);
+  const uint4 vn = ld_chained(reinterpret_cast<const uint4*>(v_new + rh) + part);
+#pragma unroll
+  for (int u = 0; u < kFirst; ++u) {
+    const int t = u * 4 + g;
+    if (t >= cur) {
+      kf4[u] = kn;
+      vf4[u] = vn;
+    }
+    bf[u] = 0.f;
+    if (bias_row != nullptr && t <= cur) bf[u] = ld_chained(bias_row + static_cast<long long>(h) * L + t);
   }
   if (g == 0) {
     const long long dst = batch_base + (row - b * beams) * slot_stride + cur * tstride;
@@ -152,7 +162,7 @@ __global__ void __launch_bounds__(kDecWarps * 32)
       const int t = t0 + u * 4 + g;
       float s = dot(ku[u]);
       if (t <= cur) {
-        if (bias_row != nullptr) s += bias_row[static_cast<long long>(h) * L + t];
+        if (bias_row != nullptr) s += ld_chained(bias_row + static_cast<long long>(h) * L + t);
         if (part == 0) sprob[warp][t] = s;
         mx = fmaxf(mx, s);
       }

@@ -28,6 +28,10 @@ struct alignas(16) Bf16x8 {
   __nv_bfloat162 v[4];
 };
 
+__device__ __forceinline__ Bf16x8 load8_chained(const Bf16x8* p) {
+  const uint4 u = ld_chained(reinterpret_cast<const uint4*>(p));
+  return *reinterpret_cast<const Bf16x8*>(&u);
+}
 __device__ __forceinline__ void unpack8(const Bf16x8& p, float* f) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -56,6 +60,8 @@ __global__ void __launch_bounds__(kNormThreads)
                        __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, int rows, int d,
                        float eps) {
   __shared__ float red[32];
+  chain_release();
+  chain_wait();
   const int nvec = d / 8;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const Bf16x8* xr = reinterpret_cast<const Bf16x8*>(x + static_cast<long long>(row) * d);
@@ -65,7 +71,7 @@ __global__ void __launch_bounds__(kNormThreads)
     for (int i = 0; i < kNormMaxVec; ++i) {
       const int v = threadIdx.x + i * kNormThreads;
       if (v < nvec) {
-        unpack8(xr[v], vals[i]);
+        unpack8(load8_chained(xr + v), vals[i]);
 #pragma unroll
         for (int j = 0; j < 8; ++j) ss += vals[i][j] * vals[i][j];
       }
@@ -258,6 +264,8 @@ __global__ void __launch_bounds__(kNormFwdThreads)
     rmsnorm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ scale,
                             __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, int rows,
                             int d, float eps) {
+  chain_release();
+  chain_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nvec = d / 8;
   const long long first = (static_cast<long long>(blockIdx.x) * (kNormFwdThreads / 32) + warp) * ROWS;
@@ -270,7 +278,7 @@ __global__ void __launch_bounds__(kNormFwdThreads)
     for (int i = 0; i < NV; ++i) {
       const int v = lane + i * 32;
       if (r < n && v < nvec)
-        u[r][i] = reinterpret_cast<const Bf16x8*>(x + (first + r) * d)[v];
+        u[r][i] = load8_chained(reinterpret_cast<const Bf16x8*>(x + (first + r) * d) + v);
     }
   float rstd[ROWS];
 #pragma unroll
@@ -322,9 +330,10 @@ template <int NV, int ROWS>
 static void launch_rmsnorm_fwd(const void* x, const void* scale, void* y, void* rstd, int rows, int d,
                                float eps, cudaStream_t st) {
   const int per_cta = kNormFwdThreads / 32 * ROWS;
-  rmsnorm_fwd_warp_kernel<NV, ROWS><<<(rows + per_cta - 1) / per_cta, kNormFwdThreads, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<const float*>(scale),
-      static_cast<__nv_bfloat16*>(y), static_cast<float*>(rstd), rows, d, eps);
+  launch_chained(rmsnorm_fwd_warp_kernel<NV, ROWS>, dim3((rows + per_cta - 1) / per_cta),
+                 dim3(kNormFwdThreads), 0, st, static_cast<const __nv_bfloat16*>(x),
+                 static_cast<const float*>(scale), static_cast<__nv_bfloat16*>(y),
+                 static_cast<float*>(rstd), rows, d, eps);
 }
 
 // AHEAD: the next row is requested while this one is worked on (us, with / without, with a
@@ -652,9 +661,9 @@ T5X_API int t5x_rmsnorm_fwd(const void* x, const void* scale, void* y, void* rst
     return 0;
   }
   int grid = rows < num_sms() * 8 ? rows : num_sms() * 8;
-  rmsnorm_fwd_kernel<<<grid, kNormThreads, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<const float*>(scale),
-      static_cast<__nv_bfloat16*>(y), static_cast<float*>(rstd), rows, d, eps);
+  launch_chained(rmsnorm_fwd_kernel, dim3(grid), dim3(kNormThreads), 0, st,
+                 static_cast<const __nv_bfloat16*>(x), static_cast<const float*>(scale),
+                 static_cast<__nv_bfloat16*>(y), static_cast<float*>(rstd), rows, d, eps);
   CHECK_LAUNCH("rmsnorm_fwd");
   return 0;
 }
@@ -793,10 +802,10 @@ __global__ void __launch_bounds__(256)
   chain_wait();  // the sums in src come from the kernel before this one
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n4;
        i += stride) {
-    float4 a = reinterpret_cast<const float4*>(src)[i];
+    float4 a = ld_chained(reinterpret_cast<const float4*>(src) + i);
     if (kClear) reinterpret_cast<float4*>(src)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (res != nullptr) {
-      const uint2 r = reinterpret_cast<const uint2*>(res)[i];
+      const uint2 r = ld_chained(reinterpret_cast<const uint2*>(res) + i);
       const float2 r0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x));
       const float2 r1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
       a.x += r0.x;
@@ -873,13 +882,13 @@ __global__ void __launch_bounds__(kNormThreads)
     const int v = threadIdx.x + i * kNormThreads;
     if (v < nvec) {
       float4* src = reinterpret_cast<float4*>(ws + row * d) + 2 * v;
-      const float4 a = src[0], b = src[1];
+      const float4 a = ld_chained(src), b = ld_chained(src + 1);
       src[0] = make_float4(0.f, 0.f, 0.f, 0.f);
       src[1] = make_float4(0.f, 0.f, 0.f, 0.f);
       float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
       if (res != nullptr) {
         float r[8];
-        unpack8(reinterpret_cast<const Bf16x8*>(res + row * d)[v], r);
+        unpack8(load8_chained(reinterpret_cast<const Bf16x8*>(res + row * d) + v), r);
 #pragma unroll
         for (int j = 0; j < 8; ++j) f[j] += r[j];
       }

@@ -172,7 +172,7 @@ __device__ __forceinline__ void load_row_bf16(const __nv_bfloat16* src, float* v
   if (vec_ok && n_valid >= 32) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      uint4 u = reinterpret_cast<const uint4*>(src)[i];
+      uint4 u = ld_chained(reinterpret_cast<const uint4*>(src) + i);
       const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&u);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -183,7 +183,7 @@ __device__ __forceinline__ void load_row_bf16(const __nv_bfloat16* src, float* v
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = (i < n_valid) ? __bfloat162float(src[i]) : 0.f;
+    for (int i = 0; i < 32; ++i) v[i] = (i < n_valid) ? __bfloat162float(ld_chained(src + i)) : 0.f;
   }
 }
 
@@ -274,7 +274,7 @@ __device__ __forceinline__ void staged_load_bf16(float* stage, const __nv_bfloat
     const int row = j * 8 + (lane >> 2);
     u[j] = make_uint4(0u, 0u, 0u, 0u);
     if (row < rows_valid)
-      u[j] = *reinterpret_cast<const uint4*>(src + static_cast<long long>(row) * ldr + c * 8);
+      u[j] = ld_chained(reinterpret_cast<const uint4*>(src + static_cast<long long>(row) * ldr + c * 8));
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j) {

@@ -268,8 +268,8 @@ __global__ void __launch_bounds__(kSkThreads, SkinnyCfg<BN>::kCtasPerSm)
         const int lrow = t / kChunks + kRowStep * it;
         const int grow = m0 + rank * rows_per + lrow;
         if (p.R != nullptr && lrow < rows_per && grow < p.M)
-          res[it] = *reinterpret_cast<const uint2*>(p.R + static_cast<long long>(grow) * p.ldr +
-                                                    n0 + cg * 4);
+          res[it] = ld_chained(reinterpret_cast<const uint2*>(
+              p.R + static_cast<long long>(grow) * p.ldr + n0 + cg * 4));
       }
       if (acc_ok) {
         // TMEM -> the outgoing tile in this CTA's ring: lane = row, 16-byte chunks of a row

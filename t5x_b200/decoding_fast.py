@@ -12,7 +12,7 @@ for decoding without a prompt, restated for the GPU:
   slot holds a beam's history; reselecting beams rewrites that table (kilobytes) instead of
   gathering every layer's cache (gigabytes);
 * cross-attention keys/values are projected once per example and shared by its beams;
-* q/k/v projections of a layer are one GEMM over a concatenated weight.
+* the q/k/v projections of a layer are one GEMM over the three weights.
 """
 from __future__ import annotations
 
@@ -266,13 +266,16 @@ def supported(module, decoder_input_tokens: torch.Tensor, decode_fn) -> bool:
           not c.float32_attention_logits)
 
 
+FEW_ROWS = 64  # up to so many rows the products of a step go through `native.gemm_few`
+
+
 class _Layer:
-  """bf16 weights of one decoder layer, q/k/v concatenated."""
+  """The bf16 weights of one decoder layer, the module's own (an update of the module shows)."""
 
   def __init__(self, layer):
     w = lambda dense: dense.kernel.bf16
     sa, ca, mlp = layer.self_attention, layer.encoder_decoder_attention, layer.mlp
-    self.qkv = torch.cat([w(sa.query), w(sa.key), w(sa.value)], dim=1).contiguous()
+    self.qkv = [w(sa.query), w(sa.key), w(sa.value)]
     self.o = w(sa.out)
     self.cq, self.co = w(ca.query), w(ca.out)
     self.ck, self.cv = w(ca.key), w(ca.value)
@@ -301,13 +304,13 @@ class GraphBeamDecoder:
                                                   termination_check_period)))
     self.replays = 0           # graph replays so far
     # Programmatic dependent launches inside the step (`native.chained_launches`): the products
-    # request their weights while the kernel in front of them finishes. On for up to 64 rows of a
-    # model up to T5.1.1 large (32 steps over 128 positions, ms, without / with: small, 8 layers,
-    # 1 row 15.8 / 14.8, 64 rows 18.7 / 17.2; base, 12 layers, 4 rows 28.6 / 26.5; large, 8 layers,
-    # 4 rows 22.3 / 20.7; but XL, 6 layers, 4 rows 22.2 / 23.0, where a wider product leaves no
-    # room beside its predecessor). Off for the tensor-parallel step: its kernels wait for other
-    # ranks.
-    chain = "2" if self.rows <= 64 and c.emb_dim <= 1024 else "0"
+    # request their weights while the kernel in front finishes. On for the rows that the kernel for
+    # few rows covers (32 steps over 128 positions, ms, without / with: small, 8 layers, 1 row 12.8 /
+    # 10.2; base, 12 layers, 4 rows 22.5 / 18.1, 64 rows 26.1 / 22.0; large, 8 layers, 4 rows 16.4 /
+    # 13.6; XL, 6 layers, 4 rows 15.9 / 13.6, 64 rows 20.5 / 18.5); with 256 rows nothing is gained (XL,
+    # 64 steps over 512 positions, 95.6 / 95.6). Off for the tensor-parallel step: its kernels wait for
+    # other ranks.
+    chain = "2" if self.rows <= FEW_ROWS else "0"
     self.chain_level = int(os.environ.get("T5X_B200_DECODE_CHAIN", chain)) if self.tp == 1 else 0
     # residual projections through the cluster split-K GEMM (sum over K slices in distributed
     # shared memory) instead of fp32 atomics into a workspace plus a finishing kernel
@@ -449,16 +452,31 @@ class GraphBeamDecoder:
       # every residual projection is followed by a norm: `_row_parallel` returns both the new
       # residual stream and its normed form (one finishing kernel on the single-GPU path)
       next_ln1 = norms[i + 1][0] if i + 1 < len(self.layers) else self.final_ln
-      qkv = native.gemm(h, ly.qkv).view(rows, 3, H, D)
-      self._self_attention(i, qkv, bias_row, ctx)
+      self._self_attention(i, self._qkv(h, ly).view(rows, 3, H, D), bias_row, ctx)
       x, h = self._row_parallel(ctx.view(rows, H * D), ly.o, x, ly.ln2)
       qc = self._skinny(h, ly.cq).view(rows, H, D)
       cc = self._cross_attention(i, qc, ctx)
       x, h = self._row_parallel(cc.reshape(rows, H * D), ly.co, x, ly.ln3)
-      g = native.gemm(h, ly.wi0, b2=ly.wi1)
+      g = self._few(h, [ly.wi0, ly.wi1], gated=True)
+      if g is None:
+        g = native.gemm(h, ly.wi0, b2=ly.wi1)
       x, h = self._row_parallel(g, ly.wo, x, next_ln1)
     logits = native.gemm(h, self.w_logits, out_dtype=torch.float32, alpha=self.logit_scale)
     return logits if self.link is None else self.link.gather_logits(logits)
+
+  def _few(self, a, weights, **kw):
+    """The products for few rows, or None where there are more."""
+    if self.rows > FEW_ROWS or self.link is not None:
+      return None
+    return native.gemm_few(a, weights, **kw)
+
+  def _qkv(self, h, ly):
+    out = self._few(h, ly.qkv)
+    if out is None:
+      n = self.H * self.D
+      out = torch.empty(self.rows, 3 * n, dtype=torch.bfloat16, device=self.dev)
+      native.gemm_shared(h, ly.qkv, into=[out[:, i * n:(i + 1) * n] for i in range(3)])
+    return out
 
   def _row_parallel(self, a, w, residual, next_norm_scale):
     """(x, h): x = a @ w + residual and h = rmsnorm(x) * next_norm_scale, for a projection whose
@@ -471,19 +489,25 @@ class GraphBeamDecoder:
       x = native.gemm(a, w, residual=residual)
       return x, native.rmsnorm_fwd(x, next_norm_scale, 1e-6)[0]
     if self.cluster_gemm:
-      x = native.gemm_skinny(a, w, residual=residual)
+      x = self._cluster(a, w, residual)
       if x is not None:
         return x, native.rmsnorm_fwd(x, next_norm_scale, 1e-6)[0]
     return native.gemm_splitk_norm(a, w, _splits(w.shape[0], w.shape[1], self.rows),
                                    residual=residual, scale=next_norm_scale, eps=1e-6,
                                    workspace=self._workspace())
 
+  def _cluster(self, a, w, residual):
+    """a @ w (+ residual) with K cut over a cluster of CTAs, or None where that is not covered."""
+    s = native.gemm_skinny_splits(self.rows, w.shape[1], w.shape[0])
+    x = self._few(a, [w], residual=residual, splits=s) if s > 0 else None
+    return native.gemm_skinny(a, w, residual=residual) if x is None else x
+
   def _skinny(self, a, w, residual=None):
     """a[rows, K] @ w[K, N] (+ residual) with K split over CTAs when rows are few."""
     if self.rows > 512:
       return native.gemm(a, w, residual=residual)
     if self.cluster_gemm:
-      x = native.gemm_skinny(a, w, residual=residual)
+      x = self._cluster(a, w, residual)
       if x is not None:
         return x
     return native.gemm_splitk(a, w, _splits(w.shape[0], w.shape[1], self.rows),

@@ -411,13 +411,16 @@ def gemm_sum(a, b) -> torch.Tensor:
   return out
 
 
-def gemm_shared(a: torch.Tensor, b, *, out=None, accumulate: bool = False, pieces: int = 0):
-  """[a @ w for w in b] (up to three) in one launch: bf16, or, with fp32 buffers `out` [M, N_i],
-  weight gradients as by `gemm_wgrad`."""
+def gemm_shared(a: torch.Tensor, b, *, out=None, into=None, accumulate: bool = False, pieces: int = 0):
+  """[a @ w for w in b] (up to three) in one launch: bf16, in the matrices `into` if given, or, with
+  fp32 buffers `out` [M, N_i], weight gradients as by `gemm_wgrad`."""
   assert a.dtype == torch.bfloat16 and all(w.dtype == torch.bfloat16 for w in b)
   M, K = a.shape
   assert all(w.shape[0] == K for w in b)
   fp32 = out is not None
+  assert not (fp32 and into is not None)
+  if into is not None:
+    out = into
   if out is None:
     out = [torch.empty((M, w.shape[1]), dtype=torch.bfloat16, device=a.device) for w in b]
   assert all(o.shape == (M, w.shape[1]) and o.stride(1) == 1 for o, w in zip(out, b))
@@ -519,6 +522,42 @@ def gemm_skinny(a: torch.Tensor, b: torch.Tensor, *, residual: Optional[torch.Te
                                 a.stride(0), ldb, out.stride(0),
                                 residual.stride(0) if residual is not None else 0, b_mn, s,
                                 tile_n, float(alpha), stream_ptr()), "gemm_skinny")
+  return out
+
+
+register_signature("t5x_gemm_few_covers", [c_int] * 6)
+register_signature("t5x_gemm_few_bf16", [c_void_p] * 4 + [c_int] * 4 + [c_ll] * 4 + [c_int] * 2 +
+                   [c_void_p])
+
+
+def gemm_few(a: torch.Tensor, weights, *, residual: Optional[torch.Tensor] = None, gated: bool = False,
+             splits: int = 1) -> Optional[torch.Tensor]:
+  """[a @ w for w in weights] side by side (+ residual) in bf16 for up to 64 rows, or, `gated`,
+  gelu(a @ weights[0]) * (a @ weights[1]). The sums are those of `gemm` (splits = 1) or `gemm_skinny`
+  with as many splits, bit by bit. None where the kernel does not cover the call."""
+  M, K = a.shape
+  n, w0 = len(weights), weights[0]
+  width = w0.shape[1]
+  if (a.dtype != torch.bfloat16 or a.stride(1) != 1 or w0.shape[0] != K or w0.stride(1) != 1 or
+      any(w.dtype != torch.bfloat16 or w.shape != w0.shape or w.stride() != w0.stride() or
+          w.data_ptr() & 15 for w in weights)):
+    return None
+  lda = a.stride(0) if M > 1 else K
+  ldb = w0.stride(0)
+  if lda % 8 or ldb % 8 or lda < K or ldb < width or a.data_ptr() & 15 or \
+      not lib().t5x_gemm_few_covers(M, K, n, width, splits, int(gated)):
+    return None
+  cols = width if gated else n * width
+  ldr = 0
+  if residual is not None:
+    if (gated or residual.dtype != torch.bfloat16 or residual.shape != (M, cols) or
+        residual.stride(1) != 1 or residual.stride(0) % 4 or residual.data_ptr() & 7):
+      return None
+    ldr = residual.stride(0)
+  out = torch.empty(M, cols, dtype=torch.bfloat16, device=a.device)
+  _check(lib().t5x_gemm_few_bf16(a.data_ptr(), (c_void_p * n)(*[w.data_ptr() for w in weights]),
+                                 out.data_ptr(), ptr(residual), M, K, n, width, lda, ldb, cols, ldr,
+                                 splits, int(gated), stream_ptr()), "gemm_few")
   return out
 
 
