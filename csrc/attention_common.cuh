@@ -51,34 +51,78 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&p);
 }
 
-// Writes 8 consecutive bf16 (one 16-byte chunk) of row r, chunk c (0..7) of a [128 x 64] K-major
-// 128B-swizzled tile.
 // Key blocks that the streaming forward kernel walks: up to the last visible key where nothing but a
-// key mask hides keys. The blocks behind it (the padding of a batch) would contribute exact zeros,
+// key mask hides keys. The blocks behind it (the padding of a batch) would contribute exact zeros (the
+// scores of visible keys being far above the -1e10 of hidden ones),
 // unless no key at all is visible: then all count, the rows are uniform over all keys. `find` leaves
-// each warp's last visible key in `words`; a __syncthreads later `visible_key_blocks` gives the number.
+// each warp's findings in `words`; a __syncthreads later `visible_key_blocks` gives the number.
 // (Keys of which 60 to 100 % are visible, us before / so: 16 x 6 heads x 1024 x 1024 181 / 165, 8 x 32 x
 // 1024 x 1024 of 128 features 656 / 566. The short-range kernel walks all of its four blocks: with a
 // number of blocks known only then it lost 8 % where none is hidden and gained 1 % where some are.)
 __device__ __forceinline__ bool key_mask_alone(const AttnParams& p) {
   return p.key_mask != nullptr && !p.causal && p.kv_seg == nullptr;
 }
-__device__ __forceinline__ void find_visible_keys(const AttnParams& p, int b, int* words) {
-  if (!key_mask_alone(p)) return;
-  int last = -1;
-  for (int k = threadIdx.x; k < p.Lk; k += blockDim.x)
-    if (p.key_mask[static_cast<long long>(b) * p.Lk + k]) last = k;
-  last = __reduce_max_sync(0xffffffffu, last);
-  if ((threadIdx.x & 31) == 0) words[threadIdx.x >> 5] = last;
+// Under a causal or prefix-LM mask of self-attention the same holds for the blocks behind a tile's
+// last query (and behind the last prefix key, if the tile has queries inside the prefix), as long as
+// each of the tile's queries sees itself. To look that up costs a CTA some 3 us, so only from more
+// than kAheadKeys keys on (us before / so: prefix LM, 16 x 12 heads x 1024, 600 tokens in the prefix,
+// 472 / 409; causal, 8 x 32 heads of 128 x 1024 670 / 514; but 8 x 32 x 256 72 / 77).
+constexpr int kAheadKeys = 512;
+__device__ __forceinline__ bool causal_self(const AttnParams& p) {
+  return p.causal && p.Lq == p.Lk && p.causal_off == 0 && p.Lk > kAheadKeys;
 }
-__device__ __forceinline__ int visible_key_blocks(const AttnParams& p, const int* words, int warps) {
+__device__ __forceinline__ bool sees_itself(const AttnParams& p, int b, int q) {
+  const long long at = static_cast<long long>(b) * p.Lk + q;
+  const int mask = p.causal == 2 ? 0x3fffffff : -1;
+  return (p.key_mask == nullptr || p.key_mask[at] != 0) &&
+         (p.kv_seg == nullptr || (p.q_seg != nullptr && ((p.q_seg[at] ^ p.kv_seg[at]) & mask) == 0));
+}
+__device__ __forceinline__ bool in_prefix(const AttnParams& p, int b, int k) {
+  return p.causal == 2 && p.kv_seg != nullptr && ((p.kv_seg[static_cast<long long>(b) * p.Lk + k] >> 30) & 1);
+}
+constexpr int kAllKeys = 0x7fffffff;
+// Leaves two words per warp: the last key that counts, and whether the tile has prefix queries.
+__device__ __forceinline__ void find_visible_keys(const AttnParams& p, int b, int q_base, int q_end,
+                                                  int* words) {
+  int last = -1, pre = 0;
+  if (key_mask_alone(p)) {
+    for (int k = threadIdx.x; k < p.Lk; k += blockDim.x)
+      if (p.key_mask[static_cast<long long>(b) * p.Lk + k]) last = k;
+  } else if (causal_self(p)) {
+    for (int k = threadIdx.x; k < p.Lk; k += blockDim.x) {
+      if (in_prefix(p, b, k)) {
+        last = max(last, k);
+        if (k >= q_base && k < q_end) pre = 1;
+      }
+      if (k >= q_base && k < q_end && !sees_itself(p, b, k)) last = kAllKeys;
+    }
+  } else {
+    return;
+  }
+  last = __reduce_max_sync(0xffffffffu, last);
+  pre = __reduce_max_sync(0xffffffffu, pre);
+  if ((threadIdx.x & 31) == 0) {
+    words[(threadIdx.x >> 5) * 2] = last;
+    words[(threadIdx.x >> 5) * 2 + 1] = pre;
+  }
+}
+__device__ __forceinline__ int visible_key_blocks(const AttnParams& p, int q_end, const int* words,
+                                                  int warps) {
   const int all = (p.Lk + 127) / 128;
-  if (!key_mask_alone(p)) return all;
-  int last = -1;
-  for (int w = 0; w < warps; ++w) last = max(last, words[w]);
-  return last < 0 ? all : last / 128 + 1;
+  const bool alone = key_mask_alone(p);
+  if (!alone && !causal_self(p)) return all;
+  int last = -1, pre = 0;
+  for (int w = 0; w < warps; ++w) {
+    last = max(last, words[2 * w]);
+    pre |= words[2 * w + 1];
+  }
+  if (alone) return last < 0 ? all : last / 128 + 1;
+  if (last == kAllKeys) return all;
+  return min(all, max(q_end - 1, pre ? last : -1) / 128 + 1);
 }
 
+// Writes 8 consecutive bf16 (one 16-byte chunk) of row r, chunk c (0..7) of a [128 x 64] K-major
+// 128B-swizzled tile.
 __device__ __forceinline__ void store_swizzled_chunk(uint8_t* tile, int r, int c, const float* v) {
   uint4 u;
   u.x = pack_bf16x2(v[0], v[1]);

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kFsThreads, 1)
   uint64_t* bar_pv = bar_p + kFsMaxTiles;    // kTiles: O_t += P_t V_j finished
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_pv + kFsMaxTiles);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* last_key = reinterpret_cast<int*>(tmem_slot + 2);  // one word per warp
+  int* last_key = reinterpret_cast<int*>(tmem_slot + 2);  // two words per warp
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.y, b = blockIdx.z;
@@ -126,12 +126,13 @@ __global__ void __launch_bounds__(kFsThreads, 1)
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish();
   }
-  find_visible_keys(p, b, last_key);
+  const int q_end = min(p.Lq, q_base + 128 * kTiles);
+  find_visible_keys(p, b, q_base, q_end, last_key);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  nblk = min(nblk, visible_key_blocks(p, last_key, kFsThreads / 32));
+  nblk = min(nblk, visible_key_blocks(p, q_end, last_key, kFsThreads / 32));
   constexpr uint32_t kStageBytes = 2 * kPanels * kFsPanel;
 
   if (warp == kFsLoadWarp) {

@@ -468,7 +468,9 @@ struct BwdSmem {
   static constexpr int kTotal = kBars + 256 + 1024;
 };
 
-template <int D>
+// kAhead: causal self-attention, where query blocks may be passed over (a variant of its own: the
+// first block held in a register costs the other one spills).
+template <int D, bool kAhead>
 __global__ void __launch_bounds__(kAttnThreads, 1)
     attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -503,8 +505,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k0 = blockIdx.x * 128, h = blockIdx.y, b = blockIdx.z;
-  const int nq = (p.Lq + 127) / 128;
-  const int lq_pad = nq * 128;
+  const int lq_pad = (p.Lq + 127) / 128 * 128;
   // TMEM columns
   // dQ partial tiles alternate between two 64-column buffers, so that the tile of query block
   // i is read out while the MMAs of block i + 1 run.
@@ -550,6 +551,20 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   const bool idle = !any_shown && key_mask_alone(p) &&
                     p.lse[(static_cast<long long>(b) * p.H + h) * p.Lq] >= -5e9f;
 
+  // Of causal self-attention the query blocks ahead of this key block see nothing of it (unless both
+  // lie in the prefix of a prefix LM), and where each of their queries sees itself their P and dS are
+  // exact zeros: the walk starts at the first block behind them. (us before / so: causal, 8 x 32 heads
+  // of 128 x 1024 1205 / 838, 32 x 12 x 256 182 / 170; prefix LM, 16 x 12 x 1024, 600 tokens in the
+  // prefix, 730 / 612, but 4 x 12 x 300 109 / 114: from more than kAheadKeys keys on.)
+  int q_first = 0;
+  if (kAhead && k0 > 0) {
+    bool keep = false;
+    for (int q = threadIdx.x; q < k0 + 128 && q < p.Lk; q += kAttnThreads)
+      keep = keep || (q < k0 ? !sees_itself(p, b, q) : in_prefix(p, b, q));
+    if (!__syncthreads_or(keep)) q_first = k0;
+  }
+  const int nq = (lq_pad - (kAhead ? q_first : 0)) / 128;
+
   if (idle) {
     for (int i = threadIdx.x; i < 128 * (D / 8); i += kAttnThreads) {
       const int k = k0 + i / (D / 8);
@@ -571,9 +586,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         mbar_expect_tx(&bar_qdo[st], 2 * kStageBytes);
         for (int c = 0; c < kPanels; ++c) {
           tma_load_4d(sQ + st * kStageBytes + c * Smem::kTile, &tmQ, &bar_qdo[st], c * 64, h,
-                      i * 128, b);
+                      (kAhead ? q_first : 0) + i * 128, b);
           tma_load_4d(sDO + st * kStageBytes + c * Smem::kTile, &tmDO, &bar_qdo[st], c * 64, h,
-                      i * 128, b);
+                      (kAhead ? q_first : 0) + i * 128, b);
         }
       };
       for (int i = 0; i < nq && i < Smem::kStages; ++i) load_qdo(i, i);
@@ -722,7 +737,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     const float* head_table =
         has_bias ? p.rel_bias + static_cast<long long>(h) * p.num_buckets : nullptr;
     auto fetch_vectors = [&](int i) {
-      const int qb = i * 128;
+      const int qb = (kAhead ? q_first : 0) + i * 128;
       const int t = threadIdx.x;
       if (t < 128) {
         const int q = qb + t;
@@ -771,7 +786,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       }
       // Four lanes exchange their 16-byte pieces, so that an instruction adds 64 contiguous bytes
       // of 8 rows instead of 16 of 32 (128 x 12 heads x 512 x 512 1009 / 976 us).
-      const int q0 = blk * 128 + quarter * 32 + (lane & ~3);
+      const int q0 = (kAhead ? q_first : 0) + blk * 128 + quarter * 32 + (lane & ~3);
       float* dst = p.dQ + ((static_cast<long long>(b) * p.Lq + q0) * p.H + h) * D +
                    part * kColsPerPart + (lane & 3) * 4;
       const long long row_step = static_cast<long long>(p.H) * D;
@@ -795,7 +810,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     publish_vectors(0);
     softmax_bar_sync();
     for (int i = 0; i < nq && ok; ++i) {
-      const int qb = i * 128;
+      const int qb = (kAhead ? q_first : 0) + i * 128;
       const float* sLse = sVec + (i & 1) * 384;
       const float* sDelta = sLse + 128;
       const int* sQseg = reinterpret_cast<const int*>(sDelta + 128);
@@ -1069,7 +1084,7 @@ T5X_API int t5x_attention_fwd(const void* q, const void* k, const void* v, void*
 }
 
 namespace t5x {
-template <int D>
+template <int D, bool kAhead>
 static int launch_attention_bwd(const void* d_o, const void* o, void* delta, const CUtensorMap* tq,
                                 const CUtensorMap* tk, const CUtensorMap* tv,
                                 const CUtensorMap* tdo, const AttnParams& p, long long do_sb,
@@ -1085,14 +1100,14 @@ static int launch_attention_bwd(const void* d_o, const void* o, void* delta, con
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<D>,
+    cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<D, kAhead>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          BwdSmem<D>::kTotal);
     if (e != cudaSuccess) return set_error("attention_bwd attr: %s", cudaGetErrorString(e));
     attr_set[dev] = true;
   }
   dim3 grid((p.Lk + 127) / 128, p.H, p.B);
-  attn_bwd_kernel<D><<<grid, kAttnThreads, BwdSmem<D>::kTotal, st>>>(*tq, *tk, *tv, *tdo, p);
+  attn_bwd_kernel<D, kAhead><<<grid, kAttnThreads, BwdSmem<D>::kTotal, st>>>(*tq, *tk, *tv, *tdo, p);
   count_launches(2);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("attention_bwd: %s", cudaGetErrorString(e));
@@ -1141,9 +1156,8 @@ T5X_API int t5x_attention_bwd(const void* q, const void* k, const void* v, const
   p.dV = static_cast<__nv_bfloat16*>(dv);
   p.dk_sb = dk_sb; p.dk_sl = dk_sl; p.dk_sh = dk_sh;
   p.status = device_status_buffer();
-  if (D == 128)
-    return launch_attention_bwd<128>(d_o, o, delta, tq, tk, tv, tdo, p, do_sb, do_sl, do_sh, o_sb,
-                                     o_sl, o_sh, st);
-  return launch_attention_bwd<64>(d_o, o, delta, tq, tk, tv, tdo, p, do_sb, do_sl, do_sh, o_sb,
-                                  o_sl, o_sh, st);
+  const bool ahead = causal && Lq == Lk && causal_off == 0 && Lq > (causal == 2 ? kAheadKeys : 128);
+  const auto launch = D == 128 ? (ahead ? launch_attention_bwd<128, true> : launch_attention_bwd<128, false>)
+                               : (ahead ? launch_attention_bwd<64, true> : launch_attention_bwd<64, false>);
+  return launch(d_o, o, delta, tq, tk, tv, tdo, p, do_sb, do_sl, do_sh, o_sb, o_sl, o_sh, st);
 }

@@ -65,3 +65,58 @@ def test_hidden_blocks(kind, lq, lk, d, bias):
     k3, v3 = k.clone(), v.clone()
     k3[hidden], v3[hidden] = 3.0, -2.0
     assert torch.equal(attention.flash_attention(q, k3, v3, bias_table=table, key_mask=mask), o)
+
+
+@pytest.mark.parametrize("mode", ["causal", "causal_padded", "causal_packed", "prefix", "prefix_padded",
+                                  "prefix_packed"])
+@pytest.mark.parametrize("l,d", [(129, 64), (384, 64), (700, 64), (300, 128), (520, 128)])
+def test_hidden_query_blocks(mode, l, d):
+  """Causal and prefix-LM self-attention over several blocks: those that nothing in a tile sees are passed
+  over, but not where a padding query sees no key at all (its row is uniform over all of them)."""
+  from t5x_b200.ops import attention, native, reference
+  g = torch.Generator(device="cuda").manual_seed(l + d)
+  b, h = 3, 2
+  rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+  q = (rnd(b, l, h, d) * d ** -0.5).bfloat16().requires_grad_()
+  k, v = (rnd(b, l, h, d).bfloat16().requires_grad_() for _ in range(2))
+  do = rnd(b, l, h, d).bfloat16()
+  table = torch.nn.Parameter(rnd(h, 32) * 0.5)
+  pos = torch.arange(l, device="cuda")
+  valid = torch.ones(b, l, dtype=torch.bool, device="cuda")
+  if mode.endswith("padded"):
+    valid[1, l // 2:] = False
+    valid[2, 3:] = False
+    if not mode.startswith("prefix"):
+      valid[2, 0] = False  # the first queries see nothing
+  seg = (pos // 100 + 1)[None].expand(b, l).contiguous() if mode.endswith("packed") else None
+  mask = (pos[None] <= pos[:, None])[None].expand(b, l, l)
+  if mode.startswith("prefix"):
+    inside = torch.zeros(b, l, dtype=torch.bool, device="cuda")
+    inside[0, :l // 3], inside[1, :l // 4], inside[2, :1] = True, True, True
+    prefix = reference.PrefixLMMask(inside, valid, seg)
+    mask = prefix.bool()[:, 0]
+    kw = dict(prefix_lm=prefix)
+  elif mode.endswith("packed"):
+    mask = mask & (seg[:, :, None] == seg[:, None, :])
+    kw = dict(causal=True, q_segment_ids=seg, kv_segment_ids=seg)
+  else:
+    mask = mask & valid[:, None, :]
+    kw = dict(causal=True, key_mask=valid if mode.endswith("padded") else None)
+  o = attention.flash_attention(q, k, v, bias_table=table, bidirectional=False, **kw)
+  grads = torch.autograd.grad(o, [q, k, v], do)
+  native.check_status()
+  q2, k2, v2 = (t.detach().double().requires_grad_() for t in (q, k, v))
+  rel = pos[None] - pos[:, None]
+  s = torch.einsum("bqhd,bkhd->bhqk", q2, k2) + \
+      table.detach().double()[:, reference.relative_position_bucket(rel, False, 32, 128)][None]
+  s = torch.where(mask[:, None], s, s * 0 - 1e10)
+  want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), v2)
+  ref = torch.autograd.grad(want, [q2, k2, v2], do.double())
+  # probabilities and their gradients are rounded to bf16 once, as is the result
+  assert float((o.double() - want).norm() / want.norm()) < 2 * 2.0 ** -8
+  # (the kernel hands q and k the dS of rows that see nothing as if they were not masked)
+  seen = mask.any(-1).all(-1)
+  for i, (x, y) in enumerate(zip(grads, ref)):
+    x, y = (x, y) if i == 2 else (x[seen], y[seen])
+    if y.numel():
+      assert float((x.double() - y).norm() / y.norm()) < 3 * 2.0 ** -8
