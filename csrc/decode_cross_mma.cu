@@ -76,46 +76,12 @@ __global__ void __launch_bounds__(kXmThreads)
   const __nv_bfloat16* vb = vt + bh * 64 * Lp;
   const uint8_t* km = key_mask == nullptr ? nullptr : key_mask + static_cast<long long>(b) * Lk;
 
-  // Keys, values and mask are constant while decoding: this CTA's part of them is pulled toward L2,
-  // and the mask and the first keys into registers, while the kernel before this one (which
-  // produces q) may still be running.
+  // Keys and values are encoder products, constant while decoding: this CTA's part of them is
+  // pulled toward L2 while the kernel before this one (which produces q) may still be running.
   chain_release();
   for (int line = threadIdx.x; line < Lp; line += kXmThreads) {  // Lp x 128 bytes each
     prefetch_l2(reinterpret_cast<const char*>(kb) + static_cast<long long>(line) * 128);
     prefetch_l2(reinterpret_cast<const char*>(vb) + static_cast<long long>(line) * 128);
-  }
-  // chunks of 32 keys; every warp takes a contiguous run of chunks
-  const int nchunks = Lp / 32;
-  const int per_warp = (nchunks + kXmWarps - 1) / kXmWarps;
-  const int first = warp * per_warp;
-  const int mine = max(0, min(per_warp, nchunks - first));
-  constexpr int kBatch = 2;  // chunks whose key rows are requested before any is used
-  uint4 kr[kBatch][4][2];
-  auto request_keys = [&](int i0) {
-#pragma unroll
-    for (int c = 0; c < kBatch; ++c) {
-      const int base = (first + min(i0 + c, mine - 1)) * 32;
-#pragma unroll
-      for (int ut = 0; ut < 4; ++ut) {
-        const int key = base + key_of_column(ut >> 1, ut & 1, g);  // the row this lane group loads
-        const uint4* src =
-            reinterpret_cast<const uint4*>(kb + static_cast<long long>(key) * 64 + 16 * t);
-        kr[c][ut][0] = src[0];
-        kr[c][ut][1] = src[1];
-      }
-    }
-  };
-  if (mine > 0) request_keys(0);
-  uint32_t shown = 0xffffffffu;  // byte i: chunk i, bit j: key 8t + j of it (the lane's columns)
-  if (km != nullptr) {
-    shown = 0u;
-#pragma unroll
-    for (int i = 0; i < kXmMaxChunks; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int kk = (first + i) * 32 + 8 * t + j;
-        if (i < mine && kk < Lk && km[kk] != 0) shown |= 1u << (8 * i + j);
-      }
   }
   chain_wait();
 
@@ -131,13 +97,30 @@ __global__ void __launch_bounds__(kXmThreads)
     qa[4] = hi.x, qa[5] = hi.y, qa[6] = hi.z, qa[7] = hi.w;
   }
 
-  // ---- scores ----
+  // ---- scores: chunks of 32 keys; every warp takes a contiguous run of chunks ----
+  const int nchunks = Lp / 32;
+  const int per_warp = (nchunks + kXmWarps - 1) / kXmWarps;
+  const int first = warp * per_warp;
+  const int mine = max(0, min(per_warp, nchunks - first));
   float sc[kXmMaxChunks][2][4];  // [chunk][half]: tile 0 columns (2t, 2t+1), tile 1 columns (2t, 2t+1)
   float mx = -3.0e38f;
+  constexpr int kBatch = 2;  // chunks whose key rows are requested before any is used
 #pragma unroll
   for (int i0 = 0; i0 < kXmMaxChunks; i0 += kBatch) {
     if (i0 >= mine) break;
-    if (i0 > 0) request_keys(i0);
+    uint4 kr[kBatch][4][2];
+#pragma unroll
+    for (int c = 0; c < kBatch; ++c) {
+      const int base = (first + min(i0 + c, mine - 1)) * 32;
+#pragma unroll
+      for (int ut = 0; ut < 4; ++ut) {
+        const int key = base + key_of_column(ut >> 1, ut & 1, g);  // the row this lane group loads
+        const uint4* src =
+            reinterpret_cast<const uint4*>(kb + static_cast<long long>(key) * 64 + 16 * t);
+        kr[c][ut][0] = src[0];
+        kr[c][ut][1] = src[1];
+      }
+    }
 #pragma unroll
     for (int c = 0; c < kBatch; ++c) {
       const int i = i0 + c;
@@ -158,7 +141,7 @@ __global__ void __launch_bounds__(kXmThreads)
           const int kk = base + key_of_column(u, tile, 2 * t + e);
           float v = acc4[e];
           const bool exists = kk < Lk;
-          if (exists && !((shown >> (8 * i + 4 * u + 2 * tile + e)) & 1u)) v = kXmMasked;
+          if (exists && km != nullptr && km[kk] == 0) v = kXmMasked;
           if (!exists) v = -3.0e38f;  // padding of the key range: weight exactly zero
           sc[i][u][2 * tile + e] = v;
           if (exists) mx = fmaxf(mx, v);
