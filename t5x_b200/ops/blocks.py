@@ -193,6 +193,7 @@ class _GatedMlpBlockFn(torch.autograd.Function):
   @staticmethod
   def backward(ctx, dy):
     x, scale, w0, w1, wo, *saved = ctx.saved_tensors
+    saved[3] = F.to_overwrite(saved[3])  # the pre-activations become their gradients
     params = [w0, w1, wo]
     flags = [bool(getattr(p, "grad_ready", False)) for p in params + [scale]]
     done = False

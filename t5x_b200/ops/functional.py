@@ -119,6 +119,18 @@ def _host_linear_bwd(dys, x, weights, needs):
   return (False, None) if done is None else (True, done[0])
 
 
+# Whether the graph of the backward pass that is running is kept, so that another pass may follow; a
+# torch without the question counts as yes.
+_graph_is_kept = getattr(torch._C._autograd, "_get_current_graph_task_keep_graph", lambda: True)
+
+
+def to_overwrite(saved: torch.Tensor) -> torch.Tensor:
+  """A saved tensor that a backward pass writes its result over: itself where nobody reads it again,
+  a copy where the graph is kept (`retain_graph`, `create_graph`) for another pass. The kernels write
+  through raw pointers, which autograd's version counter does not see."""
+  return saved.clone() if _graph_is_kept() else saved
+
+
 def _input_grad(dys, mats):
   """dys[0] @ mats[0] + dys[1] @ mats[1] + ...: two or three products in one launch where the matrices
   lie the same way, else products that add to what the ones before stored."""
@@ -282,7 +294,7 @@ class _BatchedGatedMlpInFn(torch.autograd.Function):
     x, wi_0, wi_1, h = ctx.saved_tensors
     w0, w1 = compute_weight(wi_0, torch.bfloat16), compute_weight(wi_1, torch.bfloat16)
     dff = w0.shape[2]
-    # the saved pre-activations are overwritten with their gradients (one backward per forward)
+    h = to_overwrite(h)  # the pre-activations become their gradients
     native.gated_gelu_bwd_(dg.reshape(-1, dff).contiguous(), h.view(-1, 2 * dff))
     dhs = (h[..., :dff], h[..., dff:])
     dx = None
@@ -437,6 +449,7 @@ class _GatedGeluMlpInFn(torch.autograd.Function):
   @staticmethod
   def backward(ctx, dg):
     x, wi_0, wi_1, h = ctx.saved_tensors
+    h = to_overwrite(h)  # the pre-activations become their gradients
     host, (need_dx, need_0, need_1) = native.host(), ctx.needs_input_grad[:3]
     g0, g1 = getattr(wi_0, "main_grad", None), getattr(wi_1, "main_grad", None)
     if host is not None and need_0 == need_1 and not (need_0 and (g0 is None or g1 is None)):
@@ -454,12 +467,10 @@ class _GatedGeluMlpInFn(torch.autograd.Function):
     k = x.shape[-1]
     dff = h.shape[1] // 2
     x2 = x.reshape(-1, k)
-    # The saved pre-activations are overwritten with their gradients (one backward per forward).
-    dh = h
-    native.gated_gelu_bwd_(dg.reshape(-1, dff).contiguous(), dh)  # dh <- [dh0|dh1]
+    native.gated_gelu_bwd_(dg.reshape(-1, dff).contiguous(), h)  # h <- [dh0|dh1]
     w0 = compute_weight(wi_0, torch.bfloat16)
     w1 = compute_weight(wi_1, torch.bfloat16)
-    dh0, dh1 = dh[:, :dff], dh[:, dff:]
+    dh0, dh1 = h[:, :dff], h[:, dff:]
     dx = None
     if ctx.needs_input_grad[0]:
       dx = _input_grad([dh0, dh1], [w0.t(), w1.t()]).view(x.shape)
