@@ -449,11 +449,13 @@ Tensor norm_backward(const Tensor& dh, const Tensor& x, const Tensor& scale, con
   return dx;
 }
 
-// Weights wq, wk, wv, wo of an attention block over x [B, Lq, d] and (cross attention) kv.
-bool attention_weights_ok(const Tensor& x, const Tensor& kv, const std::vector<Tensor>& w, int64_t head_dim) {
+// Weights wq, wk, wv, wo of an attention block over x [B, Lq, d] and (cross attention) kv, of `heads`
+// heads, as many as the bias table was checked for.
+bool attention_weights_ok(const Tensor& x, const Tensor& kv, const std::vector<Tensor>& w, int64_t heads,
+                          int64_t head_dim) {
   if (w.size() != 4) return false;
   const Weight q(w[0], x.size(-1)), k(w[1], kv.size(-1)), v(w[2], kv.size(-1));
-  if (!q.ok || !k.ok || !v.ok || q.n != k.n || q.n != v.n || q.n % head_dim) return false;
+  if (!q.ok || !k.ok || !v.ok || q.n != k.n || q.n != v.n || q.n != heads * head_dim) return false;
   const Weight o(w[3], q.n);
   return o.ok && o.n == x.size(-1);
 }
@@ -466,11 +468,11 @@ bool mlp_weights_ok(const Tensor& x, const std::vector<Tensor>& w) {
 }
 
 bool attention_block_ok(const Tensor& x, const optional<Tensor>& kv, const Tensor& scale,
-                        const std::vector<Tensor>& w, int64_t head_dim) {
+                        const std::vector<Tensor>& w, int64_t heads, int64_t head_dim) {
   const Tensor& in = kv ? *kv : x;
   return x.dim() == 3 && plain(x) && rows_fit(x) && norm_ok(scale, x) &&
          (!kv || (kv->dim() == 3 && plain(*kv) && rows_fit(*kv) && kv->size(0) == x.size(0))) &&
-         attention_weights_ok(x, in, w, head_dim);
+         attention_weights_ok(x, in, w, heads, head_dim);
 }
 bool mlp_block_ok(const Tensor& x, const Tensor& scale, const std::vector<Tensor>& w) {
   return x.dim() >= 2 && plain(x) && rows_fit(x) && norm_ok(scale, x) && mlp_weights_ok(x, w);
@@ -491,21 +493,21 @@ bool mlp_grads_ok(const Tensor& x, const std::vector<Tensor>& w, const std::vect
 // y = x + attention(rmsnorm(x)) wo, and what the backward pass needs: (y, h, rstd, q, k, v, o, lse).
 // The keys and values come from `kv` where there is one, else from h.
 std::vector<Tensor> attention_block(const Tensor& x, const optional<Tensor>& kv, const Tensor& scale,
-                                    double eps, const std::vector<Tensor>& weights, int64_t head_dim,
-                                    const optional<Tensor>& rel_bias, const optional<Tensor>& buckets,
-                                    const optional<Tensor>& key_mask, const optional<Tensor>& q_seg,
+                                    double eps, const std::vector<Tensor>& weights, int64_t heads,
+                                    int64_t head_dim, const optional<Tensor>& rel_bias,
+                                    const optional<Tensor>& buckets, const optional<Tensor>& key_mask,
+                                    const optional<Tensor>& q_seg,
                                     const optional<Tensor>& kv_seg, int64_t causal, int64_t causal_off,
                                     int64_t rel_off, bool short_range) {
-  if (!attention_block_ok(x, kv, scale, weights, head_dim))
+  if (!attention_block_ok(x, kv, scale, weights, heads, head_dim))
     throw std::invalid_argument("attention_block: operands are not covered");
   void* st = stream_of();
   auto [h, rstd] = norm_forward(x, scale, eps, st);
   const Tensor& in = kv ? *kv : h;
   const int64_t B = x.size(0), Lq = x.size(1), Lk = in.size(1), d = x.size(-1);
   const Weight wq(weights[0], d), wk(weights[1], in.size(-1)), wv(weights[2], in.size(-1)), wo(weights[3], wq.n);
-  const int64_t H = wq.n / head_dim;
   std::vector<Tensor> out;
-  for (int64_t l : {Lq, Lk, Lk}) out.push_back(at::empty({B, l, H, head_dim}, x.options()));
+  for (int64_t l : {Lq, Lk, Lk}) out.push_back(at::empty({B, l, heads, head_dim}, x.options()));
   if (kv) {
     forward(h, B * Lq, wq, nullptr, out[0], st);
     std::vector<Tensor> pair = {out[1], out[2]};
@@ -513,8 +515,8 @@ std::vector<Tensor> attention_block(const Tensor& x, const optional<Tensor>& kv,
   } else {
     forward_group(h, B * Lq, {wq, wk, wv}, out, st);
   }
-  Tensor o = at::empty({B, Lq, H, head_dim}, x.options());
-  Tensor lse = at::empty({B, H, Lq}, x.options().dtype(at::kFloat));
+  Tensor o = at::empty({B, Lq, heads, head_dim}, x.options());
+  Tensor lse = at::empty({B, heads, Lq}, x.options().dtype(at::kFloat));
   attention_into(out[0], out[1], out[2],
                  {rel_bias, buckets, key_mask, q_seg, kv_seg, causal, causal_off, rel_off}, short_range, o,
                  lse, st);
@@ -536,7 +538,7 @@ std::tuple<Tensor, optional<Tensor>> attention_block_bwd(
                &lse = saved[6];
   const std::vector<optional<Tensor>> g(grads.begin(), grads.end());
   if (!plain(dy) || dy.numel() != x.numel() ||
-      !attention_block_ok(x, kv, scale, weights, q.size(3)) || !attention_grads_ok(x, kv, weights, g))
+      !attention_block_ok(x, kv, scale, weights, q.size(2), q.size(3)) || !attention_grads_ok(x, kv, weights, g))
     throw std::invalid_argument("attention_block_bwd: operands are not covered");
   void* st = stream_of();
   const Tensor& in = kv ? *kv : h;

@@ -80,20 +80,21 @@ def attention(x, kv, norm, attn, norm_cls, attn_cls, dense_cls, *, bias_table=No
     return None
   scale = norm._parameters["scale"]
   weights = [F.compute_weight(p, torch.bfloat16) for p in params]
-  if not host.attention_block_ok(x, kv, scale, weights, attn.head_dim):
+  if not host.attention_block_ok(x, kv, scale, weights, attn.local_heads, attn.head_dim):
     return None
   lq, lk = x.shape[1], (x if kv is None else kv).shape[1]
   masks = attn_ops.prepare(lq, lk, attn.local_heads, x.device, bias_table, bidirectional, num_buckets,
                            max_distance, key_mask, causal, q_segment_ids, kv_segment_ids)
   short = attn_ops.forward_kernel(lq, lk, attn.head_dim, masks[5] == 2) == "classic"
   if not recording:
-    return host.attention_block(x, kv, scale, norm.epsilon, weights, attn.head_dim, *masks, short)[0]
+    return host.attention_block(x, kv, scale, norm.epsilon, weights, attn.local_heads, attn.head_dim, *masks,
+                                short)[0]
   grads = [_usable_grad(p) for p in params]
   if any(g is None for g in grads) or _usable_grad(scale) is None or \
       not host.attention_grads_ok(x, kv, weights, grads):
     return None
-  return _AttentionBlockFn.apply(x, kv, scale, *params, masks[0], norm.epsilon, attn.head_dim, masks[1:],
-                                 short)
+  return _AttentionBlockFn.apply(x, kv, scale, *params, masks[0], norm.epsilon, attn.local_heads,
+                                 attn.head_dim, masks[1:], short)
 
 
 def gated_mlp(x, norm, mlp, norm_cls, mlp_cls, dense_cls) -> Optional[torch.Tensor]:
@@ -151,9 +152,10 @@ class _Buffers:
 class _AttentionBlockFn(torch.autograd.Function):
 
   @staticmethod
-  def forward(ctx, x, kv, scale, wq, wk, wv, wo, rel_bias, eps, head_dim, masks, short):
+  def forward(ctx, x, kv, scale, wq, wk, wv, wo, rel_bias, eps, heads, head_dim, masks, short):
     weights = [F.compute_weight(w, torch.bfloat16) for w in (wq, wk, wv, wo)]
-    y, *saved = native.host().attention_block(x, kv, scale, eps, weights, head_dim, rel_bias, *masks, short)
+    y, *saved = native.host().attention_block(x, kv, scale, eps, weights, heads, head_dim, rel_bias, *masks,
+                                              short)
     ctx.save_for_backward(x, kv, scale, wq, wk, wv, wo, rel_bias, *masks[:4], *saved)
     ctx.modes = masks[4:]
     return y
@@ -178,7 +180,7 @@ class _AttentionBlockFn(torch.autograd.Function):
       if not done:
         F._restore_grad_flags([p for p in params + [scale, rel_bias] if p is not None], flags)
     dw = buf.results()
-    return (dx, dkv, dw[4], *dw[:4], dw[5] if want_bias else None, None, None, None, None)
+    return (dx, dkv, dw[4], *dw[:4], dw[5] if want_bias else None, None, None, None, None, None)
 
 
 class _GatedMlpBlockFn(torch.autograd.Function):

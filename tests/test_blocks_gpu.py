@@ -185,3 +185,27 @@ def test_a_gradient_buffer_that_goes_between_the_passes():
     loss.backward()
     grads.append(wo.main_grad.clone() if not drop else wo.grad.clone())
   assert float((grads[0] - grads[1]).norm() / grads[0].norm()) < 2 ** -8
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("heads", [2, 6])
+@pytest.mark.parametrize("cross", [False, True])
+def test_weights_of_another_head_count_are_refused(cross, heads, grad):
+  """Weights of 2 or 6 heads in the place of a layer's 4: the bias table was checked for 4."""
+  from torch.func import functional_call
+  model, other = _model(heads=4), _model(heads=heads)
+  if cross:
+    layer, prefix = model.decoder.layers_0, "encoder_decoder_attention."
+  else:
+    layer, prefix = model.encoder.layers_0, "attention."
+  source = other.decoder.layers_0 if cross else other.encoder.layers_0
+  swapped = {n: p for n, p in source.named_parameters() if n.startswith(prefix)}
+  x = torch.randn(2, 9, 256, device="cuda").bfloat16()
+  table = (model.decoder if cross else model.encoder).relpos_bias.rel_embedding
+  kw = dict(bias_table=table, decoder_key_mask=None, encoder_key_mask=None) if cross else \
+      dict(bias_table=table, key_mask=None)
+  args = (x, x) if cross else (x,)
+  with torch.set_grad_enabled(grad):
+    layer(*args, **kw)
+    with pytest.raises(RuntimeError, match="shape"):
+      functional_call(layer, swapped, args, kw)
