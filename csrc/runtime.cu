@@ -108,10 +108,19 @@ const CUtensorMap* get_tensor_map(const void* base, int elem_bytes, int rank, co
                            : elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                              : CU_TENSOR_MAP_DATA_TYPE_UINT8;
   CUtensorMap* m = new CUtensorMap;
-  CUresult r = enc(m, dt, rank, const_cast<void*>(base), gdims, gstr, gbox, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   swizzle_128b ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return enc(m, dt, rank, const_cast<void*>(base), gdims, gstr, gbox, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE,
+               swizzle_128b ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // A thread whose first call this is (autograd's, in a first backward pass) has a current device
+    // but not its context yet; the runtime binds it here.
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
+  }
   if (r != CUDA_SUCCESS) {
     delete m;
     set_error("cuTensorMapEncodeTiled failed with %d (rank %d, dims %llu x %llu, box %u x %u)",
