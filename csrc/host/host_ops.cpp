@@ -151,6 +151,12 @@ void weight_grad_group(const Tensor& x, const std::vector<const void*>& dy,
         "gemm_shared");
 }
 
+// Whether two contiguous tensors share memory.
+bool overlap(const Tensor& a, const Tensor& b) {
+  const char *pa = static_cast<const char*>(a.data_ptr()), *pb = static_cast<const char*>(b.data_ptr());
+  return pa < pb + b.nbytes() && pb < pa + a.nbytes();
+}
+
 // The gradients of x @ w_i, i < n: into `dx` (if wanted) and `grads` (if wanted).
 void backward_products(const Tensor& x, int64_t m, const std::vector<const void*>& dy,
                        const std::vector<long long>& ld_dy, const std::vector<Weight>& w,
@@ -162,9 +168,14 @@ void backward_products(const Tensor& x, int64_t m, const std::vector<const void*
   else if (dx)
     for (size_t i = 0; i < w.size(); ++i) input_grad(dy[i], ld_dy[i], m, w[i], *dx, i > 0, st);
   if (grads.empty()) return;
-  bool same = true;
-  for (size_t i = 0; i < w.size(); ++i) same = same && accumulate[i] == accumulate[0];
-  if (one_launch && same) {
+  // One launch writes its outputs side by side: a weight that stands in for two (tied projections) has
+  // one gradient buffer, to which the products have to be added one after the other.
+  bool apart = true;
+  for (size_t i = 0; i < w.size(); ++i) {
+    apart = apart && accumulate[i] == accumulate[0];
+    for (size_t j = 0; j < i; ++j) apart = apart && !overlap(grads[i], grads[j]);
+  }
+  if (one_launch && apart) {
     weight_grad_group(x, dy, ld_dy, m, w, grads, accumulate[0], st);
   } else {
     for (size_t i = 0; i < w.size(); ++i) {

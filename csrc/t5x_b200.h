@@ -84,8 +84,8 @@ int t5x_gemm_wgrad_bf16(const void* A, const void* B, void* C, int M, int N, int
                         int b_mn_major, int accumulate, int last_wave_pieces, void* stream);
 
 /* Up to three products in one launch. shared: C_i[M, widths[i]] = A[M, K] @ B_i (bf16 C_i, or fp32
- * weight gradients (+)= with out_fp32). sum: C[M, N] (bf16) = sum of A_i[M, widths[i]] @ B_i, in one
- * fp32 accumulator. */
+ * weight gradients (+)= with out_fp32), the C_i apart in memory: they are written side by side. sum:
+ * C[M, N] (bf16) = sum of A_i[M, widths[i]] @ B_i, in one fp32 accumulator. */
 int t5x_gemm_shared_bf16(const void* A, const void* const* B, void* const* C, const int* widths, int n,
                          int M, int K, long long lda, const long long* ldb, const long long* ldc,
                          int a_mn_major, int b_mn_major, int out_fp32, int accumulate,
