@@ -416,8 +416,12 @@ __device__ __forceinline__ float warp_max(float v) {
 // A kernel that becomes resident early may find lines of its inputs in the SM's L1 that an older
 // kernel read before the memory was written anew (buffers are reused along a chain), and nothing
 // drops them when the wait returns. What earlier kernels of a chain write is therefore read through
-// L2 (`ld_chained`, TMA), never through L1 or the read-only path. A kernel launched the ordinary
-// way ends a chain: what it and the kernels before it wrote may be read either way.
+// L2 (`ld_chained`, TMA), never through L1 or the read-only path.
+// A chain starts with a kernel launched the ordinary way: it runs when everything before it on the
+// stream has completed, so the kernels of the chain may read what came before it either way, and ahead
+// of their wait. A programmatic dependent does not start a chain, even behind an ordinary kernel: it
+// may run before that kernel's last writes are visible, and with it all that are chained to it.
+
 // Nanosecond timer shared by all SMs (for the optional per-CTA phase trace of the GEMM).
 __device__ __forceinline__ long long global_timer_ns() {
   long long t;

@@ -82,8 +82,8 @@ __global__ void __launch_bounds__(kDecWarps * 32)
   // With few (row, head) items the kernel is a chain of dependent loads, so with kFirst = 8 the
   // history is requested ahead of the wait for the preceding kernel: the position, the slots of the
   // first 32 positions, then the keys AND values of those positions. They come from before this
-  // chain of launches (earlier steps; the beam kernels, which are launched the ordinary way); q / k
-  // / v and the bias come from it. Later positions are streamed below, and with kFirst = 0 all are.
+  // chain of launches, which decode_begin starts; q / k / v and the bias come from it. Later
+  // positions are streamed below, and with kFirst = 0 all are.
   constexpr int kU = 4;  // positions in flight per lane group in the streams
   constexpr int kHeld = kFirst > 0 ? kFirst : 1;
   int slot[kHeld];
@@ -244,7 +244,9 @@ __global__ void __launch_bounds__(kDecWarps * 32)
 // current position and lays out the T5 bias of that position, bias_row[h][t] =
 // table[h][bucket_of_distance[cur - t]] for t <= cur (bucket 0 beyond it, as for any key not
 // before its query). One block per row, then one per head. As tensor operations this was some
-// sixteen launches of 2 us each per step.
+// sixteen launches of 2 us each per step. It is launched the ordinary way, so that a step starts a
+// chain of its own: what earlier steps and the beam kernels wrote (position, ancestry, caches) is
+// complete and visible before any kernel of the step runs, and those may read it ahead of their wait.
 constexpr int kBeginThreads = 128;
 __global__ void __launch_bounds__(kBeginThreads)
     decode_begin_kernel(const long long* __restrict__ live_seqs,  // [rows, L]
@@ -253,7 +255,6 @@ __global__ void __launch_bounds__(kBeginThreads)
                         const int* __restrict__ bucket_of_distance, float* __restrict__ bias_row,
                         int rows, int L, int d, int vocab, int num_buckets) {
   chain_release();
-  chain_wait();
   const int cur = min(max(*cur_index, 0), L - 1);
   if (static_cast<int>(blockIdx.x) < rows) {
     const int row = blockIdx.x;
@@ -495,15 +496,13 @@ T5X_API int t5x_decode_begin(const void* live_seqs, const void* cur_index, const
   if (rows <= 0 || L <= 0) return 0;
   if (d % 8 || ((reinterpret_cast<uintptr_t>(emb) | reinterpret_cast<uintptr_t>(x)) & 15))
     return set_error("decode_begin: embedding rows must be 16-byte aligned (d=%d)", d);
-  cudaError_t e = launch_chained(
-      decode_begin_kernel, dim3(rows + H), dim3(kBeginThreads), 0,
-      static_cast<cudaStream_t>(stream), static_cast<const long long*>(live_seqs),
-      static_cast<const int*>(cur_index), static_cast<const __nv_bfloat16*>(emb),
-      static_cast<__nv_bfloat16*>(x), static_cast<const float*>(table),
-      static_cast<const int*>(bucket_of_distance), static_cast<float*>(bias_row), rows, L, d, vocab,
-      num_buckets);
+  decode_begin_kernel<<<rows + H, kBeginThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const long long*>(live_seqs), static_cast<const int*>(cur_index),
+      static_cast<const __nv_bfloat16*>(emb), static_cast<__nv_bfloat16*>(x),
+      static_cast<const float*>(table), static_cast<const int*>(bucket_of_distance),
+      static_cast<float*>(bias_row), rows, L, d, vocab, num_buckets);
   count_launches(1);
-  if (e == cudaSuccess) e = cudaGetLastError();
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("decode_begin: %s", cudaGetErrorString(e));
   return 0;
 }

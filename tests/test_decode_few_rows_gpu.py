@@ -40,6 +40,33 @@ def test_a_sentence_does_not_depend_on_its_batch(emb, heads, mlp, few):
   assert torch.equal(steps[0], steps[1])
 
 
+@pytest.mark.parametrize("batch,beams", [(1, 1), (5, 1), (7, 2), (16, 4)])
+def test_steps_launched_one_by_one(batch, beams):
+  """Without a captured graph a step follows the search's kernels on the stream: its first kernel starts a
+  chain of its own, so that no kernel of the step reads the position, the ancestry or the caches before
+  they are written. Chained and not, the search is the same bit by bit, whenever it is run."""
+  from t5x_b200 import decoding_fast
+  from t5x_b200.models.t5 import network
+  from t5x_b200.ops import native
+  torch.manual_seed(batch)
+  cfg = network.T5Config(vocab_size=512, dtype="bfloat16", emb_dim=256, num_heads=4, head_dim=64,
+                         num_encoder_layers=1, num_decoder_layers=2, mlp_dim=512,
+                         mlp_activations=("gelu", "linear"), dropout_rate=0.0)
+  module = network.Transformer(cfg, device="cuda")
+  for p in module.parameters():
+    p.bf16 = (p.detach() * (20 if p.dim() == 2 and p.shape[1] == 512 else 1)).bfloat16()
+  enc = torch.randint(2, 512, (batch, 23), device="cuda")
+  plain = decoding_fast.GraphBeamDecoder(module, batch, beams, 40, 1, use_graph=False)
+  plain.chain_level = 0
+  want = plain.decode(enc)
+  chained = decoding_fast.GraphBeamDecoder(module, batch, beams, 40, 1, use_graph=False)
+  assert chained.chain_level == 2
+  for _ in range(4):
+    got = chained.decode(enc)
+    native.check_status()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
 @pytest.mark.parametrize("b,lk,h", [(1, 1, 1), (2, 31, 3), (3, 33, 2), (2, 64, 4), (1, 129, 2)])
 def test_cross_layout(b, lk, h):
   """A rearrangement: equal to the tensor-op statement bit by bit, the padding zero."""
