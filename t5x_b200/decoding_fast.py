@@ -270,7 +270,8 @@ FEW_ROWS = 64  # up to so many rows the products of a step go through `native.ge
 
 
 class _Layer:
-  """The bf16 weights of one decoder layer, the module's own (an update of the module shows)."""
+  """The bf16 weights of one decoder layer, the module's own: an update in place shows by itself, tensors
+  put in their place are noticed by `GraphBeamDecoder._weights_moved`."""
 
   def __init__(self, layer):
     w = lambda dense: dense.kernel.bf16
@@ -283,6 +284,28 @@ class _Layer:
     self.ln1 = layer.pre_self_attention_layer_norm.scale
     self.ln2 = layer.pre_cross_attention_layer_norm.scale
     self.ln3 = layer.pre_mlp_layer_norm.scale
+
+
+_PROJECTIONS = (("self_attention", ("query", "key", "value", "out")),
+                ("encoder_decoder_attention", ("query", "key", "value", "out")),
+                ("mlp", ("wi_0", "wi_1", "wo")))
+_NORMS = ("pre_self_attention_layer_norm", "pre_cross_attention_layer_norm", "pre_mlp_layer_norm")
+
+
+def _weights_in_use(module) -> List[torch.Tensor]:
+  """Every tensor of `module` that a decoder reads, as the module holds it now. Straight through the
+  modules' dictionaries, since it is asked for ahead of every search (12 layers: 40 us)."""
+  dec = module._modules["decoder"]
+  held = [module._modules["token_embedder"]._parameters["embedding"].bf16,
+          dec.logits_weight_and_scale()[0].bf16, dec._modules["decoder_norm"]._parameters["scale"],
+          dec._modules["relpos_bias"]._parameters["rel_embedding"]]
+  for i in range(module.config.num_decoder_layers):
+    parts = dec._modules[f"layers_{i}"]._modules
+    for block, names in _PROJECTIONS:
+      inner = parts[block]._modules
+      held += [inner[n]._parameters["kernel"].bf16 for n in names]
+    held += [parts[n]._parameters["scale"] for n in _NORMS]
+  return held
 
 
 class GraphBeamDecoder:
@@ -319,23 +342,11 @@ class GraphBeamDecoder:
     self.use_graph = use_graph
     dev = module.token_embedder.embedding.device
     self.dev = dev
-    dec = module.decoder
-    self.layers = [_Layer(getattr(dec, f"layers_{i}")) for i in range(c.num_decoder_layers)]
-    self.emb = module.token_embedder.embedding.bf16
+    self._bind_weights()
     self.link: Optional[_TensorParallelLink] = None
     if self.tp > 1:
-      import torch.distributed as dist
-      # token lookups need the whole (vocabulary-sharded) table: gathered once, 2 bytes a weight
-      parts = [torch.empty_like(self.emb) for _ in range(self.tp)]
-      dist.all_gather(parts, self.emb.contiguous(), group=st.model_group)
-      self.emb = torch.cat(parts, dim=0)
       self.link = _TensorParallelLink(st.model_group, self.rows, c.emb_dim,
                                       3 * c.num_decoder_layers, c.vocab_size, dev)
-    self.final_ln = dec.decoder_norm.scale
-    w, self.logit_scale = dec.logits_weight_and_scale()
-    wl = w.bf16
-    self.w_logits = wl if wl.shape[0] == c.emb_dim else wl.t()
-    self.rel_table = dec.relpos_bias.rel_embedding
     bf = dict(dtype=torch.bfloat16, device=dev)
     # [batch, beam slot, head, position, dim]: one (slot, head) history is contiguous. For the
     # tensor-core kernel the cache is padded to a multiple of 32 positions and the values are
@@ -378,6 +389,38 @@ class GraphBeamDecoder:
     self._beam_scratch = None
 
   # ------------------------------------------------------------------------------------------
+  def _bind_weights(self) -> None:
+    """Takes the weights as the module holds them now; the captured step read the ones before."""
+    dec = self.module.decoder
+    self.layers = [_Layer(getattr(dec, f"layers_{i}")) for i in range(self.c.num_decoder_layers)]
+    self.emb = self._token_table()
+    self.final_ln = dec.decoder_norm.scale
+    w, self.logit_scale = dec.logits_weight_and_scale()
+    wl = w.bf16
+    self.w_logits = wl if wl.shape[0] == self.c.emb_dim else wl.t()
+    self.rel_table = dec.relpos_bias.rel_embedding
+    self._held = [(t, t.data_ptr()) for t in _weights_in_use(self.module)]
+    self.graph = None
+
+  def _token_table(self) -> torch.Tensor:
+    """The embedding of every token: the module's own, or, with the vocabulary sharded over the model
+    axis, gathered from its ranks (2 bytes a weight)."""
+    shard = self.module.token_embedder.embedding.bf16
+    if self.tp == 1:
+      return shard
+    import torch.distributed as dist
+    from t5x_b200.parallel import state as pstate
+    parts = [torch.empty_like(shard) for _ in range(self.tp)]
+    dist.all_gather(parts, shard.contiguous(), group=pstate.get().model_group)
+    return torch.cat(parts, dim=0)
+
+  def _weights_moved(self) -> bool:
+    """Whether the module holds other tensors than those taken, or the same at another place (a working
+    copy that was made anew, fused with its neighbours or gathered from other ranks)."""
+    now = _weights_in_use(self.module)
+    return len(now) != len(self._held) or any(
+        t is not held or t.data_ptr() != at for t, (held, at) in zip(now, self._held))
+
   def _reset(self):
     self.cur.zero_()
     self.live_seqs.zero_()
@@ -592,6 +635,8 @@ class GraphBeamDecoder:
     """-> ([batch, beams, max_decode_len] sequences, [batch, beams] scores), ascending."""
     assert encoder_input_tokens.shape[0] == self.b
     with torch.no_grad():
+      if self._weights_moved():
+        self._bind_weights()
       if self.graph is not None and encoder_input_tokens.shape[1] != self._graph_enc_len:
         self.graph = None  # the captured step has the encoder length in its arguments
       self._encode(encoder_input_tokens)

@@ -112,3 +112,48 @@ def test_a_captured_step_reads_the_weights_as_they_are(batch):
   seqs, scores = old.decode(enc)
   want_seqs, want = make().decode(enc)
   assert torch.equal(seqs, want_seqs) and torch.equal(scores, want) and not torch.equal(scores, before)
+
+
+@pytest.mark.parametrize("batch", [2, 70])
+@pytest.mark.parametrize("what", ["fused", "logits", "embedding", "norm", "parameter", "data"])
+def test_weights_put_in_the_place_of_others(what, batch):
+  """Working copies that are made anew between two searches (q/k/v moved side by side, a copy gathered from
+  other ranks), or parameters and norms replaced: the next search reads them, as a new decoder does."""
+  from t5x_b200 import decoding_fast
+  from t5x_b200.models.t5 import network
+  torch.manual_seed(batch)
+  cfg = network.T5Config(vocab_size=256, dtype="bfloat16", emb_dim=128, num_heads=2, head_dim=64,
+                         num_encoder_layers=1, num_decoder_layers=2, mlp_dim=256,
+                         mlp_activations=("gelu", "linear"), dropout_rate=0.0)
+  module = network.Transformer(cfg, device="cuda")
+  for p in module.parameters():
+    p.bf16 = p.detach().bfloat16()
+  enc = torch.randint(2, 256, (batch, 19), device="cuda")
+  make = lambda: decoding_fast.GraphBeamDecoder(module, batch, 2, 8, 1)
+  old = make()
+  before = old.decode(enc)[1]
+  assert not old._weights_moved()
+  graph = old.graph
+  assert torch.equal(old.decode(enc)[1], before) and old.graph is graph
+  layer = module.decoder.layers_1
+  if what == "fused":
+    attn = layer.self_attention
+    wide = torch.cat([m.kernel.bf16 for m in (attn.query, attn.key, attn.value)], dim=1)
+    for i, m in enumerate((attn.query, attn.key, attn.value)):
+      m.kernel.bf16 = wide[:, 128 * i:128 * (i + 1)]
+    wide.mul_(1.5)  # (the optimizer writes the new copies)
+  elif what == "logits":
+    module.decoder.logits_dense.kernel.bf16 = module.decoder.logits_dense.kernel.bf16 * 2
+  elif what == "embedding":
+    module.token_embedder.embedding.bf16 = module.token_embedder.embedding.bf16 * 2
+  elif what == "norm":
+    module.decoder.decoder_norm.scale = torch.nn.Parameter(module.decoder.decoder_norm.scale.detach() * 2)
+  elif what == "parameter":
+    new = torch.nn.Parameter(layer.mlp.wo.kernel.detach() * 2)
+    new.bf16 = new.detach().bfloat16()
+    layer.mlp.wo.kernel = new
+  else:
+    layer.mlp.wi_0.kernel.bf16.data = layer.mlp.wi_0.kernel.bf16 * 2
+  seqs, scores = old.decode(enc)
+  want_seqs, want = make().decode(enc)
+  assert torch.equal(seqs, want_seqs) and torch.equal(scores, want) and not torch.equal(scores, before)
