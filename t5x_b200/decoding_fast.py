@@ -404,15 +404,18 @@ class GraphBeamDecoder:
 
   def _token_table(self) -> torch.Tensor:
     """The embedding of every token: the module's own, or, with the vocabulary sharded over the model
-    axis, gathered from its ranks (2 bytes a weight)."""
+    axis, a buffer for all of it (see `_gather_token_table`)."""
     shard = self.module.token_embedder.embedding.bf16
-    if self.tp == 1:
-      return shard
+    return shard if self.tp == 1 else shard.new_empty(self.tp * shard.shape[0], *shard.shape[1:])
+
+  def _gather_token_table(self) -> None:
+    """Collects the table from the ranks of the model axis (2 bytes a weight), ahead of every search: an
+    update of the module changes the shards, not what was gathered from them. In place: the captured
+    step reads it by its address."""
     import torch.distributed as dist
     from t5x_b200.parallel import state as pstate
-    parts = [torch.empty_like(shard) for _ in range(self.tp)]
-    dist.all_gather(parts, shard.contiguous(), group=pstate.get().model_group)
-    return torch.cat(parts, dim=0)
+    shard = self.module.token_embedder.embedding.bf16.contiguous()
+    dist.all_gather(list(self.emb.chunk(self.tp)), shard, group=pstate.get().model_group)
 
   def _weights_moved(self) -> bool:
     """Whether the module holds other tensors than those taken, or the same at another place (a working
@@ -637,6 +640,8 @@ class GraphBeamDecoder:
     with torch.no_grad():
       if self._weights_moved():
         self._bind_weights()
+      if self.tp > 1:
+        self._gather_token_table()
       if self.graph is not None and encoder_input_tokens.shape[1] != self._graph_enc_len:
         self.graph = None  # the captured step has the encoder length in its arguments
       self._encode(encoder_input_tokens)

@@ -181,3 +181,31 @@ def test_partial_gradients_of_row_sharded_norms_are_summed_over_the_model_axis(t
     assert g["n1"].tolist() == [3.0] * 4              # 1 + 2
     assert g["n2"].tolist() == [0.0, 3.0, 6.0]
     assert g["w"].tolist() == [5.0, 5.0]              # untouched
+
+
+def _token_table_worker(rank, world, port):
+  sys.path.insert(0, ROOT)
+  os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port), RANK=str(rank),
+                    WORLD_SIZE=str(world))
+  dist.init_process_group("gloo", rank=rank, world_size=world)
+  from types import SimpleNamespace
+  from t5x_b200 import decoding_fast
+  from t5x_b200.parallel import state as pstate
+  pstate.setup_mesh(model_size=world, device=torch.device("cpu"))
+  shard = SimpleNamespace(bf16=torch.zeros(5, 8, dtype=torch.bfloat16))
+  d = object.__new__(decoding_fast.GraphBeamDecoder)
+  d.module, d.tp = SimpleNamespace(token_embedder=SimpleNamespace(embedding=shard)), world
+  d.emb = d._token_table()
+  at = d.emb.data_ptr()
+  for step in range(3):  # the optimizer writes the shards between two searches
+    shard.bf16.copy_(torch.arange(40).view(5, 8) + 100 * step + 40 * rank)
+    d._gather_token_table()
+    want = torch.cat([torch.arange(40).view(5, 8) + 100 * step + 40 * r for r in range(world)])
+    assert torch.equal(d.emb, want.bfloat16()) and d.emb.data_ptr() == at
+  dist.barrier()
+  dist.destroy_process_group()
+
+
+def test_decoder_reads_the_present_token_table_under_a_model_axis():
+  """Gathered from the ranks ahead of every search, into the buffer that the captured step reads."""
+  mp.spawn(_token_table_worker, args=(2, _free_port()), nprocs=2, join=True)
