@@ -45,8 +45,12 @@ __device__ __forceinline__ float sum_over_row_groups(float x) {  // the 4 row gr
   return x;
 }
 
-// kFirst: positions per lane group whose key and value are held in registers (see below).
-template <int kFirst>
+// kFirst: positions per lane group whose key and value are held in registers (see below). kChained:
+// inside a chain of launches, where the inputs come from kernels that may still be running; by itself
+// otherwise, where everything is read at once and through L1. (One body with the choice at run time
+// cost the form by itself 7 %: us, one body / two, 256 rows x 32 heads at position 64 of 129 49.2 / 45.9,
+// at 127 79.9 / 73.7, 64 x 32 at 100 30.7 / 28.7; beam search of XL, 24 layers, 128 steps 589 / 579 ms.)
+template <int kFirst, bool kChained>
 __global__ void __launch_bounds__(kDecWarps * 32)
     decode_self_attention_kernel(const __nv_bfloat16* __restrict__ q,      // [rows, H, 64]
                                  const __nv_bfloat16* __restrict__ k_new,  // [rows, H, 64]
@@ -58,13 +62,13 @@ __global__ void __launch_bounds__(kDecWarps * 32)
                                  const int* __restrict__ cur_index,    // device scalar
                                  __nv_bfloat16* __restrict__ out,      // [rows, H, 64]
                                  long long in_ld,  // row stride of q / k_new / v_new (elements)
-                                 int rows, int beams, int H, int L, int chained) {
+                                 int rows, int beams, int H, int L) {
   __shared__ float sprob[kDecWarps][kDecMaxLen];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int item = blockIdx.x * kDecWarps + warp;  // (row, head)
-  chain_release();
+  if (kChained) chain_release();
   if (item >= rows * H) {
-    chain_wait();
+    if (kChained) chain_wait();
     return;
   }
   const int row = item / H, h = item - row * H;
@@ -79,13 +83,22 @@ __global__ void __launch_bounds__(kDecWarps * 32)
                                static_cast<long long>(h) * L * kDecHeadDim;
   const int* anc = ancestry + static_cast<long long>(row) * L;
 
-  // With few (row, head) items the kernel is a chain of dependent loads, so with kFirst = 8 the
-  // history is requested ahead of the wait for the preceding kernel: the position, the slots of the
-  // first 32 positions, then the keys AND values of those positions. They come from before this
-  // chain of launches, which decode_begin starts; q / k / v and the bias come from it. Later
-  // positions are streamed below, and with kFirst = 0 all are.
+  // With few (row, head) items the kernel is a chain of dependent loads, so with kFirst = 8 it is kept
+  // to two links: the position, the slots of the first 32 positions and (not chained) this step's
+  // vectors together, then the keys AND values of those positions. Chained, both links come ahead of
+  // the wait for the preceding kernel: the history is from before this chain of launches, which
+  // decode_begin starts; q / k / v and the bias come from it. Later positions are streamed below, and
+  // with kFirst = 0 all are.
   constexpr int kU = 4;  // positions in flight per lane group in the streams
   constexpr int kHeld = kFirst > 0 ? kFirst : 1;
+  auto input = [&](const __nv_bfloat16* x) {  // 8 dims per lane
+    const uint4* at = reinterpret_cast<const uint4*>(x + rh) + part;
+    return kChained ? ld_chained(at) : *at;
+  };
+  auto bias_at = [&](int t) {  // (by itself the lines stay in L1 for the many rows of a head)
+    const float* at = bias_row + static_cast<long long>(h) * L + t;
+    return kChained ? ld_chained(at) : *at;
+  };
   int slot[kHeld];
 #pragma unroll
   for (int u = 0; u < kFirst; ++u) {
@@ -93,32 +106,39 @@ __global__ void __launch_bounds__(kDecWarps * 32)
     slot[u] = t < L ? anc[t] : 0;
   }
   const int cur = min(max(*cur_index, 0), L - 1);
+  // 1. this step's query / key / value; append key / value at position `cur` of the row's own slot
+  uint4 qu, kn, vn;
+  if (!kChained) qu = input(q), kn = input(k_new), vn = input(v_new);
   uint4 kf4[kHeld], vf4[kHeld];
   float bf[kHeld];
 #pragma unroll
   for (int u = 0; u < kFirst; ++u) {
     const int t = u * 4 + g;
+    if (!kChained) {
+      kf4[u] = kn;
+      vf4[u] = vn;
+      bf[u] = 0.f;
+    }
     if (t < cur) {
       const long long at = batch_base + slot[u] * slot_stride + t * tstride;
       kf4[u] = reinterpret_cast<const uint4*>(cache_k + at)[part];
       vf4[u] = reinterpret_cast<const uint4*>(cache_v + at)[part];
     }
+    if (!kChained && bias_row != nullptr && t <= cur) bf[u] = bias_at(t);
   }
-  chain_wait();
-  // 1. this step's query / key / value (8 dims per lane); append key / value at position
-  //    `cur` of the row's own slot
-  const uint4 qu = ld_chained(reinterpret_cast<const uint4*>(q + rh) + part);
-  const uint4 kn = ld_chained(reinterpret_cast<const uint4*>(k_new + rh) + part);
-  const uint4 vn = ld_chained(reinterpret_cast<const uint4*>(v_new + rh) + part);
+  if (kChained) {
+    chain_wait();
+    qu = input(q), kn = input(k_new), vn = input(v_new);
 #pragma unroll
-  for (int u = 0; u < kFirst; ++u) {
-    const int t = u * 4 + g;
-    if (t >= cur) {
-      kf4[u] = kn;
-      vf4[u] = vn;
+    for (int u = 0; u < kFirst; ++u) {
+      const int t = u * 4 + g;
+      if (t >= cur) {
+        kf4[u] = kn;
+        vf4[u] = vn;
+      }
+      bf[u] = 0.f;
+      if (bias_row != nullptr && t <= cur) bf[u] = bias_at(t);
     }
-    bf[u] = 0.f;
-    if (bias_row != nullptr && t <= cur) bf[u] = ld_chained(bias_row + static_cast<long long>(h) * L + t);
   }
   if (g == 0) {
     const long long dst = batch_base + (row - b * beams) * slot_stride + cur * tstride;
@@ -136,12 +156,6 @@ __global__ void __launch_bounds__(kDecWarps * 32)
     return sum_over_row_lanes(s);
   };
 
-  // The bias comes from this chain of launches, if there is one; else its lines stay in L1 for the many
-  // rows of a head (256 rows x 32 heads, 64 steps: 25.3 us through L2, 23.2 so).
-  auto bias_at = [&](int t) {
-    const float* at = bias_row + static_cast<long long>(h) * L + t;
-    return chained ? ld_chained(at) : *at;
-  };
   // 2. scores over positions 0..cur (no 1/sqrt(d): T5 folds it into the query init)
   float mx = -INFINITY;
 #pragma unroll
@@ -524,10 +538,12 @@ T5X_API int t5x_decode_self_attention(const void* q, const void* k_new, const vo
   if (in_ld % 8) return set_error("decode_self_attention: input row stride must be a multiple of 8");
   const int items = rows * heads;
   // Up to 16 warps an SM the loads' latency counts, beyond that the warps hide it and the 118
-  // registers of the wide form cost occupancy. us, wide / narrow: 4 rows x 12 heads at position 40
-  // 5.5 / 7.2, 64 x 32 10.4 / 12.2, 256 rows x 32 heads over 64 steps 28.2 / 22.5.
-  auto kernel = items <= 16 * num_sms() ? decode_self_attention_kernel<8>
-                                        : decode_self_attention_kernel<0>;
+  // registers of the wide form (128 in a chain) cost occupancy. us, wide / narrow: 4 rows x 12 heads at
+  // position 40 5.5 / 7.2, 64 x 32 10.4 / 12.2, 256 rows x 32 heads over 64 steps 28.2 / 22.5.
+  const bool wide = items <= 16 * num_sms();
+  auto kernel = chained_launches()
+                    ? (wide ? decode_self_attention_kernel<8, true> : decode_self_attention_kernel<0, true>)
+                    : (wide ? decode_self_attention_kernel<8, false> : decode_self_attention_kernel<0, false>);
   cudaError_t e = launch_chained(
       kernel, dim3((items + kDecWarps - 1) / kDecWarps), dim3(kDecWarps * 32),
       0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(q),
@@ -535,7 +551,7 @@ T5X_API int t5x_decode_self_attention(const void* q, const void* k_new, const vo
       static_cast<__nv_bfloat16*>(cache_k), static_cast<__nv_bfloat16*>(cache_v),
       static_cast<const int*>(ancestry), static_cast<const float*>(bias_row),
       static_cast<const int*>(cur_index), static_cast<__nv_bfloat16*>(out), in_ld, rows, beams,
-      heads, max_len, chained_launches() ? 1 : 0);
+      heads, max_len);
   count_launches(1);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("decode_self_attention: %s", cudaGetErrorString(e));

@@ -67,6 +67,41 @@ def test_steps_launched_one_by_one(batch, beams):
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
+@pytest.mark.parametrize("rows,beams,heads", [(1, 1, 1), (6, 2, 5), (64, 4, 37), (64, 4, 38), (80, 1, 32)])
+def test_self_attention_in_a_chain_and_by_itself(rows, beams, heads):
+  """The wide and the narrow form (more than 16 items an SM), each in a chain of launches and by itself: the
+  same sums in the same order, against float64 too (probabilities in fp32, one rounding to bf16)."""
+  from t5x_b200 import decoding_fast
+  from t5x_b200.ops import native
+  g = torch.Generator(device="cuda").manual_seed(rows + heads)
+  n = 67
+  rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+  qkv = rnd(rows, 3, heads, 64).bfloat16()
+  history = [rnd(rows // beams, beams, heads, n, 64).bfloat16() for _ in range(2)]
+  anc = torch.randint(0, beams, (rows // beams, beams, n), device="cuda", generator=g, dtype=torch.int32)
+  bias = rnd(heads, n)
+  for cur in (0, 3, 4, 31, 32, 33, 66):
+    at = torch.tensor([cur], dtype=torch.int32, device="cuda")
+    results = []
+    for level in (0, 2):
+      ck, cv = (t.clone() for t in history)
+      out = torch.empty(rows, heads, 64, dtype=torch.bfloat16, device="cuda")
+      torch.cuda.synchronize()  # (a chain starts where all before it has completed)
+      with native.chained_launches(level):
+        decoding_fast.decode_self_attention(qkv[:, 0], qkv[:, 1], qkv[:, 2], ck, cv, anc, bias, at, out, beams)
+      results.append((out, ck, cv))
+    for a, b in zip(*results):
+      assert torch.equal(a, b)
+    out, ck, cv = (t.double() for t in results[0])
+    slot = anc.long().clone()
+    slot[:, :, cur] = torch.arange(beams, device="cuda")  # the new key and value lie in the row's own slot
+    pick = lambda c: c.transpose(2, 3).gather(1, slot[..., None, None].expand(-1, -1, -1, heads, 64))
+    k, v = (pick(c)[:, :, :cur + 1].flatten(0, 1) for c in (ck, cv))
+    s = torch.einsum("rhd,rthd->rht", qkv[:, 0].double(), k) + bias[:, :cur + 1].double()
+    want = torch.einsum("rht,rthd->rhd", torch.softmax(s, -1), v)
+    assert float((out - want).norm() / want.norm()) < 2.0 ** -8
+
+
 @pytest.mark.parametrize("b,lk,h", [(1, 1, 1), (2, 31, 3), (3, 33, 2), (2, 64, 4), (1, 129, 2)])
 def test_cross_layout(b, lk, h):
   """A rearrangement: equal to the tensor-op statement bit by bit, the padding zero."""
