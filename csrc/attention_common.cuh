@@ -51,25 +51,32 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&p);
 }
 
-// Key blocks that the streaming forward kernel walks: up to the last visible key where nothing but a
-// key mask hides keys. The blocks behind it (the padding of a batch) would contribute exact zeros (the
-// scores of visible keys being far above the -1e10 of hidden ones),
-// unless no key at all is visible: then all count, the rows are uniform over all keys. `find` leaves
-// each warp's findings in `words`; a __syncthreads later `visible_key_blocks` gives the number.
-// (Keys of which 60 to 100 % are visible, us before / so: 16 x 6 heads x 1024 x 1024 181 / 165, 8 x 32 x
-// 1024 x 1024 of 128 features 656 / 566. The short-range kernel walks all of its four blocks: with a
-// number of blocks known only then it lost 8 % where none is hidden and gained 1 % where some are.)
-__device__ __forceinline__ bool key_mask_alone(const AttnParams& p) {
+// Key blocks that the streaming forward kernel walks. Blocks that a mask hides whole from all of a
+// tile's queries would contribute exact zeros (the scores of visible keys being far above the -1e10 of
+// hidden ones), unless a query sees no key at all: its row is uniform over all keys, and all count.
+//   kLookMask    Nothing but a key mask hides keys (the padding of a batch): up to the last visible key.
+//                us before / so: 60 to 100 % of the keys visible, 16 x 6 heads x 1024 x 1024 162 / 146, 8 x
+//                32 x 1024 x 1024 of 128 features 643 / 562; all visible 162 / 163.5, 643 / 643.
+//   kLookCausal  A causal or prefix-LM mask of self-attention with a key mask or segments: up to a tile's
+//                last query (and the last prefix key, if the tile has queries inside the prefix), as long
+//                as each of its queries sees itself. To look that up costs a CTA some 3 us, so only from
+//                more than kAheadKeys keys on (prefix LM, 16 x 12 heads x 1024, 600 tokens in the prefix,
+//                375 / 303; causal with a key mask, 8 x 32 heads of 128 x 1024 655 / 472; but without
+//                that bound 8 x 32 x 256 72 / 77).
+//   kLookNone    Everything else, in a variant of its own: the look-up at run time cost it 2 to 5 % (8 x 32
+//                heads of 128 x 256, causal, 61.4 / 64.3).
+// (The short-range kernel walks all of its four blocks: with a number of blocks known only then it lost
+// 8 % where none is hidden and gained 1 % where some are.)
+enum KeyLook : int { kLookNone = 0, kLookMask = 1, kLookCausal = 2 };
+__host__ __device__ __forceinline__ bool key_mask_alone(const AttnParams& p) {
   return p.key_mask != nullptr && !p.causal && p.kv_seg == nullptr;
 }
-// Under a causal or prefix-LM mask of self-attention the same holds for the blocks behind a tile's
-// last query (and behind the last prefix key, if the tile has queries inside the prefix), as long as
-// each of the tile's queries sees itself. To look that up costs a CTA some 3 us, so only from more
-// than kAheadKeys keys on (us before / so: prefix LM, 16 x 12 heads x 1024, 600 tokens in the prefix,
-// 472 / 409; causal, 8 x 32 heads of 128 x 1024 670 / 514; but 8 x 32 x 256 72 / 77).
 constexpr int kAheadKeys = 512;
-__device__ __forceinline__ bool causal_self(const AttnParams& p) {
-  return p.causal && p.Lq == p.Lk && p.causal_off == 0 && p.Lk > kAheadKeys;
+inline KeyLook key_look(const AttnParams& p) {
+  if (key_mask_alone(p)) return kLookMask;
+  // (causal alone: the last query gives the number of blocks, see the kernel)
+  const bool self = p.causal && p.Lq == p.Lk && p.causal_off == 0 && p.Lk > kAheadKeys;
+  return self && (p.key_mask != nullptr || p.kv_seg != nullptr) ? kLookCausal : kLookNone;
 }
 __device__ __forceinline__ bool sees_itself(const AttnParams& p, int b, int q) {
   const long long at = static_cast<long long>(b) * p.Lk + q;
@@ -81,24 +88,31 @@ __device__ __forceinline__ bool in_prefix(const AttnParams& p, int b, int k) {
   return p.causal == 2 && p.kv_seg != nullptr && ((p.kv_seg[static_cast<long long>(b) * p.Lk + k] >> 30) & 1);
 }
 constexpr int kAllKeys = 0x7fffffff;
-// Leaves two words per warp: the last key that counts, and whether the tile has prefix queries.
-__device__ __forceinline__ void find_visible_keys(const AttnParams& p, int b, int q_base, int q_end,
-                                                  int* words) {
-  int last = -1, pre = 0;
-  if (key_mask_alone(p)) {
-    for (int k = threadIdx.x; k < p.Lk; k += blockDim.x)
-      if (p.key_mask[static_cast<long long>(b) * p.Lk + k]) last = k;
-  } else if (causal_self(p)) {
-    for (int k = threadIdx.x; k < p.Lk; k += blockDim.x) {
-      if (in_prefix(p, b, k)) {
-        last = max(last, k);
-        if (k >= q_base && k < q_end) pre = 1;
-      }
-      if (k >= q_base && k < q_end && !sees_itself(p, b, k)) last = kAllKeys;
-    }
-  } else {
-    return;
-  }
+// A thread's first 16 bytes of the key mask, requested as the kernel starts, so that they arrive while the
+// barriers and the tensor memory are set up.
+struct MaskAhead {
+  uint4 bytes;
+  bool vec;  // the example's mask may be read 16 bytes at a time
+};
+__device__ __forceinline__ MaskAhead request_key_mask(const AttnParams& p, int b) {
+  MaskAhead m = {make_uint4(0u, 0u, 0u, 0u), false};
+  const uint8_t* row = p.key_mask + static_cast<long long>(b) * p.Lk;
+  m.vec = p.Lk % 16 == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0;
+  if (m.vec && static_cast<int>(threadIdx.x) * 16 < p.Lk)
+    m.bytes = reinterpret_cast<const uint4*>(row)[threadIdx.x];
+  return m;
+}
+__device__ __forceinline__ int last_nonzero_byte(const uint4& u) {  // 0 .. 15, -1: none
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+  int at = -1;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (w[i] != 0u) at = 4 * i + (31 - __clz(w[i])) / 8;
+  return at;
+}
+// `find_*` leave two words per warp: the last key that counts, and whether the tile has prefix queries. A
+// __syncthreads later `visible_key_blocks` gives the number of blocks.
+__device__ __forceinline__ void leave_words(int last, int pre, int* words) {
   last = __reduce_max_sync(0xffffffffu, last);
   pre = __reduce_max_sync(0xffffffffu, pre);
   if ((threadIdx.x & 31) == 0) {
@@ -106,17 +120,42 @@ __device__ __forceinline__ void find_visible_keys(const AttnParams& p, int b, in
     words[(threadIdx.x >> 5) * 2 + 1] = pre;
   }
 }
-__device__ __forceinline__ int visible_key_blocks(const AttnParams& p, int q_end, const int* words,
-                                                  int warps) {
+__device__ __forceinline__ void find_in_mask(const AttnParams& p, const MaskAhead& ahead, int b, int* words) {
+  const uint8_t* row = p.key_mask + static_cast<long long>(b) * p.Lk;
+  int last = -1;
+  if (ahead.vec) {
+    uint4 u = ahead.bytes;
+    for (int k = threadIdx.x * 16; k < p.Lk; k += blockDim.x * 16) {
+      if (k != static_cast<int>(threadIdx.x) * 16) u = *reinterpret_cast<const uint4*>(row + k);
+      const int at = last_nonzero_byte(u);
+      if (at >= 0) last = k + at;
+    }
+  } else {
+    for (int k = threadIdx.x; k < p.Lk; k += blockDim.x)
+      if (row[k]) last = k;
+  }
+  leave_words(last, 0, words);
+}
+__device__ __forceinline__ void find_ahead(const AttnParams& p, int b, int q_base, int q_end, int* words) {
+  int last = -1, pre = 0;
+  for (int k = threadIdx.x; k < p.Lk; k += blockDim.x) {
+    if (in_prefix(p, b, k)) {
+      last = max(last, k);
+      if (k >= q_base && k < q_end) pre = 1;
+    }
+    if (k >= q_base && k < q_end && !sees_itself(p, b, k)) last = kAllKeys;
+  }
+  leave_words(last, pre, words);
+}
+template <int kLook>
+__device__ __forceinline__ int visible_key_blocks(const AttnParams& p, int q_end, const int* words, int warps) {
   const int all = (p.Lk + 127) / 128;
-  const bool alone = key_mask_alone(p);
-  if (!alone && !causal_self(p)) return all;
   int last = -1, pre = 0;
   for (int w = 0; w < warps; ++w) {
     last = max(last, words[2 * w]);
     pre |= words[2 * w + 1];
   }
-  if (alone) return last < 0 ? all : last / 128 + 1;
+  if (kLook == kLookMask) return last < 0 ? all : last / 128 + 1;
   if (last == kAllKeys) return all;
   return min(all, max(q_end - 1, pre ? last : -1) / 128 + 1);
 }

@@ -68,7 +68,8 @@ __device__ __forceinline__ uint32_t low_bits(int n) {  // n leading ones, n clam
   return n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : ((1u << n) - 1u));
 }
 
-template <int D, int kTiles>
+// kLook: whether and where the number of key blocks is looked up (KeyLook).
+template <int D, int kTiles, int kLook>
 __global__ void __launch_bounds__(kFsThreads, 1)
     attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tmQ,
                            const __grid_constant__ CUtensorMap tmK,
@@ -93,12 +94,14 @@ __global__ void __launch_bounds__(kFsThreads, 1)
   uint64_t* bar_pv = bar_p + kFsMaxTiles;    // kTiles: O_t += P_t V_j finished
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_pv + kFsMaxTiles);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* last_key = reinterpret_cast<int*>(tmem_slot + 2);  // two words per warp
+  int* last_key = reinterpret_cast<int*>(tmem_slot + 2);  // two words per warp (kLook)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.y, b = blockIdx.z;
   const int q_base = blockIdx.x * (128 * kTiles);
   const int tiles_here = min(kTiles, (p.Lq - q_base + 127) / 128);  // >= 1
+  MaskAhead ahead = {};
+  if (kLook == kLookMask) ahead = request_key_mask(p, b);
   int nblk = (p.Lk + 127) / 128;
   if (p.causal && p.key_mask == nullptr && p.kv_seg == nullptr) {
     // every row sees key 0, so blocks beyond the last visible key of the CTA's last row
@@ -126,34 +129,53 @@ __global__ void __launch_bounds__(kFsThreads, 1)
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish();
   }
+  constexpr uint32_t kStageBytes = 2 * kPanels * kFsPanel;
+  auto load_queries = [&] {
+    mbar_expect_tx(bar_q, tiles_here * kPanels * kFsPanel);
+    for (int t = 0; t < tiles_here; ++t)
+      for (int c = 0; c < kPanels; ++c)
+        tma_load_4d(sQ + (t * kPanels + c) * kFsPanel, &tmQ, bar_q, c * 64, h, q_base + t * 128, b);
+  };
+  auto load_block = [&](int j) {
+    const int s = j % kStages;
+    uint8_t* st = sKV + s * kStageBytes;
+    mbar_expect_tx(&bar_full[s], kStageBytes);
+    for (int c = 0; c < kPanels; ++c) {
+      tma_load_4d(st + c * kFsPanel, &tmK, &bar_full[s], c * 64, h, j * 128, b);
+      tma_load_4d(st + (kPanels + c) * kFsPanel, &tmV, &bar_full[s], c * 64, h, j * 128, b);
+    }
+  };
   const int q_end = min(p.Lq, q_base + 128 * kTiles);
-  find_visible_keys(p, b, q_base, q_end, last_key);
+  if (kLook == kLookCausal) find_ahead(p, b, q_base, q_end, last_key);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  nblk = min(nblk, visible_key_blocks(p, q_end, last_key, kFsThreads / 32));
-  constexpr uint32_t kStageBytes = 2 * kPanels * kFsPanel;
+  if (kLook == kLookMask) {
+    // the first block always counts: it is on its way while the mask is looked through
+    if (warp == kFsLoadWarp && lane == 0) {
+      load_queries();
+      load_block(0);
+    }
+    __syncwarp();
+    find_in_mask(p, ahead, b, last_key);
+    __syncthreads();
+  }
+  // (as a broadcast the number is uniform over a warp to the compiler: all visible, 16 x 6 heads x 1024 166.6 /
+  // 163.5 us)
+  if (kLook != kLookNone)
+    nblk = __shfl_sync(0xffffffffu, min(nblk, visible_key_blocks<kLook>(p, q_end, last_key, kFsThreads / 32)), 0);
 
   if (warp == kFsLoadWarp) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
       bool ok = true;
-      mbar_expect_tx(bar_q, tiles_here * kPanels * kFsPanel);
-      for (int t = 0; t < tiles_here; ++t)
-        for (int c = 0; c < kPanels; ++c)
-          tma_load_4d(sQ + (t * kPanels + c) * kFsPanel, &tmQ, bar_q, c * 64, h,
-                      q_base + t * 128, b);
-      for (int j = 0; j < nblk && ok; ++j) {
+      if (kLook != kLookMask) load_queries();
+      for (int j = kLook == kLookMask ? 1 : 0; j < nblk && ok; ++j) {
         const int s = j % kStages;
         if (j >= kStages) ok = mbar_wait(&bar_free[s], ((j / kStages) - 1) & 1, abort_flag);
         if (!ok) break;
-        uint8_t* st = sKV + s * kStageBytes;
-        mbar_expect_tx(&bar_full[s], kStageBytes);
-        for (int c = 0; c < kPanels; ++c) {
-          tma_load_4d(st + c * kFsPanel, &tmK, &bar_full[s], c * 64, h, j * 128, b);
-          tma_load_4d(st + (kPanels + c) * kFsPanel, &tmV, &bar_full[s], c * 64, h, j * 128, b);
-        }
+        load_block(j);
       }
       if (!ok) {
         report_status(p.status, kStatusTimeoutMma, kKernelIdAttnFwd, blockIdx.x, 100 + blockIdx.y);
@@ -458,7 +480,7 @@ __global__ void __launch_bounds__(kFsThreads, 1)
   }
 }
 
-template <int D, int kTiles>
+template <int D, int kTiles, int kLook>
 int launch_stream(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* tv,
                   const AttnParams& p, cudaStream_t st) {
   using Cfg = FsCfg<D, kTiles>;
@@ -466,13 +488,13 @@ int launch_stream(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMa
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(attn_fwd_stream_kernel<D, kTiles>,
+    cudaError_t e = cudaFuncSetAttribute(attn_fwd_stream_kernel<D, kTiles, kLook>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kTotal);
     if (e != cudaSuccess) return set_error("attention_fwd_stream attr: %s", cudaGetErrorString(e));
     attr_set[dev] = true;
   }
   dim3 grid((p.Lq + 128 * kTiles - 1) / (128 * kTiles), p.H, p.B);
-  attn_fwd_stream_kernel<D, kTiles><<<grid, kFsThreads, Cfg::kTotal, st>>>(*tq, *tk, *tv, p);
+  attn_fwd_stream_kernel<D, kTiles, kLook><<<grid, kFsThreads, Cfg::kTotal, st>>>(*tq, *tk, *tv, p);
   count_launches(1);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("attention_fwd_stream: %s", cudaGetErrorString(e));
@@ -521,7 +543,13 @@ T5X_API int t5x_attention_fwd_stream(const void* q, const void* k, const void* v
   p.lse = static_cast<float*>(lse);
   p.status = device_status_buffer();
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (D == 128) return launch_stream<128, 1>(tq, tk, tv, p, st);
-  if (Lq > 128) return launch_stream<64, 2>(tq, tk, tv, p, st);
-  return launch_stream<64, 1>(tq, tk, tv, p, st);
+  const auto by_look = [&](auto none, auto mask, auto causal) {
+    const KeyLook look = key_look(p);
+    return (look == kLookMask ? mask : look == kLookCausal ? causal : none)(tq, tk, tv, p, st);
+  };
+  if (D == 128)
+    return by_look(launch_stream<128, 1, kLookNone>, launch_stream<128, 1, kLookMask>, launch_stream<128, 1, kLookCausal>);
+  if (Lq > 128)
+    return by_look(launch_stream<64, 2, kLookNone>, launch_stream<64, 2, kLookMask>, launch_stream<64, 2, kLookCausal>);
+  return by_look(launch_stream<64, 1, kLookNone>, launch_stream<64, 1, kLookMask>, launch_stream<64, 1, kLookCausal>);
 }

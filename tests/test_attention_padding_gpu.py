@@ -120,3 +120,29 @@ def test_hidden_query_blocks(mode, l, d):
     x, y = (x, y) if i == 2 else (x[seen], y[seen])
     if y.numel():
       assert float((x.double() - y).norm() / y.norm()) < 3 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("lk,offset", [(1024, 0), (1024, 8), (1040, 0), (5200, 0), (5200, 5), (5121, 0)])
+@pytest.mark.parametrize("d", [64, 128])
+def test_last_visible_key(lk, offset, d):
+  """The last visible key at the edges of the 16 bytes that a thread reads of the mask, of the blocks of 128
+  keys and of the part read first; rows of the mask that are and are not aligned."""
+  from t5x_b200.ops import attention, native
+  g = torch.Generator(device="cuda").manual_seed(lk)
+  ends = [1, 15, 16, 17, 128, 129, lk // 2, lk - 1, lk] + [n for n in (5119, 5120, 5121) if n < lk]
+  b, lq = len(ends), 130
+  rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+  q = (rnd(b, lq, 1, d) * d ** -0.5).bfloat16()
+  k, v = (rnd(b, lk, 1, d).bfloat16() for _ in range(2))
+  mask = torch.zeros(offset + b * lk, dtype=torch.bool, device="cuda")[offset:].view(b, lk)
+  mask.copy_(torch.arange(lk, device="cuda")[None] < torch.tensor(ends, device="cuda")[:, None])
+  mask[:, ::3] = False  # holes; of the first examples nothing or one key is left
+  with torch.no_grad():
+    o = attention.flash_attention(q, k, v, key_mask=mask)
+  native.check_status()
+  s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double())
+  s = torch.where(mask[:, None, None, :], s, s * 0 - 1e10)
+  want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), v.double())
+  # probabilities and result are each rounded to bf16 once
+  for x, y in zip(o.double(), want):
+    assert float((x - y).norm() / y.norm()) < 2 * 2.0 ** -8
