@@ -295,64 +295,86 @@ __global__ void __launch_bounds__(kRtThreads)
   }
 }
 
-// dw[c, e] = sum_t x[t, c] * dlogits[t, e] in two deterministic stages: a CTA reduces a tile of
-// kDwTile tokens for 256 columns into part[tile, c, e] (a thread owns two adjacent columns, the
-// tile's dlogits sit in shared memory), then a second kernel adds the tiles in a fixed order.
+// dw[c, e] = sum_t x[t, c] * dlogits[t, e] in two deterministic stages: a CTA reduces a tile of one to
+// four times kDwChunk tokens (`router_dw_chunks`) for 256 columns into part[tile, c, e] (a thread owns
+// two adjacent columns, a chunk's dlogits sit in shared memory), then a second kernel adds the tiles in
+// a fixed order.
 // Bound by the bytes of x in flight: with tiles of 512 tokens and one 2-byte load a column,
 // 32768 tokens were 64 CTAs that waited for each row in turn (32768 and 7296 tokens x 768, 8 experts, the
 // two calls together: 532 us, 49 so).
-constexpr int kDwTile = 128;
+constexpr int kDwChunk = 128;
 constexpr int kDwThreads = 128;
 constexpr int kDwCols = 2 * kDwThreads;
 constexpr int kDwAhead = 8;  // rows requested before the first is used
+constexpr int kDwMaxChunks = 4;
 
+// Chunks a tile: as many as leave six CTAs an SM. More tiles than that do not hide more, and the partial
+// sums, which are written and read once each, only grow with them: 268 MB for 262144 tokens x 512, 64
+// experts, 67 so. us, one chunk / two / four: 131072 x 512, 64 experts 1996 / 1971 / 2162; 131072 x 768, 8
+// experts 501 / 497 / 495; 32768 x 2048, 8 experts 294 / 290 / 316; but 65536 x 512, 32 experts (two: 3.5
+// CTAs an SM) 464 / 493 / 556.
+static int router_dw_chunks(int T, int d) {
+  const long long columns = (d + kDwCols - 1) / kDwCols;
+  int n = kDwMaxChunks;
+  while (n > 1 && (T + n * kDwChunk - 1) / (n * kDwChunk) * columns < 6 * num_sms()) n /= 2;
+  return n;
+}
+
+// kMany: tiles of more than one chunk (the loop over one costs 2 us).
+template <bool kMany>
 __global__ void __launch_bounds__(kDwThreads)
     router_dw_partial_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
-                             const float* __restrict__ dlogits, const RouterDims dm, int vec_ok,
-                             float* __restrict__ part /* [tiles, d, E] */) {
-  __shared__ __align__(16) float dl[kDwTile * 8];
+                             const float* __restrict__ dlogits, const RouterDims dm, int chunks,
+                             int vec_ok, float* __restrict__ part /* [tiles, d, E] */) {
+  __shared__ __align__(16) float dl[kDwChunk * 8];
   const int tile = blockIdx.x, c = blockIdx.y * kDwCols + 2 * threadIdx.x;
-  const int t0 = tile * kDwTile, nt = min(kDwTile, dm.T - t0);
+  const int first = tile * (kMany ? chunks : 1) * kDwChunk;
+  const int last = min(first + (kMany ? chunks : 1) * kDwChunk, dm.T);
   const bool both = c + 1 < dm.d;
-  const __nv_bfloat16* col = x + static_cast<long long>(t0) * ldx + c;
   float* out = part + (static_cast<long long>(tile) * dm.d + c) * dm.E;
-  auto load = [&](int t) {
-    const __nv_bfloat16* at = col + t * ldx;
-    if (vec_ok && both) return *reinterpret_cast<const uint32_t*>(at);
-    const __nv_bfloat16 zero = __float2bfloat16(0.f);
-    const __nv_bfloat162 v = __halves2bfloat162(c < dm.d ? at[0] : zero, both ? at[1] : zero);
-    return *reinterpret_cast<const uint32_t*>(&v);
-  };
   for (int e0 = 0; e0 < dm.E; e0 += 8) {
     const int ne = min(8, dm.E - e0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < nt * 8; i += kDwThreads) {
-      const int t = i >> 3, j = i & 7;
-      dl[i] = j < ne ? dlogits[static_cast<long long>(t0 + t) * dm.E + e0 + j] : 0.f;
-    }
-    __syncthreads();
-    if (c >= dm.d) continue;
     float acc[2][8] = {};
-    auto add = [&](int t, uint32_t u) {
-      const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u));
-      const float4 a = *reinterpret_cast<const float4*>(dl + t * 8);
-      const float4 b = *reinterpret_cast<const float4*>(dl + t * 8 + 4);
-      const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        acc[0][j] = fmaf(xv.x, w[j], acc[0][j]);
-        acc[1][j] = fmaf(xv.y, w[j], acc[1][j]);
+    for (int t0 = first; t0 < last; t0 += kDwChunk) {
+      const int nt = min(kDwChunk, last - t0);
+      __syncthreads();
+      for (int i = threadIdx.x; i < nt * 8; i += kDwThreads) {
+        const int t = i >> 3, j = i & 7;
+        dl[i] = j < ne ? dlogits[static_cast<long long>(t0 + t) * dm.E + e0 + j] : 0.f;
       }
-    };
-    int t = 0;
-    for (; t + kDwAhead <= nt; t += kDwAhead) {
-      uint32_t u[kDwAhead];
+      __syncthreads();
+      if (c >= dm.d) continue;
+      const __nv_bfloat16* col = x + static_cast<long long>(t0) * ldx + c;
+      auto load = [&](int t) {
+        const __nv_bfloat16* at = col + t * ldx;
+        if (vec_ok && both) return *reinterpret_cast<const uint32_t*>(at);
+        const __nv_bfloat16 zero = __float2bfloat16(0.f);
+        const __nv_bfloat162 v = __halves2bfloat162(at[0], both ? at[1] : zero);
+        return *reinterpret_cast<const uint32_t*>(&v);
+      };
+      auto add = [&](int t, uint32_t u) {
+        const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u));
+        const float4 a = *reinterpret_cast<const float4*>(dl + t * 8);
+        const float4 b = *reinterpret_cast<const float4*>(dl + t * 8 + 4);
+        const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-      for (int i = 0; i < kDwAhead; ++i) u[i] = load(t + i);
+        for (int j = 0; j < 8; ++j) {
+          acc[0][j] = fmaf(xv.x, w[j], acc[0][j]);
+          acc[1][j] = fmaf(xv.y, w[j], acc[1][j]);
+        }
+      };
+      int t = 0;
+      for (; t + kDwAhead <= nt; t += kDwAhead) {
+        uint32_t u[kDwAhead];
 #pragma unroll
-      for (int i = 0; i < kDwAhead; ++i) add(t + i, u[i]);
+        for (int i = 0; i < kDwAhead; ++i) u[i] = load(t + i);
+#pragma unroll
+        for (int i = 0; i < kDwAhead; ++i) add(t + i, u[i]);
+      }
+      for (; t < nt; ++t) add(t, load(t));
+      if (!kMany) break;
     }
-    for (; t < nt; ++t) add(t, load(t));
+    if (c >= dm.d) continue;
     for (int j = 0; j < ne; ++j) {
       out[e0 + j] = acc[0][j];
       if (both) out[dm.E + e0 + j] = acc[1][j];
@@ -401,7 +423,10 @@ T5X_API int t5x_moe_router_parts(int T) {
   return want < cap ? (want < 1 ? 1 : want) : cap;
 }
 
-T5X_API int t5x_moe_router_dw_tiles(int T) { return (T + t5x::kDwTile - 1) / t5x::kDwTile; }
+T5X_API int t5x_moe_router_dw_tiles(int T, int d) {
+  const int tile = t5x::router_dw_chunks(T, d) * t5x::kDwChunk;
+  return (T + tile - 1) / tile;
+}
 
 // Forward. x [T, d] bf16 (row stride ldx), w [d, E] fp32. Outputs: probs [T, E], lse [T],
 // index [T, k] int32, gate [T, k] fp32 (zero where the choice lost its slot), flat_slot [T, k]
@@ -448,7 +473,7 @@ T5X_API int t5x_moe_router_fwd(const void* x, long long ldx, const void* w, int 
 
 // Backward. dgate [T, k] (gradient of the returned gates), coef [2] device floats (gradients of
 // the auxiliary and z losses). Writes dlogits [T, E] (scratch), dx [T, d] bf16 (may be null)
-// and dw [d, E] fp32; dw_part: scratch of t5x_moe_router_dw_tiles(T) * d * E floats.
+// and dw [d, E] fp32; dw_part: scratch of t5x_moe_router_dw_tiles(T, d) * d * E floats.
 T5X_API int t5x_moe_router_bwd(const void* x, long long ldx, const void* w, int T, int d, int E,
                                int k, int capacity, const void* probs, const void* lse,
                                const void* index, const void* flat_slot, const void* dgate,
@@ -466,10 +491,12 @@ T5X_API int t5x_moe_router_bwd(const void* x, long long ldx, const void* w, int 
       static_cast<const float*>(dgate), static_cast<const float*>(stats),
       static_cast<const float*>(coef), static_cast<const float*>(w), dm,
       static_cast<float*>(dlogits), static_cast<__nv_bfloat16*>(dx), lddx);
-  const int tiles = (T + kDwTile - 1) / kDwTile;
+  const int tiles = t5x_moe_router_dw_tiles(T, d);
   const int vec_ok = ldx % 2 == 0 && (reinterpret_cast<uintptr_t>(x) & 3) == 0;
-  router_dw_partial_kernel<<<dim3(tiles, (d + kDwCols - 1) / kDwCols), kDwThreads, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const float*>(dlogits), dm, vec_ok,
+  const int chunks = router_dw_chunks(T, d);
+  const auto partial = chunks > 1 ? router_dw_partial_kernel<true> : router_dw_partial_kernel<false>;
+  partial<<<dim3(tiles, (d + kDwCols - 1) / kDwCols), kDwThreads, 0, st>>>(
+      static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const float*>(dlogits), dm, chunks, vec_ok,
       static_cast<float*>(dw_part));
   router_dw_reduce_kernel<<<(d * E + 31) / 32, 256, 0, st>>>(static_cast<const float*>(dw_part), tiles,
                                                              d * E, static_cast<float*>(dw));

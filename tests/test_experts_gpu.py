@@ -32,7 +32,7 @@ def test_gated_experts(e, n, d, ff, buffers):
 
 
 @pytest.mark.parametrize("t,d,e", [(1, 64, 2), (127, 250, 8), (128, 258, 9), (129, 1024, 16), (5000, 768, 8),
-                                   (300, 33, 64)])
+                                   (300, 33, 64), (300001, 64, 2), (90001, 701, 3), (200001, 700, 2)])
 def test_router_weight_gradient(t, d, e):
   """fp32 sums over the tokens: below t 2^-24 of the sum of magnitudes, whatever the order."""
   from t5x_b200.ops import native
