@@ -54,3 +54,53 @@ def test_router_weight_gradient(t, d, e):
   assert bool(((dw.double() - ref).abs() <= (t * 2.0 ** -24 + 2.0 ** -15) * size + 1e-12).all())
   again = native.moe_router_bwd(x, w, k, capacity, fwd, dgate, coef)[1]
   assert torch.equal(dw, again)
+
+
+def test_gated_gelu_far_from_zero():
+  """gelu itself, from -8 to 8, with a gate of 1. On the negative side 1 + tanh is a difference of two numbers
+  near 1, and the fast `tanhf` is good to 2^-11 of its value: beside the rounding to bf16 (half a unit of its
+  8 bits, 2^-8 of the result) that leaves |x| / 2 times as much, for the gradient times the inner derivative
+  and a square more."""
+  from t5x_b200.ops import functional as F
+  from t5x_b200.ops import native
+  x = torch.linspace(-8, 8, 1 << 15, device="cuda").bfloat16().unique()
+  x = x[:x.numel() // 248 * 248]
+  rows = torch.zeros(x.numel() // 62, 64, device="cuda")
+  rows[:, :62], rows[:, 63] = x.view(-1, 62), 1
+  w0, w1 = torch.eye(64, device="cuda"), torch.zeros(64, 64, device="cuda")
+  w0[63], w1[63] = 0, 1
+  with torch.no_grad():
+    got = F.batched_gated_mlp_in(rows.bfloat16()[None], w0[None], w1[None])[0, :, :62].reshape(-1)
+  xd = x.double().requires_grad_()
+  want = torch.nn.functional.gelu(xd, approximate="tanh")
+  slope, = torch.autograd.grad(want.sum(), xd)
+  want, xd = want.detach(), xd.detach()
+  tanh_part = 2.0 ** -11 * (1 + xd.abs() / 2)
+  assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + tanh_part).all())
+  h = torch.cat([x, torch.ones_like(x)])[None].contiguous()
+  native.gated_gelu_bwd_(torch.ones(1, x.numel(), device="cuda").bfloat16(), h)
+  d_x, d_gate = h[0, :x.numel()].double(), h[0, x.numel():].double()
+  inner = 0.8 * (1 + 3 * 0.044715 * xd * xd)
+  assert bool(((d_x - slope).abs() <= 2.0 ** -8 * slope.abs() + tanh_part * (1 + 2 * inner)).all())
+  assert bool(((d_gate - want).abs() <= 2.0 ** -8 * want.abs() + tanh_part).all())
+
+
+@pytest.mark.parametrize("spread", [0.3, 1.0, 3.0])
+def test_gated_experts_lose_nothing_to_separate_ops(spread):
+  """The activation in the epilogue, on sums that have not been rounded, against products, activation and
+  gate as separate ops with a rounding to bf16 after each: no further from float64, the negative side of the
+  activation taken by itself too."""
+  from t5x_b200.ops import functional as F
+  g = torch.Generator(device="cuda").manual_seed(9)
+  x = torch.randn(2, 300, 128, device="cuda", generator=g).bfloat16()
+  w = [(torch.randn(2, 128, 512, device="cuda", generator=g) * spread * 128 ** -0.5).bfloat16().float()
+       for _ in range(2)]
+  with torch.no_grad():
+    got = F.batched_gated_mlp_in(x, *w)
+    h = [F.batched_linear(x, p, torch.bfloat16) for p in w]
+    apart = torch.nn.functional.gelu(h[0], approximate="tanh") * h[1]
+  hd = [x.double() @ p.double() for p in w]
+  want = torch.nn.functional.gelu(hd[0], approximate="tanh") * hd[1]
+  for part in (hd[0] < 100, hd[0] < 0, hd[0] < -1, hd[0] < -3):
+    if int(part.sum()) > 100:
+      assert float((got.double() - want)[part].norm()) < float((apart.double() - want)[part].norm())
