@@ -253,19 +253,24 @@ optional<std::tuple<optional<Tensor>>> multi_linear_bwd(
   return std::make_tuple(dx);
 }
 
-// (gelu(x @ w0) * (x @ w1), the two pre-activations side by side)
-optional<std::tuple<Tensor, Tensor>> gated_in(const Tensor& x, const Tensor& w0, const Tensor& w1) {
+// (gelu(x @ w0) * (x @ w1), the two pre-activations side by side if they are to be kept)
+optional<std::tuple<Tensor, optional<Tensor>>> gated_in(const Tensor& x, const Tensor& w0, const Tensor& w1,
+                                                        bool keep) {
   if (!plain(x)) return std::nullopt;
   const int64_t k = x.size(-1), m = x.numel() / k;
   const Weight a(w0, k), b(w1, k);
   if (!a.ok || !b.ok || !fits(m) || w0.dim() != 2 || w1.dim() != 2 || a.n != b.n || a.ld != b.ld)
     return std::nullopt;
   Tensor g = at::empty(with_last(x, a.n), x.options());
-  Tensor h = at::empty({m, 2 * a.n}, x.options());
-  char* h0 = static_cast<char*>(h.data_ptr());
+  optional<Tensor> h;
+  char* h0 = nullptr;
+  if (keep) {
+    h = at::empty({m, 2 * a.n}, x.options());
+    h0 = static_cast<char*>(h->data_ptr());
+  }
   check(t5x_gemm_bf16(x.data_ptr(), w0.data_ptr(), w1.data_ptr(), g.data_ptr(), m, a.n, k, 1, k, a.ld,
-                      a.n, 0, 0, 0, 0, 1, 0, 0, 1, nullptr, 0, 0, h0, h0 + a.n * 2, 2 * a.n, 1.f, 0,
-                      stream_of()),
+                      a.n, 0, 0, 0, 0, 1, 0, 0, 1, nullptr, 0, 0, h0, keep ? h0 + a.n * 2 : nullptr, 2 * a.n,
+                      1.f, 0, stream_of()),
         "gemm");
   return std::make_tuple(g, h);
 }

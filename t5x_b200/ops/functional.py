@@ -284,7 +284,9 @@ class _BatchedGatedMlpInFn(torch.autograd.Function):
   def forward(ctx, x, wi_0, wi_1):
     x = x.contiguous()
     w0, w1 = compute_weight(wi_0, torch.bfloat16), compute_weight(wi_1, torch.bfloat16)
-    h = torch.empty(*x.shape[:2], 2 * w0.shape[2], dtype=torch.bfloat16, device=x.device)
+    h = None  # the pre-activations, where a backward pass may read them
+    if not isinstance(ctx, _NoGraph):
+      h = torch.empty(*x.shape[:2], 2 * w0.shape[2], dtype=torch.bfloat16, device=x.device)
     g = native.gemm(x, w0, b2=w1, save_h=h)
     ctx.save_for_backward(x, wi_0, wi_1, h)
     return g
@@ -429,10 +431,10 @@ class _GatedGeluMlpInFn(torch.autograd.Function):
 
   @staticmethod
   def forward(ctx, x, wi_0, wi_1):
-    host = native.host()
+    host, keep = native.host(), not isinstance(ctx, _NoGraph)
     if host is not None:
       done = host.gated_in(x, compute_weight(wi_0, torch.bfloat16),
-                           compute_weight(wi_1, torch.bfloat16))
+                           compute_weight(wi_1, torch.bfloat16), keep)
       if done is not None:
         ctx.save_for_backward(x, wi_0, wi_1, done[1])
         return done[0]
@@ -441,7 +443,7 @@ class _GatedGeluMlpInFn(torch.autograd.Function):
     w0 = compute_weight(wi_0, torch.bfloat16)
     w1 = compute_weight(wi_1, torch.bfloat16)
     dff = w0.shape[1]
-    h = torch.empty((x2.shape[0], 2 * dff), dtype=torch.bfloat16, device=x.device)
+    h = torch.empty((x2.shape[0], 2 * dff), dtype=torch.bfloat16, device=x.device) if keep else None
     g = native.gemm(x2, w0, b2=w1, save_h=h)
     ctx.save_for_backward(x, wi_0, wi_1, h)
     return g.view(*x.shape[:-1], dff)

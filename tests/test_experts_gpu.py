@@ -104,3 +104,27 @@ def test_gated_experts_lose_nothing_to_separate_ops(spread):
   for part in (hd[0] < 100, hd[0] < 0, hd[0] < -1, hd[0] < -3):
     if int(part.sum()) > 100:
       assert float((got.double() - want)[part].norm()) < float((apart.double() - want)[part].norm())
+
+
+@pytest.mark.parametrize("kind", ["experts", "dense", "dense_general"])
+def test_pre_activations_are_kept_for_a_backward_pass_only(kind, monkeypatch):
+  """The same result bit by bit with and without gradients; without them nothing but the result is
+  allocated."""
+  from t5x_b200.ops import functional as F
+  from t5x_b200.ops import native
+  if kind == "dense_general":  # the path for calls that the compiled one does not cover
+    monkeypatch.setattr(native, "host", lambda: None)
+  g = torch.Generator(device="cuda").manual_seed(3)
+  lead = (2,) if kind == "experts" else ()
+  x = torch.randn(*lead, 640, 64, device="cuda", generator=g).bfloat16()
+  w = [torch.nn.Parameter(torch.randn(*lead, 64, 512, device="cuda", generator=g) * 0.1) for _ in range(2)]
+  for p in w:
+    p.bf16 = p.detach().bfloat16()
+  call = F.batched_gated_mlp_in if kind == "experts" else F.gated_gelu_mlp_in
+  y = call(x, *w)
+  with torch.no_grad():
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    z = call(x, *w)
+    assert torch.cuda.max_memory_allocated() - before == z.numel() * 2
+  assert y.requires_grad and torch.equal(y, z)
