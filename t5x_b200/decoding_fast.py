@@ -248,6 +248,11 @@ def supported(module, decoder_input_tokens: torch.Tensor, decode_fn) -> bool:
   if not isinstance(module, network.Transformer) or decode_fn is not decoding.beam_search:
     return False
   c = module.config
+  # the step is written for this decoder (one position bias for all layers) and its own layers
+  if type(module.decoder) is not network.Decoder or \
+      any(type(getattr(module.decoder, f"layers_{i}")) is not network.DecoderLayer
+          for i in range(c.num_decoder_layers)):
+    return False
   p = module.token_embedder.embedding
   st = pstate.get()
   zctx = getattr(getattr(p, "zero", None), "ctx", None)

@@ -272,6 +272,25 @@ def test_predict_batch_uses_graph_decoder_by_default():
   assert model.__dict__.get("_graph_decoders")
 
 
+def test_predict_batch_of_a_model_with_a_bias_per_layer():
+  """The captured step does not cover it (one position bias for all layers): the general search runs."""
+  from t5x_b200 import adafactor, models, trainer
+  from t5x_b200.data import vocabularies
+  from t5x_b200.models import base
+  from t5x_b200.models.scalable_t5 import network
+  cfg = network.T5Config(vocab_size=256, dtype="bfloat16", emb_dim=128, num_heads=2, head_dim=64,
+                         num_encoder_layers=1, num_decoder_layers=2, mlp_dim=256,
+                         mlp_activations=("gelu", "linear"), dropout_rate=0.0)
+  module = network.Transformer(cfg, device="cuda")
+  vocab = vocabularies.PassThroughVocabulary(256)
+  model = models.EncoderDecoderModel(module, vocab, vocab, adafactor.Adafactor())
+  trainer.attach_compute_buffers(base.module_param_tree(module), main_grad=False)
+  batch = {"encoder_input_tokens": torch.randint(2, 256, (2, 16), device="cuda"),
+           "decoder_input_tokens": torch.zeros(2, 8, dtype=torch.long, device="cuda")}
+  assert model.predict_batch(None, batch).shape == (2, 8)
+  assert not model.__dict__.get("_graph_decoders")
+
+
 @pytest.mark.parametrize("beams,lk", [(1, 37), (4, 512), (8, 1000), (2, 16)])
 def test_decode_cross_attention_on_tensor_cores(beams, lk):
   """The mma.sync cross-attention (permuted channel and key order, transposed values) against
