@@ -533,13 +533,15 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  // The block's key mask, where it alone hides keys: requested here, so that it arrives during the set-up
+  // (128 x 12 heads x 114 x 512, all keys visible, us without a look / with / so: 479 / 489 / 482).
+  int shown = key_mask_alone(p) ? 0 : 1;
+  if (!shown && threadIdx.x < 128 && k0 + static_cast<int>(threadIdx.x) < p.Lk)
+    shown = p.key_mask[static_cast<long long>(b) * p.Lk + k0 + threadIdx.x];
   if (p.d_rel_bias != nullptr) {
     for (int t = threadIdx.x; t < lq_pad + 128; t += kAttnThreads) sDRel[t] = 0.f;
     if (threadIdx.x < kSmemBuckets) sBucket[threadIdx.x] = 0.f;
   }
-  bool shown = p.key_mask == nullptr;
-  if (p.key_mask != nullptr && threadIdx.x < 128 && k0 + static_cast<int>(threadIdx.x) < p.Lk)
-    shown = p.key_mask[static_cast<long long>(b) * p.Lk + k0 + threadIdx.x] != 0;
   tc_fence_before();
   const bool any_shown = __syncthreads_or(shown);
   tc_fence_after();
@@ -548,7 +550,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   // any key. With nothing but a key mask all queries do or none does, as the first one's lse tells.
   // (Keys of which 60 to 100 % are visible, us before / so: 32 x 64 heads x 512 x 512 1480 / 1352, 16 x
   // 6 x 1024 x 1024 326 / 284, 8 x 32 x 1024 x 1024 of 128 features 979 / 861; none hidden: 1140 / 1140.)
-  const bool idle = !any_shown && key_mask_alone(p) &&
+  const bool idle = !any_shown &&  // (then the key mask stands alone)
                     p.lse[(static_cast<long long>(b) * p.H + h) * p.Lq] >= -5e9f;
 
   // Of causal self-attention the query blocks ahead of this key block see nothing of it (unless both
