@@ -103,19 +103,22 @@ def test_hidden_query_blocks(mode, l, d):
     mask = mask & valid[:, None, :]
     kw = dict(causal=True, key_mask=valid if mode.endswith("padded") else None)
   o = attention.flash_attention(q, k, v, bias_table=table, bidirectional=False, **kw)
-  grads = torch.autograd.grad(o, [q, k, v], do)
+  grads = torch.autograd.grad(o, [q, k, v, table], do)
   native.check_status()
-  q2, k2, v2 = (t.detach().double().requires_grad_() for t in (q, k, v))
+  q2, k2, v2, t2 = (t.detach().double().requires_grad_() for t in (q, k, v, table))
   rel = pos[None] - pos[:, None]
   s = torch.einsum("bqhd,bkhd->bhqk", q2, k2) + \
-      table.detach().double()[:, reference.relative_position_bucket(rel, False, 32, 128)][None]
+      t2[:, reference.relative_position_bucket(rel, False, 32, 128)][None]
   s = torch.where(mask[:, None], s, s * 0 - 1e10)
   want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), v2)
-  ref = torch.autograd.grad(want, [q2, k2, v2], do.double())
+  ref = torch.autograd.grad(want, [q2, k2, v2, t2], do.double())
   # probabilities and their gradients are rounded to bf16 once, as is the result
   assert float((o.double() - want).norm() / want.norm()) < 2 * 2.0 ** -8
-  # (the kernel hands q and k the dS of rows that see nothing as if they were not masked)
+  # (the kernel hands q, k and the bias the dS of rows that see nothing as if they were not masked)
   seen = mask.any(-1).all(-1)
+  if bool(seen.all()):
+    assert float((grads[3].double() - ref[3]).norm() / ref[3].norm()) < 3 * 2.0 ** -8
+  grads, ref = grads[:3], ref[:3]
   for i, (x, y) in enumerate(zip(grads, ref)):
     x, y = (x, y) if i == 2 else (x[seen], y[seen])
     if y.numel():
