@@ -3,11 +3,11 @@
 // What bounds it: a training step of a small model, and a forward pass of one sentence, are
 // limited by the host: through ctypes a GEMM took some 20 us from the Python call to the launch
 // (28 converted arguments, a dozen tensor attributes, the current stream, an output allocation)
-// while the kernel runs for 4 to 8 us. (T5.1.1 small with 8 + 8 layers, one sentence scored:
-// 9.7 ms through ctypes, 3.8 ms so, of which the device works 1.3.) These functions do the same
-// from C++ for the plain case, contiguous activations and row-major bf16 weights, one call per op
-// and direction. They return None for anything else, before doing anything; the Python wrappers
-// then take their general path, which handles or rejects the call.
+// while the kernel runs for 4 to 8 us. (T5.1.1 small with 8 + 8 layers, one sentence scored: 9.7 ms
+// through ctypes, 3.8 so, 2.0 with the blocks of a layer as one call each, of which the device
+// works 1.2.) These functions do the same from C++ for the plain case, contiguous activations and
+// row-major bf16 weights, one call per op and direction. They return None for anything else, before
+// doing anything; the Python wrappers then take their general path, which handles or rejects the call.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
