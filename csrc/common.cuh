@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <initializer_list>
 #include <utility>
 
 namespace t5x {
@@ -460,6 +461,13 @@ void count_launches(int n);     // bookkeeping: kernels launched by this library
 int num_sms();
 bool chained_launches();  // t5x_set_chained_launches: overlap each kernel's prologue with its predecessor
 bool chained_launches_constant_b();  // level 2: GEMM B operands are constant weights
+
+// Whether every pointer (null ones aside) may be accessed `bytes` bytes at a time.
+inline bool aligned_to(uintptr_t bytes, std::initializer_list<const void*> pointers) {
+  for (const void* p : pointers)
+    if (reinterpret_cast<uintptr_t>(p) % bytes != 0) return false;
+  return true;
+}
 
 // Launches `kernel`; with chained launches switched on, as a programmatic dependent of the
 // kernel before it on `stream`. Only kernels that call `chain_wait()` before touching data of

@@ -636,6 +636,7 @@ using namespace t5x;
 T5X_API int t5x_rmsnorm_fwd(const void* x, const void* scale, void* y, void* rstd, int rows, int d,
                             float eps, void* stream) {
   if (rows <= 0) return 0;
+  if (!aligned_to(16, {x, scale, y})) return set_error("rmsnorm_fwd: pointers must be 16-byte aligned");
   if (d % 8 || d > kNormThreads * 8 * kNormMaxVec)
     return set_error("rmsnorm: d=%d must be a multiple of 8 and <= %d", d,
                      kNormThreads * 8 * kNormMaxVec);
@@ -672,6 +673,7 @@ T5X_API int t5x_rmsnorm_bwd(const void* dy, const void* x, const void* scale, co
                             const void* dres, void* dx, void* dscale, int rows, int d,
                             void* stream) {
   if (rows <= 0) return 0;
+  if (!aligned_to(16, {dy, x, scale, dres, dx})) return set_error("rmsnorm_bwd: pointers must be 16-byte aligned");
   if (d % 8 || d > kNormThreads * 8 * kNormMaxVec)
     return set_error("rmsnorm: d=%d must be a multiple of 8 and <= %d", d,
                      kNormThreads * 8 * kNormMaxVec);
@@ -722,6 +724,7 @@ T5X_API int t5x_rmsnorm_bwd(const void* dy, const void* x, const void* scale, co
 T5X_API int t5x_gated_gelu_bwd(void* dg, void* h, long long rows, int dff, long long ldh,
                                long long ldg, int write_g, void* stream) {
   if (rows <= 0) return 0;
+  if (!aligned_to(16, {dg, h})) return set_error("gated_gelu_bwd: pointers must be 16-byte aligned");
   if (dff % 8 || ldh % 8 || ldg % 8) return set_error("gated_gelu: sizes must be multiples of 8");
   gated_gelu_bwd_kernel<<<ew_grid(rows * (dff / 8), 256), 256, 0,
                           static_cast<cudaStream_t>(stream)>>>(
@@ -733,6 +736,7 @@ T5X_API int t5x_gated_gelu_bwd(void* dg, void* h, long long rows, int dff, long 
 T5X_API int t5x_gated_gelu_fwd(const void* h, void* g, long long rows, int dff, long long ldh,
                                long long ldg, void* stream) {
   if (rows <= 0) return 0;
+  if (!aligned_to(16, {h, g})) return set_error("gated_gelu_fwd: pointers must be 16-byte aligned");
   if (dff % 8 || ldh % 8 || ldg % 8) return set_error("gated_gelu: sizes must be multiples of 8");
   gated_gelu_fwd_kernel<<<ew_grid(rows * (dff / 8), 256), 256, 0,
                           static_cast<cudaStream_t>(stream)>>>(
@@ -744,6 +748,7 @@ T5X_API int t5x_gated_gelu_fwd(const void* h, void* g, long long rows, int dff, 
 T5X_API int t5x_embedding_fwd(const void* ids, const void* table, void* out, long long tokens, int d,
                               int vocab_start, int vocab_rows, void* stream) {
   if (tokens <= 0) return 0;
+  if (!aligned_to(16, {table, out})) return set_error("embedding_fwd: pointers must be 16-byte aligned");
   if (d % 8) return set_error("embedding: d must be a multiple of 8");
   embedding_fwd_kernel<<<ew_grid(tokens * (d / 8), 256), 256, 0,
                          static_cast<cudaStream_t>(stream)>>>(
@@ -756,6 +761,7 @@ T5X_API int t5x_embedding_fwd(const void* ids, const void* table, void* out, lon
 T5X_API int t5x_embedding_bwd(const void* ids, const void* dout, void* dtable, long long tokens,
                               int d, int vocab_start, int vocab_rows, void* stream) {
   if (tokens <= 0) return 0;
+  if (!aligned_to(8, {dout})) return set_error("embedding_bwd: misaligned pointer");
   if (d % 8) return set_error("embedding: d must be a multiple of 8");
   // four columns per thread; whole warps, at most 256 threads
   const int threads = d / 4 >= 256 ? 256 : (d / 4 + 31) / 32 * 32;
@@ -780,6 +786,7 @@ T5X_API int t5x_embedding_bwd(const void* ids, const void* dout, void* dtable, l
 T5X_API int t5x_cast_f32_bf16(const void* src, void* dst, long long rows, int cols, long long lds,
                               long long ldd, void* stream) {
   if (rows <= 0 || cols <= 0) return 0;
+  if (!aligned_to(16, {src}) || !aligned_to(8, {dst})) return set_error("cast: misaligned pointer");
   if (cols % 4 || lds % 4 || ldd % 4) return set_error("cast: sizes must be multiples of 4");
   cast_f32_bf16_kernel<<<ew_grid(rows * (cols / 4), 256), 256, 0,
                          static_cast<cudaStream_t>(stream)>>>(
@@ -826,6 +833,8 @@ __global__ void __launch_bounds__(256)
 T5X_API int t5x_f32_to_bf16_residual(const void* src, const void* residual, void* dst,
                                      long long n, void* stream) {
   if (n <= 0) return 0;
+  if (!t5x::aligned_to(16, {src}) || !t5x::aligned_to(8, {residual, dst}))
+    return t5x::set_error("f32_to_bf16_residual: misaligned pointer");
   if (n % 4) return t5x::set_error("f32_to_bf16_residual: n must be a multiple of 4");
   const long long n4 = n / 4;
   long long blocks = (n4 + 255) / 256;
@@ -845,6 +854,8 @@ T5X_API int t5x_f32_to_bf16_residual(const void* src, const void* residual, void
 T5X_API int t5x_f32_to_bf16_residual_clear(void* src, const void* residual, void* dst, long long n,
                                            void* stream) {
   if (n <= 0) return 0;
+  if (!t5x::aligned_to(16, {src}) || !t5x::aligned_to(8, {residual, dst}))
+    return t5x::set_error("f32_to_bf16_residual_clear: misaligned pointer");
   if (n % 4) return t5x::set_error("f32_to_bf16_residual_clear: n must be a multiple of 4");
   const long long n4 = n / 4;
   long long blocks = (n4 + 255) / 256;
@@ -924,6 +935,8 @@ T5X_API int t5x_finish_residual_rmsnorm(void* ws, const void* residual, const vo
                                         void* stream) {
   using namespace t5x;
   if (rows <= 0) return 0;
+  if (!aligned_to(16, {ws, residual, scale, x, h}))
+    return set_error("finish_residual_rmsnorm: pointers must be 16-byte aligned");
   if (d % 8 || d > kNormThreads * 8 * kNormMaxVec)
     return set_error("finish_residual_rmsnorm: d=%d must be a multiple of 8 and <= %d", d,
                      kNormThreads * 8 * kNormMaxVec);

@@ -128,3 +128,16 @@ def test_pre_activations_are_kept_for_a_backward_pass_only(kind, monkeypatch):
     z = call(x, *w)
     assert torch.cuda.max_memory_allocated() - before == z.numel() * 2
   assert y.requires_grad and torch.equal(y, z)
+
+
+def test_gradient_that_is_not_aligned_is_refused():
+  """A contiguous gradient that starts between two 16-byte boundaries: an error, as from the products."""
+  from t5x_b200.ops import functional as F
+  from t5x_b200.ops import native
+  x = torch.randn(2, 16, 64, device="cuda").bfloat16().requires_grad_()
+  w = [torch.nn.Parameter(torch.randn(2, 64, 64, device="cuda")) for _ in range(2)]
+  y = F.batched_gated_mlp_in(x, *w)
+  dg = torch.randn(y.numel() + 1, device="cuda").bfloat16()[1:].view(y.shape)
+  with pytest.raises(native.NativeError, match="aligned"):
+    y.backward(dg)
+  torch.cuda.synchronize()
