@@ -669,43 +669,48 @@ T5X_API int t5x_rmsnorm_fwd(const void* x, const void* scale, void* y, void* rst
   return 0;
 }
 
+// The CTAs of the backward kernel, each of which leaves a row of d partial sums for dscale.
+static bool norm_bwd_by_warps(int d) { return d <= kNormWarpMaxVec * 32 * 8; }  // one warp per row
+static int norm_bwd_grid(int rows, int d) {
+  constexpr int kMaxParts = 1024;
+  if (norm_bwd_by_warps(d)) {  // eight rows per CTA
+    const int wpb = kNormThreads / 32;
+    const int most = num_sms() * (d <= 768 && rows >= 8192 ? 2 : 4);
+    return std::min(std::min((rows + wpb - 1) / wpb, most), kMaxParts);
+  }
+  const int nv = d <= 2048 ? 1 : (d <= 4096 ? 2 : 4);
+  return std::min(std::min(rows, num_sms() * norm_bwd_ctas(nv)), kMaxParts);
+}
+
+// Floats that t5x_rmsnorm_bwd needs in `partial`.
+T5X_API long long t5x_rmsnorm_bwd_partial(int rows, int d) {
+  return rows <= 0 || d <= 0 ? 0 : static_cast<long long>(norm_bwd_grid(rows, d)) * d;
+}
+
+// `partial`: scratch of t5x_rmsnorm_bwd_partial(rows, d) floats, the caller's own, so that calls on
+// several streams do not meet in it; dscale and partial may both be null.
 T5X_API int t5x_rmsnorm_bwd(const void* dy, const void* x, const void* scale, const void* rstd,
-                            const void* dres, void* dx, void* dscale, int rows, int d,
+                            const void* dres, void* dx, void* dscale, void* partial, int rows, int d,
                             void* stream) {
   if (rows <= 0) return 0;
-  if (!aligned_to(16, {dy, x, scale, dres, dx})) return set_error("rmsnorm_bwd: pointers must be 16-byte aligned");
+  if (!aligned_to(16, {dy, x, scale, dres, dx, partial}))
+    return set_error("rmsnorm_bwd: pointers must be 16-byte aligned");
   if (d % 8 || d > kNormThreads * 8 * kNormMaxVec)
     return set_error("rmsnorm: d=%d must be a multiple of 8 and <= %d", d,
                      kNormThreads * 8 * kNormMaxVec);
-  // Workspace for the per-CTA dscale sums: one buffer per device, allocated at the first call
-  // (so not under stream capture) and shared by all calls: backward passes on one stream.
-  constexpr int kMaxParts = 1024;
-  static float* ws[64] = {nullptr};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dscale != nullptr && ws[dev] == nullptr) {
-    if (cudaMalloc(&ws[dev], sizeof(float) * kMaxParts * kNormThreads * 8 * kNormMaxVec) !=
-        cudaSuccess)
-      return set_error("rmsnorm_bwd: workspace allocation failed");
-  }
+  if ((dscale == nullptr) != (partial == nullptr)) return set_error("rmsnorm_bwd: dscale goes with its scratch");
   const int nv = d <= 2048 ? 1 : (d <= 4096 ? 2 : 4);
-  int grid = num_sms() * norm_bwd_ctas(nv);
-  if (grid > rows) grid = rows;
-  if (grid > kMaxParts) grid = kMaxParts;
+  const int grid = norm_bwd_grid(rows, d);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  float* partial = dscale != nullptr ? ws[dev] : nullptr;
+  float* part = static_cast<float*>(partial);
   auto launch = [&](auto kernel) {
     kernel<<<grid, kNormThreads, 0, st>>>(
         static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
         static_cast<const float*>(scale), static_cast<const float*>(rstd),
-        static_cast<const __nv_bfloat16*>(dres), static_cast<__nv_bfloat16*>(dx), partial, rows, d);
+        static_cast<const __nv_bfloat16*>(dres), static_cast<__nv_bfloat16*>(dx), part, rows, d);
   };
-  if (d <= kNormWarpMaxVec * 32 * 8) {  // narrow rows: one warp per row, eight rows per CTA
-    const int wpb = kNormThreads / 32;
-    grid = (rows + wpb - 1) / wpb;
+  if (norm_bwd_by_warps(d)) {
     const bool ahead = d <= 768 && rows >= 8192;
-    const int most = std::min(num_sms() * (ahead ? 2 : 4), kMaxParts);
-    if (grid > most) grid = most;
     if (!ahead) launch(rmsnorm_bwd_warp_kernel<4, false>);
     else if (d <= 512) launch(rmsnorm_bwd_warp_kernel<2, true>);
     else launch(rmsnorm_bwd_warp_kernel<3, true>);
@@ -714,8 +719,7 @@ T5X_API int t5x_rmsnorm_bwd(const void* dy, const void* x, const void* scale, co
   else launch(rmsnorm_bwd_kernel<4>);
   if (dscale != nullptr) {
     count_launches(1);
-    rmsnorm_dscale_reduce_kernel<<<(d + 31) / 32, 256, 0, st>>>(partial, grid, d,
-                                                                  static_cast<float*>(dscale));
+    rmsnorm_dscale_reduce_kernel<<<(d + 31) / 32, 256, 0, st>>>(part, grid, d, static_cast<float*>(dscale));
   }
   CHECK_LAUNCH("rmsnorm_bwd");
   return 0;

@@ -314,6 +314,11 @@ optional<std::tuple<Tensor, Tensor>> rmsnorm(const Tensor& x, const Tensor& scal
   return std::make_tuple(y, rstd);
 }
 
+// Scratch for the partial sums of a norm's scale gradient.
+Tensor norm_partial(const Tensor& x, int64_t rows, int64_t d) {
+  return at::empty({static_cast<int64_t>(t5x_rmsnorm_bwd_partial(rows, d))}, x.options().dtype(at::kFloat));
+}
+
 // dx (+ dres); adds to `dscale`
 optional<Tensor> rmsnorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& scale,
                              const Tensor& rstd, const optional<Tensor>& dres, Tensor dscale) {
@@ -323,10 +328,11 @@ optional<Tensor> rmsnorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& sc
     return std::nullopt;
   if (dres && !(plain(*dres) && dres->numel() == x.numel())) return std::nullopt;
   const int64_t d = x.size(-1), rows = x.numel() / d;
-  Tensor dx = at::empty_like(x);
+  if (!fits(rows)) return std::nullopt;
+  Tensor dx = at::empty_like(x), partial = norm_partial(x, rows, d);
   check(t5x_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), scale.data_ptr(), rstd.data_ptr(),
-                        dres ? dres->data_ptr() : nullptr, dx.data_ptr(), dscale.data_ptr(), rows, d,
-                        stream_of()),
+                        dres ? dres->data_ptr() : nullptr, dx.data_ptr(), dscale.data_ptr(),
+                        partial.data_ptr(), rows, d, stream_of()),
         "rmsnorm_bwd");
   return dx;
 }
@@ -458,9 +464,9 @@ std::tuple<Tensor, Tensor> norm_forward(const Tensor& x, const Tensor& scale, do
 // The norm's input gradient plus that of the residual branch.
 Tensor norm_backward(const Tensor& dh, const Tensor& x, const Tensor& scale, const Tensor& rstd,
                      const Tensor& dres, Tensor& dscale, void* st) {
-  Tensor dx = at::empty_like(x);
+  Tensor dx = at::empty_like(x), partial = norm_partial(x, rows_of(x), x.size(-1));
   check(t5x_rmsnorm_bwd(dh.data_ptr(), x.data_ptr(), scale.data_ptr(), rstd.data_ptr(), dres.data_ptr(),
-                        dx.data_ptr(), dscale.data_ptr(), rows_of(x), x.size(-1), st),
+                        dx.data_ptr(), dscale.data_ptr(), partial.data_ptr(), rows_of(x), x.size(-1), st),
         "rmsnorm_bwd");
   return dx;
 }

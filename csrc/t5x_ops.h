@@ -10,8 +10,10 @@ extern "C" {
 
 int t5x_rmsnorm_fwd(const void* x, const void* scale, void* y, void* rstd, int rows, int d, float eps,
                     void* stream);
+long long t5x_rmsnorm_bwd_partial(int rows, int d);
 int t5x_rmsnorm_bwd(const void* dy, const void* x, const void* scale, const void* rstd,
-                    const void* dres, void* dx, void* dscale, int rows, int d, void* stream);
+                    const void* dres, void* dx, void* dscale, void* partial, int rows, int d,
+                    void* stream);
 int t5x_attention_fwd(const void* q, const void* k, const void* v, void* o, void* lse, int B, int H,
                       int Lq, int Lk, long long q_sb, long long q_sl, long long q_sh, long long k_sb,
                       long long k_sl, long long k_sh, long long v_sb, long long v_sl, long long v_sh,

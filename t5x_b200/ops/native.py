@@ -50,7 +50,8 @@ def _declare(lib):
       c_ll, c_float, c_int, c_void_p]
   lib.t5x_rmsnorm_fwd.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float,
                                   c_void_p]
-  lib.t5x_rmsnorm_bwd.argtypes = [c_void_p] * 7 + [c_int, c_int, c_void_p]
+  lib.t5x_rmsnorm_bwd_partial.argtypes, lib.t5x_rmsnorm_bwd_partial.restype = [c_int, c_int], c_ll
+  lib.t5x_rmsnorm_bwd.argtypes = [c_void_p] * 8 + [c_int, c_int, c_void_p]
   lib.t5x_gated_gelu_bwd.argtypes = [c_void_p, c_void_p, c_ll, c_int, c_ll, c_ll, c_int, c_void_p]
   lib.t5x_gated_gelu_fwd.argtypes = [c_void_p, c_void_p, c_ll, c_int, c_ll, c_ll, c_void_p]
   lib.t5x_embedding_fwd.argtypes = [c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int,
@@ -662,9 +663,10 @@ def rmsnorm_bwd(dy, x, scale, rstd, dres: Optional[torch.Tensor], dscale: torch.
   if dres is not None:
     dres2 = dres.reshape(-1, d)
     assert dres2.is_contiguous()
+  partial = torch.empty(lib().t5x_rmsnorm_bwd_partial(x2.shape[0], d), dtype=torch.float32, device=x.device)
   _check(lib().t5x_rmsnorm_bwd(dy2.data_ptr(), x2.data_ptr(), scale.data_ptr(), rstd.data_ptr(),
-                               ptr(dres2), dx.data_ptr(), dscale.data_ptr(), x2.shape[0], d,
-                               stream_ptr()), "rmsnorm_bwd")
+                               ptr(dres2), dx.data_ptr(), dscale.data_ptr(), partial.data_ptr(),
+                               x2.shape[0], d, stream_ptr()), "rmsnorm_bwd")
   return dx.view(x.shape)
 
 

@@ -11,7 +11,7 @@ def _calls(lib):
   norm_tail = (4, 64, ctypes.c_float(1e-6), ctypes.c_void_p(0))
   return {
       "rmsnorm_fwd": (lib.t5x_rmsnorm_fwd, [A] * 4, [0, 1, 2], norm_tail),
-      "rmsnorm_bwd": (lib.t5x_rmsnorm_bwd, [A] * 7, [0, 1, 2, 4, 5], (4, 64, 0)),
+      "rmsnorm_bwd": (lib.t5x_rmsnorm_bwd, [A] * 8, [0, 1, 2, 4, 5, 7], (4, 64, 0)),
       "gated_gelu_bwd": (lib.t5x_gated_gelu_bwd, [A] * 2, [0, 1], (4, 64, 128, 64, 0, 0)),
       "embedding_fwd": (lib.t5x_embedding_fwd, [A] * 3, [1, 2], (4, 64, 0, 8, 0)),
       "embedding_bwd": (lib.t5x_embedding_bwd, [A] * 3, [1], (4, 64, 0, 8, 0)),
