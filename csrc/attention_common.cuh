@@ -200,14 +200,14 @@ __device__ __forceinline__ void store16_bf16(__nv_bfloat16* dst, const uint32_t 
 
 // Tensor map over a [B, L, H, D] bf16 tensor with element strides (sb, sl, sh): boxes of
 // 64 channels x 128 positions of one head (one 128-byte-swizzled shared-memory panel).
-inline const CUtensorMap* bhld_map(const void* ptr, int B, int L, int H, long long sb, long long sl,
-                                   long long sh, int D = kAttnD) {
+inline bool bhld_map(CUtensorMap* map, const void* ptr, int B, int L, int H, long long sb, long long sl,
+                     long long sh, int D = kAttnD) {
   uint64_t dims[4] = {static_cast<uint64_t>(D), static_cast<uint64_t>(H),
                       static_cast<uint64_t>(L), static_cast<uint64_t>(B)};
   uint64_t strides[3] = {static_cast<uint64_t>(sh) * 2, static_cast<uint64_t>(sl) * 2,
                          static_cast<uint64_t>(sb) * 2};
   uint32_t box[4] = {64, 1, 128, 1};
-  return get_tensor_map(ptr, 2, 4, dims, strides, box, 1);
+  return get_tensor_map(map, ptr, 2, 4, dims, strides, box, 1);
 }
 
 }  // namespace t5x

@@ -524,10 +524,10 @@ T5X_API int t5x_attention_fwd_stream(const void* q, const void* k, const void* v
   if (B > 65535 || H > 65535) return set_error("attention_fwd_stream: B or H beyond the grid limit");
   if ((o_sb | o_sl | o_sh) & 7 || (reinterpret_cast<uintptr_t>(o) & 15))
     return set_error("attention_fwd_stream: output rows must be 16-byte aligned");
-  const CUtensorMap* tq = bhld_map(q, B, Lq, H, q_sb, q_sl, q_sh, D);
-  const CUtensorMap* tk = bhld_map(k, B, Lk, H, k_sb, k_sl, k_sh, D);
-  const CUtensorMap* tv = bhld_map(v, B, Lk, H, v_sb, v_sl, v_sh, D);
-  if (!tq || !tk || !tv) return -1;
+  CUtensorMap tq, tk, tv;
+  if (!bhld_map(&tq, q, B, Lq, H, q_sb, q_sl, q_sh, D) || !bhld_map(&tk, k, B, Lk, H, k_sb, k_sl, k_sh, D) ||
+      !bhld_map(&tv, v, B, Lk, H, v_sb, v_sl, v_sh, D))
+    return -1;
   AttnParams p = {};
   p.B = B; p.H = H; p.Lq = Lq; p.Lk = Lk;
   p.rel_bias = static_cast<const float*>(rel_bias);
@@ -545,7 +545,7 @@ T5X_API int t5x_attention_fwd_stream(const void* q, const void* k, const void* v
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const auto by_look = [&](auto none, auto mask, auto causal) {
     const KeyLook look = key_look(p);
-    return (look == kLookMask ? mask : look == kLookCausal ? causal : none)(tq, tk, tv, p, st);
+    return (look == kLookMask ? mask : look == kLookCausal ? causal : none)(&tq, &tk, &tv, p, st);
   };
   if (D == 128)
     return by_look(launch_stream<128, 1, kLookNone>, launch_stream<128, 1, kLookMask>, launch_stream<128, 1, kLookCausal>);

@@ -1049,10 +1049,10 @@ T5X_API int t5x_attention_fwd(const void* q, const void* k, const void* v, void*
   if (causal == 2) return set_error("attention_fwd: prefix-LM masks need the streaming kernel");
   if (Lq > kFwdMaxLq && rel_bias != nullptr)
     return set_error("attention_fwd: Lq=%d > %d with a relative bias is not covered", Lq, kFwdMaxLq);
-  const CUtensorMap* tq = bhld_map(q, B, Lq, H, q_sb, q_sl, q_sh);
-  const CUtensorMap* tk = bhld_map(k, B, Lk, H, k_sb, k_sl, k_sh);
-  const CUtensorMap* tv = bhld_map(v, B, Lk, H, v_sb, v_sl, v_sh);
-  if (!tq || !tk || !tv) return -1;
+  CUtensorMap tq, tk, tv;
+  if (!bhld_map(&tq, q, B, Lq, H, q_sb, q_sl, q_sh) || !bhld_map(&tk, k, B, Lk, H, k_sb, k_sl, k_sh) ||
+      !bhld_map(&tv, v, B, Lk, H, v_sb, v_sl, v_sh))
+    return -1;
   AttnParams p = {};
   p.B = B; p.H = H; p.Lq = Lq; p.Lk = Lk;
   p.rel_bias = static_cast<const float*>(rel_bias);
@@ -1078,7 +1078,7 @@ T5X_API int t5x_attention_fwd(const void* q, const void* k, const void* v, void*
   }
   dim3 grid(H, B);
   attn_fwd_kernel<<<grid, kAttnThreads, FwdSmem::kTotal, static_cast<cudaStream_t>(stream)>>>(
-      *tq, *tk, *tv, p);
+      tq, tk, tv, p);
   count_launches(1);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("attention_fwd: %s", cudaGetErrorString(e));
@@ -1133,11 +1133,11 @@ T5X_API int t5x_attention_bwd(const void* q, const void* k, const void* v, const
   if (D != 64 && D != 128) return set_error("attention_bwd: head_dim %d not in {64, 128}", D);
   if (Lq > 4096) return set_error("attention_bwd: Lq=%d > 4096 is not covered by this kernel", Lq);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const CUtensorMap* tq = bhld_map(q, B, Lq, H, q_sb, q_sl, q_sh, D);
-  const CUtensorMap* tk = bhld_map(k, B, Lk, H, k_sb, k_sl, k_sh, D);
-  const CUtensorMap* tv = bhld_map(v, B, Lk, H, v_sb, v_sl, v_sh, D);
-  const CUtensorMap* tdo = bhld_map(d_o, B, Lq, H, do_sb, do_sl, do_sh, D);
-  if (!tq || !tk || !tv || !tdo) return -1;
+  CUtensorMap tq, tk, tv, tdo;
+  if (!bhld_map(&tq, q, B, Lq, H, q_sb, q_sl, q_sh, D) || !bhld_map(&tk, k, B, Lk, H, k_sb, k_sl, k_sh, D) ||
+      !bhld_map(&tv, v, B, Lk, H, v_sb, v_sl, v_sh, D) ||
+      !bhld_map(&tdo, d_o, B, Lq, H, do_sb, do_sl, do_sh, D))
+    return -1;
   if ((do_sb | do_sl | do_sh | o_sb | o_sl | o_sh | dk_sb | dk_sl | dk_sh) & 7)
     return set_error("attention_bwd: dO / O / dK strides must be multiples of 8 elements");
   AttnParams p = {};
@@ -1161,5 +1161,5 @@ T5X_API int t5x_attention_bwd(const void* q, const void* k, const void* v, const
   const bool ahead = causal && Lq == Lk && causal_off == 0 && Lq > (causal == 2 ? kAheadKeys : 128);
   const auto launch = D == 128 ? (ahead ? launch_attention_bwd<128, true> : launch_attention_bwd<128, false>)
                                : (ahead ? launch_attention_bwd<64, true> : launch_attention_bwd<64, false>);
-  return launch(d_o, o, delta, tq, tk, tv, tdo, p, do_sb, do_sl, do_sh, o_sb, o_sl, o_sh, st);
+  return launch(d_o, o, delta, &tq, &tk, &tv, &tdo, p, do_sb, do_sl, do_sh, o_sb, o_sl, o_sh, st);
 }

@@ -451,11 +451,11 @@ __device__ __forceinline__ void chain_release() {
 namespace t5x {
 // Returns 0 on success, else a negative error (and keeps the message for t5x_last_error()).
 int set_error(const char* fmt, ...);
-// Encodes (and caches) a tiled bf16/fp32 tensor map. dims/strides innermost first;
-// strides in bytes for dims 1.. (dim 0 is contiguous). Returns nullptr on failure.
-const CUtensorMap* get_tensor_map(const void* base, int elem_bytes, int rank, const uint64_t* dims,
-                                  const uint64_t* strides_bytes, const uint32_t* box,
-                                  int swizzle_128b);
+// Encodes (and caches) a tiled bf16/fp32 tensor map into `map`. dims/strides innermost first;
+// strides in bytes for dims 1.. (dim 0 is contiguous). The caller has a copy of its own: the cache is
+// cleared when it is full, by whichever call or thread fills it. Returns false on failure.
+bool get_tensor_map(CUtensorMap* map, const void* base, int elem_bytes, int rank, const uint64_t* dims,
+                    const uint64_t* strides_bytes, const uint32_t* box, int swizzle_128b);
 int* device_status_buffer();  // per-device status words (zero on success)
 void count_launches(int n);     // bookkeeping: kernels launched by this library
 int num_sms();

@@ -348,9 +348,7 @@ bool few_map(CUtensorMap* out, const void* ptr, long long inner, long long outer
   uint64_t dims[3] = {static_cast<uint64_t>(inner), static_cast<uint64_t>(outer), 1};
   uint64_t strides[2] = {static_cast<uint64_t>(ld) * 2, static_cast<uint64_t>(ld) * 2 * outer};
   uint32_t box[3] = {64, box_outer, 1};
-  const CUtensorMap* m = get_tensor_map(ptr, 2, 3, dims, strides, box, 1);
-  if (m != nullptr) *out = *m;
-  return m != nullptr;
+  return get_tensor_map(out, ptr, 2, 3, dims, strides, box, 1);
 }
 
 template <int EPI>

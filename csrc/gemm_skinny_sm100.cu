@@ -400,8 +400,8 @@ __global__ void __launch_bounds__(kSkThreads, SkinnyCfg<BN>::kCtasPerSm)
   }
 }
 
-static const CUtensorMap* skinny_map(const void* ptr, int mn_major, long long rows_mn, long long k,
-                                     long long ld, uint32_t box_mn) {
+static bool skinny_map(CUtensorMap* map, const void* ptr, int mn_major, long long rows_mn, long long k,
+                       long long ld, uint32_t box_mn) {
   uint64_t dims[3];
   uint64_t strides[2];
   uint32_t box[3];
@@ -416,7 +416,7 @@ static const CUtensorMap* skinny_map(const void* ptr, int mn_major, long long ro
   box[2] = 1;
   strides[0] = static_cast<uint64_t>(ld) * 2;
   strides[1] = strides[0] * dims[1];
-  return get_tensor_map(ptr, 2, 3, dims, strides, box, 1);
+  return get_tensor_map(map, ptr, 2, 3, dims, strides, box, 1);
 }
 
 }  // namespace t5x
@@ -439,9 +439,8 @@ static int launch_skinny(const void* A, const void* B, SkinnyParams& p, long lon
                          long long ldb, void* stream) {
   using Cfg = SkinnyCfg<BN>;
   p.tiles_n = p.N / BN;
-  const CUtensorMap* tA = skinny_map(A, 0, p.M, p.K, lda, kBM);
-  const CUtensorMap* tB = skinny_map(B, p.b_mn, p.N, p.K, ldb, BN);
-  if (!tA || !tB) return -1;
+  CUtensorMap tA, tB;
+  if (!skinny_map(&tA, A, 0, p.M, p.K, lda, kBM) || !skinny_map(&tB, B, p.b_mn, p.N, p.K, ldb, BN)) return -1;
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -473,7 +472,7 @@ static int launch_skinny(const void* A, const void* B, SkinnyParams& p, long lon
   }
   cfg.attrs = attr;
   cfg.numAttrs = n_attr;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<BN>, *tA, *tB, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<BN>, tA, tB, p);
   count_launches(1);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("gemm_skinny launch: %s", cudaGetErrorString(e));

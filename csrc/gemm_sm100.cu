@@ -359,9 +359,7 @@ static bool operand_map(CUtensorMap* map, const void* ptr, int mn_major, long lo
   strides[0] = static_cast<uint64_t>(ld) * 2;
   strides[1] = static_cast<uint64_t>(batch > 1 ? batch_stride : ld * dims[1]) * 2;
   if (strides[1] == 0) strides[1] = strides[0];
-  const CUtensorMap* m = get_tensor_map(ptr, 2, 3, dims, strides, box, 1);
-  if (m != nullptr) *map = *m;
-  return m != nullptr;
+  return get_tensor_map(map, ptr, 2, 3, dims, strides, box, 1);
 }
 
 }  // namespace t5x

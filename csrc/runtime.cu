@@ -59,11 +59,10 @@ struct MapKeyHash {
 };
 
 static std::mutex g_map_mu;
-static std::unordered_map<MapKey, CUtensorMap*, MapKeyHash> g_maps;
+static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;
 
-const CUtensorMap* get_tensor_map(const void* base, int elem_bytes, int rank, const uint64_t* dims,
-                                  const uint64_t* strides_bytes, const uint32_t* box,
-                                  int swizzle_128b) {
+bool get_tensor_map(CUtensorMap* map, const void* base, int elem_bytes, int rank, const uint64_t* dims,
+                    const uint64_t* strides_bytes, const uint32_t* box, int swizzle_128b) {
   MapKey key;
   memset(&key, 0, sizeof(key));
   key.w[0] = reinterpret_cast<uint64_t>(base);
@@ -76,16 +75,19 @@ const CUtensorMap* get_tensor_map(const void* base, int elem_bytes, int rank, co
   }
   std::lock_guard<std::mutex> lk(g_map_mu);
   auto it = g_maps.find(key);
-  if (it != g_maps.end()) return it->second;
+  if (it != g_maps.end()) {
+    *map = it->second;
+    return true;
+  }
 
   EncodeTiledFn enc = encode_fn();
   if (!enc) {
     set_error("cuTensorMapEncodeTiled is not available from this driver");
-    return nullptr;
+    return false;
   }
   if ((reinterpret_cast<uint64_t>(base) & 15) != 0) {
     set_error("tensor map base %p is not 16-byte aligned", base);
-    return nullptr;
+    return false;
   }
   cuuint64_t gdims[5];
   cuuint64_t gstr[5];
@@ -100,16 +102,15 @@ const CUtensorMap* get_tensor_map(const void* base, int elem_bytes, int rank, co
       if (gstr[i - 1] % 16 != 0) {
         set_error("tensor map stride %llu is not a multiple of 16 bytes",
                   (unsigned long long)gstr[i - 1]);
-        return nullptr;
+        return false;
       }
     }
   }
   CUtensorMapDataType dt = elem_bytes == 2   ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                            : elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                              : CU_TENSOR_MAP_DATA_TYPE_UINT8;
-  CUtensorMap* m = new CUtensorMap;
   auto encode = [&] {
-    return enc(m, dt, rank, const_cast<void*>(base), gdims, gstr, gbox, estr,
+    return enc(map, dt, rank, const_cast<void*>(base), gdims, gstr, gbox, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE,
                swizzle_128b ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -122,18 +123,14 @@ const CUtensorMap* get_tensor_map(const void* base, int elem_bytes, int rank, co
     if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
   }
   if (r != CUDA_SUCCESS) {
-    delete m;
     set_error("cuTensorMapEncodeTiled failed with %d (rank %d, dims %llu x %llu, box %u x %u)",
               (int)r, rank, (unsigned long long)dims[0],
               (unsigned long long)(rank > 1 ? dims[1] : 1), box[0], rank > 1 ? box[1] : 1);
-    return nullptr;
+    return false;
   }
-  if (g_maps.size() > 65536) {  // unbounded growth guard: descriptors are cheap to rebuild
-    for (auto& kv : g_maps) delete kv.second;
-    g_maps.clear();
-  }
-  g_maps.emplace(key, m);
-  return m;
+  if (g_maps.size() > 65536) g_maps.clear();  // unbounded growth guard: descriptors are cheap to rebuild
+  g_maps.emplace(key, *map);
+  return true;
 }
 
 struct DeviceState {
