@@ -548,8 +548,11 @@ T5X_API int t5x_attention_fwd_stream(const void* q, const void* k, const void* v
     return (look == kLookMask ? mask : look == kLookCausal ? causal : none)(&tq, &tk, &tv, p, st);
   };
   if (D == 128)
-    return by_look(launch_stream<128, 1, kLookNone>, launch_stream<128, 1, kLookMask>, launch_stream<128, 1, kLookCausal>);
+    return by_look(launch_stream<128, 1, kLookNone>, launch_stream<128, 1, kLookMask>,
+                   launch_stream<128, 1, kLookCausal>);
   if (Lq > 128)
-    return by_look(launch_stream<64, 2, kLookNone>, launch_stream<64, 2, kLookMask>, launch_stream<64, 2, kLookCausal>);
-  return by_look(launch_stream<64, 1, kLookNone>, launch_stream<64, 1, kLookMask>, launch_stream<64, 1, kLookCausal>);
+    return by_look(launch_stream<64, 2, kLookNone>, launch_stream<64, 2, kLookMask>,
+                   launch_stream<64, 2, kLookCausal>);
+  return by_look(launch_stream<64, 1, kLookNone>, launch_stream<64, 1, kLookMask>,
+                 launch_stream<64, 1, kLookCausal>);
 }
