@@ -1,0 +1,903 @@
+// Flash attention backward on sm_100a for head_dim 64 and up to 512 queries: one CTA per (head, example).
+//
+// The CTA walks the key blocks of its head and, inside each, the queries 64 at a time. dQ of all (up to
+// four) query blocks stays in TMEM for the whole walk, dK and dV of a key block for its part of it, so all
+// three gradients leave the chip once and in bf16: no fp32 dQ in memory that is cleared, added to and cast,
+// and rowsum(dO * O) is computed while the first operands travel instead of by a kernel of its own.
+//
+// TMEM (512 columns): S^T 0..63, dP^T 64..127, dQ of query block i 128 + 64 i, dK 384, dV 448.
+// Shared memory: K and V of two key blocks, Q and dO of three 64-query units, P^T of two units, dS^T of two
+// query blocks. The MMA warp issues the scores of unit u + 1 as soon as the 16 softmax warps hold those of
+// unit u in registers, and the gradient products of unit u - 1 while they do their arithmetic on unit u; the
+// softmax warps never wait for one another inside the walk.
+//
+//
+// One CTA per 128-key block (attention_sm100.cu) spends 14k cycles on setting up and tearing down a CTA and
+// 6.7k on a 128 x 128 tile. Here a CTA takes 16k and a 128 x 64 unit 2 to 3k, bound by what a softmax warp does
+// one after the other for a unit (us, with rowsum(dO * O), clearing and casting of dQ where there are any,
+// before / now: 128 x 12 heads x 512 x 512 1081 / 610, 114 x 512 without a bias 385 / 202, 114 x 114 causal
+// 184 / 113, 32 x 64 x 512 x 512 1327 / 792). Of the 610, the bias gradient takes 100 (40 its additions to
+// shared memory, which are loops around a compare-and-swap), the bias 35, the exponentials 8.
+#include <type_traits>
+
+#include "attention_common.cuh"
+#include "t5x_ops.h"
+
+namespace t5x {
+namespace {
+
+constexpr int kMaxQ = 512;        // queries: 4 x 64 columns of TMEM for dQ
+constexpr int kMaxRel = 1152;     // padded queries + padded keys, with a bias table
+constexpr int kMaxKeys = 4096;    // a bit per key block
+constexpr int kBuckets = 128;     // bias tables of more buckets take the other kernel
+constexpr int kRing = 3;
+constexpr int kOutside = 255, kMixed = 254;  // in tables of buckets: none, several
+constexpr int kThreads = kSoftmaxThreads + 64;  // + MMA warp + TMA warp
+constexpr int kMmaWarp = kSoftmaxWarps, kTmaWarp = kSoftmaxWarps + 1;
+constexpr int kKernelId = 12;
+
+struct HeadSmem {
+  static constexpr int kPanel = 128 * 128;  // [128 x 64] bf16
+  static constexpr int kHalf = 64 * 128;    // [64 x 64] bf16
+  static constexpr int kK = 0;              // 2 stages
+  static constexpr int kV = kK + 2 * kPanel;
+  static constexpr int kQ = kV + 2 * kPanel;       // kRing stages
+  static constexpr int kDO = kQ + kRing * kHalf;   // kRing stages
+  static constexpr int kP = kDO + kRing * kHalf;   // 2 x [128 keys x 64 queries]
+  static constexpr int kDS = kP + 2 * kPanel;      // 2 query blocks x 2 x [128 keys x 64 queries]
+  static constexpr int kVec = kDS + 4 * kPanel;    // -lse * log2(e), -rowsum(dO * O), query codes
+  static constexpr int kRel = kVec + 3 * kMaxQ * 4;  // bias by (k - q)
+  static constexpr int kDRel = kRel + kMaxRel * 4;   // its gradient
+  static constexpr int kChange = kDRel + kMaxRel * 4;  // bit t: another bucket than at t - 1
+  static constexpr int kBucketAt = kChange + (kMaxRel / 32 + 2) * 4;  // bucket by (k - q), 255: outside the table
+  // by t / 16: the bucket of all positions t - 15 .. t + 31, or kMixed
+  static constexpr int kFlat = kBucketAt + kMaxRel;
+  static constexpr int kBucket = kFlat + (kMaxRel / 16 + 7) / 8 * 8;  // bias gradient by bucket
+  static constexpr int kWords = kBucket + kBuckets * 4;  // block flags
+  static constexpr int kBars = kWords + 4 * 4;
+  static constexpr int kTotal = kBars + 24 * 8 + 1024;
+};
+static_assert(HeadSmem::kTotal <= 232448, "shared memory of a CTA");
+static_assert(HeadSmem::kBars % 8 == 0, "barriers are 8-byte words");
+
+struct HeadParams {
+  AttnParams a;
+  const __nv_bfloat16* O;
+  const __nv_bfloat16* dO;
+  long long o_sb, o_sl, o_sh, do_sb, do_sl, do_sh;
+  int ahead;  // CTAs that run at a time
+};
+
+__device__ __forceinline__ uint64_t pair_of(float a, float b) {
+  return static_cast<uint64_t>(__float_as_uint(a)) | (static_cast<uint64_t>(__float_as_uint(b)) << 32);
+}
+__device__ __forceinline__ float low_of(uint64_t v) { return __uint_as_float(static_cast<uint32_t>(v)); }
+__device__ __forceinline__ float high_of(uint64_t v) { return __uint_as_float(static_cast<uint32_t>(v >> 32)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// Waits for the loads from TMEM into these registers.
+__device__ __forceinline__ void tmem_wait_into(uint32_t (&a)[16], uint32_t (&c)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
+                 "+r"(a[8]), "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15])
+               :
+               : "memory");
+  asm volatile("" : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(c[4]), "+r"(c[5]), "+r"(c[6]), "+r"(c[7]),
+                    "+r"(c[8]), "+r"(c[9]), "+r"(c[10]), "+r"(c[11]), "+r"(c[12]), "+r"(c[13]), "+r"(c[14]), "+r"(c[15]));
+}
+
+// kAhead: causal self-attention over more than one block, where key blocks ahead of a query block are
+// passed over (see attn_bwd_kernel for the conditions).
+template <bool kAhead>
+__global__ void __launch_bounds__(kThreads, 1)
+    attn_bwd_head_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
+                         const __grid_constant__ CUtensorMap tmDQ, const __grid_constant__ CUtensorMap tmDK,
+                         const __grid_constant__ CUtensorMap tmDV, const __grid_constant__ CUtensorMap tmO,
+                         const __grid_constant__ HeadParams hp) {
+  const AttnParams& p = hp.a;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  float* sLse = reinterpret_cast<float*>(smem + HeadSmem::kVec);
+  float* sDelta = sLse + kMaxQ;
+  int* sQseg = reinterpret_cast<int*>(sDelta + kMaxQ);
+  float* sRel = reinterpret_cast<float*>(smem + HeadSmem::kRel);
+  float* sDRel = reinterpret_cast<float*>(smem + HeadSmem::kDRel);
+  uint32_t* sChange = reinterpret_cast<uint32_t*>(smem + HeadSmem::kChange);
+  uint8_t* sBucketAt = smem + HeadSmem::kBucketAt;
+  uint8_t* sFlat = smem + HeadSmem::kFlat;
+  float* sBucket = reinterpret_cast<float*>(smem + HeadSmem::kBucket);
+  uint32_t* sWords = reinterpret_cast<uint32_t*>(smem + HeadSmem::kWords);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + HeadSmem::kBars);
+  uint64_t* bar_kv = bars;            // 2: K and V of a key block landed
+  uint64_t* bar_staged = bars + 2;    // 2: dK and dV of it have taken their place
+  uint64_t* bar_q = bars + 4;         // kRing: Q and dO of a unit landed
+  uint64_t* bar_qfree = bars + 7;     // kRing: ... and are no longer read
+  uint64_t* bar_s = bars + 10;        // S^T and dP^T of a unit are in TMEM
+  uint64_t* bar_sfree = bars + 11;    // ... and in registers
+  uint64_t* bar_p = bars + 12;        // 2: P^T and dS^T of a unit are in shared memory
+  uint64_t* bar_g = bars + 14;        // 2: the gradient products of a unit are done
+  uint64_t* bar_dq = bars + 16;       // dQ of all query blocks is in shared memory
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int h = blockIdx.x, b = blockIdx.y;
+  const int nkb = (p.Lk + 127) / 128;
+  const int lq_pad = (p.Lq + 127) / 128 * 128;
+  const int units = (p.Lq + 63) / 64;  // of a key block
+  constexpr int cS = 0, cDP = 64, cDQ = 128, cDK = 384, cDV = 448;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&bar_kv[s], 1);
+      mbar_init(&bar_staged[s], kSoftmaxWarps);
+      mbar_init(&bar_p[s], kSoftmaxWarps);
+      mbar_init(&bar_g[s], 1);
+    }
+    for (int s = 0; s < kRing; ++s) {
+      mbar_init(&bar_q[s], 1);
+      mbar_init(&bar_qfree[s], 1);
+    }
+    mbar_init(bar_s, 1);
+    mbar_init(bar_sfree, kSoftmaxWarps);
+    mbar_init(bar_dq, kSoftmaxWarps);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (threadIdx.x < 4) sWords[threadIdx.x] = 0u;
+  if (warp == kMmaWarp) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  if (warp == kTmaWarp && lane == 0) {
+    tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
+    tma_prefetch_desc(&tmDO);
+  }
+  // The softmax warps request what their tables are made of: the buckets of up to three relative
+  // positions a thread (and, in a warp's first lane, of the position before), and a query's statistics.
+  constexpr int kRelRounds = (kMaxRel + 32 + kSoftmaxThreads - 1) / kSoftmaxThreads;
+  const int rels = lq_pad + nkb * 128;  // table index t: k - q = t - lq_pad
+  int bucket[kRelRounds], left[kRelRounds];
+  // ... and of rowsum(dO * O): eight lanes a query, the first four of eight rounds of queries.
+  constexpr int kRows = kSoftmaxThreads / 8;
+  float lse = 0.f;
+  int code = 0;
+  uint4 xo[4], xd[4];
+  const int sub = threadIdx.x & 7;
+  const __nv_bfloat16* o_row = hp.O + b * hp.o_sb + h * hp.o_sh + sub * 8;
+  const __nv_bfloat16* do_row = hp.dO + b * hp.do_sb + h * hp.do_sh + sub * 8;
+  auto request_rows = [&](int q0) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int q = q0 + c * kRows;
+      xo[c] = xd[c] = make_uint4(0u, 0u, 0u, 0u);
+      if (q < p.Lq) {
+        xo[c] = *reinterpret_cast<const uint4*>(o_row + static_cast<long long>(q) * hp.o_sl);
+        xd[c] = *reinterpret_cast<const uint4*>(do_row + static_cast<long long>(q) * hp.do_sl);
+      }
+    }
+  };
+  if (warp < kSoftmaxWarps) {
+    request_rows(threadIdx.x >> 3);
+#pragma unroll
+    for (int c = 0; c < kRelRounds; ++c) {
+      const int t = threadIdx.x + c * kSoftmaxThreads, idx = t - lq_pad + p.rel_off;
+      bucket[c] = left[c] = -1;
+      if (p.rel_bias != nullptr && t <= rels) {
+        if (t < rels && idx >= 0 && idx < p.nrel) bucket[c] = __ldg(p.rel_bucket + idx);
+        if (lane == 0 && t > 0 && idx >= 1 && idx <= p.nrel) left[c] = __ldg(p.rel_bucket + idx - 1);
+      }
+    }
+    const int q = threadIdx.x;
+    if (q < p.Lq) {
+      lse = p.lse[(static_cast<long long>(b) * p.H + h) * p.Lq + q];
+      if (p.q_seg) code = p.q_seg[static_cast<long long>(b) * p.Lq + q];
+    }
+  }
+  // Key blocks that a key mask alone hides whole (words[0]: blocks with a visible key), and of causal
+  // self-attention the query blocks with a query that does not see itself (words[1]) and the key blocks
+  // with a prefix key (words[2]): what may be passed over, as in attn_bwd_kernel.
+  const bool look = key_mask_alone(p);
+  uint32_t shown = 0u, unseen = 0u, prefix = 0u;
+  float lse0 = 0.f;
+  if (look) {
+    const uint8_t* row = p.key_mask + static_cast<long long>(b) * p.Lk;
+    lse0 = p.lse[(static_cast<long long>(b) * p.H + h) * p.Lq];
+    for (int k0 = warp * 32; k0 < p.Lk; k0 += kThreads)
+      if (__any_sync(0xffffffffu, k0 + lane < p.Lk && row[k0 + lane] != 0)) shown |= 1u << (k0 >> 7);
+  }
+  if (kAhead) {
+    for (int k0 = warp * 32; k0 < p.Lk; k0 += kThreads) {
+      const int k = k0 + lane;
+      if (__any_sync(0xffffffffu, k < p.Lk && !sees_itself(p, b, k))) unseen |= 1u << (k0 >> 7);
+      if (__any_sync(0xffffffffu, k < p.Lk && in_prefix(p, b, k))) prefix |= 1u << (k0 >> 7);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  uint32_t idle = 0u;
+  if (look || kAhead) {
+    if (lane == 0) {
+      if (shown) atomicOr(&sWords[0], shown);
+      if (unseen) atomicOr(&sWords[1], unseen);
+      if (prefix) atomicOr(&sWords[2], prefix);
+    }
+    __syncthreads();
+    if (look && lse0 >= -5e9f) idle = ~sWords[0];
+    unseen = sWords[1];
+    prefix = sWords[2];
+  }
+  // first unit of key block j
+  auto first_unit = [&](int j) {
+    if (!kAhead) return 0;
+    const uint32_t before = (1u << j) - 1u;
+    return ((unseen & before) | ((prefix >> j) & 1u)) ? 0 : 2 * j;
+  };
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == kTmaWarp) {
+    if (lane == 0) {
+      bool ok = true;
+      int n = 0, u = 0;      // key blocks and units walked
+      int loaded = 0, stored = 0;      // key blocks whose K and V were requested, whose gradients were stored
+      int j_load = 0, j_store = 0;     // the next ones
+      auto skip = [&](int j) {
+        while (j < nkb && ((idle >> j) & 1u)) ++j;
+        return j;
+      };
+      // the gradients of the oldest key block that is still on the chip, from where its K and V were
+      auto store_kv = [&]() {
+        const int st = stored & 1;
+        if (!mbar_wait(&bar_staged[st], (stored >> 1) & 1, abort_flag)) return false;
+        j_store = skip(j_store);
+        tma_store_4d(&tmDK, smem + HeadSmem::kK + st * HeadSmem::kPanel, 0, h, j_store * 128, b);
+        tma_store_4d(&tmDV, smem + HeadSmem::kV + st * HeadSmem::kPanel, 0, h, j_store * 128, b);
+        bulk_commit();
+        ++stored;
+        ++j_store;
+        return true;
+      };
+      auto load_kv = [&]() {
+        j_load = skip(j_load);
+        if (j_load >= nkb) return true;
+        const int st = loaded & 1;
+        if (loaded >= 2) {
+          if (!store_kv()) return false;
+          bulk_store_wait_read();
+        }
+        mbar_expect_tx(&bar_kv[st], 2 * HeadSmem::kPanel);
+        tma_load_4d(smem + HeadSmem::kK + st * HeadSmem::kPanel, &tmK, &bar_kv[st], 0, h, j_load * 128, b);
+        tma_load_4d(smem + HeadSmem::kV + st * HeadSmem::kPanel, &tmV, &bar_kv[st], 0, h, j_load * 128, b);
+        ++loaded;
+        ++j_load;
+        return true;
+      };
+      for (int j = 0; j < nkb && ok; ++j) {
+        if ((idle >> j) & 1u) continue;
+        if (loaded == n) ok = load_kv();
+        const int first = first_unit(j);
+        for (int w = first; w < units && ok; ++w, ++u) {
+          const int st = u % kRing;
+          if (u >= kRing) ok = mbar_wait(&bar_qfree[st], (u / kRing - 1) & 1, abort_flag);
+          if (!ok) break;
+          mbar_expect_tx(&bar_q[st], 2 * HeadSmem::kHalf);
+          tma_load_4d(smem + HeadSmem::kQ + st * HeadSmem::kHalf, &tmQ, &bar_q[st], 0, h, w * 64, b);
+          tma_load_4d(smem + HeadSmem::kDO + st * HeadSmem::kHalf, &tmDO, &bar_q[st], 0, h, w * 64, b);
+          // the next key block, once the operands of this one's first units are under way (its place holds
+          // the gradients of the block before until they are stored)
+          if (w == min(first + 2, units - 1)) ok = load_kv();
+        }
+        // What the CTA after this one on the SM (about hp.ahead heads further) starts with goes to L2 now:
+        // all SMs load their 320 KB at about the same time, and wait for it.
+        if (n == 0) {
+          const long long head = static_cast<long long>(b) * p.H + h + hp.ahead;
+          const int hn = static_cast<int>(head % p.H), bn = static_cast<int>(head / p.H);
+          if (bn < p.B) {
+            for (int i = 0; i < p.Lq; i += 64) {
+              tma_prefetch_4d(&tmO, 0, hn, i, bn);
+              tma_prefetch_4d(&tmDO, 0, hn, i, bn);
+              tma_prefetch_4d(&tmQ, 0, hn, i, bn);
+            }
+            tma_prefetch_4d(&tmK, 0, hn, 0, bn);
+            tma_prefetch_4d(&tmV, 0, hn, 0, bn);
+          }
+        }
+        ++n;
+      }
+      while (ok && stored < loaded) ok = store_kv();
+      if (ok) ok = mbar_wait(bar_dq, 0, abort_flag);
+      if (ok) {
+        for (int i = 0; i < lq_pad / 128; ++i)
+          tma_store_4d(&tmDQ, smem + HeadSmem::kDS + i * HeadSmem::kPanel, 0, h, i * 128, b);
+        bulk_commit();
+      }
+      bulk_store_wait_all();
+      if (!ok) {
+        report_status(p.status, kStatusTimeoutProducer, kKernelId, blockIdx.x, blockIdx.y);
+        *abort_flag = 1;
+      }
+    }
+  } else if (warp == kMmaWarp) {
+    // The whole warp walks the units and one lane issues: with everything uniform the descriptors stay in
+    // uniform registers and an addition apart (in a branch of one lane an MMA took 90 to 120 cycles to
+    // issue, twice what it takes to run).
+    const bool leader = elect_one();
+    bool ok = true;
+    const uint32_t idesc_s = make_idesc_bf16(128, 64, 0, 0);   // [keys x queries], K = d
+    const uint32_t idesc_kd = make_idesc_bf16(128, 64, 0, 1);  // [keys x d], K = queries
+    const uint32_t idesc_qd = make_idesc_bf16(128, 64, 1, 1);  // [queries x d], K = keys
+    constexpr uint32_t kP16 = HeadSmem::kPanel >> 4, kH16 = HeadSmem::kHalf >> 4;
+    // operands with the contraction contiguous (K S-steps 32 bytes apart), and those read across it
+    const uint64_t row_major = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
+    const uint64_t col_major = make_smem_desc_sw128(smem_u32(smem), HeadSmem::kPanel, 1024);
+    uint32_t started = 0u;  // query blocks whose dQ holds something
+    // dV += P^T dO, dK += dS^T Q, and after the last unit of a query block dQ += dS K (whose A operand is
+    // the dS^T tiles read with the queries contiguous; the panel of a unit that does not exist adds to
+    // rows that nothing reads).
+    auto issue_grads = [&](int u, int ring, int kv, int w, bool first, int pair) {
+      const uint64_t qd = col_major + (HeadSmem::kQ >> 4) + static_cast<uint32_t>(ring) * kH16;
+      const uint64_t dod = col_major + (HeadSmem::kDO >> 4) + static_cast<uint32_t>(ring) * kH16;
+      const uint64_t pd = row_major + (HeadSmem::kP >> 4) + static_cast<uint32_t>(u & 1) * kP16;
+      const uint64_t dsd = row_major + (HeadSmem::kDS >> 4) + static_cast<uint32_t>(pair * 2 + (w & 1)) * kP16;
+      const bool whole = (w & 1) || w == units - 1;
+      const int i = w >> 1;
+      if (leader) {
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+          umma_bf16(tmem_base + cDV, pd + 2 * s, dod + 128 * s, idesc_kd, !first || s != 0);
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+          umma_bf16(tmem_base + cDK, dsd + 2 * s, qd + 128 * s, idesc_kd, !first || s != 0);
+        umma_commit(&bar_qfree[ring]);
+        if (whole) {
+          const uint64_t kd = col_major + (HeadSmem::kK >> 4) + static_cast<uint32_t>(kv) * kP16;
+          const uint64_t da = col_major + (HeadSmem::kDS >> 4) + static_cast<uint32_t>(pair * 2) * kP16;
+          const bool add = (started >> i) & 1u;
+#pragma unroll
+          for (int s = 0; s < 8; ++s)
+            umma_bf16(tmem_base + cDQ + i * 64, da + 128 * s, kd + 128 * s, idesc_qd, add || s != 0);
+        }
+        umma_commit(&bar_g[u & 1]);
+      }
+      if (whole) started |= 1u << i;
+    };
+    int n = 0, u = 0, pair = 0, ring = 0, ring_phase = 0;
+    int prev_ring = 0, prev_kv = 0, prev_w = 0, prev_pair = 0;
+    bool prev_first = false;
+    for (int j = 0; j < nkb && ok; ++j) {
+      if ((idle >> j) & 1u) continue;
+      const int kv = n & 1;
+      ok = mbar_wait(&bar_kv[kv], (n >> 1) & 1, abort_flag);
+      const int first = first_unit(j);
+      for (int w = first; w < units && ok; ++w) {
+        ok = mbar_wait(&bar_q[ring], ring_phase, abort_flag);
+        if (ok && u > 0) ok = mbar_wait(bar_sfree, (u - 1) & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t kd = row_major + (HeadSmem::kK >> 4) + static_cast<uint32_t>(kv) * kP16;
+        const uint64_t vd = row_major + (HeadSmem::kV >> 4) + static_cast<uint32_t>(kv) * kP16;
+        const uint64_t qd = row_major + (HeadSmem::kQ >> 4) + static_cast<uint32_t>(ring) * kH16;
+        const uint64_t dod = row_major + (HeadSmem::kDO >> 4) + static_cast<uint32_t>(ring) * kH16;
+        if (leader) {
+#pragma unroll
+          for (int s = 0; s < 4; ++s) umma_bf16(tmem_base + cS, kd + 2 * s, qd + 2 * s, idesc_s, s != 0);
+#pragma unroll
+          for (int s = 0; s < 4; ++s) umma_bf16(tmem_base + cDP, vd + 2 * s, dod + 2 * s, idesc_s, s != 0);
+          umma_commit(bar_s);
+        }
+        if (u > 0) {
+          ok = mbar_wait(&bar_p[(u - 1) & 1], ((u - 1) >> 1) & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          issue_grads(u - 1, prev_ring, prev_kv, prev_w, prev_first, prev_pair);
+        }
+        prev_ring = ring;
+        prev_kv = kv;
+        prev_w = w;
+        prev_first = w == first;
+        prev_pair = pair;
+        if ((w & 1) || w == units - 1) pair ^= 1;
+        if (++ring == kRing) {
+          ring = 0;
+          ring_phase ^= 1;
+        }
+        ++u;
+      }
+      ++n;
+    }
+    if (ok && u > 0) {
+      ok = mbar_wait(&bar_p[(u - 1) & 1], ((u - 1) >> 1) & 1, abort_flag);
+      if (ok) {
+        tc_fence_after();
+        issue_grads(u - 1, prev_ring, prev_kv, prev_w, prev_first, prev_pair);
+      }
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) {
+      if (lane == 0) report_status(p.status, kStatusTimeoutMma, kKernelId, blockIdx.x, blockIdx.y);
+      *abort_flag = 1;
+    }
+  } else {
+    // ------------------------------ softmax / gradient warps ------------------------------
+    const int quarter = warp & 3, part = warp >> 2;  // 32 keys, 16 queries of each unit
+    const int r = quarter * 32 + lane;               // key row of the tile == TMEM lane
+    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    const bool has_bias = p.rel_bias != nullptr;
+    const bool want_drel = p.d_rel_bias != nullptr;
+    bool ok = true;
+
+    if (threadIdx.x < lq_pad) {
+      sLse[threadIdx.x] = -lse * kLog2e;
+      sQseg[threadIdx.x] = code;
+    }
+    // words[3], bit g: queries 16 g .. 16 g + 15 all exist, and none of them has all its keys hidden
+    const uint32_t good = __ballot_sync(0xffffffffu, threadIdx.x < p.Lq && lse * kLog2e >= -5e9f);
+    if (lane == 0)
+      atomicOr(&sWords[3], ((good & 0xffffu) == 0xffffu ? 1u << (2 * warp) : 0u) |
+                               ((good >> 16) == 0xffffu ? 2u << (2 * warp) : 0u));
+    if (has_bias) {
+      const float* tab = p.rel_bias + static_cast<long long>(h) * p.num_buckets;
+      if (threadIdx.x < kBuckets) sBucket[threadIdx.x] = 0.f;
+#pragma unroll
+      for (int c = 0; c < kRelRounds; ++c) {
+        const int t = threadIdx.x + c * kSoftmaxThreads;
+        if (t - lane < kMaxRel + 32) {  // (whole warps)
+          const int up = __shfl_up_sync(0xffffffffu, bucket[c], 1);
+          const uint32_t change = __ballot_sync(0xffffffffu, bucket[c] != (lane == 0 ? left[c] : up));
+          if (lane == 0) sChange[t >> 5] = change;
+          if (t < kMaxRel) {
+            sRel[t] = bucket[c] >= 0 ? __ldg(tab + bucket[c]) : 0.f;
+            sDRel[t] = 0.f;
+            sBucketAt[t] = static_cast<uint8_t>(bucket[c]);
+          }
+        }
+      }
+    }
+    for (int q0 = threadIdx.x >> 3; q0 < lq_pad; q0 += 4 * kRows) {
+      if (q0 >= 4 * kRows) request_rows(q0);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const __nv_bfloat162* px = reinterpret_cast<const __nv_bfloat162*>(&xo[c]);
+        const __nv_bfloat162* py = reinterpret_cast<const __nv_bfloat162*>(&xd[c]);
+        float s = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 fx = __bfloat1622float2(px[e]), fy = __bfloat1622float2(py[e]);
+          s += fx.x * fy.x + fx.y * fy.y;
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 4);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        const int q = q0 + c * kRows;
+        if (sub == 0 && q < lq_pad) sDelta[q] = -s;
+      }
+    }
+    softmax_bar_sync();
+    if (has_bias && threadIdx.x < kMaxRel / 16) {  // no change of bucket at t - 14 .. t + 31
+      const int t = threadIdx.x * 16 - 14;
+      bool flat = false;
+      if (t > 0 && t + 45 < rels) {
+        const uint32_t a = sChange[t >> 5], c = sChange[(t >> 5) + 1], d = sChange[(t >> 5) + 2];
+        flat = (__funnelshift_r(a, c, t & 31) | (__funnelshift_r(c, d, t & 31) & 0x3fffu)) == 0u;
+      }
+      sFlat[threadIdx.x] = flat ? sBucketAt[t + 14] : kMixed;
+    }
+    softmax_bar_sync();
+    const uint32_t counting = sWords[3];
+
+    // 16 columns of a row of an accumulator, in bf16, into a panel that a tensor copy stores
+    auto stage = [&](uint32_t col, uint8_t* panel, bool zero) {
+      uint32_t v[16];
+      tmem_ld16(t_row + col + part * 16, v);
+      tmem_ld_wait();
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        const uint32_t* x = v + 8 * g;
+        uint4 out;
+        out.x = pack_bf16x2(__uint_as_float(x[0]), __uint_as_float(x[1]));
+        out.y = pack_bf16x2(__uint_as_float(x[2]), __uint_as_float(x[3]));
+        out.z = pack_bf16x2(__uint_as_float(x[4]), __uint_as_float(x[5]));
+        out.w = pack_bf16x2(__uint_as_float(x[6]), __uint_as_float(x[7]));
+        if (zero) out = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(panel + r * 128 + (((part * 2 + g) ^ (r & 7)) << 4)) = out;
+      }
+    };
+    // dK and dV of the n-th key block walked, into the place of its K and V
+    auto stage_keys = [&](int n) {
+      stage(cDK, smem + HeadSmem::kK + (n & 1) * HeadSmem::kPanel, false);
+      stage(cDV, smem + HeadSmem::kV + (n & 1) * HeadSmem::kPanel, false);
+      tc_fence_before();
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_staged[n & 1]);
+    };
+    const bool prefix_lm = p.causal == 2;
+    const int seg_mask = prefix_lm ? 0x3fffffff : -1;
+    const bool simple_mask = !p.causal && p.kv_seg == nullptr;
+    const float inv_lk = 1.f / static_cast<float>(p.Lk);
+    const uint64_t log2e2 = pair_of(kLog2e, kLog2e);
+    // A block of 32 keys x 16 queries whose relative positions share one bucket takes its bias as one
+    // number and leaves its gradient as one sum per thread, kept until another bucket comes.
+    float flat_sum = 0.f;
+    int flat_bucket = kOutside;
+    auto flush_flat = [&]() {
+      const float s = warp_sum(flat_sum);
+      if (lane == 0 && flat_bucket < kBuckets) atomicAdd(sBucket + flat_bucket, s);
+      flat_sum = 0.f;
+    };
+    auto next_block = [&](int j) {  // the first key block from j on that is walked
+      while (j < nkb && ((idle >> j) & 1u)) {
+        for (int i = threadIdx.x; i < 128 * 8; i += kSoftmaxThreads) {
+          const int k = j * 128 + i / 8;
+          if (k < p.Lk) {
+            const long long off = b * p.dk_sb + static_cast<long long>(k) * p.dk_sl + h * p.dk_sh + i % 8 * 8;
+            *reinterpret_cast<uint4*>(p.dK + off) = make_uint4(0u, 0u, 0u, 0u);
+            *reinterpret_cast<uint4*>(p.dV + off) = make_uint4(0u, 0u, 0u, 0u);
+          }
+        }
+        ++j;
+      }
+      return j;
+    };
+    // this thread's key of a block: whether it counts, and its code
+    auto request_key = [&](int j, bool& vis, int& code) {
+      const int k = j * 128 + r;
+      const long long at = static_cast<long long>(b) * p.Lk + k;
+      vis = k < p.Lk && (p.key_mask == nullptr || p.key_mask[at] != 0);
+      code = (k < p.Lk && p.kv_seg) ? p.kv_seg[at] : 0;
+    };
+    int u = 0, pair = 0, n = 0;  // units walked, key blocks walked
+    int j = next_block(0), w = 0, next_j = nkb;
+    bool kvis = false, next_kvis = false;
+    int kcode = 0, next_kcode = 0;
+    uint32_t sv[16], dpv[16];
+    auto request_scores = [&](int unit) {
+      if (!mbar_wait_relaxed(bar_s, unit & 1, abort_flag)) return false;
+      tc_fence_after();
+      tmem_ld16(t_row + cS + part * 16, sv);
+      tmem_ld16(t_row + cDP + part * 16, dpv);
+      return true;
+    };
+    bool all_keys = false;  // of this warp's quarter of the block, all keys count
+    auto enter_block = [&]() {
+      w = first_unit(j);
+      kvis = next_kvis;
+      kcode = next_kcode;
+      all_keys = __all_sync(0xffffffffu, kvis);
+      next_j = next_block(j + 1);
+      if (next_j < nkb) request_key(next_j, next_kvis, next_kcode);
+    };
+    if (j < nkb) {
+      request_key(j, next_kvis, next_kcode);
+      enter_block();
+    }
+    while (j < nkb && ok) {
+      const int k = j * 128 + r;
+      const int first = first_unit(j);
+      const int q0 = w * 64 + part * 16;  // this thread's 16 queries
+      // which of them see this key
+      uint32_t mv = kvis ? 0xffffu : 0u;
+      bool all_seen = all_keys;
+      if (!simple_mask) {
+        if (p.kv_seg) {
+          const int kseg = kcode & seg_mask;
+          const bool k_pre = prefix_lm && ((kcode >> 30) & 1);
+          uint32_t m = 0u;
+#pragma unroll 4
+          for (int x = 0; x < 16; ++x) {
+            const int code = sQseg[q0 + x];
+            bool v = kseg == (code & seg_mask);
+            if (p.causal) v = v && (k <= q0 + x + p.causal_off || (k_pre && ((code >> 30) & 1)));
+            m |= (v ? 1u : 0u) << x;
+          }
+          mv &= m;
+        } else {
+          const int hidden = k - p.causal_off - q0;  // the first of them do not
+          mv &= hidden <= 0 ? 0xffffu : (hidden >= 16 ? 0u : 0xffffu << hidden);
+        }
+        all_seen = __all_sync(0xffffffffu, (mv & 0xffffu) == 0xffffu);
+      }
+      const bool fast = all_seen && ((counting >> (q0 >> 4)) & 1u);
+      // relative positions k - q of the warp's block: table indexes t0 - 15 .. t0 + 31
+      const int t0 = j * 128 + quarter * 32 - q0 + lq_pad;
+      const int flat = has_bias ? sFlat[t0 >> 4] : kOutside;
+
+      ok = request_scores(u);
+      if (!ok) break;
+      tmem_wait_into(sv, dpv);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_sfree);
+
+      float ds[16];
+      uint32_t pp[8], pd[8];  // P and dS as the MMAs read them
+      const float* rel = sRel + t0 + lane;  // rel[-x]
+      if (fast) {
+        const float one = has_bias ? sRel[t0] : 0.f;
+        const uint64_t b0 = pair_of(one, one);
+        // kEach: every score has a bias of its own
+        auto visible = [&](auto each) {
+          constexpr bool kEach = decltype(each)::value;
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {  // 16-byte broadcast loads of the per-query values
+            const ulonglong2 l2 = reinterpret_cast<const ulonglong2*>(sLse + q0)[g];
+            const ulonglong2 d2 = reinterpret_cast<const ulonglong2*>(sDelta + q0)[g];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int x = 4 * g + 2 * e;
+              uint64_t s = pair_of(__uint_as_float(sv[x]), __uint_as_float(sv[x + 1]));
+              s = add2(s, kEach ? pair_of(rel[-x], rel[-x - 1]) : b0);
+              s = fma2(s, log2e2, e ? l2.y : l2.x);
+              const float p0 = exp2f(low_of(s)), p1 = exp2f(high_of(s));
+              uint64_t dp = pair_of(__uint_as_float(dpv[x]), __uint_as_float(dpv[x + 1]));
+              dp = mul2(pair_of(p0, p1), add2(dp, e ? d2.y : d2.x));
+              ds[x] = low_of(dp);
+              ds[x + 1] = high_of(dp);
+              pp[x >> 1] = pack_bf16x2(p0, p1);
+              pd[x >> 1] = pack_bf16x2(ds[x], ds[x + 1]);
+            }
+          }
+        };
+        if (flat == kMixed)
+          visible(std::true_type());
+        else
+          visible(std::false_type());
+      } else {
+#pragma unroll
+        for (int x = 0; x < 16; x += 2) {
+          float e2[2];
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int xx = x + c;
+            float s = __uint_as_float(sv[xx]);
+            if (has_bias) s += rel[-xx];
+            s = ((mv >> xx) & 1u) ? s : kMaskValue;
+            const float nl = sLse[q0 + xx];
+            float e = exp2f(fmaf(s, kLog2e, nl));
+            // A row with every key masked has lse = -1e10 + log(Lk), which fp32 rounds to -1e10:
+            // its probabilities are uniform over the Lk keys.
+            if (nl > 5e9f) e = inv_lk;
+            if (k >= p.Lk || q0 + xx >= p.Lq) e = 0.f;
+            e2[c] = e;
+            ds[xx] = e * (__uint_as_float(dpv[xx]) + sDelta[q0 + xx]);
+          }
+          pp[x >> 1] = pack_bf16x2(e2[0], e2[1]);
+          pd[x >> 1] = pack_bf16x2(ds[x], ds[x + 1]);
+        }
+      }
+      // the products of unit u - 2 read these panels last (and dQ of the query block before the last)
+      if (u >= 2) {
+        ok = mbar_wait_relaxed(&bar_g[u & 1], ((u >> 1) - 1) & 1, abort_flag);
+        if (!ok) break;
+      }
+      uint8_t* pt = smem + HeadSmem::kP + (u & 1) * HeadSmem::kPanel + r * 128;
+      uint8_t* dst = smem + HeadSmem::kDS + (pair * 2 + (w & 1)) * HeadSmem::kPanel + r * 128;
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        const int at = ((part * 2 + g) ^ (r & 7)) << 4;
+        *reinterpret_cast<uint4*>(pt + at) = make_uint4(pp[4 * g], pp[4 * g + 1], pp[4 * g + 2], pp[4 * g + 3]);
+        *reinterpret_cast<uint4*>(dst + at) = make_uint4(pd[4 * g], pd[4 * g + 1], pd[4 * g + 2], pd[4 * g + 3]);
+      }
+      // dK and dV of the key block before: complete with the products of unit u - 1, read before those
+      // of this unit may start
+      if (w == first && n > 0) {
+        ok = mbar_wait_relaxed(&bar_g[(u - 1) & 1], ((u - 1) >> 1) & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        stage_keys(n - 1);
+      }
+      tc_fence_before();
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_p[u & 1]);
+
+      if ((w & 1) || w == units - 1) pair ^= 1;
+      ++u;
+      if (++w == units) {
+        j = next_j;
+        ++n;
+        if (j < nkb) enter_block();
+      }
+      if (want_drel) {
+        if (flat != kMixed) {
+          if (flat != flat_bucket) {
+            flush_flat();
+            flat_bucket = flat;
+          }
+          uint64_t s = pair_of(ds[0], ds[1]);
+#pragma unroll
+          for (int x = 2; x < 16; x += 2) s = add2(s, pair_of(ds[x], ds[x + 1]));
+          flat_sum += low_of(s) + high_of(s);
+        } else {
+          // dS[key r][query c] belongs to position r - c. Lane L collects the diagonals L and L - 32 of
+          // the warp's block: at column x it fetches the value of lane (L + x) mod 32.
+          float diag_pos[2] = {0.f, 0.f}, diag_neg[2] = {0.f, 0.f};
+#pragma unroll
+          for (int x = 0; x < 16; ++x) {
+            const float v = __shfl_sync(0xffffffffu, ds[x], lane + x);  // (modulo 32)
+            if (lane + x < 32) {
+              diag_pos[x & 1] += v;
+            } else {
+              diag_neg[x & 1] += v;
+            }
+          }
+          atomicAdd(sDRel + t0 + lane, diag_pos[0] + diag_pos[1]);
+          if (lane > 16) atomicAdd(sDRel + t0 + lane - 32, diag_neg[0] + diag_neg[1]);
+        }
+      }
+    }
+    if (ok && u > 0) {
+      ok = mbar_wait_relaxed(&bar_g[(u - 1) & 1], ((u - 1) >> 1) & 1, abort_flag);
+      if (ok) {
+        tc_fence_after();
+        stage_keys(n - 1);
+      }
+    }
+    if (ok) {
+      for (int i = 0; i < lq_pad / 128; ++i)
+        stage(cDQ + i * 64, smem + HeadSmem::kDS + i * HeadSmem::kPanel, u == 0);
+      tc_fence_before();
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_dq);
+      if (want_drel) {
+        flush_flat();
+        softmax_bar_sync();
+        // The relative positions are folded into their buckets here. Neighbouring positions share
+        // buckets: each run of equal buckets in a warp is summed by shuffles and added once.
+        float* out = p.d_rel_bias + static_cast<long long>(h) * p.num_buckets;
+        for (int t = threadIdx.x; t < rels; t += kSoftmaxThreads) {  // whole warps
+          float g = sDRel[t];
+          const int bucket = sBucketAt[t];
+          const int prev = __shfl_up_sync(0xffffffffu, bucket, 1);
+          const bool head = lane == 0 || prev != bucket;
+          const uint32_t heads = __ballot_sync(0xffffffffu, head);
+          const uint32_t later = lane == 31 ? 0u : heads >> (lane + 1);
+          const int run_end = later ? lane + __ffs(later) : 32;  // first lane of the next run
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const float v = __shfl_down_sync(0xffffffffu, g, o);
+            if (lane + o < run_end) g += v;
+          }
+          if (head && bucket < kBuckets && g != 0.f) atomicAdd(sBucket + bucket, g);
+        }
+        softmax_bar_sync();
+        for (int t = threadIdx.x; t < p.num_buckets; t += kSoftmaxThreads)
+          if (sBucket[t] != 0.f) atomicAdd(out + t, sBucket[t]);
+      }
+    } else if (lane == 0) {
+      report_status(p.status, kStatusTimeoutEpilogue, kKernelId, blockIdx.x, blockIdx.y);
+      *abort_flag = 1;
+    }
+  }
+  if (*abort_flag && threadIdx.x == 0)
+    for (int it = 0; it < 2000; ++it) __nanosleep(1000);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kMmaWarp) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+template <bool kAhead>
+int launch_head(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* tv, const CUtensorMap* tdo,
+                const CUtensorMap* tdq, const CUtensorMap* tdk, const CUtensorMap* tdv, const CUtensorMap* to,
+                const HeadParams& hp, cudaStream_t st) {
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!attr_set[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(attn_bwd_head_kernel<kAhead>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, HeadSmem::kTotal);
+    if (e != cudaSuccess) return set_error("attention_bwd_head attr: %s", cudaGetErrorString(e));
+    attr_set[dev] = true;
+  }
+  attn_bwd_head_kernel<kAhead>
+      <<<dim3(hp.a.H, hp.a.B), kThreads, HeadSmem::kTotal, st>>>(*tq, *tk, *tv, *tdo, *tdq, *tdk, *tdv, *to, hp);
+  count_launches(1);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return set_error("attention_bwd_head: %s", cudaGetErrorString(e));
+  return 0;
+}
+
+// Boxes of 64 channels x 64 positions of one head.
+bool half_map(CUtensorMap* map, const void* ptr, int B, int L, int H, long long sb, long long sl, long long sh) {
+  uint64_t dims[4] = {64, static_cast<uint64_t>(H), static_cast<uint64_t>(L), static_cast<uint64_t>(B)};
+  uint64_t strides[3] = {static_cast<uint64_t>(sh) * 2, static_cast<uint64_t>(sl) * 2,
+                         static_cast<uint64_t>(sb) * 2};
+  uint32_t box[4] = {64, 1, 64, 1};
+  return get_tensor_map(map, ptr, 2, 4, dims, strides, box, 1);
+}
+}  // namespace
+}  // namespace t5x
+
+using namespace t5x;
+
+// Whether t5x_attention_bwd_head takes these sizes and is the faster of the two backward kernels.
+T5X_API int t5x_attention_bwd_head_covers(int B, int H, int Lq, int Lk, int D, int num_buckets) {
+  if (D != 64 || B <= 0 || B > 65535 || H <= 0 || Lq <= 0 || Lq > kMaxQ || Lk <= 0 || Lk > kMaxKeys) return 0;
+  const int nkb = (Lk + 127) / 128, nq = (Lq + 127) / 128;
+  if (num_buckets > 0 && (num_buckets > kBuckets || (nkb + nq) * 128 > kMaxRel)) return 0;
+  // Thousands of cycles, measured: 14 for a CTA and 3 for each of its 128 x 64 units; the other kernel, with a
+  // CTA per key block, 14 and 7 for each 128 x 128 tile, and some 10 for its three further launches. (512 x
+  // 512, us, other / this: 16 x 6 heads 128 / 62, 74 heads even, 12 heads 27 / 58.)
+  const long long sms = num_sms(), heads = static_cast<long long>(B) * H;
+  const long long here = (heads + sms - 1) / sms * (14 + 3 * nkb * ((Lq + 63) / 64));
+  return here <= (heads * nkb + sms - 1) / sms * (14 + 7 * nq) + 10;
+}
+
+// q [B,Lq,H,64], k/v [B,Lk,H,64], o and d_o like q, bf16 with element strides (sb, sl, sh), innermost
+// contiguous; dq, dk and dv (the strides of dk) are written whole, in bf16. The rest as t5x_attention_bwd.
+T5X_API int t5x_attention_bwd_head(const void* q, const void* k, const void* v, const void* o, const void* d_o,
+                                   const void* lse, void* dq, void* dk, void* dv, int B, int H, int Lq, int Lk,
+                                   long long q_sb, long long q_sl, long long q_sh, long long k_sb,
+                                   long long k_sl, long long k_sh, long long v_sb, long long v_sl,
+                                   long long v_sh, long long o_sb, long long o_sl, long long o_sh,
+                                   long long do_sb, long long do_sl, long long do_sh, long long dq_sb,
+                                   long long dq_sl, long long dq_sh, long long dk_sb, long long dk_sl,
+                                   long long dk_sh, const void* rel_bias, const void* rel_bucket,
+                                   void* d_rel_bias, int num_buckets, int nrel, int rel_off,
+                                   const void* key_mask, const void* q_seg, const void* kv_seg, int causal,
+                                   int causal_off, void* stream) {
+  if (B <= 0 || H <= 0 || Lq <= 0 || Lk <= 0) return 0;
+  if (Lq > kMaxQ || Lk > kMaxKeys || B > 65535)
+    return set_error("attention_bwd_head: %d examples of %d queries and %d keys are not covered", B, Lq, Lk);
+  const int nkb = (Lk + 127) / 128, nq = (Lq + 127) / 128;
+  if (rel_bias != nullptr && (num_buckets > kBuckets || (nkb + nq) * 128 > kMaxRel))
+    return set_error("attention_bwd_head: %d buckets over %d + %d positions are not covered", num_buckets, Lq, Lk);
+  if ((do_sb | do_sl | do_sh | o_sb | o_sl | o_sh | dq_sb | dq_sl | dq_sh | dk_sb | dk_sl | dk_sh) & 7)
+    return set_error("attention_bwd_head: dO / O / dQ / dK strides must be multiples of 8 elements");
+  if (!aligned_to(16, {o, d_o, dq, dk, dv}))
+    return set_error("attention_bwd_head: O, dO and the gradients must be 16-byte aligned");
+  CUtensorMap tq, tk, tv, tdo, tdq, tdk, tdv, to;
+  if (!half_map(&tq, q, B, Lq, H, q_sb, q_sl, q_sh) || !bhld_map(&tk, k, B, Lk, H, k_sb, k_sl, k_sh) ||
+      !bhld_map(&tv, v, B, Lk, H, v_sb, v_sl, v_sh) || !half_map(&tdo, d_o, B, Lq, H, do_sb, do_sl, do_sh) ||
+      !half_map(&to, o, B, Lq, H, o_sb, o_sl, o_sh) || !bhld_map(&tdq, dq, B, Lq, H, dq_sb, dq_sl, dq_sh) || !bhld_map(&tdk, dk, B, Lk, H, dk_sb, dk_sl, dk_sh) ||
+      !bhld_map(&tdv, dv, B, Lk, H, dk_sb, dk_sl, dk_sh))
+    return -1;
+  HeadParams hp = {};
+  AttnParams& p = hp.a;
+  p.B = B; p.H = H; p.Lq = Lq; p.Lk = Lk;
+  p.rel_bias = static_cast<const float*>(rel_bias);
+  p.rel_bucket = static_cast<const int*>(rel_bucket);
+  p.num_buckets = num_buckets;
+  p.d_rel_bias = rel_bias != nullptr ? static_cast<float*>(d_rel_bias) : nullptr;
+  p.nrel = nrel; p.rel_off = rel_off;
+  p.key_mask = static_cast<const uint8_t*>(key_mask);
+  p.q_seg = static_cast<const int*>(q_seg);
+  p.kv_seg = static_cast<const int*>(kv_seg);
+  p.causal = causal; p.causal_off = causal_off;
+  p.lse = const_cast<float*>(static_cast<const float*>(lse));
+  p.dK = static_cast<__nv_bfloat16*>(dk);
+  p.dV = static_cast<__nv_bfloat16*>(dv);
+  p.dk_sb = dk_sb; p.dk_sl = dk_sl; p.dk_sh = dk_sh;
+  p.status = device_status_buffer();
+  hp.O = static_cast<const __nv_bfloat16*>(o);
+  hp.dO = static_cast<const __nv_bfloat16*>(d_o);
+  hp.o_sb = o_sb; hp.o_sl = o_sl; hp.o_sh = o_sh;
+  hp.do_sb = do_sb; hp.do_sl = do_sl; hp.do_sh = do_sh;
+  hp.ahead = num_sms();
+  const bool ahead = causal && Lq == Lk && causal_off == 0 && Lq > 128;
+  return (ahead ? launch_head<true> : launch_head<false>)(&tq, &tk, &tv, &tdo, &tdq, &tdk, &tdv, &to, hp,
+                                                          static_cast<cudaStream_t>(stream));
+}

@@ -29,6 +29,11 @@ native.register_signature("t5x_attention_fwd_stream", [c_void_p] * 5 + [c_int] *
                           [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
                            c_int, c_int, c_void_p])
 
+native.register_signature("t5x_attention_bwd_head", [c_void_p] * 9 + [c_int] * 4 + [c_ll] * 21 +
+                          [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
+                           c_void_p, c_int, c_int, c_void_p])
+native.register_signature("t5x_attention_bwd_head_covers", [c_int] * 6)
+
 # The short-range forward kernel keeps the scores of a whole key range in TMEM.
 CLASSIC_MAX_LK = 512
 CLASSIC_MAX_LQ = 512
@@ -145,21 +150,32 @@ class _FlashAttentionFn(torch.autograd.Function):
     B, Lq, H, D = q.shape
     Lk = k.shape[1]
     do = do if _strides_ok(do) else do.contiguous()
-    dq32 = torch.zeros((B, Lq, H, D), dtype=torch.float32, device=q.device)
+    nb, nrel = _bias_sizes(rel_bias, buckets)
+    head = bool(native.lib().t5x_attention_bwd_head_covers(B, H, Lq, Lk, D, nb))
     if packed:
       dqkv = torch.empty((B, Lq, 3, H, D), dtype=torch.bfloat16, device=q.device)
       dq, dk, dv = dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]
     else:
       dk = torch.empty((B, Lk, H, D), dtype=torch.bfloat16, device=q.device)
       dv = torch.empty((B, Lk, H, D), dtype=torch.bfloat16, device=q.device)
+    tail = (native.ptr(rel_bias), native.ptr(buckets), native.ptr(d_rel), nb, nrel, rel_off,
+            native.ptr(key_mask), native.ptr(q_seg), native.ptr(kv_seg), int(causal), causal_off,
+            native.stream_ptr())
+    if head:
+      if not packed:
+        dq = torch.empty((B, Lq, H, D), dtype=torch.bfloat16, device=q.device)
+      rc = native.lib().t5x_attention_bwd_head(
+          q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
+          dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Lq, Lk, *_sbh(q), *_sbh(k), *_sbh(v),
+          *_sbh(o), *_sbh(do), *_sbh(dq), *_sbh(dk), *tail)
+      native._check(rc, "attention_bwd")
+      return dq, dk, dv, ret_rel, None, None, None, None, None, None, None
+    dq32 = torch.zeros((B, Lq, H, D), dtype=torch.float32, device=q.device)
     delta = torch.empty((B, H, Lq), dtype=torch.float32, device=q.device)
-    nb, nrel = _bias_sizes(rel_bias, buckets)
     rc = native.lib().t5x_attention_bwd(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
         delta.data_ptr(), dq32.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Lq, Lk, D,
-        *_sbh(q), *_sbh(k), *_sbh(v), *_sbh(o), *_sbh(do), *_sbh(dk), native.ptr(rel_bias),
-        native.ptr(buckets), native.ptr(d_rel), nb, nrel, rel_off, native.ptr(key_mask),
-        native.ptr(q_seg), native.ptr(kv_seg), int(causal), causal_off, native.stream_ptr())
+        *_sbh(q), *_sbh(k), *_sbh(v), *_sbh(o), *_sbh(do), *_sbh(dk), *tail)
     native._check(rc, "attention_bwd")
     if packed:
       dq.copy_(dq32)

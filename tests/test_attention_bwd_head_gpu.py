@@ -1,0 +1,93 @@
+"""The backward kernel that keeps dQ of a head in TMEM, at the edges of its units of 64 queries and blocks of
+128 keys, under every kind of mask, against float64 (the entry point is called as it is: by itself the choice
+of the kernel goes by the number of heads)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _call(q, k, v, o, do, lse, table, lq, lk, key_mask, qs, ks, mode):
+  from t5x_b200.ops import attention as A, native
+  b, h = q.shape[0], q.shape[2]
+  dq, dk, dv = (torch.full_like(t, 7.0) for t in (q, k, v))
+  buckets = d_table = None
+  if table is not None:
+    buckets = A._rel_buckets(lq, lk, 0, mode == 0, 32, 128, q.device)
+    d_table = torch.zeros_like(table)
+  nb, nrel = A._bias_sizes(table, buckets)
+  p = native.ptr
+  native._check(native.lib().t5x_attention_bwd_head(
+      *(t.data_ptr() for t in (q, k, v, o, do, lse, dq, dk, dv)), b, h, lq, lk,
+      *(s for t in (q, k, v, o, do, dq, dk) for s in A._sbh(t)), p(table), p(buckets), p(d_table), nb, nrel,
+      lq - 1, p(key_mask), p(qs), p(ks), mode, lk - lq if mode else 0, native.stream_ptr()), "head")
+  native.check_status()
+  return dq, dk, dv, d_table
+
+
+@pytest.mark.parametrize("mask", ["none", "padded", "unseen", "causal", "packed", "prefix"])
+@pytest.mark.parametrize("lq,lk,bias", [(1, 1, True), (31, 129, False), (64, 128, True), (65, 257, True),
+                                        (129, 129, True), (200, 200, False), (512, 512, True),
+                                        (511, 640, True), (130, 1100, False)])
+def test_against_float64(lq, lk, bias, mask):
+  from t5x_b200.ops import attention as A, reference as ref
+  if mask in ("causal", "packed", "prefix") and lq != lk:
+    pytest.skip("self-attention")
+  g = torch.Generator(device="cuda").manual_seed(lq + lk)
+  b, h = 3, 2
+  rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+  q = (rnd(b, lq, h, 64) * 0.3).bfloat16()
+  k, v, do = rnd(b, lk, h, 64).bfloat16(), rnd(b, lk, h, 64).bfloat16(), rnd(b, lq, h, 64).bfloat16()
+  table = rnd(h, 32) if bias else None
+  pos = torch.arange(lk, device="cuda")
+  km = seg = None
+  mode, kw, allowed = 0, {}, torch.ones(b, lq, lk, dtype=torch.bool, device="cuda")
+  if mask in ("padded", "unseen"):
+    km = torch.ones(b, lk, dtype=torch.bool, device="cuda")
+    km[1, max(1, lk // 3):] = False
+    if mask == "unseen":
+      km[2] = False  # an example in which no query sees a key: uniform rows
+    allowed = allowed & km[:, None]
+    kw = dict(key_mask=km)
+  elif mask != "none":
+    mode, allowed = 1, allowed & (pos[None] <= pos[:, None])
+    kw = dict(causal=True)
+    if mask == "packed":
+      seg = (pos // 70 + 1).int()[None].expand(b, lk).contiguous()
+      allowed = allowed & (seg[:, :, None] == seg[:, None])
+      kw = dict(causal=True, q_segment_ids=seg, kv_segment_ids=seg)
+    if mask == "prefix":
+      inside = pos[None] < torch.tensor([lk // 3, 0, lk], device="cuda")[:, None]
+      prefix = ref.PrefixLMMask(inside, torch.ones_like(inside), None)
+      mode, allowed, kw = 2, prefix.bool()[:, 0], dict(prefix_lm=prefix)
+  prep = A.prepare(lq, lk, h, q.device, table, mode == 0, 32, 128, kw.get("key_mask"),
+                   kw.get("causal", False), seg, seg, 0, kw.get("prefix_lm"))
+  q2, k2, v2 = (t.double().requires_grad_() for t in (q, k, v))
+  s = torch.einsum("bqhd,bkhd->bhqk", q2, k2)
+  leaves = [q2, k2, v2]
+  if bias:
+    t2 = table.double().requires_grad_()
+    leaves.append(t2)
+    rel = pos[None] - torch.arange(lq, device="cuda")[:, None]
+    s = s + t2[:, ref.relative_position_bucket(rel, mode == 0, 32, 128)][None]
+  # the mask is an addition to the scores: it hides them, and hands on their gradients
+  s = s + torch.where(allowed[:, None], 0.0, -1e10 - s.detach())
+  probs = torch.softmax(s, -1)
+  want = torch.autograd.grad(torch.einsum("bhqk,bkhd->bqhd", probs, v2), leaves, do.double())
+  o = torch.einsum("bhqk,bkhd->bqhd", probs, v2).detach().bfloat16()
+  lse = torch.logsumexp(s, -1).detach().float().contiguous()
+  got = _call(q, k, v, o, do, lse, table, lq, lk, prep[2], prep[3], prep[4], mode)
+  # P, dS and the results are each rounded to bf16 once, and rowsum(dO * O) takes a rounded O. (Of a single
+  # key dq, dk and dbias are zero; dS is then the rounding of two equal 32-bit sums of 64 products, up to
+  # 64 * 2^-24 * |dO| |v| or 1e-4 with norms of 8.)
+  for name, a, w in zip(("dq", "dk", "dv", "dbias"), got, want):
+    assert float((a.double() - w).norm() / (w.norm() + 1e-2)) < 4 * 2.0 ** -8, name
+
+
+def test_both_kernels_are_reached():
+  from t5x_b200.ops import native
+  covers = native.lib().t5x_attention_bwd_head_covers
+  assert covers(128, 12, 512, 512, 64, 32) and covers(8, 6, 64, 64, 64, 32) and covers(64, 12, 114, 512, 64, 0)
+  assert not covers(1, 12, 512, 512, 64, 32)  # too few CTAs
+  assert not covers(128, 12, 513, 512, 64, 32) and not covers(128, 12, 512, 512, 128, 32)
+  assert not covers(128, 12, 512, 700, 64, 32) and not covers(128, 12, 512, 512, 64, 300)
