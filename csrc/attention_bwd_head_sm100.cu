@@ -68,27 +68,6 @@ struct HeadParams {
   int ahead;  // CTAs that run at a time
 };
 
-__device__ __forceinline__ uint64_t pair_of(float a, float b) {
-  return static_cast<uint64_t>(__float_as_uint(a)) | (static_cast<uint64_t>(__float_as_uint(b)) << 32);
-}
-__device__ __forceinline__ float low_of(uint64_t v) { return __uint_as_float(static_cast<uint32_t>(v)); }
-__device__ __forceinline__ float high_of(uint64_t v) { return __uint_as_float(static_cast<uint32_t>(v >> 32)); }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-
 // Waits for the loads from TMEM into these registers.
 __device__ __forceinline__ void tmem_wait_into(uint32_t (&a)[16], uint32_t (&c)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;"
@@ -819,15 +798,6 @@ int launch_head(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap*
   if (e != cudaSuccess) return set_error("attention_bwd_head: %s", cudaGetErrorString(e));
   return 0;
 }
-
-// Boxes of 64 channels x 64 positions of one head.
-bool half_map(CUtensorMap* map, const void* ptr, int B, int L, int H, long long sb, long long sl, long long sh) {
-  uint64_t dims[4] = {64, static_cast<uint64_t>(H), static_cast<uint64_t>(L), static_cast<uint64_t>(B)};
-  uint64_t strides[3] = {static_cast<uint64_t>(sh) * 2, static_cast<uint64_t>(sl) * 2,
-                         static_cast<uint64_t>(sb) * 2};
-  uint32_t box[4] = {64, 1, 64, 1};
-  return get_tensor_map(map, ptr, 2, 4, dims, strides, box, 1);
-}
 }  // namespace
 }  // namespace t5x
 
@@ -870,9 +840,9 @@ T5X_API int t5x_attention_bwd_head(const void* q, const void* k, const void* v, 
   if (!aligned_to(16, {o, d_o, dq, dk, dv}))
     return set_error("attention_bwd_head: O, dO and the gradients must be 16-byte aligned");
   CUtensorMap tq, tk, tv, tdo, tdq, tdk, tdv, to;
-  if (!half_map(&tq, q, B, Lq, H, q_sb, q_sl, q_sh) || !bhld_map(&tk, k, B, Lk, H, k_sb, k_sl, k_sh) ||
-      !bhld_map(&tv, v, B, Lk, H, v_sb, v_sl, v_sh) || !half_map(&tdo, d_o, B, Lq, H, do_sb, do_sl, do_sh) ||
-      !half_map(&to, o, B, Lq, H, o_sb, o_sl, o_sh) || !bhld_map(&tdq, dq, B, Lq, H, dq_sb, dq_sl, dq_sh) || !bhld_map(&tdk, dk, B, Lk, H, dk_sb, dk_sl, dk_sh) ||
+  if (!bhld_map(&tq, q, B, Lq, H, q_sb, q_sl, q_sh, 64, 64) || !bhld_map(&tk, k, B, Lk, H, k_sb, k_sl, k_sh) ||
+      !bhld_map(&tv, v, B, Lk, H, v_sb, v_sl, v_sh) || !bhld_map(&tdo, d_o, B, Lq, H, do_sb, do_sl, do_sh, 64, 64) ||
+      !bhld_map(&to, o, B, Lq, H, o_sb, o_sl, o_sh, 64, 64) || !bhld_map(&tdq, dq, B, Lq, H, dq_sb, dq_sl, dq_sh) || !bhld_map(&tdk, dk, B, Lk, H, dk_sb, dk_sl, dk_sh) ||
       !bhld_map(&tdv, dv, B, Lk, H, dk_sb, dk_sl, dk_sh))
     return -1;
   HeadParams hp = {};

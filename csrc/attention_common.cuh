@@ -1,5 +1,6 @@
-// Declarations shared by the attention kernels (attention_sm100.cu: forward for short key
-// ranges and the backward pass; attention_fwd_sm100.cu: the streaming forward pass).
+// Declarations shared by the attention kernels: forward, attention_fwd_rows_sm100.cu (64 channels, up to 2048
+// keys) and attention_fwd_sm100.cu (any length, 64 or 128 channels); backward, attention_bwd_head_sm100.cu (64
+// channels, up to 512 queries) and attention_sm100.cu.
 #pragma once
 #include "common.cuh"
 
@@ -65,8 +66,6 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 //                that bound 8 x 32 x 256 72 / 77).
 //   kLookNone    Everything else, in a variant of its own: the look-up at run time cost it 2 to 5 % (8 x 32
 //                heads of 128 x 256, causal, 61.4 / 64.3).
-// (The short-range kernel walks all of its four blocks: with a number of blocks known only then it lost
-// 8 % where none is hidden and gained 1 % where some are.)
 enum KeyLook : int { kLookNone = 0, kLookMask = 1, kLookCausal = 2 };
 __host__ __device__ __forceinline__ bool key_mask_alone(const AttnParams& p) {
   return p.key_mask != nullptr && !p.causal && p.kv_seg == nullptr;
@@ -198,15 +197,47 @@ __device__ __forceinline__ void store16_bf16(__nv_bfloat16* dst, const uint32_t 
 }
 
 
+// Two fp32 values in one register pair and the arithmetic on both at once (each rounded as by itself).
+__device__ __forceinline__ uint64_t pair_of(float a, float b) {
+  return static_cast<uint64_t>(__float_as_uint(a)) | (static_cast<uint64_t>(__float_as_uint(b)) << 32);
+}
+__device__ __forceinline__ float low_of(uint64_t v) { return __uint_as_float(static_cast<uint32_t>(v)); }
+__device__ __forceinline__ float high_of(uint64_t v) { return __uint_as_float(static_cast<uint32_t>(v >> 32)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+      :
+      : "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+      : "memory");
+}
+
 // Tensor map over a [B, L, H, D] bf16 tensor with element strides (sb, sl, sh): boxes of
-// 64 channels x 128 positions of one head (one 128-byte-swizzled shared-memory panel).
+// 64 channels x 128 (or `rows`) positions of one head (one 128-byte-swizzled shared-memory panel).
 inline bool bhld_map(CUtensorMap* map, const void* ptr, int B, int L, int H, long long sb, long long sl,
-                     long long sh, int D = kAttnD) {
+                     long long sh, int D = kAttnD, uint32_t rows = 128) {
   uint64_t dims[4] = {static_cast<uint64_t>(D), static_cast<uint64_t>(H),
                       static_cast<uint64_t>(L), static_cast<uint64_t>(B)};
   uint64_t strides[3] = {static_cast<uint64_t>(sh) * 2, static_cast<uint64_t>(sl) * 2,
                          static_cast<uint64_t>(sb) * 2};
-  uint32_t box[4] = {64, 1, 128, 1};
+  uint32_t box[4] = {64, 1, rows, 1};
   return get_tensor_map(map, ptr, 2, 4, dims, strides, box, 1);
 }
 

@@ -34,19 +34,18 @@ native.register_signature("t5x_attention_bwd_head", [c_void_p] * 9 + [c_int] * 4
                            c_void_p, c_int, c_int, c_void_p])
 native.register_signature("t5x_attention_bwd_head_covers", [c_int] * 6)
 
-# The short-range forward kernel keeps the scores of a whole key range in TMEM.
-CLASSIC_MAX_LK = 512
-CLASSIC_MAX_LQ = 512
+# The forward kernel for head_dim 64 keeps the bias by relative position of all keys in shared memory.
+CLASSIC_MAX_LK = 2048
 # The backward kernel keeps bias-gradient bins for the whole query range in shared memory.
 BWD_MAX_LQ = 4096
 
 
 def forward_kernel(Lq: int, Lk: int, D: int, prefix_lm: bool = False) -> str:
-  """'classic' (head_dim 64, up to 512 x 512 keys, scores of the whole key range in TMEM: the
-  faster of the two on the shapes it covers) or 'stream' (any length, head_dim 64 or 128,
-  prefix-LM masks). `T5X_B200_ATTN_FWD=stream` forces the streaming kernel everywhere."""
+  """'classic' (csrc/attention_fwd_rows_sm100.cu: head_dim 64, up to 2048 keys; the faster of the two on
+  the shapes it covers) or 'stream' (any length, head_dim 64 or 128). `T5X_B200_ATTN_FWD=stream` forces
+  the streaming kernel everywhere."""
   import os
-  classic_ok = D == 64 and Lq <= CLASSIC_MAX_LQ and Lk <= CLASSIC_MAX_LK and not prefix_lm
+  classic_ok = D == 64 and Lk <= CLASSIC_MAX_LK
   want = os.environ.get("T5X_B200_ATTN_FWD", "classic")
   return "classic" if (classic_ok and want == "classic") else "stream"
 
