@@ -1,3 +1,4 @@
+import gc
 import os
 import sys
 
@@ -16,3 +17,11 @@ def _reset_parallel_state():
   pstate.reset()
   yield
   pstate.reset()
+
+
+@pytest.fixture(autouse=True, scope="module")
+def _no_garbage_of_other_modules():
+  """Decoders and optimizers of earlier tests hold device memory in reference cycles; freed in the middle of
+  a test that measures what is allocated, they change its figure."""
+  gc.collect()
+  yield
