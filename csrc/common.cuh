@@ -411,6 +411,15 @@ __device__ __forceinline__ float gelu_tanh_grad(float x) {
   return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * du;
 }
 
+// gelu(x) as above, and its derivative h + 2 x h (1 - h) u'(x) with h = (1 + tanh u) / 2, in nine operations.
+__device__ __forceinline__ void gelu_tanh_both(float x, float& y, float& dy) {
+  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  const float x2 = x * x;
+  const float h = fmaf(0.5f, tanhf(x * fmaf(k0 * k1, x2, k0)), 0.5f);
+  y = x * h;
+  dy = fmaf(fmaf(-h, y, y), fmaf(6.f * k0 * k1, x2, 2.f * k0), h);
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -31,6 +31,9 @@ enum GemmEpilogue : int {
   // The product is a logits matrix that is consumed in the epilogue and never stored:
   kEpiCeStats = 3,  // per (row, column tile) softmax partials for the cross-entropy forward
   kEpiCeGrad = 4,   // gradient of the cross-entropy w.r.t. the logits, written as bf16
+  // The product is the gradient of gelu(h0) * h1 and never stored either: h0 and h1 (in H0 and H1) become
+  // their gradients.
+  kEpiGatedGrad = 5,
 };
 
 // Several products in one launch, three at most (the projections that share an input).
@@ -59,7 +62,7 @@ struct GemmParams {
   long long ldc, c_batch_stride;  // elements
   const __nv_bfloat16* R;         // residual (bf16), same shape as C
   long long ldr, r_batch_stride;
-  __nv_bfloat16* H0;  // gated-GELU: optional copies of the two pre-activations
+  __nv_bfloat16* H0;  // gated GELU: optional copies of the two pre-activations; its gradient: in and out
   __nv_bfloat16* H1;
   long long ldh, h_batch_stride;
   float alpha;
@@ -543,6 +546,81 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, const Ge
       }
     }
   }
+}
+
+// Epilogue of the gradient of gelu(h0) * h1 (kEpiGatedGrad): the accumulator holds dg; 32 columns at a time h0 and
+// h1 come in, and dg h1 gelu'(h0) and dg gelu(h0) go out in their place, rows 64 bytes at a time through the
+// warp's staging block. `GatedRows` holds a block that is on its way: two of them are, across the ends of tiles
+// (one of them within a tile: 335 us below; the reads wait for memory, the arithmetic costs nothing).
+//
+// As a pass of its own this reads dg, h0 and h1 and writes two of them, at the rate of memory; here two fifths of
+// that traffic are gone and the rest runs under the MMAs of other tiles (us, product and pass / in one: 65536 x
+// 768 x 2048 415 / 324, 14592 x 768 x 2048 101 / 92, 16384 x 4096 x 10240 1380 / 1100, 16384 x 1472 x 3584
+// 332 / 250, 3024 x 1472 x 3584 80 / 70). With K = 768 the epilogue is the slower side, by its traffic.
+struct GatedRows {
+  uint4 h0[4], h1[4];
+};
+__device__ __forceinline__ void gated_request(const GemmParams& p, int first_row, int col, int rows_valid, int lane,
+                                              GatedRows& in) {
+  const long long at = static_cast<long long>(first_row + (lane >> 2)) * p.ldh + col + (lane & 3) * 8;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    in.h0[j] = in.h1[j] = make_uint4(0u, 0u, 0u, 0u);
+    if (j * 8 + (lane >> 2) < rows_valid) {
+      in.h0[j] = ld_chained(reinterpret_cast<const uint4*>(p.H0 + at + j * 8 * p.ldh));
+      in.h1[j] = ld_chained(reinterpret_cast<const uint4*>(p.H1 + at + j * 8 * p.ldh));
+    }
+  }
+}
+// One block: 32 accumulator columns from t_cols on, columns col.. of the rows from first_row on. `next` requests what
+// is to take the place of `in`.
+template <typename Next>
+__device__ __forceinline__ void gated_block(const GemmParams& p, uint32_t t_cols, int first_row, int col, int lane,
+                                            float* stage, GatedRows& in, Next next) {
+  const int rows_valid = p.M - first_row;
+  uint4* st4 = reinterpret_cast<uint4*>(stage);  // 32 rows of 8 pieces: 0..3 h0, 4..7 h1, exchanged by row
+  uint32_t r[32];
+  tmem_ld32(t_cols, r);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int row = j * 8 + (lane >> 2);
+    st4[row * 8 + ((lane & 3) ^ (row & 7))] = in.h0[j];
+    st4[row * 8 + (((lane & 3) + 4) ^ (row & 7))] = in.h1[j];
+  }
+  __syncwarp();
+  next();
+  tmem_ld_wait();
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {  // eight columns of this lane's row
+    uint4& u0 = st4[lane * 8 + (k ^ (lane & 7))];
+    uint4& u1 = st4[lane * 8 + ((k + 4) ^ (lane & 7))];
+    uint4 a = u0, b = u1;
+    __nv_bfloat162* ha = reinterpret_cast<__nv_bfloat162*>(&a);
+    __nv_bfloat162* hb = reinterpret_cast<__nv_bfloat162*>(&b);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 x = __bfloat1622float2(ha[e]), y = __bfloat1622float2(hb[e]);
+      const float g0 = __uint_as_float(r[k * 8 + e * 2]), g1 = __uint_as_float(r[k * 8 + e * 2 + 1]);
+      float v0, v1, d0, d1;
+      gelu_tanh_both(x.x, v0, d0);
+      gelu_tanh_both(x.y, v1, d1);
+      ha[e] = __floats2bfloat162_rn(g0 * y.x * d0, g1 * y.y * d1);
+      hb[e] = __floats2bfloat162_rn(g0 * v0, g1 * v1);
+    }
+    u0 = a;
+    u1 = b;
+  }
+  __syncwarp();
+  const long long at = static_cast<long long>(first_row + (lane >> 2)) * p.ldh + col + (lane & 3) * 8;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int row = j * 8 + (lane >> 2);
+    if (row < rows_valid) {
+      *reinterpret_cast<uint4*>(p.H0 + at + j * 8 * p.ldh) = st4[row * 8 + ((lane & 3) ^ (row & 7))];
+      *reinterpret_cast<uint4*>(p.H1 + at + j * 8 * p.ldh) = st4[row * 8 + (((lane & 3) + 4) ^ (row & 7))];
+    }
+  }
+  __syncwarp();  // the block may be overwritten
 }
 
 // Cross-entropy forward epilogue of kCeTileCols columns (part `part` of the tile) of an

@@ -415,6 +415,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
                                     (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
     const uint32_t drained = mapa_shared(smem_u32(&tmem_empty[0]), 0);
     GemmWork work(p, pair, num_pairs, total_tiles, num_kb);
+    // kEpiGatedGrad: the blocks of this warp's walk over its tiles, two of them requested ahead
+    GemmWork fetch(p, pair, num_pairs, total_tiles, num_kb);
+    GatedRows ahead0, ahead1;
+    int fetch_row = 0, fetch_col = 0, fetch_left = 0;
+    bool odd = false;
+    auto gated_blocks = [&](int n0) {  // of this warp's half of a tile's columns (N is a multiple of 32)
+      return max(0, min(BN / 64, (p.N - n0 - part * (BN / 2)) / 32));
+    };
+    auto request = [&](GatedRows& in) {
+      while (fetch_left == 0) {
+        int tile, kb0, kb1, fb, fm, fn;
+        if (!fetch.next(tile, kb0, kb1)) return;
+        gemm_tile_coords(p, tile, tiles_per_batch, fb, fm, fn);
+        fetch_row = fm * (2 * kBM) + static_cast<int>(cta) * kBM + q * 32;
+        fetch_col = fn * kTileN + part * (BN / 2);
+        fetch_left = gated_blocks(fn * kTileN);
+      }
+      gated_request(p, fetch_row, fetch_col, p.M - fetch_row, lane, in);
+      fetch_col += 32;
+      --fetch_left;
+    };
+    if (EPI == kEpiGatedGrad) {
+      request(ahead0);
+      request(ahead1);
+    }
     for (int tile, kb0, kb1; ok && work.next(tile, kb0, kb1); ++local) {
       const int acc = local & 1;
       const uint32_t acc_phase = (local >> 1) & 1;
@@ -436,7 +461,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<MODE>()
       if (MODE == kTpReduceScatter)
         gemm_epilogue_tile_rs<BN, EPI>(p, tp, t_row, m0, n0, q, lane,
                                        staging + (warp - 2) * kRsStageBytesPerWarp);
-      else if (EPI == kEpiCeStats)
+      else if (EPI == kEpiGatedGrad) {
+        float* block = reinterpret_cast<float*>(staging + (warp - 2) * kEpiStageBytesPerWarp);
+        for (int c = 0, n = gated_blocks(n0); c < n; ++c, odd = !odd) {
+          const uint32_t t_cols = t_row + part * (BN / 2) + c * 32;
+          const int col = n0 + part * (BN / 2) + c * 32;
+          if (odd)
+            gated_block(p, t_cols, m0 + q * 32, col, lane, block, ahead1, [&] { request(ahead1); });
+          else
+            gated_block(p, t_cols, m0 + q * 32, col, lane, block, ahead0, [&] { request(ahead0); });
+        }
+      } else if (EPI == kEpiCeStats)
         gemm_epilogue_ce_stats<BN>(p, t_row, m0, n0, q, part, lane);
       else if (EPI == kEpiCeGrad)
         gemm_epilogue_ce_grad<BN, 2>(
@@ -544,6 +579,9 @@ static int launch_pair_mode(int epilogue, const GemmMaps<false>& maps, GemmParam
     case kEpiCeGrad:
       if (MODE != kTpNone) break;
       return launch_pair<kEpiCeGrad, kTpNone>(maps, p, tp, max_ctas, stream);
+    case kEpiGatedGrad:
+      if (MODE != kTpNone) break;
+      return launch_pair<kEpiGatedGrad, kTpNone>(maps, p, tp, max_ctas, stream);
     default:
       break;
   }

@@ -539,6 +539,11 @@ static int gemm_impl(const void* A, const void* B, const void* B2, void* C, int 
     return epilogue == kEpiCeStats ? launch_gemm<256, kEpiCeStats>(maps, p, max_ctas, st)
                                    : launch_gemm<256, kEpiCeGrad>(maps, p, max_ctas, st);
   }
+  if (epilogue == kEpiGatedGrad) {
+    p.tiles_m = pair_tiles_m;
+    p.tiles_n = (N + 255) / 256;
+    return launch_gemm_pair(epilogue, maps, p, max_ctas, st);
+  }
   if (epilogue == kEpiGatedGelu) {
     if (out_fp32 || accumulate) return set_error("gated-GELU epilogue writes bf16 without accumulate");
     if (!operand_map(&maps.b[1], B2, b_mn_major, N, K, ldb, b_batch_stride, batch, 128)) return -1;
@@ -954,4 +959,23 @@ T5X_API int t5x_gemm_ce_grad(const void* A, const void* B, void* dlogits, long l
                            alpha, 0, stream, nullptr, 0);
   g_ce_extras = nullptr;
   return rc;
+}
+
+// Whether t5x_gemm_gated_grad takes these sizes: whole 32-column blocks, and tiles for most of the CTA pairs.
+T5X_API int t5x_gemm_gated_grad_covers(int M, int N) {
+  using namespace t5x;
+  const long long tiles = ((M + 2 * kBM - 1ll) / (2 * kBM)) * ((N + 255) / 256);
+  return gemm_pair_mode() != 0 && M >= 2 * kBM && N >= 256 && N % 32 == 0 && tiles >= num_sms() / 4;
+}
+
+// Gradient of gelu(h0) * h1 from that of its product with a matrix: with dg = dy[M, K] @ B[K, N] (which is not
+// stored), h0 <- dg h1 gelu'(h0) and h1 <- dg gelu(h0), bf16, rows ldh elements apart.
+T5X_API int t5x_gemm_gated_grad(const void* dy, const void* B, void* h0, void* h1, int M, int N, int K,
+                                long long ld_dy, long long ldb, long long ldh, int b_mn_major, void* stream) {
+  using namespace t5x;
+  if (M <= 0 || N <= 0) return 0;
+  if (N % 32 || ldh % 8) return set_error("gemm_gated_grad: N and ldh must be multiples of 32 and 8");
+  if (!aligned_to(16, {h0, h1})) return set_error("gemm_gated_grad: pointers must be 16-byte aligned");
+  return gemm_impl(dy, B, nullptr, nullptr, M, N, K, 1, ld_dy, ldb, N, 0, 0, 0, 0, b_mn_major, 0, 0,
+                   kEpiGatedGrad, nullptr, 0, 0, h0, h1, ldh, 1.f, 0, stream, nullptr, 0);
 }

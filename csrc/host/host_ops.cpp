@@ -639,13 +639,22 @@ Tensor mlp_block_bwd(const Tensor& dy, const Tensor& x, const Tensor& scale,
   void* st = stream_of();
   const int64_t m = rows_of(x), d = x.size(-1);
   const Weight a(weights[0], d), b(weights[1], d), wo(weights[2], a.n);
-  Tensor dg = at::empty_like(g);
+  const bool fused = t5x_gemm_gated_grad_covers(m, a.n) != 0;
+  Tensor dg;
+  if (!fused) dg = at::empty_like(g);
   optional<Tensor> dh = at::empty_like(x);  // what can run out of memory comes before `pre` is overwritten
-  input_grad(dy.data_ptr(), wo.n, m, wo, dg, false, st);
+  char* d0 = static_cast<char*>(pre.data_ptr());
   Tensor gwo = grads[2];
-  weight_grad(g, dy.data_ptr(), wo.n, m, wo, gwo, accumulate[2], st);
-  check(t5x_gated_gelu_bwd(dg.data_ptr(), pre.data_ptr(), m, a.n, 2 * a.n, a.n, 0, st), "gated_gelu_bwd");
-  const char* d0 = static_cast<const char*>(pre.data_ptr());
+  if (fused) {
+    weight_grad(g, dy.data_ptr(), wo.n, m, wo, gwo, accumulate[2], st);
+    check(t5x_gemm_gated_grad(dy.data_ptr(), wo.t.data_ptr(), d0, d0 + a.n * 2, m, a.n, wo.n, wo.n, wo.ld, 2 * a.n,
+                              0, st),
+          "gemm_gated_grad");
+  } else {
+    input_grad(dy.data_ptr(), wo.n, m, wo, dg, false, st);
+    weight_grad(g, dy.data_ptr(), wo.n, m, wo, gwo, accumulate[2], st);
+    check(t5x_gated_gelu_bwd(dg.data_ptr(), pre.data_ptr(), m, a.n, 2 * a.n, a.n, 0, st), "gated_gelu_bwd");
+  }
   backward_products(h, m, {d0, d0 + a.n * 2}, {2 * a.n, 2 * a.n}, {a, b}, dh, {grads[0], grads[1]},
                     {accumulate[0], accumulate[1]}, st);
   return norm_backward(*dh, x, scale, rstd, dy, dscale, st);
