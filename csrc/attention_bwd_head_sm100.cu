@@ -1,4 +1,4 @@
-// Flash attention backward on sm_100a for head_dim 64 and up to 512 queries: one CTA per (head, example).
+// Flash attention backward on sm_100a for head_dim 64: one CTA per head, example and 512 queries.
 //
 // The CTA walks the key blocks of its head and, inside each, the queries 64 at a time. dQ of all (up to
 // four) query blocks stays in TMEM for the whole walk, dK and dV of a key block for its part of it, so all
@@ -16,7 +16,7 @@
 // 6.7k on a 128 x 128 tile. Here a CTA takes 16k and a 128 x 64 unit 2 to 3k, bound by what a softmax warp does
 // one after the other for a unit (us, with rowsum(dO * O), clearing and casting of dQ where there are any,
 // before / now: 128 x 12 heads x 512 x 512 1081 / 610, 114 x 512 without a bias 385 / 202, 114 x 114 causal
-// 184 / 113, 32 x 64 x 512 x 512 1327 / 792). Of the 610, the bias gradient takes 100 (40 its additions to
+// 184 / 113, 24 x 12 x 509 packed 258 / 157, 32 x 64 x 512 x 512 1327 / 792). Of the 610, the bias gradient takes 100 (40 its additions to
 // shared memory, which are loops around a compare-and-swap), the bias 35, the exponentials 8.
 #include <type_traits>
 
@@ -27,16 +27,22 @@ namespace t5x {
 namespace {
 
 constexpr int kMaxQ = 512;        // queries: 4 x 64 columns of TMEM for dQ
-constexpr int kMaxRel = 1152;     // padded queries + padded keys, with a bias table
+// Padded queries and keys together, with a bias table; and stages of Q and dO. Where the queries are cut into
+// parts the tables are longer, in the place of a stage.
+template <bool kParts>
+constexpr int kMaxRelOf = kParts ? 1664 : 1152;
+template <bool kParts>
+constexpr int kRingOf = kParts ? 2 : 3;
 constexpr int kMaxKeys = 4096;    // a bit per key block
 constexpr int kBuckets = 128;     // bias tables of more buckets take the other kernel
-constexpr int kRing = 3;
 constexpr int kOutside = 255, kMixed = 254;  // in tables of buckets: none, several
 constexpr int kThreads = kSoftmaxThreads + 64;  // + MMA warp + TMA warp
 constexpr int kMmaWarp = kSoftmaxWarps, kTmaWarp = kSoftmaxWarps + 1;
 constexpr int kKernelId = 12;
 
+template <bool kParts>
 struct HeadSmem {
+  static constexpr int kMaxRel = kMaxRelOf<kParts>, kRing = kRingOf<kParts>;
   static constexpr int kPanel = 128 * 128;  // [128 x 64] bf16
   static constexpr int kHalf = 64 * 128;    // [64 x 64] bf16
   static constexpr int kK = 0;              // 2 stages
@@ -54,11 +60,11 @@ struct HeadSmem {
   static constexpr int kFlat = kBucketAt + kMaxRel;
   static constexpr int kBucket = kFlat + (kMaxRel / 16 + 7) / 8 * 8;  // bias gradient by bucket
   static constexpr int kWords = kBucket + kBuckets * 4;  // block flags
-  static constexpr int kBars = kWords + 4 * 4;
+  static constexpr int kBars = kWords + 6 * 4;
   static constexpr int kTotal = kBars + 24 * 8 + 1024;
 };
-static_assert(HeadSmem::kTotal <= 232448, "shared memory of a CTA");
-static_assert(HeadSmem::kBars % 8 == 0, "barriers are 8-byte words");
+static_assert(HeadSmem<false>::kTotal <= 232448 && HeadSmem<true>::kTotal <= 232448, "shared memory of a CTA");
+static_assert(HeadSmem<false>::kBars % 8 == 0 && HeadSmem<true>::kBars % 8 == 0, "barriers are 8-byte words");
 
 struct HeadParams {
   AttnParams a;
@@ -66,6 +72,7 @@ struct HeadParams {
   const __nv_bfloat16* dO;
   long long o_sb, o_sl, o_sh, do_sb, do_sl, do_sh;
   int ahead;  // CTAs that run at a time
+  float *dK32, *dV32;  // kParts: [B, Lk, H, 64], added to
 };
 
 // Waits for the loads from TMEM into these registers.
@@ -81,13 +88,18 @@ __device__ __forceinline__ void tmem_wait_into(uint32_t (&a)[16], uint32_t (&c)[
 
 // kAhead: causal self-attention over more than one block, where key blocks ahead of a query block are
 // passed over (see attn_bwd_kernel for the conditions).
-template <bool kAhead>
+// kParts: more than 512 queries, a CTA for each 512 of them. dQ leaves as above; dK and dV of the parts are added in
+// fp32 memory and cast afterwards. (us, by
+// key blocks in attention_sm100.cu / so, with all launches: prefix LM, 16 x 12 heads x 1024, 591 / 400.)
+template <bool kAhead, bool kParts>
 __global__ void __launch_bounds__(kThreads, 1)
     attn_bwd_head_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                          const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                          const __grid_constant__ CUtensorMap tmDQ, const __grid_constant__ CUtensorMap tmDK,
                          const __grid_constant__ CUtensorMap tmDV, const __grid_constant__ CUtensorMap tmO,
                          const __grid_constant__ HeadParams hp) {
+  using HeadSmem = HeadSmem<kParts>;
+  constexpr int kMaxRel = HeadSmem::kMaxRel, kRing = HeadSmem::kRing;
   const AttnParams& p = hp.a;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -118,8 +130,11 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.x, b = blockIdx.y;
   const int nkb = (p.Lk + 127) / 128;
-  const int lq_pad = (p.Lq + 127) / 128 * 128;
-  const int units = (p.Lq + 63) / 64;  // of a key block
+  // queries count from here (the last part first: of causal attention it has the most keys)
+  const int q_base = kParts ? static_cast<int>(gridDim.z - 1 - blockIdx.z) * kMaxQ : 0;
+  const int lq = kParts ? min(p.Lq - q_base, kMaxQ) : p.Lq;
+  const int lq_pad = (lq + 127) / 128 * 128;
+  const int units = (lq + 63) / 64;  // of a key block
   constexpr int cS = 0, cDP = 64, cDQ = 128, cDK = 384, cDV = 448;
 
   if (threadIdx.x == 0) {
@@ -139,7 +154,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (threadIdx.x < 4) sWords[threadIdx.x] = 0u;
+  if (threadIdx.x < 6) sWords[threadIdx.x] = 0u;
   if (warp == kMmaWarp) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
@@ -153,7 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   // The softmax warps request what their tables are made of: the buckets of up to three relative
   // positions a thread (and, in a warp's first lane, of the position before), and a query's statistics.
   constexpr int kRelRounds = (kMaxRel + 32 + kSoftmaxThreads - 1) / kSoftmaxThreads;
-  const int rels = lq_pad + nkb * 128;  // table index t: k - q = t - lq_pad
+  const int rels = lq_pad + nkb * 128;  // table index t: k - q = t - lq_pad - q_base
   int bucket[kRelRounds], left[kRelRounds];
   // ... and of rowsum(dO * O): eight lanes a query, the first four of eight rounds of queries.
   constexpr int kRows = kSoftmaxThreads / 8;
@@ -161,14 +176,14 @@ __global__ void __launch_bounds__(kThreads, 1)
   int code = 0;
   uint4 xo[4], xd[4];
   const int sub = threadIdx.x & 7;
-  const __nv_bfloat16* o_row = hp.O + b * hp.o_sb + h * hp.o_sh + sub * 8;
-  const __nv_bfloat16* do_row = hp.dO + b * hp.do_sb + h * hp.do_sh + sub * 8;
+  const __nv_bfloat16* o_row = hp.O + b * hp.o_sb + q_base * hp.o_sl + h * hp.o_sh + sub * 8;
+  const __nv_bfloat16* do_row = hp.dO + b * hp.do_sb + q_base * hp.do_sl + h * hp.do_sh + sub * 8;
   auto request_rows = [&](int q0) {
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const int q = q0 + c * kRows;
       xo[c] = xd[c] = make_uint4(0u, 0u, 0u, 0u);
-      if (q < p.Lq) {
+      if (q < lq) {
         xo[c] = *reinterpret_cast<const uint4*>(o_row + static_cast<long long>(q) * hp.o_sl);
         xd[c] = *reinterpret_cast<const uint4*>(do_row + static_cast<long long>(q) * hp.do_sl);
       }
@@ -178,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     request_rows(threadIdx.x >> 3);
 #pragma unroll
     for (int c = 0; c < kRelRounds; ++c) {
-      const int t = threadIdx.x + c * kSoftmaxThreads, idx = t - lq_pad + p.rel_off;
+      const int t = threadIdx.x + c * kSoftmaxThreads, idx = t - lq_pad - q_base + p.rel_off;
       bucket[c] = left[c] = -1;
       if (p.rel_bias != nullptr && t <= rels) {
         if (t < rels && idx >= 0 && idx < p.nrel) bucket[c] = __ldg(p.rel_bucket + idx);
@@ -186,9 +201,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
     const int q = threadIdx.x;
-    if (q < p.Lq) {
-      lse = p.lse[(static_cast<long long>(b) * p.H + h) * p.Lq + q];
-      if (p.q_seg) code = p.q_seg[static_cast<long long>(b) * p.Lq + q];
+    if (q < lq) {
+      lse = p.lse[(static_cast<long long>(b) * p.H + h) * p.Lq + q_base + q];
+      if (p.q_seg) code = p.q_seg[static_cast<long long>(b) * p.Lq + q_base + q];
     }
   }
   // Key blocks that a key mask alone hides whole (words[0]: blocks with a visible key), and of causal
@@ -225,11 +240,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     unseen = sWords[1];
     prefix = sWords[2];
   }
-  // first unit of key block j
+  // First unit of key block j (of a part's units there may be none).
   auto first_unit = [&](int j) {
     if (!kAhead) return 0;
     const uint32_t before = (1u << j) - 1u;
-    return ((unseen & before) | ((prefix >> j) & 1u)) ? 0 : 2 * j;
+    return ((unseen & before) | ((prefix >> j) & 1u)) ? 0 : max(0, 2 * j - q_base / 64);
+  };
+  auto passed_over = [&](int j) {
+    return ((idle >> j) & 1u) != 0u || (kAhead && kParts && first_unit(j) >= units);
   };
   const uint32_t tmem_base = *tmem_slot;
 
@@ -240,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       int loaded = 0, stored = 0;      // key blocks whose K and V were requested, whose gradients were stored
       int j_load = 0, j_store = 0;     // the next ones
       auto skip = [&](int j) {
-        while (j < nkb && ((idle >> j) & 1u)) ++j;
+        while (j < nkb && passed_over(j)) ++j;
         return j;
       };
       // the gradients of the oldest key block that is still on the chip, from where its K and V were
@@ -248,10 +266,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int st = stored & 1;
         if (!mbar_wait(&bar_staged[st], (stored >> 1) & 1, abort_flag)) return false;
         j_store = skip(j_store);
+        ++stored;
+        if (kParts) return true;  // (they have been added to memory)
         tma_store_4d(&tmDK, smem + HeadSmem::kK + st * HeadSmem::kPanel, 0, h, j_store * 128, b);
         tma_store_4d(&tmDV, smem + HeadSmem::kV + st * HeadSmem::kPanel, 0, h, j_store * 128, b);
         bulk_commit();
-        ++stored;
         ++j_store;
         return true;
       };
@@ -271,7 +290,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         return true;
       };
       for (int j = 0; j < nkb && ok; ++j) {
-        if ((idle >> j) & 1u) continue;
+        if (passed_over(j)) continue;
         if (loaded == n) ok = load_kv();
         const int first = first_unit(j);
         for (int w = first; w < units && ok; ++w, ++u) {
@@ -279,15 +298,15 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (u >= kRing) ok = mbar_wait(&bar_qfree[st], (u / kRing - 1) & 1, abort_flag);
           if (!ok) break;
           mbar_expect_tx(&bar_q[st], 2 * HeadSmem::kHalf);
-          tma_load_4d(smem + HeadSmem::kQ + st * HeadSmem::kHalf, &tmQ, &bar_q[st], 0, h, w * 64, b);
-          tma_load_4d(smem + HeadSmem::kDO + st * HeadSmem::kHalf, &tmDO, &bar_q[st], 0, h, w * 64, b);
+          tma_load_4d(smem + HeadSmem::kQ + st * HeadSmem::kHalf, &tmQ, &bar_q[st], 0, h, q_base + w * 64, b);
+          tma_load_4d(smem + HeadSmem::kDO + st * HeadSmem::kHalf, &tmDO, &bar_q[st], 0, h, q_base + w * 64, b);
           // the next key block, once the operands of this one's first units are under way (its place holds
           // the gradients of the block before until they are stored)
           if (w == min(first + 2, units - 1)) ok = load_kv();
         }
         // What the CTA after this one on the SM (about hp.ahead heads further) starts with goes to L2 now:
         // all SMs load their 320 KB at about the same time, and wait for it.
-        if (n == 0) {
+        if (!kParts && n == 0) {
           const long long head = static_cast<long long>(b) * p.H + h + hp.ahead;
           const int hn = static_cast<int>(head % p.H), bn = static_cast<int>(head / p.H);
           if (bn < p.B) {
@@ -306,7 +325,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (ok) ok = mbar_wait(bar_dq, 0, abort_flag);
       if (ok) {
         for (int i = 0; i < lq_pad / 128; ++i)
-          tma_store_4d(&tmDQ, smem + HeadSmem::kDS + i * HeadSmem::kPanel, 0, h, i * 128, b);
+          tma_store_4d(&tmDQ, smem + HeadSmem::kDS + i * HeadSmem::kPanel, 0, h, q_base + i * 128, b);
         bulk_commit();
       }
       bulk_store_wait_all();
@@ -363,7 +382,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     int prev_ring = 0, prev_kv = 0, prev_w = 0, prev_pair = 0;
     bool prev_first = false;
     for (int j = 0; j < nkb && ok; ++j) {
-      if ((idle >> j) & 1u) continue;
+      if (passed_over(j)) continue;
       const int kv = n & 1;
       ok = mbar_wait(&bar_kv[kv], (n >> 1) & 1, abort_flag);
       const int first = first_unit(j);
@@ -429,10 +448,16 @@ __global__ void __launch_bounds__(kThreads, 1)
       sQseg[threadIdx.x] = code;
     }
     // words[3], bit g: queries 16 g .. 16 g + 15 all exist, and none of them has all its keys hidden
-    const uint32_t good = __ballot_sync(0xffffffffu, threadIdx.x < p.Lq && lse * kLog2e >= -5e9f);
-    if (lane == 0)
-      atomicOr(&sWords[3], ((good & 0xffffu) == 0xffffu ? 1u << (2 * warp) : 0u) |
-                               ((good >> 16) == 0xffffu ? 2u << (2 * warp) : 0u));
+    const uint32_t good = __ballot_sync(0xffffffffu, threadIdx.x < lq && lse * kLog2e >= -5e9f);
+    // words[4], bit g: they have one code
+    const uint32_t alike = __ballot_sync(0xffffffffu, code == __shfl_sync(0xffffffffu, code, lane & 16));
+    auto both_halves = [&](uint32_t bits) {
+      return ((bits & 0xffffu) == 0xffffu ? 1u << (2 * warp) : 0u) | ((bits >> 16) == 0xffffu ? 2u << (2 * warp) : 0u);
+    };
+    if (lane == 0) {
+      atomicOr(&sWords[3], both_halves(good));
+      atomicOr(&sWords[4], both_halves(alike));
+    }
     if (has_bias) {
       const float* tab = p.rel_bias + static_cast<long long>(h) * p.num_buckets;
       if (threadIdx.x < kBuckets) sBucket[threadIdx.x] = 0.f;
@@ -481,7 +506,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       sFlat[threadIdx.x] = flat ? sBucketAt[t + 14] : kMixed;
     }
     softmax_bar_sync();
-    const uint32_t counting = sWords[3];
+    const uint32_t counting = sWords[3], one_code = sWords[4];
 
     // 16 columns of a row of an accumulator, in bf16, into a panel that a tensor copy stores
     auto stage = [&](uint32_t col, uint8_t* panel, bool zero) {
@@ -500,8 +525,33 @@ __global__ void __launch_bounds__(kThreads, 1)
         *reinterpret_cast<uint4*>(panel + r * 128 + (((part * 2 + g) ^ (r & 7)) << 4)) = out;
       }
     };
-    // dK and dV of the n-th key block walked, into the place of its K and V
-    auto stage_keys = [&](int n) {
+    // kParts: 16 columns of a row are added to memory. Four lanes exchange their 16-byte pieces, so that an
+    // instruction adds 64 contiguous bytes of 8 rows.
+    auto add_rows = [&](uint32_t col, float* to, int j) {
+      uint32_t v[16];
+      tmem_ld16(t_row + col + part * 16, v);
+      tmem_ld_wait();
+      transpose_pieces(v, lane);
+      const int k = j * 128 + quarter * 32 + (lane & ~3);
+      float* dst = to + ((static_cast<long long>(b) * p.Lk + k) * p.H + h) * 64 + part * 16 + (lane & 3) * 4;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (k + i < p.Lk)
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + i * static_cast<long long>(p.H) * 64),
+                       "f"(__uint_as_float(v[4 * i])), "f"(__uint_as_float(v[4 * i + 1])),
+                       "f"(__uint_as_float(v[4 * i + 2])), "f"(__uint_as_float(v[4 * i + 3]))
+                       : "memory");
+    };
+    // dK and dV of the n-th key block walked, block j, into the place of its K and V (or to memory)
+    auto stage_keys = [&](int n, int j) {
+      if (kParts) {
+        add_rows(cDK, hp.dK32, j);
+        add_rows(cDV, hp.dV32, j);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_staged[n & 1]);
+        return;
+      }
       stage(cDK, smem + HeadSmem::kK + (n & 1) * HeadSmem::kPanel, false);
       stage(cDV, smem + HeadSmem::kV + (n & 1) * HeadSmem::kPanel, false);
       tc_fence_before();
@@ -524,8 +574,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       flat_sum = 0.f;
     };
     auto next_block = [&](int j) {  // the first key block from j on that is walked
-      while (j < nkb && ((idle >> j) & 1u)) {
-        for (int i = threadIdx.x; i < 128 * 8; i += kSoftmaxThreads) {
+      while (j < nkb && passed_over(j)) {
+        for (int i = threadIdx.x; !kParts && i < 128 * 8; i += kSoftmaxThreads) {
           const int k = j * 128 + i / 8;
           if (k < p.Lk) {
             const long long off = b * p.dk_sb + static_cast<long long>(k) * p.dk_sl + h * p.dk_sh + i % 8 * 8;
@@ -545,7 +595,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       code = (k < p.Lk && p.kv_seg) ? p.kv_seg[at] : 0;
     };
     int u = 0, pair = 0, n = 0;  // units walked, key blocks walked
-    int j = next_block(0), w = 0, next_j = nkb;
+    int j = next_block(0), w = 0, next_j = nkb, last_j = 0;
     bool kvis = false, next_kvis = false;
     int kcode = 0, next_kcode = 0;
     uint32_t sv[16], dpv[16];
@@ -577,21 +627,27 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t mv = kvis ? 0xffffu : 0u;
       bool all_seen = all_keys;
       if (!simple_mask) {
-        if (p.kv_seg) {
+        // of causal attention the first of them come before the key
+        const int hidden = p.causal ? k - p.causal_off - q_base - q0 : 0;
+        const uint32_t behind = hidden <= 0 ? 0xffffu : (hidden >= 16 ? 0u : 0xffffu << hidden);
+        if (p.kv_seg == nullptr) {
+          mv &= behind;
+        } else {
           const int kseg = kcode & seg_mask;
           const bool k_pre = prefix_lm && ((kcode >> 30) & 1);
-          uint32_t m = 0u;
+          if ((one_code >> (q0 >> 4)) & 1u) {
+            const int code = sQseg[q0];
+            mv &= kseg == (code & seg_mask) ? ((k_pre && ((code >> 30) & 1)) ? 0xffffu : behind) : 0u;
+          } else {
+            uint32_t m = 0u;
 #pragma unroll 4
-          for (int x = 0; x < 16; ++x) {
-            const int code = sQseg[q0 + x];
-            bool v = kseg == (code & seg_mask);
-            if (p.causal) v = v && (k <= q0 + x + p.causal_off || (k_pre && ((code >> 30) & 1)));
-            m |= (v ? 1u : 0u) << x;
+            for (int x = 0; x < 16; ++x) {
+              const int code = sQseg[q0 + x];
+              const bool v = kseg == (code & seg_mask) && (((behind >> x) & 1u) || (k_pre && ((code >> 30) & 1)));
+              m |= (v ? 1u : 0u) << x;
+            }
+            mv &= m;
           }
-          mv &= m;
-        } else {
-          const int hidden = k - p.causal_off - q0;  // the first of them do not
-          mv &= hidden <= 0 ? 0xffffu : (hidden >= 16 ? 0u : 0xffffu << hidden);
         }
         all_seen = __all_sync(0xffffffffu, (mv & 0xffffu) == 0xffffu);
       }
@@ -655,7 +711,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             // A row with every key masked has lse = -1e10 + log(Lk), which fp32 rounds to -1e10:
             // its probabilities are uniform over the Lk keys.
             if (nl > 5e9f) e = inv_lk;
-            if (k >= p.Lk || q0 + xx >= p.Lq) e = 0.f;
+            if (k >= p.Lk || q0 + xx >= lq) e = 0.f;
             e2[c] = e;
             ds[xx] = e * (__uint_as_float(dpv[xx]) + sDelta[q0 + xx]);
           }
@@ -682,7 +738,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         ok = mbar_wait_relaxed(&bar_g[(u - 1) & 1], ((u - 1) >> 1) & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        stage_keys(n - 1);
+        stage_keys(n - 1, last_j);
       }
       tc_fence_before();
       fence_proxy_async_smem();
@@ -692,6 +748,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if ((w & 1) || w == units - 1) pair ^= 1;
       ++u;
       if (++w == units) {
+        last_j = j;
         j = next_j;
         ++n;
         if (j < nkb) enter_block();
@@ -728,7 +785,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       ok = mbar_wait_relaxed(&bar_g[(u - 1) & 1], ((u - 1) >> 1) & 1, abort_flag);
       if (ok) {
         tc_fence_after();
-        stage_keys(n - 1);
+        stage_keys(n - 1, last_j);
       }
     }
     if (ok) {
@@ -778,7 +835,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-template <bool kAhead>
+template <bool kAhead, bool kParts>
 int launch_head(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* tv, const CUtensorMap* tdo,
                 const CUtensorMap* tdq, const CUtensorMap* tdk, const CUtensorMap* tdv, const CUtensorMap* to,
                 const HeadParams& hp, cudaStream_t st) {
@@ -786,13 +843,13 @@ int launch_head(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap*
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_head_kernel<kAhead>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, HeadSmem::kTotal);
+    cudaError_t e = cudaFuncSetAttribute(attn_bwd_head_kernel<kAhead, kParts>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, HeadSmem<kParts>::kTotal);
     if (e != cudaSuccess) return set_error("attention_bwd_head attr: %s", cudaGetErrorString(e));
     attr_set[dev] = true;
   }
-  attn_bwd_head_kernel<kAhead>
-      <<<dim3(hp.a.H, hp.a.B), kThreads, HeadSmem::kTotal, st>>>(*tq, *tk, *tv, *tdo, *tdq, *tdk, *tdv, *to, hp);
+  attn_bwd_head_kernel<kAhead, kParts><<<dim3(hp.a.H, hp.a.B, (hp.a.Lq + kMaxQ - 1) / kMaxQ), kThreads,
+                                         HeadSmem<kParts>::kTotal, st>>>(*tq, *tk, *tv, *tdo, *tdq, *tdk, *tdv, *to, hp);
   count_launches(1);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("attention_bwd_head: %s", cudaGetErrorString(e));
@@ -803,23 +860,35 @@ int launch_head(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap*
 
 using namespace t5x;
 
-// Whether t5x_attention_bwd_head takes these sizes and is the faster of the two backward kernels.
+// Whether t5x_attention_bwd_head takes these sizes and is the faster of the two backward kernels: 0, or 1 as it
+// stands, or 2 with fp32 buffers for dK and dV.
 T5X_API int t5x_attention_bwd_head_covers(int B, int H, int Lq, int Lk, int D, int num_buckets) {
-  if (D != 64 || B <= 0 || B > 65535 || H <= 0 || Lq <= 0 || Lq > kMaxQ || Lk <= 0 || Lk > kMaxKeys) return 0;
-  const int nkb = (Lk + 127) / 128, nq = (Lq + 127) / 128;
-  if (num_buckets > 0 && (num_buckets > kBuckets || (nkb + nq) * 128 > kMaxRel)) return 0;
+  if (D != 64 || B <= 0 || B > 65535 || H <= 0 || Lq <= 0 || Lq > 8 * kMaxQ || Lk <= 0 || Lk > kMaxKeys) return 0;
+  const int nkb = (Lk + 127) / 128, nq = (Lq + 127) / 128, parts = (Lq + kMaxQ - 1) / kMaxQ;
+  if (num_buckets > 0 && (num_buckets > kBuckets || (nkb + (nq < 4 ? nq : 4)) * 128 >
+                                                        (parts > 1 ? kMaxRelOf<true> : kMaxRelOf<false>)))
+    return 0;
   // Thousands of cycles, measured: 14 for a CTA and 3 for each of its 128 x 64 units; the other kernel, with a
-  // CTA per key block, 14 and 7 for each 128 x 128 tile, and some 10 for its three further launches. (512 x
-  // 512, us, other / this: 16 x 6 heads 128 / 62, 74 heads even, 12 heads 27 / 58.)
+  // CTA per key block, 14 and 7 for each 128 x 128 tile, and some 10 for its three further launches; clearing and
+  // casting dQ (there) or the dK and dV of parts (here), ten bytes an element at 3.4 MB a thousand cycles. (512 x
+  // 512, us, other / this: 16 x 6 heads 128 / 62, 74 heads even, 12 heads 27 / 58; 1024 x 1024: 16 x 12 heads 591 /
+  // 400, 16 x 6 225 / 235.)
   const long long sms = num_sms(), heads = static_cast<long long>(B) * H;
-  const long long here = (heads + sms - 1) / sms * (14 + 3 * nkb * ((Lq + 63) / 64));
-  return here <= (heads * nkb + sms - 1) / sms * (14 + 7 * nq) + 10;
+  const int units = parts > 1 ? kMaxQ / 64 : (Lq + 63) / 64;
+  const double cast = heads * 640.0 / 3.4e6;
+  const double here = static_cast<double>((heads * parts + sms - 1) / sms) * (14 + 3 * nkb * units) +
+                      (parts > 1 ? 2 * Lk * cast : 0.0);
+  const double other = static_cast<double>((heads * nkb + sms - 1) / sms) * (14 + 7 * nq) + 10 + Lq * cast;
+  if (here > other) return 0;
+  return parts > 1 ? 2 : 1;
 }
 
 // q [B,Lq,H,64], k/v [B,Lk,H,64], o and d_o like q, bf16 with element strides (sb, sl, sh), innermost
-// contiguous; dq, dk and dv (the strides of dk) are written whole, in bf16. The rest as t5x_attention_bwd.
+// contiguous; dq, dk and dv (the strides of dk) are written whole, in bf16; of more than 512 queries, dk32 and dv32
+// (fp32, [B,Lk,H,64], cleared) are added to instead of dk and dv. The rest as t5x_attention_bwd.
 T5X_API int t5x_attention_bwd_head(const void* q, const void* k, const void* v, const void* o, const void* d_o,
-                                   const void* lse, void* dq, void* dk, void* dv, int B, int H, int Lq, int Lk,
+                                   const void* lse, void* dq, void* dk, void* dv, void* dk32, void* dv32, int B,
+                                   int H, int Lq, int Lk,
                                    long long q_sb, long long q_sl, long long q_sh, long long k_sb,
                                    long long k_sl, long long k_sh, long long v_sb, long long v_sl,
                                    long long v_sh, long long o_sb, long long o_sl, long long o_sh,
@@ -830,11 +899,15 @@ T5X_API int t5x_attention_bwd_head(const void* q, const void* k, const void* v, 
                                    const void* key_mask, const void* q_seg, const void* kv_seg, int causal,
                                    int causal_off, void* stream) {
   if (B <= 0 || H <= 0 || Lq <= 0 || Lk <= 0) return 0;
-  if (Lq > kMaxQ || Lk > kMaxKeys || B > 65535)
-    return set_error("attention_bwd_head: %d examples of %d queries and %d keys are not covered", B, Lq, Lk);
   const int nkb = (Lk + 127) / 128, nq = (Lq + 127) / 128;
-  if (rel_bias != nullptr && (num_buckets > kBuckets || (nkb + nq) * 128 > kMaxRel))
+  const bool parts = Lq > kMaxQ;
+  if (Lq > 8 * kMaxQ || Lk > kMaxKeys || B > 65535)
+    return set_error("attention_bwd_head: %d examples of %d queries and %d keys are not covered", B, Lq, Lk);
+  if (rel_bias != nullptr && (num_buckets > kBuckets || (nkb + (nq < 4 ? nq : 4)) * 128 >
+                                                            (parts ? kMaxRelOf<true> : kMaxRelOf<false>)))
     return set_error("attention_bwd_head: %d buckets over %d + %d positions are not covered", num_buckets, Lq, Lk);
+  if (parts && (dk32 == nullptr || dv32 == nullptr || !aligned_to(16, {dk32, dv32})))
+    return set_error("attention_bwd_head: more than %d queries need fp32 buffers for dK and dV", kMaxQ);
   if ((do_sb | do_sl | do_sh | o_sb | o_sl | o_sh | dq_sb | dq_sl | dq_sh | dk_sb | dk_sl | dk_sh) & 7)
     return set_error("attention_bwd_head: dO / O / dQ / dK strides must be multiples of 8 elements");
   if (!aligned_to(16, {o, d_o, dq, dk, dv}))
@@ -867,7 +940,11 @@ T5X_API int t5x_attention_bwd_head(const void* q, const void* k, const void* v, 
   hp.o_sb = o_sb; hp.o_sl = o_sl; hp.o_sh = o_sh;
   hp.do_sb = do_sb; hp.do_sl = do_sl; hp.do_sh = do_sh;
   hp.ahead = num_sms();
+  hp.dK32 = static_cast<float*>(dk32);
+  hp.dV32 = static_cast<float*>(dv32);
   const bool ahead = causal && Lq == Lk && causal_off == 0 && Lq > 128;
-  return (ahead ? launch_head<true> : launch_head<false>)(&tq, &tk, &tv, &tdo, &tdq, &tdk, &tdv, &to, hp,
+  const auto launch = parts ? (ahead ? launch_head<true, true> : launch_head<false, true>)
+                            : (ahead ? launch_head<true, false> : launch_head<false, false>);
+  return launch(&tq, &tk, &tv, &tdo, &tdq, &tdk, &tdv, &to, hp,
                                                           static_cast<cudaStream_t>(stream));
 }

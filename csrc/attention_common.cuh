@@ -1,6 +1,6 @@
 // Declarations shared by the attention kernels: forward, attention_fwd_rows_sm100.cu (64 channels, up to 2048
 // keys) and attention_fwd_sm100.cu (any length, 64 or 128 channels); backward, attention_bwd_head_sm100.cu (64
-// channels, up to 512 queries) and attention_sm100.cu.
+// channels, where there are heads enough) and attention_sm100.cu.
 #pragma once
 #include "common.cuh"
 
@@ -227,6 +227,28 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       : "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
         "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
       : "memory");
+}
+
+// The 4 x 4 transpose of 16-byte pieces among four adjacent lanes: lane j brings pieces 0..3 of its
+// row and leaves with piece j of the four rows, in order of the lanes.
+__device__ __forceinline__ void transpose_pieces(uint32_t* v, int lane) {
+  const bool odd = lane & 1, high = lane & 2;
+#pragma unroll
+  for (int c = 0; c < 16; c += 8)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {  // pieces c / 4 and c / 4 + 1 with the neighbour
+      const uint32_t a = v[c + e], b = v[c + 4 + e];
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+      v[c + e] = odd ? got : a;
+      v[c + 4 + e] = odd ? b : got;
+    }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {  // the pairs with the lane two away
+    const uint32_t a = v[c], b = v[c + 8];
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, high ? a : b, 2);
+    v[c] = high ? got : a;
+    v[c + 8] = high ? b : got;
+  }
 }
 
 // Tensor map over a [B, L, H, D] bf16 tensor with element strides (sb, sl, sh): boxes of

@@ -13,7 +13,7 @@
 //
 // One CTA per (128-key block, head, batch), looping over query blocks; dK/dV accumulate in TMEM, dQ partial
 // tiles are added to an fp32 buffer with vector red.global.add. (attention_bwd_head_sm100.cu is the faster one
-// for up to 512 queries of 64 channels where there are heads enough.)
+// for 64 channels where there are heads enough.)
 #include "attention_common.cuh"
 #include "t5x_ops.h"
 
@@ -94,28 +94,6 @@ __device__ __forceinline__ void visible_scores(const uint32_t (&sv)[16], const u
     s = fmaxf(s, kMaskValue);
     pr[x] = exp2f(fmaf(s, kLog2e, -lse[x]));
     ds[x] = pr[x] * (__uint_as_float(dpv[x]) - delta[x]);
-  }
-}
-
-// The 4 x 4 transpose of 16-byte pieces among four adjacent lanes: lane j brings pieces 0..3 of its
-// row and leaves with piece j of the four rows, in order of the lanes.
-__device__ __forceinline__ void transpose_pieces(uint32_t* v, int lane) {
-  const bool odd = lane & 1, high = lane & 2;
-#pragma unroll
-  for (int c = 0; c < 16; c += 8)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {  // pieces c / 4 and c / 4 + 1 with the neighbour
-      const uint32_t a = v[c + e], b = v[c + 4 + e];
-      const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
-      v[c + e] = odd ? got : a;
-      v[c + 4 + e] = odd ? b : got;
-    }
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {  // the pairs with the lane two away
-    const uint32_t a = v[c], b = v[c + 8];
-    const uint32_t got = __shfl_xor_sync(0xffffffffu, high ? a : b, 2);
-    v[c] = high ? got : a;
-    v[c + 8] = high ? b : got;
   }
 }
 

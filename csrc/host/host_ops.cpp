@@ -401,7 +401,7 @@ std::tuple<Tensor, Tensor, Tensor> attention_gradients(const Tensor& d_o, const 
                                                        bool packed, void* st) {
   const int B = q.size(0), Lq = q.size(1), H = q.size(2), D = q.size(3), Lk = k.size(1);
   const auto f32 = q.options().dtype(at::kFloat);
-  const bool head = t5x_attention_bwd_head_covers(B, H, Lq, Lk, D, m.num_buckets()) != 0;
+  const int head = t5x_attention_bwd_head_covers(B, H, Lq, Lk, D, m.num_buckets());
   Tensor dq, dk, dv;
   if (packed) {
     Tensor all = at::empty({B, Lq, 3, H, D}, q.options());
@@ -414,9 +414,15 @@ std::tuple<Tensor, Tensor, Tensor> attention_gradients(const Tensor& d_o, const 
     dv = at::empty({B, Lk, H, D}, q.options());
   }
   if (head) {
+    optional<Tensor> dk32, dv32;  // what parts of the queries add to
+    if (head == 2) {
+      dk32 = at::zeros({B, Lk, H, D}, f32);
+      dv32 = at::zeros({B, Lk, H, D}, f32);
+    }
     check(t5x_attention_bwd_head(
               q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), lse.data_ptr(),
-              dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Lq, Lk, q.stride(0), q.stride(1),
+              dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dk32 ? dk32->data_ptr() : nullptr,
+              dv32 ? dv32->data_ptr() : nullptr, B, H, Lq, Lk, q.stride(0), q.stride(1),
               q.stride(2), k.stride(0), k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2),
               o.stride(0), o.stride(1), o.stride(2), d_o.stride(0), d_o.stride(1), d_o.stride(2),
               dq.stride(0), dq.stride(1), dq.stride(2), dk.stride(0), dk.stride(1), dk.stride(2),
@@ -424,6 +430,10 @@ std::tuple<Tensor, Tensor, Tensor> attention_gradients(const Tensor& d_o, const 
               m.num_buckets(), m.nrel(), m.rel_off, data_or_null(m.key_mask), data_or_null(m.q_seg),
               data_or_null(m.kv_seg), m.causal, m.causal_off, st),
           "attention_bwd");
+    if (dk32) {
+      dk.copy_(*dk32);
+      dv.copy_(*dv32);
+    }
     return std::make_tuple(dq, dk, dv);
   }
   Tensor dq32 = at::zeros({B, Lq, H, D}, f32), delta = at::empty({B, H, Lq}, f32);

@@ -29,7 +29,7 @@ native.register_signature("t5x_attention_fwd_stream", [c_void_p] * 5 + [c_int] *
                           [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
                            c_int, c_int, c_void_p])
 
-native.register_signature("t5x_attention_bwd_head", [c_void_p] * 9 + [c_int] * 4 + [c_ll] * 21 +
+native.register_signature("t5x_attention_bwd_head", [c_void_p] * 11 + [c_int] * 4 + [c_ll] * 21 +
                           [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
                            c_void_p, c_int, c_int, c_void_p])
 native.register_signature("t5x_attention_bwd_head_covers", [c_int] * 6)
@@ -150,7 +150,7 @@ class _FlashAttentionFn(torch.autograd.Function):
     Lk = k.shape[1]
     do = do if _strides_ok(do) else do.contiguous()
     nb, nrel = _bias_sizes(rel_bias, buckets)
-    head = bool(native.lib().t5x_attention_bwd_head_covers(B, H, Lq, Lk, D, nb))
+    head = native.lib().t5x_attention_bwd_head_covers(B, H, Lq, Lk, D, nb)
     if packed:
       dqkv = torch.empty((B, Lq, 3, H, D), dtype=torch.bfloat16, device=q.device)
       dq, dk, dv = dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]
@@ -163,11 +163,17 @@ class _FlashAttentionFn(torch.autograd.Function):
     if head:
       if not packed:
         dq = torch.empty((B, Lq, H, D), dtype=torch.bfloat16, device=q.device)
+      # what parts of the queries add to
+      wide = [torch.zeros((B, Lk, H, D), dtype=torch.float32, device=q.device) if head == 2 else None
+              for _ in range(2)]
       rc = native.lib().t5x_attention_bwd_head(
           q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
-          dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Lq, Lk, *_sbh(q), *_sbh(k), *_sbh(v),
-          *_sbh(o), *_sbh(do), *_sbh(dq), *_sbh(dk), *tail)
+          dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), *map(native.ptr, wide), B, H, Lq, Lk, *_sbh(q),
+          *_sbh(k), *_sbh(v), *_sbh(o), *_sbh(do), *_sbh(dq), *_sbh(dk), *tail)
       native._check(rc, "attention_bwd")
+      if head == 2:
+        dk.copy_(wide[0])
+        dv.copy_(wide[1])
       return dq, dk, dv, ret_rel, None, None, None, None, None, None, None
     dq32 = torch.zeros((B, Lq, H, D), dtype=torch.float32, device=q.device)
     delta = torch.empty((B, H, Lq), dtype=torch.float32, device=q.device)

@@ -16,19 +16,23 @@ def _call(q, k, v, o, do, lse, table, lq, lk, key_mask, qs, ks, mode):
     buckets = A._rel_buckets(lq, lk, 0, mode == 0, 32, 128, q.device)
     d_table = torch.zeros_like(table)
   nb, nrel = A._bias_sizes(table, buckets)
+  wide = [torch.zeros_like(t, dtype=torch.float32) if lq > 512 else None for t in (k, v)]
   p = native.ptr
   native._check(native.lib().t5x_attention_bwd_head(
-      *(t.data_ptr() for t in (q, k, v, o, do, lse, dq, dk, dv)), b, h, lq, lk,
+      *(t.data_ptr() for t in (q, k, v, o, do, lse, dq, dk, dv)), *map(p, wide), b, h, lq, lk,
       *(s for t in (q, k, v, o, do, dq, dk) for s in A._sbh(t)), p(table), p(buckets), p(d_table), nb, nrel,
       lq - 1, p(key_mask), p(qs), p(ks), mode, lk - lq if mode else 0, native.stream_ptr()), "head")
   native.check_status()
+  if lq > 512:
+    dk, dv = wide
   return dq, dk, dv, d_table
 
 
 @pytest.mark.parametrize("mask", ["none", "padded", "unseen", "causal", "packed", "prefix"])
 @pytest.mark.parametrize("lq,lk,bias", [(1, 1, True), (31, 129, False), (64, 128, True), (65, 257, True),
                                         (129, 129, True), (200, 200, False), (512, 512, True),
-                                        (511, 640, True), (130, 1100, False)])
+                                        (511, 640, True), (130, 1100, False), (513, 130, True),
+                                        (1000, 1000, True), (1100, 300, False)])
 def test_against_float64(lq, lk, bias, mask):
   from t5x_b200.ops import attention as A, reference as ref
   if mask in ("causal", "packed", "prefix") and lq != lk:
@@ -89,5 +93,35 @@ def test_both_kernels_are_reached():
   covers = native.lib().t5x_attention_bwd_head_covers
   assert covers(128, 12, 512, 512, 64, 32) and covers(8, 6, 64, 64, 64, 32) and covers(64, 12, 114, 512, 64, 0)
   assert not covers(1, 12, 512, 512, 64, 32)  # too few CTAs
-  assert not covers(128, 12, 513, 512, 64, 32) and not covers(128, 12, 512, 512, 128, 32)
-  assert not covers(128, 12, 512, 700, 64, 32) and not covers(128, 12, 512, 512, 64, 300)
+  assert covers(16, 12, 1024, 1024, 64, 32) == 2 and not covers(16, 12, 1024, 1300, 64, 32)
+  assert not covers(128, 12, 512, 512, 128, 32) and not covers(128, 12, 512, 700, 64, 32)
+  assert not covers(128, 12, 512, 512, 64, 300)
+
+
+@pytest.mark.parametrize("compiled", [True, False])
+def test_the_choice_makes_no_difference(compiled, monkeypatch):
+  """A batch that goes to the kernel in parts of 512 queries, projections side by side in one buffer, against its
+  examples one by one, which do not."""
+  from t5x_b200.ops import attention as A, native
+  if not compiled:
+    monkeypatch.setattr(native, "host", lambda: None)
+  b, l, h = 16, 1024, 12
+  covers = native.lib().t5x_attention_bwd_head_covers
+  assert covers(b, h, l, l, 64, 32) == 2 and not covers(1, h, l, l, 64, 32)
+  g = torch.Generator(device="cuda").manual_seed(0)
+  qkv = torch.randn(b, l, 3, h, 64, device="cuda", generator=g).mul_(0.3).bfloat16()
+  do = torch.randn(b, l, h, 64, device="cuda", generator=g).bfloat16()
+  seg = (torch.arange(l, device="cuda") // 300)[None].expand(b, l).contiguous()
+  grads = []
+  for rows in ([slice(0, b)], [slice(i, i + 1) for i in range(b)]):
+    table = torch.nn.Parameter(torch.linspace(-1, 1, h * 32, device="cuda").view(h, 32))
+    parts = []
+    for r in rows:
+      q, k, v = (qkv[r, :, i].detach().requires_grad_() for i in range(3))
+      o = A.flash_attention(q, k, v, bias_table=table, bidirectional=False, causal=True,
+                            q_segment_ids=seg[r], kv_segment_ids=seg[r])
+      parts.append(torch.autograd.grad(o, (q, k, v, table), do[r]))
+    native.check_status()
+    grads.append([torch.cat([p[i] for p in parts]) for i in range(3)] + [sum(p[3] for p in parts)])
+  for x, y in zip(*grads):  # sums in another order, results rounded to bf16
+    assert float((x.float() - y.float()).norm() / y.float().norm()) < 2.0 ** -8
