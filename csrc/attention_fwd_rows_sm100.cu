@@ -3,12 +3,12 @@
 //
 // A softmax group of four warps owns 128 query rows, a thread a row: nothing is exchanged between threads. A
 // CTA has two groups (256 queries of a head; of 128 queries or fewer the groups take every other block of 64
-// keys and join their results at the end), and two CTAs share an SM. What bounds the kernel is the chain of
+// keys), and two CTAs share an SM. What bounds the kernel is the chain of
 // steps of a group (scores from TMEM, exponentials, probabilities to shared memory, fences, barriers): four
 // groups in different phases fill one another's gaps, to 60 % of the issue slots.
 // (us, T5-like scores; one CTA of 16 warps per SM with the scores of all keys in TMEM / here: 128 x 12 heads x
-// 512 x 512 with bias, 60 to 100 % of the keys visible 410 / 302, 114 x 512 without bias 117 / 103, 114 x 114
-// causal 80 / 59. Two groups of four warps per SM in blocks of 128 keys, the kernel in attention_fwd_sm100.cu /
+// 512 x 512 with bias, 60 to 100 % of the keys visible 410 / 305, 114 x 512 without bias 117 / 103, 114 x 114
+// causal 80 / 60. Two groups of four warps per SM in blocks of 128 keys, the kernel in attention_fwd_sm100.cu /
 // here: 16 x 6 x 1024 x 1024 148 / 89, 16 x 12 x 1024 prefix LM 341 / 184, 16 x 6 x 189 x 1024 52 / 37.)
 //
 // A step is 32 keys of a row. P goes to a panel of 64 keys, in halves; the P V products are issued by halves.
@@ -110,6 +110,9 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
   const int q_base = blockIdx.x * 256;
   const bool pair = p.Lq - q_base > 128;  // each group has queries of its own
   const int all_blocks = (p.Lk + 63) / 64;
+  // groups that share their queries, and the maximum, add to one O, in the order of the keys
+  const bool one_o = kShort && !pair;
+  const bool once = kShort && all_blocks == 1;  // the scores stay where they are for the second walk
   constexpr int cO = 128;
 
   if (threadIdx.x == 0) {
@@ -154,7 +157,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
     mbar_expect_tx(bar_q, (pair ? 2 : 1) * RowsSmem::kPanel);
     tma_load_4d(smem + RowsSmem::kQ, &tmQ, bar_q, 0, h, q_base, b);
     if (pair) tma_load_4d(smem + RowsSmem::kQ + RowsSmem::kPanel, &tmQ, bar_q, 0, h, q_base + 128, b);
-    load_block(0, 0, !kShort);
+    load_block(0, 0, !kShort || once);
   }
   __syncwarp();
 
@@ -247,7 +250,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
   if (warp == kRowsTma) {
     if (lane == 0) {
       bool ok = true;
-      for (int n = 1; n < (kShort ? 2 : 1) * blocks && ok; ++n) {
+      for (int n = 1; n < (kShort && !once ? 2 : 1) * blocks && ok; ++n) {
         if (n >= ring) ok = mbar_wait(&bar_kvfree[stage_of(n)], (use_of(n) - 1) & 1, abort_flag);
         const bool values = !kShort || n >= blocks;
         if (ok) load_block(n, kShort && values ? n - blocks : n, values);
@@ -270,7 +273,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
     // The scores of the i-th block of a group (of the first walk, in two buffers in turn; where they stay, the
     // first buffer goes on).
     auto issue_scores = [&](int g, int i, bool walk) {
-      if (i >= count[g] || !ok) return;
+      if (i >= count[g] || !ok || (once && !walk)) return;
       const int j = pair ? i : 2 * i + g;
       const int n = walk || !kShort ? j : blocks + j, st = stage_of(n);
       const int buf = walk ? i & 1 : 0;
@@ -281,7 +284,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
       tc_fence_after();
       const uint64_t qd = row_major + (RowsSmem::kQ >> 4) + (pair ? g : 0) * kP16;
       const uint64_t kd = row_major + static_cast<uint32_t>(place_of(st) >> 4);
-      const bool last = walk && (!pair || g == 1 || i >= count[1]);
+      const bool last = walk && !once && (!pair || g == 1 || i >= count[1]);
       if (leader) {
 #pragma unroll
         for (int s = 0; s < 4; ++s)
@@ -298,14 +301,15 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
       tc_fence_after();
       const int j = pair ? i : 2 * i + g;
       const uint64_t pd = row_major + (RowsSmem::kP >> 4) + g * kP16 + static_cast<uint32_t>(half) * 4;
-      const int st = stage_of(kShort ? blocks + j : j);
+      const int st = stage_of(kShort && !once ? blocks + j : j);
       const uint64_t vd = col_major + static_cast<uint32_t>(place_of(st) >> 4) + kB16 +
                           static_cast<uint32_t>(half) * 256;
       const bool last = half == 1 && (!pair || g == 1 || i >= count[1]);
       if (leader) {
 #pragma unroll
         for (int s = 0; s < 2; ++s)
-          umma_bf16(tmem_base + cO + g * 64, pd + 2 * s, vd + 128 * s, idesc_o, (i | half | s) != 0);
+          umma_bf16(tmem_base + cO + (one_o ? 0 : g * 64), pd + 2 * s, vd + 128 * s, idesc_o,
+                    ((one_o ? j : i) | half | s) != 0);
         umma_commit(&bar_pv[g * 2 + half]);
         if (last) umma_commit(&bar_kvfree[st]);
       }
@@ -320,9 +324,10 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
     issue_scores(1, 0, false);
     for (int i = 0; i < max(count[0], count[1]) && ok; ++i) {
       issue_values(0, i, 0);
-      issue_values(1, i, 0);
+      if (!one_o) issue_values(1, i, 0);
       issue_scores(0, i + 1, false);
       issue_values(0, i, 1);
+      if (one_o) issue_values(1, i, 0);
       issue_scores(1, i + 1, false);
       issue_values(1, i, 1);
     }
@@ -401,7 +406,8 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
 #pragma unroll 1
       for (i = 0; i < blocks_here && ok; ++i) {
         const int buf = look ? i & 1 : 0;
-        ok = __all_sync(0xffffffffu, mbar_wait(&bar_s[2 * g + buf], (look ? i >> 1 : uses + i) & 1, abort_flag));
+        if (look || !once)
+          ok = __all_sync(0xffffffffu, mbar_wait(&bar_s[2 * g + buf], (look ? i >> 1 : uses + i) & 1, abort_flag));
         if (!ok) break;
         tc_fence_after();
 #pragma unroll 1
@@ -551,7 +557,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
     // (past a wait that gave up the group barriers are passed all the same, and nothing is stored)
     float l = (sum + sum1) + (sum2 + sum3), mine_by = 1.f, other_by = 0.f;
     if (!pair) {
-      // group 1 leaves its maxima and sums; its O is in the same lanes of TMEM
+      // group 1 leaves its maxima and sums; its O (if it has one) is in the same lanes of TMEM
       if (g == 1) {
         tc_fence_before();
         sJoin[2 * r] = i > 0 ? m : -3.0e38f;
@@ -568,7 +574,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
         other_by = c;
       }
     }
-    const bool joined = !pair && n0 > 1;  // (group 1 has had a block)
+    const bool joined = !pair && !one_o && n0 > 1;  // (group 1 has had a block)
     const float scale = 1.f / l;
     if (pair || g == 0) {
 #pragma unroll 1
