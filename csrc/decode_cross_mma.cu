@@ -26,6 +26,11 @@
 // 1024: 32 values per lane), the row
 // maximum and sum cross the eight warps through shared memory, and the partial outputs of the
 // warps are added there at the end. Masked keys take the additive -1e10 of the reference.
+//
+// A chunk of which the mask hides every key (the padding of a batch) is not read: its scores are -1e10 whatever
+// the keys, and its probabilities exact zeros wherever any key of the example is visible. Bound by memory (64 x 4
+// beams x 32 heads x 512 keys, us, read whole and requested ahead / so: 60 to 100 % visible 59.9 / 52.3, all
+// visible 59.7 / 57.8).
 #include "common.cuh"
 #include "t5x_b200.h"
 
@@ -57,7 +62,9 @@ __device__ __forceinline__ int key_of_column(int u, int tile, int n) {
   return 8 * (n >> 1) + 4 * u + 2 * tile + (n & 1);
 }
 
-template <int BEAMS>
+// kLook: hidden chunks are passed over (not in a chain of launches of few rows, where the look takes longer than it
+// saves; there the operands are requested ahead instead).
+template <int BEAMS, bool kLook>
 __global__ void __launch_bounds__(kXmThreads)
     decode_cross_mma_kernel(const __nv_bfloat16* __restrict__ q,   // [B*beams, H, 64], row stride q_ld
                             const __nv_bfloat16* __restrict__ k,   // [B, H, Lp, 64]
@@ -68,6 +75,7 @@ __global__ void __launch_bounds__(kXmThreads)
   __shared__ float s_max[kXmWarps][8];
   __shared__ float s_sum[kXmWarps][8];
   __shared__ float s_out[kXmWarps][8][64];
+  __shared__ uint32_t s_shown;  // bit c: a key of chunk c is visible (or there is no mask)
   const int b = blockIdx.x / H, h = blockIdx.x - b * H;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -77,9 +85,24 @@ __global__ void __launch_bounds__(kXmThreads)
   const uint8_t* km = key_mask == nullptr ? nullptr : key_mask + static_cast<long long>(b) * Lk;
 
   // Keys and values are encoder products, constant while decoding: this CTA's part of them is
-  // pulled toward L2 while the kernel before this one (which produces q) may still be running.
+  // pulled toward L2 while the kernel before this one (which produces q) may still be running. (Where nothing
+  // runs before, the requests only get into the way of the loads: 56.9 / 52.3 us for the shape above.)
   chain_release();
-  for (int line = threadIdx.x; line < Lp; line += kXmThreads) {  // Lp x 128 bytes each
+  const int nchunks = Lp / 32;
+  uint32_t shown = 0xffffffffu;
+  if (kLook && km != nullptr) {  // (constant, too)
+    if (threadIdx.x == 0) s_shown = 0u;
+    uint32_t mine = 0u;
+    for (int c = warp; c < nchunks; c += kXmWarps) {
+      const int key = c * 32 + lane;
+      if (__any_sync(0xffffffffu, key < Lk && km[key] != 0)) mine |= 1u << c;
+    }
+    __syncthreads();
+    if (lane == 0 && mine != 0u) atomicOr(&s_shown, mine);
+    __syncthreads();
+    shown = s_shown;
+  }
+  for (int line = threadIdx.x; !kLook && line < Lp; line += kXmThreads) {  // Lp x 128 bytes each
     prefetch_l2(reinterpret_cast<const char*>(kb) + static_cast<long long>(line) * 128);
     prefetch_l2(reinterpret_cast<const char*>(vb) + static_cast<long long>(line) * 128);
   }
@@ -98,7 +121,6 @@ __global__ void __launch_bounds__(kXmThreads)
   }
 
   // ---- scores: chunks of 32 keys; every warp takes a contiguous run of chunks ----
-  const int nchunks = Lp / 32;
   const int per_warp = (nchunks + kXmWarps - 1) / kXmWarps;
   const int first = warp * per_warp;
   const int mine = max(0, min(per_warp, nchunks - first));
@@ -111,7 +133,12 @@ __global__ void __launch_bounds__(kXmThreads)
     uint4 kr[kBatch][4][2];
 #pragma unroll
     for (int c = 0; c < kBatch; ++c) {
-      const int base = (first + min(i0 + c, mine - 1)) * 32;
+      const int chunk = first + min(i0 + c, mine - 1), base = chunk * 32;
+      if (kLook && !((shown >> chunk) & 1u)) {
+#pragma unroll
+        for (int ut = 0; ut < 4; ++ut) kr[c][ut][0] = kr[c][ut][1] = make_uint4(0u, 0u, 0u, 0u);
+        continue;
+      }
 #pragma unroll
       for (int ut = 0; ut < 4; ++ut) {
         const int key = base + key_of_column(ut >> 1, ut & 1, g);  // the row this lane group loads
@@ -165,10 +192,12 @@ __global__ void __launch_bounds__(kXmThreads)
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
   float sum = 0.f;
+  const bool all = !kLook || __any_sync(0xffffffffu, g < BEAMS && mx < -5e9f);  // no key is visible
 #pragma unroll
   for (int i = 0; i < kXmMaxChunks; ++i) {
     if (i >= mine) break;
     const int base = (first + i) * 32;
+    if (!all && !((shown >> (first + i)) & 1u)) continue;
     uint4 vv[8];
 #pragma unroll
     for (int n = 0; n < 8; ++n)
@@ -241,19 +270,23 @@ T5X_API int t5x_decode_cross_attention_mma(const void* q, const void* k, const v
   auto vp = static_cast<const __nv_bfloat16*>(vt);
   auto mp = static_cast<const uint8_t*>(key_mask);
   auto op = static_cast<__nv_bfloat16*>(out);
+  const bool look = !chained_launches();
+  const auto go = [&](auto kernel) {
+    return launch_chained(kernel, grid, dim3(kXmThreads), 0, st, qp, kp, vp, mp, op, q_ld, heads, Lk, Lp);
+  };
   cudaError_t le = cudaSuccess;
   switch (beams) {
     case 1:
-      le = launch_chained(decode_cross_mma_kernel<1>, grid, dim3(kXmThreads), 0, st, qp, kp, vp, mp, op, q_ld, heads, Lk, Lp);
+      le = look ? go(decode_cross_mma_kernel<1, true>) : go(decode_cross_mma_kernel<1, false>);
       break;
     case 2:
-      le = launch_chained(decode_cross_mma_kernel<2>, grid, dim3(kXmThreads), 0, st, qp, kp, vp, mp, op, q_ld, heads, Lk, Lp);
+      le = look ? go(decode_cross_mma_kernel<2, true>) : go(decode_cross_mma_kernel<2, false>);
       break;
     case 4:
-      le = launch_chained(decode_cross_mma_kernel<4>, grid, dim3(kXmThreads), 0, st, qp, kp, vp, mp, op, q_ld, heads, Lk, Lp);
+      le = look ? go(decode_cross_mma_kernel<4, true>) : go(decode_cross_mma_kernel<4, false>);
       break;
     case 8:
-      le = launch_chained(decode_cross_mma_kernel<8>, grid, dim3(kXmThreads), 0, st, qp, kp, vp, mp, op, q_ld, heads, Lk, Lp);
+      le = look ? go(decode_cross_mma_kernel<8, true>) : go(decode_cross_mma_kernel<8, false>);
       break;
     default:
       return set_error("decode_cross_attention_mma: beams must be 1, 2, 4 or 8 (got %d)", beams);
