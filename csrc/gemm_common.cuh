@@ -34,6 +34,9 @@ enum GemmEpilogue : int {
   // The product is the gradient of gelu(h0) * h1 and never stored either: h0 and h1 (in H0 and H1) become
   // their gradients.
   kEpiGatedGrad = 5,
+  // CTA pairs only: ReLU of the product; the product where R is positive, zero elsewhere (ReLU's gradient).
+  kEpiRelu = 6,
+  kEpiReluGrad = 7,
 };
 
 // Several products in one launch, three at most (the projections that share an input).
@@ -287,6 +290,22 @@ __device__ __forceinline__ void staged_load_bf16(float* stage, const __nv_bfloat
   __syncwarp();
 }
 
+__device__ __forceinline__ void staged_keep_positive(const float* stage, float (&v)[32], int lane) {
+  const uint4* st4 = reinterpret_cast<const uint4*>(stage);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const uint4 u = st4[lane * 8 + (c ^ (lane & 7))];
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __bfloat1622float2(h[j]);
+      v[c * 8 + j * 2] = f.x > 0.f ? v[c * 8 + j * 2] : 0.f;
+      v[c * 8 + j * 2 + 1] = f.y > 0.f ? v[c * 8 + j * 2 + 1] : 0.f;
+    }
+  }
+  __syncwarp();  // the block may be overwritten
+}
+
 __device__ __forceinline__ void staged_add_row(const float* stage, float (&v)[32], int lane) {
   const uint4* st4 = reinterpret_cast<const uint4*>(stage);
 #pragma unroll
@@ -435,7 +454,8 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, const Ge
   } else {
     const bool f32_vec_ok = o.ldc % 4 == 0 && p.c_batch_stride % 4 == 0 &&
                             (reinterpret_cast<uintptr_t>(o.C) & 15) == 0;
-    const bool r_vec_ok = EPI == kEpiResidual && p.ldr % 8 == 0 && p.r_batch_stride % 8 == 0 &&
+    constexpr bool kReadsR = EPI == kEpiResidual || EPI == kEpiReluGrad;
+    const bool r_vec_ok = kReadsR && p.ldr % 8 == 0 && p.r_batch_stride % 8 == 0 &&
                           (reinterpret_cast<uintptr_t>(p.R) & 15) == 0;
 #pragma unroll 1
     for (int c = part * (BN / 32 / PARTS); c < (part + 1) * (BN / 32 / PARTS); ++c) {
@@ -449,7 +469,7 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, const Ge
                           (p.out_fp32 ? f32_vec_ok
                                       : (c_vec_ok && (accumulate == 0 || EPI != kEpiResidual)));
       if (staged) {
-        if (EPI == kEpiResidual && r_vec_ok)
+        if (kReadsR && r_vec_ok)
           staged_load_bf16(stage, p.R + b * p.r_batch_stride +
                                       static_cast<long long>(m0 + q * 32) * p.ldr + col,
                            p.ldr, rows_valid, lane);
@@ -466,6 +486,17 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, const Ge
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
         if (add_c) staged_add_row(stage, v, lane);
+        if (EPI == kEpiRelu) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = v[i] < 0.f ? 0.f : v[i];  // (a NaN stays)
+        }
+        if (EPI == kEpiReluGrad && r_vec_ok) staged_keep_positive(stage, v, lane);
+        if (EPI == kEpiReluGrad && !r_vec_ok && row_ok) {
+          float rr[32];
+          load_row_bf16(p.R + b * p.r_batch_stride + static_cast<long long>(row) * p.ldr + col, rr, n_valid, false);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = rr[i] > 0.f ? v[i] : 0.f;
+        }
         if (EPI == kEpiResidual) {
           if (r_vec_ok) {
             staged_add_row(stage, v, lane);
@@ -495,6 +526,17 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, const Ge
         float v[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
+        if (EPI == kEpiRelu) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = v[i] < 0.f ? 0.f : v[i];
+        }
+        if (EPI == kEpiReluGrad) {
+          float rr[32];
+          load_row_bf16(p.R + b * p.r_batch_stride + static_cast<long long>(row) * p.ldr + col, rr, n_valid,
+                        r_vec_ok);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = rr[i] > 0.f ? v[i] : 0.f;
+        }
         if (EPI == kEpiResidual) {
           float rr[32];
           load_row_bf16(p.R + b * p.r_batch_stride + static_cast<long long>(row) * p.ldr + col,

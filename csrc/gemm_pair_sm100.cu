@@ -579,6 +579,12 @@ static int launch_pair_mode(int epilogue, const GemmMaps<false>& maps, GemmParam
     case kEpiCeGrad:
       if (MODE != kTpNone) break;
       return launch_pair<kEpiCeGrad, kTpNone>(maps, p, tp, max_ctas, stream);
+    case kEpiRelu:
+      if (MODE != kTpNone) break;
+      return launch_pair<kEpiRelu, kTpNone>(maps, p, tp, max_ctas, stream);
+    case kEpiReluGrad:
+      if (MODE != kTpNone) break;
+      return launch_pair<kEpiReluGrad, kTpNone>(maps, p, tp, max_ctas, stream);
     case kEpiGatedGrad:
       if (MODE != kTpNone) break;
       return launch_pair<kEpiGatedGrad, kTpNone>(maps, p, tp, max_ctas, stream);

@@ -637,6 +637,56 @@ std::vector<Tensor> mlp_block(const Tensor& x, const Tensor& scale, double eps,
   return {y, h, rstd, g, pre};
 }
 
+// The same with one ReLU: y = x + relu(h wi) wo, weights wi, wo; (y, h, rstd, g). Covered where the products can
+// do the activation and its gradient themselves.
+bool relu_block_ok(const Tensor& x, const Tensor& scale, const std::vector<Tensor>& w) {
+  if (x.dim() < 2 || !plain(x) || !rows_fit(x) || !norm_ok(scale, x) || w.size() != 2 || w[0].dim() != 2)
+    return false;
+  const Weight a(w[0], x.size(-1));
+  if (!a.ok || !t5x_gemm_gated_grad_covers(rows_of(x), a.n)) return false;
+  const Weight o(w[1], a.n);
+  return o.ok && o.n == x.size(-1);
+}
+bool relu_grads_ok(const Tensor& x, const std::vector<Tensor>& w, const std::vector<optional<Tensor>>& g) {
+  const Weight a(w[0], x.size(-1)), o(w[1], a.n);
+  return grad_ok(g[0], a, rows_of(x)) && grad_ok(g[1], o, rows_of(x)) && !overlap(*g[0], *g[1]);
+}
+std::vector<Tensor> relu_block(const Tensor& x, const Tensor& scale, double eps, const std::vector<Tensor>& weights,
+                               bool keep) {
+  if (!relu_block_ok(x, scale, weights)) throw std::invalid_argument("relu_block: operands are not covered");
+  void* st = stream_of();
+  auto [h, rstd] = norm_forward(x, scale, eps, st);
+  const int64_t m = rows_of(x), d = x.size(-1);
+  const Weight a(weights[0], d), wo(weights[1], a.n);
+  Tensor g = at::empty({m, a.n}, x.options());
+  check(t5x_gemm_relu(h.data_ptr(), a.t.data_ptr(), g.data_ptr(), nullptr, m, a.n, d, d, a.ld, a.n, 0, 1, st),
+        "gemm_relu");
+  Tensor y = at::empty_like(x);
+  forward(g, m, wo, &x, y, st);
+  if (!keep) return {y};
+  return {y, h, rstd, g};
+}
+Tensor relu_block_bwd(const Tensor& dy, const Tensor& x, const Tensor& scale, const std::vector<Tensor>& weights,
+                      const std::vector<Tensor>& saved, const std::vector<Tensor>& grads,
+                      const std::vector<bool>& accumulate, Tensor dscale) {
+  const Tensor &h = saved[0], &rstd = saved[1], &g = saved[2];
+  const std::vector<optional<Tensor>> have(grads.begin(), grads.end());
+  if (!plain(dy) || dy.numel() != x.numel() || !relu_block_ok(x, scale, weights) || !relu_grads_ok(x, weights, have))
+    throw std::invalid_argument("relu_block_bwd: operands are not covered");
+  void* st = stream_of();
+  const int64_t m = rows_of(x), d = x.size(-1);
+  const Weight a(weights[0], d), wo(weights[1], a.n);
+  Tensor dg = at::empty_like(g);
+  optional<Tensor> dh = at::empty_like(x);
+  check(t5x_gemm_relu(dy.data_ptr(), wo.t.data_ptr(), dg.data_ptr(), g.data_ptr(), m, a.n, wo.n, wo.n, wo.ld, a.n,
+                      a.n, 0, st),
+        "gemm_relu");
+  Tensor gwo = grads[1];
+  weight_grad(g, dy.data_ptr(), wo.n, m, wo, gwo, accumulate[1], st);
+  backward_products(h, m, {dg.data_ptr()}, {a.n}, {a}, dh, {grads[0]}, {accumulate[0]}, st);
+  return norm_backward(*dh, x, scale, rstd, dy, dscale, st);
+}
+
 // Input gradient of mlp_block; the saved pre-activations are overwritten with their gradients.
 Tensor mlp_block_bwd(const Tensor& dy, const Tensor& x, const Tensor& scale,
                      const std::vector<Tensor>& weights, const std::vector<Tensor>& saved,
@@ -692,4 +742,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("mlp_grads_ok", mlp_grads_ok);
   m.def("mlp_block", torch::wrap_pybind_function_no_gil(mlp_block));
   m.def("mlp_block_bwd", torch::wrap_pybind_function_no_gil(mlp_block_bwd));
+  m.def("relu_block_ok", relu_block_ok);
+  m.def("relu_grads_ok", relu_grads_ok);
+  m.def("relu_block", torch::wrap_pybind_function_no_gil(relu_block));
+  m.def("relu_block_bwd", torch::wrap_pybind_function_no_gil(relu_block_bwd));
 }

@@ -70,7 +70,8 @@ def _mlp_half(x, norm, mlp, dropout_rate: float):
   if dropout_rate > 0:
     x, h = norm(x, with_residual=True)
     return x + _dropout(mlp(h, enable_dropout=True), dropout_rate, True)
-  y = blocks.gated_mlp(x, norm, mlp, layers.LayerNorm, layers.MlpBlock, layers.DenseGeneral)
+  block = blocks.relu_mlp if getattr(mlp, "activations", None) == ("relu",) else blocks.gated_mlp
+  y = block(x, norm, mlp, layers.LayerNorm, layers.MlpBlock, layers.DenseGeneral)
   if y is not None:
     return y
   x, h = norm(x, with_residual=True)

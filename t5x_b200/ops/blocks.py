@@ -1,10 +1,11 @@
-"""Residual blocks of a T5 layer (norm, projections, attention or gated MLP, residual) as one call.
+"""Residual blocks of a T5 layer (norm, projections, attention or MLP, residual) as one call.
 
 What bounds it: a pass of a small model, or over one sentence, waits for the host. Op by op a block
 is five to eight module calls, four or five autograd nodes and as many calls into the library, 20 to
 40 us each on the host for kernels of 3 to 8 us. Here a block is one autograd node whose forward and
 backward are one compiled call each (csrc/host/host_ops.cpp); without gradients it is the call alone.
-The kernels and their order are those of the op by op path. (One sentence scored by T5.1.1 small,
+The kernels and their order are those of the op by op path, but that of wide enough MLPs the products do the
+activation and its gradient themselves. (One sentence scored by T5.1.1 small,
 8 + 8 layers: 3.83 ms op by op, 1.97 so, with the cheaper `_owns` of models/base.py; a training step of
 one small layer pair 3.48, 2.71.)
 
@@ -119,6 +120,28 @@ def gated_mlp(x, norm, mlp, norm_cls, mlp_cls, dense_cls) -> Optional[torch.Tens
   return _GatedMlpBlockFn.apply(x, scale, *params, norm.epsilon)
 
 
+def relu_mlp(x, norm, mlp, norm_cls, mlp_cls, dense_cls) -> Optional[torch.Tensor]:
+  """x + mlp(norm(x)) for the MLP of one ReLU, or None where it is not covered."""
+  host, recording = _host_for(x)
+  if (host is None or type(mlp) is not mlp_cls or mlp.activations != ("relu",) or
+      not _unhooked(mlp) or not _norm_ok(norm, norm_cls) or mlp.dtype is not torch.bfloat16):
+    return None
+  params = _kernels(mlp, ("wi", "wo"), dense_cls)
+  if params is None:
+    return None
+  scale = norm._parameters["scale"]
+  weights = [F.compute_weight(p, torch.bfloat16) for p in params]
+  if not host.relu_block_ok(x, scale, weights):
+    return None
+  if not recording:
+    return host.relu_block(x, scale, norm.epsilon, weights, False)[0]
+  grads = [_usable_grad(p) for p in params]
+  if any(g is None for g in grads) or _usable_grad(scale) is None or \
+      not host.relu_grads_ok(x, weights, grads):
+    return None
+  return _ReluMlpBlockFn.apply(x, scale, *params, norm.epsilon)
+
+
 class _Buffers:
   """Where a backward pass writes the gradients of `params` (weights first, `extra` small ones after
   them that are added to): their fp32 buffers, or, where a buffer has gone since the forward pass, a
@@ -211,3 +234,32 @@ class _GatedMlpBlockFn(torch.autograd.Function):
         F._restore_grad_flags(params + [scale], flags)
     dw = buf.results()
     return (dx, dw[3], *dw[:3], None)
+
+
+class _ReluMlpBlockFn(torch.autograd.Function):
+
+  @staticmethod
+  def forward(ctx, x, scale, wi, wo, eps):
+    weights = [F.compute_weight(w, torch.bfloat16) for w in (wi, wo)]
+    y, *saved = native.host().relu_block(x, scale, eps, weights, True)
+    ctx.save_for_backward(x, scale, wi, wo, *saved)
+    return y
+
+  @staticmethod
+  def backward(ctx, dy):
+    x, scale, wi, wo, *saved = ctx.saved_tensors
+    params = [wi, wo]
+    flags = [bool(getattr(p, "grad_ready", False)) for p in params + [scale]]
+    done = False
+    try:
+      buf = _Buffers(params, [scale])
+      grads, accumulate = buf.weights(2)
+      dx = native.host().relu_block_bwd(dy.contiguous(), x, scale,
+                                        [F.compute_weight(w, torch.bfloat16) for w in params], saved, grads,
+                                        accumulate, buf.out[2])
+      done = True
+    finally:
+      if not done:
+        F._restore_grad_flags(params + [scale], flags)
+    dw = buf.results()
+    return (dx, dw[2], *dw[:2], None)

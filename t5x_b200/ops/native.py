@@ -133,7 +133,7 @@ class _HostOps:
   NAMES = ("linear", "multi_linear", "multi_linear_bwd", "gated_in", "gated_in_bwd", "rmsnorm",
            "rmsnorm_bwd", "attention", "attention_bwd", "attention_block_ok", "attention_grads_ok",
            "attention_block", "attention_block_bwd", "mlp_block_ok", "mlp_grads_ok", "mlp_block",
-           "mlp_block_bwd")
+           "mlp_block_bwd", "relu_block_ok", "relu_grads_ok", "relu_block", "relu_block_bwd")
 
   def __init__(self, module):
     for name in self.NAMES:
@@ -751,6 +751,7 @@ register_signature("t5x_gemm_ce_grad", [c_void_p, c_void_p, c_void_p, c_ll, c_in
                                         c_void_p, c_void_p, c_float, c_float, c_float, c_void_p])
 register_signature("t5x_gemm_gated_grad", [c_void_p] * 4 + [c_int] * 3 + [c_ll] * 3 + [c_int, c_void_p])
 register_signature("t5x_gemm_gated_grad_covers", [c_int, c_int])
+register_signature("t5x_gemm_relu", [c_void_p] * 4 + [c_int] * 3 + [c_ll] * 4 + [c_int, c_void_p])
 register_signature("t5x_ce_merge", [c_void_p] * 7 + [c_int, c_int, c_int, c_int, c_void_p])
 
 
