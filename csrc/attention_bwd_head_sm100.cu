@@ -11,13 +11,13 @@
 // unit u in registers, and the gradient products of unit u - 1 while they do their arithmetic on unit u; the
 // softmax warps never wait for one another inside the walk.
 //
-//
 // One CTA per 128-key block (attention_sm100.cu) spends 14k cycles on setting up and tearing down a CTA and
 // 6.7k on a 128 x 128 tile. Here a CTA takes 16k and a 128 x 64 unit 2 to 3k, bound by what a softmax warp does
 // one after the other for a unit (us, with rowsum(dO * O), clearing and casting of dQ where there are any,
 // before / now: 128 x 12 heads x 512 x 512 1081 / 610, 114 x 512 without a bias 385 / 202, 114 x 114 causal
-// 184 / 113, 24 x 12 x 509 packed 258 / 157, 32 x 64 x 512 x 512 1327 / 792). Of the 610, the bias gradient takes 100 (40 its additions to
-// shared memory, which are loops around a compare-and-swap), the bias 35, the exponentials 8.
+// 184 / 113, 24 x 12 x 509 packed 258 / 157, 32 x 64 x 512 x 512 1327 / 792). Of the 610, the bias gradient
+// takes 100 (40 its additions to shared memory, which are loops around a compare-and-swap), the bias 35, the
+// exponentials 8.
 #include <type_traits>
 
 #include "attention_common.cuh"

@@ -34,7 +34,8 @@ enum GemmEpilogue : int {
   // The product is the gradient of gelu(h0) * h1 and never stored either: h0 and h1 (in H0 and H1) become
   // their gradients.
   kEpiGatedGrad = 5,
-  // CTA pairs only: ReLU of the product; the product where R is positive, zero elsewhere (ReLU's gradient).
+  // CTA pairs only: ReLU of the product; the product, zero where R is not positive (ReLU's gradient; a NaN in R
+  // lets it through, as torch does).
   kEpiRelu = 6,
   kEpiReluGrad = 7,
 };
@@ -299,8 +300,8 @@ __device__ __forceinline__ void staged_keep_positive(const float* stage, float (
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float2 f = __bfloat1622float2(h[j]);
-      v[c * 8 + j * 2] = f.x > 0.f ? v[c * 8 + j * 2] : 0.f;
-      v[c * 8 + j * 2 + 1] = f.y > 0.f ? v[c * 8 + j * 2 + 1] : 0.f;
+      v[c * 8 + j * 2] = f.x <= 0.f ? 0.f : v[c * 8 + j * 2];
+      v[c * 8 + j * 2 + 1] = f.y <= 0.f ? 0.f : v[c * 8 + j * 2 + 1];
     }
   }
   __syncwarp();  // the block may be overwritten
@@ -495,7 +496,7 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, const Ge
           float rr[32];
           load_row_bf16(p.R + b * p.r_batch_stride + static_cast<long long>(row) * p.ldr + col, rr, n_valid, false);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = rr[i] > 0.f ? v[i] : 0.f;
+          for (int i = 0; i < 32; ++i) v[i] = rr[i] <= 0.f ? 0.f : v[i];
         }
         if (EPI == kEpiResidual) {
           if (r_vec_ok) {
@@ -535,7 +536,7 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmParams& p, const Ge
           load_row_bf16(p.R + b * p.r_batch_stride + static_cast<long long>(row) * p.ldr + col, rr, n_valid,
                         r_vec_ok);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = rr[i] > 0.f ? v[i] : 0.f;
+          for (int i = 0; i < 32; ++i) v[i] = rr[i] <= 0.f ? 0.f : v[i];
         }
         if (EPI == kEpiResidual) {
           float rr[32];

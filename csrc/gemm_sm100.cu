@@ -981,8 +981,8 @@ T5X_API int t5x_gemm_gated_grad(const void* dy, const void* B, void* h0, void* h
                    kEpiGatedGrad, nullptr, 0, 0, h0, h1, ldh, 1.f, 0, stream, nullptr, 0);
 }
 
-// C[M, N] (bf16) = relu(A[M, K] @ B[K, N]), or with `positive` (bf16 [M, N], rows ldp apart) the product where that is
-// positive and zero elsewhere: the gradient of a ReLU whose output it is. Sizes as t5x_gemm_gated_grad_covers has
+// C[M, N] (bf16) = relu(A[M, K] @ B[K, N]), or with `positive` (bf16 [M, N], rows ldp apart) the product, zero where
+// that is zero or negative: the gradient of a ReLU whose output it is. Sizes as t5x_gemm_gated_grad_covers has
 // them. (A pass of its own reads and writes the activations, its gradient reads two tensors and writes one: 8192 x
 // 1024 x 16384, us, product and pass / in one: forward 286 / 214, backward 312 / 256.)
 T5X_API int t5x_gemm_relu(const void* A, const void* B, void* C, const void* positive, int M, int N, int K,

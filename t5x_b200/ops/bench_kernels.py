@@ -76,7 +76,7 @@ def bench_gemm(pair_modes=(0, 1)):
 
 
 def bench_attention():
-  """Forward (both kernels where the short-range one applies) and forward + backward times of
+  """Forward (both kernels where that of head_dim 64 applies) and forward + backward times of
   the flash-attention kernels with the T5 relative bias, against torch SDPA without a bias."""
   import os
   from t5x_b200.ops import attention as attn

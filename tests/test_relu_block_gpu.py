@@ -15,6 +15,7 @@ def test_product_with_relu(m, n, k):
   rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
   a, w, act = rnd(m, k), rnd(k, n), rnd(m, n).relu()
   act[::3, ::5] = 0.0
+  act[1, 1:40] = float("nan")
   a[0, 0] = float("nan")
   for positive in (None, act):
     out = torch.full((m, n), 7.0, device="cuda").bfloat16()
@@ -22,7 +23,7 @@ def test_product_with_relu(m, n, k):
                                              k, k, n, n, n, 1, native.stream_ptr()), "gemm_relu")
     native.check_status()
     want = a.double() @ w.double()
-    want = want.relu() if positive is None else want * (positive > 0)
+    want = want.relu() if positive is None else want * ~(positive <= 0)
     if positive is None:
       assert bool(out[0].isnan().all())  # as torch's
     else:
