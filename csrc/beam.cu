@@ -314,6 +314,13 @@ __global__ void __launch_bounds__(kBeamThreads) beam_update_kernel(const BeamSta
     }
   }
   __syncthreads();
+  // Where an example has fewer than K2 candidates (logits of NaN or minus infinity), what is missing is a token of
+  // beam 0 that ends nothing, at the lowest score: the marker "no candidate" is no place to read from.
+  auto take = [&](int r, float v, int f) {
+    const bool none = f == 0x7fffffff;
+    top_lp[r] = none ? -FLT_MAX : v;
+    top_flat[r] = none ? (st.eos == 0 ? 1 : 0) : f;
+  };
   // best K2 over beams x vocabulary, descending: by one warp from its registers where they hold the candidates, as
   // block-wide rounds cost three barriers each (64 x 4 beams x 32128, us for the launch: 15.9 / 14.8)
   constexpr int kHeld = 16;
@@ -344,10 +351,7 @@ __global__ void __launch_bounds__(kBeamThreads) beam_update_kernel(const BeamSta
             cv[j] = -FLT_MAX;
             cf[j] = 0x7fffffff;
           }
-        if (tid == 0) {
-          top_lp[r] = v;
-          top_flat[r] = f;
-        }
+        if (tid == 0) take(r, v, f);
       }
     }
     __syncthreads();
@@ -363,10 +367,7 @@ __global__ void __launch_bounds__(kBeamThreads) beam_update_kernel(const BeamSta
     block_best(v, f, red_v, red_i);
     for (int c = tid; c < ncand; c += kBeamThreads)
       if (cflat[c] == f) cscore[c] = -FLT_MAX, cflat[c] = 0x7fffffff;
-    if (tid == 0) {
-      top_lp[r] = v;
-      top_flat[r] = f;
-    }
+    if (tid == 0) take(r, v, f);
     __syncthreads();
   }
   if (tid == 0) {

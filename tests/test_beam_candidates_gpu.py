@@ -39,3 +39,28 @@ def test_candidates(beams, kind, vocab):
   want = torch.stack([flat[i][[int(j) for j in order[i] if int(j) % vocab != eos][:beams][::-1]] for i in range(b)])
   # 32-bit sums of up to 4096 exponentials, and their logarithm
   torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("beams,vocab", [(1, 37), (4, 300), (4, 9001), (8, 20000)])
+@pytest.mark.parametrize("eos", [1, 0])
+def test_examples_without_enough_candidates(beams, vocab, eos):
+  """An example of NaNs, one with a single finite logit per row and one with none: parents stay among the beams and
+  tokens in the vocabulary, and the other examples are what they are by themselves."""
+  from t5x_b200.ops import native
+  g = torch.Generator(device="cuda").manual_seed(vocab)
+  dev, b, steps = torch.device("cuda"), 5, 4
+  st, alone = _State(b, beams, steps + 2, eos, 0.6, dev), _State(2, beams, steps + 2, eos, 0.6, dev)
+  for _ in range(steps):
+    x = torch.randn(b, beams, vocab, device="cuda", generator=g) * 3
+    x[1] = float("nan")
+    x[2, :, 1:] = float("-inf")
+    x[3] = float("-inf")
+    st.d._beam_step(x.view(b * beams, vocab).clone())
+    alone.d._beam_step(x[[0, 4]].view(2 * beams, vocab).clone())
+    s, a = st.snapshot(), alone.snapshot()
+    for n in ("anc", "live_seqs", "fin_seqs"):
+      assert int(s[n].min()) >= 0 and int(s[n].max()) < (beams if n == "anc" else vocab), n
+    for n in ("live_seqs", "anc", "fin_seqs", "live_lp", "fin_scores", "fin_flags"):
+      assert torch.equal(s[n][[0, 4]], a[n]), n
+  assert int(s["cur"]) == steps
+  native.check_status()
