@@ -661,7 +661,8 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SamplePara
       if (cand_better(x[i], i, v, bi)) v = x[i], bi = i;
     block_best(v, bi, red_v, red_i);
     if (threadIdx.x == 0) {
-      p.tokens[row] = bi;
+      // (a row of NaNs or minus infinities alone has no best entry: token 0, here and below)
+      p.tokens[row] = bi == 0x7fffffff ? 0 : bi;
       p.log_probs[row] = p.rescale_log_probs ? 0.f : v - lse_raw;
     }
     return;
@@ -686,6 +687,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SamplePara
   z = block_sum(z, red);
   block_best(best, best_i, red_v, red_i);
   if (threadIdx.x == 0) {
+    if (best_i == 0x7fffffff) best_i = 0;
     p.tokens[row] = best_i;
     const float xt = x[best_i];
     p.log_probs[row] = p.rescale_log_probs ? (xt * inv_t - (m_scaled + logf(z))) : (xt - lse_raw);
