@@ -1,5 +1,6 @@
 // Declarations shared by the attention kernels: forward, attention_fwd_rows_sm100.cu (64 channels, up to 2048
-// keys) and attention_fwd_sm100.cu (any length, 64 or 128 channels); backward, attention_bwd_head_sm100.cu (64
+// keys), attention_fwd_few_sm100.cu (the same for few heads and up to 512) and attention_fwd_sm100.cu (any
+// length, 64 or 128 channels); backward, attention_bwd_head_sm100.cu (64
 // channels, where there are heads enough) and attention_sm100.cu.
 #pragma once
 #include "common.cuh"

@@ -356,17 +356,19 @@ struct Masks {
   const void* bucket_data() const { return rel_bias ? buckets->data_ptr() : nullptr; }
 };
 
-void attention_into(const Tensor& q, const Tensor& k, const Tensor& v, const Masks& m, bool short_range,
+// `kernel`: 0, 1 or 2, of KERNELS in t5x_b200/ops/attention.py.
+void attention_into(const Tensor& q, const Tensor& k, const Tensor& v, const Masks& m, int64_t kernel,
                     Tensor& o, Tensor& lse, void* st) {
   const int B = q.size(0), Lq = q.size(1), H = q.size(2), D = q.size(3), Lk = k.size(1);
-  if (short_range)
-    check(t5x_attention_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), B,
-                            H, Lq, Lk, q.stride(0), q.stride(1), q.stride(2), k.stride(0),
-                            k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2),
-                            o.stride(0), o.stride(1), o.stride(2), data_or_null(m.rel_bias),
-                            m.bucket_data(), m.num_buckets(), m.nrel(), m.rel_off,
-                            data_or_null(m.key_mask), data_or_null(m.q_seg), data_or_null(m.kv_seg),
-                            m.causal, m.causal_off, st),
+  if (kernel != 0)
+    check((kernel == 2 ? t5x_attention_fwd_few : t5x_attention_fwd)(
+              q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), B,
+              H, Lq, Lk, q.stride(0), q.stride(1), q.stride(2), k.stride(0),
+              k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2),
+              o.stride(0), o.stride(1), o.stride(2), data_or_null(m.rel_bias),
+              m.bucket_data(), m.num_buckets(), m.nrel(), m.rel_off,
+              data_or_null(m.key_mask), data_or_null(m.q_seg), data_or_null(m.kv_seg),
+              m.causal, m.causal_off, st),
           "attention_fwd");
   else
     check(t5x_attention_fwd_stream(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
@@ -384,12 +386,12 @@ optional<std::tuple<Tensor, Tensor>> attention(
     const Tensor& q, const Tensor& k, const Tensor& v, const optional<Tensor>& rel_bias,
     const optional<Tensor>& buckets, const optional<Tensor>& key_mask, const optional<Tensor>& q_seg,
     const optional<Tensor>& kv_seg, int64_t causal, int64_t causal_off, int64_t rel_off,
-    bool short_range) {
+    int64_t kernel) {
   if (!heads_ok(q) || !heads_ok(k) || !heads_ok(v)) return std::nullopt;
   Tensor o = at::empty(q.sizes(), q.options());
   Tensor lse = at::empty({q.size(0), q.size(2), q.size(1)}, q.options().dtype(at::kFloat));
   attention_into(q, k, v, {rel_bias, buckets, key_mask, q_seg, kv_seg, causal, causal_off, rel_off},
-                 short_range, o, lse, stream_of());
+                 kernel, o, lse, stream_of());
   return std::make_tuple(o, lse);
 }
 
@@ -545,7 +547,7 @@ std::vector<Tensor> attention_block(const Tensor& x, const optional<Tensor>& kv,
                                     const optional<Tensor>& buckets, const optional<Tensor>& key_mask,
                                     const optional<Tensor>& q_seg,
                                     const optional<Tensor>& kv_seg, int64_t causal, int64_t causal_off,
-                                    int64_t rel_off, bool short_range) {
+                                    int64_t rel_off, int64_t kernel) {
   if (!attention_block_ok(x, kv, scale, weights, heads, head_dim))
     throw std::invalid_argument("attention_block: operands are not covered");
   void* st = stream_of();
@@ -565,7 +567,7 @@ std::vector<Tensor> attention_block(const Tensor& x, const optional<Tensor>& kv,
   Tensor o = at::empty({B, Lq, heads, head_dim}, x.options());
   Tensor lse = at::empty({B, heads, Lq}, x.options().dtype(at::kFloat));
   attention_into(out[0], out[1], out[2],
-                 {rel_bias, buckets, key_mask, q_seg, kv_seg, causal, causal_off, rel_off}, short_range, o,
+                 {rel_bias, buckets, key_mask, q_seg, kv_seg, causal, causal_off, rel_off}, kernel, o,
                  lse, st);
   Tensor y = at::empty_like(x);
   forward(o, B * Lq, wo, &x, y, st);

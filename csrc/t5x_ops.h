@@ -21,6 +21,13 @@ int t5x_attention_fwd(const void* q, const void* k, const void* v, void* o, void
                       const void* rel_bucket, int num_buckets, int nrel, int rel_off,
                       const void* key_mask, const void* q_seg, const void* kv_seg, int causal,
                       int causal_off, void* stream);
+int t5x_attention_fwd_few(const void* q, const void* k, const void* v, void* o, void* lse, int B, int H,
+                          int Lq, int Lk, long long q_sb, long long q_sl, long long q_sh, long long k_sb,
+                          long long k_sl, long long k_sh, long long v_sb, long long v_sl, long long v_sh,
+                          long long o_sb, long long o_sl, long long o_sh, const void* rel_bias,
+                          const void* rel_bucket, int num_buckets, int nrel, int rel_off,
+                          const void* key_mask, const void* q_seg, const void* kv_seg, int causal,
+                          int causal_off, void* stream);
 int t5x_attention_fwd_stream(const void* q, const void* k, const void* v, void* o, void* lse, int B,
                              int H, int Lq, int Lk, int D, long long q_sb, long long q_sl,
                              long long q_sh, long long k_sb, long long k_sl, long long k_sh,

@@ -10,6 +10,7 @@ backward, 27 to 57 us a layer for the sort-based index backward alone.)
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional
 
 import torch
@@ -18,9 +19,10 @@ from t5x_b200.ops import native
 from t5x_b200.ops import reference as ref
 
 c_void_p, c_int, c_ll = native.c_void_p, native.c_int, native.c_ll
-native.register_signature("t5x_attention_fwd", [c_void_p] * 5 + [c_int] * 4 + [c_ll] * 12 +
-                          [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
-                           c_int, c_int, c_void_p])
+for _name in ("t5x_attention_fwd", "t5x_attention_fwd_few"):
+  native.register_signature(_name, [c_void_p] * 5 + [c_int] * 4 + [c_ll] * 12 +
+                            [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                             c_int, c_int, c_void_p])
 native.register_signature("t5x_attention_bwd", [c_void_p] * 10 + [c_int] * 5 + [c_ll] * 18 +
                           [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
                            c_void_p, c_int, c_int, c_void_p])
@@ -34,20 +36,36 @@ native.register_signature("t5x_attention_bwd_head", [c_void_p] * 11 + [c_int] * 
                            c_void_p, c_int, c_int, c_void_p])
 native.register_signature("t5x_attention_bwd_head_covers", [c_int] * 6)
 
-# The forward kernel for head_dim 64 keeps the bias by relative position of all keys in shared memory.
-CLASSIC_MAX_LK = 2048
+# The forward kernel for head_dim 64 keeps the bias by relative position of all keys in shared memory, that for few
+# heads the scores of all keys in TMEM.
+CLASSIC_MAX_LK, FEW_MAX_LQ, FEW_MAX_LK = 2048, 256, 512
+KERNELS = {"stream": 0, "classic": 1, "few": 2}  # as csrc/host/host_ops.cpp has them
 # The backward kernel keeps bias-gradient bins for the whole query range in shared memory.
 BWD_MAX_LQ = 4096
 
 
-def forward_kernel(Lq: int, Lk: int, D: int, prefix_lm: bool = False) -> str:
-  """'classic' (csrc/attention_fwd_rows_sm100.cu: head_dim 64, up to 2048 keys; the faster of the two on
-  the shapes it covers) or 'stream' (any length, head_dim 64 or 128). `T5X_B200_ATTN_FWD=stream` forces
-  the streaming kernel everywhere."""
+@functools.lru_cache(maxsize=None)
+def _sms() -> int:
+  return torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+
+
+def forward_kernel(Lq: int, Lk: int, D: int, prefix_lm: bool = False, heads: int = 0) -> str:
+  """'classic' (csrc/attention_fwd_rows_sm100.cu: head_dim 64, up to 2048 keys), 'few'
+  (csrc/attention_fwd_few_sm100.cu: `heads`, those of all examples together, leave SMs idle, and the queries
+  are one or two of its blocks) or 'stream' (any length, head_dim 64 or 128). `T5X_B200_ATTN_FWD=stream`
+  forces the streaming kernel everywhere.
+
+  'few' has a CTA per head, 'classic' two per SM, whose waits fill one another. us, few / classic, key mask and bias:
+  128 x 128 queries x keys, 6 heads 7.2 / 8.4, 148 7.1 / 9.1, 156 (a second wave) 13.1 / 10.0; 114 x 512, 6 heads
+  12.1 / 16.8, 148 13.2 / 17.3, 156 23.8 / 18.7; 256 x 256, 148 heads 14.3 / 17.8; 257 x 257, three blocks in
+  turn against two CTAs, 6 heads 24.1 / 14.0, 148 25.1 / 21.4. Both give the same bits."""
   import os
   classic_ok = D == 64 and Lk <= CLASSIC_MAX_LK
   want = os.environ.get("T5X_B200_ATTN_FWD", "classic")
-  return "classic" if (classic_ok and want == "classic") else "stream"
+  if not (classic_ok and want == "classic"):
+    return "stream"
+  few = 0 < heads <= _sms() and Lq <= FEW_MAX_LQ and Lk <= FEW_MAX_LK and not prefix_lm
+  return "few" if few else "classic"
 
 
 def _strides_ok(t: torch.Tensor) -> bool:
@@ -96,9 +114,9 @@ class _FlashAttentionFn(torch.autograd.Function):
     ctx.cfg = (causal, causal_off, rel_off)
     host = native.host()
     if host is not None:
-      short = forward_kernel(q.shape[1], k.shape[1], q.shape[3], int(causal) == 2) == "classic"
+      kernel = forward_kernel(q.shape[1], k.shape[1], q.shape[3], int(causal) == 2, q.shape[0] * q.shape[2])
       done = host.attention(q, k, v, rel_bias, buckets, key_mask, q_seg, kv_seg, int(causal),
-                            causal_off, rel_off, short)
+                            causal_off, rel_off, KERNELS[kernel])
       if done is not None:
         ctx.save_for_backward(q, k, v, *done, rel_bias, buckets, key_mask, q_seg, kv_seg)
         return done[0]
@@ -113,9 +131,10 @@ class _FlashAttentionFn(torch.autograd.Function):
     tail = (*_sbh(q), *_sbh(k), *_sbh(v), *_sbh(o), native.ptr(rel_bias), native.ptr(buckets), nb,
             nrel, rel_off, native.ptr(key_mask), native.ptr(q_seg), native.ptr(kv_seg),
             int(causal), causal_off, native.stream_ptr())
-    if forward_kernel(Lq, Lk, D, int(causal) == 2) == "classic":
-      rc = native.lib().t5x_attention_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
-                                          lse.data_ptr(), B, H, Lq, Lk, *tail)
+    kernel = forward_kernel(Lq, Lk, D, int(causal) == 2, B * H)
+    if kernel != "stream":
+      fwd = native.lib().t5x_attention_fwd_few if kernel == "few" else native.lib().t5x_attention_fwd
+      rc = fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), B, H, Lq, Lk, *tail)
     else:
       rc = native.lib().t5x_attention_fwd_stream(q.data_ptr(), k.data_ptr(), v.data_ptr(),
                                                  o.data_ptr(), lse.data_ptr(), B, H, Lq, Lk, D,

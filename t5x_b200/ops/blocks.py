@@ -86,16 +86,17 @@ def attention(x, kv, norm, attn, norm_cls, attn_cls, dense_cls, *, bias_table=No
   lq, lk = x.shape[1], (x if kv is None else kv).shape[1]
   masks = attn_ops.prepare(lq, lk, attn.local_heads, x.device, bias_table, bidirectional, num_buckets,
                            max_distance, key_mask, causal, q_segment_ids, kv_segment_ids)
-  short = attn_ops.forward_kernel(lq, lk, attn.head_dim, masks[5] == 2) == "classic"
+  kernel = attn_ops.KERNELS[attn_ops.forward_kernel(lq, lk, attn.head_dim, masks[5] == 2,
+                                                    x.shape[0] * attn.local_heads)]
   if not recording:
     return host.attention_block(x, kv, scale, norm.epsilon, weights, attn.local_heads, attn.head_dim, *masks,
-                                short)[0]
+                                kernel)[0]
   grads = [_usable_grad(p) for p in params]
   if any(g is None for g in grads) or _usable_grad(scale) is None or \
       not host.attention_grads_ok(x, kv, weights, grads):
     return None
   return _AttentionBlockFn.apply(x, kv, scale, *params, masks[0], norm.epsilon, attn.local_heads,
-                                 attn.head_dim, masks[1:], short)
+                                 attn.head_dim, masks[1:], kernel)
 
 
 def gated_mlp(x, norm, mlp, norm_cls, mlp_cls, dense_cls) -> Optional[torch.Tensor]:
@@ -175,10 +176,10 @@ class _Buffers:
 class _AttentionBlockFn(torch.autograd.Function):
 
   @staticmethod
-  def forward(ctx, x, kv, scale, wq, wk, wv, wo, rel_bias, eps, heads, head_dim, masks, short):
+  def forward(ctx, x, kv, scale, wq, wk, wv, wo, rel_bias, eps, heads, head_dim, masks, kernel):
     weights = [F.compute_weight(w, torch.bfloat16) for w in (wq, wk, wv, wo)]
     y, *saved = native.host().attention_block(x, kv, scale, eps, weights, heads, head_dim, rel_bias, *masks,
-                                              short)
+                                              kernel)
     ctx.save_for_backward(x, kv, scale, wq, wk, wv, wo, rel_bias, *masks[:4], *saved)
     ctx.modes = masks[4:]
     return y
