@@ -641,13 +641,16 @@ std::vector<Tensor> mlp_block(const Tensor& x, const Tensor& scale, double eps,
 
 // The same with one ReLU: y = x + relu(h wi) wo, weights wi, wo; (y, h, rstd, g). Covered where the products can
 // do the activation and its gradient themselves.
-bool relu_block_ok(const Tensor& x, const Tensor& scale, const std::vector<Tensor>& w) {
+bool relu_operands_ok(const Tensor& x, const Tensor& scale, const std::vector<Tensor>& w) {
   if (x.dim() < 2 || !plain(x) || !rows_fit(x) || !norm_ok(scale, x) || w.size() != 2 || w[0].dim() != 2)
     return false;
   const Weight a(w[0], x.size(-1));
-  if (!a.ok || !t5x_gemm_gated_grad_covers(rows_of(x), a.n)) return false;
+  if (!a.ok) return false;
   const Weight o(w[1], a.n);
   return o.ok && o.n == x.size(-1);
+}
+bool relu_block_ok(const Tensor& x, const Tensor& scale, const std::vector<Tensor>& w) {
+  return relu_operands_ok(x, scale, w) && t5x_gemm_gated_grad_covers(rows_of(x), Weight(w[0], x.size(-1)).n);
 }
 bool relu_grads_ok(const Tensor& x, const std::vector<Tensor>& w, const std::vector<optional<Tensor>>& g) {
   const Weight a(w[0], x.size(-1)), o(w[1], a.n);
@@ -673,16 +676,23 @@ Tensor relu_block_bwd(const Tensor& dy, const Tensor& x, const Tensor& scale, co
                       const std::vector<bool>& accumulate, Tensor dscale) {
   const Tensor &h = saved[0], &rstd = saved[1], &g = saved[2];
   const std::vector<optional<Tensor>> have(grads.begin(), grads.end());
-  if (!plain(dy) || dy.numel() != x.numel() || !relu_block_ok(x, scale, weights) || !relu_grads_ok(x, weights, have))
+  if (!plain(dy) || dy.numel() != x.numel() || !relu_operands_ok(x, scale, weights) ||
+      !relu_grads_ok(x, weights, have))
     throw std::invalid_argument("relu_block_bwd: operands are not covered");
   void* st = stream_of();
   const int64_t m = rows_of(x), d = x.size(-1);
   const Weight a(weights[0], d), wo(weights[1], a.n);
   Tensor dg = at::empty_like(g);
   optional<Tensor> dh = at::empty_like(x);
-  check(t5x_gemm_relu(dy.data_ptr(), wo.t.data_ptr(), dg.data_ptr(), g.data_ptr(), m, a.n, wo.n, wo.n, wo.ld, a.n,
-                      a.n, 0, st),
-        "gemm_relu");
+  // (CTA pairs may have been switched off since the forward pass)
+  if (t5x_gemm_gated_grad_covers(m, a.n)) {
+    check(t5x_gemm_relu(dy.data_ptr(), wo.t.data_ptr(), dg.data_ptr(), g.data_ptr(), m, a.n, wo.n, wo.n, wo.ld, a.n,
+                        a.n, 0, st),
+          "gemm_relu");
+  } else {
+    input_grad(dy.data_ptr(), wo.n, m, wo, dg, false, st);
+    dg = at::threshold_backward(dg, g, 0);
+  }
   Tensor gwo = grads[1];
   weight_grad(g, dy.data_ptr(), wo.n, m, wo, gwo, accumulate[1], st);
   backward_products(h, m, {dg.data_ptr()}, {a.n}, {a}, dh, {grads[0]}, {accumulate[0]}, st);

@@ -49,3 +49,29 @@ def test_same_as_op_by_op(monkeypatch):
   assert [n for n in g1 if g1[n] is None] == [n for n in g2 if g2[n] is None]
   for n in (n for n in g1 if g1[n] is not None):  # up to the order of atomic adds
     assert float((g1[n].float() - g2[n].float()).norm() / g2[n].float().norm()) < 1e-3, n
+
+
+def test_pair_mode_between_the_passes():
+  """The forward pass through the products with ReLU, the backward pass after CTA pairs were switched off."""
+  from t5x_b200.ops import blocks, native
+  grads = []
+  for mode in (1, 0):
+    module = _model(act=("relu",), mlp=1024)
+    mlp, norm = module.encoder.layers_0.mlp, module.encoder.layers_0.pre_mlp_layer_norm
+    for p in module.parameters():
+      p.grad_ready = False
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(5000, 256, device="cuda", generator=g).bfloat16().requires_grad_()
+    dy = torch.randn(5000, 256, device="cuda", generator=g).bfloat16()
+    y = blocks.relu_mlp(x, norm, mlp, type(norm), type(mlp), type(mlp.wi))
+    assert y is not None
+    native.gemm_set_pair_mode(mode)
+    try:
+      y.backward(dy)
+    finally:
+      native.gemm_set_pair_mode(1)
+    native.check_status()
+    grads.append([x.grad] + [p.main_grad for p in (mlp.wi.kernel, mlp.wo.kernel, norm.scale)])
+  # dg is rounded to bf16 either way; other tiles add in another order
+  for a, b in zip(*grads):
+    assert float((a.float() - b.float()).norm() / b.float().norm()) < 2.0 ** -8
