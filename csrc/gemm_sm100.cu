@@ -961,12 +961,25 @@ T5X_API int t5x_gemm_ce_grad(const void* A, const void* B, void* dlogits, long l
   return rc;
 }
 
-// Whether the epilogues for CTA pairs alone (t5x_gemm_gated_grad, t5x_gemm_relu) take these sizes: whole 32-column
-// blocks, and tiles for half of the pairs.
-T5X_API int t5x_gemm_gated_grad_covers(int M, int N) {
+// Whether t5x_gemm_relu takes these sizes and saves time: whole 32-column blocks, and tiles for half of the pairs.
+T5X_API int t5x_gemm_relu_covers(int M, int N) {
   using namespace t5x;
   const long long tiles = ((M + 2 * kBM - 1ll) / (2 * kBM)) * ((N + 255) / 256);
   return gemm_pair_mode() != 0 && M >= 2 * kBM && N >= 256 && N % 32 == 0 && tiles >= num_sms() / 4;
+}
+
+// The same for t5x_gemm_gated_grad, whose tile takes longer to leave than a plain product's, while the pass that it
+// saves goes by the elements there are: of the elements that the waves of tiles have room for, 57 % have to be
+// there, of several waves 52 %. (us, M x N from K, product and pass / in one: 300 x 10240 from 4096, 32 %, 50.2 /
+// 72.3; 384 x 10240, 41 %, 45.7 / 59.8; 4864 x 1024 from 512, 51 % of two waves, 22.1 / 24.1; 512 x 5120 from 2048,
+// 54 % of one, 22.5 / 23.1; 1000 x 2816 from 1024, 58 %, 18.2 / 18.0; 512 x 10240 from 4096, 54 % of two, 60.0 /
+// 57.3; 3000 x 1024 from 512, 63 %, 15.8 / 15.6; 768 x 5120 from 2048, 81 %, 24.8 / 23.5; the gain grows from there.)
+T5X_API int t5x_gemm_gated_grad_covers(int M, int N) {
+  using namespace t5x;
+  if (!t5x_gemm_relu_covers(M, N)) return 0;
+  const long long tiles = ((M + 2 * kBM - 1ll) / (2 * kBM)) * ((N + 255) / 256), pairs = num_sms() / 2;
+  const long long waves = (tiles + pairs - 1) / pairs;
+  return 100ll * M * N >= (waves == 1 ? 57 : 52) * waves * pairs * (2 * kBM * 256);
 }
 
 // Gradient of gelu(h0) * h1 from that of its product with a matrix: with dg = dy[M, K] @ B[K, N] (which is not
@@ -982,7 +995,7 @@ T5X_API int t5x_gemm_gated_grad(const void* dy, const void* B, void* h0, void* h
 }
 
 // C[M, N] (bf16) = relu(A[M, K] @ B[K, N]), or with `positive` (bf16 [M, N], rows ldp apart) the product, zero where
-// that is zero or negative: the gradient of a ReLU whose output it is. Sizes as t5x_gemm_gated_grad_covers has
+// that is zero or negative: the gradient of a ReLU whose output it is. Sizes as t5x_gemm_relu_covers has
 // them. (A pass of its own reads and writes the activations, its gradient reads two tensors and writes one: 8192 x
 // 1024 x 16384, us, product and pass / in one: forward 286 / 214, backward 312 / 256.)
 T5X_API int t5x_gemm_relu(const void* A, const void* B, void* C, const void* positive, int M, int N, int K,

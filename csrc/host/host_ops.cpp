@@ -650,7 +650,7 @@ bool relu_operands_ok(const Tensor& x, const Tensor& scale, const std::vector<Te
   return o.ok && o.n == x.size(-1);
 }
 bool relu_block_ok(const Tensor& x, const Tensor& scale, const std::vector<Tensor>& w) {
-  return relu_operands_ok(x, scale, w) && t5x_gemm_gated_grad_covers(rows_of(x), Weight(w[0], x.size(-1)).n);
+  return relu_operands_ok(x, scale, w) && t5x_gemm_relu_covers(rows_of(x), Weight(w[0], x.size(-1)).n);
 }
 bool relu_grads_ok(const Tensor& x, const std::vector<Tensor>& w, const std::vector<optional<Tensor>>& g) {
   const Weight a(w[0], x.size(-1)), o(w[1], a.n);
@@ -685,7 +685,7 @@ Tensor relu_block_bwd(const Tensor& dy, const Tensor& x, const Tensor& scale, co
   Tensor dg = at::empty_like(g);
   optional<Tensor> dh = at::empty_like(x);
   // (CTA pairs may have been switched off since the forward pass)
-  if (t5x_gemm_gated_grad_covers(m, a.n)) {
+  if (t5x_gemm_relu_covers(m, a.n)) {
     check(t5x_gemm_relu(dy.data_ptr(), wo.t.data_ptr(), dg.data_ptr(), g.data_ptr(), m, a.n, wo.n, wo.n, wo.ld, a.n,
                         a.n, 0, st),
           "gemm_relu");

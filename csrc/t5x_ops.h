@@ -57,6 +57,7 @@ int t5x_attention_bwd_head(const void* q, const void* k, const void* v, const vo
                            int rel_off, const void* key_mask, const void* q_seg, const void* kv_seg,
                            int causal, int causal_off, void* stream);
 int t5x_gemm_gated_grad_covers(int M, int N);
+int t5x_gemm_relu_covers(int M, int N);
 int t5x_gemm_relu(const void* A, const void* B, void* C, const void* positive, int M, int N, int K, long long lda,
                   long long ldb, long long ldc, long long ldp, int b_mn_major, void* stream);
 int t5x_gemm_gated_grad(const void* dy, const void* B, void* h0, void* h1, int M, int N, int K, long long ld_dy,

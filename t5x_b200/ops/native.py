@@ -751,6 +751,7 @@ register_signature("t5x_gemm_ce_grad", [c_void_p, c_void_p, c_void_p, c_ll, c_in
                                         c_void_p, c_void_p, c_float, c_float, c_float, c_void_p])
 register_signature("t5x_gemm_gated_grad", [c_void_p] * 4 + [c_int] * 3 + [c_ll] * 3 + [c_int, c_void_p])
 register_signature("t5x_gemm_gated_grad_covers", [c_int, c_int])
+register_signature("t5x_gemm_relu_covers", [c_int, c_int])
 register_signature("t5x_gemm_relu", [c_void_p] * 4 + [c_int] * 3 + [c_ll] * 4 + [c_int, c_void_p])
 register_signature("t5x_ce_merge", [c_void_p] * 7 + [c_int, c_int, c_int, c_int, c_void_p])
 
