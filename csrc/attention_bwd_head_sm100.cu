@@ -18,6 +18,7 @@
 // 184 / 113, 24 x 12 x 509 packed 258 / 157, 32 x 64 x 512 x 512 1327 / 792). Of the 610, the bias gradient
 // takes 100 (40 its additions to shared memory, which are loops around a compare-and-swap), the bias 35, the
 // exponentials 8.
+#include <algorithm>
 #include <type_traits>
 
 #include "attention_common.cuh"
@@ -868,17 +869,26 @@ T5X_API int t5x_attention_bwd_head_covers(int B, int H, int Lq, int Lk, int D, i
   if (num_buckets > 0 && (num_buckets > kBuckets || (nkb + (nq < 4 ? nq : 4)) * 128 >
                                                         (parts > 1 ? kMaxRelOf<true> : kMaxRelOf<false>)))
     return 0;
-  // Thousands of cycles, measured: 14 for a CTA and 3 for each of its 128 x 64 units; the other kernel, with a
-  // CTA per key block, 14 and 7 for each 128 x 128 tile, and some 10 for its three further launches; clearing and
-  // casting dQ (there) or the dK and dV of parts (here), ten bytes an element at 3.4 MB a thousand cycles. (512 x
-  // 512, us, other / this: 16 x 6 heads 128 / 62, 74 heads even, 12 heads 27 / 58; 1024 x 1024: 16 x 12 heads 591 /
-  // 400, 16 x 6 225 / 235.)
+  // Thousands of cycles, measured: 14 for a CTA and 3 for each of its 128 x 64 units, 2.2 without a bias (of parts 2.9
+  // and 2.7); the other kernel, with a CTA per key block, 14 and 7.2 for each 128 x 128 tile, 5.2 without a bias;
+  // some 10 for its three further launches or for those of parts; clearing and casting dQ (there) or the dK and dV of
+  // parts (here), ten bytes an element at 3.4 MB a thousand cycles. Up to a head per SM the last part, which has
+  // fewer units, makes room for a whole one. (us, other / this, with a bias and without: 512 x 512, 48 heads 53 / 55
+  // and 41 / 43, 96 heads 78 / 55, 60 / 43; 1024 x 1024, 48 heads 124 / 116, 91 / 106, 148 heads 333 / 250, 247 /
+  // 231, 300 heads 694 / 601, 513 / 555; 600 x 600, 144 heads 152 / 125, 122 / 113; 1100 x 300, 6 heads 50 / 54,
+  // 42 / 45.)
+  const bool bias = num_buckets > 0;
   const long long sms = num_sms(), heads = static_cast<long long>(B) * H;
-  const int units = parts > 1 ? kMaxQ / 64 : (Lq + 63) / 64;
   const double cast = heads * 640.0 / 3.4e6;
-  const double here = static_cast<double>((heads * parts + sms - 1) / sms) * (14 + 3 * nkb * units) +
-                      (parts > 1 ? 2 * Lk * cast : 0.0);
-  const double other = static_cast<double>((heads * nkb + sms - 1) / sms) * (14 + 7 * nq) + 10 + Lq * cast;
+  auto cta = [&](int queries) {
+    return 14 + (parts > 1 ? (bias ? 2.9 : 2.7) : (bias ? 3 : 2.2)) * nkb * ((queries + 63) / 64);
+  };
+  const double whole = cta(Lq < kMaxQ ? Lq : kMaxQ);
+  double here = static_cast<double>((heads * parts + sms - 1) / sms) * whole;
+  if (heads <= sms) here = std::min(here, (parts - 1) * whole + cta(Lq - (parts - 1) * kMaxQ));
+  if (parts > 1) here += 10 + 2 * Lk * cast;
+  const double other =
+      static_cast<double>((heads * nkb + sms - 1) / sms) * (14 + (bias ? 7.2 : 5.2) * nq) + 10 + Lq * cast;
   if (here > other) return 0;
   return parts > 1 ? 2 : 1;
 }

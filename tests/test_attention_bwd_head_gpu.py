@@ -96,6 +96,11 @@ def test_both_kernels_are_reached():
   assert covers(16, 12, 1024, 1024, 64, 32) == 2 and not covers(16, 12, 1024, 1300, 64, 32)
   assert not covers(128, 12, 512, 512, 128, 32) and not covers(128, 12, 512, 700, 64, 32)
   assert not covers(128, 12, 512, 512, 64, 300)
+  # without a bias the kernel by key blocks is the faster one for longer
+  assert covers(8, 6, 1024, 1024, 64, 32) == 2 and not covers(8, 6, 1024, 1024, 64, 0)
+  assert covers(50, 6, 1024, 1024, 64, 32) == 2 and not covers(50, 6, 1024, 1024, 64, 0)
+  assert not covers(1, 6, 1100, 300, 64, 32) and not covers(1, 6, 1100, 300, 64, 0)
+  assert covers(24, 6, 600, 600, 64, 0) == 2 and not covers(12, 6, 600, 600, 64, 0)
 
 
 @pytest.mark.parametrize("compiled", [True, False])
