@@ -29,8 +29,8 @@
 //
 // A chunk of which the mask hides every key (the padding of a batch) is not read: its scores are -1e10 whatever
 // the keys, and its probabilities exact zeros wherever any key of the example is visible. Bound by memory (64 x 4
-// beams x 32 heads x 512 keys, us, read whole and requested ahead / so: 60 to 100 % visible 59.9 / 52.3, all
-// visible 59.7 / 57.8).
+// beams x 32 heads x 512 keys, us, read whole and requested ahead / so: 60 to 100 % visible 58.0 / 49.3, all
+// visible 58.4 / 55.0). That is so where a warp has several chunks; the line is at the launch.
 #include "common.cuh"
 #include "t5x_b200.h"
 
@@ -62,8 +62,8 @@ __device__ __forceinline__ int key_of_column(int u, int tile, int n) {
   return 8 * (n >> 1) + 4 * u + 2 * tile + (n & 1);
 }
 
-// kLook: hidden chunks are passed over (not in a chain of launches of few rows, where the look takes longer than it
-// saves; there the operands are requested ahead instead).
+// kLook: hidden chunks are passed over (not in a chain of launches of few rows nor over few keys, where the look takes
+// longer than it saves; there the operands are requested ahead instead).
 template <int BEAMS, bool kLook>
 __global__ void __launch_bounds__(kXmThreads)
     decode_cross_mma_kernel(const __nv_bfloat16* __restrict__ q,   // [B*beams, H, 64], row stride q_ld
@@ -85,8 +85,8 @@ __global__ void __launch_bounds__(kXmThreads)
   const uint8_t* km = key_mask == nullptr ? nullptr : key_mask + static_cast<long long>(b) * Lk;
 
   // Keys and values are encoder products, constant while decoding: this CTA's part of them is
-  // pulled toward L2 while the kernel before this one (which produces q) may still be running. (Where nothing
-  // runs before, the requests only get into the way of the loads: 56.9 / 52.3 us for the shape above.)
+  // pulled toward L2 while the kernel before this one (which produces q) may still be running. (Over many keys
+  // and with nothing running before, the requests only get into the way of the loads: 56.9 / 52.3 us above.)
   chain_release();
   const int nchunks = Lp / 32;
   uint32_t shown = 0xffffffffu;
@@ -270,7 +270,12 @@ T5X_API int t5x_decode_cross_attention_mma(const void* q, const void* k, const v
   auto vp = static_cast<const __nv_bfloat16*>(vt);
   auto mp = static_cast<const uint8_t*>(key_mask);
   auto op = static_cast<__nv_bfloat16*>(out);
-  const bool look = !chained_launches();
+  // Up to 256 keys a warp has one chunk: to request all of it at once is what counts, and the look delays that. (64 x
+  // 32 heads, us, requested ahead / with a look, 60 to 100 % visible: one beam, 64 keys 19.1 / 25.0, 256 30.8 / 34.2,
+  // 384 42.9 / 44.4, 512 52.4 / 49.4, three chunks a warp of which one comes alone, 640 64.4 / 69.5, 1000 104 / 84;
+  // four beams, 64 keys 20.2 / 25.4, 256 33.1 / 35.5, 320 45.8 / 40.4, 512 58.0 / 49.3, 1000 106 / 80.)
+  const bool worth = beams >= 4 ? Lp > 256 : Lp > 768 || (Lp > 384 && Lp <= 512);
+  const bool look = !chained_launches() && worth;
   const auto go = [&](auto kernel) {
     return launch_chained(kernel, grid, dim3(kXmThreads), 0, st, qp, kp, vp, mp, op, q_ld, heads, Lk, Lp);
   };
