@@ -7,10 +7,10 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _call(q, k, v, o, do, lse, table, lq, lk, key_mask, qs, ks, mode):
+def _call(q, k, v, o, do, lse, table, lq, lk, key_mask, qs, ks, mode, outs=None):
   from t5x_b200.ops import attention as A, native
   b, h = q.shape[0], q.shape[2]
-  dq, dk, dv = (torch.full_like(t, 7.0) for t in (q, k, v))
+  dq, dk, dv = outs or (torch.full_like(t, 7.0) for t in (q, k, v))
   buckets = d_table = None
   if table is not None:
     buckets = A._rel_buckets(lq, lk, 0, mode == 0, 32, 128, q.device)
@@ -85,6 +85,80 @@ def test_against_float64(lq, lk, bias, mask):
   # key dq, dk and dbias are zero; dS is then the rounding of two equal 32-bit sums of 64 products, up to
   # 64 * 2^-24 * |dO| |v| or 1e-4 with norms of 8.)
   for name, a, w in zip(("dq", "dk", "dv", "dbias"), got, want):
+    assert float((a.double() - w).norm() / (w.norm() + 1e-2)) < 4 * 2.0 ** -8, name
+
+
+def _prefix(lq, kind):
+  """A prefix-LM mask of three examples: whole, padded (a padding query sees nothing), padded within its prefix."""
+  from t5x_b200.ops import reference as ref
+  pos = torch.arange(lq, device="cuda")
+  inside = pos[None] < torch.tensor([lq // 3, lq // 2, lq], device="cuda")[:, None]
+  valid = pos[None] < torch.tensor([lq, lq - lq // 4, lq // 2], device="cuda")[:, None]
+  seg = (pos * 3 // lq + 1).int()[None].expand(3, lq).contiguous() if "packed" in kind else None
+  return ref.PrefixLMMask(inside, valid, seg)
+
+
+@pytest.mark.parametrize("kind", ["causal", "causal masked", "causal packed", "causal packed masked", "prefix",
+                                  "prefix packed", "holes"])
+@pytest.mark.parametrize("lq,lk,bias", [(300, 300, True), (512, 512, True), (512, 512, False), (700, 700, True),
+                                        (1100, 1100, True), (300, 460, True), (460, 300, True), (130, 700, False),
+                                        (600, 1100, True), (1100, 600, True), (513, 140, False)])
+def test_passed_over_blocks_and_offsets(lq, lk, bias, kind):
+  """Blocks of keys or queries that are passed over, and those that must not be: queries that do not see themselves,
+  prefixes, leading hidden blocks and holes; causal attention of more or fewer queries than keys."""
+  from t5x_b200.ops import attention as A, reference as ref
+  if "prefix" in kind and lq != lk:
+    pytest.skip("self-attention")
+  g = torch.Generator(device="cuda").manual_seed(lq * 5 + lk)
+  b, h, outs = 3, 2, None
+  rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+  if lq == lk and lq <= 512:  # projections and their gradients side by side
+    q, k, v = rnd(b, lq, 3, h, 64).bfloat16().unbind(2)
+    q.mul_(0.3)
+    outs = torch.full((b, lq, 3, h, 64), 7.0, device="cuda").bfloat16().unbind(2)
+  else:
+    q = (rnd(b, lq, h, 64) * 0.3).bfloat16()
+    k, v = rnd(b, lk, h, 64).bfloat16(), rnd(b, lk, h, 64).bfloat16()
+  do = rnd(b, lq, h, 64).bfloat16()
+  table = rnd(h, 32) if bias else None
+  qpos, kpos = torch.arange(lq, device="cuda"), torch.arange(lk, device="cuda")
+  allowed = torch.ones(b, lq, lk, dtype=torch.bool, device="cuda")
+  km = qs = ks = prefix = None
+  if "prefix" in kind:
+    prefix = _prefix(lq, kind)
+    allowed = prefix.bool()[:, 0]
+  elif "causal" in kind:
+    allowed = allowed & (kpos[None] <= qpos[:, None] + lk - lq)
+  if "masked" in kind or kind == "holes":
+    km = torch.ones(b, lk, dtype=torch.bool, device="cuda")
+    km[1, :140] = False
+    km[2, 120:260] = False
+    km[2, lk - 1] = True
+    allowed = allowed & km[:, None]
+  if "packed" in kind and prefix is None:
+    qs, ks = ((p * 4 // p.numel()).int()[None].expand(b, -1).contiguous() for p in (qpos, kpos))
+    allowed = allowed & (qs[:, :, None] == ks[:, None])
+  prep = A.prepare(lq, lk, h, q.device, table, "causal" not in kind and prefix is None, 32, 128, km, "causal" in kind,
+                   qs, ks, 0, prefix)
+  q2, k2, v2, do2 = (t.double() for t in (q, k, v, do))
+  bucket = ref.relative_position_bucket(kpos[None] - qpos[:, None], prep[5] == 0, 32, 128)
+  s = torch.einsum("bqhd,bkhd->bhqk", q2, k2)
+  if bias:
+    s = s + table.double()[:, bucket][None]
+  s = torch.where(allowed[:, None], s, -1e10)
+  probs = torch.softmax(s, -1)
+  o = torch.einsum("bhqk,bkhd->bqhd", probs, v2).bfloat16()
+  lse = torch.logsumexp(s, -1).float().contiguous()
+  # the gradients as the inputs give them, with rowsum(dO * O) of the rounded O: where all keys of a row share a
+  # bucket, dbias is what that sum is off by
+  ds = probs * (torch.einsum("bqhd,bkhd->bhqk", do2, v2) - (do2 * o.double()).sum(-1).transpose(1, 2)[..., None])
+  want = [torch.einsum("bhqk,bkhd->bqhd", ds, k2), torch.einsum("bhqk,bqhd->bkhd", ds, q2),
+          torch.einsum("bhqk,bqhd->bkhd", probs, do2)]
+  if bias:
+    want.append(torch.zeros(h, 32, dtype=torch.float64, device="cuda").index_add_(
+        1, bucket.flatten(), ds.sum(0).flatten(1)))
+  got = _call(q, k, v, o, do, lse, table, lq, lk, *prep[2:5], prep[5], outs)
+  for name, a, w in zip(("dq", "dk", "dv", "dbias"), got, want):  # P, dS and the results rounded once, as above
     assert float((a.double() - w).norm() / (w.norm() + 1e-2)) < 4 * 2.0 ** -8, name
 
 

@@ -61,3 +61,45 @@ def test_against_float64(lq, lk, bias, mask):
   # the probabilities and the result are each rounded to bf16 once; log-sum-exps are 32-bit
   assert float((o.double() - want).norm() / want.norm()) < 2 * 2.0 ** -8
   assert float(((lse.double() - torch.logsumexp(s, -1)).abs() / (1 + s.amax(-1).abs())).max()) < 1e-5
+
+
+@pytest.mark.parametrize("kind", ["causal", "causal masked", "causal packed", "causal packed masked"])
+@pytest.mark.parametrize("lq,lk,bias", [(300, 460, True), (460, 300, True), (130, 700, False), (64, 40, True),
+                                        (600, 1100, True), (1100, 600, True), (513, 140, False)])
+def test_causal_of_other_lengths(lq, lk, bias, kind):
+  """More or fewer queries than keys: the last query sees the last key, and the first ones may see none."""
+  from t5x_b200.ops import attention as A, native, reference as ref
+  g = torch.Generator(device="cuda").manual_seed(lq * 5 + lk)
+  b, h = 3, 2
+  rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+  q = (rnd(b, lq, h, 64) * 0.3).bfloat16()
+  k, v = rnd(b, lk, h, 64).bfloat16(), rnd(b, lk, h, 64).bfloat16()
+  table = rnd(h, 32) if bias else None
+  qpos, kpos = torch.arange(lq, device="cuda"), torch.arange(lk, device="cuda")
+  allowed = (kpos[None] <= qpos[:, None] + lk - lq).expand(b, lq, lk)
+  km = qs = ks = None
+  if "masked" in kind:
+    km = torch.ones(b, lk, dtype=torch.bool, device="cuda")
+    km[1, :30], km[2, lk // 2:] = False, False
+    allowed = allowed & km[:, None]
+  if "packed" in kind:
+    qs, ks = ((p * 4 // p.numel()).int()[None].expand(b, -1).contiguous() for p in (qpos, kpos))
+    allowed = allowed & (qs[:, :, None] == ks[:, None])
+  rel_bias, buckets, km8, qc, kc, mode, off, rel_off = A.prepare(lq, lk, h, q.device, table, False, 32, 128, km, True,
+                                                                 qs, ks, 0, None)
+  s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double())
+  if bias:
+    s = s + table.double()[:, ref.relative_position_bucket(kpos[None] - qpos[:, None], False, 32, 128)][None]
+  s = torch.where(allowed[:, None], s, -1e10)
+  want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), v.double())
+  p, (nb, nrel) = native.ptr, A._bias_sizes(rel_bias, buckets)
+  entries = ["t5x_attention_fwd"] + (["t5x_attention_fwd_few"] if max(lq, lk) <= 512 else [])
+  for entry in entries:
+    o = torch.full_like(q, 7.0)
+    lse = torch.full((b, h, lq), 7.0, device="cuda")
+    native._check(getattr(native.lib(), entry)(
+        *(t.data_ptr() for t in (q, k, v, o, lse)), b, h, lq, lk, *(s for t in (q, k, v, o) for s in A._sbh(t)),
+        p(rel_bias), p(buckets), nb, nrel, rel_off, p(km8), p(qc), p(kc), mode, off, native.stream_ptr()), entry)
+    native.check_status()
+    assert float((o.double() - want).norm() / want.norm()) < 2 * 2.0 ** -8, entry
+    assert float(((lse.double() - torch.logsumexp(s, -1)).abs() / (1 + s.amax(-1).abs())).max()) < 1e-5, entry
