@@ -12,8 +12,8 @@
 // softmax warps never wait for one another inside the walk.
 //
 // One CTA per 128-key block (attention_sm100.cu) spends 14k cycles on setting up and tearing down a CTA and
-// 6.7k on a 128 x 128 tile. Here a CTA takes 16k and a 128 x 64 unit 2 to 3k, bound by what a softmax warp does
-// one after the other for a unit (us, with rowsum(dO * O), clearing and casting of dQ where there are any,
+// 6.7k on a 128 x 128 tile. Here a CTA takes some 14k and a 128 x 64 unit 2 to 3k, bound by what a softmax warp
+// does one after the other for a unit (us, with rowsum(dO * O), clearing and casting of dQ where there are any,
 // before / now: 128 x 12 heads x 512 x 512 1081 / 610, 114 x 512 without a bias 385 / 202, 114 x 114 causal
 // 184 / 113, 24 x 12 x 509 packed 258 / 157, 32 x 64 x 512 x 512 1327 / 792). Of the 610, the bias gradient
 // takes 100 (40 its additions to shared memory, which are loops around a compare-and-swap), the bias 35, the
@@ -90,8 +90,10 @@ __device__ __forceinline__ void tmem_wait_into(uint32_t (&a)[16], uint32_t (&c)[
 // kAhead: causal self-attention over more than one block, where key blocks ahead of a query block are
 // passed over (see attn_bwd_kernel for the conditions).
 // kParts: more than 512 queries, a CTA for each 512 of them. dQ leaves as above; dK and dV of the parts are added in
-// fp32 memory and cast afterwards. (us, by
-// key blocks in attention_sm100.cu / so, with all launches: prefix LM, 16 x 12 heads x 1024, 591 / 400.)
+// fp32 memory (two buffers of [B, Lk, H, 64]) and cast afterwards. The parts arrive in any order: up to two of them
+// give the same sums whatever it is, of more than 1024 queries dK and dV can differ from run to run in the last
+// bits (by key blocks in attention_sm100.cu dQ does). (us, by key blocks / so, with all launches: prefix LM, 16 x 12
+// heads x 1024, 591 / 400.)
 template <bool kAhead, bool kParts>
 __global__ void __launch_bounds__(kThreads, 1)
     attn_bwd_head_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -849,8 +851,9 @@ int launch_head(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap*
     if (e != cudaSuccess) return set_error("attention_bwd_head attr: %s", cudaGetErrorString(e));
     attr_set[dev] = true;
   }
-  attn_bwd_head_kernel<kAhead, kParts><<<dim3(hp.a.H, hp.a.B, (hp.a.Lq + kMaxQ - 1) / kMaxQ), kThreads,
-                                         HeadSmem<kParts>::kTotal, st>>>(*tq, *tk, *tv, *tdo, *tdq, *tdk, *tdv, *to, hp);
+  const dim3 grid(hp.a.H, hp.a.B, (hp.a.Lq + kMaxQ - 1) / kMaxQ);
+  attn_bwd_head_kernel<kAhead, kParts><<<grid, kThreads, HeadSmem<kParts>::kTotal, st>>>(*tq, *tk, *tv, *tdo, *tdq,
+                                                                                         *tdk, *tdv, *to, hp);
   count_launches(1);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("attention_bwd_head: %s", cudaGetErrorString(e));
@@ -898,10 +901,9 @@ T5X_API int t5x_attention_bwd_head_covers(int B, int H, int Lq, int Lk, int D, i
 // (fp32, [B,Lk,H,64], cleared) are added to instead of dk and dv. The rest as t5x_attention_bwd.
 T5X_API int t5x_attention_bwd_head(const void* q, const void* k, const void* v, const void* o, const void* d_o,
                                    const void* lse, void* dq, void* dk, void* dv, void* dk32, void* dv32, int B,
-                                   int H, int Lq, int Lk,
-                                   long long q_sb, long long q_sl, long long q_sh, long long k_sb,
-                                   long long k_sl, long long k_sh, long long v_sb, long long v_sl,
-                                   long long v_sh, long long o_sb, long long o_sl, long long o_sh,
+                                   int H, int Lq, int Lk, long long q_sb, long long q_sl, long long q_sh,
+                                   long long k_sb, long long k_sl, long long k_sh, long long v_sb,
+                                   long long v_sl, long long v_sh, long long o_sb, long long o_sl, long long o_sh,
                                    long long do_sb, long long do_sl, long long do_sh, long long dq_sb,
                                    long long dq_sl, long long dq_sh, long long dk_sb, long long dk_sl,
                                    long long dk_sh, const void* rel_bias, const void* rel_bucket,
@@ -925,7 +927,8 @@ T5X_API int t5x_attention_bwd_head(const void* q, const void* k, const void* v, 
   CUtensorMap tq, tk, tv, tdo, tdq, tdk, tdv, to;
   if (!bhld_map(&tq, q, B, Lq, H, q_sb, q_sl, q_sh, 64, 64) || !bhld_map(&tk, k, B, Lk, H, k_sb, k_sl, k_sh) ||
       !bhld_map(&tv, v, B, Lk, H, v_sb, v_sl, v_sh) || !bhld_map(&tdo, d_o, B, Lq, H, do_sb, do_sl, do_sh, 64, 64) ||
-      !bhld_map(&to, o, B, Lq, H, o_sb, o_sl, o_sh, 64, 64) || !bhld_map(&tdq, dq, B, Lq, H, dq_sb, dq_sl, dq_sh) || !bhld_map(&tdk, dk, B, Lk, H, dk_sb, dk_sl, dk_sh) ||
+      !bhld_map(&to, o, B, Lq, H, o_sb, o_sl, o_sh, 64, 64) ||
+      !bhld_map(&tdq, dq, B, Lq, H, dq_sb, dq_sl, dq_sh) || !bhld_map(&tdk, dk, B, Lk, H, dk_sb, dk_sl, dk_sh) ||
       !bhld_map(&tdv, dv, B, Lk, H, dk_sb, dk_sl, dk_sh))
     return -1;
   HeadParams hp = {};
@@ -955,6 +958,5 @@ T5X_API int t5x_attention_bwd_head(const void* q, const void* k, const void* v, 
   const bool ahead = causal && Lq == Lk && causal_off == 0 && Lq > 128;
   const auto launch = parts ? (ahead ? launch_head<true, true> : launch_head<false, true>)
                             : (ahead ? launch_head<true, false> : launch_head<false, false>);
-  return launch(&tq, &tk, &tv, &tdo, &tdq, &tdk, &tdv, &to, hp,
-                                                          static_cast<cudaStream_t>(stream));
+  return launch(&tq, &tk, &tv, &tdo, &tdq, &tdk, &tdv, &to, hp, static_cast<cudaStream_t>(stream));
 }

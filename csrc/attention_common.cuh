@@ -57,14 +57,13 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 // tile's queries would contribute exact zeros (the scores of visible keys being far above the -1e10 of
 // hidden ones), unless a query sees no key at all: its row is uniform over all keys, and all count.
 //   kLookMask    Nothing but a key mask hides keys (the padding of a batch): up to the last visible key.
-//                us before / so: 60 to 100 % of the keys visible, 16 x 6 heads x 1024 x 1024 162 / 146, 8 x
-//                32 x 1024 x 1024 of 128 features 643 / 562; all visible 162 / 163.5, 643 / 643.
+//                us before / so, 8 x 32 heads of 128 features x 1024 x 1024: 60 to 100 % of the keys visible
+//                643 / 562; all visible 643 / 643.
 //   kLookCausal  A causal or prefix-LM mask of self-attention with a key mask or segments: up to a tile's
 //                last query (and the last prefix key, if the tile has queries inside the prefix), as long
 //                as each of its queries sees itself. To look that up costs a CTA some 3 us, so only from
-//                more than kAheadKeys keys on (prefix LM, 16 x 12 heads x 1024, 600 tokens in the prefix,
-//                375 / 303; causal with a key mask, 8 x 32 heads of 128 x 1024 655 / 472; but without
-//                that bound 8 x 32 x 256 72 / 77).
+//                more than kAheadKeys keys on (causal with a key mask, 8 x 32 heads of 128 x 1024 655 / 472;
+//                but without that bound 8 x 32 x 256 72 / 77).
 //   kLookNone    Everything else, in a variant of its own: the look-up at run time cost it 2 to 5 % (8 x 32
 //                heads of 128 x 256, causal, 61.4 / 64.3).
 enum KeyLook : int { kLookNone = 0, kLookMask = 1, kLookCausal = 2 };

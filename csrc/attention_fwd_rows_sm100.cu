@@ -5,7 +5,8 @@
 // CTA has two groups (256 queries of a head; of 128 queries or fewer the groups take every other block of 64
 // keys), and two CTAs share an SM. What bounds the kernel is the chain of
 // steps of a group (scores from TMEM, exponentials, probabilities to shared memory, fences, barriers): four
-// groups in different phases fill one another's gaps, to 60 % of the issue slots.
+// groups in different phases fill one another's gaps (52 % of the issue slots are taken with 16 x 12 heads x 512 x
+// 512). Where heads leave SMs idle, attention_fwd_few_sm100.cu is the faster one.
 // (us, T5-like scores; one CTA of 16 warps per SM with the scores of all keys in TMEM / here: 128 x 12 heads x
 // 512 x 512 with bias, 60 to 100 % of the keys visible 410 / 305, 114 x 512 without bias 117 / 103, 114 x 114
 // causal 80 / 60. Two groups of four warps per SM in blocks of 128 keys, the kernel in attention_fwd_sm100.cu /

@@ -48,10 +48,10 @@ int t5x_attention_bwd(const void* q, const void* k, const void* v, const void* o
 int t5x_attention_bwd_head_covers(int B, int H, int Lq, int Lk, int D, int num_buckets);
 int t5x_attention_bwd_head(const void* q, const void* k, const void* v, const void* o, const void* d_o,
                            const void* lse, void* dq, void* dk, void* dv, void* dk32, void* dv32, int B,
-                           int H, int Lq, int Lk, long long q_sb, long long q_sl, long long q_sh, long long k_sb, long long k_sl,
-                           long long k_sh, long long v_sb, long long v_sl, long long v_sh, long long o_sb,
-                           long long o_sl, long long o_sh, long long do_sb, long long do_sl,
-                           long long do_sh, long long dq_sb, long long dq_sl, long long dq_sh,
+                           int H, int Lq, int Lk, long long q_sb, long long q_sl, long long q_sh,
+                           long long k_sb, long long k_sl, long long k_sh, long long v_sb, long long v_sl,
+                           long long v_sh, long long o_sb, long long o_sl, long long o_sh, long long do_sb,
+                           long long do_sl, long long do_sh, long long dq_sb, long long dq_sl, long long dq_sh,
                            long long dk_sb, long long dk_sl, long long dk_sh, const void* rel_bias,
                            const void* rel_bucket, void* d_rel_bias, int num_buckets, int nrel,
                            int rel_off, const void* key_mask, const void* q_seg, const void* kv_seg,

@@ -11,6 +11,7 @@ backward, 27 to 57 us a layer for the sort-based index backward alone.)
 from __future__ import annotations
 
 import functools
+import os
 from typing import Optional
 
 import torch
@@ -59,7 +60,6 @@ def forward_kernel(Lq: int, Lk: int, D: int, prefix_lm: bool = False, heads: int
   128 x 128 queries x keys, 6 heads 7.2 / 8.4, 148 7.1 / 9.1, 156 (a second wave) 13.1 / 10.0; 114 x 512, 6 heads
   12.1 / 16.8, 148 13.2 / 17.3, 156 23.8 / 18.7; 256 x 256, 148 heads 14.3 / 17.8; 257 x 257, three blocks in
   turn against two CTAs, 6 heads 24.1 / 14.0, 148 25.1 / 21.4. Both give the same bits."""
-  import os
   classic_ok = D == 64 and Lk <= CLASSIC_MAX_LK
   want = os.environ.get("T5X_B200_ATTN_FWD", "classic")
   if not (classic_ok and want == "classic"):

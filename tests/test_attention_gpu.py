@@ -19,7 +19,7 @@ CASES = [
     (1, 2, 200, 300, True, True, False, True, True),
     (2, 3, 64, 40, False, True, True, False, False),
 ]
-# beyond the short-range forward kernel: the streaming forward with the same backward
+# more than 512 queries or keys: both forward kernels cover them
 LONG_CASES = [
     (1, 2, 640, 640, True, True, False, True, False),
     (1, 2, 1024, 1024, True, False, True, False, False),
@@ -38,7 +38,7 @@ def test_flash_attention_matches_reference(case, kernel, monkeypatch):
   B, H, Lq, Lk, use_bias, bidir, causal, use_mask, use_seg = case
   monkeypatch.setenv("T5X_B200_ATTN_FWD", kernel)
   if A.forward_kernel(Lq, Lk, 64) != kernel:
-    pytest.skip("the short-range forward kernel does not cover this shape")
+    pytest.skip("that forward kernel does not cover this shape")
   torch.manual_seed(0)
   dev = "cuda"
   q = (torch.randn(B, Lq, H, 64, device=dev) * 0.5).bfloat16().requires_grad_(True)

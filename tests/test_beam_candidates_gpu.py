@@ -1,5 +1,6 @@
-"""The beam step's choice of candidates: logits with many equal entries (more than one warp holds: every thread then
-keeps its own), hidden ones, rows that hold fewer than are asked for, against a sort that puts the lower index first."""
+"""The beam step's choice of candidates: logits with many equal entries (more than there is room for: every thread then
+keeps its own), hidden ones, chunks that hold fewer than are asked for, against a sort that puts the lower index
+first; and examples that hold fewer."""
 import pytest
 import torch
 
